@@ -6,6 +6,7 @@ fallback.  ``load()`` raises if the shared object is missing, and every launch h
 """
 from __future__ import annotations
 
+import copy
 import ctypes as C
 from pathlib import Path
 
@@ -242,6 +243,25 @@ def load() -> C.CDLL:
     return lib
 
 
+_native = None
+
+
+def native():
+    """The native call layer (``_native.so``, csrc/native.cpp); raises if it has not been built."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise RuntimeError(
+                "_native.so is missing or does not load: build it with `python -m jvp_flash_attention_b200.build` "
+                f"(this package has no fallback path): {e}"
+            ) from e
+        _native = module
+    return _native
+
+
 def device_status(clear: bool = True) -> int:
     """Synchronises and returns the status word of the tcgen05 kernels (0 = no wait gave up)."""
     lib = load()
@@ -276,7 +296,7 @@ class MaskSpec:
     bias, or int32 kv_len) and ``strides`` are the broadcast element strides of a (B,H,L,L) view.
     """
 
-    __slots__ = ("kind", "tensor", "strides", "bias_dtype", "tile_live", "tile_live_t", "fp32_mode")
+    __slots__ = ("kind", "tensor", "strides", "bias_dtype", "tile_live", "tile_live_t", "fp32_mode", "_native")
 
     def __init__(self, kind=MASK_NONE, tensor=None, strides=(0, 0, 0, 0), bias_dtype=FP32):
         self.kind = kind
@@ -285,7 +305,15 @@ class MaskSpec:
         self.bias_dtype = bias_dtype
         self.tile_live = None  # MASK_BOOL: bitmap from mask_tiles(), lets the forward step over dead tiles
         self.tile_live_t = None  # ... and its transpose (per 128-key tile), for the backward launch that owns keys
+        self._native = None  # the native layer's form of this description, made on first use
         self.fp32_mode = None  # fp32 precision the forward of this call ran under ("3xtf32" / "tf32"); None = current
+
+    def native(self):
+        """This (by now complete) description as the native layer takes it."""
+        if self._native is None:
+            self._native = native().MaskDesc(self.kind, self.bias_dtype, self.tensor, self.strides, self.tile_live,
+                                             self.tile_live_t, copy.copy(self))
+        return self._native
 
     def to_c(self) -> Mask:
         m = Mask()

@@ -3,7 +3,8 @@
 Usage: ``python -m jvp_flash_attention_b200.build [--force] [--verbose]``.
 Each ``csrc/*.cu`` is compiled to an object file under ``csrc/_obj`` (in parallel) and the
 objects are linked into ``jvp_flash_attention_b200/libjvpfa.so``.  A translation unit is rebuilt
-only when it or a header is newer than its object.
+only when it or a header is newer than its object.  ``csrc/native.cpp``, the host side of a call
+(``_native.so``, a Python extension module linked against torch and libjvpfa.so), is built with g++.
 """
 from __future__ import annotations
 
@@ -11,6 +12,7 @@ import argparse
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -18,6 +20,7 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 OBJ = CSRC / "_obj"
 LIB = PKG_DIR / "libjvpfa.so"
+NATIVE = PKG_DIR / "_native.so"
 INCLUDE = PKG_DIR.parent / "include"
 
 NVCC_FLAGS = [
@@ -43,6 +46,22 @@ def _nvcc() -> str:
 def _newest_header() -> float:
     hs = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list(INCLUDE.glob("*.h"))
     return max(h.stat().st_mtime for h in hs)
+
+
+def _native_cmd() -> list[str]:
+    import torch
+    from torch.utils import cpp_extension
+
+    torch_lib = Path(torch.__file__).parent / "lib"
+    return [
+        os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_EXTENSION_NAME=_native",
+        "-I", str(INCLUDE), "-I", sysconfig.get_paths()["include"],
+        *(f"-isystem{p}" for p in cpp_extension.include_paths("cuda")),
+        str(CSRC / "native.cpp"), "-o", str(NATIVE),
+        f"-L{torch_lib}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10",
+        f"-L{PKG_DIR}", "-l:libjvpfa.so", "-Wl,-rpath,$ORIGIN",
+    ]
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -79,6 +98,12 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    src = CSRC / "native.cpp"
+    if force or not NATIVE.exists() or NATIVE.stat().st_mtime < max(src.stat().st_mtime, (INCLUDE / "jvpfa.h").stat().st_mtime):
+        r = subprocess.run(_native_cmd(), capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError("g++ failed for native.cpp")
     return LIB
 
 

@@ -1,0 +1,555 @@
+// Host side of an attention call in C++: argument checks, output allocation, the launches of libjvpfa.so and the
+// autograd graph around them, behind one Python entry point (`attend`).
+//
+// What bounds the calls it serves is host time, not the GPU: up to a few hundred microseconds of kernels, the pass of a
+// program was the Python layer's.  Measured on a B200 machine before and after (a pass through the public API, kernels
+// excluded): attention() 55 -> 9 us, fwd_dual + gradients through both outputs on forward-AD dual tensors about 400 -> 90 us,
+// under torch.func.jvp about 600 -> 250 us (of which torch.func.jvp itself takes some 150).
+//
+// Graph: one node with two outputs, O and tO.  Autograd hands it both cotangents at once, so a loss on both outputs is
+// one backward launch.  Under create_graph the gradient through O is a node that can be differentiated once more (the
+// Hessian-vector product of upstream's missing double backward); the gradient through tO refuses a second differentiation.
+// The tangent rides on O as its forward-mode gradient, set directly instead of through make_dual's view.
+//
+// CUDA tensors go straight to the library.  For tensors of another device the launch is handed back to the Python
+// module's _launch_fwd / _launch_bwd (the CPU suite puts its oracle there), so there is one graph, not two.
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <atomic>
+#include <memory>
+#include <optional>
+#include <string>
+
+#include "jvpfa.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+namespace {
+
+// Process-wide switches of the Python module (its attributes of the same meaning are forwarded here when they are set).
+std::atomic<int> g_impl{JVPFA_IMPL_AUTO};
+std::atomic<bool> g_single_pass{true};
+
+py::object& python_module() {
+  static py::object* m = new py::object(py::module_::import("jvp_flash_attention_b200.jvp_attention"));  // lives as long as the process
+  return *m;
+}
+
+// The kernel-side mask description, built once per mask.  `spec` is the Python object it was made from.
+struct MaskDesc {
+  jvpfa_mask c{};
+  Tensor tensor, tile_live, tile_live_t;
+  std::shared_ptr<py::object> spec;
+
+  MaskDesc(int kind, int bias_dtype, std::optional<Tensor> t, std::array<int64_t, 4> strides, std::optional<Tensor> live,
+           std::optional<Tensor> live_t, py::object spec_)
+      : spec(new py::object(std::move(spec_)), [](py::object* o) {
+          py::gil_scoped_acquire gil;
+          delete o;
+        }) {
+    c.kind = kind;
+    c.bias_dtype = bias_dtype;
+    for (int i = 0; i < 4; ++i) c.stride[i] = strides[i];
+    if (t) tensor = *t;
+    if (live) tile_live = *live;
+    if (live_t) tile_live_t = *live_t;
+    if (kind == JVPFA_MASK_KVLEN)
+      c.kv_len = static_cast<const int32_t*>(tensor.data_ptr());
+    else if (kind == JVPFA_MASK_BOOL || kind == JVPFA_MASK_BIAS)
+      c.ptr = tensor.data_ptr();
+  }
+};
+using MaskPtr = std::shared_ptr<MaskDesc>;
+
+// What a call's backward has to know besides its tensors.
+struct Call {
+  MaskPtr mask;
+  double scale;
+  bool tf32;  // fp32 tensors: one TF32 product instead of three, recorded so that the backward recomputes what the forward saw
+};
+
+bool is_wrapped(const Tensor& x) {
+  return x.key_set().has(c10::DispatchKey::FuncTorchGradWrapper) || x.key_set().has(c10::DispatchKey::FuncTorchBatched);
+}
+
+// The tensor under functorch's wrappers (met only when a transform is differentiated around the call: the slow way).
+Tensor unwrap(Tensor x) {
+  while (x.defined() && is_wrapped(x)) {
+    py::gil_scoped_acquire gil;
+    x = py::module_::import("torch._C._functorch").attr("get_unwrapped")(x).cast<Tensor>();
+  }
+  return x;
+}
+
+const void* data(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
+
+int dtype_of(const Tensor& t, bool tf32) {
+  switch (t.scalar_type()) {
+    case at::kBFloat16:
+      return JVPFA_BF16;
+    case at::kHalf:
+      return JVPFA_FP16;
+    case at::kFloat:
+      return tf32 ? JVPFA_FP32_TF32 : JVPFA_FP32;
+    default:
+      return -1;
+  }
+}
+
+void check_status(int rc, const char* what) {
+  if (rc == JVPFA_OK) return;
+  std::string msg = std::string(what) + " failed: [" + std::to_string(rc) + "] " + jvpfa_strerror(rc);
+  const std::string cuda = jvpfa_last_cuda_error();
+  if (!cuda.empty()) msg += " | " + cuda;
+  throw std::runtime_error(msg);
+}
+
+// Allocation without the dispatcher: these run inside functorch levels as well, and a call makes up to nine of them.
+Tensor empty(at::IntArrayRef sizes, at::ScalarType dtype, at::Device device) {
+  return Tensor(at::detail::empty_cuda(sizes, dtype, device, std::nullopt));
+}
+
+// Operators on plain tensors while a functorch level may be active: without its dispatch keys.
+struct NoFunctorch {
+  c10::impl::ExcludeDispatchKeyGuard guard;
+  NoFunctorch()
+      : guard(c10::DispatchKeySet({c10::DispatchKey::FuncTorchDynamicLayerFrontMode, c10::DispatchKey::FuncTorchDynamicLayerBackMode})) {}
+};
+
+struct NoFunctorchScope {  // the same as a Python context manager
+  std::optional<NoFunctorch> guard;
+};
+
+// Common (batch, head, row) strides of tensors the kernels can read in place.  True with st all zero: row-major.
+bool common_layout(std::initializer_list<const Tensor*> ts, int64_t* st) {
+  bool dense = true;
+  for (auto* t : ts) dense = dense && (!t->defined() || t->is_contiguous());
+  st[0] = st[1] = st[2] = 0;
+  if (dense) return true;
+  const auto ref = (*ts.begin())->strides();
+  for (auto* t : ts) {
+    if (!t->defined()) continue;
+    if (t->strides() != ref || ref[3] != 1 || (reinterpret_cast<uintptr_t>(t->const_data_ptr()) & 15u) != 0) return false;
+    for (int d = 0; d < 3; ++d)
+      if (ref[d] <= 0 || (ref[d] & 7) != 0) return false;
+  }
+  for (int d = 0; d < 3; ++d) st[d] = ref[d];
+  return true;
+}
+
+struct FwdResult {
+  Tensor o, to, lse, mu;
+};
+using Grads = std::array<Tensor, 3>;
+
+// The six inputs as plain tensors, copied to row-major only when they share no layout the kernels read in place.
+struct Inputs {
+  Tensor q, k, v, tq, tk, tv;
+  int64_t st[3];
+
+  Inputs(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& tq_, const Tensor& tk_, const Tensor& tv_)
+      : q(q_), k(k_), v(v_), tq(tq_), tk(tk_), tv(tv_) {
+    if (!common_layout({&q, &k, &v, &tq, &tk, &tv}, st)) make_dense();
+  }
+  bool strided() const { return st[0] != 0; }
+  void make_dense() {
+    NoFunctorch nf;
+    at::AutoDispatchBelowADInplaceOrView below;
+    for (Tensor* t : {&q, &k, &v, &tq, &tk, &tv})
+      if (t->defined()) *t = t->contiguous();
+    st[0] = st[1] = st[2] = 0;
+  }
+};
+
+// ---- launches ------------------------------------------------------------------------------------------------------
+py::object or_none(const Tensor& t) { return t.defined() ? py::cast(t) : py::object(py::none()); }
+
+FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& tq, const Tensor& tk, const Tensor& tv,
+                     const Call& call) {
+  const bool dual = tq.defined();
+  FwdResult r;
+  if (!q.is_cuda()) {
+    py::gil_scoped_acquire gil;
+    NoFunctorch nf;
+    at::AutoGradMode no_grad(false);
+    py::tuple out = python_module().attr("_launch_fwd")(or_none(q), or_none(k), or_none(v), or_none(tq), or_none(tk), or_none(tv),
+                                                        *call.mask->spec, call.scale);
+    r.o = out[0].cast<Tensor>();
+    if (!out[1].is_none()) r.to = out[1].cast<Tensor>();
+    r.lse = out[2].cast<Tensor>();
+    if (!out[3].is_none()) r.mu = out[3].cast<Tensor>();
+    return r;
+  }
+  c10::cuda::OptionalCUDAGuard guard;
+  if (q.get_device() != c10::cuda::current_device()) guard.set_index(q.get_device());
+  Inputs in(q, k, v, tq, tk, tv);
+  const auto sizes = q.sizes();
+  r.o = empty(sizes, q.scalar_type(), q.device());
+  r.lse = empty(sizes.slice(0, 3), at::kFloat, q.device());
+  if (dual) {
+    r.to = empty(sizes, q.scalar_type(), q.device());
+    r.mu = empty(sizes.slice(0, 3), at::kFloat, q.device());
+  }
+  jvpfa_fwd_args a{};
+  a.struct_size = sizeof(a);
+  a.dtype = dtype_of(q, call.tf32);
+  a.B = (int)sizes[0], a.H = (int)sizes[1], a.L = (int)sizes[2], a.D = (int)sizes[3];
+  a.impl = g_impl;
+  a.sm_scale = (float)call.scale;
+  a.o = r.o.data_ptr();
+  a.lse = static_cast<float*>(r.lse.data_ptr());
+  a.to = dual ? r.to.data_ptr() : nullptr;
+  a.mu = dual ? static_cast<float*>(r.mu.data_ptr()) : nullptr;
+  a.mask = call.mask->c;
+  a.mask_tile_live = data(call.mask->tile_live);
+  void* stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
+  for (;;) {
+    a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
+    a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
+    for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
+    const int rc = jvpfa_fwd(&a, stream);
+    if (rc == JVPFA_ERR_UNSUPPORTED && in.strided()) {  // this kernel family wants row-major inputs
+      in.make_dense();
+      continue;
+    }
+    check_status(rc, "jvpfa_fwd");
+    return r;
+  }
+}
+
+// Gradients of <go, O> + <gto, tO> with respect to q, k, v.
+Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, Tensor tk, Tensor tv, const Tensor& o, Tensor to,
+                 const Tensor& lse, Tensor mu, Tensor go, Tensor gto, const Call& call) {
+  if (!q.is_cuda()) {
+    py::gil_scoped_acquire gil;
+    NoFunctorch nf;
+    at::AutoGradMode no_grad(false);
+    py::tuple out = python_module().attr("_launch_bwd")(or_none(q), or_none(k), or_none(v), or_none(tq), or_none(tk), or_none(tv),
+                                                        or_none(o), or_none(to), or_none(lse), or_none(mu), or_none(go),
+                                                        or_none(gto), *call.mask->spec, call.scale);
+    return {out[0].cast<Tensor>(), out[1].cast<Tensor>(), out[2].cast<Tensor>()};
+  }
+  c10::cuda::OptionalCUDAGuard guard;
+  if (q.get_device() != c10::cuda::current_device()) guard.set_index(q.get_device());
+  for (Tensor* t : {&go, &gto}) {
+    if (!t->defined()) continue;
+    *t = unwrap(*t);
+    if (!t->is_contiguous() || t->scalar_type() != q.scalar_type()) {
+      NoFunctorch nf;
+      at::AutoDispatchBelowADInplaceOrView below;
+      *t = t->to(q.scalar_type()).contiguous();
+    }
+  }
+  if (!gto.defined()) tq = tk = tv = to = mu = Tensor();
+  Inputs in(q, k, v, tq, tk, tv);
+  const auto sizes = q.sizes();
+  const int64_t rows = sizes[0] * sizes[1] * sizes[2];
+  const MaskDesc& m = *call.mask;
+  void* stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
+
+  // One scratch allocation: the three row statistics, and fp32 dQ where the single-pass kernels want it (head dimension
+  // 64, 16-bit; index masks, a boolean mask without tile bitmaps, or through O alone a bias of the tensors' type).
+  const bool index_mask = m.c.kind == JVPFA_MASK_NONE || m.c.kind == JVPFA_MASK_CAUSAL || m.c.kind == JVPFA_MASK_KVLEN;
+  const bool dense_bool = m.c.kind == JVPFA_MASK_BOOL && !m.tile_live.defined() && !m.tile_live_t.defined();
+  const bool bias_o = m.c.kind == JVPFA_MASK_BIAS && !gto.defined() && m.c.bias_dtype == dtype_of(q, false);
+  const bool single = g_single_pass && sizes[3] == 64 && q.scalar_type() != at::kFloat && (index_mask || dense_bool || bias_o);
+  const int64_t stat = (rows + 63) / 64 * 64;  // 256-byte steps
+  Tensor scratch = empty({3 * stat + (single ? rows * sizes[3] : 0)}, at::kFloat, q.device());
+  float* f = static_cast<float*>(scratch.data_ptr());
+
+  jvpfa_pre_args p{};
+  p.struct_size = sizeof(p);
+  p.dtype = dtype_of(q, call.tf32);
+  p.B = (int)sizes[0], p.H = (int)sizes[1], p.L = (int)sizes[2], p.D = (int)sizes[3];
+  p.o = data(o), p.to = data(to), p.go = data(go), p.gto = data(gto);
+  p.mu = static_cast<const float*>(data(mu));
+  p.delta = f, p.eps = f + stat, p.cterm = f + 2 * stat;
+  check_status(jvpfa_bwd_preprocess(&p, stream), "jvpfa_bwd_preprocess");
+
+  Grads g;
+  for (Tensor& t : g) t = empty(sizes, q.scalar_type(), q.device());
+  jvpfa_bwd_args a{};
+  a.struct_size = sizeof(a);
+  a.dtype = p.dtype;
+  a.B = p.B, a.H = p.H, a.L = p.L, a.D = p.D;
+  a.impl = g_impl;
+  a.sm_scale = (float)call.scale;
+  a.go = p.go, a.gto = p.gto;
+  a.lse = static_cast<const float*>(data(lse));
+  a.mu = p.mu;
+  a.delta = p.delta, a.eps = p.eps, a.cterm = p.cterm;
+  a.dq = g[0].data_ptr(), a.dk = g[1].data_ptr(), a.dv = g[2].data_ptr();
+  a.mask = m.c;
+  if (m.tile_live.defined() && m.tile_live_t.defined() && a.L <= 8192) {
+    a.mask_tile_live = data(m.tile_live);
+    a.mask_tile_live_t = data(m.tile_live_t);
+  }
+  a.dq_accum = single ? f + 3 * stat : nullptr;
+  for (;;) {
+    a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
+    a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
+    for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
+    const int rc = jvpfa_bwd(&a, stream);
+    if (rc == JVPFA_ERR_UNSUPPORTED && in.strided()) {
+      in.make_dense();
+      continue;
+    }
+    check_status(rc, "jvpfa_bwd");
+    return g;
+  }
+}
+
+Tensor zeros_like_input(const Tensor& q) {
+  NoFunctorch nf;
+  at::AutoDispatchBelowADInplaceOrView below;
+  return at::zeros_like(q);
+}
+
+// ---- graph ---------------------------------------------------------------------------------------------------------
+// Stands behind gradients that cannot be differentiated again, and says so when asked.
+struct Refuse : public Node {
+  std::string message;
+  explicit Refuse(std::string m) : message(std::move(m)) {}
+  variable_list apply(variable_list&&) override { throw std::runtime_error(message); }
+  std::string name() const override { return "JVPAttnRefuse"; }
+};
+
+template <typename... Ts>
+void attach_refusal(const char* message, std::initializer_list<Tensor*> outs, const Ts&... inputs) {
+  if (!torch::autograd::compute_requires_grad(inputs...)) return;
+  auto node = std::shared_ptr<Refuse>(new Refuse(message), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(inputs...));
+  for (Tensor* t : outs)
+    if (t->defined()) torch::autograd::set_history(*t, node);
+}
+
+Tensor primal_of(const Tensor& x) {  // inside a forward-AD level the saved tensors are still dual
+  return x.defined() && x._fw_grad(0).defined() ? x._fw_primal(0) : x;
+}
+
+// (dq, dk, dv) = d<do, O>/d(q, k, v), as a node that can be differentiated once more.  With u the incoming gradients of
+// (dq, dk, dv):  d<(dq,dk,dv), u>/d(q,k,v) = d<tO(q,k,v; u), do>/d(q,k,v)  and  d<...>/d(do) = tO(q,k,v; u), so a
+// Hessian-vector product is one primal + tangent forward with tangents u and one backward through the tangent output.
+struct AttnBwdNode : public Node {
+  Call call;
+  SavedVariable q, k, v, go;
+
+  variable_list apply(variable_list&& u) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(4);
+    if (!u[0].defined() && !u[1].defined() && !u[2].defined()) return out;
+    const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), go_ = go.unpack();
+    const Tensor qp = unwrap(q_), kp = unwrap(k_), vp = unwrap(v_), gop = unwrap(go_);
+    Tensor t[3];
+    {
+      NoFunctorch nf;
+      at::AutoDispatchBelowADInplaceOrView below;
+      for (int i = 0; i < 3; ++i) t[i] = u[i].defined() ? unwrap(u[i]).contiguous() : at::zeros_like(qp, at::MemoryFormat::Contiguous);
+    }
+    FwdResult f = launch_fwd(qp, kp, vp, t[0], t[1], t[2], call);
+    if (task_should_compute_output(0) || task_should_compute_output(1) || task_should_compute_output(2)) {
+      Grads h = launch_bwd(qp, kp, vp, t[0], t[1], t[2], f.o, f.to, f.lse, f.mu, Tensor(), gop, call);
+      for (int i = 0; i < 3; ++i) out[i] = h[i];
+    }
+    if (task_should_compute_output(3)) out[3] = f.to;
+    if (at::GradMode::is_enabled())
+      attach_refusal("trying to differentiate twice a function that was marked with @once_differentiable",
+                     {&out[0], &out[1], &out[2], &out[3]}, q_, k_, v_, go_, u[0], u[1], u[2]);
+    return out;
+  }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable* s : {&q, &k, &v, &go}) s->reset_data();
+  }
+  std::string name() const override { return "JVPAttnBackwardBackward"; }
+};
+
+Grads backward_through_o(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& go,
+                         const Call& call) {
+  Grads g = launch_bwd(unwrap(q), unwrap(k), unwrap(v), Tensor(), Tensor(), Tensor(), o, Tensor(), lse, Tensor(), go, Tensor(), call);
+  if (torch::autograd::compute_requires_grad(q, k, v, go)) {  // create_graph: a second differentiation was asked for
+    auto node = std::shared_ptr<AttnBwdNode>(new AttnBwdNode(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(q, k, v, go));
+    node->call = call;
+    node->q = SavedVariable(q, false);
+    node->k = SavedVariable(k, false);
+    node->v = SavedVariable(v, false);
+    node->go = SavedVariable(go, false);
+    for (Tensor& t : g) torch::autograd::set_history(t, node);
+  }
+  return g;
+}
+
+// The node of a call: outputs O (0) and, with tangents, tO (1); edges to q, k, v and the three tangents.
+struct AttnNode : public Node {
+  Call call;
+  bool dual = false;
+  SavedVariable q, k, v, tq, tk, tv, o, to, lse, mu;
+
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(dual ? 6 : 3);
+    const Tensor go = primal_of(grads[0]);
+    const Tensor gto = grads.size() > 1 ? primal_of(grads[1]) : Tensor();
+    if (!go.defined() && !gto.defined()) return out;
+    const auto self = shared_from_this();
+    const Tensor q_ = primal_of(q.unpack()), k_ = primal_of(k.unpack()), v_ = primal_of(v.unpack());
+    const Tensor o_ = unwrap(o.unpack(self)), lse_ = lse.unpack();
+    const bool need_primals = task_should_compute_output(0) || task_should_compute_output(1) || task_should_compute_output(2);
+    if (!gto.defined()) {
+      if (need_primals) {
+        Grads g = backward_through_o(q_, k_, v_, o_, lse_, go, call);
+        for (int i = 0; i < 3; ++i) out[i] = g[i];
+      }
+      return out;
+    }
+    const Tensor tq_ = tq.unpack(), tk_ = tk.unpack(), tv_ = tv.unpack();
+    const Tensor to_ = unwrap(to.unpack(self)), mu_ = mu.unpack();
+    const Tensor qp = unwrap(q_), kp = unwrap(k_), vp = unwrap(v_), tqp = unwrap(tq_), tkp = unwrap(tk_), tvp = unwrap(tv_);
+    static constexpr const char* kOnce = "the gradient through the tangent output of JVPAttn cannot be differentiated a second time";
+    if (need_primals) {
+      const bool again = at::GradMode::is_enabled();  // a second differentiation was asked for: the part through O stays a node of its own
+      Grads g = launch_bwd(qp, kp, vp, tqp, tkp, tvp, o_, to_, lse_, mu_, again ? Tensor() : go, gto, call);
+      if (again) {
+        attach_refusal(kOnce, {&g[0], &g[1], &g[2]}, q_, k_, v_, tq_, tk_, tv_, gto);
+        if (go.defined()) {
+          Grads h = backward_through_o(q_, k_, v_, o_, lse_, go, call);
+          for (int i = 0; i < 3; ++i) g[i] = h[i] + g[i];
+        }
+      }
+      for (int i = 0; i < 3; ++i) out[i] = g[i];
+    }
+    if (task_should_compute_output(3) || task_should_compute_output(4) || task_should_compute_output(5)) {
+      // with respect to the tangents tO is an ordinary attention output with cotangent gto
+      Grads g = launch_bwd(qp, kp, vp, Tensor(), Tensor(), Tensor(), o_, Tensor(), lse_, Tensor(), gto, Tensor(), call);
+      if (at::GradMode::is_enabled()) attach_refusal(kOnce, {&g[0], &g[1], &g[2]}, q_, k_, v_, tq_, tk_, tv_, gto);
+      for (int i = 0; i < 3; ++i) out[3 + i] = g[i];
+    }
+    return out;
+  }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable* s : {&q, &k, &v, &tq, &tk, &tv, &o, &to, &lse, &mu}) s->reset_data();
+  }
+  std::string name() const override { return "JVPAttnBackward"; }
+};
+
+// ---- entry point ---------------------------------------------------------------------------------------------------
+// What the kernels and the single graph node take: 4-D q, k, v of one shape, type and device, head dimension 32, 64 or
+// 128, and (upstream's check, unless lifted) an even length of at least 32.  Everything else goes back to the Python
+// layer, which words the errors.
+bool acceptable(const Tensor& q, const Tensor& k, const Tensor& v, bool strict_length) {
+  if (q.dim() != 4 || q.layout() != at::kStrided) return false;
+  if (k.sizes() != q.sizes() || v.sizes() != q.sizes()) return false;
+  if (k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return false;
+  if (k.device() != q.device() || v.device() != q.device()) return false;
+  const int64_t L = q.size(2), D = q.size(3);
+  if (strict_length && (L % 2 != 0 || L < 32)) return false;
+  if (D != 32 && D != 64 && D != 128) return false;
+  return !q.is_cuda() || dtype_of(q, false) >= 0;
+}
+
+// Tangent as the kernels read it: q's type, zero where there is none.
+Tensor tangent(const Tensor& t, const Tensor& q) {
+  if (!t.defined()) return zeros_like_input(q);
+  if (t.scalar_type() == q.scalar_type()) return t;
+  NoFunctorch nf;
+  return t.to(q.scalar_type());
+}
+
+struct Outputs {
+  Tensor o, to;
+};
+
+// The call itself on plain tensors; tangents all undefined or all given.  nullopt: not a case for this path.
+std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, Tensor tk, Tensor tv,
+                                    const MaskPtr& mask, std::optional<double> scale, bool tf32, bool strict_length) {
+  for (const Tensor& t : {q, k, v, tq, tk, tv})
+    if (t.defined() && is_wrapped(t)) return std::nullopt;
+  if (!acceptable(q, k, v, strict_length)) return std::nullopt;
+  const bool dual = tq.defined() || tk.defined() || tv.defined();
+  if (dual) {
+    for (const Tensor* t : {&tq, &tk, &tv})
+      if (t->defined() && (t->sizes() != q.sizes() || t->device() != q.device())) return std::nullopt;
+    tq = tangent(tq, q), tk = tangent(tk, q), tv = tangent(tv, q);
+  }
+  Call call{mask, scale ? *scale : 1.0 / std::sqrt((double)q.size(3)), tf32};
+  FwdResult r = launch_fwd(q, k, v, tq, tk, tv, call);
+  const bool grad_primals = torch::autograd::compute_requires_grad(q, k, v);
+  if (grad_primals || torch::autograd::compute_requires_grad(tq, tk, tv)) {
+    auto node = std::shared_ptr<AttnNode>(new AttnNode(), torch::autograd::deleteNode);
+    node->call = call;
+    node->dual = dual;
+    node->set_next_edges(dual ? torch::autograd::collect_next_edges(q, k, v, tq, tk, tv)
+                              : torch::autograd::collect_next_edges(q, k, v));
+    node->q = SavedVariable(q, false);
+    node->k = SavedVariable(k, false);
+    node->v = SavedVariable(v, false);
+    if (grad_primals)
+      torch::autograd::set_history(r.o, node);
+    else
+      node->add_input_metadata(Node::undefined_input());
+    if (dual) {
+      torch::autograd::set_history(r.to, node);
+      node->tq = SavedVariable(tq, false);
+      node->tk = SavedVariable(tk, false);
+      node->tv = SavedVariable(tv, false);
+      node->to = SavedVariable(r.to, true);
+      node->mu = SavedVariable(r.mu, false);
+    }
+    node->o = SavedVariable(r.o, grad_primals);
+    node->lse = SavedVariable(r.lse, false);
+  }
+  return Outputs{r.o, r.to};
+}
+
+// attention (dual = false) or fwd_dual (true) on plain or forward-AD dual tensors outside functorch transforms.  None:
+// not a case for this path (bad arguments, wrapped tensors, dual inputs of a primal-only call); the caller takes its
+// general route.
+py::object attend(const Tensor& q, const Tensor& k, const Tensor& v, const MaskPtr& mask, std::optional<double> scale, bool tf32,
+                  bool dual, bool strict_length) {
+  const Tensor tq = q._fw_grad(0), tk = k._fw_grad(0), tv = v._fw_grad(0);
+  if (!dual && (tq.defined() || tk.defined() || tv.defined())) return py::none();
+  auto out = attend_plain(q, k, v, tq, tk, tv, mask, scale, tf32, strict_length);
+  if (!out) return py::none();
+  if (out->to.defined()) out->o._set_fw_grad(out->to, /*level=*/0, /*is_inplace_op=*/false);
+  return py::cast(out->o);
+}
+
+// The same with the tangents as explicit arguments, for torch.func.jvp: returns (O, tO) on plain tensors, which the
+// caller wraps again.
+py::object attend_dual(const Tensor& q, const Tensor& k, const Tensor& v, std::optional<Tensor> tq, std::optional<Tensor> tk,
+                       std::optional<Tensor> tv, const MaskPtr& mask, std::optional<double> scale, bool tf32, bool strict_length) {
+  auto out = attend_plain(q, k, v, tq.value_or(Tensor()), tk.value_or(Tensor()), tv.value_or(Tensor()), mask, scale, tf32, strict_length);
+  if (!out || !out->to.defined()) return py::none();
+  return py::make_tuple(out->o, out->to);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_native, m) {
+  py::class_<NoFunctorchScope>(m, "NoFunctorch")
+      .def(py::init<>())
+      .def("__enter__", [](NoFunctorchScope& s) { s.guard.emplace(); })
+      .def("__exit__", [](NoFunctorchScope& s, py::args) { s.guard.reset(); });
+  py::class_<MaskDesc, MaskPtr>(m, "MaskDesc")
+      .def(py::init<int, int, std::optional<Tensor>, std::array<int64_t, 4>, std::optional<Tensor>, std::optional<Tensor>, py::object>());
+  m.def("attend", &attend);
+  m.def("attend_dual", &attend_dual);
+  m.def("tangent_of", [](const Tensor& x) { return or_none(x._fw_grad(0)); });
+  m.def("set_tangent", [](const Tensor& x, const Tensor& t) { x._set_fw_grad(t, /*level=*/0, /*is_inplace_op=*/false); });
+  m.def("set_impl", [](int v) { g_impl = v; });
+  m.def("set_single_pass", [](bool v) { g_single_pass = v; });
+}

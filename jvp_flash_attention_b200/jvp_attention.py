@@ -23,6 +23,8 @@ from __future__ import annotations
 
 import copy
 import inspect
+import sys
+import types
 import weakref
 from typing import Any, Literal, NamedTuple
 
@@ -90,17 +92,6 @@ def _unwrap(x):
     return x
 
 
-def _lone_jvp_interpreter():
-    """The interpreter of torch.func.jvp when that is the only functorch transform in force, else None (nested
-    transforms take the generic route for autograd Functions)."""
-    top = torch._C._functorch.peek_interpreter_stack()
-    if top is None or top.level() != 1 or top.key() != torch._C._functorch.TransformType.Jvp:
-        return None
-    from torch._functorch.pyfunctorch import retrieve_current_functorch_interpreter
-
-    return retrieve_current_functorch_interpreter()
-
-
 def _require_cuda(*ts: Tensor) -> None:
     for t in ts:
         if t is not None and not t.is_cuda:
@@ -134,6 +125,14 @@ _MASK_MEMO: dict = {}
 _MASK_MEMO_MAX = 16
 
 
+def _remembered_mask(attn_mask: Tensor, q_shape) -> _lib.MaskSpec | None:
+    """The description classify_mask found for this very tensor, unmodified since, or None."""
+    hit = _MASK_MEMO.get(id(attn_mask)) if MASK_MEMO_ENABLED else None
+    if hit is not None and hit[0]() is attn_mask and hit[1] == (*q_shape[:3], True, attn_mask._version):
+        return hit[2][0]
+    return None
+
+
 def classify_mask(attn_mask: Tensor | None, causal: bool, Z: int, H: int, N: int, qdtype: torch.dtype,
                   verify: bool) -> tuple[_lib.MaskSpec, int, Tensor | None]:
     """Turns the user's mask into the kernel's description.
@@ -160,7 +159,7 @@ def classify_mask(attn_mask: Tensor | None, causal: bool, Z: int, H: int, N: int
         # the entry goes when the caller's tensor object does (the description holds a view of the mask's storage and
         # must not keep it alive)
         k_id = id(attn_mask)
-        _MASK_MEMO[k_id] = (weakref.ref(attn_mask, lambda _r, k_id=k_id: _MASK_MEMO.pop(k_id, None)), key,
+        _MASK_MEMO[k_id] = (weakref.ref(attn_mask, lambda _r, k_id=k_id, pop=_MASK_MEMO.pop: pop(k_id, None)), key,
                             (copy.copy(spec), mask_type))
     except TypeError:  # an object that cannot be weakly referenced: no memo
         pass
@@ -398,13 +397,8 @@ def _zero_scalar(device) -> Tensor:
     return z.detach()
 
 
-def _forward_impl(q, k, v, q_t, k_t, v_t, attn_mask, dropout_p, causal, sm_scale, verify_attn_mask):
-    """Checks, mask classification and the launch of the fused forward, shared by JVPAttn.forward and its lean twin
-    (JVPAttn's nested types are looked up when it is called).
-    Returns (o, o_t, M, mu, mask_spec, MASK_TYPE, mask_tensor, sm_scale, HEAD_DIM_K, grid)."""
-    if dropout_p != 0.0:
-        raise NotImplementedError("Dropout is not currently supported in JVP attention.")
-
+def _check_args(q, k, v, q_t, k_t, v_t, attn_mask, causal):
+    """Upstream's argument checks, with its wording (jvp_attention.py:2356-2400)."""
     Z, H, N_CTX, HEAD_DIM_Q = q.shape
     HEAD_DIM_K = k.shape[-1]
     HEAD_DIM_V = v.shape[-1]
@@ -430,6 +424,16 @@ def _forward_impl(q, k, v, q_t, k_t, v_t, attn_mask, dropout_p, causal, sm_scale
     if q.dtype not in _lib.DTYPE_ENUM:
         raise TypeError(f"unsupported dtype {q.dtype}; expected bfloat16, float16 or float32")
     _require_cuda(q, k, v, q_t, k_t, v_t, attn_mask)
+
+
+def _forward_impl(q, k, v, q_t, k_t, v_t, attn_mask, dropout_p, causal, sm_scale, verify_attn_mask):
+    """Checks, mask classification and the launch of the fused forward, shared by JVPAttn.forward and its lean twin
+    (JVPAttn's nested types are looked up when it is called).
+    Returns (o, o_t, M, mu, mask_spec, MASK_TYPE, mask_tensor, sm_scale, HEAD_DIM_K, grid)."""
+    if dropout_p != 0.0:
+        raise NotImplementedError("Dropout is not currently supported in JVP attention.")
+    _check_args(q, k, v, q_t, k_t, v_t, attn_mask, causal)
+    Z, H, N_CTX, HEAD_DIM_K = q.shape
 
     if sm_scale is None:
         sm_scale = HEAD_DIM_K**-0.5
@@ -577,8 +581,7 @@ class JVPAttn(Function):
         """Primal-only attention (upstream: jvp_attention.py:2701-2752).  Returns O."""
         if dropout_p != 0.0:
             raise NotImplementedError("Dropout is not currently supported in JVP attention.")
-        # every positional argument given: the quick signature binding applies
-        return _Attn.apply(q, k, v, None, None, None, attn_mask, causal, sm_scale, True)[0]
+        return _attend(q, k, v, attn_mask, causal, sm_scale, False)
 
     @staticmethod
     def fwd_dual(
@@ -600,15 +603,7 @@ class JVPAttn(Function):
         """
         if dropout_p != 0.0:
             raise NotImplementedError("Dropout is not currently supported in JVP attention.")
-        interp = _lone_jvp_interpreter()
-        if interp is not None:
-            out = _fwd_dual_inside_func_jvp(interp, q, k, v, attn_mask, causal, sm_scale)
-            if out is not None:
-                return out
-        _, q_t = fwAD.unpack_dual(q)
-        _, k_t = fwAD.unpack_dual(k)
-        _, v_t = fwAD.unpack_dual(v)
-        return _Attn.apply(q, k, v, q_t, k_t, v_t, attn_mask, causal, sm_scale, True)[0]
+        return _attend(q, k, v, attn_mask, causal, sm_scale, True)
 
     @staticmethod
     def jvp(ctx: "JVPAttn.FnCtx", gq: Tensor, gk: Tensor, gv: Tensor, *_) -> "JVPAttn.JVPOut":
@@ -653,27 +648,53 @@ def _backward_impl(ctx, do):
     return _AttnBwd.apply(q, k, v, o.detach(), M, fwAD.unpack_dual(do).primal, ctx.mask_spec, ctx.sm_scale)
 
 
-def _fwd_dual_inside_func_jvp(interp, q, k, v, attn_mask, causal, sm_scale):
-    """``fwd_dual`` when ``torch.func.jvp`` is the only transform in force, done the way the transform treats a
-    built-in operator: take primals and tangents off the transform's wrappers, run one level down on plain tensors
-    (the tangents as explicit arguments, as the kernel wants them anyway), and put the two results back together as
-    a dual tensor of the transform's level.  The generic route for an ``autograd.Function`` (a class generated per
-    call, every argument and output flattened as a pytree once per level) costs several times the kernels at
-    moderate sizes: 0.42 ms against 0.1 ms per call.  Returns None when a tangent is missing (generic route)."""
-    fc = torch._C._functorch
-    level = interp.level()
-    duals = [fwAD.unpack_dual(x) for x in (q, k, v)]
-    if any(d.tangent is None for d in duals):
-        return None
-    raw = [fc._unwrap_for_grad(d.primal, level) for d in duals] + [fc._unwrap_for_grad(d.tangent, level) for d in duals]
-    if isinstance(attn_mask, Tensor):
-        attn_mask = fc._unwrap_for_grad(fwAD.unpack_dual(attn_mask).primal, level)
-    with interp.lower():  # the caller's grad mode stays as it is
-        o, aux, relay = _Attn.apply(*raw, attn_mask, causal, sm_scale, True)
-        o_t, M, mu, spec, scale, link = aux.value
-        if torch.is_grad_enabled() and any(x.requires_grad for x in raw):  # the tangent output carries a gradient: same node as in _Attn.jvp
-            o_t = _TangentBridge.apply(*raw, o_t, o, M, mu, spec, scale, relay, link)
-    return fwAD.make_dual(fc._wrap_for_grad(o, level), fc._wrap_for_grad(o_t, level))
+_NO_MASK = _lib.MaskSpec(_lib.MASK_NONE)
+_CAUSAL = _lib.MaskSpec(_lib.MASK_CAUSAL)
+_functorch = torch._C._functorch
+_peek_functorch = _functorch.peek_interpreter_stack
+_JVP = _functorch.TransformType.Jvp
+
+
+def _attend(q, k, v, attn_mask, causal, sm_scale, dual):
+    """The call behind ``fwd`` and ``fwd_dual``: the mask is looked up or classified here, everything else happens in
+    the native layer (csrc/native.cpp).  What that does not take (bad arguments, nested transforms) goes through the
+    Python Function, which words the errors."""
+    interp = _peek_functorch()
+    in_jvp = interp is not None and dual and interp.level() == 1 and interp.key() == _JVP  # torch.func.jvp alone
+    if interp is None or in_jvp:
+        native = _lib.native()
+        if attn_mask is None:
+            spec = _CAUSAL if causal else _NO_MASK
+            if not q.is_cuda:
+                _check_args(q, k, v, None, None, None, None, causal)
+        else:
+            if in_jvp and _functorch.is_functorch_wrapped_tensor(attn_mask):
+                attn_mask = _functorch._unwrap_for_grad(attn_mask, 1)
+            spec = None if causal else _remembered_mask(attn_mask, q.shape)
+            if spec is None:
+                _check_args(q, k, v, None, None, None, attn_mask, causal)
+                with native.NoFunctorch():  # the mask is a plain tensor, and so is what is found out about it
+                    spec = classify_mask(attn_mask, causal, *q.shape[:3], q.dtype, True)[0]
+        tf32 = _lib.FP32_PRECISION == "tf32"
+        if not in_jvp:
+            out = native.attend(q, k, v, spec.native(), sm_scale, tf32, dual, STRICT_SEQUENCE_LENGTH)
+            if out is not None:
+                return out
+        else:
+            # Primals and tangents are taken off the transform's wrappers, the call runs one level down on plain
+            # tensors, and the two results become a dual tensor of its level again, as for a built-in operator.
+            raw = [_functorch._unwrap_for_grad(x, 1) for x in (q, k, v)]
+            for x in (q, k, v):
+                t = native.tangent_of(x)
+                raw.append(None if t is None else _functorch._unwrap_for_grad(t, 1))
+            out = native.attend_dual(*raw, spec.native(), sm_scale, tf32, STRICT_SEQUENCE_LENGTH)
+            if out is not None:
+                o = _functorch._wrap_for_grad(out[0], 1)
+                native.set_tangent(o, _functorch._wrap_for_grad(out[1], 1))
+                return o
+    q_t, k_t, v_t = (fwAD.unpack_dual(x).tangent for x in (q, k, v)) if dual else (None, None, None)
+    # every positional argument given: the quick signature binding applies
+    return _Attn.apply(q, k, v, q_t, k_t, v_t, attn_mask, causal, sm_scale, True)[0]
 
 
 class _Box:
@@ -687,8 +708,8 @@ class _Box:
 
 
 class _Attn(Function):
-    """What ``JVPAttn.fwd`` and ``JVPAttn.fwd_dual`` call: the same forward, jvp and backward as ``JVPAttn``, whose
-    second output is one opaque holder of (o_t, M, mu, mask description, scale) instead of upstream's nested
+    """The general route of ``JVPAttn.fwd`` and ``JVPAttn.fwd_dual`` (functorch transforms other than a lone
+    ``torch.func.jvp``): the same forward, jvp and backward as ``JVPAttn``, whose second output is one opaque holder of (o_t, M, mu, mask description, scale) instead of upstream's nested
     NamedTuples.  Under ``torch.func.jvp`` every output of a custom Function is wrapped and unwrapped as a pytree once
     per transform level; the NamedTuples (some twenty leaves) made that the larger part of a call's host time.
     ``JVPAttn.apply`` keeps upstream's output structure for callers that use it directly."""
@@ -784,3 +805,17 @@ def scaled_dot_product_attention(query: Tensor, key: Tensor, value: Tensor, attn
     """
     return JVPAttn.fwd_dual(query, key, value, attn_mask=attn_mask, dropout_p=dropout_p, causal=is_causal,
                             sm_scale=scale)
+
+
+class _Module(types.ModuleType):
+    """Forwards the launch switches to the native layer when they are set."""
+
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        if name == "KERNEL_IMPL":
+            _lib.native().set_impl(value)
+        elif name == "SINGLE_PASS_BACKWARD":
+            _lib.native().set_single_pass(value)
+
+
+sys.modules[__name__].__class__ = _Module

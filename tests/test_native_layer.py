@@ -1,0 +1,62 @@
+"""CPU tests of the native call layer (csrc/native.cpp): what the existing wiring tests do not reach.  Launches go to
+the float64 stand-ins of tests/_oracle_launchers.py."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwAD
+
+import jvp_flash_attention_b200.jvp_attention as ja
+from jvp_flash_attention_b200 import _lib
+from oracle import jvp_attention_oracle as orc
+from tests import _oracle_launchers as stand_in
+from tests.test_autograd_wiring import _inputs, cpu_kernels  # noqa: F401
+
+
+def test_a_released_graph_refuses_a_second_backward(cpu_kernels):  # noqa: F811
+    q, k, v, tq, tk, tv, w, _ = _inputs(11)
+    q.requires_grad_()
+    o, to = torch.func.jvp(ja.JVPAttn.fwd_dual, (q, k, v), (tq, tk, tv))
+    torch.autograd.grad((o * w).sum() + (to * w).sum(), q)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad((o * w).sum(), q)
+
+
+@pytest.mark.parametrize("given", ["q", "kv"])
+@pytest.mark.parametrize("route", ["func_jvp", "fwad"])
+def test_missing_tangents_count_as_zero(cpu_kernels, given, route):  # noqa: F811
+    q, k, v, tq, tk, tv, _, w = _inputs(12)
+    z = torch.zeros_like(q)
+    t = [tq if given == "q" else z, tk if given == "kv" else z, tv if given == "kv" else z]
+    a = [x.clone().requires_grad_() for x in (q, k, v)]
+    if route == "fwad":
+        with fwAD.dual_level():
+            d = [fwAD.make_dual(x, y) if y is not z else x for x, y in zip(a, t)]
+            o, to = fwAD.unpack_dual(ja.JVPAttn.fwd_dual(*d))
+    elif given == "q":
+        o, to = torch.func.jvp(lambda x: ja.JVPAttn.fwd_dual(x, a[1], a[2]), (a[0],), (tq,))
+    else:
+        o, to = torch.func.jvp(lambda x, y: ja.JVPAttn.fwd_dual(a[0], x, y), (a[1], a[2]), (tk, tv))
+    g = torch.autograd.grad((to * w).sum(), a)
+    ro, rto, *rg = orc.grads_through_both(q, k, v, *t, None, w)
+    assert orc.max_abs_err(o, ro) < 1e-10 and orc.max_abs_err(to, rto) < 1e-10
+    for x, y in zip(g, rg):
+        assert orc.max_abs_err(x, y) < 1e-9
+
+
+def test_a_mask_is_verified_once_inside_func_jvp(cpu_kernels, monkeypatch):  # noqa: F811
+    """The mask that a function under torch.func.jvp closes over is the caller's own tensor: its memo entry holds."""
+    q, k, v, tq, tk, tv, _, _ = _inputs(13)
+    mask = torch.rand(1, 2, 32, 32, generator=torch.Generator().manual_seed(1)) > 0.4
+    mask[..., 0] = True
+    calls = []
+    monkeypatch.setattr(_lib, "mask_tiles", lambda *a: (calls.append(1), stand_in.mask_tiles(*a))[1])
+    for _ in range(3):
+        o, to = torch.func.jvp(lambda x, y, z: ja.JVPAttn.fwd_dual(x, y, z, attn_mask=mask), (q, k, v), (tq, tk, tv))
+    ro, rto = orc.sdpa_jvp(q, k, v, tq, tk, tv, attn_mask=mask)
+    assert len(calls) == 1 and orc.max_abs_err(o, ro) < 1e-10 and orc.max_abs_err(to, rto) < 1e-10
+
+
+def test_nested_transforms_take_the_general_route(cpu_kernels):  # noqa: F811
+    q, k, v, tq, tk, tv, w, _ = _inputs(14)
+    g = torch.func.grad(lambda x: (ja.attention(x, k, v) * w).sum())(q)
+    _, _, rdq, _, _ = orc.grads_through_both(q, k, v, tq, tk, tv, w, None)
+    assert orc.max_abs_err(g, rdq) < 1e-9
