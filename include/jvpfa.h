@@ -185,7 +185,13 @@ typedef struct {
    * end, so dQ is reproducible to rounding but not bitwise from run to run.  NULL: the two-launch kernels, which
    * recompute the score tiles for dQ (as upstream does, jvp_attention.py:1415-1707) and are bitwise reproducible. */
   float* dq_accum;
+  /* Gradients nobody asked for: JVPFA_SKIP_DQ or JVPFA_SKIP_DKDV (not both); 0 = all three are formed.  The pointers of
+   * skipped gradients may be NULL.  A caller built without this field (struct_size up to dq_accum) gets all three. */
+  int32_t skip;
 } jvpfa_bwd_args;
+
+#define JVPFA_SKIP_DQ 1
+#define JVPFA_SKIP_DKDV 2
 
 int jvpfa_bwd(const jvpfa_bwd_args* args, void* stream);
 

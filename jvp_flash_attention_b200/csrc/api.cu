@@ -1,5 +1,6 @@
 // C ABI of libjvpfa.so: argument validation and dispatch.  No allocation, no device
 // synchronisation, no exceptions across the boundary.
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 
@@ -12,6 +13,20 @@ static thread_local char g_last_cuda_error[256] = {0};
 void set_last_cuda_error(cudaError_t e, const char* where) {
   snprintf(g_last_cuda_error, sizeof(g_last_cuda_error), "%s: %s (%s)", where, cudaGetErrorName(e),
            cudaGetErrorString(e));
+}
+
+bool SmemOptIn::ensure(const void* kernel, size_t bytes) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (e == cudaSuccess && (__atomic_load_n(&done, __ATOMIC_RELAXED) & bit)) return true;
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e != cudaSuccess) {
+    set_last_cuda_error(e, "cudaFuncSetAttribute");
+    return false;
+  }
+  __atomic_fetch_or(&done, bit, __ATOMIC_RELAXED);
+  return true;
 }
 
 static int check_arch() {
@@ -100,7 +115,10 @@ static int validate_bwd(const jvpfa_bwd_args* a) {
   if (a->struct_size != (int32_t)sizeof(jvpfa_bwd_args)) return JVPFA_ERR_STRUCT;
   int rc = check_shape(a->dtype, a->B, a->H, a->L, a->D);
   if (rc) return rc;
-  if (!a->q || !a->k || !a->v || !a->lse || !a->delta || !a->dq || !a->dk || !a->dv) return JVPFA_ERR_NULL;
+  if (a->skip != 0 && a->skip != JVPFA_SKIP_DQ && a->skip != JVPFA_SKIP_DKDV) return JVPFA_ERR_UNSUPPORTED;
+  if (!a->q || !a->k || !a->v || !a->lse || !a->delta) return JVPFA_ERR_NULL;
+  if (!(a->skip & JVPFA_SKIP_DQ) && !a->dq) return JVPFA_ERR_NULL;
+  if (!(a->skip & JVPFA_SKIP_DKDV) && (!a->dk || !a->dv)) return JVPFA_ERR_NULL;
   if (!a->go && !a->gto) return JVPFA_ERR_NULL;
   if (a->gto && (!a->tq || !a->tk || !a->tv || !a->mu || !a->eps || !a->cterm)) return JVPFA_ERR_NULL;
   const void* ptrs[] = {a->q, a->k, a->v, a->tq, a->tk, a->tv, a->go, a->gto, a->dq, a->dk, a->dv};
@@ -111,6 +129,16 @@ static int validate_bwd(const jvpfa_bwd_args* a) {
   rc = check_strides(a->in_stride);
   if (rc) return rc;
   return check_mask(a->mask);
+}
+
+// The arguments as this build knows them: a caller built before `skip` was added passes a shorter struct.
+static const jvpfa_bwd_args* current_bwd_args(const jvpfa_bwd_args* a, jvpfa_bwd_args* full) {
+  constexpr int32_t kBeforeSkip = (int32_t)offsetof(jvpfa_bwd_args, skip);
+  if (!a || a->struct_size != kBeforeSkip) return a;
+  *full = jvpfa_bwd_args{};
+  memcpy(full, a, kBeforeSkip);
+  full->struct_size = (int32_t)sizeof(jvpfa_bwd_args);
+  return full;
 }
 
 static int validate_pre(const jvpfa_pre_args* a) {
@@ -157,7 +185,9 @@ int jvpfa_fwd_uses_tcgen05(const jvpfa_fwd_args* a) {
   return fwd_tc5_eligible(*a) ? 1 : 0;
 }
 
-int jvpfa_bwd_uses_tcgen05(const jvpfa_bwd_args* a) {
+int jvpfa_bwd_uses_tcgen05(const jvpfa_bwd_args* args) {
+  jvpfa_bwd_args full;
+  const jvpfa_bwd_args* a = current_bwd_args(args, &full);
   if (validate_bwd(a) != JVPFA_OK) return 0;
   if (impl_family(a->impl) == JVPFA_IMPL_GENERIC) return 0;
   return bwd_tc5_eligible(*a) ? 1 : 0;
@@ -185,7 +215,9 @@ int jvpfa_bwd_preprocess(const jvpfa_pre_args* a, void* stream) {
   return launch_pre(*a, static_cast<cudaStream_t>(stream));
 }
 
-int jvpfa_bwd(const jvpfa_bwd_args* a, void* stream) {
+int jvpfa_bwd(const jvpfa_bwd_args* args, void* stream) {
+  jvpfa_bwd_args full;
+  const jvpfa_bwd_args* a = current_bwd_args(args, &full);
   const int rc = check_bwd_request(a);
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -223,9 +255,7 @@ int jvpfa_mask_tiles(const jvpfa_mask_tiles_args* a, void* stream) {
   if (a->mask.kind != JVPFA_MASK_BOOL || !a->mask.ptr) return JVPFA_ERR_MASK;
   for (int d = 0; d < 4; ++d)
     if (a->mask.stride[d] < 0) return JVPFA_ERR_MASK;
-  if (a->mask.stride[3] != 1 || (a->L & 15) != 0 || !aligned16(a->mask.ptr) || (a->mask.stride[0] & 15) != 0 ||
-      (a->mask.stride[1] & 15) != 0 || (a->mask.stride[2] & 15) != 0)
-    return JVPFA_ERR_UNSUPPORTED;
+  if (!tc5_mask_layout(a->mask, JVPFA_BF16, a->L)) return JVPFA_ERR_UNSUPPORTED;
   const int rc = check_arch();
   if (rc) return rc;
   return launch_mask_tiles(*a, static_cast<cudaStream_t>(stream));

@@ -121,20 +121,32 @@ int launch_pre(const jvpfa_pre_args& a, cudaStream_t s) {
 }
 
 // ----------------------------------------------------------------------------------------------
-// Main kernels
+// Main kernels.  A CTA of RG x KG warps owns 16*RG rows (keys for dK / dV, queries for dQ) and loops over tiles of the
+// other side; warp (rg, kg) owns 16 of the rows and the kg-th part of every loop tile, sums its own dK, dV or dQ, and the
+// KG partial sums are added once at the end (a fixed order: results stay reproducible bit for bit).  As in the forward
+// (fwd_generic.cu) the bound is mma.sync, three instructions for an fp32 product, and the split puts two warps on each
+// quarter of an SM that shared memory would otherwise leave with one, and lets small shapes use more SMs.
+//
+// All score products of a tile are formed in two sweeps over D, {S, tS} and {E, F + dP}, so that an operand fragment is
+// read and split once for everything it multiplies.
 // ----------------------------------------------------------------------------------------------
-template <typename T, int D>
+template <typename T, int D, int RG, int KG>
 struct BwdCfg {
-  static constexpr int OWN = 64;  // rows owned by the CTA (4 warps x 16)
-  static constexpr int LOOP = (Elem<T>::k16 && D <= 64) ? 64 : 32;
+  static constexpr int OWN = 16 * RG;  // rows owned by the CTA
+  static constexpr int NTHREADS = 32 * RG * KG;
+  static constexpr int LOOP = Elem<T>::k16 ? (D > 64 ? 32 : 64) : (KG >= 8 ? 64 : 32);
+  static constexpr int LW = LOOP / KG;  // loop rows of a warp
   static constexpr int LD = D + Elem<T>::kPad;
-  static constexpr int NTHREADS = 128;
-  static constexpr int STAGES = (!Elem<T>::k16 && D >= 128) ? 1 : 2;
+  static constexpr int STAGES = (!Elem<T>::k16 && D > 64 && (RG >= 4 || LOOP > 32)) ? 1 : 2;
   static constexpr int NSTAT = 5;  // lse, delta, eps, cterm, mu
-  // own_tiles / loop_tiles = number of [rows][D] operand tiles of each kind
+  // own_tiles / loop_tiles = number of [rows][D] operand tiles of each kind; outs = accumulators that are merged
+  static constexpr size_t ring(int loop_tiles) {
+    const size_t r = sizeof(T) * (size_t)STAGES * loop_tiles * LOOP * LD;
+    const size_t merge = sizeof(float) * (size_t)(RG * KG / 2) * 16 * D;  // reuses the ring
+    return r > merge ? r : merge;
+  }
   static constexpr size_t smem(int own_tiles, int loop_tiles, bool stats) {
-    return sizeof(T) * ((size_t)own_tiles * OWN * LD + (size_t)STAGES * loop_tiles * LOOP * LD) +
-           (stats ? sizeof(float) * STAGES * NSTAT * LOOP : 0);
+    return sizeof(T) * (size_t)own_tiles * OWN * LD + ring(loop_tiles) + (stats ? sizeof(float) * STAGES * NSTAT * LOOP : 0);
   }
 };
 
@@ -149,66 +161,77 @@ __device__ __forceinline__ void zero_acc(float (*x)[4]) {
   }
 }
 
-// acc[NTILES][4] += A[r0..r0+15][0..D) * B[0..8*NTILES)[0..D)^T   (both operands D-contiguous)
-template <typename T, int D, int NTILES>
-__device__ __forceinline__ void gemm_nt(float (*acc)[4], const T* sA, const T* sB, int ld, int r0, int lane) {
+// x += A0 B0^T and, where asked for, y += A1 B0^T (HAS_Y1) + A0 B1^T (HAS_Y2); rows r0.. of A0 / A1, all operands D-contiguous.
+// {S, tS} with (Q, tQ; K, tK), {E, F + dP} with (V, tV; G, gO) of the side in question.
+template <typename T, int D, int NT_, bool HAS_Y1, bool HAS_Y2>
+__device__ __forceinline__ void gemm_pair(float (*x)[4], float (*y)[4], const T* sA0, const T* sA1, const T* sB0, const T* sB1, int ld,
+                                          int r0, int lane) {
   constexpr int KS = Elem<T>::kKStep;
-#pragma unroll
+#pragma unroll 4
   for (int k0 = 0; k0 < D; k0 += KS) {
-    FragA<T> fa;
-    load_a<T>(fa, sA, ld, r0, k0, lane);
+    FragA<T> a0, a1;
+    load_a<T>(a0, sA0, ld, r0, k0, lane);
+    if constexpr (HAS_Y1) load_a<T>(a1, sA1, ld, r0, k0, lane);
+    FragB<T> b0[NT_], b1[HAS_Y2 ? NT_ : 1];
 #pragma unroll
-    for (int nt = 0; nt < NTILES; ++nt) {
-      FragB<T> fb;
-      load_b_nt<T>(fb, sB, ld, nt * 8, k0, lane);
-      mma<T>(acc[nt], fa, fb);
+    for (int nt = 0; nt < NT_; ++nt) {
+      load_b_nt<T>(b0[nt], sB0, ld, nt * 8, k0, lane);
+      if constexpr (HAS_Y2) load_b_nt<T>(b1[nt], sB1, ld, nt * 8, k0, lane);
     }
+    auto pass = [&](auto P) {
+#pragma unroll
+      for (int nt = 0; nt < NT_; ++nt) {
+        mma_pass<P()>(x[nt], a0, b0[nt]);
+        if constexpr (HAS_Y1) mma_pass<P()>(y[nt], a1, b0[nt]);
+      }
+      if constexpr (HAS_Y2) {
+#pragma unroll
+        for (int nt = 0; nt < NT_; ++nt) mma_pass<P()>(y[nt], a0, b1[nt]);
+      }
+    };
+    pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
   }
 }
 
-// out[D/8][4] += Atile(accumulator layout, 16 x KROWS) * B[0..KROWS)[0..D)   (B is [k][d], d contiguous)
-template <typename T, int D, int KROWS>
-__device__ __forceinline__ void gemm_acc_nn(float (*out)[4], const float (*atile)[4], const T* sB, int ld,
-                                            int lane) {
+// out[D/8][4] += A0 B0 (+ A1 B1): A from accumulator tiles (16 x KROWS), B = [k][d] tiles, d contiguous.
+// fp32: the tensor core adds into its fp32 accumulator with truncation, and hundreds of such adds into one long-lived
+// accumulator show up as a bias of ~1e-5.  Each contraction step is therefore formed in fresh registers and added rounded.
+template <typename T, int D, int KROWS, bool HAS_0, bool HAS_1>
+__device__ __forceinline__ void gemm_out(float (*out)[4], const float (*at0)[4], const float (*at1)[4], const T* sB0, const T* sB1,
+                                         int ld, int lane) {
   constexpr int KS = Elem<T>::kKStep;
-  if constexpr (Elem<T>::k16) {
+  constexpr int G = 4;  // output tiles at a time
 #pragma unroll
-    for (int kk = 0; kk < KROWS / KS; ++kk) {
-      FragA<T> fa;
-      a_from_acc<T>(fa, atile, kk);
+  for (int kk = 0; kk < KROWS / KS; ++kk) {
+    FragA<T> a0, a1;
+    if constexpr (HAS_0) a_from_acc<T>(a0, at0, kk);
+    if constexpr (HAS_1) a_from_acc<T>(a1, at1, kk);
 #pragma unroll
-      for (int dt = 0; dt < D / 8; ++dt) {
-        FragB<T> fb;
-        load_b_nn<T>(fb, sB, ld, kk * KS, dt * 8, lane);
-        mma<T>(out[dt], fa, fb);
+    for (int d0 = 0; d0 < D / 8; d0 += G) {
+      FragB<T> b0[G], b1[G];
+      float tmp[G][4];
+#pragma unroll
+      for (int i = 0; i < G; ++i) {
+        if constexpr (HAS_0) load_b_nn<T>(b0[i], sB0, ld, kk * KS, (d0 + i) * 8, lane);
+        if constexpr (HAS_1) load_b_nn<T>(b1[i], sB1, ld, kk * KS, (d0 + i) * 8, lane);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) tmp[i][e] = Elem<T>::k16 ? out[d0 + i][e] : 0.f;
       }
-    }
-  } else {
-    // fp32: the tensor core adds into its fp32 accumulator with truncation, and hundreds of such
-    // adds into one long-lived accumulator show up as a bias of ~1e-5.  Accumulate this tile's
-    // contribution in a fresh register tile (32 columns at a time) and add it once, rounded.
+      auto pass = [&](auto P) {
+        if constexpr (HAS_0) {
 #pragma unroll
-    for (int d0 = 0; d0 < D / 8; d0 += 4) {
-      float tmp[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) tmp[i][0] = tmp[i][1] = tmp[i][2] = tmp[i][3] = 0.f;
-#pragma unroll
-      for (int kk = 0; kk < KROWS / KS; ++kk) {
-        FragA<T> fa;
-        a_from_acc<T>(fa, atile, kk);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          FragB<T> fb;
-          load_b_nn<T>(fb, sB, ld, kk * KS, (d0 + i) * 8, lane);
-          mma<T>(tmp[i], fa, fb);
+          for (int i = 0; i < G; ++i) mma_pass<P()>(tmp[i], a0, b0[i]);
         }
-      }
+        if constexpr (HAS_1) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        out[d0 + i][0] += tmp[i][0];
-        out[d0 + i][1] += tmp[i][1];
-        out[d0 + i][2] += tmp[i][2];
-        out[d0 + i][3] += tmp[i][3];
+          for (int i = 0; i < G; ++i) mma_pass<P()>(tmp[i], a1, b1[i]);
+        }
+      };
+      pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
+#pragma unroll
+      for (int i = 0; i < G; ++i) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) out[d0 + i][e] = Elem<T>::k16 ? tmp[i][e] : out[d0 + i][e] + tmp[i][e];
       }
     }
   }
@@ -243,14 +266,15 @@ __device__ __forceinline__ void smem_tile_to_global(T* ghead, const T* s, int ld
 
 // ---- dK, dV: CTA owns 64 keys, loops over query tiles.  Tiles are held transposed
 // (rows = keys, columns = queries) so that P^T etc. feed the second MMAs from registers. ----
-template <typename T, int D, bool HAS_GO, bool HAS_GT>
-__global__ void __launch_bounds__(128) bwd_dkdv_kernel(const jvpfa_bwd_args a) {
-  using C = BwdCfg<T, D>;
-  constexpr int BN = C::OWN, BM = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES;
-  constexpr int NQ = BM / 8;
+template <typename T, int D, bool HAS_GO, bool HAS_GT, int RG, int KG>
+__global__ void __launch_bounds__(32 * RG * KG) bwd_dkdv_kernel(const jvpfa_bwd_args a) {
+  using C = BwdCfg<T, D, RG, KG>;
+  constexpr int BN = C::OWN, BM = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES, LW = C::LW;
+  constexpr int NQ = LW / 8;
   constexpr int ND = D / 8;
   constexpr int OWN_TILES = HAS_GT ? 4 : 2;
   constexpr int LOOP_TILES = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0);
+  static_assert(LW % Elem<T>::kKStep == 0, "a warp's loop rows are whole contraction steps");
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sK = reinterpret_cast<T*>(smem_raw);
@@ -258,9 +282,10 @@ __global__ void __launch_bounds__(128) bwd_dkdv_kernel(const jvpfa_bwd_args a) {
   T* sTK = sK + 2 * BN * LD;  // HAS_GT only
   T* sTV = sK + 3 * BN * LD;  // HAS_GT only
   T* sLoop = sK + OWN_TILES * BN * LD;
-  float* sStat = reinterpret_cast<float*>(sLoop + (size_t)STAGES * LOOP_TILES * BM * LD);
+  float* sStat = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(sLoop) + C::ring(LOOP_TILES));
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rg = warp % RG, kg = warp / RG;
   const int g = lane >> 2, t = lane & 3;
   const int L = a.L;
   const int bh = blockIdx.y;
@@ -323,7 +348,7 @@ __global__ void __launch_bounds__(128) bwd_dkdv_kernel(const jvpfa_bwd_args a) {
   cp_async_commit();
 
   const float scale_log2 = a.sm_scale * kLog2e;
-  const int r0 = warp * 16;
+  const int r0 = rg * 16;
   const int key_lo = n0 + r0 + g, key_hi = key_lo + 8;
 
   float dk[ND][4], dv[ND][4];
@@ -346,106 +371,86 @@ __global__ void __launch_bounds__(128) bwd_dkdv_kernel(const jvpfa_bwd_args a) {
     }
     __syncthreads();
 
-    const T* base = sLoop + (size_t)stage * LOOP_TILES * BM * LD;
-    const T* sQ = base;
-    const T* sGO = base + BM * LD;                       // HAS_GO
-    const T* sTQ = base + (1 + (HAS_GO ? 1 : 0)) * BM * LD;  // HAS_GT
-    const T* sG = sTQ + BM * LD;                          // HAS_GT
-    const float* st = sStat + stage * C::NSTAT * BM;
+    // this warp's queries of the tile (none of them may see its keys: nothing to do)
+    const int mw = m0 + kg * LW;
+    if (mw < L && !(mv.kind == JVPFA_MASK_CAUSAL && mw + LW <= n0 + r0)) {
+      const T* sQ = sLoop + (size_t)stage * LOOP_TILES * BM * LD + kg * LW * LD;
+      const T* sGO = sQ + BM * LD;                           // HAS_GO
+      const T* sTQ = sQ + (1 + (HAS_GO ? 1 : 0)) * BM * LD;  // HAS_GT
+      const T* sG = sTQ + BM * LD;                           // HAS_GT
+      const float* st = sStat + stage * C::NSTAT * BM + kg * LW;
 
-    // P^T
-    float p[NQ][4];
-    zero_acc<NQ>(p);
-    gemm_nt<T, D, NQ>(p, sK, sQ, LD, r0, lane);
+      bool ok[NQ][4];  // fetched ahead of the products that hide its latency
+      float bias[NQ][4];
 #pragma unroll
-    for (int nt = 0; nt < NQ; ++nt) {
+      for (int nt = 0; nt < NQ; ++nt) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int j = (e < 2) ? key_lo : key_hi;
-        const int ci = nt * 8 + 2 * t + (e & 1);
-        const int i = m0 + ci;
-        float v = 0.f;
-        if (mv.allowed(i, j)) {
-          const float x = p[nt][e] * scale_log2 + mv.bias(i, j) * kLog2e;
-          v = exp2f(x - st[ci]);
+        for (int e = 0; e < 4; ++e) {
+          const int i = mw + nt * 8 + 2 * t + (e & 1), j = (e < 2) ? key_lo : key_hi;
+          ok[nt][e] = mv.allowed(i, j);
+          bias[nt][e] = ok[nt][e] ? mv.bias(i, j) : 0.f;
         }
-        p[nt][e] = v;
       }
-    }
-    if constexpr (HAS_GO) gemm_acc_nn<T, D, BM>(dv, p, sGO, LD, lane);
-
-    float acc[NQ][4];
-    zero_acc<NQ>(acc);
-    if constexpr (HAS_GT) {
-      float ts[NQ][4];
+      // S^T, tS^T; E^T (or dP^T), F^T + dP^T
+      float p[NQ][4], ts[NQ][4], e_[NQ][4], f[NQ][4];
+      zero_acc<NQ>(p);
       zero_acc<NQ>(ts);
-      gemm_nt<T, D, NQ>(ts, sK, sTQ, LD, r0, lane);
-      gemm_nt<T, D, NQ>(ts, sTK, sQ, LD, r0, lane);
-      gemm_nt<T, D, NQ>(acc, sV, sG, LD, r0, lane);  // E^T
-      {
-        float w[NQ][4];
-#pragma unroll
-        for (int nt = 0; nt < NQ; ++nt) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int ci = nt * 8 + 2 * t + (e & 1);
-            ts[nt][e] *= a.sm_scale;
-            w[nt][e] = p[nt][e] * (ts[nt][e] - st[4 * BM + ci]);
-          }
-        }
-        gemm_acc_nn<T, D, BM>(dv, w, sG, LD, lane);  // (P*(tS-mu))^T G
-#pragma unroll
-        for (int nt = 0; nt < NQ; ++nt) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int ci = nt * 8 + 2 * t + (e & 1);
-            w[nt][e] = p[nt][e] * (acc[nt][e] - st[2 * BM + ci]);
-          }
-        }
-        gemm_acc_nn<T, D, BM>(dk, w, sTQ, LD, lane);  // gtS^T tQ
-      }
+      zero_acc<NQ>(e_);
+      zero_acc<NQ>(f);
+      gemm_pair<T, D, NQ, HAS_GT, HAS_GT>(p, ts, sK, sTK, sQ, sTQ, LD, r0, lane);
+      if constexpr (HAS_GT)
+        gemm_pair<T, D, NQ, true, HAS_GO>(e_, f, sV, sTV, sG, sGO, LD, r0, lane);
+      else
+        gemm_pair<T, D, NQ, false, false>(f, f, sV, sV, sGO, sGO, LD, r0, lane);
+
 #pragma unroll
       for (int nt = 0; nt < NQ; ++nt) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int ci = nt * 8 + 2 * t + (e & 1);
-          const float tsv = ts[nt][e];
-          acc[nt][e] = acc[nt][e] * (tsv - st[4 * BM + ci]) - st[2 * BM + ci] * tsv;
+          float pv = 0.f;
+          if (ok[nt][e]) pv = exp2f(p[nt][e] * scale_log2 + bias[nt][e] * kLog2e - st[ci]);
+          float sub = st[1 * BM + ci];
+          if constexpr (HAS_GT) {
+            const float tsv = ts[nt][e] * a.sm_scale, ev = e_[nt][e], eps = st[2 * BM + ci], mu = st[4 * BM + ci];
+            sub += st[3 * BM + ci];
+            f[nt][e] += ev * (tsv - mu) - eps * tsv;
+            e_[nt][e] = pv * (ev - eps);  // gtS
+            ts[nt][e] = pv * (tsv - mu);  // A
+          }
+          f[nt][e] = pv * (f[nt][e] - sub);  // gS
+          p[nt][e] = pv;
         }
       }
-      gemm_nt<T, D, NQ>(acc, sTV, sG, LD, r0, lane);  // + F^T
+      // dV += P^T gO + (P*(tS-mu))^T G ;  dK += gS^T Q + gtS^T tQ
+      gemm_out<T, D, LW, HAS_GO, HAS_GT>(dv, p, ts, sGO, sG, LD, lane);
+      gemm_out<T, D, LW, true, HAS_GT>(dk, f, e_, sQ, sTQ, LD, lane);
     }
-    if constexpr (HAS_GO) gemm_nt<T, D, NQ>(acc, sV, sGO, LD, r0, lane);  // + dP^T
-#pragma unroll
-    for (int nt = 0; nt < NQ; ++nt) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int ci = nt * 8 + 2 * t + (e & 1);
-        float sub = st[1 * BM + ci];
-        if constexpr (HAS_GT) sub += st[3 * BM + ci];
-        acc[nt][e] = p[nt][e] * (acc[nt][e] - sub);
-      }
-    }
-    gemm_acc_nn<T, D, BM>(dk, acc, sQ, LD, lane);  // gS^T Q
     __syncthreads();
   }
   cp_async_wait<0>();
   __syncthreads();
+  if constexpr (KG > 1) {
+    merge_parts<RG, KG, ND>(reinterpret_cast<float4*>(sLoop), dk, rg, kg, lane);
+    merge_parts<RG, KG, ND>(reinterpret_cast<float4*>(sLoop), dv, rg, kg, lane);
+  }
 
   // Own K / V buffers are idle now: reuse them to coalesce the stores.
-  acc_to_smem<T, D>(sK, LD, r0, lane, dk, a.sm_scale);
-  acc_to_smem<T, D>(sV, LD, r0, lane, dv, 1.f);
+  if (kg == 0) {
+    acc_to_smem<T, D>(sK, LD, r0, lane, dk, a.sm_scale);
+    acc_to_smem<T, D>(sV, LD, r0, lane, dv, 1.f);
+  }
   __syncthreads();
   smem_tile_to_global<T, BN, D, NT>(reinterpret_cast<T*>(a.dk) + head_off, sK, LD, n0, L, tid);
   smem_tile_to_global<T, BN, D, NT>(reinterpret_cast<T*>(a.dv) + head_off, sV, LD, n0, L, tid);
 }
 
 // ---- dQ: CTA owns 64 queries, loops over key tiles (rows = queries, columns = keys). ----
-template <typename T, int D, bool HAS_GO, bool HAS_GT>
-__global__ void __launch_bounds__(128) bwd_dq_kernel(const jvpfa_bwd_args a) {
-  using C = BwdCfg<T, D>;
-  constexpr int BM = C::OWN, BN = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES;
-  constexpr int NK = BN / 8;
+template <typename T, int D, bool HAS_GO, bool HAS_GT, int RG, int KG>
+__global__ void __launch_bounds__(32 * RG * KG) bwd_dq_kernel(const jvpfa_bwd_args a) {
+  using C = BwdCfg<T, D, RG, KG>;
+  constexpr int BM = C::OWN, BN = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES, LW = C::LW;
+  constexpr int NK = LW / 8;
   constexpr int ND = D / 8;
   constexpr int OWN_TILES = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0);
   constexpr int LOOP_TILES = HAS_GT ? 4 : 2;
@@ -458,6 +463,7 @@ __global__ void __launch_bounds__(128) bwd_dq_kernel(const jvpfa_bwd_args a) {
   T* sLoop = sQ + OWN_TILES * BM * LD;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rg = warp % RG, kg = warp / RG;
   const int g = lane >> 2, t = lane & 3;
   const int L = a.L;
   const int bh = blockIdx.y;
@@ -507,7 +513,7 @@ __global__ void __launch_bounds__(128) bwd_dq_kernel(const jvpfa_bwd_args a) {
   cp_async_commit();
 
   const float scale_log2 = a.sm_scale * kLog2e;
-  const int r0 = warp * 16;
+  const int r0 = rg * 16;
   const int row[2] = {m0 + r0 + g, m0 + r0 + g + 8};
   float lse[2], sub[2], eps[2] = {0.f, 0.f}, mu[2] = {0.f, 0.f};
 #pragma unroll
@@ -541,96 +547,80 @@ __global__ void __launch_bounds__(128) bwd_dq_kernel(const jvpfa_bwd_args a) {
     }
     __syncthreads();
 
-    const T* sK = sLoop + (size_t)stage * LOOP_TILES * BN * LD;
-    const T* sV = sK + BN * LD;
-    const T* sTK = sK + 2 * BN * LD;
-    const T* sTV = sK + 3 * BN * LD;
+    const int nw = n0 + kg * LW;  // this warp's keys of the tile
+    if (nw < n_end && !(mv.kind == JVPFA_MASK_CAUSAL && nw > m0 + r0 + 15)) {
+      const T* sK = sLoop + (size_t)stage * LOOP_TILES * BN * LD + kg * LW * LD;
+      const T* sV = sK + BN * LD;
+      const T* sTK = sK + 2 * BN * LD;
+      const T* sTV = sK + 3 * BN * LD;
 
-    float p[NK][4];
-    zero_acc<NK>(p);
-    gemm_nt<T, D, NK>(p, sQ, sK, LD, r0, lane);
+      bool ok[NK][4];  // fetched ahead of the products that hide its latency
+      float bias[NK][4];
 #pragma unroll
-    for (int nt = 0; nt < NK; ++nt) {
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {  // accumulator elements 2r, 2r+1: one query row, keys j and j + 1
-        bool ok[2];
-        float bias[2];
-        mv.pair(row[r], n0 + nt * 8 + 2 * t, ok, bias);
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int e = 2 * r + c;
-          float v = 0.f;
-          if (ok[c]) v = exp2f(p[nt][e] * scale_log2 + bias[c] * kLog2e - lse[r]);
-          p[nt][e] = v;
-        }
+      for (int nt = 0; nt < NK; ++nt) {
+        mv.pair(row[0], nw + nt * 8 + 2 * t, &ok[nt][0], &bias[nt][0]);
+        mv.pair(row[1], nw + nt * 8 + 2 * t, &ok[nt][2], &bias[nt][2]);
       }
-    }
-
-    float acc[NK][4];
-    zero_acc<NK>(acc);
-    if constexpr (HAS_GT) {
-      float ts[NK][4];
+      float p[NK][4], ts[NK][4], e_[NK][4], f[NK][4];
+      zero_acc<NK>(p);
       zero_acc<NK>(ts);
-      gemm_nt<T, D, NK>(ts, sTQ, sK, LD, r0, lane);
-      gemm_nt<T, D, NK>(ts, sQ, sTK, LD, r0, lane);
-      gemm_nt<T, D, NK>(acc, sG, sV, LD, r0, lane);  // E
-      {
-        float w[NK][4];
-#pragma unroll
-        for (int nt = 0; nt < NK; ++nt) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            ts[nt][e] *= a.sm_scale;
-            w[nt][e] = p[nt][e] * (acc[nt][e] - eps[e >> 1]);
-          }
-        }
-        gemm_acc_nn<T, D, BN>(dq, w, sTK, LD, lane);  // gtS tK
+      zero_acc<NK>(e_);
+      zero_acc<NK>(f);
+      gemm_pair<T, D, NK, HAS_GT, HAS_GT>(p, ts, sQ, sTQ, sK, sTK, LD, r0, lane);
+      if constexpr (HAS_GT) {
+        // E = G V^T, F = G tV^T; dP = gO V^T shares V
+        gemm_pair<T, D, NK, HAS_GO, true>(e_, f, sG, sGO, sV, sTV, LD, r0, lane);
+      } else {
+        gemm_pair<T, D, NK, false, false>(f, f, sGO, sGO, sV, sV, LD, r0, lane);
       }
+
 #pragma unroll
       for (int nt = 0; nt < NK; ++nt) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float tsv = ts[nt][e];
-          acc[nt][e] = acc[nt][e] * (tsv - mu[e >> 1]) - eps[e >> 1] * tsv;
+        for (int r = 0; r < 2; ++r) {  // accumulator elements 2r, 2r+1: one query row, keys j and j + 1
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int e = 2 * r + c;
+            float pv = 0.f;
+            if (ok[nt][e]) pv = exp2f(p[nt][e] * scale_log2 + bias[nt][e] * kLog2e - lse[r]);
+            if constexpr (HAS_GT) {
+              const float tsv = ts[nt][e] * a.sm_scale, ev = e_[nt][e];
+              f[nt][e] += ev * (tsv - mu[r]) - eps[r] * tsv;
+              e_[nt][e] = pv * (ev - eps[r]);  // gtS
+            }
+            f[nt][e] = pv * (f[nt][e] - sub[r]);  // gS
+          }
         }
       }
-      gemm_nt<T, D, NK>(acc, sG, sTV, LD, r0, lane);  // + F
+      gemm_out<T, D, LW, true, HAS_GT>(dq, f, e_, sK, sTK, LD, lane);  // gS K + gtS tK
     }
-    if constexpr (HAS_GO) gemm_nt<T, D, NK>(acc, sGO, sV, LD, r0, lane);  // + dP
-#pragma unroll
-    for (int nt = 0; nt < NK; ++nt) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[nt][e] = p[nt][e] * (acc[nt][e] - sub[e >> 1]);
-    }
-    gemm_acc_nn<T, D, BN>(dq, acc, sK, LD, lane);  // gS K
     __syncthreads();
   }
   cp_async_wait<0>();
   __syncthreads();
+  if constexpr (KG > 1) merge_parts<RG, KG, ND>(reinterpret_cast<float4*>(sLoop), dq, rg, kg, lane);
 
-  acc_to_smem<T, D>(sQ, LD, r0, lane, dq, a.sm_scale);
+  if (kg == 0) acc_to_smem<T, D>(sQ, LD, r0, lane, dq, a.sm_scale);
   __syncthreads();
   smem_tile_to_global<T, BM, D, NT>(reinterpret_cast<T*>(a.dq) + head_off, sQ, LD, m0, L, tid);
 }
 
-template <typename T, int D, bool HAS_GO, bool HAS_GT>
+template <typename T, int D, bool HAS_GO, bool HAS_GT, int RG, int KG>
 static int launch_bwd_one(const jvpfa_bwd_args& a, cudaStream_t stream) {
-  using C = BwdCfg<T, D>;
-  const int go = HAS_GO ? 1 : 0, gt = HAS_GT ? 1 : 0;
-  const size_t smem_kv = C::smem(gt ? 4 : 2, 1 + go + 2 * gt, true);
-  const size_t smem_q = C::smem(1 + go + 2 * gt, gt ? 4 : 2, false);
-  auto k1 = bwd_dkdv_kernel<T, D, HAS_GO, HAS_GT>;
-  auto k2 = bwd_dq_kernel<T, D, HAS_GO, HAS_GT>;
-  cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q);
-  if (e != cudaSuccess) {
-    set_last_cuda_error(e, "cudaFuncSetAttribute(bwd_generic)");
+  using C = BwdCfg<T, D, RG, KG>;
+  constexpr int go = HAS_GO ? 1 : 0, gt = HAS_GT ? 1 : 0;
+  constexpr size_t smem_kv = C::smem(gt ? 4 : 2, 1 + go + 2 * gt, true);
+  constexpr size_t smem_q = C::smem(1 + go + 2 * gt, gt ? 4 : 2, false);
+  static_assert(smem_kv <= 227 * 1024 && smem_q <= 227 * 1024, "shared memory of one CTA");
+  auto k1 = bwd_dkdv_kernel<T, D, HAS_GO, HAS_GT, RG, KG>;
+  auto k2 = bwd_dq_kernel<T, D, HAS_GO, HAS_GT, RG, KG>;
+  static SmemOptIn opt_in1, opt_in2;
+  if (!opt_in1.ensure(reinterpret_cast<const void*>(k1), smem_kv) || !opt_in2.ensure(reinterpret_cast<const void*>(k2), smem_q))
     return JVPFA_ERR_CUDA;
-  }
   dim3 grid((a.L + C::OWN - 1) / C::OWN, a.B * a.H);
-  k1<<<grid, C::NTHREADS, smem_kv, stream>>>(a);
-  k2<<<grid, C::NTHREADS, smem_q, stream>>>(a);
-  e = cudaGetLastError();
+  if (!(a.skip & JVPFA_SKIP_DKDV)) k1<<<grid, C::NTHREADS, smem_kv, stream>>>(a);
+  if (!(a.skip & JVPFA_SKIP_DQ)) k2<<<grid, C::NTHREADS, smem_q, stream>>>(a);
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch bwd_generic");
     return JVPFA_ERR_CUDA;
@@ -638,12 +628,23 @@ static int launch_bwd_one(const jvpfa_bwd_args& a, cudaStream_t stream) {
   return JVPFA_OK;
 }
 
+template <typename T, int D, int RG, int KG>
+static int launch_bwd_split(const jvpfa_bwd_args& a, cudaStream_t s) {
+  const bool go = a.go != nullptr, gt = a.gto != nullptr;
+  if (go && gt) return launch_bwd_one<T, D, true, true, RG, KG>(a, s);
+  if (gt) return launch_bwd_one<T, D, false, true, RG, KG>(a, s);
+  return launch_bwd_one<T, D, true, false, RG, KG>(a, s);
+}
+
+// Rows x loop parts of a CTA, by the same rule as in the forward.
 template <typename T, int D>
 static int launch_bwd_d(const jvpfa_bwd_args& a, cudaStream_t s) {
-  const bool go = a.go != nullptr, gt = a.gto != nullptr;
-  if (go && gt) return launch_bwd_one<T, D, true, true>(a, s);
-  if (gt) return launch_bwd_one<T, D, false, true>(a, s);
-  return launch_bwd_one<T, D, true, false>(a, s);
+  if constexpr (!Elem<T>::k16) {
+    const long long rows16 = (long long)((a.L + 15) / 16) * a.B * a.H;
+    if (rows16 < 2 * 148) return launch_bwd_split<T, D, 1, 8>(a, s);
+    if (rows16 < 4 * 148) return launch_bwd_split<T, D, 2, 4>(a, s);
+  }
+  return launch_bwd_split<T, D, 4, 2>(a, s);
 }
 
 template <typename T>

@@ -267,10 +267,10 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
       const int i = it.own0 + tid;
       if (tid < OWN && i < L) {
         if constexpr (OWN_KEYS) {
-          poison_row<T>(a.dk, (size_t)it.bh * L + i, D);
-          poison_row<T>(a.dv, (size_t)it.bh * L + i, D);
+          poison_row<T>(a.dk, (size_t)it.bh * L + i, a.D);
+          poison_row<T>(a.dv, (size_t)it.bh * L + i, a.D);
         } else {
-          poison_row<T>(a.dq, (size_t)it.bh * L + i, D);
+          poison_row<T>(a.dq, (size_t)it.bh * L + i, a.D);
         }
       }
     }
@@ -492,6 +492,7 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
         constexpr uint32_t id = wide ? idesc_sc2 : idesc_sc;
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
+          if (ks >= 2 && a.D <= 32) continue;
           if (first && ks == 0)
             umma_ss_lo<false>(d, own_lo + slot * OWN16 + ks * 2, b_lo + ks * 2, id);
           else
@@ -644,8 +645,8 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
 
     // group 0 stores columns [0,32) of every output, group 1 columns [32,64)
     auto store_half = [&](void* gptr, int bh, int own_idx, const uint32_t (&r)[32], float mul) {
-      if (own_idx >= L) return;
-      T* gp = reinterpret_cast<T*>(gptr) + ((size_t)bh * L + own_idx) * D + 32 * wg;
+      if (own_idx >= L || 32 * wg >= a.D) return;
+      T* gp = reinterpret_cast<T*>(gptr) + ((size_t)bh * L + own_idx) * a.D + 32 * wg;
       uint32_t pk[16];
 #pragma unroll
       for (int x = 0; x < 16; ++x)
@@ -751,7 +752,7 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
 #pragma unroll
             for (int j = 0; j < 2 * MESZ; ++j) {
               uint4 r = make_uint4(0u, 0u, 0u, 0u);
-              if (l0 + (j + 1) * (16 / MESZ) <= L) r = ldg_nc_v4(p + 16 * j);
+              if (l0 + j * (16 / MESZ) < L) r = ldg_nc_v4(p + 16 * j);
               raw[4 * j] = r.x, raw[4 * j + 1] = r.y, raw[4 * j + 2] = r.z, raw[4 * j + 3] = r.w;
             }
           }
@@ -921,14 +922,14 @@ static int launch_half64(const jvpfa_bwd_args& a, cudaStream_t stream, int* stat
   const int qry_rows = OWN_KEYS ? C::BL : C::OWN;
   // (64, L, H, B) maps; q, k, v and their tangents may be strided views (in_stride), the cotangents are row-major
   const int64_t* st = a.in_stride;
-  bool ok = encode_map4(&m.k, dt, a.k, a.L, a.H, a.B, st, key_rows) && encode_map4(&m.v, dt, a.v, a.L, a.H, a.B, st, key_rows) &&
-            encode_map4(&m.q, dt, a.q, a.L, a.H, a.B, st, qry_rows);
+  bool ok = encode_map4d(&m.k, dt, a.k, a.D, a.L, a.H, a.B, st, key_rows) && encode_map4d(&m.v, dt, a.v, a.D, a.L, a.H, a.B, st, key_rows) &&
+            encode_map4d(&m.q, dt, a.q, a.D, a.L, a.H, a.B, st, qry_rows);
   m.tk = m.tv = m.k;
   m.go = m.tq = m.g = m.q;
-  if (HAS_GO) ok = ok && encode_map4(&m.go, dt, a.go, a.L, a.H, a.B, nullptr, qry_rows);
+  if (HAS_GO) ok = ok && encode_map4d(&m.go, dt, a.go, a.D, a.L, a.H, a.B, nullptr, qry_rows);
   if (HAS_GT)
-    ok = ok && encode_map4(&m.tk, dt, a.tk, a.L, a.H, a.B, st, key_rows) && encode_map4(&m.tv, dt, a.tv, a.L, a.H, a.B, st, key_rows) &&
-         encode_map4(&m.tq, dt, a.tq, a.L, a.H, a.B, st, qry_rows) && encode_map4(&m.g, dt, a.gto, a.L, a.H, a.B, nullptr, qry_rows);
+    ok = ok && encode_map4d(&m.tk, dt, a.tk, a.D, a.L, a.H, a.B, st, key_rows) && encode_map4d(&m.tv, dt, a.tv, a.D, a.L, a.H, a.B, st, key_rows) &&
+         encode_map4d(&m.tq, dt, a.tq, a.D, a.L, a.H, a.B, st, qry_rows) && encode_map4d(&m.g, dt, a.gto, a.D, a.L, a.H, a.B, nullptr, qry_rows);
   if (!ok) {
     set_last_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled(bwd d64)");
     return JVPFA_ERR_CUDA;
@@ -969,10 +970,12 @@ static int launch_both64(const jvpfa_bwd_args& a, cudaStream_t s) {
     set_last_cuda_error(cudaErrorUnknown, "status word address");
     return JVPFA_ERR_CUDA;
   }
+  // Without the own-keys launch before it, the own-queries launch must not start early: it reads what the preprocess wrote.
+  const bool keys = !(a.skip & JVPFA_SKIP_DKDV);
   int rc = JVPFA_OK;
-  rc = launch_half64<T, true, HAS_GO, HAS_GT, MK>(a, s, status, false);
-  if (rc) return rc;
-  rc = launch_half64<T, false, HAS_GO, HAS_GT, MK>(a, s, status, true);
+  if (keys) rc = launch_half64<T, true, HAS_GO, HAS_GT, MK>(a, s, status, false);
+  if (rc || (a.skip & JVPFA_SKIP_DQ)) return rc;
+  rc = launch_half64<T, false, HAS_GO, HAS_GT, MK>(a, s, status, keys);
   return rc;
 }
 

@@ -199,9 +199,9 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       if (!get_item(k, it)) continue;
       const int i = it.own0 + tid;
       if (tid < OWN && i < L) {
-        poison_row<T>(a.dk, (size_t)it.bh * L + i, D);
-        poison_row<T>(a.dv, (size_t)it.bh * L + i, D);
-        dq_acc[((size_t)it.bh * L + i) * D] = poison_f32();
+        poison_row<T>(a.dk, (size_t)it.bh * L + i, a.D);
+        poison_row<T>(a.dv, (size_t)it.bh * L + i, a.D);
+        dq_acc[((size_t)it.bh * L + i) * a.D] = poison_f32();
       }
     }
   };
@@ -364,7 +364,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           else
             umma_ss_lo<true>(tmem + col, a_lo, b_lo, id);
 #pragma unroll
-          for (int ks = 1; ks < D / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 2, id);
+          for (int ks = 1; ks < D / 16; ++ks)
+            if (ks < 2 || a.D > 32) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 2, id);
         };
         for (int k = 0; ok && k < k_max; ++k) {
           if (!get_item(k, it) || it.n_sub == 0) continue;
@@ -498,7 +499,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 
     auto store_row = [&](void* gptr, int bh, int own_idx, const uint32_t (&r0)[32], const uint32_t (&r1)[32], float mul) {
       if (own_idx >= L) return;
-      T* gp = reinterpret_cast<T*>(gptr) + ((size_t)bh * L + own_idx) * D;
+      T* gp = reinterpret_cast<T*>(gptr) + ((size_t)bh * L + own_idx) * a.D;
 #pragma unroll
       for (int x = 0; x < 4; ++x)
         reinterpret_cast<uint4*>(gp)[x] = make_uint4(
@@ -506,6 +507,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             Elem<T>::pack(__uint_as_float(r0[8 * x + 2]) * mul, __uint_as_float(r0[8 * x + 3]) * mul),
             Elem<T>::pack(__uint_as_float(r0[8 * x + 4]) * mul, __uint_as_float(r0[8 * x + 5]) * mul),
             Elem<T>::pack(__uint_as_float(r0[8 * x + 6]) * mul, __uint_as_float(r0[8 * x + 7]) * mul));
+      if (a.D <= 32) return;
 #pragma unroll
       for (int x = 0; x < 4; ++x)
         reinterpret_cast<uint4*>(gp)[4 + x] = make_uint4(
@@ -717,7 +719,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
         if (tid == 384) {
           const int i0 = it.loop_begin + s * BL;
           tma_reduce_add_4d(&maps.dq, dqs, 0, i0, it.h, it.b);
-          tma_reduce_add_4d(&maps.dq, dqs + 8192, 32, i0, it.h, it.b);
+          if (a.D > 32) tma_reduce_add_4d(&maps.dq, dqs + 8192, 32, i0, it.h, it.b);
           bulk_commit();
         }
       }
@@ -774,15 +776,15 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
   BwdFMaps m;
   const CUtensorMapDataType dt = Fmt<T>::kTma;
   const int64_t* st = a.in_stride;
-  bool ok = encode_map4(&m.k, dt, a.k, a.L, a.H, a.B, st, C::OWN) && encode_map4(&m.v, dt, a.v, a.L, a.H, a.B, st, C::OWN) &&
-            encode_map4(&m.q, dt, a.q, a.L, a.H, a.B, st, C::BL);
+  bool ok = encode_map4d(&m.k, dt, a.k, a.D, a.L, a.H, a.B, st, C::OWN) && encode_map4d(&m.v, dt, a.v, a.D, a.L, a.H, a.B, st, C::OWN) &&
+            encode_map4d(&m.q, dt, a.q, a.D, a.L, a.H, a.B, st, C::BL);
   m.tk = m.tv = m.k;
   m.go = m.tq = m.g = m.q;
-  if (HAS_GO) ok = ok && encode_map4(&m.go, dt, a.go, a.L, a.H, a.B, nullptr, C::BL);
+  if (HAS_GO) ok = ok && encode_map4d(&m.go, dt, a.go, a.D, a.L, a.H, a.B, nullptr, C::BL);
   if (HAS_GT)
-    ok = ok && encode_map4(&m.tk, dt, a.tk, a.L, a.H, a.B, st, C::OWN) && encode_map4(&m.tv, dt, a.tv, a.L, a.H, a.B, st, C::OWN) &&
-         encode_map4(&m.tq, dt, a.tq, a.L, a.H, a.B, st, C::BL) && encode_map4(&m.g, dt, a.gto, a.L, a.H, a.B, nullptr, C::BL);
-  ok = ok && encode_map4d_f32(&m.dq, a.dq_accum, C::D, a.L, a.H, a.B, C::BL);
+    ok = ok && encode_map4d(&m.tk, dt, a.tk, a.D, a.L, a.H, a.B, st, C::OWN) && encode_map4d(&m.tv, dt, a.tv, a.D, a.L, a.H, a.B, st, C::OWN) &&
+         encode_map4d(&m.tq, dt, a.tq, a.D, a.L, a.H, a.B, st, C::BL) && encode_map4d(&m.g, dt, a.gto, a.D, a.L, a.H, a.B, nullptr, C::BL);
+  ok = ok && encode_map4d_f32(&m.dq, a.dq_accum, a.D, a.L, a.H, a.B, C::BL);
   if (!ok) {
     set_last_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled(bwd fused64)");
     return JVPFA_ERR_CUDA;
@@ -792,7 +794,7 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
     set_last_cuda_error(cudaErrorUnknown, "multiprocessor count");
     return JVPFA_ERR_CUDA;
   }
-  const size_t n = (size_t)a.B * a.H * a.L * 64;
+  const size_t n = (size_t)a.B * a.H * a.L * a.D;
   cudaError_t e = cudaMemsetAsync(a.dq_accum, 0, n * sizeof(float), stream);
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "cudaMemsetAsync(dq_accum)");
@@ -813,6 +815,7 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
     return JVPFA_ERR_CUDA;
   }
   const long long n8 = (long long)(n / 8);
+  if (a.skip & JVPFA_SKIP_DQ) return JVPFA_OK;
   dq_convert_kernel<T><<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(a.dq_accum, reinterpret_cast<T*>(a.dq), n8, a.sm_scale);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -841,7 +844,7 @@ static int launch_fused64_t(const jvpfa_bwd_args& a, cudaStream_t s) {
 // The single-pass kernel serves D = 64 with index masks (none, causal, key padding) and boolean masks that come without
 // tile bitmaps, when the caller provides the fp32 accumulation buffer for dQ.
 bool bwd_tc5_fused64_eligible(const jvpfa_bwd_args& a) {
-  if (a.D != 64 || a.dq_accum == nullptr) return false;
+  if (a.D > 64 || a.dq_accum == nullptr) return false;
   if ((reinterpret_cast<uintptr_t>(a.dq_accum) & 15u) != 0) return false;
   const int k = a.mask.kind;
   // A boolean mask without tile bitmaps (dense, or not looked at beforehand): with them the two-launch kernels, which

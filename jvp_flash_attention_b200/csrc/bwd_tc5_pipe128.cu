@@ -525,7 +525,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
 #pragma unroll
           for (int j = 0; j < MESZ; ++j) {
             uint4 r = make_uint4(0u, 0u, 0u, 0u);
-            if (c0 + (j + 1) * (16 / MESZ) <= L) r = ldg_nc_v4(pm + 16 * j);
+            if (c0 + j * (16 / MESZ) < L) r = ldg_nc_v4(pm + 16 * j);
             w[4 * j] = r.x, w[4 * j + 1] = r.y, w[4 * j + 2] = r.z, w[4 * j + 3] = r.w;
           }
 #pragma unroll
@@ -721,9 +721,12 @@ static int launch_pipe_both(const jvpfa_bwd_args& a, cudaStream_t s) {
     set_last_cuda_error(cudaErrorUnknown, "status word address");
     return JVPFA_ERR_CUDA;
   }
-  int rc = launch_pipe_half<T, true, HAS_GO, HAS_GT, MK>(a, s, status, false);
-  if (rc) return rc;
-  return launch_pipe_half<T, false, HAS_GO, HAS_GT, MK>(a, s, status, true);
+  // Without the own-keys launch before it, the own-queries launch must not start early: it reads what the preprocess wrote.
+  const bool keys = !(a.skip & JVPFA_SKIP_DKDV);
+  int rc = JVPFA_OK;
+  if (keys) rc = launch_pipe_half<T, true, HAS_GO, HAS_GT, MK>(a, s, status, false);
+  if (rc || (a.skip & JVPFA_SKIP_DQ)) return rc;
+  return launch_pipe_half<T, false, HAS_GO, HAS_GT, MK>(a, s, status, keys);
 }
 
 template <typename T, int MK>

@@ -79,7 +79,7 @@ struct Elem<tf32x1> {
 // ----------------------------------------------------------------------------------------------
 __device__ __forceinline__ void mma_16816(const __nv_bfloat16*, float c[4], const uint32_t a[4],
                                           const uint32_t b[2]) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};\n"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -87,25 +87,36 @@ __device__ __forceinline__ void mma_16816(const __nv_bfloat16*, float c[4], cons
 }
 __device__ __forceinline__ void mma_16816(const __half*, float c[4], const uint32_t a[4],
                                           const uint32_t b[2]) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};\n"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 __device__ __forceinline__ void mma_1688_tf32(float c[4], const uint32_t a[4], const uint32_t b[2]) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};\n"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// Split an fp32 value into a TF32 "hi" part and the TF32 rounding of the remainder.
+template <int I>
+struct IntC {  // a compile-time int as an argument
+  static constexpr int value = I;
+  __host__ __device__ constexpr int operator()() const { return I; }
+};
+
+// Split an fp32 value into a TF32 "hi" part (11 significant bits) and the TF32 rounding of the remainder.  Dekker's
+// splitting (T. J. Dekker, "A floating-point technique for extending the available precision", Numer. Math. 18, 1971)
+// rounds hi in three operations of the FMA pipe; a tensor core ignores the low 13 bits of a TF32 operand, so half a unit
+// of the last used bit, added as an integer, rounds lo.  A NaN stays one in hi.  Two cvt.rna.tf32 instead cost more issue
+// slots than all the rest of a fragment: D = 128, B2 H8 L1024 primal + tangent forward MEASURED1.
 __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
-  float r = x - __uint_as_float(hi);
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(r));
+  const float c = __fmul_rn(x, 8193.f);  // 2^13 + 1
+  const float h = __fsub_rn(c, __fsub_rn(c, x));
+  hi = __float_as_uint(h);
+  lo = __float_as_uint(__fsub_rn(x, h)) + 0x1000u;
 }
 // The same for element type T: types that multiply in one pass have no lo part.
 template <typename T>
@@ -155,6 +166,21 @@ __device__ __forceinline__ void mma(float c[4], const FragA<T, false>& a, const 
     mma_1688_tf32(c, a.hi, b.lo);
   }
   mma_1688_tf32(c, a.hi, b.hi);
+}
+
+// One of the up to three instructions of a logical MMA: 0 = lo*hi, 1 = hi*lo, 2 = hi*hi (types that multiply in one pass
+// have the last only).  Accumulators that take several products interleave the passes of all of them: an instruction
+// returns after 21 cycles, and the next one on the same accumulator should be three issue slots (of 8 cycles) away.
+template <int PASS, typename T>
+__device__ __forceinline__ void mma_pass(float c[4], const FragA<T, true>& a, const FragB<T, true>& b) {
+  if constexpr (PASS == 2) mma_16816(static_cast<const T*>(nullptr), c, a.r, b.r);
+}
+template <int PASS, typename T>
+__device__ __forceinline__ void mma_pass(float c[4], const FragA<T, false>& a, const FragB<T, false>& b) {
+  if constexpr (PASS == 2)
+    mma_1688_tf32(c, a.hi, b.hi);
+  else if constexpr (Elem<T>::kSplit)
+    mma_1688_tf32(c, PASS == 0 ? a.lo : a.hi, PASS == 0 ? b.hi : b.lo);
 }
 
 // A fragment from a row-major smem tile s[row][k] (k contiguous, leading dimension ld elements):
@@ -376,6 +402,35 @@ __device__ __forceinline__ float quad_sum(float x) {
   return x;
 }
 
+// Sums the register tiles x[ND][4] of the KG warps that share a row group into the kg = 0 warp, halving the number of
+// parts in each step.  buf: (RG * KG / 2) * ND * 32 float4; ends (and begins) with nobody reading it.
+template <int RG, int KG, int ND>
+__device__ __forceinline__ void merge_parts(float4* buf, float (*x)[4], int rg, int kg, int lane) {
+#pragma unroll
+  for (int half = KG / 2; half > 0; half /= 2) {
+    float4* p = buf + (size_t)((kg % half) * RG + rg) * ND * 32 + lane;
+    if (kg >= half && kg < 2 * half) {
+#pragma unroll
+      for (int i = 0; i < ND; ++i) p[i * 32] = make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
+    }
+    __syncthreads();
+    if (kg < half) {
+#pragma unroll
+      for (int i = 0; i < ND; ++i) {
+        const float4 v = p[i * 32];
+        x[i][0] += v.x, x[i][1] += v.y, x[i][2] += v.z, x[i][3] += v.w;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// Raises a kernel's dynamic shared-memory limit once per device (the call costs about a microsecond of host time).
+struct SmemOptIn {
+  unsigned long long done = 0;  // bit per device; setting it twice does no harm
+  bool ensure(const void* kernel, size_t bytes);
+};
+
 // Host-side launch helpers implemented by each kernel translation unit.
 int launch_fwd_generic(const jvpfa_fwd_args& a, cudaStream_t stream);
 int launch_pre(const jvpfa_pre_args& a, cudaStream_t stream);
@@ -384,6 +439,8 @@ int launch_mask_check(const jvpfa_mask_check_args& a, cudaStream_t stream);
 int launch_mask_tiles(const jvpfa_mask_tiles_args& a, cudaStream_t stream);
 int launch_fwd_tc5(const jvpfa_fwd_args& a, cudaStream_t stream);
 bool fwd_tc5_eligible(const jvpfa_fwd_args& a);
+bool tc5_head_dim(int D, int L);
+bool tc5_mask_layout(const jvpfa_mask& m, int dtype, int L);
 int tc5_read_status(int* out, int clear);
 int tc5_status_peek();
 int tc5_inject_status(int code);

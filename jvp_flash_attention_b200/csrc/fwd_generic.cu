@@ -1,9 +1,10 @@
 // Fused primal (+ tangent) attention forward on warp-level tensor-core MMAs.
 //
-// One CTA of 4 warps owns a 64-row query tile of one (batch, head); each warp owns 16 rows.
-// K, tK, V, tV tiles stream through a two-stage cp.async ring in shared memory.  Per tile the
-// warp forms S = Q K^T and tS = tQ K^T + Q tK^T in registers, applies the mask / bias, runs the
-// online softmax (running max m, denominator l and mu = sum P*tS) and feeds P and P*tS straight
+// A CTA of RG x KG warps owns 16*RG query rows of one (batch, head).  Warp (rg, kg) owns 16 of the rows and the kg-th part
+// of every key tile: it keeps a running maximum, denominator, mu and output of its own over its keys, and the KG partial
+// results of a row are merged once, through shared memory, when the keys are through.  K, tK, V, tV tiles stream through
+// a cp.async ring in shared memory.  Per tile the warp forms S = Q K^T and tS = tQ K^T + Q tK^T in registers, applies the
+// mask / bias, runs the online softmax (running max m, denominator l and mu = sum P*tS) and feeds P and P*tS straight
 // from the accumulator registers into the second set of MMAs (O += P V, tO' += (P*tS) V + P tV).
 // Epilogue: O = acc/l, tO = tO'/l - (mu/l) O, lse = m + log2(l)  (base 2, scaled scores).
 //
@@ -11,37 +12,53 @@
 // epilogue at jvp_attention.py:1011-1033, with two deliberate differences: the additive bias
 // is applied as scale*QK^T + bias (SDPA semantics; upstream scales the bias too,
 // jvp_attention.py:247-251), and boolean masking uses -inf rather than adding -100.
+//
+// What bounds it: mma.sync, at 512 (TF32) or 1024 (16-bit) multiply-adds per clock and SM, measured; an fp32 product is
+// three TF32 instructions.  One instruction occupies its quarter of the SM for 8 cycles and returns after 21, and the
+// fp32 products of one accumulator are a chain, so the split matters: 64 rows x D=128 fp32 fill the shared memory of an
+// SM, and with one warp for each 16 rows (KG = 1) a quarter had a single warp to wait for.  With KG = 2 it has two, and
+// shapes with few row tiles use shorter ones with more key parts (see launch_d) instead of leaving SMs idle.
 #include "common.cuh"
 
 namespace jvpfa {
 
-template <typename T, int D>
+template <typename T, int D, int RG, int KG>
 struct FwdCfg {
-  static constexpr int BM = 64;
-  static constexpr int BN = (!Elem<T>::k16 || D > 64) ? 32 : 64;
+  static constexpr int BM = 16 * RG;
+  static constexpr int NTHREADS = 32 * RG * KG;
+  // keys of a warp per tile: enough for one contraction step of the second products; two where the tile fits twice
+  static constexpr int BN = Elem<T>::k16 ? (D > 64 ? 32 : 64) : (KG >= 8 ? 64 : 32);
+  static constexpr int BW = BN / KG;
   static constexpr int LD = D + Elem<T>::kPad;
-  static constexpr int NTHREADS = 128;
-  static constexpr int STAGES = 2;
+  static constexpr int STAGES = (!Elem<T>::k16 && D > 64 && BN > 32) ? 1 : 2;
+  static constexpr size_t tiles(bool dual) {
+    const size_t ring = sizeof(T) * (size_t)STAGES * BN * LD * (dual ? 4 : 2);
+    const size_t merge = sizeof(float) * (size_t)(RG * KG / 2) * 16 * D * (dual ? 2 : 1);  // reuses the ring
+    return ring > merge ? ring : merge;
+  }
   static constexpr size_t smem(bool dual) {
-    return sizeof(T) * ((size_t)BM * LD * (dual ? 2 : 1) + (size_t)STAGES * BN * LD * (dual ? 4 : 2));
+    return sizeof(T) * (size_t)BM * LD * (dual ? 2 : 1) + tiles(dual) + sizeof(float) * 3 * KG * BM;
   }
 };
 
-template <typename T, int D, bool DUAL>
-__global__ void __launch_bounds__(128) fwd_generic_kernel(const jvpfa_fwd_args a) {
-  using C = FwdCfg<T, D>;
-  constexpr int BM = C::BM, BN = C::BN, LD = C::LD, NT = C::NTHREADS;
+template <typename T, int D, bool DUAL, int RG, int KG>
+__global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_fwd_args a) {
+  using C = FwdCfg<T, D, RG, KG>;
+  constexpr int BM = C::BM, BN = C::BN, BW = C::BW, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES;
   constexpr int KS = Elem<T>::kKStep;
-  constexpr int NS = BN / 8;   // score n-tiles per warp row-strip
+  constexpr int NS = BW / 8;   // score n-tiles per warp row-strip
   constexpr int ND = D / 8;    // output n-tiles
   constexpr int NKV = DUAL ? 4 : 2;
+  static_assert(BW % KS == 0, "a warp's keys are whole contraction steps");
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sQ = reinterpret_cast<T*>(smem_raw);
   T* sTQ = sQ + BM * LD;  // only valid when DUAL
   T* sKV = sQ + BM * LD * (DUAL ? 2 : 1);
+  float* sRow = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(sKV) + C::tiles(DUAL));  // [3][KG][BM]
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rg = warp % RG, kg = warp / RG;
   const int g = lane >> 2, t = lane & 3;
   const int L = a.L;
   const int bh = blockIdx.y;
@@ -82,11 +99,11 @@ __global__ void __launch_bounds__(128) fwd_generic_kernel(const jvpfa_fwd_args a
   // Prologue: Q (+tQ) and the first K/V tile in one cp.async group.
   stage_tile<T, BM, D, NT>(sQ, gQ, m0, L, tid, in_rs);
   if constexpr (DUAL) stage_tile<T, BM, D, NT>(sTQ, gTQ, m0, L, tid, in_rs);
-  if (n_tiles > 0) stage_kv(0, 0);
+  if (STAGES == 2 && n_tiles > 0) stage_kv(0, 0);
   cp_async_commit();
 
   const float scale_log2 = a.sm_scale * kLog2e;
-  const int r0 = warp * 16;
+  const int r0 = rg * 16;
   const int row_lo = m0 + r0 + g, row_hi = row_lo + 8;
 
   float acc_o[ND][4];
@@ -104,16 +121,40 @@ __global__ void __launch_bounds__(128) fwd_generic_kernel(const jvpfa_fwd_args a
   float mu_run[2] = {0.f, 0.f};
 
   for (int it = 0; it < n_tiles; ++it) {
-    const int n0 = it * BN;
-    if (it + 1 < n_tiles) stage_kv((it + 1) & 1, n0 + BN);
-    cp_async_commit();
-    cp_async_wait<1>();
+    int stage = 0;
+    if constexpr (STAGES == 2) {
+      if (it + 1 < n_tiles) stage_kv((it + 1) & 1, (it + 1) * BN);
+      cp_async_commit();
+      cp_async_wait<1>();
+      stage = it & 1;
+    } else {
+      stage_kv(0, it * BN);
+      cp_async_commit();
+      cp_async_wait<0>();
+    }
     __syncthreads();
 
-    const T* sK = sKV + (size_t)(it & 1) * NKV * BN * LD;
+    const int n0 = it * BN + kg * BW;  // this warp's keys of the tile
+    // (a part beyond the end, or above the diagonal of the warp's rows, is nobody's work; the barrier below is everybody's)
+    if (n0 < n_end && !(mv.kind == JVPFA_MASK_CAUSAL && n0 > m0 + r0 + 15)) {
+    const T* sK = sKV + (size_t)stage * NKV * BN * LD + kg * BW * LD;
     const T* sV = sK + BN * LD;
     const T* sTK = sK + 2 * BN * LD;
     const T* sTV = sK + 3 * BN * LD;
+
+    // ---- user mask: fetched ahead of the products that hide its latency ----
+    const bool full_tile = (mv.kind == JVPFA_MASK_NONE && n0 + BW <= L && m0 + BM <= L) ||
+                           (mv.kind == JVPFA_MASK_CAUSAL && n0 + BW - 1 <= m0 + r0 && m0 + BM <= L) ||
+                           (mv.kind == JVPFA_MASK_KVLEN && n0 + BW <= mv.kv_len && m0 + BM <= L);
+    bool ok[NS][4];
+    float bias[NS][4];
+    if (!full_tile) {
+#pragma unroll
+      for (int nt = 0; nt < NS; ++nt) {
+        mv.pair(row_lo, n0 + nt * 8 + 2 * t, &ok[nt][0], &bias[nt][0]);
+        mv.pair(row_hi, n0 + nt * 8 + 2 * t, &ok[nt][2], &bias[nt][2]);
+      }
+    }
 
     // ---- scores ----
     float s[NS][4];
@@ -126,46 +167,44 @@ __global__ void __launch_bounds__(128) fwd_generic_kernel(const jvpfa_fwd_args a
         if constexpr (DUAL) ts[i][j] = 0.f;
       }
     }
-#pragma unroll
+#pragma unroll 4
     for (int k0 = 0; k0 < D; k0 += KS) {
       FragA<T> fq, ftq;
       load_a<T>(fq, sQ, LD, r0, k0, lane);
       if constexpr (DUAL) load_a<T>(ftq, sTQ, LD, r0, k0, lane);
+      FragB<T> fk[NS], ftk[DUAL ? NS : 1];
 #pragma unroll
       for (int nt = 0; nt < NS; ++nt) {
-        FragB<T> fk;
-        load_b_nt<T>(fk, sK, LD, nt * 8, k0, lane);
-        mma<T>(s[nt], fq, fk);
-        if constexpr (DUAL) {
-          FragB<T> ftk;
-          load_b_nt<T>(ftk, sTK, LD, nt * 8, k0, lane);
-          mma<T>(ts[nt], ftq, fk);
-          mma<T>(ts[nt], fq, ftk);
-        }
+        load_b_nt<T>(fk[nt], sK, LD, nt * 8, k0, lane);
+        if constexpr (DUAL) load_b_nt<T>(ftk[nt], sTK, LD, nt * 8, k0, lane);
       }
+      auto pass = [&](auto P) {
+#pragma unroll
+        for (int nt = 0; nt < NS; ++nt) {
+          mma_pass<P()>(s[nt], fq, fk[nt]);
+          if constexpr (DUAL) mma_pass<P()>(ts[nt], ftq, fk[nt]);
+        }
+        if constexpr (DUAL) {
+#pragma unroll
+          for (int nt = 0; nt < NS; ++nt) mma_pass<P()>(ts[nt], fq, ftk[nt]);
+        }
+      };
+      pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
     }
 
     // ---- mask / bias, move to the base-2 domain ----
-    const bool full_tile = (mv.kind == JVPFA_MASK_NONE && n0 + BN <= L && m0 + BM <= L) ||
-                           (mv.kind == JVPFA_MASK_CAUSAL && n0 + BN - 1 <= m0 && m0 + BM <= L) ||
-                           (mv.kind == JVPFA_MASK_KVLEN && n0 + BN <= mv.kv_len && m0 + BM <= L);
     float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int nt = 0; nt < NS; ++nt) {
 #pragma unroll
       for (int r = 0; r < 2; ++r) {  // accumulator elements 2r, 2r+1: row_lo / row_hi, keys j, j + 1
-        const int i = r == 0 ? row_lo : row_hi;
-        const int j = n0 + nt * 8 + 2 * t;
-        bool ok[2] = {true, true};
-        float bias[2] = {0.f, 0.f};
-        if (!full_tile) mv.pair(i, j, ok, bias);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           const int e = 2 * r + c;
           float x = s[nt][e] * scale_log2;
           if (!full_tile) {
-            if (ok[c]) {
-              x += bias[c] * kLog2e;
+            if (ok[nt][e]) {
+              x += bias[nt][e] * kLog2e;
             } else {
               x = -INFINITY;
               if constexpr (DUAL) ts[nt][e] = 0.f;
@@ -220,69 +259,96 @@ __global__ void __launch_bounds__(128) fwd_generic_kernel(const jvpfa_fwd_args a
     }
 
     // ---- second MMAs: contraction over the keys of this tile ----
-    if constexpr (Elem<T>::k16) {
+    // fp32: the tensor core adds into its fp32 accumulator with truncation; over a thousand keys that bias reaches
+    // ~1e-5.  Each contraction step is therefore formed in fresh registers and added to the running sums rounded.
 #pragma unroll
-      for (int kk = 0; kk < BN / KS; ++kk) {
-        FragA<T> fp, fw;
-        a_from_acc<T>(fp, s, kk);
-        if constexpr (DUAL) a_from_acc<T>(fw, ts, kk);
+    for (int kk = 0; kk < BW / KS; ++kk) {
+      FragA<T> fp, fw;
+      a_from_acc<T>(fp, s, kk);
+      if constexpr (DUAL) a_from_acc<T>(fw, ts, kk);
+      constexpr int G = 2;  // output tiles at a time
 #pragma unroll
-        for (int dt = 0; dt < ND; ++dt) {
-          FragB<T> fv;
-          load_b_nn<T>(fv, sV, LD, kk * KS, dt * 8, lane);
-          mma<T>(acc_o[dt], fp, fv);
-          if constexpr (DUAL) {
-            FragB<T> ftv;
-            load_b_nn<T>(ftv, sTV, LD, kk * KS, dt * 8, lane);
-            mma<T>(acc_t[dt], fw, fv);
-            mma<T>(acc_t[dt], fp, ftv);
-          }
-        }
-      }
-    } else {
-      // fp32: the tensor core adds into its fp32 accumulator with truncation; over a thousand keys
-      // that bias reaches ~1e-5.  This tile's contribution is therefore accumulated in a fresh
-      // register tile (32 output columns at a time) and added to the running sums once, rounded.
+      for (int d0 = 0; d0 < ND; d0 += G) {
+        FragB<T> fv[G], ftv[DUAL ? G : 1];
+        float xo[G][4], xt[DUAL ? G : 1][4];
 #pragma unroll
-      for (int d0 = 0; d0 < ND; d0 += 4) {
-        float to_[4][4], tt_[DUAL ? 4 : 1][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          to_[i][0] = to_[i][1] = to_[i][2] = to_[i][3] = 0.f;
-          if constexpr (DUAL) tt_[i][0] = tt_[i][1] = tt_[i][2] = tt_[i][3] = 0.f;
-        }
-#pragma unroll
-        for (int kk = 0; kk < BN / KS; ++kk) {
-          FragA<T> fp, fw;
-          a_from_acc<T>(fp, s, kk);
-          if constexpr (DUAL) a_from_acc<T>(fw, ts, kk);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            FragB<T> fv;
-            load_b_nn<T>(fv, sV, LD, kk * KS, (d0 + i) * 8, lane);
-            mma<T>(to_[i], fp, fv);
-            if constexpr (DUAL) {
-              FragB<T> ftv;
-              load_b_nn<T>(ftv, sTV, LD, kk * KS, (d0 + i) * 8, lane);
-              mma<T>(tt_[i], fw, fv);
-              mma<T>(tt_[i], fp, ftv);
-            }
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < G; ++i) {
+          load_b_nn<T>(fv[i], sV, LD, kk * KS, (d0 + i) * 8, lane);
+          if constexpr (DUAL) load_b_nn<T>(ftv[i], sTV, LD, kk * KS, (d0 + i) * 8, lane);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            acc_o[d0 + i][e] += to_[i][e];
-            if constexpr (DUAL) acc_t[d0 + i][e] += tt_[i][e];
+            xo[i][e] = Elem<T>::k16 ? acc_o[d0 + i][e] : 0.f;
+            if constexpr (DUAL) xt[i][e] = Elem<T>::k16 ? acc_t[d0 + i][e] : 0.f;
+          }
+        }
+        auto pass = [&](auto P) {
+#pragma unroll
+          for (int i = 0; i < G; ++i) {
+            mma_pass<P()>(xo[i], fp, fv[i]);
+            if constexpr (DUAL) mma_pass<P()>(xt[i], fw, fv[i]);
+          }
+          if constexpr (DUAL) {
+#pragma unroll
+            for (int i = 0; i < G; ++i) mma_pass<P()>(xt[i], fp, ftv[i]);
+          }
+        };
+        pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            acc_o[d0 + i][e] = Elem<T>::k16 ? xo[i][e] : acc_o[d0 + i][e] + xo[i][e];
+            if constexpr (DUAL) acc_t[d0 + i][e] = Elem<T>::k16 ? xt[i][e] : acc_t[d0 + i][e] + xt[i][e];
           }
         }
       }
     }
+    }  // this warp's part of the tile
     __syncthreads();  // every warp is done with this stage before it is refilled
   }
   cp_async_wait<0>();
   __syncthreads();
+
+  // ---- merge the key parts of a row ----
+  if constexpr (KG > 1) {
+    if (t == 0) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int i = r0 + g + 8 * r;
+        sRow[kg * BM + i] = m_run[r];
+        sRow[(KG + kg) * BM + i] = l_run[r];
+        sRow[(2 * KG + kg) * BM + i] = mu_run[r];
+      }
+    }
+    __syncthreads();
+    float f[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int i = r0 + g + 8 * r;
+      float m = -INFINITY, l = 0.f, mu = 0.f;
+#pragma unroll
+      for (int k = 0; k < KG; ++k) m = fmaxf(m, sRow[k * BM + i]);
+      const float mz = m == -INFINITY ? 0.f : m;
+#pragma unroll
+      for (int k = 0; k < KG; ++k) {
+        const float x = exp2f(sRow[k * BM + i] - mz);
+        l += x * sRow[(KG + k) * BM + i];
+        mu += x * sRow[(2 * KG + k) * BM + i];
+      }
+      f[r] = exp2f(m_run[r] - mz);
+      m_run[r] = m, l_run[r] = l, mu_run[r] = mu;
+    }
+#pragma unroll
+    for (int dt = 0; dt < ND; ++dt) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        acc_o[dt][e] *= f[e >> 1];
+        if constexpr (DUAL) acc_t[dt][e] *= f[e >> 1];
+      }
+    }
+    merge_parts<RG, KG, ND>(reinterpret_cast<float4*>(sKV), acc_o, rg, kg, lane);
+    if constexpr (DUAL) merge_parts<RG, KG, ND>(reinterpret_cast<float4*>(sKV), acc_t, rg, kg, lane);
+  }
 
   // ---- epilogue ----
   float inv_l[2], mu_n[2];
@@ -292,12 +358,13 @@ __global__ void __launch_bounds__(128) fwd_generic_kernel(const jvpfa_fwd_args a
     inv_l[r] = empty ? 0.f : 1.f / l_run[r];
     mu_n[r] = DUAL ? mu_run[r] * inv_l[r] : 0.f;
     const int row = r == 0 ? row_lo : row_hi;
-    if (t == 0 && row < L) {
+    if (kg == 0 && t == 0 && row < L) {
       a.lse[(size_t)bh * L + row] = empty ? INFINITY : (m_run[r] + log2f(l_run[r]));
       if constexpr (DUAL) a.mu[(size_t)bh * L + row] = mu_n[r];
     }
   }
   // Stage the output tiles through the (now idle) Q / tQ buffers for 16-byte coalesced stores.
+  if (kg == 0) {
 #pragma unroll
   for (int dt = 0; dt < ND; ++dt) {
     float o0 = acc_o[dt][0] * inv_l[0], o1 = acc_o[dt][1] * inv_l[0];
@@ -318,6 +385,7 @@ __global__ void __launch_bounds__(128) fwd_generic_kernel(const jvpfa_fwd_args a
       qhi[1] = Elem<T>::from_float(acc_t[dt][3] * inv_l[1] - mu_n[1] * o3);
     }
   }
+  }
   __syncthreads();
   {
     constexpr int VEC = 16 / (int)sizeof(T);
@@ -337,19 +405,17 @@ __global__ void __launch_bounds__(128) fwd_generic_kernel(const jvpfa_fwd_args a
   }
 }
 
-template <typename T, int D, bool DUAL>
+template <typename T, int D, bool DUAL, int RG, int KG>
 static int launch_one(const jvpfa_fwd_args& a, cudaStream_t stream) {
-  using C = FwdCfg<T, D>;
-  const size_t smem = C::smem(DUAL);
-  auto kern = fwd_generic_kernel<T, D, DUAL>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) {
-    set_last_cuda_error(e, "cudaFuncSetAttribute(fwd_generic)");
-    return JVPFA_ERR_CUDA;
-  }
+  using C = FwdCfg<T, D, RG, KG>;
+  constexpr size_t smem = C::smem(DUAL);
+  static_assert(smem <= 227 * 1024, "shared memory of one CTA");
+  auto kern = fwd_generic_kernel<T, D, DUAL, RG, KG>;
+  static SmemOptIn opt_in;
+  if (!opt_in.ensure(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_CUDA;
   dim3 grid((a.L + C::BM - 1) / C::BM, a.B * a.H);
   kern<<<grid, C::NTHREADS, smem, stream>>>(a);
-  e = cudaGetLastError();
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch fwd_generic");
     return JVPFA_ERR_CUDA;
@@ -357,9 +423,16 @@ static int launch_one(const jvpfa_fwd_args& a, cudaStream_t stream) {
   return JVPFA_OK;
 }
 
+// Rows x key parts of a CTA.  64 rows share every key tile that is brought in, so they are the choice once they give
+// each of the 148 SMs a CTA; below that shorter row tiles (whose warps share out the keys) put more SMs to work.
 template <typename T, int D>
 static int launch_d(const jvpfa_fwd_args& a, cudaStream_t s) {
-  return a.tq ? launch_one<T, D, true>(a, s) : launch_one<T, D, false>(a, s);
+  if constexpr (!Elem<T>::k16) {
+    const long long rows16 = (long long)((a.L + 15) / 16) * a.B * a.H;
+    if (rows16 < 2 * 148) return a.tq ? launch_one<T, D, true, 1, 8>(a, s) : launch_one<T, D, false, 1, 8>(a, s);
+    if (rows16 < 4 * 148) return a.tq ? launch_one<T, D, true, 2, 4>(a, s) : launch_one<T, D, false, 2, 4>(a, s);
+  }
+  return a.tq ? launch_one<T, D, true, 4, 2>(a, s) : launch_one<T, D, false, 4, 2>(a, s);
 }
 
 template <typename T>

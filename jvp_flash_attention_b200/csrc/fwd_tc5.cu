@@ -1,6 +1,6 @@
 // What the tcgen05 kernels share on the host side: the device status word of the bounded waits (with its host-visible
 // mirror), the TMA tensor-map encoders, and the forward dispatch
-//   D = 64  -> fwd_tc5_pair64.cu  (two query tiles per CTA share every key stage)
+//   D <= 64 -> fwd_tc5_pair64.cu  (two query tiles per CTA share every key stage)
 //   D = 128 -> fwd_tc5_pipe128.cu (score products of the next key tile under the softmax of this one)
 // Both follow the register-tiled kernel in fwd_generic.cu in what they compute (jvp_attention.py:125-336, 1011-1033).
 #include "tc5_common.cuh"
@@ -110,33 +110,39 @@ bool encode_map4d_f32(CUtensorMap* m, const void* ptr, int D, int L, int H, int 
   return r == CUDA_SUCCESS;
 }
 
-bool encode_map4(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int L, int H, int B, const int64_t* st,
-                 int box_rows) {
-  return encode_map4d(m, dt, ptr, 64, L, H, B, st, box_rows);
-}
-
 }  // namespace tc5
+
+// Head dimension 32 runs on the D = 64 kernels: the tensor maps end at column 32, so TMA fills the other half of every
+// tile with zeros and clips what is stored, and the contractions over D stop half-way.  An MMA costs the same for 32
+// output columns as for 64, so little is wasted (DRATE).  Up to one
+// 64-row tile the register-tiled kernels stay: a 256-row pair of query tiles would be mostly padding.
+bool tc5_head_dim(int D, int L) { return D == 64 || D == 128 || (D == 32 && L > 64); }
 
 bool fwd_tc5_eligible(const jvpfa_fwd_args& a) {
   if (a.dtype != JVPFA_BF16 && a.dtype != JVPFA_FP16) return false;
-  if (a.D != 64 && a.D != 128) return false;
-  // The D = 64 kernel takes the row maximum before scaling and therefore needs a positive softmax scale (any other
+  if (!tc5_head_dim(a.D, a.L)) return false;
+  // The D <= 64 kernel takes the row maximum before scaling and therefore needs a positive softmax scale (any other
   // goes to the register-tiled kernels).
-  if (a.D == 64 && !(a.sm_scale > 0.f)) return false;
+  if (a.D <= 64 && !(a.sm_scale > 0.f)) return false;
   const int k = a.mask.kind;
   if (k == JVPFA_MASK_NONE || k == JVPFA_MASK_CAUSAL || k == JVPFA_MASK_KVLEN) return true;
-  // Boolean masks and bias: the softmax threads read 16-byte pieces of mask rows
-  if ((a.L & 15) != 0) return false;
-  if (k == JVPFA_MASK_BIAS && a.mask.bias_dtype != a.dtype) return false;
-  const long long esz = k == JVPFA_MASK_BOOL ? 1 : 2;
-  if (a.mask.stride[3] != 1 || (reinterpret_cast<uintptr_t>(a.mask.ptr) & 15u) != 0) return false;
+  return tc5_mask_layout(a.mask, a.dtype, a.L);
+}
+
+// Boolean masks and bias of the tensors' type: the kernels read 16-byte pieces of mask rows, the last piece of a row as
+// well when only its head lies inside the row (what is beyond key L is then switched off by index).  That takes rows
+// padded to whole pieces, which the Python layer makes of a mask whose length does not fill them.
+bool tc5_mask_layout(const jvpfa_mask& m, int dtype, int L) {
+  if (m.kind == JVPFA_MASK_BIAS && m.bias_dtype != dtype) return false;
+  const long long esz = m.kind == JVPFA_MASK_BOOL ? 1 : 2;
+  if (m.stride[3] != 1 || (reinterpret_cast<uintptr_t>(m.ptr) & 15u) != 0) return false;
   for (int d = 0; d < 3; ++d)
-    if (a.mask.stride[d] < 0 || ((a.mask.stride[d] * esz) & 15) != 0) return false;
-  return true;
+    if (m.stride[d] < 0 || ((m.stride[d] * esz) & 15) != 0) return false;
+  return (L & 15) == 0 || (m.stride[2] * esz >= ((L * esz + 15) & ~15ll));
 }
 
 int launch_fwd_tc5(const jvpfa_fwd_args& a, cudaStream_t s) {
-  if (a.D == 64) return launch_fwd_tc5_pair64(a, s);
+  if (a.D <= 64) return launch_fwd_tc5_pair64(a, s);
   return launch_fwd_tc5_pipe128(a, s);
 }
 

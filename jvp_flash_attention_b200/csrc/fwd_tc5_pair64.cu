@@ -381,13 +381,16 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
             if constexpr (DUAL) {
               umma_ss_lo<false>(tq + C::COL_S, q_lo, k_lo, idesc_s2);  // [S | tS] = Q [K ; tK]^T
 #pragma unroll
-              for (int ks = 1; ks < D / 16; ++ks) umma_ss_lo<true>(tq + C::COL_S, q_lo + ks * 2, k_lo + ks * 2, idesc_s2);
+              for (int ks = 1; ks < D / 16; ++ks)
+                if (ks < 2 || a.D > 32) umma_ss_lo<true>(tq + C::COL_S, q_lo + ks * 2, k_lo + ks * 2, idesc_s2);
 #pragma unroll
-              for (int ks = 0; ks < D / 16; ++ks) umma_ss_lo<true>(tq + C::COL_TS, tq_lo + ks * 2, k_lo + ks * 2, idesc_s);  // tS += tQ K^T
+              for (int ks = 0; ks < D / 16; ++ks)
+                if (ks < 2 || a.D > 32) umma_ss_lo<true>(tq + C::COL_TS, tq_lo + ks * 2, k_lo + ks * 2, idesc_s);  // tS += tQ K^T
             } else {
               umma_ss_lo<false>(tq + C::COL_S, q_lo, k_lo, idesc_s);
 #pragma unroll
-              for (int ks = 1; ks < D / 16; ++ks) umma_ss_lo<true>(tq + C::COL_S, q_lo + ks * 2, k_lo + ks * 2, idesc_s);
+              for (int ks = 1; ks < D / 16; ++ks)
+                if (ks < 2 || a.D > 32) umma_ss_lo<true>(tq + C::COL_S, q_lo + ks * 2, k_lo + ks * 2, idesc_s);
             }
             tc_commit_u32(bar_s_full);
             if (j == my_last) tc_commit_u32(bar_q_empty);  // arrives when the item's last scores are complete
@@ -552,7 +555,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
 #pragma unroll
           for (int q4 = 0; q4 < MW / 4; ++q4) {
             uint4 r = make_uint4(0u, 0u, 0u, 0u);
-            if (n0 + (q4 + 1) * (16 / MESZ) <= L) r = ldg_nc_v4(mrow + (size_t)n0 * MESZ + 16 * q4);
+            if (n0 + q4 * (16 / MESZ) < L) r = ldg_nc_v4(mrow + (size_t)n0 * MESZ + 16 * q4);
             mw[4 * q4] = r.x, mw[4 * q4 + 1] = r.y, mw[4 * q4 + 2] = r.z, mw[4 * q4 + 3] = r.w;
           }
         }
@@ -783,16 +786,16 @@ static int launch_pair64(const jvpfa_fwd_args& a, cudaStream_t stream) {
   const CUtensorMapDataType dt = Fmt<T>::kTma;
   // (64, L, H, B) maps: the inputs may be strided views (in_stride), e.g. (B,L,H,D) tensors seen as (B,H,L,D)
   const int64_t* st = a.in_stride;
-  bool ok = encode_map4(&maps.q, dt, a.q, a.L, a.H, a.B, st, C::BM) && encode_map4(&maps.k, dt, a.k, a.L, a.H, a.B, st, C::BN) &&
-            encode_map4(&maps.v, dt, a.v, a.L, a.H, a.B, st, C::BN);
+  bool ok = encode_map4d(&maps.q, dt, a.q, a.D, a.L, a.H, a.B, st, C::BM) && encode_map4d(&maps.k, dt, a.k, a.D, a.L, a.H, a.B, st, C::BN) &&
+            encode_map4d(&maps.v, dt, a.v, a.D, a.L, a.H, a.B, st, C::BN);
   if (DUAL)
-    ok = ok && encode_map4(&maps.tq, dt, a.tq, a.L, a.H, a.B, st, C::BM) &&
-         encode_map4(&maps.tk, dt, a.tk, a.L, a.H, a.B, st, C::BN) && encode_map4(&maps.tv, dt, a.tv, a.L, a.H, a.B, st, C::BN);
+    ok = ok && encode_map4d(&maps.tq, dt, a.tq, a.D, a.L, a.H, a.B, st, C::BM) &&
+         encode_map4d(&maps.tk, dt, a.tk, a.D, a.L, a.H, a.B, st, C::BN) && encode_map4d(&maps.tv, dt, a.tv, a.D, a.L, a.H, a.B, st, C::BN);
   else
     maps.tq = maps.tk = maps.tv = maps.q;
-  ok = ok && encode_map4(&maps.o, dt, a.o, a.L, a.H, a.B, nullptr, C::BM);
+  ok = ok && encode_map4d(&maps.o, dt, a.o, a.D, a.L, a.H, a.B, nullptr, C::BM);
   if (DUAL)
-    ok = ok && encode_map4(&maps.to, dt, a.to, a.L, a.H, a.B, nullptr, C::BM);
+    ok = ok && encode_map4d(&maps.to, dt, a.to, a.D, a.L, a.H, a.B, nullptr, C::BM);
   else
     maps.to = maps.o;
   if (!ok) {

@@ -298,7 +298,7 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
 #pragma unroll
         for (int q4 = 0; q4 < MW / 4; ++q4) {
           uint4 r = make_uint4(0u, 0u, 0u, 0u);
-          if (n0 + (q4 + 1) * (16 / MESZ) <= L) r = ldg_nc_v4(mrow + (size_t)n0 * MESZ + 16 * q4);
+          if (n0 + q4 * (16 / MESZ) < L) r = ldg_nc_v4(mrow + (size_t)n0 * MESZ + 16 * q4);
           mw[4 * q4] = r.x, mw[4 * q4 + 1] = r.y, mw[4 * q4 + 2] = r.z, mw[4 * q4 + 3] = r.w;
         }
       }

@@ -95,6 +95,9 @@ __global__ void __launch_bounds__(kCheckThreads) mask_check_kernel(const jvpfa_m
   }
 }
 
+// The first n bytes of a word (n may be negative or beyond 4).
+__device__ __forceinline__ unsigned int word_mask(int n) { return n >= 4 ? ~0u : n <= 0 ? 0u : (1u << (8 * n)) - 1u; }
+
 // Tile summary of a boolean mask.  One CTA = one 128-row tile row of one head x eight 64-key tiles
 // (512 bytes of each row): lane l of a warp reads bytes [16 l, 16 l + 16) of a row, so four
 // neighbouring lanes cover one tile; the eight warps share out the rows.
@@ -112,11 +115,14 @@ __global__ void __launch_bounds__(256) mask_tiles_kernel(const jvpfa_mask m, int
   const int col = kg * 512 + lane * 16;
   const int r0 = qt * 128, r1 = min(n_rows, r0 + 128);
   unsigned int any = 0u;
-  if (col + 16 <= L) {
+  if (col < L) {
+    // bytes of the row's last piece that lie beyond its end do not count
+    const int valid = min(16, L - col);
+    const unsigned int keep[4] = {word_mask(valid), word_mask(valid - 4), word_mask(valid - 8), word_mask(valid - 12)};
 #pragma unroll 4
     for (int r = r0 + warp; r < r1; r += 8) {
       const uint4 x = __ldg(reinterpret_cast<const uint4*>(base + (long long)r * m.stride[2] + col));
-      any |= x.x | x.y | x.z | x.w;
+      any |= (x.x & keep[0]) | (x.y & keep[1]) | (x.z & keep[2]) | (x.w & keep[3]);
     }
   }
   const unsigned int vote = __ballot_sync(0xffffffffu, any != 0u);  // bit l: lane l saw a true entry

@@ -229,9 +229,9 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   }
 }
 
-// Gradients of <go, O> + <gto, tO> with respect to q, k, v.
+// Gradients of <go, O> + <gto, tO> with respect to q, k, v; those named in `skip` (JVPFA_SKIP_*) stay undefined.
 Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, Tensor tk, Tensor tv, const Tensor& o, Tensor to,
-                 const Tensor& lse, Tensor mu, Tensor go, Tensor gto, const Call& call) {
+                 const Tensor& lse, Tensor mu, Tensor go, Tensor gto, const Call& call, int skip = 0) {
   if (!q.is_cuda()) {
     py::gil_scoped_acquire gil;
     NoFunctorch nf;
@@ -260,11 +260,11 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   void* stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
 
   // One scratch allocation: the three row statistics, and fp32 dQ where the single-pass kernels want it (head dimension
-  // 64, 16-bit; index masks, a boolean mask without tile bitmaps, or through O alone a bias of the tensors' type).
+  // up to 64, 16-bit; index masks, a boolean mask without tile bitmaps, or through O alone a bias of the tensors' type).
   const bool index_mask = m.c.kind == JVPFA_MASK_NONE || m.c.kind == JVPFA_MASK_CAUSAL || m.c.kind == JVPFA_MASK_KVLEN;
   const bool dense_bool = m.c.kind == JVPFA_MASK_BOOL && !m.tile_live.defined() && !m.tile_live_t.defined();
   const bool bias_o = m.c.kind == JVPFA_MASK_BIAS && !gto.defined() && m.c.bias_dtype == dtype_of(q, false);
-  const bool single = g_single_pass && sizes[3] == 64 && q.scalar_type() != at::kFloat && (index_mask || dense_bool || bias_o);
+  const bool single = g_single_pass && !(skip & JVPFA_SKIP_DKDV) && sizes[3] <= 64 && q.scalar_type() != at::kFloat && (index_mask || dense_bool || bias_o);
   const int64_t stat = (rows + 63) / 64 * 64;  // 256-byte steps
   Tensor scratch = empty({3 * stat + (single ? rows * sizes[3] : 0)}, at::kFloat, q.device());
   float* f = static_cast<float*>(scratch.data_ptr());
@@ -279,7 +279,9 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   check_status(jvpfa_bwd_preprocess(&p, stream), "jvpfa_bwd_preprocess");
 
   Grads g;
-  for (Tensor& t : g) t = empty(sizes, q.scalar_type(), q.device());
+  if (!(skip & JVPFA_SKIP_DQ)) g[0] = empty(sizes, q.scalar_type(), q.device());
+  if (!(skip & JVPFA_SKIP_DKDV))
+    for (int i = 1; i < 3; ++i) g[i] = empty(sizes, q.scalar_type(), q.device());
   jvpfa_bwd_args a{};
   a.struct_size = sizeof(a);
   a.dtype = p.dtype;
@@ -290,7 +292,9 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.lse = static_cast<const float*>(data(lse));
   a.mu = p.mu;
   a.delta = p.delta, a.eps = p.eps, a.cterm = p.cterm;
-  a.dq = g[0].data_ptr(), a.dk = g[1].data_ptr(), a.dv = g[2].data_ptr();
+  a.skip = skip;
+  if (g[0].defined()) a.dq = g[0].data_ptr();
+  if (g[1].defined()) a.dk = g[1].data_ptr(), a.dv = g[2].data_ptr();
   a.mask = m.c;
   if (m.tile_live.defined() && m.tile_live_t.defined() && a.L <= 8192) {
     a.mask_tile_live = data(m.tile_live);
@@ -310,6 +314,9 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
     return g;
   }
 }
+
+// What autograd will not use of a node's gradients with respect to q, k, v (its first three outputs).
+int unused_gradients(bool need_q, bool need_kv) { return (need_q ? 0 : JVPFA_SKIP_DQ) | (need_kv ? 0 : JVPFA_SKIP_DKDV); }
 
 Tensor zeros_like_input(const Tensor& q) {
   NoFunctorch nf;
@@ -359,8 +366,9 @@ struct AttnBwdNode : public Node {
       for (int i = 0; i < 3; ++i) t[i] = u[i].defined() ? unwrap(u[i]).contiguous() : at::zeros_like(qp, at::MemoryFormat::Contiguous);
     }
     FwdResult f = launch_fwd(qp, kp, vp, t[0], t[1], t[2], call);
-    if (task_should_compute_output(0) || task_should_compute_output(1) || task_should_compute_output(2)) {
-      Grads h = launch_bwd(qp, kp, vp, t[0], t[1], t[2], f.o, f.to, f.lse, f.mu, Tensor(), gop, call);
+    const int skip = unused_gradients(task_should_compute_output(0), task_should_compute_output(1) || task_should_compute_output(2));
+    if (skip != (JVPFA_SKIP_DQ | JVPFA_SKIP_DKDV)) {
+      Grads h = launch_bwd(qp, kp, vp, t[0], t[1], t[2], f.o, f.to, f.lse, f.mu, Tensor(), gop, call, skip);
       for (int i = 0; i < 3; ++i) out[i] = h[i];
     }
     if (task_should_compute_output(3)) out[3] = f.to;
@@ -377,8 +385,8 @@ struct AttnBwdNode : public Node {
 };
 
 Grads backward_through_o(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& go,
-                         const Call& call) {
-  Grads g = launch_bwd(unwrap(q), unwrap(k), unwrap(v), Tensor(), Tensor(), Tensor(), o, Tensor(), lse, Tensor(), go, Tensor(), call);
+                         const Call& call, int skip) {
+  Grads g = launch_bwd(unwrap(q), unwrap(k), unwrap(v), Tensor(), Tensor(), Tensor(), o, Tensor(), lse, Tensor(), go, Tensor(), call, skip);
   if (torch::autograd::compute_requires_grad(q, k, v, go)) {  // create_graph: a second differentiation was asked for
     auto node = std::shared_ptr<AttnBwdNode>(new AttnBwdNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(q, k, v, go));
@@ -407,10 +415,11 @@ struct AttnNode : public Node {
     const auto self = shared_from_this();
     const Tensor q_ = primal_of(q.unpack()), k_ = primal_of(k.unpack()), v_ = primal_of(v.unpack());
     const Tensor o_ = unwrap(o.unpack(self)), lse_ = lse.unpack();
-    const bool need_primals = task_should_compute_output(0) || task_should_compute_output(1) || task_should_compute_output(2);
+    const int skip = unused_gradients(task_should_compute_output(0), task_should_compute_output(1) || task_should_compute_output(2));
+    const bool need_primals = skip != (JVPFA_SKIP_DQ | JVPFA_SKIP_DKDV);
     if (!gto.defined()) {
       if (need_primals) {
-        Grads g = backward_through_o(q_, k_, v_, o_, lse_, go, call);
+        Grads g = backward_through_o(q_, k_, v_, o_, lse_, go, call, skip);
         for (int i = 0; i < 3; ++i) out[i] = g[i];
       }
       return out;
@@ -421,19 +430,21 @@ struct AttnNode : public Node {
     static constexpr const char* kOnce = "the gradient through the tangent output of JVPAttn cannot be differentiated a second time";
     if (need_primals) {
       const bool again = at::GradMode::is_enabled();  // a second differentiation was asked for: the part through O stays a node of its own
-      Grads g = launch_bwd(qp, kp, vp, tqp, tkp, tvp, o_, to_, lse_, mu_, again ? Tensor() : go, gto, call);
+      Grads g = launch_bwd(qp, kp, vp, tqp, tkp, tvp, o_, to_, lse_, mu_, again ? Tensor() : go, gto, call, skip);
       if (again) {
         attach_refusal(kOnce, {&g[0], &g[1], &g[2]}, q_, k_, v_, tq_, tk_, tv_, gto);
         if (go.defined()) {
-          Grads h = backward_through_o(q_, k_, v_, o_, lse_, go, call);
-          for (int i = 0; i < 3; ++i) g[i] = h[i] + g[i];
+          Grads h = backward_through_o(q_, k_, v_, o_, lse_, go, call, skip);
+          for (int i = 0; i < 3; ++i)
+            if (h[i].defined()) g[i] = h[i] + g[i];
         }
       }
       for (int i = 0; i < 3; ++i) out[i] = g[i];
     }
     if (task_should_compute_output(3) || task_should_compute_output(4) || task_should_compute_output(5)) {
       // with respect to the tangents tO is an ordinary attention output with cotangent gto
-      Grads g = launch_bwd(qp, kp, vp, Tensor(), Tensor(), Tensor(), o_, Tensor(), lse_, Tensor(), gto, Tensor(), call);
+      Grads g = launch_bwd(qp, kp, vp, Tensor(), Tensor(), Tensor(), o_, Tensor(), lse_, Tensor(), gto, Tensor(), call,
+                           unused_gradients(task_should_compute_output(3), task_should_compute_output(4) || task_should_compute_output(5)));
       if (at::GradMode::is_enabled()) attach_refusal(kOnce, {&g[0], &g[1], &g[2]}, q_, k_, v_, tq_, tk_, tv_, gto);
       for (int i = 0; i < 3; ++i) out[3 + i] = g[i];
     }

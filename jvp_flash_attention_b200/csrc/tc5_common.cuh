@@ -102,12 +102,9 @@ __device__ __forceinline__ uint32_t ldg_nc_u16(const void* p) {
   return r;
 }
 
-// Host: (64, L, H, B) view of a 16-bit tensor whose batch / head / row strides (in elements) are given
-// (all zero: (B,H,L,64) row-major); box = 64 columns x box_rows rows, 128-byte swizzle, out-of-range
-// rows read as zero.  Defined in fwd_tc5.cu.
-bool encode_map4(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int L, int H, int B, const int64_t* stride_bhl,
-                 int box_rows);
-// The same for head dimension D (64-column boxes: a D = 128 tile is two loads).
+// Host: (D, L, H, B) view of a 16-bit tensor whose batch / head / row strides (in elements) are given
+// (all zero: (B,H,L,D) row-major); box = 64 columns x box_rows rows (a D = 128 tile is two loads), 128-byte swizzle,
+// out-of-range rows and columns read as zero.  Defined in fwd_tc5.cu.
 bool encode_map4d(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int D, int L, int H, int B, const int64_t* stride_bhl,
                   int box_rows);
 // Row-major fp32 (B, H, L, D) tensor, 32-column boxes with 128-byte swizzle (target of TMA reductions).
@@ -418,10 +415,6 @@ __device__ __forceinline__ void poison_row(void* base, size_t row, int D) {  // 
                       : make_uint4(0x7fc00000u, 0x7fc00000u, 0x7fc00000u, 0x7fc00000u);
 }
 
-template <int I>
-struct IntC {
-  static constexpr int value = I;
-};
 
 }  // namespace tc5
 }  // namespace jvpfa

@@ -146,13 +146,13 @@ def classify_mask(attn_mask: Tensor | None, causal: bool, Z: int, H: int, N: int
     if attn_mask is None:
         return _lib.MaskSpec(_lib.MASK_NONE), 0, None
     if not MASK_MEMO_ENABLED:
-        return _classify_mask_tensor(attn_mask, Z, H, N, verify)
+        return _classify_mask_tensor(attn_mask, Z, H, N, qdtype, verify)
     key = (Z, H, N, verify, _unwrap(attn_mask)._version)
     hit = _MASK_MEMO.get(id(attn_mask))
     if hit is not None and hit[0]() is attn_mask and hit[1] == key:
         spec, mask_type = hit[2]
         return copy.copy(spec), mask_type, attn_mask  # a copy: the caller writes per-call state into the description
-    spec, mask_type, _ = _classify_mask_tensor(attn_mask, Z, H, N, verify)
+    spec, mask_type, _ = _classify_mask_tensor(attn_mask, Z, H, N, qdtype, verify)
     if len(_MASK_MEMO) >= _MASK_MEMO_MAX:
         _MASK_MEMO.clear()
     try:
@@ -166,7 +166,15 @@ def classify_mask(attn_mask: Tensor | None, causal: bool, Z: int, H: int, N: int
     return spec, mask_type, attn_mask
 
 
-def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, verify: bool):
+def _padded_rows(m: Tensor, N: int) -> Tensor:
+    """``m`` with its rows padded to whole 16-byte pieces, the form in which the 16-bit tensor-core kernels read a mask
+    (what lies beyond the row's end is not looked at)."""
+    step = 16 // m.element_size()
+    out = torch.empty((*m.shape[:3], (N + step - 1) // step * step), device=m.device, dtype=m.dtype)[..., :N]
+    return out.copy_(m)
+
+
+def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, qdtype: torch.dtype, verify: bool):
     """classify_mask for a mask tensor: shape checks, key-padding recognition, verification passes."""
     assert attn_mask.dim() == 4, "The provided attention mask must have 4 dimensions (Z, H, N_CTX, N_CTX)."
     mz, mh, mi, mj = attn_mask.shape
@@ -176,11 +184,13 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, verify: boo
     assert attn_mask.dtype == torch.bool or attn_mask.dtype.is_floating_point, (
         "The attention mask must be of the dtype bool or a floating-point dtype."
     )
-    m = _unwrap(attn_mask)
+    m = _unwrap(attn_mask).detach()  # the description keeps the storage, not the caller's tensor object (see the memo)
 
     def bstrides(t: Tensor) -> tuple[int, int, int, int]:
         return tuple(0 if t.shape[d] == 1 else t.stride(d) for d in range(4))
 
+    # up to one tile of keys the mask is read element by element, whatever its layout
+    ragged = N > 64 and N * m.element_size() % 16 != 0 and qdtype in (torch.bfloat16, torch.float16)
     if m.dtype == torch.bool:
         if mh == 1 and mi == 1:
             # Candidate key-padding mask: valid keys form a prefix of each row.  Lengths, the prefix test and
@@ -194,6 +204,8 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, verify: boo
                     assert min_len > 0, "The attention mask cannot be all False for any head."
                 kv_len = lens.expand(Z).contiguous() if mz == 1 else lens.contiguous()
                 return _lib.MaskSpec(_lib.MASK_KVLEN, kv_len), 1, attn_mask
+        if ragged and mi > 1:
+            m = _padded_rows(m, N)
         m8 = m.view(torch.uint8) if m.is_contiguous() or m.stride(-1) == 1 else m.contiguous().view(torch.uint8)
         spec = _lib.MaskSpec(_lib.MASK_BOOL, m8, bstrides(m8))
         every_head_live = True
@@ -215,6 +227,8 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, verify: boo
 
     if m.dtype not in _lib.DTYPE_ENUM:
         m = m.to(torch.float32)
+    elif ragged and mi > 1 and m.dtype == qdtype:
+        m = _padded_rows(m, N)
     spec = _lib.MaskSpec(_lib.MASK_BIAS, m, bstrides(m), _lib.DTYPE_ENUM[m.dtype])
     if verify:
         # one pass and one read-back for upstream's isinf / isnan / "all MASK_CONST" sweeps (jvp_attention.py:2447-2457)
@@ -276,7 +290,7 @@ def _launch_bwd(q, k, v, tq, tk, tv, o, to, lse, mu, go, gto, spec: _lib.MaskSpe
     acc = None
     dense_bool = spec.kind == _lib.MASK_BOOL and spec.tile_live is None and spec.tile_live_t is None  # no tiles to step over
     bias_o = spec.kind == _lib.MASK_BIAS and gto is None and spec.bias_dtype == _lib.DTYPE_ENUM.get(q.dtype)  # through O alone
-    if SINGLE_PASS_BACKWARD and q.shape[-1] == 64 and q.dtype != torch.float32 and (
+    if SINGLE_PASS_BACKWARD and q.shape[-1] <= 64 and q.dtype != torch.float32 and (
             spec.kind in _lib.INDEX_MASKS or dense_bool or bias_o):
         acc = torch.empty(q.shape, device=q.device, dtype=torch.float32)
     if st is not None:

@@ -1,0 +1,107 @@
+"""GPU tests at the edges of the dispatch: head dimension 32 on the D = 64 tensor-core kernels, masks whose rows do not
+fill 16-byte pieces, the row / key splits of the register-tiled kernels, and gradients that nobody asked for."""
+import pytest
+import torch
+
+import jvp_flash_attention_b200.jvp_attention as ja
+from jvp_flash_attention_b200 import _lib
+from oracle import jvp_attention_oracle as orc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+DT = {"bf16": torch.bfloat16, "fp16": torch.float16, "fp32": torch.float32}
+
+
+def _inputs(B, H, L, D, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    ts = [torch.randn(B, H, L, D, generator=g) for _ in range(8)]
+    for i in (3, 4, 5):  # small tangents: |tO| stays where the spacing of bfloat16 is below the tolerance
+        ts[i] = ts[i] * 0.1
+    return [t.to(dtype) for t in ts]
+
+
+def _mask(kind, B, H, L, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    if kind == "keys":
+        lens = torch.randint(1, L + 1, (B,), generator=g)
+        return (torch.arange(L)[None, :] < lens[:, None])[:, None, None, :]
+    if kind == "bool":
+        return (torch.rand(B, 1, L, L, generator=g) > 0.7) | torch.eye(L, dtype=torch.bool)
+    if kind == "window":
+        i = torch.arange(L)
+        return ((i[:, None] - i[None, :]).abs() <= 40)[None, None]
+    if kind == "bias":
+        return torch.randn(B, H, L, L, generator=g).clamp(-5, 5).to(dtype)
+    return None
+
+
+def _check(B, H, L, D, dt, kind, cot, seed=0):
+    """O, tO and the gradients through the asked-for outputs against the float64 oracle: 1e-5 of the largest entry for
+    fp32 (three TF32 products), 2e-2 (scaled with the gradients' magnitude) for 16 bits, as in the parity tests."""
+    dtype = DT[dt]
+    q, k, v, tq, tk, tv, go, gt = _inputs(B, H, L, D, dtype, seed + L + D)
+    mask, causal = _mask(kind, B, H, L, dtype, seed + 1), kind == "causal"
+    go, gt = (go if cot != "t" else None), (gt if cot != "o" else None)
+    ref = orc.grads_through_both(q, k, v, tq, tk, tv, go, gt, attn_mask=mask, causal=causal)
+    cu = lambda x: None if x is None else x.to(DEV)  # noqa: E731
+    a = [cu(x).requires_grad_() for x in (q, k, v)]
+    m = cu(mask)
+    o, to = torch.func.jvp(lambda x, y, z: ja.JVPAttn.fwd_dual(x, y, z, attn_mask=m, causal=causal), tuple(a),
+                           tuple(cu(x) for x in (tq, tk, tv)))
+    outs = [(x, cu(w)) for x, w in ((o, go), (to, gt)) if w is not None]
+    got = (o, to, *torch.autograd.grad([x for x, _ in outs], a, [w for _, w in outs]))
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    for name, x, r in zip(("O", "tO", "dq", "dk", "dv"), got, ref):
+        top = r.abs().max().item()
+        e = orc.max_abs_err(x, r)
+        assert e <= (1e-5 * top if dt == "fp32" else 2e-2 * max(1.0, top)), (name, e, top)
+
+
+@pytest.mark.parametrize("dt,B,H,L,kind,cot", [
+    ("bf16", 1, 2, 66, "none", "both"), ("bf16", 2, 3, 128, "causal", "t"), ("fp16", 2, 2, 200, "keys", "both"),
+    ("bf16", 1, 3, 258, "none", "o"), ("fp16", 2, 1, 320, "window", "both"), ("bf16", 1, 2, 130, "bias", "t"),
+    ("bf16", 3, 8, 1000, "none", "both"),
+])
+def test_head_dimension_32_on_the_tensor_core_kernels(dt, B, H, L, kind, cot):
+    _check(B, H, L, 32, dt, kind, cot)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dt,L,kind,cot", [
+    ("bf16", 66, "bool", "both"), ("fp16", 130, "bias", "both"), ("bf16", 250, "bias", "o"), ("bf16", 334, "window", "t"),
+    ("fp16", 506, "bool", "t"),
+])
+def test_masks_whose_rows_do_not_fill_16_byte_pieces(D, dt, L, kind, cot):
+    _check(2, 2, L, D, dt, kind, cot)
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("B,H,L,kind,cot", [
+    (1, 1, 34, "none", "both"), (1, 3, 100, "causal", "t"), (2, 8, 320, "keys", "both"), (4, 10, 250, "bool", "o"),
+    (2, 12, 450, "bias", "both"),
+])
+def test_row_and_key_splits_of_the_register_tiled_kernels(D, B, H, L, kind, cot):
+    """16-row tiles below 296 of them run as 1 x 8 warps, below 592 as 2 x 4, above as 4 x 2."""
+    _check(B, H, L, D, "fp32", kind, cot)
+
+
+@pytest.mark.parametrize("dt,D", [("fp32", 64), ("fp32", 128), ("bf16", 64), ("bf16", 128), ("fp16", 32)])
+@pytest.mark.parametrize("want", ["q", "kv"])
+def test_gradients_nobody_asked_for_are_left_out(dt, D, want):
+    """The gradients that are asked for are those of the full call (bit for bit where the same kernel forms them; dQ of
+    the single pass is summed in another order than by the own-queries launch: the 16-bit tolerance)."""
+    q, k, v, tq, tk, tv, go, gt = (x.to(DEV) for x in _inputs(2, 3, 200, D, DT[dt], 5))
+
+    def run(names):
+        a = {n: x.clone().requires_grad_(n in names) for n, x in (("q", q), ("k", k), ("v", v))}
+        o, to = torch.func.jvp(lambda x, y, z: ja.JVPAttn.fwd_dual(x, y, z, causal=True), tuple(a.values()), (tq, tk, tv))
+        return torch.autograd.grad((o, to), [a[n] for n in names], (go, gt))
+
+    full = dict(zip("qkv", run("qkv")))
+    for n, x in zip(want, run(want)):
+        if dt == "fp32" or D == 128 or want == "kv":
+            assert torch.equal(x, full[n]), n
+        else:
+            assert (x.float() - full[n].float()).abs().max().item() <= 2e-2 * max(1.0, full[n].abs().max().item())
+    assert _lib.device_status() == 0
