@@ -118,6 +118,9 @@ typedef struct {
   /* Optional, JVPFA_MASK_BOOL only: the bitmap written by jvpfa_mask_tiles for this mask.  The tcgen05
    * kernel then steps over 128 x 64 tiles without a true entry; other kernels ignore it.  NULL = none. */
   const void* mask_tile_live;
+  /* Optional, JVPFA_MASK_BOOL only: `bits` of jvpfa_mask_tiles.  The tcgen05 kernels read it instead of the bytes, whose
+   * layout then does not matter to them.  A caller built without this field (struct_size up to mask_tile_live): NULL. */
+  const void* mask_bits;
 } jvpfa_fwd_args;
 
 int jvpfa_fwd(const jvpfa_fwd_args* args, void* stream);
@@ -142,6 +145,9 @@ typedef struct {
   const void *go, *gto;
   const float* mu;
   float *delta, *eps, *cterm; /* (B,H,L) each; caller-owned scratch */
+  /* Optional: the B*H*L*D floats of jvpfa_bwd_args.dq_accum, set to zero on the way (give JVPFA_DQ_ACCUM_IS_ZERO to
+   * jvpfa_bwd then).  A caller built without this field (struct_size up to cterm) has nothing cleared. */
+  float* dq_accum;
 } jvpfa_pre_args;
 
 int jvpfa_bwd_preprocess(const jvpfa_pre_args* args, void* stream);
@@ -185,13 +191,18 @@ typedef struct {
    * end, so dQ is reproducible to rounding but not bitwise from run to run.  NULL: the two-launch kernels, which
    * recompute the score tiles for dQ (as upstream does, jvp_attention.py:1415-1707) and are bitwise reproducible. */
   float* dq_accum;
-  /* Gradients nobody asked for: JVPFA_SKIP_DQ or JVPFA_SKIP_DKDV (not both); 0 = all three are formed.  The pointers of
-   * skipped gradients may be NULL.  A caller built without this field (struct_size up to dq_accum) gets all three. */
-  int32_t skip;
+  /* JVPFA_SKIP_DQ or JVPFA_SKIP_DKDV (not both): gradients nobody asked for are not formed, and their pointers may be
+   * NULL.  JVPFA_DQ_ACCUM_IS_ZERO: see jvpfa_pre_args.dq_accum.  A caller built without this field (struct_size up to
+   * dq_accum) passes none of them. */
+  int32_t flags;
+  /* Optional, JVPFA_MASK_BOOL only, both or neither: `bits` and `bits_t` of jvpfa_mask_tiles, as in jvpfa_fwd_args. */
+  const void* mask_bits;
+  const void* mask_bits_t;
 } jvpfa_bwd_args;
 
 #define JVPFA_SKIP_DQ 1
 #define JVPFA_SKIP_DKDV 2
+#define JVPFA_DQ_ACCUM_IS_ZERO 4
 
 int jvpfa_bwd(const jvpfa_bwd_args* args, void* stream);
 
@@ -264,8 +275,7 @@ int jvpfa_mask_check(const jvpfa_mask_check_args* args, void* stream);
  * jvpfa_mask_check from the same pass.  No upstream counterpart: upstream reads every L x L mask tile
  * in every kernel (jvp_attention.py:453) and has no block skipping.
  *
- * The mask (kind BOOL) must have key stride 1, 16-byte aligned rows and L % 16 == 0 (else
- * JVPFA_ERR_UNSUPPORTED).  n_b, n_h, n_rows are its own extents (1 where it broadcasts, i.e. where its
+ * The mask (kind BOOL) may have any layout; n_b, n_h, n_rows are its own extents (1 where it broadcasts, i.e. where its
  * stride is 0; n_rows is 1 or L).  Tiles are 128 queries x 64 keys (one tile row when n_rows == 1).
  *   tile_live  n_b*n_h * n_qt * n_words uint64, n_qt = n_rows == 1 ? 1 : ceil(L/128),
  *              n_words = ceil(ceil(L/64) / 64); bit (t % 64) of word t / 64 of entry [b*n_h + h][qt] is
@@ -284,6 +294,12 @@ typedef struct {
   void* tile_live;
   int32_t* head_live;
   void* tile_live_t;
+  /* Optional: the mask as one bit per entry (0 beyond the ends).  bits: [head][row][2*ceil(L/64)] 32-bit words, key j of a
+   * row in bit j % 32 of word j / 32; bits_t: the transpose, [head][key][2*ceil(L/64)] words over the queries, or one word
+   * per key (all ones or zero) when n_rows is 1.  Heads are the mask's own (n_b*n_h).  16-byte aligned.  A caller built
+   * without these fields (struct_size up to tile_live_t) gets neither. */
+  void* bits;
+  void* bits_t;
 } jvpfa_mask_tiles_args;
 
 int jvpfa_mask_tiles(const jvpfa_mask_tiles_args* args, void* stream);

@@ -56,7 +56,7 @@ def _native_cmd() -> list[str]:
     return [
         os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_EXTENSION_NAME=_native",
-        "-I", str(INCLUDE), "-I", sysconfig.get_paths()["include"],
+        "-I", str(INCLUDE), "-I", str(CSRC / "compat"), "-I", sysconfig.get_paths()["include"],
         *(f"-isystem{p}" for p in cpp_extension.include_paths("cuda")),
         str(CSRC / "native.cpp"), "-o", str(NATIVE),
         f"-L{torch_lib}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10",

@@ -115,10 +115,11 @@ static int validate_bwd(const jvpfa_bwd_args* a) {
   if (a->struct_size != (int32_t)sizeof(jvpfa_bwd_args)) return JVPFA_ERR_STRUCT;
   int rc = check_shape(a->dtype, a->B, a->H, a->L, a->D);
   if (rc) return rc;
-  if (a->skip != 0 && a->skip != JVPFA_SKIP_DQ && a->skip != JVPFA_SKIP_DKDV) return JVPFA_ERR_UNSUPPORTED;
+  constexpr int kSkip = JVPFA_SKIP_DQ | JVPFA_SKIP_DKDV;
+  if ((a->flags & ~(kSkip | JVPFA_DQ_ACCUM_IS_ZERO)) != 0 || (a->flags & kSkip) == kSkip) return JVPFA_ERR_UNSUPPORTED;
   if (!a->q || !a->k || !a->v || !a->lse || !a->delta) return JVPFA_ERR_NULL;
-  if (!(a->skip & JVPFA_SKIP_DQ) && !a->dq) return JVPFA_ERR_NULL;
-  if (!(a->skip & JVPFA_SKIP_DKDV) && (!a->dk || !a->dv)) return JVPFA_ERR_NULL;
+  if (!(a->flags & JVPFA_SKIP_DQ) && !a->dq) return JVPFA_ERR_NULL;
+  if (!(a->flags & JVPFA_SKIP_DKDV) && (!a->dk || !a->dv)) return JVPFA_ERR_NULL;
   if (!a->go && !a->gto) return JVPFA_ERR_NULL;
   if (a->gto && (!a->tq || !a->tk || !a->tv || !a->mu || !a->eps || !a->cterm)) return JVPFA_ERR_NULL;
   const void* ptrs[] = {a->q, a->k, a->v, a->tq, a->tk, a->tv, a->go, a->gto, a->dq, a->dk, a->dv};
@@ -131,14 +132,17 @@ static int validate_bwd(const jvpfa_bwd_args* a) {
   return check_mask(a->mask);
 }
 
-// The arguments as this build knows them: a caller built before `skip` was added passes a shorter struct.
-static const jvpfa_bwd_args* current_bwd_args(const jvpfa_bwd_args* a, jvpfa_bwd_args* full) {
-  constexpr int32_t kBeforeSkip = (int32_t)offsetof(jvpfa_bwd_args, skip);
-  if (!a || a->struct_size != kBeforeSkip) return a;
-  *full = jvpfa_bwd_args{};
-  memcpy(full, a, kBeforeSkip);
-  full->struct_size = (int32_t)sizeof(jvpfa_bwd_args);
+// The arguments as this build knows them: a caller built before the last field was added passes a shorter struct.
+template <typename Args>
+static const Args* current_args(const Args* a, Args* full, size_t size_before) {
+  if (!a || a->struct_size != (int32_t)size_before) return a;
+  *full = Args{};
+  memcpy(full, a, size_before);
+  full->struct_size = (int32_t)sizeof(Args);
   return full;
+}
+static const jvpfa_bwd_args* current_bwd_args(const jvpfa_bwd_args* a, jvpfa_bwd_args* full) {
+  return current_args(a, full, offsetof(jvpfa_bwd_args, flags));
 }
 
 static int validate_pre(const jvpfa_pre_args* a) {
@@ -149,7 +153,7 @@ static int validate_pre(const jvpfa_pre_args* a) {
   if (!a->o || !a->delta || !a->eps || !a->cterm) return JVPFA_ERR_NULL;
   if (!a->go && !a->gto) return JVPFA_ERR_NULL;
   if (a->gto && (!a->to || !a->mu)) return JVPFA_ERR_NULL;
-  const void* ptrs[] = {a->o, a->to, a->go, a->gto};
+  const void* ptrs[] = {a->o, a->to, a->go, a->gto, a->dq_accum};
   for (const void* p : ptrs)
     if (p && !aligned16(p)) return JVPFA_ERR_ALIGN;
   return JVPFA_OK;
@@ -179,7 +183,9 @@ using namespace jvpfa;
 
 extern "C" {
 
-int jvpfa_fwd_uses_tcgen05(const jvpfa_fwd_args* a) {
+int jvpfa_fwd_uses_tcgen05(const jvpfa_fwd_args* args) {
+  jvpfa_fwd_args full;
+  const jvpfa_fwd_args* a = current_args(args, &full, offsetof(jvpfa_fwd_args, mask_bits));
   if (validate_fwd(a) != JVPFA_OK) return 0;
   if (a->impl == JVPFA_IMPL_GENERIC) return 0;
   return fwd_tc5_eligible(*a) ? 1 : 0;
@@ -193,7 +199,9 @@ int jvpfa_bwd_uses_tcgen05(const jvpfa_bwd_args* args) {
   return bwd_tc5_eligible(*a) ? 1 : 0;
 }
 
-int jvpfa_fwd(const jvpfa_fwd_args* a, void* stream) {
+int jvpfa_fwd(const jvpfa_fwd_args* args, void* stream) {
+  jvpfa_fwd_args full;
+  const jvpfa_fwd_args* a = current_args(args, &full, offsetof(jvpfa_fwd_args, mask_bits));
   int rc = validate_fwd(a);
   if (rc) return rc;
   rc = check_arch();
@@ -209,7 +217,9 @@ int jvpfa_fwd(const jvpfa_fwd_args* a, void* stream) {
   return launch_fwd_generic(*a, s);
 }
 
-int jvpfa_bwd_preprocess(const jvpfa_pre_args* a, void* stream) {
+int jvpfa_bwd_preprocess(const jvpfa_pre_args* args, void* stream) {
+  jvpfa_pre_args full;
+  const jvpfa_pre_args* a = current_args(args, &full, offsetof(jvpfa_pre_args, dq_accum));
   const int rc = check_pre_request(a);
   if (rc) return rc;
   return launch_pre(*a, static_cast<cudaStream_t>(stream));
@@ -246,7 +256,9 @@ int jvpfa_mask_check(const jvpfa_mask_check_args* a, void* stream) {
   return launch_mask_check(*a, static_cast<cudaStream_t>(stream));
 }
 
-int jvpfa_mask_tiles(const jvpfa_mask_tiles_args* a, void* stream) {
+int jvpfa_mask_tiles(const jvpfa_mask_tiles_args* args, void* stream) {
+  jvpfa_mask_tiles_args full;
+  const jvpfa_mask_tiles_args* a = current_args(args, &full, offsetof(jvpfa_mask_tiles_args, bits));
   if (!a) return JVPFA_ERR_NULL;
   if (a->struct_size != (int32_t)sizeof(jvpfa_mask_tiles_args)) return JVPFA_ERR_STRUCT;
   if (a->n_b < 1 || a->n_h < 1 || a->L < 1 || (a->n_rows != 1 && a->n_rows != a->L)) return JVPFA_ERR_SHAPE;
@@ -255,7 +267,6 @@ int jvpfa_mask_tiles(const jvpfa_mask_tiles_args* a, void* stream) {
   if (a->mask.kind != JVPFA_MASK_BOOL || !a->mask.ptr) return JVPFA_ERR_MASK;
   for (int d = 0; d < 4; ++d)
     if (a->mask.stride[d] < 0) return JVPFA_ERR_MASK;
-  if (!tc5_mask_layout(a->mask, JVPFA_BF16, a->L)) return JVPFA_ERR_UNSUPPORTED;
   const int rc = check_arch();
   if (rc) return rc;
   return launch_mask_tiles(*a, static_cast<cudaStream_t>(stream));

@@ -39,6 +39,12 @@ __global__ void __launch_bounds__(256) pre_kernel(const jvpfa_pre_args a, long l
   const int c = (tid % TPR) * VEC;
   const bool ok = row < rows;
   const bool has_go = a.go != nullptr, has_g = a.gto != nullptr;
+  // dQ's accumulation buffer, cleared on the way: one launch and its gap less than a memset of its own
+  if (ok && a.dq_accum != nullptr) {
+    float4* z = reinterpret_cast<float4*>(a.dq_accum + (size_t)row * D + c);
+#pragma unroll
+    for (int i = 0; i < VEC / 4; ++i) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
 
   float d = 0.f, e = 0.f, dd = 0.f;
   if (ok) {
@@ -618,8 +624,8 @@ static int launch_bwd_one(const jvpfa_bwd_args& a, cudaStream_t stream) {
   if (!opt_in1.ensure(reinterpret_cast<const void*>(k1), smem_kv) || !opt_in2.ensure(reinterpret_cast<const void*>(k2), smem_q))
     return JVPFA_ERR_CUDA;
   dim3 grid((a.L + C::OWN - 1) / C::OWN, a.B * a.H);
-  if (!(a.skip & JVPFA_SKIP_DKDV)) k1<<<grid, C::NTHREADS, smem_kv, stream>>>(a);
-  if (!(a.skip & JVPFA_SKIP_DQ)) k2<<<grid, C::NTHREADS, smem_q, stream>>>(a);
+  if (!(a.flags & JVPFA_SKIP_DKDV)) k1<<<grid, C::NTHREADS, smem_kv, stream>>>(a);
+  if (!(a.flags & JVPFA_SKIP_DQ)) k2<<<grid, C::NTHREADS, smem_q, stream>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch bwd_generic");

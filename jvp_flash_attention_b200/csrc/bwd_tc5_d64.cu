@@ -712,6 +712,13 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
                 ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1]) * MESZ;
         mpitch = a.mask.stride[2] * MESZ;
       }
+      const uint32_t* bits = nullptr;  // packed boolean mask: this thread's row of it (of the transpose for keys)
+      if constexpr (BOOLM) {
+        const void* packed = OWN_KEYS ? a.mask_bits_t : a.mask_bits;
+        const long long hm = mask_head(a.mask, it.b, it.h, a.H);
+        if (packed != nullptr)
+          bits = OWN_KEYS ? mask_bit_col(packed, a.mask, hm, min(own_idx, L - 1), L) : mask_bit_row(packed, a.mask, hm, min(own_idx, L - 1), L);
+      }
 
       float r_nlse = -INFINITY, r_nmu = 0.f, r_neps = 0.f, r_nsub = 0.f;
       if constexpr (!OWN_KEYS) {
@@ -737,15 +744,26 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
         const int l0 = sub_l0<BL>(it, s);
         // MK != 0: the thread's 32 mask / bias elements of this sub-tile, requested before the waits.
         // Indices are clamped into the tensor; what lies outside is switched off by col_lo / col_hi below.
-        constexpr int NRAW = MK == 0 ? 1 : (OWN_KEYS ? 32 : 8 * MESZ);
+        constexpr int NRAW = MK != 2 ? 1 : (OWN_KEYS ? 32 : 16);
         uint32_t raw[NRAW];
-        if constexpr (MK != 0) {
+        uint32_t live = 0xffffffffu;  // BOOLM: bit col = the mask lets the pair attend
+        if (BOOLM && bits != nullptr) {
+          live = l0 < L ? ldg_nc_u32(bits + (OWN_KEYS && !a.mask.stride[2] ? 0 : l0 >> 5)) : 0u;
+        } else if constexpr (BOOLM && OWN_KEYS) {
+          const unsigned char* p = mbase + (long long)min(own_idx, L - 1);
+          live = 0u;
+#pragma unroll
+          for (int col = 0; col < 32; ++col) live |= (ldg_nc_u8(p + (long long)min(l0 + col, L - 1) * mpitch) != 0u ? 1u : 0u) << col;
+        } else if constexpr (BOOLM) {
+          const unsigned char* p = mbase + (long long)min(own_idx, L - 1) * mpitch + l0;
+          live = mask_piece_bits(p, l0, L) | mask_piece_bits(p + 16, l0 + 16, L) << 16;
+        } else if constexpr (MK == 2) {
           if constexpr (OWN_KEYS) {
             const unsigned char* p = mbase + (long long)min(own_idx, L - 1) * MESZ;
 #pragma unroll
             for (int col = 0; col < 32; ++col) {
               const unsigned char* e = p + (long long)min(l0 + col, L - 1) * mpitch;
-              raw[col] = BOOLM ? ldg_nc_u8(e) : ldg_nc_u16(e);
+              raw[col] = ldg_nc_u16(e);
             }
           } else {
             const unsigned char* p = mbase + (long long)min(own_idx, L - 1) * mpitch + (size_t)l0 * MESZ;
@@ -781,18 +799,8 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
         }
         // MK = 1: bit col of live = column col may attend (mask and index range together);
         // MK = 2: mb[x] = the bias of columns 2x, 2x+1 as a packed pair
-        uint32_t live = 0xffffffffu;
         uint32_t mb[MK == 2 ? 16 : 1];
         if constexpr (BOOLM) {
-          live = 0u;
-          if constexpr (OWN_KEYS) {
-#pragma unroll
-            for (int col = 0; col < 32; ++col) live |= (raw[col] != 0u ? 1u : 0u) << col;
-          } else {
-#pragma unroll
-            for (int w = 0; w < 8; ++w)  // bytes -> 0/1 -> four bits
-              live |= (((__vcmpne4(raw[w], 0u) & 0x01010101u) * 0x01020408u) >> 24) << (4 * w);
-          }
           const int lo = max(col_lo, 0), hi = min(col_hi, BL);
           live &= hi > lo ? ((hi - lo >= 32 ? 0xffffffffu : ((1u << (hi - lo)) - 1u)) << lo) : 0u;
         }
@@ -940,11 +948,8 @@ static int launch_half64(const jvpfa_bwd_args& a, cudaStream_t stream, int* stat
     return JVPFA_ERR_CUDA;
   }
   auto kern = bwd_tc5_d64_kernel<T, OWN_KEYS, HAS_GO, HAS_GT, MK>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-  if (e != cudaSuccess) {
-    set_last_cuda_error(e, "cudaFuncSetAttribute(bwd_tc5_d64)");
-    return JVPFA_ERR_CUDA;
-  }
+  static SmemOptIn opt_in;
+  if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return JVPFA_ERR_CUDA;
   const long long n_items = (long long)((a.L + C::OWN - 1) / C::OWN) * BH;
   const int grid = (int)(n_items < sms ? n_items : sms);
   cudaLaunchConfig_t cfg = {};
@@ -954,7 +959,7 @@ static int launch_half64(const jvpfa_bwd_args& a, cudaStream_t stream, int* stat
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr, cfg.numAttrs = overlap_previous ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, a, m, status);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a, m, status);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch bwd_tc5_d64");
@@ -971,10 +976,10 @@ static int launch_both64(const jvpfa_bwd_args& a, cudaStream_t s) {
     return JVPFA_ERR_CUDA;
   }
   // Without the own-keys launch before it, the own-queries launch must not start early: it reads what the preprocess wrote.
-  const bool keys = !(a.skip & JVPFA_SKIP_DKDV);
+  const bool keys = !(a.flags & JVPFA_SKIP_DKDV);
   int rc = JVPFA_OK;
   if (keys) rc = launch_half64<T, true, HAS_GO, HAS_GT, MK>(a, s, status, false);
-  if (rc || (a.skip & JVPFA_SKIP_DQ)) return rc;
+  if (rc || (a.flags & JVPFA_SKIP_DQ)) return rc;
   rc = launch_half64<T, false, HAS_GO, HAS_GT, MK>(a, s, status, keys);
   return rc;
 }

@@ -529,15 +529,22 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
         continue;
       }
       const int n_valid = valid_keys(it.b);
+      const uint32_t* bcol = nullptr;  // packed boolean mask: this key's bits over the queries
+      if (MK == 1 && a.mask_bits_t != nullptr)
+        bcol = mask_bit_col(a.mask_bits_t, a.mask, mask_head(a.mask, it.b, it.h, a.H), min(own_idx, L - 1), L);
       for (int s = 0; s < it.n_sub; ++s, ++g) {
         const int st = g % STAGES;
         const int l0 = it.loop_begin + s * BL + 32 * wg;  // first query of this group's columns
-        // MK = 1: this key's mask bytes for the 32 queries, requested before the waits (indices clamped into the
-        // tensor; what lies outside is switched off by col_hi and by lse = +inf of the padding queries)
+        // MK = 1: this key's mask bits for the 32 queries, requested before the waits (packed: one word; else byte by
+        // byte, indices clamped into the tensor; what lies outside is switched off by col_hi and by lse = +inf of the
+        // padding queries)
         // MK = 2 (backward through O alone: the variants with tangents have no registers to spare): the bias elements
         // of the same positions, 16 bit each, of the tensors' type.
-        uint32_t mraw[MK != 0 ? 32 : 1];
-        if constexpr (MK != 0) {
+        uint32_t live = 0xffffffffu;  // MK = 1: bit col = the mask lets query l0 + col attend this key
+        uint32_t mraw[MK == 2 ? 32 : 1];
+        if (MK == 1 && bcol != nullptr) {
+          live = l0 < L ? ldg_nc_u32(bcol + (a.mask.stride[2] ? l0 >> 5 : 0)) : 0u;
+        } else if constexpr (MK != 0) {
           constexpr int MESZ = MK == 1 ? 1 : 2;
           const unsigned char* pm = reinterpret_cast<const unsigned char*>(a.mask.ptr) +
                                     ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] +
@@ -545,7 +552,12 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 #pragma unroll
           for (int col = 0; col < 32; ++col) {
             const unsigned char* el = pm + (long long)min(l0 + col, L - 1) * a.mask.stride[2] * MESZ;
-            mraw[col] = MK == 1 ? ldg_nc_u8(el) : ldg_nc_u16(el);
+            if constexpr (MK == 1) {
+              if (col == 0) live = 0u;
+              live |= (ldg_nc_u8(el) != 0u ? 1u : 0u) << col;
+            } else {
+              mraw[col] = ldg_nc_u16(el);
+            }
           }
         }
         if (!mbar_wait(stat_full + st, (g / STAGES) & 1, ab, kAbortBwdLoopFull) ||
@@ -554,12 +566,6 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           break;
         }
         tc_fence_after();
-        uint32_t live = 0xffffffffu;  // MK = 1: bit col = the mask lets query l0 + col attend this key
-        if constexpr (MK == 1) {
-          live = 0u;
-#pragma unroll
-          for (int col = 0; col < 32; ++col) live |= (mraw[col] != 0u ? 1u : 0u) << col;
-        }
         uint32_t sv[32], fp[32], ts[HAS_GT ? 32 : 1], ev[HAS_GT ? 32 : 1];
         tmem_ld32(tbase + C::COL_S, sv);
         tmem_ld32(tbase + C::COL_FP, fp);
@@ -618,7 +624,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           const int lo = max(col_lo, 0), hi = min(col_hi, 32);
           live &= hi > lo ? ((hi - lo >= 32 ? 0xffffffffu : ((1u << (hi - lo)) - 1u)) << lo) : 0u;
         }
-        if (MK == 1 || __any_sync(0xffffffffu, col_lo > 0 || col_hi < 32)) {
+        if (__any_sync(0xffffffffu, MK == 1 ? live != 0xffffffffu : (col_lo > 0 || col_hi < 32))) {
 #pragma unroll
           for (int x = 0; x < 16; ++x) pair(x, IntC<1>{});
         } else {
@@ -795,17 +801,15 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
     return JVPFA_ERR_CUDA;
   }
   const size_t n = (size_t)a.B * a.H * a.L * a.D;
-  cudaError_t e = cudaMemsetAsync(a.dq_accum, 0, n * sizeof(float), stream);
+  cudaError_t e = cudaSuccess;
+  if (!(a.flags & JVPFA_DQ_ACCUM_IS_ZERO)) e = cudaMemsetAsync(a.dq_accum, 0, n * sizeof(float), stream);
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "cudaMemsetAsync(dq_accum)");
     return JVPFA_ERR_CUDA;
   }
   auto kern = bwd_tc5_fused64_kernel<T, HAS_GO, HAS_GT, MK>;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-  if (e != cudaSuccess) {
-    set_last_cuda_error(e, "cudaFuncSetAttribute(bwd_tc5_fused64)");
-    return JVPFA_ERR_CUDA;
-  }
+  static SmemOptIn opt_in;
+  if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return JVPFA_ERR_CUDA;
   const long long n_items = (long long)((a.L + C::OWN - 1) / C::OWN) * a.B * a.H;
   const int grid = (int)(n_items < sms ? n_items : sms);
   kern<<<grid, C::NTHREADS, C::SMEM_BYTES, stream>>>(a, m, a.dq_accum, status);
@@ -815,7 +819,7 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
     return JVPFA_ERR_CUDA;
   }
   const long long n8 = (long long)(n / 8);
-  if (a.skip & JVPFA_SKIP_DQ) return JVPFA_OK;
+  if (a.flags & JVPFA_SKIP_DQ) return JVPFA_OK;
   dq_convert_kernel<T><<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(a.dq_accum, reinterpret_cast<T*>(a.dq), n8, a.sm_scale);
   e = cudaGetLastError();
   if (e != cudaSuccess) {

@@ -502,6 +502,13 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
               ((long long)tma_b * a.mask.stride[0] + (long long)tma_h * a.mask.stride[1]) * MESZ;
       mpitch = a.mask.stride[2] * MESZ;
     }
+    const uint32_t* bits = nullptr;  // packed boolean mask: this thread's row of it (of the transpose for keys)
+    if constexpr (BOOLM) {
+      const void* packed = OWN_KEYS ? a.mask_bits_t : a.mask_bits;
+      const long long hm = mask_head(a.mask, tma_b, tma_h, a.H);
+      if (packed != nullptr)
+        bits = OWN_KEYS ? mask_bit_col(packed, a.mask, hm, min(own_idx, L - 1), L) : mask_bit_row(packed, a.mask, hm, min(own_idx, L - 1), L);
+    }
 
     auto walk = walk0;
     for (int t = 0; t < n_tiles; ++t) {
@@ -509,15 +516,25 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
       const int l0 = MK == 3 ? walk.next() * BL : loop_begin + t * BL;
       // MK != 0: the piece's 16 mask / bias elements, one per column (indices clamped into the tensor; what lies
       // outside is switched off by the index tests below)
-      uint32_t mraw[MK == 0 ? 1 : 16];
-      if constexpr (MK != 0) {
-        const int c0 = l0 + 16 * piece;  // first loop-side index of this thread's columns
+      uint32_t mraw[MK == 2 ? 16 : 1];
+      uint32_t live = 0xffffu;  // BOOLM: bit x = the mask lets column x attend
+      const int c0 = l0 + 16 * piece;  // first loop-side index of this thread's columns (a multiple of 16)
+      if (BOOLM && bits != nullptr) {
+        live = c0 < L ? (ldg_nc_u32(bits + (OWN_KEYS && !a.mask.stride[2] ? 0 : c0 >> 5)) >> (c0 & 16)) & 0xffffu : 0u;
+      } else if constexpr (BOOLM && OWN_KEYS) {
+        const unsigned char* pm = mbase + (long long)min(own_idx, L - 1);
+        live = 0u;
+#pragma unroll
+        for (int x = 0; x < 16; ++x) live |= (ldg_nc_u8(pm + (long long)min(c0 + x, L - 1) * mpitch) != 0u ? 1u : 0u) << x;
+      } else if constexpr (BOOLM) {
+        live = mask_piece_bits(mbase + (long long)min(own_idx, L - 1) * mpitch + c0, c0, L);
+      } else if constexpr (MK == 2) {
         if constexpr (OWN_KEYS) {
           const unsigned char* pm = mbase + (long long)min(own_idx, L - 1) * MESZ;
 #pragma unroll
           for (int x = 0; x < 16; ++x) {
             const unsigned char* el = pm + (long long)min(c0 + x, L - 1) * mpitch;
-            mraw[x] = BOOLM ? ldg_nc_u8(el) : ldg_nc_u16(el);
+            mraw[x] = ldg_nc_u16(el);
           }
         } else {
           const unsigned char* pm = mbase + (long long)min(own_idx, L - 1) * mpitch + (size_t)c0 * MESZ;
@@ -530,7 +547,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
           }
 #pragma unroll
           for (int x = 0; x < 16; ++x)
-            mraw[x] = BOOLM ? ((w[x >> 2] >> ((x & 3) * 8)) & 0xffu) : ((w[x >> 1] >> ((x & 1) * 16)) & 0xffffu);
+            mraw[x] = (w[x >> 1] >> ((x & 1) * 16)) & 0xffffu;
         }
       }
       if constexpr (OWN_KEYS) {
@@ -585,7 +602,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
           if constexpr (MK == 2) arg = fmaf(unpack1<T>(mraw[col]), kLog2e, arg);  // scores are in log2 units
           float p = fast_exp2(arg);
           if constexpr (BOOLM)
-            if (mraw[col] == 0u) p = 0.f;
+            if (!((live >> col) & 1u)) p = 0.f;
           if (partial && (j >= n_valid || (causal && j > i))) p = 0.f;
           pv[h] = p;
           if constexpr (HAS_GT) {
@@ -692,11 +709,8 @@ static int launch_pipe_half(const jvpfa_bwd_args& a, cudaStream_t stream, int* s
     return JVPFA_ERR_CUDA;
   }
   auto kern = bwd_tc5_pipe128_kernel<T, OWN_KEYS, HAS_GO, HAS_GT, MK>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-  if (e != cudaSuccess) {
-    set_last_cuda_error(e, "cudaFuncSetAttribute(bwd_tc5_pipe128)");
-    return JVPFA_ERR_CUDA;
-  }
+  static SmemOptIn opt_in;
+  if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return JVPFA_ERR_CUDA;
   dim3 grid((a.L + C::OWN - 1) / C::OWN, a.B * a.H);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid, cfg.blockDim = dim3(C::NTHREADS);
@@ -705,7 +719,7 @@ static int launch_pipe_half(const jvpfa_bwd_args& a, cudaStream_t stream, int* s
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr, cfg.numAttrs = overlap_previous ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, a, m, status);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a, m, status);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch bwd_tc5_pipe128");
@@ -722,10 +736,10 @@ static int launch_pipe_both(const jvpfa_bwd_args& a, cudaStream_t s) {
     return JVPFA_ERR_CUDA;
   }
   // Without the own-keys launch before it, the own-queries launch must not start early: it reads what the preprocess wrote.
-  const bool keys = !(a.skip & JVPFA_SKIP_DKDV);
+  const bool keys = !(a.flags & JVPFA_SKIP_DKDV);
   int rc = JVPFA_OK;
   if (keys) rc = launch_pipe_half<T, true, HAS_GO, HAS_GT, MK>(a, s, status, false);
-  if (rc || (a.skip & JVPFA_SKIP_DQ)) return rc;
+  if (rc || (a.flags & JVPFA_SKIP_DQ)) return rc;
   return launch_pipe_half<T, false, HAS_GO, HAS_GT, MK>(a, s, status, keys);
 }
 

@@ -281,9 +281,14 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
     bool alive = true;
 
     constexpr bool BOOLM = MK == 1 || MK == 3;
-    constexpr int MESZ = BOOLM ? 1 : 2;        // bytes per mask element
-    constexpr int MW = MK == 0 ? 1 : 16 * MESZ;  // 32-bit words per row of a 64-key tile
+    constexpr int MESZ = BOOLM ? 1 : 2;   // bytes per mask element
+    constexpr int MW = MK == 2 ? 32 : 1;  // 32-bit words per row of a 64-key tile of bias elements
     const unsigned char* mrow = nullptr;
+    const uint32_t* brow = nullptr;  // packed boolean mask
+    if constexpr (BOOLM) {
+      if (a.mask_bits != nullptr)
+        brow = mask_bit_row(a.mask_bits, a.mask, mask_head(a.mask, tma_b, tma_h, a.H), min(i, L - 1), L);
+    }
     if constexpr (MK != 0)
       mrow = reinterpret_cast<const unsigned char*>(a.mask.ptr) +
              ((long long)tma_b * a.mask.stride[0] + (long long)tma_h * a.mask.stride[1] +
@@ -294,7 +299,16 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
       const int st = t & 1;
       const uint32_t tS = tmem + lane_off + st * C::SC_COLS, tTS = tS + BN;
       uint32_t mw[MW];
-      if constexpr (MK != 0) {  // issued before the wait: the loads fly while the scores are formed
+      uint2 keys = make_uint2(~0u, ~0u);  // BOOLM: bit c of (x, y) = the mask lets this row attend key n0 + c
+      if constexpr (BOOLM) {
+        if (brow != nullptr) {
+          keys = ldg_nc_v2(brow + (n0 >> 5));
+        } else {
+          keys.x = mask_piece_bits(mrow + n0, n0, L) | mask_piece_bits(mrow + n0 + 16, n0 + 16, L) << 16;
+          keys.y = mask_piece_bits(mrow + n0 + 32, n0 + 32, L) | mask_piece_bits(mrow + n0 + 48, n0 + 48, L) << 16;
+        }
+      }
+      if constexpr (MK == 2) {  // issued before the wait: the loads fly while the scores are formed
 #pragma unroll
         for (int q4 = 0; q4 < MW / 4; ++q4) {
           uint4 r = make_uint4(0u, 0u, 0u, 0u);
@@ -315,13 +329,25 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
       int col_hi = min(BN, n_valid - n0);
       if (causal) col_hi = min(col_hi, i - n0 + 1);
       const bool partial = (n0 + BN > n_valid) || (causal && n0 + BN - 1 > m0);
-      // Row maximum of the tile in log2 units.  Without a mask or bias and with a positive scale it is taken over
-      // the raw scores and the scaling is folded into the exponent's multiply-add; otherwise the scores are scaled,
-      // biased and masked first.
-      const bool raw_max = MK == 0 && a.sm_scale > 0.f;
+      // Row maximum of the tile in log2 units.  Without a bias and with a positive scale it is taken over the raw
+      // scores and the scaling is folded into the exponent's multiply-add; otherwise the scores are scaled, biased and
+      // masked first.
+      const bool raw_max = MK != 2 && a.sm_scale > 0.f;
       float mx;
+      if constexpr (BOOLM) {
+        if (partial) keys.x &= first_columns(col_hi), keys.y &= first_columns(col_hi - 32);
+      }
       if (raw_max) {
-        if (partial) {
+        if constexpr (BOOLM) {
+          if (__any_sync(0xffffffffu, (keys.x & keys.y) != ~0u)) {  // (inside a window or a document no entry is False)
+#pragma unroll
+            for (int c = 0; c < 32; ++c) {
+              if (!((keys.x >> c) & 1u)) x0[c] = 0xff800000u;  // -inf
+              if (!((keys.y >> c) & 1u)) x1[c] = 0xff800000u;
+            }
+          }
+        }
+        if (MK == 0 && partial) {
 #pragma unroll
           for (int c = 0; c < 32; ++c) {
             if (c >= col_hi) x0[c] = 0xff800000u;  // -inf
@@ -343,20 +369,18 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
         for (int c = 0; c < 16; ++c) {
           float2 v0 = __fmul2_rn(pf2(x0[2 * c], x0[2 * c + 1]), c2);
           float2 v1 = __fmul2_rn(pf2(x1[2 * c], x1[2 * c + 1]), c2);
-          if constexpr (BOOLM) {  // one byte per key: columns 2c, 2c+1 and 32+2c, 33+2c
-            constexpr uint32_t kLoByte = 0xffu, kHiByte = 0xff00u;
-            const uint32_t wa = mw[c >> 1] >> ((c & 1) * 16), wb = mw[8 + (c >> 1)] >> ((c & 1) * 16);
-            if (!(wa & kLoByte)) v0.x = -INFINITY;
-            if (!(wa & kHiByte)) v0.y = -INFINITY;
-            if (!(wb & kLoByte)) v1.x = -INFINITY;
-            if (!(wb & kHiByte)) v1.y = -INFINITY;
+          if constexpr (BOOLM) {
+            if (!((keys.x >> (2 * c)) & 1u)) v0.x = -INFINITY;
+            if (!((keys.x >> (2 * c + 1)) & 1u)) v0.y = -INFINITY;
+            if (!((keys.y >> (2 * c)) & 1u)) v1.x = -INFINITY;
+            if (!((keys.y >> (2 * c + 1)) & 1u)) v1.y = -INFINITY;
           }
           if constexpr (MK == 2) {  // scores are in log2 units: bias * log2(e)
             const float2 l2 = make_float2(kLog2e, kLog2e);
             v0 = __ffma2_rn(unpack2<T>(mw[c]), l2, v0);
             v1 = __ffma2_rn(unpack2<T>(mw[16 + c]), l2, v1);
           }
-          if (partial) {
+          if (!BOOLM && partial) {
             if (2 * c >= col_hi) v0.x = -INFINITY;
             if (2 * c + 1 >= col_hi) v0.y = -INFINITY;
             if (32 + 2 * c >= col_hi) v1.x = -INFINITY;
@@ -541,14 +565,11 @@ static int launch_pipe128(const jvpfa_fwd_args& a, cudaStream_t stream) {
     return JVPFA_ERR_CUDA;
   }
   auto kern = fwd_tc5_pipe128_kernel<T, DUAL, MK>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-  if (e != cudaSuccess) {
-    set_last_cuda_error(e, "cudaFuncSetAttribute(fwd_tc5_pipe128)");
-    return JVPFA_ERR_CUDA;
-  }
+  static SmemOptIn opt_in;
+  if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return JVPFA_ERR_CUDA;
   dim3 grid((a.L + C::BM - 1) / C::BM, a.B * a.H);
   kern<<<grid, C::NTHREADS, C::SMEM_BYTES, stream>>>(a, maps, status);
-  e = cudaGetLastError();
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch fwd_tc5_pipe128");
     return JVPFA_ERR_CUDA;

@@ -15,6 +15,8 @@
 // module's _launch_fwd / _launch_bwd (the CPU suite puts its oracle there), so there is one graph, not two.
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/functorch/DynamicLayer.h>
+#include <ATen/functorch/TensorWrapper.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
@@ -50,11 +52,11 @@ py::object& python_module() {
 // The kernel-side mask description, built once per mask.  `spec` is the Python object it was made from.
 struct MaskDesc {
   jvpfa_mask c{};
-  Tensor tensor, tile_live, tile_live_t;
+  Tensor tensor, tile_live, tile_live_t, bits, bits_t;
   std::shared_ptr<py::object> spec;
 
   MaskDesc(int kind, int bias_dtype, std::optional<Tensor> t, std::array<int64_t, 4> strides, std::optional<Tensor> live,
-           std::optional<Tensor> live_t, py::object spec_)
+           std::optional<Tensor> live_t, std::optional<Tensor> bits_, std::optional<Tensor> bits_t_, py::object spec_)
       : spec(new py::object(std::move(spec_)), [](py::object* o) {
           py::gil_scoped_acquire gil;
           delete o;
@@ -65,6 +67,8 @@ struct MaskDesc {
     if (t) tensor = *t;
     if (live) tile_live = *live;
     if (live_t) tile_live_t = *live_t;
+    if (bits_) bits = *bits_;
+    if (bits_t_) bits_t = *bits_t_;
     if (kind == JVPFA_MASK_KVLEN)
       c.kv_len = static_cast<const int32_t*>(tensor.data_ptr());
     else if (kind == JVPFA_MASK_BOOL || kind == JVPFA_MASK_BIAS)
@@ -84,11 +88,12 @@ bool is_wrapped(const Tensor& x) {
   return x.key_set().has(c10::DispatchKey::FuncTorchGradWrapper) || x.key_set().has(c10::DispatchKey::FuncTorchBatched);
 }
 
-// The tensor under functorch's wrappers (met only when a transform is differentiated around the call: the slow way).
+// The tensor under functorch's wrappers.
 Tensor unwrap(Tensor x) {
-  while (x.defined() && is_wrapped(x)) {
-    py::gil_scoped_acquire gil;
-    x = py::module_::import("torch._C._functorch").attr("get_unwrapped")(x).cast<Tensor>();
+  while (x.defined()) {
+    auto* w = at::functorch::maybeGetTensorWrapper(x);
+    if (!w) break;
+    x = Tensor(w->value());
   }
   return x;
 }
@@ -214,6 +219,7 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   a.mu = dual ? static_cast<float*>(r.mu.data_ptr()) : nullptr;
   a.mask = call.mask->c;
   a.mask_tile_live = data(call.mask->tile_live);
+  a.mask_bits = data(call.mask->bits);
   void* stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
   for (;;) {
     a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
@@ -276,6 +282,7 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   p.o = data(o), p.to = data(to), p.go = data(go), p.gto = data(gto);
   p.mu = static_cast<const float*>(data(mu));
   p.delta = f, p.eps = f + stat, p.cterm = f + 2 * stat;
+  p.dq_accum = single ? f + 3 * stat : nullptr;
   check_status(jvpfa_bwd_preprocess(&p, stream), "jvpfa_bwd_preprocess");
 
   Grads g;
@@ -292,7 +299,7 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.lse = static_cast<const float*>(data(lse));
   a.mu = p.mu;
   a.delta = p.delta, a.eps = p.eps, a.cterm = p.cterm;
-  a.skip = skip;
+  a.flags = skip | (single ? JVPFA_DQ_ACCUM_IS_ZERO : 0);
   if (g[0].defined()) a.dq = g[0].data_ptr();
   if (g[1].defined()) a.dk = g[1].data_ptr(), a.dv = g[2].data_ptr();
   a.mask = m.c;
@@ -300,7 +307,9 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
     a.mask_tile_live = data(m.tile_live);
     a.mask_tile_live_t = data(m.tile_live_t);
   }
-  a.dq_accum = single ? f + 3 * stat : nullptr;
+  a.dq_accum = p.dq_accum;
+  a.mask_bits = data(m.bits);
+  a.mask_bits_t = data(m.bits_t);
   for (;;) {
     a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
     a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
@@ -487,8 +496,8 @@ struct Outputs {
 // The call itself on plain tensors; tangents all undefined or all given.  nullopt: not a case for this path.
 std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, Tensor tk, Tensor tv,
                                     const MaskPtr& mask, std::optional<double> scale, bool tf32, bool strict_length) {
-  for (const Tensor& t : {q, k, v, tq, tk, tv})
-    if (t.defined() && is_wrapped(t)) return std::nullopt;
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&q, &k, &v, &tq, &tk, &tv})
+    if (t->defined() && is_wrapped(*t)) return std::nullopt;
   if (!acceptable(q, k, v, strict_length)) return std::nullopt;
   const bool dual = tq.defined() || tk.defined() || tv.defined();
   if (dual) {
@@ -526,26 +535,35 @@ std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tens
   return Outputs{r.o, r.to};
 }
 
-// attention (dual = false) or fwd_dual (true) on plain or forward-AD dual tensors outside functorch transforms.  None:
-// not a case for this path (bad arguments, wrapped tensors, dual inputs of a primal-only call); the caller takes its
-// general route.
-py::object attend(const Tensor& q, const Tensor& k, const Tensor& v, const MaskPtr& mask, std::optional<double> scale, bool tf32,
-                  bool dual, bool strict_length) {
-  const Tensor tq = q._fw_grad(0), tk = k._fw_grad(0), tv = v._fw_grad(0);
-  if (!dual && (tq.defined() || tk.defined() || tv.defined())) return py::none();
+// attention (dual = false) or fwd_dual (true).  None: not a case for this path (bad arguments, dual inputs of a
+// primal-only call, functorch transforms other than a lone torch.func.jvp); the caller takes its general route.
+py::object attend(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const MaskPtr& mask, std::optional<double> scale,
+                  bool tf32, bool dual, bool strict_length) {
+  const auto& stack = at::functorch::getDynamicLayerStack();
+  Tensor q = q_in, k = k_in, v = v_in, tq = q._fw_grad(0), tk = k._fw_grad(0), tv = v._fw_grad(0);
+  const bool any_tangent = tq.defined() || tk.defined() || tv.defined();
+  if (!dual && any_tangent) return py::none();
+  int64_t level = -1;
+  if (!stack.empty()) {
+    // Primals and tangents are taken off the transform's wrappers, the call runs one level down on plain tensors, and
+    // the two results become a dual tensor of its level again: what torch.func.jvp does for a built-in operator.
+    if (!any_tangent || stack.size() != 1 || stack.back().key() != at::functorch::TransformType::Jvp) return py::none();
+    level = stack.back().layerId();
+    for (Tensor* t : {&q, &k, &v, &tq, &tk, &tv}) {
+      auto* w = t->defined() ? at::functorch::maybeGetTensorWrapper(*t) : nullptr;
+      if (w && w->level() == level) *t = Tensor(w->value());
+    }
+  }
   auto out = attend_plain(q, k, v, tq, tk, tv, mask, scale, tf32, strict_length);
   if (!out) return py::none();
-  if (out->to.defined()) out->o._set_fw_grad(out->to, /*level=*/0, /*is_inplace_op=*/false);
-  return py::cast(out->o);
-}
-
-// The same with the tangents as explicit arguments, for torch.func.jvp: returns (O, tO) on plain tensors, which the
-// caller wraps again.
-py::object attend_dual(const Tensor& q, const Tensor& k, const Tensor& v, std::optional<Tensor> tq, std::optional<Tensor> tk,
-                       std::optional<Tensor> tv, const MaskPtr& mask, std::optional<double> scale, bool tf32, bool strict_length) {
-  auto out = attend_plain(q, k, v, tq.value_or(Tensor()), tk.value_or(Tensor()), tv.value_or(Tensor()), mask, scale, tf32, strict_length);
-  if (!out || !out->to.defined()) return py::none();
-  return py::make_tuple(out->o, out->to);
+  if (!out->to.defined()) return py::cast(out->o);
+  Tensor o = out->o, to = out->to;
+  if (level >= 0) {
+    o = at::functorch::makeTensorWrapper(o, level);
+    to = at::functorch::makeTensorWrapper(to, level);
+  }
+  o._set_fw_grad(to, /*level=*/0, /*is_inplace_op=*/false);
+  return py::cast(o);
 }
 
 }  // namespace
@@ -556,11 +574,9 @@ PYBIND11_MODULE(_native, m) {
       .def("__enter__", [](NoFunctorchScope& s) { s.guard.emplace(); })
       .def("__exit__", [](NoFunctorchScope& s, py::args) { s.guard.reset(); });
   py::class_<MaskDesc, MaskPtr>(m, "MaskDesc")
-      .def(py::init<int, int, std::optional<Tensor>, std::array<int64_t, 4>, std::optional<Tensor>, std::optional<Tensor>, py::object>());
+      .def(py::init<int, int, std::optional<Tensor>, std::array<int64_t, 4>, std::optional<Tensor>, std::optional<Tensor>, std::optional<Tensor>,
+                    std::optional<Tensor>, py::object>());
   m.def("attend", &attend);
-  m.def("attend_dual", &attend_dual);
-  m.def("tangent_of", [](const Tensor& x) { return or_none(x._fw_grad(0)); });
-  m.def("set_tangent", [](const Tensor& x, const Tensor& t) { x._set_fw_grad(t, /*level=*/0, /*is_inplace_op=*/false); });
   m.def("set_impl", [](int v) { g_impl = v; });
   m.def("set_single_pass", [](bool v) { g_single_pass = v; });
 }

@@ -102,6 +102,41 @@ __device__ __forceinline__ uint32_t ldg_nc_u16(const void* p) {
   return r;
 }
 
+// Boolean masks.  A mask packed by jvpfa_mask_tiles is read as words; otherwise its bytes are turned into the same words.
+__device__ __forceinline__ uint2 ldg_nc_v2(const void* p) {
+  uint2 r;
+  asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ uint32_t ldg_nc_u32(const void* p) {
+  uint32_t r;
+  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(r) : "l"(p));
+  return r;
+}
+// index of (b, h) among the mask's own heads, and the words of one of its packed rows
+__device__ __forceinline__ long long mask_head(const jvpfa_mask& m, int b, int h, int H) {
+  return (m.stride[0] ? (long long)b * (m.stride[1] ? H : 1) : 0) + (m.stride[1] ? h : 0);
+}
+__device__ __forceinline__ const uint32_t* mask_bit_row(const void* bits, const jvpfa_mask& m, long long head, int i, int L) {
+  const long long row = m.stride[2] ? head * L + i : head;
+  return reinterpret_cast<const uint32_t*>(bits) + row * (((L + 63) >> 6) * 2);
+}
+// ... and of one of its packed columns (a single word that stands for every query when the mask has one row)
+__device__ __forceinline__ const uint32_t* mask_bit_col(const void* bits_t, const jvpfa_mask& m, long long head, int j, int L) {
+  return reinterpret_cast<const uint32_t*>(bits_t) + (head * L + j) * (m.stride[2] ? ((L + 63) >> 6) * 2 : 1);
+}
+__device__ __forceinline__ uint32_t bits_of_bytes(uint32_t w) {  // bytes -> four bits
+  return (((__vcmpne4(w, 0u) & 0x01010101u) * 0x01020408u) >> 24) & 0xfu;
+}
+// 16 mask bytes at p (a 16-byte piece that starts at key j of its row; 0 beyond the row) as 16 bits
+__device__ __forceinline__ uint32_t mask_piece_bits(const unsigned char* p, int j, int L) {
+  if (j >= L) return 0u;
+  const uint4 r = ldg_nc_v4(p);
+  return bits_of_bytes(r.x) | bits_of_bytes(r.y) << 4 | bits_of_bytes(r.z) << 8 | bits_of_bytes(r.w) << 12;
+}
+// the first n of 32 columns (n may be negative or beyond 32)
+__device__ __forceinline__ uint32_t first_columns(int n) { return n >= 32 ? ~0u : n <= 0 ? 0u : (1u << n) - 1u; }
+
 // Host: (D, L, H, B) view of a 16-bit tensor whose batch / head / row strides (in elements) are given
 // (all zero: (B,H,L,D) row-major); box = 64 columns x box_rows rows (a D = 128 tile is two loads), 128-byte swizzle,
 // out-of-range rows and columns read as zero.  Defined in fwd_tc5.cu.

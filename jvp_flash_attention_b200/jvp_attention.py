@@ -189,7 +189,7 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, qdtype: tor
     def bstrides(t: Tensor) -> tuple[int, int, int, int]:
         return tuple(0 if t.shape[d] == 1 else t.stride(d) for d in range(4))
 
-    # up to one tile of keys the mask is read element by element, whatever its layout
+    # up to one tile of keys a bias is read element by element, whatever its layout
     ragged = N > 64 and N * m.element_size() % 16 != 0 and qdtype in (torch.bfloat16, torch.float16)
     if m.dtype == torch.bool:
         if mh == 1 and mi == 1:
@@ -204,15 +204,13 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, qdtype: tor
                     assert min_len > 0, "The attention mask cannot be all False for any head."
                 kv_len = lens.expand(Z).contiguous() if mz == 1 else lens.contiguous()
                 return _lib.MaskSpec(_lib.MASK_KVLEN, kv_len), 1, attn_mask
-        if ragged and mi > 1:
-            m = _padded_rows(m, N)
         m8 = m.view(torch.uint8) if m.is_contiguous() or m.stride(-1) == 1 else m.contiguous().view(torch.uint8)
         spec = _lib.MaskSpec(_lib.MASK_BOOL, m8, bstrides(m8))
         every_head_live = True
         if verify:
-            # One pass answers upstream's check and says which 128 x 64 tiles have a True at all; forward and
-            # backward step over the others.  (Without verification the mask is not looked at beforehand, so
-            # there is no block skipping either: whether it would pay is known only from the pass's counts.)
+            # One pass answers upstream's check, packs the mask into bits and says which 128 x 64 tiles have a True at
+            # all; forward and backward step over the others.  (Without verification the mask is not looked at
+            # beforehand and is read byte by byte.)
             try:
                 spec.tile_live, head_live, spec.tile_live_t = _lib.mask_tiles(spec, N)
                 *heads, n_live = head_live.tolist()  # the one read-back
@@ -220,7 +218,7 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, qdtype: tor
                 n_entries = spec.tile_live.numel() // (((N + 63) // 64 + 63) // 64)
                 if n_live > 0.85 * n_entries * ((N + 63) // 64):
                     spec.tile_live = spec.tile_live_t = None  # (nearly) every tile is live: the plain loops are quicker
-            except _lib.Unsupported:  # layout not readable as 16-byte pieces: no skipping, element-wise check
+            except _lib.Unsupported:  # no summary of this mask: no skipping, element-wise check
                 every_head_live = _lib.mask_check(spec, m8.shape)[0]
         assert every_head_live, "The attention mask cannot be all False for any head."
         return spec, 1, attn_mask
@@ -674,38 +672,23 @@ def _attend(q, k, v, attn_mask, causal, sm_scale, dual):
     the native layer (csrc/native.cpp).  What that does not take (bad arguments, nested transforms) goes through the
     Python Function, which words the errors."""
     interp = _peek_functorch()
-    in_jvp = interp is not None and dual and interp.level() == 1 and interp.key() == _JVP  # torch.func.jvp alone
-    if interp is None or in_jvp:
+    if interp is None or (dual and interp.level() == 1 and interp.key() == _JVP):  # none, or torch.func.jvp alone
         native = _lib.native()
         if attn_mask is None:
             spec = _CAUSAL if causal else _NO_MASK
             if not q.is_cuda:
                 _check_args(q, k, v, None, None, None, None, causal)
         else:
-            if in_jvp and _functorch.is_functorch_wrapped_tensor(attn_mask):
+            if interp is not None and _functorch.is_functorch_wrapped_tensor(attn_mask):
                 attn_mask = _functorch._unwrap_for_grad(attn_mask, 1)
             spec = None if causal else _remembered_mask(attn_mask, q.shape)
             if spec is None:
                 _check_args(q, k, v, None, None, None, attn_mask, causal)
                 with native.NoFunctorch():  # the mask is a plain tensor, and so is what is found out about it
                     spec = classify_mask(attn_mask, causal, *q.shape[:3], q.dtype, True)[0]
-        tf32 = _lib.FP32_PRECISION == "tf32"
-        if not in_jvp:
-            out = native.attend(q, k, v, spec.native(), sm_scale, tf32, dual, STRICT_SEQUENCE_LENGTH)
-            if out is not None:
-                return out
-        else:
-            # Primals and tangents are taken off the transform's wrappers, the call runs one level down on plain
-            # tensors, and the two results become a dual tensor of its level again, as for a built-in operator.
-            raw = [_functorch._unwrap_for_grad(x, 1) for x in (q, k, v)]
-            for x in (q, k, v):
-                t = native.tangent_of(x)
-                raw.append(None if t is None else _functorch._unwrap_for_grad(t, 1))
-            out = native.attend_dual(*raw, spec.native(), sm_scale, tf32, STRICT_SEQUENCE_LENGTH)
-            if out is not None:
-                o = _functorch._wrap_for_grad(out[0], 1)
-                native.set_tangent(o, _functorch._wrap_for_grad(out[1], 1))
-                return o
+        out = native.attend(q, k, v, spec.native(), sm_scale, _lib.FP32_PRECISION == "tf32", dual, STRICT_SEQUENCE_LENGTH)
+        if out is not None:
+            return out
     q_t, k_t, v_t = (fwAD.unpack_dual(x).tangent for x in (q, k, v)) if dual else (None, None, None)
     # every positional argument given: the quick signature binding applies
     return _Attn.apply(q, k, v, q_t, k_t, v_t, attn_mask, causal, sm_scale, True)[0]
