@@ -297,7 +297,8 @@ typedef struct {
   /* Optional: the mask as one bit per entry (0 beyond the ends).  bits: [head][row][2*ceil(L/64)] 32-bit words, key j of a
    * row in bit j % 32 of word j / 32; bits_t: the transpose, [head][key][2*ceil(L/64)] words over the queries, or one word
    * per key (all ones or zero) when n_rows is 1.  Heads are the mask's own (n_b*n_h).  16-byte aligned.  A caller built
-   * without these fields (struct_size up to tile_live_t) gets neither. */
+   * without these fields (struct_size up to tile_live_t) gets neither.  For the bits alone tile_live, head_live and
+   * tile_live_t are NULL. */
   void* bits;
   void* bits_t;
 } jvpfa_mask_tiles_args;

@@ -302,8 +302,7 @@ class MaskSpec:
     bias, or int32 kv_len) and ``strides`` are the broadcast element strides of a (B,H,L,L) view.
     """
 
-    __slots__ = ("kind", "tensor", "strides", "bias_dtype", "tile_live", "tile_live_t", "bits", "bits_t", "fp32_mode",
-                 "_native")
+    __slots__ = ("kind", "tensor", "strides", "bias_dtype", "tile_live", "tile_live_t", "fp32_mode", "_native")
 
     def __init__(self, kind=MASK_NONE, tensor=None, strides=(0, 0, 0, 0), bias_dtype=FP32):
         self.kind = kind
@@ -312,7 +311,6 @@ class MaskSpec:
         self.bias_dtype = bias_dtype
         self.tile_live = None  # MASK_BOOL: bitmap from mask_tiles(), lets the forward step over dead tiles
         self.tile_live_t = None  # ... and its transpose (per 128-key tile), for the backward launch that owns keys
-        self.bits = self.bits_t = None  # MASK_BOOL: the mask packed by mask_tiles(), by rows and transposed
         self._native = None  # the native layer's form of this description, made on first use
         self.fp32_mode = None  # fp32 precision the forward of this call ran under ("3xtf32" / "tf32"); None = current
 
@@ -320,7 +318,7 @@ class MaskSpec:
         """This (by now complete) description as the native layer takes it."""
         if self._native is None:
             self._native = native().MaskDesc(self.kind, self.bias_dtype, self.tensor, self.strides, self.tile_live,
-                                             self.tile_live_t, self.bits, self.bits_t, copy.copy(self))
+                                             self.tile_live_t, copy.copy(self))
         return self._native
 
     def to_c(self) -> Mask:
@@ -390,7 +388,6 @@ def fwd(q, k, v, tq, tk, tv, o, to, lse, mu, mask: MaskSpec, sm_scale: float, im
     a.o, a.to, a.lse, a.mu = ptr(o), ptr(to), ptr(lse), ptr(mu)
     a.mask = mask.to_c()
     a.mask_tile_live = ptr(mask.tile_live)
-    a.mask_bits = ptr(mask.bits)
     if in_stride is not None:
         a.in_stride[0], a.in_stride[1], a.in_stride[2] = in_stride
     rc = _launch(q, lib.jvpfa_fwd, a)
@@ -421,8 +418,7 @@ def mask_tiles(mask: "MaskSpec", L: int):
     """Launches jvpfa_mask_tiles over a boolean mask (no synchronisation).  Returns ``(tile_live, head_live,
     tile_live_t)``: the int64 bitmap of 128 x 64 tiles with a true entry, which jvpfa_fwd / jvpfa_bwd take for block
     skipping, the int32 per-head flags followed by the count of live tiles, and the bitmap per 128-key tile.  The mask's
-    own extents follow its strides (0 = broadcast).  The mask itself, packed as bits, goes to ``mask.bits`` and
-    ``mask.bits_t``."""
+    own extents follow its strides (0 = broadcast)."""
     lib = load()
     t = mask.tensor
     n_b, n_h = (t.shape[d] if mask.strides[d] else 1 for d in (0, 1))
@@ -442,13 +438,8 @@ def mask_tiles(mask: "MaskSpec", L: int):
     a.tile_live = tile_live.data_ptr()
     a.head_live = head_live.data_ptr()
     a.tile_live_t = tile_live_t.data_ptr()
-    w = (L + 63) // 64 * 2
-    bits = torch.empty(n_b * n_h * n_rows * w, device=t.device, dtype=torch.int32)
-    bits_t = torch.empty(n_b * n_h * L * (w if n_rows > 1 else 1), device=t.device, dtype=torch.int32)
-    a.bits, a.bits_t = bits.data_ptr(), bits_t.data_ptr()
     rc = _launch(t, lib.jvpfa_mask_tiles, a)
     check(rc, "jvpfa_mask_tiles")
-    mask.bits, mask.bits_t = bits, bits_t
     return tile_live, head_live, tile_live_t
 
 
@@ -485,7 +476,6 @@ def bwd(q, k, v, tq, tk, tv, go, gto, lse, mu, delta, eps, cterm, dq, dk, dv, ma
     a.delta, a.eps, a.cterm = ptr(delta), ptr(eps), ptr(cterm)
     a.dq, a.dk, a.dv = ptr(dq), ptr(dk), ptr(dv)
     a.mask = mask.to_c()
-    a.mask_bits, a.mask_bits_t = ptr(mask.bits), ptr(mask.bits_t)
     if mask.tile_live is not None and mask.tile_live_t is not None and L <= 8192:
         a.mask_tile_live, a.mask_tile_live_t = ptr(mask.tile_live), ptr(mask.tile_live_t)
     if in_stride is not None:

@@ -263,7 +263,7 @@ int jvpfa_mask_tiles(const jvpfa_mask_tiles_args* args, void* stream) {
   if (a->struct_size != (int32_t)sizeof(jvpfa_mask_tiles_args)) return JVPFA_ERR_STRUCT;
   if (a->n_b < 1 || a->n_h < 1 || a->L < 1 || (a->n_rows != 1 && a->n_rows != a->L)) return JVPFA_ERR_SHAPE;
   if ((long long)a->n_b * a->n_h > 65535LL || (a->L + 127) / 128 > 65535) return JVPFA_ERR_TOO_LARGE;  // grid limits
-  if (!a->tile_live) return JVPFA_ERR_NULL;
+  if (!a->tile_live && (!(a->bits || a->bits_t) || a->head_live || a->tile_live_t)) return JVPFA_ERR_NULL;
   if (a->mask.kind != JVPFA_MASK_BOOL || !a->mask.ptr) return JVPFA_ERR_MASK;
   for (int d = 0; d < 4; ++d)
     if (a->mask.stride[d] < 0) return JVPFA_ERR_MASK;

@@ -131,7 +131,7 @@ bool fwd_tc5_eligible(const jvpfa_fwd_args& a) {
 
 // Boolean masks and bias of the tensors' type: the kernels read 16-byte pieces of mask rows, the last piece of a row as
 // well when only its head lies inside the row (what is beyond key L is then switched off by index).  That takes rows
-// padded to whole pieces, which the Python layer makes of a mask whose length does not fill them.
+// padded to whole pieces, which the native layer makes of a bias whose length does not fill them.
 bool tc5_mask_layout(const jvpfa_mask& m, int dtype, int L) {
   if (m.kind == JVPFA_MASK_BIAS && m.bias_dtype != dtype) return false;
   const long long esz = m.kind == JVPFA_MASK_BOOL ? 1 : 2;

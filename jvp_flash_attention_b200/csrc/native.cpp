@@ -52,11 +52,11 @@ py::object& python_module() {
 // The kernel-side mask description, built once per mask.  `spec` is the Python object it was made from.
 struct MaskDesc {
   jvpfa_mask c{};
-  Tensor tensor, tile_live, tile_live_t, bits, bits_t;
+  Tensor tensor, tile_live, tile_live_t;
   std::shared_ptr<py::object> spec;
 
   MaskDesc(int kind, int bias_dtype, std::optional<Tensor> t, std::array<int64_t, 4> strides, std::optional<Tensor> live,
-           std::optional<Tensor> live_t, std::optional<Tensor> bits_, std::optional<Tensor> bits_t_, py::object spec_)
+           std::optional<Tensor> live_t, py::object spec_)
       : spec(new py::object(std::move(spec_)), [](py::object* o) {
           py::gil_scoped_acquire gil;
           delete o;
@@ -67,8 +67,6 @@ struct MaskDesc {
     if (t) tensor = *t;
     if (live) tile_live = *live;
     if (live_t) tile_live_t = *live_t;
-    if (bits_) bits = *bits_;
-    if (bits_t_) bits_t = *bits_t_;
     if (kind == JVPFA_MASK_KVLEN)
       c.kv_len = static_cast<const int32_t*>(tensor.data_ptr());
     else if (kind == JVPFA_MASK_BOOL || kind == JVPFA_MASK_BIAS)
@@ -82,6 +80,19 @@ struct Call {
   MaskPtr mask;
   double scale;
   bool tf32;  // fp32 tensors: one TF32 product instead of three, recorded so that the backward recomputes what the forward saw
+  // The mask's entries in the form the 16-bit tensor-core kernels read best, made by this call for its forward and
+  // backward (prepare_mask): a boolean mask as bits, by rows and transposed, a ragged bias with its rows padded.
+  Tensor bits, bits_t, padded;
+
+  jvpfa_mask c_mask() const {
+    jvpfa_mask m = mask->c;
+    if (padded.defined()) {
+      m.ptr = padded.const_data_ptr();
+      for (int d = 0; d < 4; ++d) m.stride[d] = padded.size(d) == 1 ? 0 : padded.stride(d);
+    }
+    return m;
+  }
+  void drop_tensors() { bits = bits_t = padded = Tensor(); }
 };
 
 bool is_wrapped(const Tensor& x) {
@@ -217,9 +228,9 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   a.lse = static_cast<float*>(r.lse.data_ptr());
   a.to = dual ? r.to.data_ptr() : nullptr;
   a.mu = dual ? static_cast<float*>(r.mu.data_ptr()) : nullptr;
-  a.mask = call.mask->c;
+  a.mask = call.c_mask();
   a.mask_tile_live = data(call.mask->tile_live);
-  a.mask_bits = data(call.mask->bits);
+  a.mask_bits = data(call.bits);
   void* stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
   for (;;) {
     a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
@@ -232,6 +243,54 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     }
     check_status(rc, "jvpfa_fwd");
     return r;
+  }
+}
+
+// Fills in the call's forms of its mask.  They are made anew by every call and not kept with the mask's description: what
+// the kernels read is then what the mask holds when they run, also where it was written behind torch's version counter
+// (a replayed graph, a foreign kernel, `.data`).
+//
+// Packing reads the mask once (HBM bound) and saves a kernel that reads it one 16-byte piece per row and sub-tile.
+// B2 H12 L2048 D64, 100 MB of mask: packing 25 us; forward with tangents 168 -> 151 us, backward through tO 239 -> 186.
+// So it pays with a backward, for a mask that several heads share, and where the bytes' layout would send the call to
+// the register-tiled kernels.
+void prepare_mask(Call& call, const Tensor& q, bool backward) {
+  const MaskDesc& m = *call.mask;
+  if (!q.is_cuda() || q.scalar_type() == at::kFloat || g_impl == JVPFA_IMPL_GENERIC) return;
+  const int64_t L = q.size(2), esz = m.tensor.defined() ? m.tensor.element_size() : 0;
+  if (m.c.kind == JVPFA_MASK_BOOL) {
+    const int64_t n_b = m.c.stride[0] ? m.tensor.size(0) : 1, n_h = m.c.stride[1] ? m.tensor.size(1) : 1;
+    const int64_t n_rows = m.c.stride[2] ? L : 1;
+    bool pieces = m.c.stride[3] == 1 && (reinterpret_cast<uintptr_t>(m.c.ptr) & 15u) == 0 && L % 16 == 0;
+    for (int d = 0; d < 3; ++d) pieces = pieces && m.c.stride[d] % 16 == 0;
+    if (!backward && pieces && 4 * n_b * n_h > q.size(0) * q.size(1)) return;
+    c10::cuda::OptionalCUDAGuard guard;
+    if (q.get_device() != c10::cuda::current_device()) guard.set_index(q.get_device());
+    const int64_t w = (L + 63) / 64 * 2;
+    jvpfa_mask_tiles_args a{};
+    a.struct_size = sizeof(a);
+    a.n_b = (int)n_b, a.n_h = (int)n_h, a.n_rows = (int)n_rows, a.L = (int)L;
+    a.mask = m.c;
+    Tensor bits = empty({n_b * n_h * n_rows * w}, at::kInt, q.device()), bits_t;
+    a.bits = bits.data_ptr();
+    if (backward) {
+      bits_t = empty({n_b * n_h * L * (n_rows > 1 ? w : 1)}, at::kInt, q.device());
+      a.bits_t = bits_t.data_ptr();
+    }
+    const int rc = jvpfa_mask_tiles(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream());
+    if (rc == JVPFA_ERR_TOO_LARGE) return;  // the kernels read the bytes
+    check_status(rc, "jvpfa_mask_tiles");
+    call.bits = bits, call.bits_t = bits_t;
+  } else if (m.c.kind == JVPFA_MASK_BIAS && m.tensor.scalar_type() == q.scalar_type() && m.c.stride[2] != 0 && L > 64 && L * esz % 16 != 0) {
+    // rows padded to whole 16-byte pieces, the form in which those kernels take a bias (what lies beyond the row's end is
+    // not looked at); up to one tile of keys it is read element by element, whatever its layout
+    NoFunctorch nf;
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::cuda::OptionalCUDAGuard guard(q.device());
+    const int64_t step = 16 / esz;
+    const auto s = m.tensor.sizes();
+    call.padded = at::empty({s[0], s[1], s[2], (L + step - 1) / step * step}, m.tensor.options()).narrow(3, 0, L);
+    call.padded.copy_(m.tensor);
   }
 }
 
@@ -302,14 +361,14 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.flags = skip | (single ? JVPFA_DQ_ACCUM_IS_ZERO : 0);
   if (g[0].defined()) a.dq = g[0].data_ptr();
   if (g[1].defined()) a.dk = g[1].data_ptr(), a.dv = g[2].data_ptr();
-  a.mask = m.c;
+  a.mask = call.c_mask();
   if (m.tile_live.defined() && m.tile_live_t.defined() && a.L <= 8192) {
     a.mask_tile_live = data(m.tile_live);
     a.mask_tile_live_t = data(m.tile_live_t);
   }
   a.dq_accum = p.dq_accum;
-  a.mask_bits = data(m.bits);
-  a.mask_bits_t = data(m.bits_t);
+  a.mask_bits = data(call.bits);
+  a.mask_bits_t = data(call.bits_t);
   for (;;) {
     a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
     a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
@@ -389,6 +448,7 @@ struct AttnBwdNode : public Node {
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
     for (SavedVariable* s : {&q, &k, &v, &go}) s->reset_data();
+    call.drop_tensors();
   }
   std::string name() const override { return "JVPAttnBackwardBackward"; }
 };
@@ -462,6 +522,7 @@ struct AttnNode : public Node {
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
     for (SavedVariable* s : {&q, &k, &v, &tq, &tk, &tv, &o, &to, &lse, &mu}) s->reset_data();
+    call.drop_tensors();
   }
   std::string name() const override { return "JVPAttnBackward"; }
 };
@@ -506,9 +567,11 @@ std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tens
     tq = tangent(tq, q), tk = tangent(tk, q), tv = tangent(tv, q);
   }
   Call call{mask, scale ? *scale : 1.0 / std::sqrt((double)q.size(3)), tf32};
-  FwdResult r = launch_fwd(q, k, v, tq, tk, tv, call);
   const bool grad_primals = torch::autograd::compute_requires_grad(q, k, v);
-  if (grad_primals || torch::autograd::compute_requires_grad(tq, tk, tv)) {
+  const bool backward = grad_primals || torch::autograd::compute_requires_grad(tq, tk, tv);
+  prepare_mask(call, q, backward);
+  FwdResult r = launch_fwd(q, k, v, tq, tk, tv, call);
+  if (backward) {
     auto node = std::shared_ptr<AttnNode>(new AttnNode(), torch::autograd::deleteNode);
     node->call = call;
     node->dual = dual;
@@ -574,8 +637,7 @@ PYBIND11_MODULE(_native, m) {
       .def("__enter__", [](NoFunctorchScope& s) { s.guard.emplace(); })
       .def("__exit__", [](NoFunctorchScope& s, py::args) { s.guard.reset(); });
   py::class_<MaskDesc, MaskPtr>(m, "MaskDesc")
-      .def(py::init<int, int, std::optional<Tensor>, std::array<int64_t, 4>, std::optional<Tensor>, std::optional<Tensor>, std::optional<Tensor>,
-                    std::optional<Tensor>, py::object>());
+      .def(py::init<int, int, std::optional<Tensor>, std::array<int64_t, 4>, std::optional<Tensor>, std::optional<Tensor>, py::object>());
   m.def("attend", &attend);
   m.def("set_impl", [](int v) { g_impl = v; });
   m.def("set_single_pass", [](bool v) { g_single_pass = v; });

@@ -146,13 +146,13 @@ def classify_mask(attn_mask: Tensor | None, causal: bool, Z: int, H: int, N: int
     if attn_mask is None:
         return _lib.MaskSpec(_lib.MASK_NONE), 0, None
     if not MASK_MEMO_ENABLED:
-        return _classify_mask_tensor(attn_mask, Z, H, N, qdtype, verify)
+        return _classify_mask_tensor(attn_mask, Z, H, N, verify)
     key = (Z, H, N, verify, _unwrap(attn_mask)._version)
     hit = _MASK_MEMO.get(id(attn_mask))
     if hit is not None and hit[0]() is attn_mask and hit[1] == key:
         spec, mask_type = hit[2]
         return copy.copy(spec), mask_type, attn_mask  # a copy: the caller writes per-call state into the description
-    spec, mask_type, _ = _classify_mask_tensor(attn_mask, Z, H, N, qdtype, verify)
+    spec, mask_type, _ = _classify_mask_tensor(attn_mask, Z, H, N, verify)
     if len(_MASK_MEMO) >= _MASK_MEMO_MAX:
         _MASK_MEMO.clear()
     try:
@@ -166,15 +166,7 @@ def classify_mask(attn_mask: Tensor | None, causal: bool, Z: int, H: int, N: int
     return spec, mask_type, attn_mask
 
 
-def _padded_rows(m: Tensor, N: int) -> Tensor:
-    """``m`` with its rows padded to whole 16-byte pieces, the form in which the 16-bit tensor-core kernels read a mask
-    (what lies beyond the row's end is not looked at)."""
-    step = 16 // m.element_size()
-    out = torch.empty((*m.shape[:3], (N + step - 1) // step * step), device=m.device, dtype=m.dtype)[..., :N]
-    return out.copy_(m)
-
-
-def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, qdtype: torch.dtype, verify: bool):
+def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, verify: bool):
     """classify_mask for a mask tensor: shape checks, key-padding recognition, verification passes."""
     assert attn_mask.dim() == 4, "The provided attention mask must have 4 dimensions (Z, H, N_CTX, N_CTX)."
     mz, mh, mi, mj = attn_mask.shape
@@ -189,8 +181,6 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, qdtype: tor
     def bstrides(t: Tensor) -> tuple[int, int, int, int]:
         return tuple(0 if t.shape[d] == 1 else t.stride(d) for d in range(4))
 
-    # up to one tile of keys a bias is read element by element, whatever its layout
-    ragged = N > 64 and N * m.element_size() % 16 != 0 and qdtype in (torch.bfloat16, torch.float16)
     if m.dtype == torch.bool:
         if mh == 1 and mi == 1:
             # Candidate key-padding mask: valid keys form a prefix of each row.  Lengths, the prefix test and
@@ -208,9 +198,9 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, qdtype: tor
         spec = _lib.MaskSpec(_lib.MASK_BOOL, m8, bstrides(m8))
         every_head_live = True
         if verify:
-            # One pass answers upstream's check, packs the mask into bits and says which 128 x 64 tiles have a True at
-            # all; forward and backward step over the others.  (Without verification the mask is not looked at
-            # beforehand and is read byte by byte.)
+            # One pass answers upstream's check and says which 128 x 64 tiles have a True at all; forward and
+            # backward step over the others.  (Without verification the mask is not looked at beforehand, so
+            # there is no block skipping either: whether it would pay is known only from the pass's counts.)
             try:
                 spec.tile_live, head_live, spec.tile_live_t = _lib.mask_tiles(spec, N)
                 *heads, n_live = head_live.tolist()  # the one read-back
@@ -225,8 +215,6 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, qdtype: tor
 
     if m.dtype not in _lib.DTYPE_ENUM:
         m = m.to(torch.float32)
-    elif ragged and mi > 1 and m.dtype == qdtype:
-        m = _padded_rows(m, N)
     spec = _lib.MaskSpec(_lib.MASK_BIAS, m, bstrides(m), _lib.DTYPE_ENUM[m.dtype])
     if verify:
         # one pass and one read-back for upstream's isinf / isnan / "all MASK_CONST" sweeps (jvp_attention.py:2447-2457)

@@ -105,3 +105,41 @@ def test_gradients_nobody_asked_for_are_left_out(dt, D, want):
         else:
             assert (x.float() - full[n].float()).abs().max().item() <= 2e-2 * max(1.0, full[n].abs().max().item())
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("kind,L,D", [("bool", 128, 64), ("bool", 250, 64), ("bool", 192, 128), ("bias", 250, 64), ("bias", 250, 128)])
+@pytest.mark.parametrize("how", ["data", "graph"])
+def test_a_mask_written_behind_the_version_counter_is_read_as_it_is(kind, L, D, how):
+    """Neither a write through ``.data`` nor one between two replays of a graph moves the counter that the mask's
+    verification is remembered by; what the kernels read has to be the new entries all the same."""
+    q, k, v, tq, tk, tv, _, _ = (x.to(DEV) for x in _inputs(2, 3, L, D, torch.bfloat16, 6))
+    first, second = (_mask(kind, 2, 3, L, torch.bfloat16, s).to(DEV) for s in (1, 2))
+    a = [x.clone().requires_grad_() for x in (q, k, v)]
+
+    def run(m):
+        o, to = torch.func.jvp(lambda x, y, z: ja.JVPAttn.fwd_dual(x, y, z, attn_mask=m), tuple(a), (tq, tk, tv))
+        return (o, to, *torch.autograd.grad((o, to), a, (q, v)))
+
+    want = [x.detach().clone() for x in run(second.clone())]
+    mask = first.clone()
+    if how == "data":
+        run(mask)
+        mask.data.copy_(second)
+        got = run(mask)
+    else:
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            run(mask)
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = run(mask)
+        mask.copy_(second)
+        graph.replay()
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    for x, y in zip(got[:2], want[:2]):
+        assert torch.equal(x, y)
+    for x, y in zip(got[2:], want[2:]):  # dQ may be summed by reductions: the order of two runs differs
+        assert (x.float() - y.float()).abs().max().item() <= 2e-2 * max(1.0, y.abs().max().item())
