@@ -47,7 +47,7 @@ typedef enum {
 typedef enum {
   JVPFA_BF16 = 0,
   JVPFA_FP16 = 1,
-  JVPFA_FP32 = 2,      /* fp32 tensors; every product as three TF32 MMAs on a hi/lo split (error ~1e-6 relative) */
+  JVPFA_FP32 = 2,      /* fp32 tensors; every product as three MMAs on a hi/lo split of 22 bits (error ~1e-6 relative) */
   JVPFA_FP32_TF32 = 3  /* fp32 tensors; every product as one TF32 MMA, the precision of upstream's fp32 path
                           (tl.dot on TF32 tensor cores, jvp_attention.py:233-236); error ~5e-4 relative, about
                           2.5x faster.  Not a bias dtype: an fp32 bias is JVPFA_FP32. */

@@ -130,7 +130,7 @@ int launch_pre(const jvpfa_pre_args& a, cudaStream_t s) {
 // Main kernels.  A CTA of RG x KG warps owns 16*RG rows (keys for dK / dV, queries for dQ) and loops over tiles of the
 // other side; warp (rg, kg) owns 16 of the rows and the kg-th part of every loop tile, sums its own dK, dV or dQ, and the
 // KG partial sums are added once at the end (a fixed order: results stay reproducible bit for bit).  As in the forward
-// (fwd_generic.cu) the bound is mma.sync, three instructions for an fp32 product, and the split puts two warps on each
+// (fwd_generic.cu) the bound is mma.sync, and the split puts two warps on each
 // quarter of an SM that shared memory would otherwise leave with one, and lets small shapes use more SMs.
 //
 // All score products of a tile are formed in two sweeps over D, {S, tS} and {E, F + dP}, so that an operand fragment is
@@ -184,23 +184,20 @@ __device__ __forceinline__ void gemm_pair(float (*x)[4], float (*y)[4], const T*
       load_b_nt<T>(b0[nt], sB0, ld, nt * 8, k0, lane);
       if constexpr (HAS_Y2) load_b_nt<T>(b1[nt], sB1, ld, nt * 8, k0, lane);
     }
-    auto pass = [&](auto P) {
 #pragma unroll
-      for (int nt = 0; nt < NT_; ++nt) {
-        mma_pass<P()>(x[nt], a0, b0[nt]);
-        if constexpr (HAS_Y1) mma_pass<P()>(y[nt], a1, b0[nt]);
-      }
-      if constexpr (HAS_Y2) {
+    for (int nt = 0; nt < NT_; ++nt) {
+      mma<T>(x[nt], a0, b0[nt]);
+      if constexpr (HAS_Y1) mma<T>(y[nt], a1, b0[nt]);
+    }
+    if constexpr (HAS_Y2) {
 #pragma unroll
-        for (int nt = 0; nt < NT_; ++nt) mma_pass<P()>(y[nt], a0, b1[nt]);
-      }
-    };
-    pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
+      for (int nt = 0; nt < NT_; ++nt) mma<T>(y[nt], a0, b1[nt]);
+    }
   }
 }
 
 // out[D/8][4] += A0 B0 (+ A1 B1): A from accumulator tiles (16 x KROWS), B = [k][d] tiles, d contiguous.
-// fp32: the tensor core adds into its fp32 accumulator with truncation, and hundreds of such adds into one long-lived
+// TF32: the tensor core adds into its fp32 accumulator with truncation, and hundreds of such adds into one long-lived
 // accumulator show up as a bias of ~1e-5.  Each contraction step is therefore formed in fresh registers and added rounded.
 template <typename T, int D, int KROWS, bool HAS_0, bool HAS_1>
 __device__ __forceinline__ void gemm_out(float (*out)[4], const float (*at0)[4], const float (*at1)[4], const T* sB0, const T* sB1,
@@ -223,17 +220,14 @@ __device__ __forceinline__ void gemm_out(float (*out)[4], const float (*at0)[4],
 #pragma unroll
         for (int e = 0; e < 4; ++e) tmp[i][e] = Elem<T>::k16 ? out[d0 + i][e] : 0.f;
       }
-      auto pass = [&](auto P) {
-        if constexpr (HAS_0) {
+      if constexpr (HAS_0) {
 #pragma unroll
-          for (int i = 0; i < G; ++i) mma_pass<P()>(tmp[i], a0, b0[i]);
-        }
-        if constexpr (HAS_1) {
+        for (int i = 0; i < G; ++i) mma<T>(tmp[i], a0, b0[i]);
+      }
+      if constexpr (HAS_1) {
 #pragma unroll
-          for (int i = 0; i < G; ++i) mma_pass<P()>(tmp[i], a1, b1[i]);
-        }
-      };
-      pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
+        for (int i = 0; i < G; ++i) mma<T>(tmp[i], a1, b1[i]);
+      }
 #pragma unroll
       for (int i = 0; i < G; ++i) {
 #pragma unroll
@@ -674,7 +668,7 @@ int launch_bwd_generic(const jvpfa_bwd_args& a, cudaStream_t s) {
     case JVPFA_FP16:
       return launch_bwd_t<__half>(a, s);
     case JVPFA_FP32:
-      return launch_bwd_t<float>(a, s);
+      return launch_bwd_fp32(a, s);
     case JVPFA_FP32_TF32:
       return launch_bwd_t<tf32x1>(a, s);
     default:

@@ -13,11 +13,13 @@
 // is applied as scale*QK^T + bias (SDPA semantics; upstream scales the bias too,
 // jvp_attention.py:247-251), and boolean masking uses -inf rather than adding -100.
 //
-// What bounds it: mma.sync, at 512 (TF32) or 1024 (16-bit) multiply-adds per clock and SM, measured; an fp32 product is
-// three TF32 instructions.  One instruction occupies its quarter of the SM for 8 cycles and returns after 21, and the
-// fp32 products of one accumulator are a chain, so the split matters: 64 rows x D=128 fp32 fill the shared memory of an
-// SM, and with one warp for each 16 rows (KG = 1) a quarter had a single warp to wait for.  With KG = 2 it has two, and
-// shapes with few row tiles use shorter ones with more key parts (see launch_d) instead of leaving SMs idle.
+// It serves what the tcgen05 kernels do not take (16-bit: short or oddly laid out requests) and fp32 inputs multiplied in
+// one TF32 pass (JVPFA_FP32_TF32); fp32 at full precision: fwd_fp32.cu.
+// What bounds it: mma.sync, at 512 (TF32) or 1024 (16-bit) multiply-adds per clock and SM, measured.  One instruction
+// occupies its quarter of the SM for 8 cycles and returns after 21, so the split matters: 64 rows x D=128 of 4-byte
+// elements fill the shared memory of an SM, and with one warp for each 16 rows (KG = 1) a quarter had a single warp to wait
+// for.  With KG = 2 it has two, and shapes with few row tiles use shorter ones with more key parts (see launch_d) instead
+// of leaving SMs idle.
 #include "common.cuh"
 
 namespace jvpfa {
@@ -178,18 +180,15 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
         load_b_nt<T>(fk[nt], sK, LD, nt * 8, k0, lane);
         if constexpr (DUAL) load_b_nt<T>(ftk[nt], sTK, LD, nt * 8, k0, lane);
       }
-      auto pass = [&](auto P) {
 #pragma unroll
-        for (int nt = 0; nt < NS; ++nt) {
-          mma_pass<P()>(s[nt], fq, fk[nt]);
-          if constexpr (DUAL) mma_pass<P()>(ts[nt], ftq, fk[nt]);
-        }
-        if constexpr (DUAL) {
+      for (int nt = 0; nt < NS; ++nt) {
+        mma<T>(s[nt], fq, fk[nt]);
+        if constexpr (DUAL) mma<T>(ts[nt], ftq, fk[nt]);
+      }
+      if constexpr (DUAL) {
 #pragma unroll
-          for (int nt = 0; nt < NS; ++nt) mma_pass<P()>(ts[nt], fq, ftk[nt]);
-        }
-      };
-      pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
+        for (int nt = 0; nt < NS; ++nt) mma<T>(ts[nt], fq, ftk[nt]);
+      }
     }
 
     // ---- mask / bias, move to the base-2 domain ----
@@ -259,7 +258,7 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
     }
 
     // ---- second MMAs: contraction over the keys of this tile ----
-    // fp32: the tensor core adds into its fp32 accumulator with truncation; over a thousand keys that bias reaches
+    // TF32: the tensor core adds into its fp32 accumulator with truncation; over a thousand keys that bias reaches
     // ~1e-5.  Each contraction step is therefore formed in fresh registers and added to the running sums rounded.
 #pragma unroll
     for (int kk = 0; kk < BW / KS; ++kk) {
@@ -281,18 +280,15 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
             if constexpr (DUAL) xt[i][e] = Elem<T>::k16 ? acc_t[d0 + i][e] : 0.f;
           }
         }
-        auto pass = [&](auto P) {
 #pragma unroll
-          for (int i = 0; i < G; ++i) {
-            mma_pass<P()>(xo[i], fp, fv[i]);
-            if constexpr (DUAL) mma_pass<P()>(xt[i], fw, fv[i]);
-          }
-          if constexpr (DUAL) {
+        for (int i = 0; i < G; ++i) {
+          mma<T>(xo[i], fp, fv[i]);
+          if constexpr (DUAL) mma<T>(xt[i], fw, fv[i]);
+        }
+        if constexpr (DUAL) {
 #pragma unroll
-            for (int i = 0; i < G; ++i) mma_pass<P()>(xt[i], fp, ftv[i]);
-          }
-        };
-        pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
+          for (int i = 0; i < G; ++i) mma<T>(xt[i], fp, ftv[i]);
+        }
 #pragma unroll
         for (int i = 0; i < G; ++i) {
 #pragma unroll
@@ -456,7 +452,7 @@ int launch_fwd_generic(const jvpfa_fwd_args& a, cudaStream_t s) {
     case JVPFA_FP16:
       return launch_t<__half>(a, s);
     case JVPFA_FP32:
-      return launch_t<float>(a, s);
+      return launch_fwd_fp32(a, s);
     case JVPFA_FP32_TF32:
       return launch_t<tf32x1>(a, s);
     default:

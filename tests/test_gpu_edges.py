@@ -143,3 +143,36 @@ def test_a_mask_written_behind_the_version_counter_is_read_as_it_is(kind, L, D, 
         assert torch.equal(x, y)
     for x, y in zip(got[2:], want[2:]):  # dQ may be summed by reductions: the order of two runs differs
         assert (x.float() - y.float()).abs().max().item() <= 2e-2 * max(1.0, y.abs().max().item())
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("B,H,L", [(1, 2, 34), (2, 10, 250), (2, 12, 450)])
+def test_fp32_rows_of_very_different_magnitude(B, H, L, D):
+    """A pair of fp16 numbers carries 22 bits of an entry relative to its own row only: rows of V and its tangent up to a
+    factor of 2^40 apart, and masked-out keys that hold 1e15, must cost no precision.  Every product is within 2^-21 of its
+    operands' magnitudes; a gradient passes three in a row and sums a few hundred terms: 1e-5 of P |V| for O, of the head's
+    largest V for tO, of the head's largest entry for a gradient."""
+    q, k, v, tq, tk, tv, go, gt = _inputs(B, H, L, D, torch.float32, L + D)
+    g = torch.Generator().manual_seed(L)
+    vscale = torch.exp2(torch.randint(-20, 21, (B, H, L, 1), generator=g).float())
+    v, tv = v * vscale, tv * vscale
+    dead = torch.rand(B, 1, L, 1, generator=g) > 0.8
+    dead[:, :, 0] = False
+    mask = (torch.rand(B, 1, L, L, generator=g) > 0.3) & ~dead.transpose(2, 3)
+    mask[..., 0] = True
+    clean = [x.masked_fill(dead, 0.0) for x in (k, v, tk, tv)]
+    ref = orc.grads_through_both(q, clean[0], clean[1], tq, clean[2], clean[3], go, gt, attn_mask=mask)
+    k, v, tk, tv = (x.masked_fill(dead, 1e15) for x in (k, v, tk, tv))
+    a = [x.to(DEV).requires_grad_() for x in (q, k, v)]
+    m = mask.to(DEV)
+    o, to = torch.func.jvp(lambda x, y, z: ja.JVPAttn.fwd_dual(x, y, z, attn_mask=m), tuple(a), tuple(x.to(DEV) for x in (tq, tk, tv)))
+    got = (o, to, *torch.autograd.grad((o, to), a, (go.to(DEV), gt.to(DEV))))
+    head = lambda x: x.double().abs().amax(dim=(2, 3), keepdim=True)  # noqa: E731
+    scores = (q.double() @ clean[0].double().transpose(-1, -2) * D**-0.5).masked_fill(~mask, float("-inf"))
+    weight = torch.softmax(scores, -1) @ clean[1].double().abs()
+    for name, x, r in zip(("O", "tO", "dq", "dk", "dv"), got, ref):
+        x = x.detach().cpu().double()
+        assert torch.isfinite(x).all(), name
+        top = weight if name == "O" else head(clean[1]) if name == "tO" else head(r)
+        off = ((x - r.double()).abs() / top.clamp(min=1e-30)).max().item()
+        assert off <= 1e-5, (name, off)
