@@ -99,104 +99,149 @@ __global__ void __launch_bounds__(kCheckThreads) mask_check_kernel(const jvpfa_m
 // one bit per entry, by rows and transposed.  The attention kernels then read 8 bytes of a mask row per 64-key tile
 // instead of 64, and where a thread owns a key one word instead of 32 single bytes, each from another row.
 //
-// HBM bound (1 byte read and 1/4 byte written per entry).  A warp takes 32 rows x 512 keys: lane l reads bytes
-// [16 l, 16 l + 16) of each row, keeps them as 16 bits, and builds its 16 transposed words bit by bit on the way; the
-// CTA's eight warps (256 rows) pass those through shared memory so that they leave as 32-byte pieces.
+// HBM bound (1 byte read and 1/4 byte written per entry), if enough of it is in flight: a warp takes 32 rows x 256 keys and
+// a lane asks for its 8 bytes of all 32 rows at once.  Four lanes put a row's word together; eight rows at a time are
+// transposed as 8 x 8 bits, and the CTA's eight warps (256 rows) pass the transposed words through shared memory so that
+// they leave as 32-byte pieces.  B2 H12 L2048 (100 MB) 32 us, one head of L4096 (17 MB) 8
+// us; 16 bytes of up to eight rows at a time and a transposition bit by bit took 60 and 25 us.
 // With the packed mask, B2 H12 L2048 D64 and nine tenths random False: forward with tangents 168 -> 151 us, backward
 // through tO 239 -> 186 us.
-constexpr int kPackRows = 256, kPackKeys = 512;
+constexpr int kPackRows = 256, kPackKeys = 256;
 
 __device__ __forceinline__ uint32_t nonzero_bits(uint32_t w) {  // bytes -> four bits
-  return (((__vcmpne4(w, 0u) & 0x01010101u) * 0x01020408u) >> 24) & 0xfu;
+  const uint32_t top = (((w & 0x7f7f7f7fu) + 0x7f7f7f7fu) | w) & 0x80808080u;
+  return (top * 0x00204081u) >> 28;  // bits 7, 15, 23, 31 -> 28 .. 31
+}
+
+// 8 x 8 bits, byte r of (lo, hi) = row r, transposed in place (H. S. Warren, "Hacker's Delight", 7-3).
+__device__ __forceinline__ void transpose8(uint32_t& lo, uint32_t& hi) {
+  uint32_t t = (lo ^ (lo >> 7)) & 0x00aa00aau;
+  lo ^= t ^ (t << 7);
+  t = (hi ^ (hi >> 7)) & 0x00aa00aau;
+  hi ^= t ^ (t << 7);
+  t = (lo ^ (lo >> 14)) & 0x0000ccccu;
+  lo ^= t ^ (t << 14);
+  t = (hi ^ (hi >> 14)) & 0x0000ccccu;
+  hi ^= t ^ (t << 14);
+  t = (lo ^ (hi << 4)) & 0xf0f0f0f0u;
+  lo ^= t;
+  hi ^= t >> 4;
+}
+
+// Bytes j of a, b, c, d -> word j.
+__device__ __forceinline__ void transpose_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t* w) {
+  const uint32_t ab = __byte_perm(a, b, 0x5140), cd = __byte_perm(c, d, 0x5140);  // a0 b0 a1 b1
+  const uint32_t ab2 = __byte_perm(a, b, 0x7362), cd2 = __byte_perm(c, d, 0x7362);
+  w[0] = __byte_perm(ab, cd, 0x5410), w[1] = __byte_perm(ab, cd, 0x7632);
+  w[2] = __byte_perm(ab2, cd2, 0x5410), w[3] = __byte_perm(ab2, cd2, 0x7632);
 }
 
 __global__ void __launch_bounds__(256) mask_pack_kernel(const jvpfa_mask m, int n_h, int n_rows, int L, int n_qt, int n_words,
                                                         unsigned char* tile_live, int32_t* head_live,
                                                         unsigned long long* tile_live_t, int n_kt128, int n_words_t,
                                                         uint32_t* bits, uint32_t* bits_t) {
-  __shared__ unsigned int s_tiles[2];                       // of the CTA's two 128-row tiles
-  __shared__ uint32_t s_t[kPackKeys * 8 + kPackKeys / 16];  // [key][warp], one word of padding per 16 keys
-  const int head = blockIdx.z, kg = blockIdx.x;             // kg: group of eight key tiles
+  __shared__ unsigned int s_tiles[2];                      // of the CTA's two 128-row tiles
+  __shared__ uint32_t s_t[kPackKeys * 8 + kPackKeys / 8];  // [key][warp], one word of padding per 8 keys
+  const int head = blockIdx.z, kg = blockIdx.x;            // kg: group of four key tiles
   const int b = head / n_h, h = head - b * n_h;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned char* base = reinterpret_cast<const unsigned char*>(m.ptr) + (long long)b * m.stride[0] + (long long)h * m.stride[1];
   const long long rs = m.stride[2], ks = m.stride[3];
   if (threadIdx.x < 2) s_tiles[threadIdx.x] = 0u;
-  const int col = kg * kPackKeys + lane * 16;
+  const int col = kg * kPackKeys + lane * 8;
   const int row0 = blockIdx.y * kPackRows + warp * 32;
-  const bool vec = ks == 1 && (rs & 15) == 0 && (reinterpret_cast<uintptr_t>(base) & 15u) == 0 && col + 16 <= L;
-  const int w_rows = ((L + 63) / 64) * 2;  // words of a row
-  uint32_t t[16];
+  const bool vec = ks == 1 && (rs & 7) == 0 && (reinterpret_cast<uintptr_t>(base) & 7u) == 0 && col + 8 <= L;
+  const unsigned char* p0 = base + (long long)row0 * rs + (long long)col * ks;
+  uint32_t x[8];  // byte i of x[j]: row 4j + i, a bit per column
+  if (vec) {
+    uint2 v[32];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) t[j] = 0u;
-  uint32_t any = 0u;
-#pragma unroll 8
-  for (int r = 31; r >= 0; --r) {  // downwards: the first row ends up in bit 0
-    const int row = row0 + r;
-    uint32_t x = 0u;
-    if (row < n_rows && col < L) {
-      const unsigned char* p = base + (long long)row * rs + (long long)col * ks;
-      if (vec) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
-        x = nonzero_bits(v.x) | nonzero_bits(v.y) << 4 | nonzero_bits(v.z) << 8 | nonzero_bits(v.w) << 12;
-      } else {
-        const int n = min(16, L - col);
-        for (int j = 0; j < n; ++j) x |= (p[j * ks] != 0 ? 1u : 0u) << j;
+    for (int r = 0; r < 32; ++r) {
+      v[r] = make_uint2(0u, 0u);
+      if (row0 + r < n_rows) v[r] = __ldg(reinterpret_cast<const uint2*>(p0 + (long long)r * rs));
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      x[j] = 0u;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[j] |= (nonzero_bits(v[4 * j + i].x) | nonzero_bits(v[4 * j + i].y) << 4) << (8 * i);
+    }
+  } else {
+    const int n = min(8, L - col);  // <= 0: beyond the end
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      x[j] = 0u;
+      for (int i = 0; i < 4; ++i) {
+        const unsigned char* p = p0 + (long long)(4 * j + i) * rs;
+        if (row0 + 4 * j + i < n_rows)
+          for (int c = 0; c < n; ++c) x[j] |= (p[c * ks] != 0 ? 1u : 0u) << (8 * i + c);
       }
     }
-    any |= x;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) t[j] = (t[j] << 1) | ((x >> j) & 1u);
-    const uint32_t other = __shfl_xor_sync(0xffffffffu, x, 1);
-    const int word = kg * (kPackKeys / 32) + (lane >> 1);
-    if (bits != nullptr && (lane & 1) == 0 && row < n_rows && word < w_rows)
-      bits[((long long)head * n_rows + row) * w_rows + word] = x | other << 16;
   }
+  uint32_t any = 0u;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) any |= x[j];
   const unsigned int vote = __ballot_sync(0xffffffffu, any != 0u);  // bit l: lane l saw a true entry
+  if (bits != nullptr) {  // of four rows, lane l of four neighbours puts row l together: a 4 x 4 transpose of bytes across lanes
+    const int w_rows = ((L + 63) / 64) * 2, word = kg * (kPackKeys / 32) + (lane >> 2);
+    const uint32_t sel1 = lane & 1 ? 0x3715u : 0x6240u, sel2 = lane & 2 ? 0x3276u : 0x5410u;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      uint32_t y = __byte_perm(x[j], __shfl_xor_sync(0xffffffffu, x[j], 1), sel1);
+      y = __byte_perm(y, __shfl_xor_sync(0xffffffffu, y, 2), sel2);
+      const int row = row0 + 4 * j + (lane & 3);
+      if (row < n_rows && word < w_rows) bits[((long long)head * n_rows + row) * w_rows + word] = y;
+    }
+  }
   __syncthreads();
   if (lane == 0 && vote != 0u) {
     unsigned int tiles = 0u;
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (vote & (0xfu << (4 * k))) tiles |= 1u << k;
+    for (int k = 0; k < 4; ++k)
+      if (vote & (0xffu << (8 * k))) tiles |= 1u << k;
     atomicOr(&s_tiles[warp >> 2], tiles);
   }
   if (bits_t != nullptr) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) s_t[(lane * 16 + j) * 8 + warp + lane] = t[j];
+    for (int q = 0; q < 4; ++q) transpose8(x[2 * q], x[2 * q + 1]);  // byte c: column c (the second word: 4 + c) of eight rows
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      uint32_t t[4];  // columns 4i .. 4i+3, a bit per row
+      transpose_bytes(x[i], x[2 + i], x[4 + i], x[6 + i], t);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s_t[(lane * 8 + 4 * i + j) * 8 + warp + lane] = t[j];
+    }
   }
   __syncthreads();
   if (threadIdx.x < 2 && s_tiles[threadIdx.x] != 0u && tile_live != nullptr) {
     const unsigned int tiles = s_tiles[threadIdx.x];
     const int qt = blockIdx.y * 2 + threadIdx.x;
-    // byte kg of the entry's words (little endian: byte k of a word holds its bits 8k .. 8k+7)
-    tile_live[((long long)head * n_qt + qt) * n_words * 8 + kg] = (unsigned char)tiles;
+    // tiles 4 kg .. 4 kg + 3 of the entry's words
+    atomicOr(reinterpret_cast<unsigned int*>(tile_live) + ((long long)head * n_qt + qt) * n_words * 2 + (kg >> 3), tiles << (4 * (kg & 7)));
     if (head_live) {
       head_live[head] = 1;
       atomicAdd(head_live + gridDim.z, __popc(tiles));  // live tiles of the whole mask
     }
     if (tile_live_t) {  // the transposed summary: per 128-key tile, one bit per 128-query tile
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < 2; ++j)
         if ((tiles >> (2 * j)) & 3u)
-          atomicOr(tile_live_t + ((long long)head * n_kt128 + 4 * kg + j) * n_words_t + (qt >> 6), 1ull << (qt & 63));
+          atomicOr(tile_live_t + ((long long)head * n_kt128 + 2 * kg + j) * n_words_t + (qt >> 6), 1ull << (qt & 63));
     }
   }
   if (bits_t != nullptr) {
-    for (int k = threadIdx.x; k < kPackKeys; k += 256) {
-      const int key = kg * kPackKeys + k;
-      if (key >= L) break;
-      const uint32_t* src = s_t + k * 8 + (k >> 4);
-      if (n_rows == 1) {  // one row for every query: all bits of the key's only word alike
-        bits_t[(long long)head * L + key] = (src[0] & 1u) ? ~0u : 0u;
-        continue;
-      }
-      const int w_cols = ((n_rows + 63) / 64) * 2, w0 = blockIdx.y * (kPackRows / 32);
-      uint2* dst = reinterpret_cast<uint2*>(bits_t + ((long long)head * L + key) * w_cols + w0);
-#pragma unroll
-      for (int w = 0; w < 4; ++w)
-        if (w0 + 2 * w < w_cols) dst[w] = make_uint2(src[2 * w], src[2 * w + 1]);
+    const int k = threadIdx.x, key = kg * kPackKeys + k;
+    if (key >= L) return;
+    const uint32_t* src = s_t + k * 8 + (k >> 3);
+    if (n_rows == 1) {  // one row for every query: all bits of the key's only word alike
+      bits_t[(long long)head * L + key] = (src[0] & 1u) ? ~0u : 0u;
+      return;
     }
+    const int w_cols = ((n_rows + 63) / 64) * 2, w0 = blockIdx.y * (kPackRows / 32);
+    uint2* dst = reinterpret_cast<uint2*>(bits_t + ((long long)head * L + key) * w_cols + w0);
+#pragma unroll
+    for (int w = 0; w < 4; ++w)
+      if (w0 + 2 * w < w_cols) dst[w] = make_uint2(src[2 * w], src[2 * w + 1]);
   }
 }
 
@@ -206,7 +251,7 @@ int launch_mask_tiles(const jvpfa_mask_tiles_args& a, cudaStream_t stream) {
   const int n_kt = (a.L + 63) / 64;
   const int n_words = (n_kt + 63) / 64;
   const int n_qt = a.n_rows == 1 ? 1 : (a.L + 127) / 128;
-  const dim3 grid((unsigned)((n_kt + 7) / 8), (unsigned)((a.n_rows + kPackRows - 1) / kPackRows), (unsigned)(a.n_b * a.n_h));
+  const dim3 grid((unsigned)((n_kt + 3) / 4), (unsigned)((a.n_rows + kPackRows - 1) / kPackRows), (unsigned)(a.n_b * a.n_h));
   const int n_kt128 = (a.L + 127) / 128;
   const int n_words_t = (n_qt + 63) / 64;
   mask_pack_kernel<<<grid, 256, 0, stream>>>(a.mask, a.n_h, a.n_rows, a.L, n_qt, n_words,
