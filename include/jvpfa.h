@@ -121,6 +121,8 @@ typedef struct {
   /* Optional, JVPFA_MASK_BOOL only: `bits` of jvpfa_mask_tiles.  The tcgen05 kernels read it instead of the bytes, whose
    * layout then does not matter to them.  A caller built without this field (struct_size up to mask_tile_live): NULL. */
   const void* mask_bits;
+  /* 0 or JVPFA_ZERO_TKV.  (struct_size up to mask_tile_live: 0.) */
+  int32_t flags;
 } jvpfa_fwd_args;
 
 int jvpfa_fwd(const jvpfa_fwd_args* args, void* stream);
@@ -203,6 +205,9 @@ typedef struct {
 #define JVPFA_SKIP_DQ 1
 #define JVPFA_SKIP_DKDV 2
 #define JVPFA_DQ_ACCUM_IS_ZERO 4
+/* K and V have no tangents (they count as zero): tk and tv are NULL, tq is given.  JVPFA_FP32 only, in the backward only
+ * for a cotangent of tO alone; anything else answers JVPFA_ERR_UNSUPPORTED. */
+#define JVPFA_ZERO_TKV 8
 
 int jvpfa_bwd(const jvpfa_bwd_args* args, void* stream);
 

@@ -89,6 +89,7 @@ class FwdArgs(C.Structure):
         ("in_stride", C.c_int64 * 3),
         ("mask_tile_live", C.c_void_p),
         ("mask_bits", C.c_void_p),
+        ("flags", C.c_int32),
     ]
 
 

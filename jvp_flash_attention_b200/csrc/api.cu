@@ -98,7 +98,9 @@ static int validate_fwd(const jvpfa_fwd_args* a) {
   if (!a->q || !a->k || !a->v || !a->o || !a->lse) return JVPFA_ERR_NULL;
   const int nt = (a->tq != nullptr) + (a->tk != nullptr) + (a->tv != nullptr) + (a->to != nullptr) +
                  (a->mu != nullptr);
-  if (nt != 0 && nt != 5) return JVPFA_ERR_NULL;
+  const bool zero_tkv = (a->flags & JVPFA_ZERO_TKV) != 0;
+  if ((a->flags & ~JVPFA_ZERO_TKV) != 0 || (zero_tkv && a->dtype != JVPFA_FP32)) return JVPFA_ERR_UNSUPPORTED;
+  if (zero_tkv ? (nt != 3 || a->tk || a->tv) : (nt != 0 && nt != 5)) return JVPFA_ERR_NULL;
   const void* ptrs[] = {a->q, a->k, a->v, a->tq, a->tk, a->tv, a->o, a->to};
   for (const void* p : ptrs)
     if (p && !aligned16(p)) return JVPFA_ERR_ALIGN;
@@ -116,12 +118,15 @@ static int validate_bwd(const jvpfa_bwd_args* a) {
   int rc = check_shape(a->dtype, a->B, a->H, a->L, a->D);
   if (rc) return rc;
   constexpr int kSkip = JVPFA_SKIP_DQ | JVPFA_SKIP_DKDV;
-  if ((a->flags & ~(kSkip | JVPFA_DQ_ACCUM_IS_ZERO)) != 0 || (a->flags & kSkip) == kSkip) return JVPFA_ERR_UNSUPPORTED;
+  if ((a->flags & ~(kSkip | JVPFA_DQ_ACCUM_IS_ZERO | JVPFA_ZERO_TKV)) != 0 || (a->flags & kSkip) == kSkip) return JVPFA_ERR_UNSUPPORTED;
+  const bool zero_tkv = (a->flags & JVPFA_ZERO_TKV) != 0;
+  if (zero_tkv && (a->dtype != JVPFA_FP32 || a->go || !a->gto)) return JVPFA_ERR_UNSUPPORTED;
   if (!a->q || !a->k || !a->v || !a->lse || !a->delta) return JVPFA_ERR_NULL;
   if (!(a->flags & JVPFA_SKIP_DQ) && !a->dq) return JVPFA_ERR_NULL;
   if (!(a->flags & JVPFA_SKIP_DKDV) && (!a->dk || !a->dv)) return JVPFA_ERR_NULL;
   if (!a->go && !a->gto) return JVPFA_ERR_NULL;
-  if (a->gto && (!a->tq || !a->tk || !a->tv || !a->mu || !a->eps || !a->cterm)) return JVPFA_ERR_NULL;
+  if (a->gto && (!a->tq || !a->mu || !a->eps || !a->cterm)) return JVPFA_ERR_NULL;
+  if (a->gto && (zero_tkv ? (a->tk || a->tv) : (!a->tk || !a->tv))) return JVPFA_ERR_NULL;
   const void* ptrs[] = {a->q, a->k, a->v, a->tq, a->tk, a->tv, a->go, a->gto, a->dq, a->dk, a->dv};
   for (const void* p : ptrs)
     if (p && !aligned16(p)) return JVPFA_ERR_ALIGN;

@@ -45,16 +45,17 @@ struct HeadView {  // where this CTA's head lies
   __device__ const float* dense(const void* p) const { return reinterpret_cast<const float*>(p) + off; }
 };
 
+// TKV: K and V have tangents (JVPFA_ZERO_TKV leaves out what they would be multiplied by).
 // ---- dK, dV.  Tiles are held transposed (rows = keys, columns = queries), so that P^T etc. feed the second products from
 // registers. ----
-template <int D, bool HAS_GO, bool HAS_GT, int RG, int KG>
-using DkdvCfg = BwdCfg<D, HAS_GT ? 4 : 2, 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0), RG, KG, true, RG == 4 && D <= 64 ? 2 : 1>;
+template <int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
+using DkdvCfg = BwdCfg<D, TKV ? 4 : 2, 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0), RG, KG, true, RG == 4 && D <= 64 ? 2 : 1>;
 
-template <int D, bool HAS_GO, bool HAS_GT, int RG, int KG>
-__global__ void __launch_bounds__(32 * RG * KG, DkdvCfg<D, HAS_GO, HAS_GT, RG, KG>::kResident) bwd_dkdv_fp32_kernel(const jvpfa_bwd_args a) {
-  using C = DkdvCfg<D, HAS_GO, HAS_GT, RG, KG>;
+template <int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
+__global__ void __launch_bounds__(32 * RG * KG, DkdvCfg<D, HAS_GO, HAS_GT, TKV, RG, KG>::kResident) bwd_dkdv_fp32_kernel(const jvpfa_bwd_args a) {
+  using C = DkdvCfg<D, HAS_GO, HAS_GT, TKV, RG, KG>;
   constexpr int BN = C::OWN, BM = C::LOOP, NT = C::NT, STAGES = C::STAGES, ND = D / 8;
-  constexpr int OWN_TILES = HAS_GT ? 4 : 2, LOOP_TILES = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0);
+  constexpr int OWN_TILES = TKV ? 4 : 2, LOOP_TILES = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0);
   constexpr int kGO = 1, kTQ = 1 + (HAS_GO ? 1 : 0), kG = kTQ + 1;  // loop tiles after Q
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -109,7 +110,7 @@ __global__ void __launch_bounds__(32 * RG * KG, DkdvCfg<D, HAS_GO, HAS_GT, RG, K
 
   copy_tile<BN, D, NT>(sOwn, hv.in(a.k), n0, L, tid, hv.in_rs);
   copy_tile<BN, D, NT>(sOwn + C::kOwn, hv.in(a.v), n0, L, tid, hv.in_rs);
-  if constexpr (HAS_GT) {
+  if constexpr (TKV) {
     copy_tile<BN, D, NT>(sOwn + 2 * C::kOwn, hv.in(a.tk), n0, L, tid, hv.in_rs);
     copy_tile<BN, D, NT>(sOwn + 3 * C::kOwn, hv.in(a.tv), n0, L, tid, hv.in_rs);
   }
@@ -156,10 +157,10 @@ __global__ void __launch_bounds__(32 * RG * KG, DkdvCfg<D, HAS_GO, HAS_GT, RG, K
       float p[2][4], ts[2][4], e_[2][4], f[2][4];
       {
         float y2[2][4];
-        scores<D, HAS_GT, HAS_GT, C::kResident == 1>(p, ts, y2, aK, aTK, aQ, aTQ, r0, qr, lane);
+        scores<D, TKV, HAS_GT, C::kResident == 1>(p, ts, y2, aK, aTK, aQ, aTQ, r0, qr, lane);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const float ik = iOwn[r0 + g + 8 * r], itk = HAS_GT ? iOwn[2 * BN + r0 + g + 8 * r] : 0.f;
+          const float ik = iOwn[r0 + g + 8 * r], itk = TKV ? iOwn[2 * BN + r0 + g + 8 * r] : 0.f;
 #pragma unroll
           for (int n = 0; n < 2; ++n) {
 #pragma unroll
@@ -167,7 +168,10 @@ __global__ void __launch_bounds__(32 * RG * KG, DkdvCfg<D, HAS_GO, HAS_GT, RG, K
               const int e = 2 * r + c, j = n * 8 + 2 * t + c;
               const float s = p[n][e] * ik * iq[j];
               p[n][e] = ok[n][e] ? exp2f(s * scale_log2 + bias[n][e] * kLog2e - st[j]) : 0.f;
-              if constexpr (HAS_GT) ts[n][e] = fmaf(ts[n][e] * itk, iq[j], y2[n][e] * ik * itq[j]) * a.sm_scale;
+              if constexpr (TKV)
+                ts[n][e] = fmaf(ts[n][e] * itk, iq[j], y2[n][e] * ik * itq[j]) * a.sm_scale;
+              else if constexpr (HAS_GT)
+                ts[n][e] = y2[n][e] * ik * itq[j] * a.sm_scale;
             }
           }
         }
@@ -175,12 +179,12 @@ __global__ void __launch_bounds__(32 * RG * KG, DkdvCfg<D, HAS_GO, HAS_GT, RG, K
       {
         float y1[2][4], y2[2][4];
         if constexpr (HAS_GT)
-          scores<D, true, HAS_GO, C::kResident == 1>(e_, y1, y2, aV, aTV, aG, aGO, r0, qr, lane);
+          scores<D, TKV, HAS_GO, C::kResident == 1>(e_, y1, y2, aV, aTV, aG, aGO, r0, qr, lane);
         else
           scores<D, false, false, C::kResident == 1>(y2, y1, y1, aV, aV, aGO, aGO, r0, qr, lane);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const float iv = iOwn[BN + r0 + g + 8 * r], itv = HAS_GT ? iOwn[3 * BN + r0 + g + 8 * r] : 0.f;
+          const float iv = iOwn[BN + r0 + g + 8 * r], itv = TKV ? iOwn[3 * BN + r0 + g + 8 * r] : 0.f;
 #pragma unroll
           for (int n = 0; n < 2; ++n) {
 #pragma unroll
@@ -190,7 +194,7 @@ __global__ void __launch_bounds__(32 * RG * KG, DkdvCfg<D, HAS_GO, HAS_GT, RG, K
               float x = HAS_GO ? y2[n][e] * iv * igo[j] : 0.f, sub = st[BM + j];
               if constexpr (HAS_GT) {
                 const float tsv = ts[n][e], ev = e_[n][e] * iv * ig[j], eps = st[2 * BM + j], mu = st[4 * BM + j];
-                x = fmaf(y1[n][e] * itv, ig[j], x);
+                if constexpr (TKV) x = fmaf(y1[n][e] * itv, ig[j], x);
                 sub += st[3 * BM + j];
                 x += ev * (tsv - mu) - eps * tsv;
                 e_[n][e] = pv * (ev - eps);  // gtS
@@ -232,15 +236,15 @@ __global__ void __launch_bounds__(32 * RG * KG, DkdvCfg<D, HAS_GO, HAS_GT, RG, K
 }
 
 // ---- dQ (rows = queries, columns = keys) ----
-template <int D, bool HAS_GO, bool HAS_GT, int RG, int KG>
-using DqCfg = BwdCfg<D, 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0), HAS_GT ? 4 : 2, RG, KG, false,
+template <int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
+using DqCfg = BwdCfg<D, 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0), TKV ? 4 : 2, RG, KG, false,
                      RG == 4 && (D <= 64 || !HAS_GT) ? 2 : 1>;
 
-template <int D, bool HAS_GO, bool HAS_GT, int RG, int KG>
-__global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, RG, KG>::kResident) bwd_dq_fp32_kernel(const jvpfa_bwd_args a) {
-  using C = DqCfg<D, HAS_GO, HAS_GT, RG, KG>;
+template <int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
+__global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, TKV, RG, KG>::kResident) bwd_dq_fp32_kernel(const jvpfa_bwd_args a) {
+  using C = DqCfg<D, HAS_GO, HAS_GT, TKV, RG, KG>;
   constexpr int BM = C::OWN, BN = C::LOOP, NT = C::NT, STAGES = C::STAGES, ND = D / 8;
-  constexpr int OWN_TILES = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0), LOOP_TILES = HAS_GT ? 4 : 2;
+  constexpr int OWN_TILES = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0), LOOP_TILES = TKV ? 4 : 2;
   constexpr int kGO = 1, kTQ = 1 + (HAS_GO ? 1 : 0), kG = kTQ + 1;  // own tiles after Q
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -267,7 +271,7 @@ __global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, RG, KG>
     unsigned char* base = sLoop + (it & (STAGES - 1)) * LOOP_TILES * C::kLoop;
     copy_tile<BN, D, NT>(base, hv.in(a.k), it * BN, L, tid, hv.in_rs);
     copy_tile<BN, D, NT>(base + C::kLoop, hv.in(a.v), it * BN, L, tid, hv.in_rs);
-    if constexpr (HAS_GT) {
+    if constexpr (TKV) {
       copy_tile<BN, D, NT>(base + 2 * C::kLoop, hv.in(a.tk), it * BN, L, tid, hv.in_rs);
       copy_tile<BN, D, NT>(base + 3 * C::kLoop, hv.in(a.tv), it * BN, L, tid, hv.in_rs);
     }
@@ -332,7 +336,7 @@ __global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, RG, KG>
       float p[2][4], ts[2][4], e_[2][4], f[2][4];
       {
         float y2[2][4];
-        scores<D, HAS_GT, HAS_GT, C::kResident == 1>(p, ts, y2, aQ, aTQ, aK, aTK, r0, kr, lane);
+        scores<D, HAS_GT, TKV, C::kResident == 1>(p, ts, y2, aQ, aTQ, aK, aTK, r0, kr, lane);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const float iq = iOwn[r0 + g + 8 * r], itq = HAS_GT ? iOwn[kTQ * BM + r0 + g + 8 * r] : 0.f;
@@ -343,7 +347,10 @@ __global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, RG, KG>
               const int e = 2 * r + c, j = n * 8 + 2 * t + c;
               const float s = p[n][e] * iq * ik[j];
               p[n][e] = ok[n][e] ? exp2f(s * scale_log2 + bias[n][e] * kLog2e - lse[r]) : 0.f;
-              if constexpr (HAS_GT) ts[n][e] = fmaf(ts[n][e] * itq, ik[j], y2[n][e] * iq * itk[j]) * a.sm_scale;
+              if constexpr (TKV)
+                ts[n][e] = fmaf(ts[n][e] * itq, ik[j], y2[n][e] * iq * itk[j]) * a.sm_scale;
+              else if constexpr (HAS_GT)
+                ts[n][e] = ts[n][e] * itq * ik[j] * a.sm_scale;
             }
           }
         }
@@ -352,7 +359,7 @@ __global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, RG, KG>
         // E = G V^T, dP = gO V^T, F = G tV^T
         float y1[2][4], y2[2][4];
         if constexpr (HAS_GT)
-          scores<D, HAS_GO, true, C::kResident == 1>(e_, y1, y2, aG, aGO, aV, aTV, r0, kr, lane);
+          scores<D, HAS_GO, TKV, C::kResident == 1>(e_, y1, y2, aG, aGO, aV, aTV, r0, kr, lane);
         else
           scores<D, false, false, C::kResident == 1>(y1, y2, y2, aGO, aGO, aV, aV, r0, kr, lane);
 #pragma unroll
@@ -367,7 +374,7 @@ __global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, RG, KG>
               float x = HAS_GO ? y1[n][e] * igo * iv[j] : 0.f;
               if constexpr (HAS_GT) {
                 const float tsv = ts[n][e], ev = e_[n][e] * ig * iv[j];
-                x = fmaf(y2[n][e] * ig, itv[j], x);
+                if constexpr (TKV) x = fmaf(y2[n][e] * ig, itv[j], x);
                 x += ev * (tsv - mu[r]) - eps[r] * tsv;
                 e_[n][e] = pv * (ev - eps[r]);  // gtS
               }
@@ -379,8 +386,8 @@ __global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, RG, KG>
       PairA f0, f1;  // gS K + gtS tK
       float k0[2], k1[2];
       a_from_acc(f0, k0, f, ik, lane);
-      if constexpr (HAS_GT) a_from_acc(f1, k1, e_, itk, lane);
-      outputs<D, true, HAS_GT>(dq, f0, k0, f1, k1, aK, aTK, kr, lane);
+      if constexpr (TKV) a_from_acc(f1, k1, e_, itk, lane);
+      outputs<D, true, TKV>(dq, f0, k0, f1, k1, aK, aTK, kr, lane);
     }
     if (it + 1 < n_tiles) {
       if constexpr (STAGES == 1) {
@@ -400,13 +407,13 @@ __global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, RG, KG>
   store_strip<D>(reinterpret_cast<float*>(a.dq) + hv.off, dq, fq, row_lo, L, lane);
 }
 
-template <int D, bool HAS_GO, bool HAS_GT, int RG, int KG>
+template <int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
 int launch_one(const jvpfa_bwd_args& a, cudaStream_t stream) {
-  using C1 = DkdvCfg<D, HAS_GO, HAS_GT, RG, KG>;
-  using C2 = DqCfg<D, HAS_GO, HAS_GT, RG, KG>;
+  using C1 = DkdvCfg<D, HAS_GO, HAS_GT, TKV, RG, KG>;
+  using C2 = DqCfg<D, HAS_GO, HAS_GT, TKV, RG, KG>;
   static_assert(C1::smem <= 227 * 1024 && C2::smem <= 227 * 1024, "shared memory of one CTA");
-  auto k1 = bwd_dkdv_fp32_kernel<D, HAS_GO, HAS_GT, RG, KG>;
-  auto k2 = bwd_dq_fp32_kernel<D, HAS_GO, HAS_GT, RG, KG>;
+  auto k1 = bwd_dkdv_fp32_kernel<D, HAS_GO, HAS_GT, TKV, RG, KG>;
+  auto k2 = bwd_dq_fp32_kernel<D, HAS_GO, HAS_GT, TKV, RG, KG>;
   static SmemOptIn opt_in1, opt_in2;
   if (!opt_in1.ensure(reinterpret_cast<const void*>(k1), C1::smem) || !opt_in2.ensure(reinterpret_cast<const void*>(k2), C2::smem))
     return JVPFA_ERR_CUDA;
@@ -425,9 +432,9 @@ template <int D>
 int launch_d(const jvpfa_bwd_args& a, cudaStream_t s) {
   return dispatch_split<D>(a.B, a.H, a.L, [&](auto rg, auto kg) {
     constexpr int RG = decltype(rg)::value, KG = decltype(kg)::value;
-    if (a.go && a.gto) return launch_one<D, true, true, RG, KG>(a, s);
-    if (a.gto) return launch_one<D, false, true, RG, KG>(a, s);
-    return launch_one<D, true, false, RG, KG>(a, s);
+    if (!a.gto) return launch_one<D, true, false, false, RG, KG>(a, s);
+    if (a.flags & JVPFA_ZERO_TKV) return launch_one<D, false, true, false, RG, KG>(a, s);  // (go is refused with it)
+    return a.go ? launch_one<D, true, true, true, RG, KG>(a, s) : launch_one<D, false, true, true, RG, KG>(a, s);
   });
 }
 

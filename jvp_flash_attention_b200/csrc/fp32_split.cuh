@@ -266,8 +266,8 @@ __device__ __forceinline__ void outputs(float (*out)[4], const PairA& a0, const 
   }
 }
 
-// The forward's pair of outputs in one sweep over V: o += A0 B0, t += A1 B0 + A2 B1 (O += P V, tO += W V + P tV).
-template <int D>
+// The forward's pair of outputs in one sweep over V: o += A0 B0, t += A1 B0 (+ A2 B1)   (O += P V, tO += W V + P tV).
+template <int D, bool HAS_2>
 __device__ __forceinline__ void outputs_dual(float (*o)[4], float (*t)[4], const PairA& a0, const float* k0, const PairA& a1, const float* k1,
                                              const PairA& a2, const float* k2, uint32_t b0, uint32_t b1, int row0, int lane) {
   constexpr int G = 2;
@@ -278,14 +278,14 @@ __device__ __forceinline__ void outputs_dual(float (*o)[4], float (*t)[4], const
 #pragma unroll
     for (int i = 0; i < G; ++i) {
       load_b_nn<D>(f0[i], b0, row0, (d0 + i) * 8, lane);
-      load_b_nn<D>(f1[i], b1, row0, (d0 + i) * 8, lane);
+      if constexpr (HAS_2) load_b_nn<D>(f1[i], b1, row0, (d0 + i) * 8, lane);
     }
     auto pass = [&](auto P) {
 #pragma unroll
       for (int i = 0; i < G; ++i) {
         mma_pass<P(), P() == 0>(x[i], a0, f0[i]);
         mma_pass<P(), P() == 0>(y[i], a1, f0[i]);
-        mma_pass<P(), P() == 0>(z[i], a2, f1[i]);
+        if constexpr (HAS_2) mma_pass<P(), P() == 0>(z[i], a2, f1[i]);
       }
     };
     pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
@@ -294,7 +294,8 @@ __device__ __forceinline__ void outputs_dual(float (*o)[4], float (*t)[4], const
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         o[d0 + i][e] = fmaf(x[i][e], k0[e >> 1], o[d0 + i][e]);
-        t[d0 + i][e] = fmaf(z[i][e], k2[e >> 1], fmaf(y[i][e], k1[e >> 1], t[d0 + i][e]));
+        t[d0 + i][e] = fmaf(y[i][e], k1[e >> 1], t[d0 + i][e]);
+        if constexpr (HAS_2) t[d0 + i][e] = fmaf(z[i][e], k2[e >> 1], t[d0 + i][e]);
       }
     }
   }

@@ -23,10 +23,12 @@ namespace {
 
 using namespace f32;
 
-template <int D, bool DUAL, int RG, int KG>
+// TKV: K and V have tangents (JVPFA_ZERO_TKV leaves them, and two of the six products, out: B2 H8 L1024 D128 with bias 402
+// -> 301 us, the backward through tO for dQ 438 -> 267 us).
+template <int D, bool DUAL, bool TKV, int RG, int KG>
 struct FwdCfg {
   static constexpr int BM = 16 * RG, BN = 16 * KG, NT = 32 * RG * KG;
-  static constexpr int NQ = DUAL ? 2 : 1, NKV = DUAL ? 4 : 2;
+  static constexpr int NQ = DUAL ? 2 : 1, NKV = TKV ? 4 : 2;
   static constexpr int kTile = BN * D * 4;
   // Two CTAs on an SM where registers allow (one output to accumulate, or a head dimension of 32) and there are enough of
   // them (64-row tiles): they wait at different times.  B2 H8 L2048: one output, D 64, 404 -> 316 us; both, D 32, 548 -> 437
@@ -39,9 +41,9 @@ struct FwdCfg {
   static constexpr size_t smem = (size_t)NQ * BM * D * 4 + kRing + 4 * (kScales + kRow);
 };
 
-template <int D, bool DUAL, int RG, int KG>
-__global__ void __launch_bounds__(32 * RG * KG, FwdCfg<D, DUAL, RG, KG>::kResident) fwd_fp32_kernel(const jvpfa_fwd_args a) {
-  using C = FwdCfg<D, DUAL, RG, KG>;
+template <int D, bool DUAL, bool TKV, int RG, int KG>
+__global__ void __launch_bounds__(32 * RG * KG, FwdCfg<D, DUAL, TKV, RG, KG>::kResident) fwd_fp32_kernel(const jvpfa_fwd_args a) {
+  using C = FwdCfg<D, DUAL, TKV, RG, KG>;
   constexpr int BM = C::BM, BN = C::BN, NT = C::NT, STAGES = C::STAGES, NKV = C::NKV, ND = D / 8;
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -76,7 +78,7 @@ __global__ void __launch_bounds__(32 * RG * KG, FwdCfg<D, DUAL, RG, KG>::kReside
     unsigned char* base = sKV + (it & (STAGES - 1)) * NKV * C::kTile;
     copy_tile<BN, D, NT>(base, head(a.k), it * BN, L, tid, in_rs);
     copy_tile<BN, D, NT>(base + C::kTile, head(a.v), it * BN, L, tid, in_rs);
-    if constexpr (DUAL) {
+    if constexpr (TKV) {
       copy_tile<BN, D, NT>(base + 2 * C::kTile, head(a.tk), it * BN, L, tid, in_rs);
       copy_tile<BN, D, NT>(base + 3 * C::kTile, head(a.tv), it * BN, L, tid, in_rs);
     }
@@ -131,7 +133,7 @@ __global__ void __launch_bounds__(32 * RG * KG, FwdCfg<D, DUAL, RG, KG>::kReside
       }
 
       float s[2][4], y1[2][4], y2[2][4];
-      scores<D, DUAL, DUAL, C::kResident == 1>(s, y1, y2, aQ, aTQ, aK, aTK, r0, kr, lane);
+      scores<D, DUAL, TKV, C::kResident == 1>(s, y1, y2, aQ, aTQ, aK, aTK, r0, kr, lane);
 
       // take the scales back, mask / bias, move to the base-2 domain
       float mx[2] = {-INFINITY, -INFINITY};
@@ -144,7 +146,10 @@ __global__ void __launch_bounds__(32 * RG * KG, FwdCfg<D, DUAL, RG, KG>::kReside
           for (int c = 0; c < 2; ++c) {
             const int e = 2 * r + c, j = n * 8 + 2 * t + c;
             float x = s[n][e] * iq * ik[j] * scale_log2;
-            if constexpr (DUAL) y1[n][e] = fmaf(y1[n][e] * itq, ik[j], y2[n][e] * iq * itk[j]);
+            if constexpr (TKV)
+              y1[n][e] = fmaf(y1[n][e] * itq, ik[j], y2[n][e] * iq * itk[j]);
+            else if constexpr (DUAL)
+              y1[n][e] *= itq * ik[j];
             if (!full_tile) {
               if (ok[n][e]) {
                 x += bias[n][e] * kLog2e;
@@ -203,8 +208,8 @@ __global__ void __launch_bounds__(32 * RG * KG, FwdCfg<D, DUAL, RG, KG>::kReside
         PairA fw, ft;
         float kw[2], kt[2];
         a_from_acc(fw, kw, y1, iv, lane);
-        a_from_acc(ft, kt, s, itv, lane);
-        outputs_dual<D>(acc_o, acc_t, fp, kp, fw, kw, ft, kt, aV, aTV, kr, lane);
+        if constexpr (TKV) a_from_acc(ft, kt, s, itv, lane);
+        outputs_dual<D, TKV>(acc_o, acc_t, fp, kp, fw, kw, ft, kt, aV, aTV, kr, lane);
       } else {
         outputs<D, true, false>(acc_o, fp, kp, fp, kp, aV, aV, kr, lane);
       }
@@ -292,11 +297,11 @@ __global__ void __launch_bounds__(32 * RG * KG, FwdCfg<D, DUAL, RG, KG>::kReside
   if constexpr (DUAL) store_strip<D>(reinterpret_cast<float*>(a.to) + head_off, acc_t, inv_l, row_lo, L, lane);
 }
 
-template <int D, bool DUAL, int RG, int KG>
+template <int D, bool DUAL, bool TKV, int RG, int KG>
 int launch_one(const jvpfa_fwd_args& a, cudaStream_t stream) {
-  using C = FwdCfg<D, DUAL, RG, KG>;
+  using C = FwdCfg<D, DUAL, TKV, RG, KG>;
   static_assert(C::smem <= 227 * 1024, "shared memory of one CTA");
-  auto kern = fwd_fp32_kernel<D, DUAL, RG, KG>;
+  auto kern = fwd_fp32_kernel<D, DUAL, TKV, RG, KG>;
   static SmemOptIn opt_in;
   if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::smem)) return JVPFA_ERR_CUDA;
   kern<<<dim3((a.L + C::BM - 1) / C::BM, a.B * a.H), C::NT, C::smem, stream>>>(a);
@@ -311,8 +316,9 @@ int launch_one(const jvpfa_fwd_args& a, cudaStream_t stream) {
 template <int D>
 int launch_d(const jvpfa_fwd_args& a, cudaStream_t s) {
   return dispatch_split<D>(a.B, a.H, a.L, [&](auto rg, auto kg) {
-    return a.tq ? launch_one<D, true, decltype(rg)::value, decltype(kg)::value>(a, s)
-                : launch_one<D, false, decltype(rg)::value, decltype(kg)::value>(a, s);
+    constexpr int RG = decltype(rg)::value, KG = decltype(kg)::value;
+    if (!a.tq) return launch_one<D, false, false, RG, KG>(a, s);
+    return a.flags & JVPFA_ZERO_TKV ? launch_one<D, true, false, RG, KG>(a, s) : launch_one<D, true, true, RG, KG>(a, s);
   });
 }
 

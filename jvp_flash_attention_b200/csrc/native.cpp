@@ -192,6 +192,7 @@ struct Inputs {
 // ---- launches ------------------------------------------------------------------------------------------------------
 py::object or_none(const Tensor& t) { return t.defined() ? py::cast(t) : py::object(py::none()); }
 
+// tq without tk and tv: JVPFA_ZERO_TKV.
 FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& tq, const Tensor& tk, const Tensor& tv,
                      const Call& call) {
   const bool dual = tq.defined();
@@ -231,6 +232,7 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   a.mask = call.c_mask();
   a.mask_tile_live = data(call.mask->tile_live);
   a.mask_bits = data(call.bits);
+  a.flags = dual && !tk.defined() ? JVPFA_ZERO_TKV : 0;
   void* stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
   for (;;) {
     a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
@@ -251,7 +253,7 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
 // (a replayed graph, a foreign kernel, `.data`).
 //
 // Packing reads the mask once (HBM bound) and saves a kernel that reads it one 16-byte piece per row and sub-tile.
-// B2 H12 L2048 D64, 100 MB of mask: packing 25 us; forward with tangents 168 -> 151 us, backward through tO 239 -> 186.
+// B2 H12 L2048 D64, 100 MB of mask: packing 32 us; forward with tangents 168 -> 151 us, backward through tO 239 -> 186.
 // So it pays with a backward, for a mask that several heads share, and where the bytes' layout would send the call to
 // the register-tiled kernels.
 void prepare_mask(Call& call, const Tensor& q, bool backward) {
@@ -358,7 +360,7 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.lse = static_cast<const float*>(data(lse));
   a.mu = p.mu;
   a.delta = p.delta, a.eps = p.eps, a.cterm = p.cterm;
-  a.flags = skip | (single ? JVPFA_DQ_ACCUM_IS_ZERO : 0);
+  a.flags = skip | (single ? JVPFA_DQ_ACCUM_IS_ZERO : 0) | (tq.defined() && !tk.defined() ? JVPFA_ZERO_TKV : 0);
   if (g[0].defined()) a.dq = g[0].data_ptr();
   if (g[1].defined()) a.dk = g[1].data_ptr(), a.dv = g[2].data_ptr();
   a.mask = call.c_mask();
@@ -428,10 +430,13 @@ struct AttnBwdNode : public Node {
     const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), go_ = go.unpack();
     const Tensor qp = unwrap(q_), kp = unwrap(k_), vp = unwrap(v_), gop = unwrap(go_);
     Tensor t[3];
+    // a product with a vector that is zero on K and V (only q is differentiated): the fp32 kernels leave their terms out
+    const bool zero_tkv = u[0].defined() && !u[1].defined() && !u[2].defined() && qp.is_cuda() && qp.scalar_type() == at::kFloat &&
+                          !call.tf32;
     {
       NoFunctorch nf;
       at::AutoDispatchBelowADInplaceOrView below;
-      for (int i = 0; i < 3; ++i) t[i] = u[i].defined() ? unwrap(u[i]).contiguous() : at::zeros_like(qp, at::MemoryFormat::Contiguous);
+      for (int i = 0; i < (zero_tkv ? 1 : 3); ++i) t[i] = u[i].defined() ? unwrap(u[i]).contiguous() : at::zeros_like(qp, at::MemoryFormat::Contiguous);
     }
     FwdResult f = launch_fwd(qp, kp, vp, t[0], t[1], t[2], call);
     const int skip = unused_gradients(task_should_compute_output(0), task_should_compute_output(1) || task_should_compute_output(2));

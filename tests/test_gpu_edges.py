@@ -176,3 +176,24 @@ def test_fp32_rows_of_very_different_magnitude(B, H, L, D):
         top = weight if name == "O" else head(clean[1]) if name == "tO" else head(r)
         off = ((x - r.double()).abs() / top.clamp(min=1e-30)).max().item()
         assert off <= 1e-5, (name, off)
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("B,H,L,kind", [(1, 2, 34, "none"), (2, 10, 250, "bias"), (2, 12, 450, "causal")])
+def test_fp32_second_differentiation_along_q_alone(B, H, L, D, kind):
+    """With K and V held fixed their zero tangents are left out (both routes form the same products otherwise): against the
+    general route, which a zero direction for K and V takes.  1e-5 of the largest entry, the fp32 bound of this file."""
+    q, k, v, u, _, _, go, _ = (x.to(DEV) for x in _inputs(B, H, L, D, torch.float32, L + D))
+    mask = _mask(kind, B, H, L, torch.float32, 1)
+    mask = None if mask is None else mask.to(DEV)
+
+    def second(leaves):
+        a = [x.clone().requires_grad_(n in leaves) for n, x in (("q", q), ("k", k), ("v", v))]
+        w = go.clone().requires_grad_()
+        o = ja.attention(*a, attn_mask=mask, causal=kind == "causal")
+        first = torch.autograd.grad(o, [x for x in a if x.requires_grad], w, create_graph=True)
+        z = [u] + [torch.zeros_like(k) for _ in first[1:]]
+        return torch.autograd.grad(first, [a[0], w], z)
+
+    for x, y in zip(second("q"), second("qkv")):
+        assert (x - y).abs().max().item() <= 1e-5 * y.abs().max().item()
