@@ -116,8 +116,8 @@ struct LoopWalk {
 // bitmaps (loop tiles without a true entry are not visited).  For 1 and 2 every elementwise
 // thread fetches the 16 mask elements of its piece of the tile from global memory before it waits for the scores (own
 // queries: one or two 16-byte loads of the thread's mask row; own keys: one element of each of 16 query rows, the lanes
-// of a warp reading neighbouring keys).  Key stride 1, 16-byte aligned rows and L % 16 == 0 are the host's
-// responsibility.
+// of a warp reading neighbouring keys).  A boolean mask given as bits is read as those instead, 16 bits of one word.  The
+// layout is the host's responsibility (tc5_mask_layout).
 template <typename T, bool OWN_KEYS, bool HAS_GO, bool HAS_GT, int MK>
 __global__ void __launch_bounds__(BwdPipeCfg<OWN_KEYS, HAS_GO, HAS_GT>::NTHREADS, 1)
 bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMaps maps, int* status) {

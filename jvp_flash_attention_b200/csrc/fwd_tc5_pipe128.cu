@@ -57,8 +57,8 @@ struct FwdPipeMaps {
 };
 
 // MK: 0 = none / causal / key padding; 1 = uint8 mask; 2 = bias of the element type T (the softmax thread of a
-// query row reads its 64 mask elements of the tile with 16-byte loads before it waits for the scores; key stride 1,
-// 16-byte aligned rows and L % 16 == 0 are the host's responsibility); 3 = uint8 mask with the bitmap of 128 x 64
+// query row reads its 64 mask elements of the tile with 16-byte loads before it waits for the scores, or 8 bytes of a boolean
+// mask given as bits; the layout is the host's responsibility: tc5_mask_layout); 3 = uint8 mask with the bitmap of 128 x 64
 // tiles that hold a true entry (jvpfa_mask_tiles): the CTA lists its query tile's live key tiles once and every role
 // walks that list, so tiles without a true entry are neither loaded nor multiplied.
 template <typename T, bool DUAL, int MK>
