@@ -5,7 +5,7 @@
 //
 // Bound like the forward (fwd_fp32.cu) by latency: dK and dV together take the registers that two outputs take there.
 // B200, B2 H8 L1024 D128, against three TF32 products split in every warp: dQ through tO with bias 798 -> 438 us, through O
-// 440 -> 250 us; B2 H4 L256 D64, both outputs: dK and dV 27.6 -> 21.4 us, dQ 22.5 -> 18.3 us.  Error against 64 bits: 3e-7 to
+// 440 -> 230 us; B2 H4 L256 D64, both outputs: dK and dV 27.6 -> 21.4 us, dQ 22.5 -> 18.3 us.  Error against 64 bits: 3e-7 to
 // 1.2e-6 (TF32 pairs: 6e-7 to 4.3e-6).
 #include "fp32_split.cuh"
 
@@ -298,6 +298,9 @@ __global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, TKV, RG
 
   const float scale_log2 = a.sm_scale * kLog2e;
   const int r0 = rg * 16, kr = kg * 16;
+  // D = 128 with two CTAs on an SM: the addresses of fully unrolled products are what spills (432 -> 64 bytes; 242 -> 223 us at
+  // B2 H8 L1024 through O).  Elsewhere the loop costs more than it saves (D = 64, same shape: 114 -> 122 us).
+  constexpr int kUnroll = D == 128 && C::kResident == 2 ? 2 : D / 16;
   const int row_lo = m0 + r0 + g;
   const uint32_t aQ = smem_addr(sOwn), aGO = aQ + kGO * C::kOwn, aTQ = aQ + kTQ * C::kOwn, aG = aQ + kG * C::kOwn;
   float lse[2], sub[2], eps[2] = {0.f, 0.f}, mu[2] = {0.f, 0.f};
@@ -336,7 +339,7 @@ __global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, TKV, RG
       float p[2][4], ts[2][4], e_[2][4], f[2][4];
       {
         float y2[2][4];
-        scores<D, HAS_GT, TKV, C::kResident == 1>(p, ts, y2, aQ, aTQ, aK, aTK, r0, kr, lane);
+        scores<D, HAS_GT, TKV, C::kResident == 1, kUnroll>(p, ts, y2, aQ, aTQ, aK, aTK, r0, kr, lane);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const float iq = iOwn[r0 + g + 8 * r], itq = HAS_GT ? iOwn[kTQ * BM + r0 + g + 8 * r] : 0.f;
@@ -359,9 +362,9 @@ __global__ void __launch_bounds__(32 * RG * KG, DqCfg<D, HAS_GO, HAS_GT, TKV, RG
         // E = G V^T, dP = gO V^T, F = G tV^T
         float y1[2][4], y2[2][4];
         if constexpr (HAS_GT)
-          scores<D, HAS_GO, TKV, C::kResident == 1>(e_, y1, y2, aG, aGO, aV, aTV, r0, kr, lane);
+          scores<D, HAS_GO, TKV, C::kResident == 1, kUnroll>(e_, y1, y2, aG, aGO, aV, aTV, r0, kr, lane);
         else
-          scores<D, false, false, C::kResident == 1>(y1, y2, y2, aGO, aGO, aV, aV, r0, kr, lane);
+          scores<D, false, false, C::kResident == 1, kUnroll>(y1, y2, y2, aGO, aGO, aV, aV, r0, kr, lane);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const float igo = HAS_GO ? iOwn[kGO * BM + r0 + g + 8 * r] : 0.f, ig = HAS_GT ? iOwn[kG * BM + r0 + g + 8 * r] : 0.f;

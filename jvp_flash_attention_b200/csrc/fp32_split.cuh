@@ -176,7 +176,7 @@ __device__ __forceinline__ void zero(float (*x)[4]) {
 // x[n-tile] = A0 B0^T, and where asked for y1 = A1 B0^T, y2 = A0 B1^T; 16 rows, 16 columns (two n-tiles), over D.
 // AHEAD: the next step's operands are fetched ahead of this one's products (32 registers that two CTAs on an SM do not have,
 // nor need: their warps cover for one another).
-template <int D, bool HAS_Y1, bool HAS_Y2, bool AHEAD>
+template <int D, bool HAS_Y1, bool HAS_Y2, bool AHEAD, int UNROLL = D / 16>
 __device__ __forceinline__ void scores(float (*x)[4], float (*y1)[4], float (*y2)[4], uint32_t a0, uint32_t a1, uint32_t b0, uint32_t b1,
                                        int r0, int n0, int lane) {
   PairA fa0[2], fa1[2];
@@ -192,7 +192,7 @@ __device__ __forceinline__ void scores(float (*x)[4], float (*y1)[4], float (*y2
     }
   };
   if constexpr (AHEAD) fetch(0);
-#pragma unroll
+#pragma unroll UNROLL
   for (int k0 = 0; k0 < D; k0 += 16) {
     const int i = AHEAD ? (k0 / 16) & 1 : 0;
     if constexpr (AHEAD) {
