@@ -16,6 +16,8 @@
 // over query tiles (dK, dV) and one that owns a query tile and loops over key tiles (dQ); score
 // tiles are recomputed from the saved base-2 logsumexp, so results are deterministic and no
 // L x L tensor or atomic accumulation is needed.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace jvpfa {
@@ -130,7 +132,7 @@ int launch_pre(const jvpfa_pre_args& a, cudaStream_t s) {
 // Main kernels.  A CTA of RG x KG warps owns 16*RG rows (keys for dK / dV, queries for dQ) and loops over tiles of the
 // other side; warp (rg, kg) owns 16 of the rows and the kg-th part of every loop tile, sums its own dK, dV or dQ, and the
 // KG partial sums are added once at the end (a fixed order: results stay reproducible bit for bit).  As in the forward
-// (fwd_generic.cu) the bound is mma.sync, and the split puts two warps on each
+// (fwd_generic.cu) the bound is mma.sync, three instructions for an fp32 product, and the split puts two warps on each
 // quarter of an SM that shared memory would otherwise leave with one, and lets small shapes use more SMs.
 //
 // All score products of a tile are formed in two sweeps over D, {S, tS} and {E, F + dP}, so that an operand fragment is
@@ -184,20 +186,23 @@ __device__ __forceinline__ void gemm_pair(float (*x)[4], float (*y)[4], const T*
       load_b_nt<T>(b0[nt], sB0, ld, nt * 8, k0, lane);
       if constexpr (HAS_Y2) load_b_nt<T>(b1[nt], sB1, ld, nt * 8, k0, lane);
     }
+    auto pass = [&](auto P) {
 #pragma unroll
-    for (int nt = 0; nt < NT_; ++nt) {
-      mma<T>(x[nt], a0, b0[nt]);
-      if constexpr (HAS_Y1) mma<T>(y[nt], a1, b0[nt]);
-    }
-    if constexpr (HAS_Y2) {
+      for (int nt = 0; nt < NT_; ++nt) {
+        mma_pass<P()>(x[nt], a0, b0[nt]);
+        if constexpr (HAS_Y1) mma_pass<P()>(y[nt], a1, b0[nt]);
+      }
+      if constexpr (HAS_Y2) {
 #pragma unroll
-      for (int nt = 0; nt < NT_; ++nt) mma<T>(y[nt], a0, b1[nt]);
-    }
+        for (int nt = 0; nt < NT_; ++nt) mma_pass<P()>(y[nt], a0, b1[nt]);
+      }
+    };
+    pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
   }
 }
 
 // out[D/8][4] += A0 B0 (+ A1 B1): A from accumulator tiles (16 x KROWS), B = [k][d] tiles, d contiguous.
-// TF32: the tensor core adds into its fp32 accumulator with truncation, and hundreds of such adds into one long-lived
+// fp32: the tensor core adds into its fp32 accumulator with truncation, and hundreds of such adds into one long-lived
 // accumulator show up as a bias of ~1e-5.  Each contraction step is therefore formed in fresh registers and added rounded.
 template <typename T, int D, int KROWS, bool HAS_0, bool HAS_1>
 __device__ __forceinline__ void gemm_out(float (*out)[4], const float (*at0)[4], const float (*at1)[4], const T* sB0, const T* sB1,
@@ -220,14 +225,17 @@ __device__ __forceinline__ void gemm_out(float (*out)[4], const float (*at0)[4],
 #pragma unroll
         for (int e = 0; e < 4; ++e) tmp[i][e] = Elem<T>::k16 ? out[d0 + i][e] : 0.f;
       }
-      if constexpr (HAS_0) {
+      auto pass = [&](auto P) {
+        if constexpr (HAS_0) {
 #pragma unroll
-        for (int i = 0; i < G; ++i) mma<T>(tmp[i], a0, b0[i]);
-      }
-      if constexpr (HAS_1) {
+          for (int i = 0; i < G; ++i) mma_pass<P()>(tmp[i], a0, b0[i]);
+        }
+        if constexpr (HAS_1) {
 #pragma unroll
-        for (int i = 0; i < G; ++i) mma<T>(tmp[i], a1, b1[i]);
-      }
+          for (int i = 0; i < G; ++i) mma_pass<P()>(tmp[i], a1, b1[i]);
+        }
+      };
+      pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
 #pragma unroll
       for (int i = 0; i < G; ++i) {
 #pragma unroll
@@ -266,21 +274,22 @@ __device__ __forceinline__ void smem_tile_to_global(T* ghead, const T* s, int ld
 
 // ---- dK, dV: CTA owns 64 keys, loops over query tiles.  Tiles are held transposed
 // (rows = keys, columns = queries) so that P^T etc. feed the second MMAs from registers. ----
-template <typename T, int D, bool HAS_GO, bool HAS_GT, int RG, int KG>
+// TKV: K and V have tangents (JVPFA_ZERO_TKV leaves out what they would be multiplied by; it comes without gO).
+template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
 __global__ void __launch_bounds__(32 * RG * KG) bwd_dkdv_kernel(const jvpfa_bwd_args a) {
   using C = BwdCfg<T, D, RG, KG>;
   constexpr int BN = C::OWN, BM = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES, LW = C::LW;
   constexpr int NQ = LW / 8;
   constexpr int ND = D / 8;
-  constexpr int OWN_TILES = HAS_GT ? 4 : 2;
+  constexpr int OWN_TILES = TKV ? 4 : 2;
   constexpr int LOOP_TILES = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0);
   static_assert(LW % Elem<T>::kKStep == 0, "a warp's loop rows are whole contraction steps");
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sK = reinterpret_cast<T*>(smem_raw);
   T* sV = sK + BN * LD;
-  T* sTK = sK + 2 * BN * LD;  // HAS_GT only
-  T* sTV = sK + 3 * BN * LD;  // HAS_GT only
+  T* sTK = sK + 2 * BN * LD;  // TKV only
+  T* sTV = sK + 3 * BN * LD;  // TKV only
   T* sLoop = sK + OWN_TILES * BN * LD;
   float* sStat = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(sLoop) + C::ring(LOOP_TILES));
 
@@ -302,8 +311,8 @@ __global__ void __launch_bounds__(32 * RG * KG) bwd_dkdv_kernel(const jvpfa_bwd_
   const T* gK = reinterpret_cast<const T*>(a.k) + in_off;
   const T* gV = reinterpret_cast<const T*>(a.v) + in_off;
   const T* gTQ = HAS_GT ? reinterpret_cast<const T*>(a.tq) + in_off : nullptr;
-  const T* gTK = HAS_GT ? reinterpret_cast<const T*>(a.tk) + in_off : nullptr;
-  const T* gTV = HAS_GT ? reinterpret_cast<const T*>(a.tv) + in_off : nullptr;
+  const T* gTK = TKV ? reinterpret_cast<const T*>(a.tk) + in_off : nullptr;
+  const T* gTV = TKV ? reinterpret_cast<const T*>(a.tv) + in_off : nullptr;
   const T* gGO = HAS_GO ? reinterpret_cast<const T*>(a.go) + head_off : nullptr;
   const T* gG = HAS_GT ? reinterpret_cast<const T*>(a.gto) + head_off : nullptr;
 
@@ -340,7 +349,7 @@ __global__ void __launch_bounds__(32 * RG * KG) bwd_dkdv_kernel(const jvpfa_bwd_
 
   stage_tile<T, BN, D, NT>(sK, gK, n0, L, tid, in_rs);
   stage_tile<T, BN, D, NT>(sV, gV, n0, L, tid, in_rs);
-  if constexpr (HAS_GT) {
+  if constexpr (TKV) {
     stage_tile<T, BN, D, NT>(sTK, gTK, n0, L, tid, in_rs);
     stage_tile<T, BN, D, NT>(sTV, gTV, n0, L, tid, in_rs);
   }
@@ -397,9 +406,9 @@ __global__ void __launch_bounds__(32 * RG * KG) bwd_dkdv_kernel(const jvpfa_bwd_
       zero_acc<NQ>(ts);
       zero_acc<NQ>(e_);
       zero_acc<NQ>(f);
-      gemm_pair<T, D, NQ, HAS_GT, HAS_GT>(p, ts, sK, sTK, sQ, sTQ, LD, r0, lane);
+      gemm_pair<T, D, NQ, TKV, HAS_GT>(p, ts, sK, sTK, sQ, sTQ, LD, r0, lane);
       if constexpr (HAS_GT)
-        gemm_pair<T, D, NQ, true, HAS_GO>(e_, f, sV, sTV, sG, sGO, LD, r0, lane);
+        gemm_pair<T, D, NQ, TKV, HAS_GO>(e_, f, sV, sTV, sG, sGO, LD, r0, lane);
       else
         gemm_pair<T, D, NQ, false, false>(f, f, sV, sV, sGO, sGO, LD, r0, lane);
 
@@ -446,14 +455,14 @@ __global__ void __launch_bounds__(32 * RG * KG) bwd_dkdv_kernel(const jvpfa_bwd_
 }
 
 // ---- dQ: CTA owns 64 queries, loops over key tiles (rows = queries, columns = keys). ----
-template <typename T, int D, bool HAS_GO, bool HAS_GT, int RG, int KG>
+template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
 __global__ void __launch_bounds__(32 * RG * KG) bwd_dq_kernel(const jvpfa_bwd_args a) {
   using C = BwdCfg<T, D, RG, KG>;
   constexpr int BM = C::OWN, BN = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES, LW = C::LW;
   constexpr int NK = LW / 8;
   constexpr int ND = D / 8;
   constexpr int OWN_TILES = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0);
-  constexpr int LOOP_TILES = HAS_GT ? 4 : 2;
+  constexpr int LOOP_TILES = TKV ? 4 : 2;
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sQ = reinterpret_cast<T*>(smem_raw);
@@ -481,8 +490,8 @@ __global__ void __launch_bounds__(32 * RG * KG) bwd_dq_kernel(const jvpfa_bwd_ar
   const T* gK = reinterpret_cast<const T*>(a.k) + in_off;
   const T* gV = reinterpret_cast<const T*>(a.v) + in_off;
   const T* gTQ = HAS_GT ? reinterpret_cast<const T*>(a.tq) + in_off : nullptr;
-  const T* gTK = HAS_GT ? reinterpret_cast<const T*>(a.tk) + in_off : nullptr;
-  const T* gTV = HAS_GT ? reinterpret_cast<const T*>(a.tv) + in_off : nullptr;
+  const T* gTK = TKV ? reinterpret_cast<const T*>(a.tk) + in_off : nullptr;
+  const T* gTV = TKV ? reinterpret_cast<const T*>(a.tv) + in_off : nullptr;
   const T* gGO = HAS_GO ? reinterpret_cast<const T*>(a.go) + head_off : nullptr;
   const T* gG = HAS_GT ? reinterpret_cast<const T*>(a.gto) + head_off : nullptr;
 
@@ -497,7 +506,7 @@ __global__ void __launch_bounds__(32 * RG * KG) bwd_dq_kernel(const jvpfa_bwd_ar
     T* base = sLoop + (size_t)stage * LOOP_TILES * BN * LD;
     stage_tile<T, BN, D, NT>(base, gK, n0, L, tid, in_rs);
     stage_tile<T, BN, D, NT>(base + BN * LD, gV, n0, L, tid, in_rs);
-    if constexpr (HAS_GT) {
+    if constexpr (TKV) {
       stage_tile<T, BN, D, NT>(base + 2 * BN * LD, gTK, n0, L, tid, in_rs);
       stage_tile<T, BN, D, NT>(base + 3 * BN * LD, gTV, n0, L, tid, in_rs);
     }
@@ -566,10 +575,10 @@ __global__ void __launch_bounds__(32 * RG * KG) bwd_dq_kernel(const jvpfa_bwd_ar
       zero_acc<NK>(ts);
       zero_acc<NK>(e_);
       zero_acc<NK>(f);
-      gemm_pair<T, D, NK, HAS_GT, HAS_GT>(p, ts, sQ, sTQ, sK, sTK, LD, r0, lane);
+      gemm_pair<T, D, NK, HAS_GT, TKV>(p, ts, sQ, sTQ, sK, sTK, LD, r0, lane);
       if constexpr (HAS_GT) {
         // E = G V^T, F = G tV^T; dP = gO V^T shares V
-        gemm_pair<T, D, NK, HAS_GO, true>(e_, f, sG, sGO, sV, sTV, LD, r0, lane);
+        gemm_pair<T, D, NK, HAS_GO, TKV>(e_, f, sG, sGO, sV, sTV, LD, r0, lane);
       } else {
         gemm_pair<T, D, NK, false, false>(f, f, sGO, sGO, sV, sV, LD, r0, lane);
       }
@@ -592,7 +601,7 @@ __global__ void __launch_bounds__(32 * RG * KG) bwd_dq_kernel(const jvpfa_bwd_ar
           }
         }
       }
-      gemm_out<T, D, LW, true, HAS_GT>(dq, f, e_, sK, sTK, LD, lane);  // gS K + gtS tK
+      gemm_out<T, D, LW, true, TKV>(dq, f, e_, sK, sTK, LD, lane);  // gS K + gtS tK
     }
     __syncthreads();
   }
@@ -605,15 +614,15 @@ __global__ void __launch_bounds__(32 * RG * KG) bwd_dq_kernel(const jvpfa_bwd_ar
   smem_tile_to_global<T, BM, D, NT>(reinterpret_cast<T*>(a.dq) + head_off, sQ, LD, m0, L, tid);
 }
 
-template <typename T, int D, bool HAS_GO, bool HAS_GT, int RG, int KG>
+template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
 static int launch_bwd_one(const jvpfa_bwd_args& a, cudaStream_t stream) {
   using C = BwdCfg<T, D, RG, KG>;
-  constexpr int go = HAS_GO ? 1 : 0, gt = HAS_GT ? 1 : 0;
-  constexpr size_t smem_kv = C::smem(gt ? 4 : 2, 1 + go + 2 * gt, true);
-  constexpr size_t smem_q = C::smem(1 + go + 2 * gt, gt ? 4 : 2, false);
+  constexpr int keys = TKV ? 4 : 2, queries = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0);  // tiles of each side
+  constexpr size_t smem_kv = C::smem(keys, queries, true);
+  constexpr size_t smem_q = C::smem(queries, keys, false);
   static_assert(smem_kv <= 227 * 1024 && smem_q <= 227 * 1024, "shared memory of one CTA");
-  auto k1 = bwd_dkdv_kernel<T, D, HAS_GO, HAS_GT, RG, KG>;
-  auto k2 = bwd_dq_kernel<T, D, HAS_GO, HAS_GT, RG, KG>;
+  auto k1 = bwd_dkdv_kernel<T, D, HAS_GO, HAS_GT, TKV, RG, KG>;
+  auto k2 = bwd_dq_kernel<T, D, HAS_GO, HAS_GT, TKV, RG, KG>;
   static SmemOptIn opt_in1, opt_in2;
   if (!opt_in1.ensure(reinterpret_cast<const void*>(k1), smem_kv) || !opt_in2.ensure(reinterpret_cast<const void*>(k2), smem_q))
     return JVPFA_ERR_CUDA;
@@ -631,9 +640,11 @@ static int launch_bwd_one(const jvpfa_bwd_args& a, cudaStream_t stream) {
 template <typename T, int D, int RG, int KG>
 static int launch_bwd_split(const jvpfa_bwd_args& a, cudaStream_t s) {
   const bool go = a.go != nullptr, gt = a.gto != nullptr;
-  if (go && gt) return launch_bwd_one<T, D, true, true, RG, KG>(a, s);
-  if (gt) return launch_bwd_one<T, D, false, true, RG, KG>(a, s);
-  return launch_bwd_one<T, D, true, false, RG, KG>(a, s);
+  if (go && gt) return launch_bwd_one<T, D, true, true, true, RG, KG>(a, s);
+  if constexpr (std::is_same_v<T, float>)  // (the only type the flag is accepted for, and without gO)
+    if (a.flags & JVPFA_ZERO_TKV) return launch_bwd_one<T, D, false, true, false, RG, KG>(a, s);
+  if (gt) return launch_bwd_one<T, D, false, true, true, RG, KG>(a, s);
+  return launch_bwd_one<T, D, true, false, false, RG, KG>(a, s);
 }
 
 // Rows x loop parts of a CTA, by the same rule as in the forward.
@@ -668,7 +679,7 @@ int launch_bwd_generic(const jvpfa_bwd_args& a, cudaStream_t s) {
     case JVPFA_FP16:
       return launch_bwd_t<__half>(a, s);
     case JVPFA_FP32:
-      return launch_bwd_fp32(a, s);
+      return launch_bwd_t<float>(a, s);
     case JVPFA_FP32_TF32:
       return launch_bwd_t<tf32x1>(a, s);
     default:

@@ -1,7 +1,7 @@
 // Shared device helpers for the register-tiled (mma.sync) attention kernels:
-// warp-level MMA fragments for bf16 / fp16 (m16n8k16) and single-pass TF32 (m16n8k8),
-// cp.async tile staging, and the mask / bias accessor used inside every tile loop.
-// (fp32 at full precision: fp32_split.cuh.)
+// warp-level MMA fragments for bf16 / fp16 (m16n8k16) and fp32 (m16n8k8 TF32 issued
+// three times on a hi/lo split, "3xTF32"), cp.async tile staging, and the mask /
+// bias accessor used inside every tile loop.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -50,7 +50,12 @@ struct Elem<__half> {
 
 template <>
 struct Elem<float> {
+  static constexpr bool k16 = false;
+  static constexpr bool kSplit = true;  // every product is three TF32 MMAs on a hi/lo split
+  static constexpr int kPad = 4;
+  static constexpr int kKStep = 8;
   __device__ static __forceinline__ float to_float(float x) { return x; }
+  __device__ static __forceinline__ float from_float(float x) { return x; }
 };
 
 // fp32 in memory, products as one TF32 MMA (JVPFA_FP32_TF32): the precision of upstream's fp32 path, whose
@@ -61,6 +66,7 @@ struct tf32x1 {
 template <>
 struct Elem<tf32x1> {
   static constexpr bool k16 = false;
+  static constexpr bool kSplit = false;
   static constexpr int kPad = 4;
   static constexpr int kKStep = 8;
   __device__ static __forceinline__ float to_float(tf32x1 x) { return x.v; }
@@ -101,22 +107,60 @@ struct IntC {  // a compile-time int as an argument
   __host__ __device__ constexpr int operator()() const { return I; }
 };
 
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
+// Split an fp32 value into a TF32 "hi" part (11 significant bits) and the TF32 rounding of the remainder.  Dekker's
+// splitting (T. J. Dekker, "A floating-point technique for extending the available precision", Numer. Math. 18, 1971)
+// rounds hi on the FMA pipe, here at 2^-14 of x's magnitude: his factor of 2^13 + 1 would overflow from 2^115 on, where an
+// entry must stay itself.  A tensor core ignores the low 13 bits of a TF32 operand, so half a unit of the last used bit,
+// added as an integer, rounds lo.  A NaN stays one in hi.  Two cvt.rna.tf32 instead cost more issue slots than all the
+// rest of a fragment (D = 128, B2 H8 L1024 with bias, primal + tangent forward: 900 us with them and the bias fetched
+// behind the products, 683 us without either).
+//
+// Every entry has an exponent of its own, hence 22 significant bits whatever else its row or column holds, and an Inf or a
+// NaN reaches only the results that it belongs to.  Pairs of fp16 numbers with one exponent for a row multiply at twice the
+// rate, but leave an entry 40 bits below its row's largest nothing: one V entry of 1e8 cost the other columns of those keys
+// 4e-5, one of 1e15 or Inf the keys themselves.
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
+  constexpr float kDown = 0x1p-14f;
+  const float c = __fmul_rn(x, 8193.f * kDown);  // 2^13 + 1
+  const float h = __fmul_rn(__fsub_rn(c, __fmaf_rn(x, -kDown, c)), 1.f / kDown);
+  hi = __float_as_uint(h);
+  lo = __float_as_uint(__fsub_rn(x, h)) + 0x1000u;
+}
+// The same for element type T: types that multiply in one pass have no lo part.
+template <typename T>
+__device__ __forceinline__ void split_t(float x, uint32_t& hi, uint32_t& lo) {
+  if constexpr (Elem<T>::kSplit) {
+    split_tf32(x, hi, lo);
+  } else {
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+    lo = 0u;
+  }
 }
 
 // ----------------------------------------------------------------------------------------------
-// Fragments: the packed register set of m16n8k16 (16-bit types) or m16n8k8 (TF32).
+// Fragments.  For 16-bit types a fragment is the packed register set of m16n8k16; for fp32 it
+// carries the hi and lo TF32 halves so that one logical MMA is lo*hi + hi*lo + hi*hi.
 // ----------------------------------------------------------------------------------------------
 template <typename T, bool k16 = Elem<T>::k16>
-struct FragA {
+struct FragA;
+template <typename T, bool k16 = Elem<T>::k16>
+struct FragB;
+
+template <typename T>
+struct FragA<T, true> {
   uint32_t r[4];
 };
-template <typename T, bool k16 = Elem<T>::k16>
-struct FragB {
+template <typename T>
+struct FragB<T, true> {
   uint32_t r[2];
+};
+template <typename T>
+struct FragA<T, false> {
+  uint32_t hi[4], lo[4];
+};
+template <typename T>
+struct FragB<T, false> {
+  uint32_t hi[2], lo[2];
 };
 
 template <typename T>
@@ -125,7 +169,26 @@ __device__ __forceinline__ void mma(float c[4], const FragA<T, true>& a, const F
 }
 template <typename T>
 __device__ __forceinline__ void mma(float c[4], const FragA<T, false>& a, const FragB<T, false>& b) {
-  mma_1688_tf32(c, a.r, b.r);
+  if constexpr (Elem<T>::kSplit) {
+    mma_1688_tf32(c, a.lo, b.hi);
+    mma_1688_tf32(c, a.hi, b.lo);
+  }
+  mma_1688_tf32(c, a.hi, b.hi);
+}
+
+// One of the up to three instructions of a logical MMA: 0 = lo*hi, 1 = hi*lo, 2 = hi*hi (types that multiply in one pass
+// have the last only).  Accumulators that take several products interleave the passes of all of them: an instruction
+// returns after 21 cycles, and the next one on the same accumulator should be three issue slots (of 8 cycles) away.
+template <int PASS, typename T>
+__device__ __forceinline__ void mma_pass(float c[4], const FragA<T, true>& a, const FragB<T, true>& b) {
+  if constexpr (PASS == 2) mma_16816(static_cast<const T*>(nullptr), c, a.r, b.r);
+}
+template <int PASS, typename T>
+__device__ __forceinline__ void mma_pass(float c[4], const FragA<T, false>& a, const FragB<T, false>& b) {
+  if constexpr (PASS == 2)
+    mma_1688_tf32(c, a.hi, b.hi);
+  else if constexpr (Elem<T>::kSplit)
+    mma_1688_tf32(c, PASS == 0 ? a.lo : a.hi, PASS == 0 ? b.hi : b.lo);
 }
 
 // A fragment from a row-major smem tile s[row][k] (k contiguous, leading dimension ld elements):
@@ -145,10 +208,10 @@ __device__ __forceinline__ void load_a(FragA<T, false>& f, const T* s, int ld, i
   const int g = lane >> 2, t = lane & 3;
   const float* p0 = reinterpret_cast<const float*>(s) + (r0 + g) * ld + k0 + t;
   const float* p1 = p0 + 8 * ld;
-  f.r[0] = to_tf32(p0[0]);
-  f.r[1] = to_tf32(p1[0]);
-  f.r[2] = to_tf32(p0[4]);
-  f.r[3] = to_tf32(p1[4]);
+  split_t<T>(p0[0], f.hi[0], f.lo[0]);
+  split_t<T>(p1[0], f.hi[1], f.lo[1]);
+  split_t<T>(p0[4], f.hi[2], f.lo[2]);
+  split_t<T>(p1[4], f.hi[3], f.lo[3]);
 }
 
 // B fragment, "NT": the smem tile is s[n][k] with k contiguous (C = A * s^T).
@@ -163,13 +226,13 @@ template <typename T>
 __device__ __forceinline__ void load_b_nt(FragB<T, false>& f, const T* s, int ld, int n0, int k0, int lane) {
   const int g = lane >> 2, t = lane & 3;
   const float* p = reinterpret_cast<const float*>(s) + (n0 + g) * ld + k0 + t;
-  f.r[0] = to_tf32(p[0]);
-  f.r[1] = to_tf32(p[4]);
+  split_t<T>(p[0], f.hi[0], f.lo[0]);
+  split_t<T>(p[4], f.hi[1], f.lo[1]);
 }
 
 // B fragment, "NN": the smem tile is s[k][n] with n contiguous (C = A * s).
 // 16-bit: slot pairs (2t,2t+1) and (2t+8,2t+9) are two consecutive rows of s.
-// TF32: the A operand of these products comes straight from an accumulator tile whose
+// fp32: the A operand of these products comes straight from an accumulator tile whose
 // columns (2t, 2t+1) sit in MMA k-slots (t, t+4) (see a_from_acc); the same permutation
 // of the contraction index is applied here, so slot t reads row k0+2t and slot t+4 reads
 // row k0+2t+1.
@@ -184,8 +247,8 @@ template <typename T>
 __device__ __forceinline__ void load_b_nn(FragB<T, false>& f, const T* s, int ld, int k0, int n0, int lane) {
   const int g = lane >> 2, t = lane & 3;
   const float* p = reinterpret_cast<const float*>(s) + (k0 + 2 * t) * ld + n0 + g;
-  f.r[0] = to_tf32(p[0]);
-  f.r[1] = to_tf32(p[ld]);
+  split_t<T>(p[0], f.hi[0], f.lo[0]);
+  split_t<T>(p[ld], f.hi[1], f.lo[1]);
 }
 
 // A fragment taken from an accumulator-layout tile acc[n_tile][4] (16 rows x 8*n_tiles cols),
@@ -202,10 +265,10 @@ __device__ __forceinline__ void a_from_acc(FragA<T, true>& f, const float (*acc)
 template <typename T>
 __device__ __forceinline__ void a_from_acc(FragA<T, false>& f, const float (*acc)[4], int kk) {
   const float* c = acc[kk];
-  f.r[0] = to_tf32(c[0]);  // slot t    <- column 2t,   row g
-  f.r[1] = to_tf32(c[2]);  // slot t    <- column 2t,   row g+8
-  f.r[2] = to_tf32(c[1]);  // slot t+4  <- column 2t+1, row g
-  f.r[3] = to_tf32(c[3]);  // slot t+4  <- column 2t+1, row g+8
+  split_t<T>(c[0], f.hi[0], f.lo[0]);  // slot t    <- column 2t,   row g
+  split_t<T>(c[2], f.hi[1], f.lo[1]);  // slot t    <- column 2t,   row g+8
+  split_t<T>(c[1], f.hi[2], f.lo[2]);  // slot t+4  <- column 2t+1, row g
+  split_t<T>(c[3], f.hi[3], f.lo[3]);  // slot t+4  <- column 2t+1, row g+8
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -378,8 +441,6 @@ struct SmemOptIn {
 
 // Host-side launch helpers implemented by each kernel translation unit.
 int launch_fwd_generic(const jvpfa_fwd_args& a, cudaStream_t stream);
-int launch_fwd_fp32(const jvpfa_fwd_args& a, cudaStream_t stream);
-int launch_bwd_fp32(const jvpfa_bwd_args& a, cudaStream_t stream);
 int launch_pre(const jvpfa_pre_args& a, cudaStream_t stream);
 int launch_bwd_generic(const jvpfa_bwd_args& a, cudaStream_t stream);
 int launch_mask_check(const jvpfa_mask_check_args& a, cudaStream_t stream);

@@ -13,13 +13,13 @@
 // is applied as scale*QK^T + bias (SDPA semantics; upstream scales the bias too,
 // jvp_attention.py:247-251), and boolean masking uses -inf rather than adding -100.
 //
-// It serves what the tcgen05 kernels do not take (16-bit: short or oddly laid out requests) and fp32 inputs multiplied in
-// one TF32 pass (JVPFA_FP32_TF32); fp32 at full precision: fwd_fp32.cu.
-// What bounds it: mma.sync, at 512 (TF32) or 1024 (16-bit) multiply-adds per clock and SM, measured.  One instruction
-// occupies its quarter of the SM for 8 cycles and returns after 21, so the split matters: 64 rows x D=128 of 4-byte
-// elements fill the shared memory of an SM, and with one warp for each 16 rows (KG = 1) a quarter had a single warp to wait
-// for.  With KG = 2 it has two, and shapes with few row tiles use shorter ones with more key parts (see launch_d) instead
-// of leaving SMs idle.
+// What bounds it: mma.sync, at 512 (TF32) or 1024 (16-bit) multiply-adds per clock and SM, measured; an fp32 product is
+// three TF32 instructions.  One instruction occupies its quarter of the SM for 8 cycles and returns after 21, and the
+// fp32 products of one accumulator are a chain, so the split matters: 64 rows x D=128 fp32 fill the shared memory of an
+// SM, and with one warp for each 16 rows (KG = 1) a quarter had a single warp to wait for.  With KG = 2 it has two, and
+// shapes with few row tiles use shorter ones with more key parts (see launch_d) instead of leaving SMs idle.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace jvpfa {
@@ -33,31 +33,32 @@ struct FwdCfg {
   static constexpr int BW = BN / KG;
   static constexpr int LD = D + Elem<T>::kPad;
   static constexpr int STAGES = (!Elem<T>::k16 && D > 64 && BN > 32) ? 1 : 2;
-  static constexpr size_t tiles(bool dual) {
-    const size_t ring = sizeof(T) * (size_t)STAGES * BN * LD * (dual ? 4 : 2);
+  static constexpr size_t tiles(bool dual, bool tkv) {
+    const size_t ring = sizeof(T) * (size_t)STAGES * BN * LD * (tkv ? 4 : 2);
     const size_t merge = sizeof(float) * (size_t)(RG * KG / 2) * 16 * D * (dual ? 2 : 1);  // reuses the ring
     return ring > merge ? ring : merge;
   }
-  static constexpr size_t smem(bool dual) {
-    return sizeof(T) * (size_t)BM * LD * (dual ? 2 : 1) + tiles(dual) + sizeof(float) * 3 * KG * BM;
+  static constexpr size_t smem(bool dual, bool tkv) {
+    return sizeof(T) * (size_t)BM * LD * (dual ? 2 : 1) + tiles(dual, tkv) + sizeof(float) * 3 * KG * BM;
   }
 };
 
-template <typename T, int D, bool DUAL, int RG, int KG>
+// TKV: K and V have tangents (JVPFA_ZERO_TKV leaves them, and two of the six products, out).
+template <typename T, int D, bool DUAL, bool TKV, int RG, int KG>
 __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_fwd_args a) {
   using C = FwdCfg<T, D, RG, KG>;
   constexpr int BM = C::BM, BN = C::BN, BW = C::BW, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES;
   constexpr int KS = Elem<T>::kKStep;
   constexpr int NS = BW / 8;   // score n-tiles per warp row-strip
   constexpr int ND = D / 8;    // output n-tiles
-  constexpr int NKV = DUAL ? 4 : 2;
+  constexpr int NKV = TKV ? 4 : 2;
   static_assert(BW % KS == 0, "a warp's keys are whole contraction steps");
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sQ = reinterpret_cast<T*>(smem_raw);
   T* sTQ = sQ + BM * LD;  // only valid when DUAL
   T* sKV = sQ + BM * LD * (DUAL ? 2 : 1);
-  float* sRow = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(sKV) + C::tiles(DUAL));  // [3][KG][BM]
+  float* sRow = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(sKV) + C::tiles(DUAL, TKV));  // [3][KG][BM]
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rg = warp % RG, kg = warp / RG;
@@ -78,8 +79,8 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
   const T* gK = reinterpret_cast<const T*>(a.k) + in_off;
   const T* gV = reinterpret_cast<const T*>(a.v) + in_off;
   const T* gTQ = DUAL ? reinterpret_cast<const T*>(a.tq) + in_off : nullptr;
-  const T* gTK = DUAL ? reinterpret_cast<const T*>(a.tk) + in_off : nullptr;
-  const T* gTV = DUAL ? reinterpret_cast<const T*>(a.tv) + in_off : nullptr;
+  const T* gTK = TKV ? reinterpret_cast<const T*>(a.tk) + in_off : nullptr;
+  const T* gTV = TKV ? reinterpret_cast<const T*>(a.tv) + in_off : nullptr;
 
   const MaskView mv = make_mask_view(a.mask, b, h, L);
 
@@ -92,7 +93,7 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
     T* base = sKV + (size_t)stage * NKV * BN * LD;
     stage_tile<T, BN, D, NT>(base, gK, n0, L, tid, in_rs);
     stage_tile<T, BN, D, NT>(base + BN * LD, gV, n0, L, tid, in_rs);
-    if constexpr (DUAL) {
+    if constexpr (TKV) {
       stage_tile<T, BN, D, NT>(base + 2 * BN * LD, gTK, n0, L, tid, in_rs);
       stage_tile<T, BN, D, NT>(base + 3 * BN * LD, gTV, n0, L, tid, in_rs);
     }
@@ -174,21 +175,24 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
       FragA<T> fq, ftq;
       load_a<T>(fq, sQ, LD, r0, k0, lane);
       if constexpr (DUAL) load_a<T>(ftq, sTQ, LD, r0, k0, lane);
-      FragB<T> fk[NS], ftk[DUAL ? NS : 1];
+      FragB<T> fk[NS], ftk[TKV ? NS : 1];
 #pragma unroll
       for (int nt = 0; nt < NS; ++nt) {
         load_b_nt<T>(fk[nt], sK, LD, nt * 8, k0, lane);
-        if constexpr (DUAL) load_b_nt<T>(ftk[nt], sTK, LD, nt * 8, k0, lane);
+        if constexpr (TKV) load_b_nt<T>(ftk[nt], sTK, LD, nt * 8, k0, lane);
       }
+      auto pass = [&](auto P) {
 #pragma unroll
-      for (int nt = 0; nt < NS; ++nt) {
-        mma<T>(s[nt], fq, fk[nt]);
-        if constexpr (DUAL) mma<T>(ts[nt], ftq, fk[nt]);
-      }
-      if constexpr (DUAL) {
+        for (int nt = 0; nt < NS; ++nt) {
+          mma_pass<P()>(s[nt], fq, fk[nt]);
+          if constexpr (DUAL) mma_pass<P()>(ts[nt], ftq, fk[nt]);
+        }
+        if constexpr (TKV) {
 #pragma unroll
-        for (int nt = 0; nt < NS; ++nt) mma<T>(ts[nt], fq, ftk[nt]);
-      }
+          for (int nt = 0; nt < NS; ++nt) mma_pass<P()>(ts[nt], fq, ftk[nt]);
+        }
+      };
+      pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
     }
 
     // ---- mask / bias, move to the base-2 domain ----
@@ -258,7 +262,7 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
     }
 
     // ---- second MMAs: contraction over the keys of this tile ----
-    // TF32: the tensor core adds into its fp32 accumulator with truncation; over a thousand keys that bias reaches
+    // fp32: the tensor core adds into its fp32 accumulator with truncation; over a thousand keys that bias reaches
     // ~1e-5.  Each contraction step is therefore formed in fresh registers and added to the running sums rounded.
 #pragma unroll
     for (int kk = 0; kk < BW / KS; ++kk) {
@@ -268,27 +272,30 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
       constexpr int G = 2;  // output tiles at a time
 #pragma unroll
       for (int d0 = 0; d0 < ND; d0 += G) {
-        FragB<T> fv[G], ftv[DUAL ? G : 1];
+        FragB<T> fv[G], ftv[TKV ? G : 1];
         float xo[G][4], xt[DUAL ? G : 1][4];
 #pragma unroll
         for (int i = 0; i < G; ++i) {
           load_b_nn<T>(fv[i], sV, LD, kk * KS, (d0 + i) * 8, lane);
-          if constexpr (DUAL) load_b_nn<T>(ftv[i], sTV, LD, kk * KS, (d0 + i) * 8, lane);
+          if constexpr (TKV) load_b_nn<T>(ftv[i], sTV, LD, kk * KS, (d0 + i) * 8, lane);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             xo[i][e] = Elem<T>::k16 ? acc_o[d0 + i][e] : 0.f;
             if constexpr (DUAL) xt[i][e] = Elem<T>::k16 ? acc_t[d0 + i][e] : 0.f;
           }
         }
+        auto pass = [&](auto P) {
 #pragma unroll
-        for (int i = 0; i < G; ++i) {
-          mma<T>(xo[i], fp, fv[i]);
-          if constexpr (DUAL) mma<T>(xt[i], fw, fv[i]);
-        }
-        if constexpr (DUAL) {
+          for (int i = 0; i < G; ++i) {
+            mma_pass<P()>(xo[i], fp, fv[i]);
+            if constexpr (DUAL) mma_pass<P()>(xt[i], fw, fv[i]);
+          }
+          if constexpr (TKV) {
 #pragma unroll
-          for (int i = 0; i < G; ++i) mma<T>(xt[i], fp, ftv[i]);
-        }
+            for (int i = 0; i < G; ++i) mma_pass<P()>(xt[i], fp, ftv[i]);
+          }
+        };
+        pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
 #pragma unroll
         for (int i = 0; i < G; ++i) {
 #pragma unroll
@@ -401,12 +408,12 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
   }
 }
 
-template <typename T, int D, bool DUAL, int RG, int KG>
+template <typename T, int D, bool DUAL, bool TKV, int RG, int KG>
 static int launch_one(const jvpfa_fwd_args& a, cudaStream_t stream) {
   using C = FwdCfg<T, D, RG, KG>;
-  constexpr size_t smem = C::smem(DUAL);
+  constexpr size_t smem = C::smem(DUAL, TKV);
   static_assert(smem <= 227 * 1024, "shared memory of one CTA");
-  auto kern = fwd_generic_kernel<T, D, DUAL, RG, KG>;
+  auto kern = fwd_generic_kernel<T, D, DUAL, TKV, RG, KG>;
   static SmemOptIn opt_in;
   if (!opt_in.ensure(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_CUDA;
   dim3 grid((a.L + C::BM - 1) / C::BM, a.B * a.H);
@@ -419,16 +426,24 @@ static int launch_one(const jvpfa_fwd_args& a, cudaStream_t stream) {
   return JVPFA_OK;
 }
 
+template <typename T, int D, int RG, int KG>
+static int launch_split(const jvpfa_fwd_args& a, cudaStream_t s) {
+  if (!a.tq) return launch_one<T, D, false, false, RG, KG>(a, s);
+  if constexpr (std::is_same_v<T, float>)  // (the only type the flag is accepted for)
+    if (a.flags & JVPFA_ZERO_TKV) return launch_one<T, D, true, false, RG, KG>(a, s);
+  return launch_one<T, D, true, true, RG, KG>(a, s);
+}
+
 // Rows x key parts of a CTA.  64 rows share every key tile that is brought in, so they are the choice once they give
 // each of the 148 SMs a CTA; below that shorter row tiles (whose warps share out the keys) put more SMs to work.
 template <typename T, int D>
 static int launch_d(const jvpfa_fwd_args& a, cudaStream_t s) {
   if constexpr (!Elem<T>::k16) {
     const long long rows16 = (long long)((a.L + 15) / 16) * a.B * a.H;
-    if (rows16 < 2 * 148) return a.tq ? launch_one<T, D, true, 1, 8>(a, s) : launch_one<T, D, false, 1, 8>(a, s);
-    if (rows16 < 4 * 148) return a.tq ? launch_one<T, D, true, 2, 4>(a, s) : launch_one<T, D, false, 2, 4>(a, s);
+    if (rows16 < 2 * 148) return launch_split<T, D, 1, 8>(a, s);
+    if (rows16 < 4 * 148) return launch_split<T, D, 2, 4>(a, s);
   }
-  return a.tq ? launch_one<T, D, true, 4, 2>(a, s) : launch_one<T, D, false, 4, 2>(a, s);
+  return launch_split<T, D, 4, 2>(a, s);
 }
 
 template <typename T>
@@ -452,7 +467,7 @@ int launch_fwd_generic(const jvpfa_fwd_args& a, cudaStream_t s) {
     case JVPFA_FP16:
       return launch_t<__half>(a, s);
     case JVPFA_FP32:
-      return launch_fwd_fp32(a, s);
+      return launch_t<float>(a, s);
     case JVPFA_FP32_TF32:
       return launch_t<tf32x1>(a, s);
     default:

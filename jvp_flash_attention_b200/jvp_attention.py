@@ -104,8 +104,7 @@ def _require_cuda(*ts: Tensor) -> None:
 def set_fp32_precision(mode: str) -> str:
     """How fp32 inputs are multiplied from now on; returns the previous mode.
 
-    ``"3xtf32"`` (default): every product as three tensor-core MMAs on a hi/lo split, 22 significant bits
-    an operand, about 1e-6 relative error.
+    ``"3xtf32"`` (default): every product as three TF32 MMAs on a hi/lo split, about 1e-6 relative error.
     ``"tf32"``: one TF32 MMA per product, about 5e-4 -- what upstream's fp32 path computes (its ``tl.dot`` calls
     run on TF32 tensor cores, jvp_attention.py:233-236; its fp32 tolerance is 2.35e-2), about 2.5x faster.
     A call's backward (and double backward) runs at the precision its forward ran at: the mode is recorded with the

@@ -37,7 +37,7 @@ def _mask(kind, B, H, L, dtype, seed):
 
 def _check(B, H, L, D, dt, kind, cot, seed=0):
     """O, tO and the gradients through the asked-for outputs against the float64 oracle: 1e-5 of the largest entry for
-    fp32 (three TF32 products), 2e-2 (scaled with the gradients' magnitude) for 16 bits, as in the parity tests."""
+    fp32 (every product as three, on TF32 pairs), 2e-2 (scaled with the gradients' magnitude) for 16 bits, as in the parity tests."""
     dtype = DT[dt]
     q, k, v, tq, tk, tv, go, gt = _inputs(B, H, L, D, dtype, seed + L + D)
     mask, causal = _mask(kind, B, H, L, dtype, seed + 1), kind == "causal"
@@ -148,10 +148,9 @@ def test_a_mask_written_behind_the_version_counter_is_read_as_it_is(kind, L, D, 
 @pytest.mark.parametrize("D", [32, 64, 128])
 @pytest.mark.parametrize("B,H,L", [(1, 2, 34), (2, 10, 250), (2, 12, 450)])
 def test_fp32_rows_of_very_different_magnitude(B, H, L, D):
-    """A pair of fp16 numbers carries 22 bits of an entry relative to its own row only: rows of V and its tangent up to a
-    factor of 2^40 apart, and masked-out keys that hold 1e15, must cost no precision.  Every product is within 2^-21 of its
-    operands' magnitudes; a gradient passes three in a row and sums a few hundred terms: 1e-5 of P |V| for O, of the head's
-    largest V for tO, of the head's largest entry for a gradient."""
+    """Rows of V and its tangent up to a factor of 2^40 apart, and masked-out keys that hold 1e15, must cost no precision.
+    Every product is within 2^-21 of its operands' magnitudes; a gradient passes three in a row and sums a few hundred
+    terms: 1e-5 of P |V| for O, of the head's largest V for tO, of the head's largest entry for a gradient."""
     q, k, v, tq, tk, tv, go, gt = _inputs(B, H, L, D, torch.float32, L + D)
     g = torch.Generator().manual_seed(L)
     vscale = torch.exp2(torch.randint(-20, 21, (B, H, L, 1), generator=g).float())
@@ -176,6 +175,51 @@ def test_fp32_rows_of_very_different_magnitude(B, H, L, D):
         top = weight if name == "O" else head(clean[1]) if name == "tO" else head(r)
         off = ((x - r.double()).abs() / top.clamp(min=1e-30)).max().item()
         assert off <= 1e-5, (name, off)
+
+
+def _grads_fp32(a, tangents, go, gt):
+    a = [x.to(DEV).requires_grad_() for x in a]
+    o, to = torch.func.jvp(ja.JVPAttn.fwd_dual, tuple(a), tuple(x.to(DEV) for x in tangents))
+    return (o, to, *torch.autograd.grad((o, to), a, (go.to(DEV), gt.to(DEV))))
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("B,H,L", [(1, 2, 34), (2, 10, 250), (2, 12, 450)])
+@pytest.mark.parametrize("big", [1e8, 1e15, 1e36, float("inf"), float("nan")])
+def test_fp32_a_large_entry_costs_the_others_nothing(D, B, H, L, big):
+    """One entry of V (of gO for dV) that is very large, Inf or NaN: the other columns are what they are without it.  Every
+    product is within 2^-21 of its own operands and a column sums a few hundred: 1e-5 of P |V| (of P^T |gO|) there."""
+    q, k, v, tq, tk, tv, go, gt = _inputs(B, H, L, D, torch.float32, L + D)
+    v[:, :, L // 2, 5] = big
+    o, to, *_ = _grads_fp32((q, k, v), (tq, tk, tv), go, gt)
+    rest = [c for c in range(D) if c != 5]
+    p = torch.softmax(q.double() @ k.double().transpose(-1, -2) * D**-0.5, -1)
+    ts = (tq.double() @ k.double().transpose(-1, -2) + q.double() @ tk.double().transpose(-1, -2)) * D**-0.5
+    w = p * (ts - (p * ts).sum(-1, keepdim=True))
+    vd, tvd = v.double()[..., rest], tv.double()[..., rest]
+    for x, r, top in ((o, p @ vd, p @ vd.abs()), (to, w @ vd + p @ tvd, (p * ts.abs().amax(-1, keepdim=True)) @ vd.abs() + p @ tvd.abs())):
+        assert ((x.detach().cpu().double()[..., rest] - r).abs() / top).max().item() <= 1e-5
+        assert big < 1e30 or not torch.isfinite(x[..., 5]).any() or big == 1e36
+    v[:, :, L // 2, 5] = 1.0
+    go[:, :, L // 3, 5] = big
+    dv = _grads_fp32((q, k, v), (tq, tk, tv), go, torch.zeros_like(gt))[4].cpu().double()[..., rest]
+    pt, god = p.transpose(-1, -2), go.double()[..., rest]
+    assert ((dv - pt @ god).abs() / (pt @ god.abs())).max().item() <= 1e-5
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("B,H,L", [(1, 2, 34), (2, 10, 250), (2, 12, 450)])
+def test_fp32_channels_of_very_different_magnitude(D, B, H, L):
+    """One channel of q and its tangent scaled by 1e6 and of k by 1e-6, another the other way round: the scores are those of
+    the unscaled tensors, and so are the results but for the scales.  1e-5 of the largest entry, as in the rest of this file."""
+    q, k, v, tq, tk, tv, go, gt = _inputs(B, H, L, D, torch.float32, L + D)
+    s = torch.ones(D)
+    s[1], s[2] = 1e6, 1e-6
+    ref = orc.grads_through_both(q * s, k / s, v, tq * s, tk / s, tv, go, gt)
+    got = _grads_fp32((q * s, k / s, v), (tq * s, tk / s, tv), go, gt)
+    for name, x, r, scale in zip(("O", "tO", "dq", "dk", "dv"), got, ref, (1.0, 1.0, s, 1 / s, 1.0)):
+        x, r = x.detach().cpu().double() * scale, r.double() * scale
+        assert ((x - r).abs().max() / r.abs().max()).item() <= 1e-5, name
 
 
 @pytest.mark.parametrize("D", [32, 64, 128])
