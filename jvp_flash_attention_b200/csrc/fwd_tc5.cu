@@ -141,7 +141,20 @@ bool tc5_mask_layout(const jvpfa_mask& m, int dtype, int L) {
   return (L & 15) == 0 || (m.stride[2] * esz >= ((L * esz + 15) & ~15ll));
 }
 
-int launch_fwd_tc5(const jvpfa_fwd_args& a, cudaStream_t s) {
+// With the exact running maximum as its reference a row's largest probability is 1, which 16 bits hold without rounding;
+// with a reference up to 2^8 below it (lazy rescaling) it is rounded like the others.  At a few hundred keys that is a part
+// of the error that shows: O against 64 bits, B2 H4 D32, L512 fp16 with bias 2.56e-4 -> 2.90e-4, L1000 bf16 2.21e-3 ->
+// 2.33e-3.  What the register-tiled kernels (exact) served before these kernels could, keeps their error: head dimension
+// 32, and masks and bias that cannot be read in place as whole 16-byte pieces of rows.
+static bool exact_row_max(const jvpfa_fwd_args& a) {
+  if (a.D == 32) return true;
+  const bool by_element = a.mask.kind == JVPFA_MASK_BOOL || a.mask.kind == JVPFA_MASK_BIAS;
+  return by_element && ((a.L & 15) != 0 || !tc5_mask_layout(a.mask, a.dtype, a.L));
+}
+
+int launch_fwd_tc5(const jvpfa_fwd_args& args, cudaStream_t s) {
+  jvpfa_fwd_args a = args;
+  if (exact_row_max(a)) a.flags |= tc5::kExactRowMax;
   if (a.D <= 64) return launch_fwd_tc5_pair64(a, s);
   return launch_fwd_tc5_pipe128(a, s);
 }

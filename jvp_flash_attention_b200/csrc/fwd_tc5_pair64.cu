@@ -532,6 +532,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         alive = epilogue(it, i, -INFINITY, 0.f, 0.f, false);
         continue;
       }
+      const float slack = a.flags & kExactRowMax ? 0.f : 8.f;
       float m_used = -INFINITY, l_run = 0.f, mu_run = 0.f;
       // MK != 0: this thread's row of the mask / bias (rows past L are clamped; their results are not stored)
       constexpr bool BOOLM = MK == 1 || MK == 3;
@@ -649,8 +650,8 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
           }
           mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
         }
-        // Lazy running max: keep the old reference while the new maximum is at most 2^8 above it.
-        const bool grow = mx > m_used + 8.f;
+        // Lazy running max: keep the old reference while the new maximum is at most 2^8 above it (kExactRowMax: never).
+        const bool grow = mx > m_used + slack;
         float alpha = 1.f;
         if (grow) {
           alpha = fast_exp2(m_used - mx);

@@ -277,6 +277,7 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
     const float scale_log2 = a.sm_scale * kLog2e;
     const float2 c2 = make_float2(scale_log2, scale_log2);
     const float2 sc2 = make_float2(a.sm_scale, a.sm_scale);
+    const float slack = a.flags & kExactRowMax ? 0.f : 8.f;
     float m_used = -INFINITY, l_run = 0.f, mu_run = 0.f;
     bool alive = true;
 
@@ -392,8 +393,8 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
         }
         mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
       }
-      // Lazy running max: keep the old reference while the new maximum is at most 2^8 above it.
-      const bool grow = mx > m_used + 8.f;
+      // Lazy running max: keep the old reference while the new maximum is at most 2^8 above it (kExactRowMax: never).
+      const bool grow = mx > m_used + slack;
       float alpha = 1.f;
       if (grow) {
         alpha = fast_exp2(m_used - mx);

@@ -102,6 +102,9 @@ __device__ __forceinline__ uint32_t ldg_nc_u16(const void* p) {
   return r;
 }
 
+// In jvpfa_fwd_args.flags of the forward kernels, set by their launch: the running maximum is the reference of every tile.
+constexpr int kExactRowMax = 1 << 30;
+
 // Boolean masks.  A mask packed by jvpfa_mask_tiles is read as words; otherwise its bytes are turned into the same words.
 __device__ __forceinline__ uint2 ldg_nc_v2(const void* p) {
   uint2 r;

@@ -241,3 +241,29 @@ def test_fp32_second_differentiation_along_q_alone(B, H, L, D, kind):
 
     for x, y in zip(second("q"), second("qkv")):
         assert (x - y).abs().max().item() <= 1e-5 * y.abs().max().item()
+
+
+@pytest.mark.parametrize("dt", ["bf16", "fp16"])
+@pytest.mark.parametrize("D,L,kind", [(32, 250, "none"), (32, 256, "bias"), (64, 250, "bool"), (64, 250, "bias"), (128, 250, "bool"),
+                                      (128, 250, "bias")])
+def test_the_largest_probability_of_a_row_is_held_exactly(dt, D, L, kind):
+    """Head dimension 32 and masks with ragged rows: the running maximum is the reference, as on the register-tiled kernels,
+    so a row's largest probability is 1 and not rounded.  Here it outweighs the rest (2^-5.6 at most) and lies in a later tile
+    than a runner-up within the 2^8 that lazy rescaling would leave: all that is left of O's error is its own rounding to 16
+    bits, plus 2^-5.6 of a probability's."""
+    B, H, dtype = 2, 2, DT[dt]
+    g = torch.Generator().manual_seed(D + L)
+    q, k = torch.zeros(B, H, L, D), torch.zeros(B, H, L, D)
+    q[..., 0], q[..., 1] = 1.0, torch.rand(B, H, L, generator=g)
+    unit = D**0.5 * 0.6931471805599453  # one of the softmax's powers of two
+    k[..., 0] = -40 * unit
+    k[:, :, 3, 0], k[:, :, 200, 0], k[:, :, 200, 1] = unit, 7 * unit, unit
+    q, k = q.to(dtype), k.to(dtype)
+    v = torch.randn(B, H, L, D, generator=g).to(dtype)
+    mask = torch.ones(B, 1, L, L, dtype=torch.bool) if kind == "bool" else torch.zeros(B, H, L, L, dtype=dtype)
+    if kind == "bool":
+        mask[:, :, ::2, 5] = False
+    m = None if kind == "none" else mask.to(DEV)
+    o = ja.attention(q.to(DEV), k.to(DEV), v.to(DEV), attn_mask=m).cpu().double()
+    ref = torch.softmax(q.double() @ k.double().transpose(-1, -2) * D**-0.5, -1) @ v.double()
+    assert (o - ref).norm() <= 1.1 * (ref.to(dtype).double() - ref).norm()
