@@ -199,9 +199,9 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       if (!get_item(k, it)) continue;
       const int i = it.own0 + tid;
       if (tid < OWN && i < L) {
-        poison_row<T>(a.dk, (size_t)it.bh * L + i, a.D);
-        poison_row<T>(a.dv, (size_t)it.bh * L + i, a.D);
-        dq_acc[((size_t)it.bh * L + i) * a.D] = poison_f32();
+        poison_row<T>(a.dk, (size_t)it.bh * L + i, D);
+        poison_row<T>(a.dv, (size_t)it.bh * L + i, D);
+        dq_acc[((size_t)it.bh * L + i) * D] = poison_f32();
       }
     }
   };
@@ -364,8 +364,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           else
             umma_ss_lo<true>(tmem + col, a_lo, b_lo, id);
 #pragma unroll
-          for (int ks = 1; ks < D / 16; ++ks)
-            if (ks < 2 || a.D > 32) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 2, id);
+          for (int ks = 1; ks < D / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 2, id);
         };
         for (int k = 0; ok && k < k_max; ++k) {
           if (!get_item(k, it) || it.n_sub == 0) continue;
@@ -499,7 +498,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 
     auto store_row = [&](void* gptr, int bh, int own_idx, const uint32_t (&r0)[32], const uint32_t (&r1)[32], float mul) {
       if (own_idx >= L) return;
-      T* gp = reinterpret_cast<T*>(gptr) + ((size_t)bh * L + own_idx) * a.D;
+      T* gp = reinterpret_cast<T*>(gptr) + ((size_t)bh * L + own_idx) * D;
 #pragma unroll
       for (int x = 0; x < 4; ++x)
         reinterpret_cast<uint4*>(gp)[x] = make_uint4(
@@ -507,7 +506,6 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             Elem<T>::pack(__uint_as_float(r0[8 * x + 2]) * mul, __uint_as_float(r0[8 * x + 3]) * mul),
             Elem<T>::pack(__uint_as_float(r0[8 * x + 4]) * mul, __uint_as_float(r0[8 * x + 5]) * mul),
             Elem<T>::pack(__uint_as_float(r0[8 * x + 6]) * mul, __uint_as_float(r0[8 * x + 7]) * mul));
-      if (a.D <= 32) return;
 #pragma unroll
       for (int x = 0; x < 4; ++x)
         reinterpret_cast<uint4*>(gp)[4 + x] = make_uint4(
@@ -725,7 +723,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
         if (tid == 384) {
           const int i0 = it.loop_begin + s * BL;
           tma_reduce_add_4d(&maps.dq, dqs, 0, i0, it.h, it.b);
-          if (a.D > 32) tma_reduce_add_4d(&maps.dq, dqs + 8192, 32, i0, it.h, it.b);
+          tma_reduce_add_4d(&maps.dq, dqs + 8192, 32, i0, it.h, it.b);
           bulk_commit();
         }
       }
@@ -782,15 +780,15 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
   BwdFMaps m;
   const CUtensorMapDataType dt = Fmt<T>::kTma;
   const int64_t* st = a.in_stride;
-  bool ok = encode_map4d(&m.k, dt, a.k, a.D, a.L, a.H, a.B, st, C::OWN) && encode_map4d(&m.v, dt, a.v, a.D, a.L, a.H, a.B, st, C::OWN) &&
-            encode_map4d(&m.q, dt, a.q, a.D, a.L, a.H, a.B, st, C::BL);
+  bool ok = encode_map4d(&m.k, dt, a.k, C::D, a.L, a.H, a.B, st, C::OWN) && encode_map4d(&m.v, dt, a.v, C::D, a.L, a.H, a.B, st, C::OWN) &&
+            encode_map4d(&m.q, dt, a.q, C::D, a.L, a.H, a.B, st, C::BL);
   m.tk = m.tv = m.k;
   m.go = m.tq = m.g = m.q;
-  if (HAS_GO) ok = ok && encode_map4d(&m.go, dt, a.go, a.D, a.L, a.H, a.B, nullptr, C::BL);
+  if (HAS_GO) ok = ok && encode_map4d(&m.go, dt, a.go, C::D, a.L, a.H, a.B, nullptr, C::BL);
   if (HAS_GT)
-    ok = ok && encode_map4d(&m.tk, dt, a.tk, a.D, a.L, a.H, a.B, st, C::OWN) && encode_map4d(&m.tv, dt, a.tv, a.D, a.L, a.H, a.B, st, C::OWN) &&
-         encode_map4d(&m.tq, dt, a.tq, a.D, a.L, a.H, a.B, st, C::BL) && encode_map4d(&m.g, dt, a.gto, a.D, a.L, a.H, a.B, nullptr, C::BL);
-  ok = ok && encode_map4d_f32(&m.dq, a.dq_accum, a.D, a.L, a.H, a.B, C::BL);
+    ok = ok && encode_map4d(&m.tk, dt, a.tk, C::D, a.L, a.H, a.B, st, C::OWN) && encode_map4d(&m.tv, dt, a.tv, C::D, a.L, a.H, a.B, st, C::OWN) &&
+         encode_map4d(&m.tq, dt, a.tq, C::D, a.L, a.H, a.B, st, C::BL) && encode_map4d(&m.g, dt, a.gto, C::D, a.L, a.H, a.B, nullptr, C::BL);
+  ok = ok && encode_map4d_f32(&m.dq, a.dq_accum, C::D, a.L, a.H, a.B, C::BL);
   if (!ok) {
     set_last_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled(bwd fused64)");
     return JVPFA_ERR_CUDA;
@@ -800,7 +798,7 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
     set_last_cuda_error(cudaErrorUnknown, "multiprocessor count");
     return JVPFA_ERR_CUDA;
   }
-  const size_t n = (size_t)a.B * a.H * a.L * a.D;
+  const size_t n = (size_t)a.B * a.H * a.L * C::D;
   cudaError_t e = cudaSuccess;
   if (!(a.flags & JVPFA_DQ_ACCUM_IS_ZERO)) e = cudaMemsetAsync(a.dq_accum, 0, n * sizeof(float), stream);
   if (e != cudaSuccess) {
@@ -845,18 +843,21 @@ static int launch_fused64_t(const jvpfa_bwd_args& a, cudaStream_t s) {
 
 }  // namespace tc5
 
-// The single-pass kernel serves D = 64 with index masks (none, causal, key padding) and boolean masks that come without
-// tile bitmaps, when the caller provides the fp32 accumulation buffer for dQ.
+// The single-pass kernel serves D = 64 with index masks (none, causal, key padding), boolean masks that come without tile
+// bitmaps, and through O alone a bias of the tensors' type, when the caller provides the fp32 accumulation buffer for dQ.
+// What it sums there in no fixed order, so it takes only what callers know to be summed so: not head dimension 32, nor masks
+// and bias whose rows are not whole 16-byte pieces, which the kernels of a fixed order have always served (B4 H8 L1000 D32,
+// both outputs, a whole step: 209 us with either).
 bool bwd_tc5_fused64_eligible(const jvpfa_bwd_args& a) {
-  if (a.D > 64 || a.dq_accum == nullptr) return false;
+  if (a.D != 64 || a.dq_accum == nullptr) return false;
   if ((reinterpret_cast<uintptr_t>(a.dq_accum) & 15u) != 0) return false;
   const int k = a.mask.kind;
+  if (k == JVPFA_MASK_NONE || k == JVPFA_MASK_CAUSAL || k == JVPFA_MASK_KVLEN) return true;
+  if ((a.L & 15) != 0 || !tc5_mask_layout(a.mask, a.dtype, a.L)) return false;
   // A boolean mask without tile bitmaps (dense, or not looked at beforehand): with them the two-launch kernels, which
   // step over dead tiles, are the better choice.
   if (k == JVPFA_MASK_BOOL) return a.mask_tile_live == nullptr && a.mask_tile_live_t == nullptr;
-  // An additive bias of the tensors' type: only the backward through O alone has the registers for it.
-  if (k == JVPFA_MASK_BIAS) return a.gto == nullptr && a.mask.bias_dtype == a.dtype;
-  return k == JVPFA_MASK_NONE || k == JVPFA_MASK_CAUSAL || k == JVPFA_MASK_KVLEN;
+  return a.gto == nullptr;  // a bias: only the backward through O alone has the registers for it
 }
 
 int launch_bwd_tc5_fused64(const jvpfa_bwd_args& a, cudaStream_t s) {

@@ -248,6 +248,14 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   }
 }
 
+// Whether the mask's own entries can be read as 16-byte pieces of its rows.
+bool whole_pieces(const MaskDesc& m, int64_t L) {
+  const int64_t esz = m.tensor.element_size();
+  bool ok = m.c.stride[3] == 1 && (reinterpret_cast<uintptr_t>(m.c.ptr) & 15u) == 0 && L % 16 == 0;
+  for (int d = 0; d < 3; ++d) ok = ok && m.c.stride[d] * esz % 16 == 0;
+  return ok;
+}
+
 // Fills in the call's forms of its mask.  They are made anew by every call and not kept with the mask's description: what
 // the kernels read is then what the mask holds when they run, also where it was written behind torch's version counter
 // (a replayed graph, a foreign kernel, `.data`).
@@ -263,9 +271,7 @@ void prepare_mask(Call& call, const Tensor& q, bool backward) {
   if (m.c.kind == JVPFA_MASK_BOOL) {
     const int64_t n_b = m.c.stride[0] ? m.tensor.size(0) : 1, n_h = m.c.stride[1] ? m.tensor.size(1) : 1;
     const int64_t n_rows = m.c.stride[2] ? L : 1;
-    bool pieces = m.c.stride[3] == 1 && (reinterpret_cast<uintptr_t>(m.c.ptr) & 15u) == 0 && L % 16 == 0;
-    for (int d = 0; d < 3; ++d) pieces = pieces && m.c.stride[d] % 16 == 0;
-    if (!backward && pieces && 4 * n_b * n_h > q.size(0) * q.size(1)) return;
+    if (!backward && whole_pieces(m, L) && 4 * n_b * n_h > q.size(0) * q.size(1)) return;
     c10::cuda::OptionalCUDAGuard guard;
     if (q.get_device() != c10::cuda::current_device()) guard.set_index(q.get_device());
     const int64_t w = (L + 63) / 64 * 2;
@@ -326,12 +332,14 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   const MaskDesc& m = *call.mask;
   void* stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
 
-  // One scratch allocation: the three row statistics, and fp32 dQ where the single-pass kernels want it (head dimension
-  // up to 64, 16-bit; index masks, a boolean mask without tile bitmaps, or through O alone a bias of the tensors' type).
-  const bool index_mask = m.c.kind == JVPFA_MASK_NONE || m.c.kind == JVPFA_MASK_CAUSAL || m.c.kind == JVPFA_MASK_KVLEN;
-  const bool dense_bool = m.c.kind == JVPFA_MASK_BOOL && !m.tile_live.defined() && !m.tile_live_t.defined();
-  const bool bias_o = m.c.kind == JVPFA_MASK_BIAS && !gto.defined() && m.c.bias_dtype == dtype_of(q, false);
-  const bool single = g_single_pass && !(skip & JVPFA_SKIP_DKDV) && sizes[3] <= 64 && q.scalar_type() != at::kFloat && (index_mask || dense_bool || bias_o);
+  // One scratch allocation: the three row statistics, and fp32 dQ where the single-pass kernel takes it (head dimension 64,
+  // 16-bit; index masks, and as far as rows are whole 16-byte pieces a boolean mask without tile bitmaps or, through O
+  // alone, a bias of the tensors' type).
+  bool single = g_single_pass && !(skip & JVPFA_SKIP_DKDV) && sizes[3] == 64 && q.scalar_type() != at::kFloat;
+  if (m.c.kind == JVPFA_MASK_BOOL)
+    single = single && !m.tile_live.defined() && !m.tile_live_t.defined() && whole_pieces(m, sizes[2]);
+  else if (m.c.kind == JVPFA_MASK_BIAS)
+    single = single && !gto.defined() && m.c.bias_dtype == dtype_of(q, false) && whole_pieces(m, sizes[2]);
   const int64_t stat = (rows + 63) / 64 * 64;  // 256-byte steps
   Tensor scratch = empty({3 * stat + (single ? rows * sizes[3] : 0)}, at::kFloat, q.device());
   float* f = static_cast<float*>(scratch.data_ptr());

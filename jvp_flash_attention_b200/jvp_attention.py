@@ -49,9 +49,10 @@ _UPSTREAM_HEAD_DIMS = {16, 32, 64, 128, 256}
 # Tests flip it to cross-check the two families against each other.
 KERNEL_IMPL = _lib.IMPL_AUTO
 
-# The backward of head-dimension-64 16-bit calls with no / causal / key-padding masks runs as one pass that sums dQ
-# with floating-point reductions (reproducible to rounding).  False: always the two-launch kernels, whose results
-# are bitwise reproducible from run to run.
+# The backward of head-dimension-64 16-bit calls runs as one pass that sums dQ with floating-point reductions (reproducible
+# to rounding) where the mask is none, causal, key padding, or, with rows of whole 16-byte pieces, boolean without dead
+# tiles or (through O alone) a bias of the tensors' type.  False: always the two-launch kernels, whose results are bitwise
+# reproducible from run to run, as those of all other calls are.
 SINGLE_PASS_BACKWARD = True
 
 
@@ -276,7 +277,7 @@ def _launch_bwd(q, k, v, tq, tk, tv, o, to, lse, mu, go, gto, spec: _lib.MaskSpe
     acc = None
     dense_bool = spec.kind == _lib.MASK_BOOL and spec.tile_live is None and spec.tile_live_t is None  # no tiles to step over
     bias_o = spec.kind == _lib.MASK_BIAS and gto is None and spec.bias_dtype == _lib.DTYPE_ENUM.get(q.dtype)  # through O alone
-    if SINGLE_PASS_BACKWARD and q.shape[-1] <= 64 and q.dtype != torch.float32 and (
+    if SINGLE_PASS_BACKWARD and q.shape[-1] == 64 and q.dtype != torch.float32 and (
             spec.kind in _lib.INDEX_MASKS or dense_bool or bias_o):
         acc = torch.empty(q.shape, device=q.device, dtype=torch.float32)
     if st is not None:

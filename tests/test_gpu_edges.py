@@ -267,3 +267,24 @@ def test_the_largest_probability_of_a_row_is_held_exactly(dt, D, L, kind):
     o = ja.attention(q.to(DEV), k.to(DEV), v.to(DEV), attn_mask=m).cpu().double()
     ref = torch.softmax(q.double() @ k.double().transpose(-1, -2) * D**-0.5, -1) @ v.double()
     assert (o - ref).norm() <= 1.1 * (ref.to(dtype).double() - ref).norm()
+
+
+@pytest.mark.parametrize("D,L,kind,cot", [(32, 1000, "none", "both"), (32, 514, "causal", "t"), (32, 512, "bias", "o"),
+                                          (64, 506, "bool", "both"), (64, 1000, "bias", "o"), (64, 506, "bias", "o")])
+def test_gradients_summed_in_a_fixed_order(D, L, kind, cot):
+    """Head dimension 32, and masks whose rows are not whole 16-byte pieces: bit for bit the same from run to run."""
+    B, H = 3, 6
+    q, k, v, tq, tk, tv, go, gt = (x.to(DEV) for x in _inputs(B, H, L, D, torch.bfloat16, L))
+    mask = _mask(kind, B, H, L, torch.bfloat16, 1)
+    mask = None if mask is None else mask.to(DEV)
+    a = [x.clone().requires_grad_() for x in (q, k, v)]
+
+    def run():
+        o, to = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, attn_mask=mask, causal=kind == "causal"), tuple(a), (tq, tk, tv))
+        outs = [(o, go)] * (cot != "t") + [(to, gt)] * (cot != "o")
+        return torch.autograd.grad([x for x, _ in outs], a, [w for _, w in outs])
+
+    first = run()
+    for _ in range(10):
+        for x, y in zip(run(), first):
+            assert torch.equal(x, y)
