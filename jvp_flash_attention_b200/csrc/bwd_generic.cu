@@ -171,10 +171,15 @@ __device__ __forceinline__ void zero_acc(float (*x)[4]) {
 
 // x += A0 B0^T and, where asked for, y += A1 B0^T (HAS_Y1) + A0 B1^T (HAS_Y2); rows r0.. of A0 / A1, all operands D-contiguous.
 // {S, tS} with (Q, tQ; K, tK), {E, F + dP} with (V, tV; G, gO) of the side in question.
+// TF32: the two products of y have an accumulator each and are added once, rounded (see gemm_out): in a single one the larger
+// of the two was truncated by the adds of both (tangents of a tenth, D128 L500 causal: dQ 2.0e-6 -> 2.7e-6).
 template <typename T, int D, int NT_, bool HAS_Y1, bool HAS_Y2>
 __device__ __forceinline__ void gemm_pair(float (*x)[4], float (*y)[4], const T* sA0, const T* sA1, const T* sB0, const T* sB1, int ld,
                                           int r0, int lane) {
   constexpr int KS = Elem<T>::kKStep;
+  constexpr bool kApart = HAS_Y1 && HAS_Y2 && !Elem<T>::k16;
+  float apart[kApart ? NT_ : 1][4];
+  if constexpr (kApart) zero_acc<NT_>(apart);
 #pragma unroll 4
   for (int k0 = 0; k0 < D; k0 += KS) {
     FragA<T> a0, a1;
@@ -194,10 +199,17 @@ __device__ __forceinline__ void gemm_pair(float (*x)[4], float (*y)[4], const T*
       }
       if constexpr (HAS_Y2) {
 #pragma unroll
-        for (int nt = 0; nt < NT_; ++nt) mma_pass<P()>(y[nt], a0, b1[nt]);
+        for (int nt = 0; nt < NT_; ++nt) mma_pass<P()>(kApart ? apart[nt] : y[nt], a0, b1[nt]);
       }
     };
     pass(IntC<0>{}), pass(IntC<1>{}), pass(IntC<2>{});
+  }
+  if constexpr (kApart) {
+#pragma unroll
+    for (int nt = 0; nt < NT_; ++nt) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[nt][e] += apart[nt][e];
+    }
   }
 }
 
@@ -275,8 +287,9 @@ __device__ __forceinline__ void smem_tile_to_global(T* ghead, const T* s, int ld
 // ---- dK, dV: CTA owns 64 keys, loops over query tiles.  Tiles are held transposed
 // (rows = keys, columns = queries) so that P^T etc. feed the second MMAs from registers. ----
 // TKV: K and V have tangents (JVPFA_ZERO_TKV leaves out what they would be multiplied by; it comes without gO).
+// (Head dimension 32 with 64-row tiles: 128 registers for two CTAs on an SM; the compiler would take 163.)
 template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
-__global__ void __launch_bounds__(32 * RG * KG) bwd_dkdv_kernel(const jvpfa_bwd_args a) {
+__global__ void __launch_bounds__(32 * RG * KG, !Elem<T>::k16 && D == 32 && HAS_GT && RG == 4 ? 2 : 0) bwd_dkdv_kernel(const jvpfa_bwd_args a) {
   using C = BwdCfg<T, D, RG, KG>;
   constexpr int BN = C::OWN, BM = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES, LW = C::LW;
   constexpr int NQ = LW / 8;

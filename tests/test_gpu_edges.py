@@ -288,3 +288,22 @@ def test_gradients_summed_in_a_fixed_order(D, L, kind, cot):
     for _ in range(10):
         for x, y in zip(run(), first):
             assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("D,L", [(32, 500), (64, 1024), (128, 500), (128, 1410)])
+@pytest.mark.parametrize("std", [0.1, 1.0])
+def test_fp32_gradients_through_both_outputs_are_as_exact_as_through_one(D, L, std):
+    """Each score product has an accumulator of its own.  A tensor core adds with truncation: 3 D / 8 adds, each losing half a
+    unit (0.72 x 2^-24 on average) of a partial sum that is two thirds of the result, come to 0.18 D 2^-24.  A gradient passes
+    two such products, independent of one another: 0.25 D 2^-24; a third more is allowed.  With two products in one
+    accumulator it was 0.35."""
+    B, H = 2, 4
+    x = [t.float() for t in _inputs(B, H, L, D, torch.float32, L + D)]
+    for i in (3, 4, 5):
+        x[i] = x[i] * (10 * std)
+    ref = orc.grads_through_both(*x, causal=True)
+    a = [t.to(DEV).requires_grad_() for t in x[:3]]
+    o, to = torch.func.jvp(lambda *t: ja.JVPAttn.fwd_dual(*t, causal=True), tuple(a), tuple(t.to(DEV) for t in x[3:6]))
+    got = torch.autograd.grad((o, to), a, (x[6].to(DEV), x[7].to(DEV)))
+    for name, y, r in zip(("dq", "dk", "dv"), got, ref[2:]):
+        assert ((y.cpu().double() - r).norm() / r.norm()).item() <= D / 3 * 2**-24, name
