@@ -60,3 +60,17 @@ def test_nested_transforms_take_the_general_route(cpu_kernels):  # noqa: F811
     g = torch.func.grad(lambda x: (ja.attention(x, k, v) * w).sum())(q)
     _, _, rdq, _, _ = orc.grads_through_both(q, k, v, tq, tk, tv, w, None)
     assert orc.max_abs_err(g, rdq) < 1e-9
+
+
+def test_a_remembered_mask_does_not_let_host_tensors_past_the_checks(cpu_kernels, monkeypatch):  # noqa: F811
+    q, k, v, *_ = _inputs(15)
+    mask = torch.randn(1, 2, 32, 32, dtype=torch.float64)
+    ja.attention(q, k, v, attn_mask=mask)
+    assert id(mask) in ja._MASK_MEMO
+
+    def require_cuda(*ts):
+        raise RuntimeError("runs only on CUDA tensors")
+
+    monkeypatch.setattr(ja, "_require_cuda", require_cuda)
+    with pytest.raises(RuntimeError, match="runs only on CUDA tensors"):
+        ja.attention(q, k, v, attn_mask=mask)
