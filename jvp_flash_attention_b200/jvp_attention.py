@@ -654,6 +654,7 @@ _CAUSAL = _lib.MaskSpec(_lib.MASK_CAUSAL)
 _functorch = torch._C._functorch
 _peek_functorch = _functorch.peek_interpreter_stack
 _JVP = _functorch.TransformType.Jvp
+_is_tracing = torch._C._is_tracing
 
 
 def _attend(q, k, v, attn_mask, causal, sm_scale, dual):
@@ -661,7 +662,8 @@ def _attend(q, k, v, attn_mask, causal, sm_scale, dual):
     the native layer (csrc/native.cpp).  What that does not take (bad arguments, nested transforms) goes through the
     Python Function, which words the errors."""
     interp = _peek_functorch()
-    if interp is None or (dual and interp.level() == 1 and interp.key() == _JVP):  # none, or torch.func.jvp alone
+    # no transform, or torch.func.jvp alone (a torch.jit.trace would record the native call's result as a constant)
+    if (interp is None or (dual and interp.level() == 1 and interp.key() == _JVP)) and not _is_tracing():
         native = _lib.native()
         if attn_mask is None:
             spec = _CAUSAL if causal else _NO_MASK

@@ -307,3 +307,14 @@ def test_fp32_gradients_through_both_outputs_are_as_exact_as_through_one(D, L, s
     got = torch.autograd.grad((o, to), a, (x[6].to(DEV), x[7].to(DEV)))
     for name, y, r in zip(("dq", "dk", "dv"), got, ref[2:]):
         assert ((y.cpu().double() - r).norm() / r.norm()).item() <= D / 3 * 2**-24, name
+
+
+@pytest.mark.parametrize("kind", ["none", "bias"])
+def test_a_trace_is_refused_rather_than_recorded_as_a_constant(kind):
+    """Under torch.jit.trace sizes are tensors, which the argument checks refuse.  A call that went past them left the output
+    of the traced input in the trace."""
+    q, k, v, *_ = (x.to(DEV) for x in _inputs(1, 2, 64, 64, torch.bfloat16, 1))
+    mask = None if kind == "none" else _mask(kind, 1, 2, 64, torch.bfloat16, 1).to(DEV)
+    ja.attention(q, k, v, attn_mask=mask)
+    with pytest.raises(AssertionError, match="HEAD_DIM"):
+        torch.jit.trace(lambda x: ja.attention(x, k, v, attn_mask=mask), (q,), check_trace=False)
