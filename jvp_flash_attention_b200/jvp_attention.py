@@ -117,7 +117,8 @@ def set_fp32_precision(mode: str) -> str:
 
 
 # What classify_mask found out about a mask tensor, kept while the same tensor object is passed again unmodified
-# (same Python object, same version counter: every in-place operation of torch bumps it).  A mask is typically
+# (same Python object, same version counter, which every in-place operation of torch bumps, and still the same memory and
+# layout, which an assignment to `.data` changes).  A mask is typically
 # built once and used by every layer and step; its verification is a pass over B*H*L*L elements and a read-back.
 # Writes that bypass torch (a foreign kernel writing through the raw pointer) are not seen; MASK_MEMO_ENABLED = False
 # turns the memo off.
@@ -126,10 +127,15 @@ _MASK_MEMO: dict = {}
 _MASK_MEMO_MAX = 16
 
 
+def _mask_state(m: Tensor) -> tuple:
+    """What tells a mask tensor's present contents from those that were verified."""
+    return m._version, m.data_ptr(), m.stride(), m.dtype
+
+
 def _remembered_mask(attn_mask: Tensor, q_shape) -> _lib.MaskSpec | None:
     """The description classify_mask found for this very tensor, unmodified since, or None."""
     hit = _MASK_MEMO.get(id(attn_mask)) if MASK_MEMO_ENABLED else None
-    if hit is not None and hit[0]() is attn_mask and hit[1] == (*q_shape[:3], True, attn_mask._version):
+    if hit is not None and hit[0]() is attn_mask and hit[1] == (*q_shape[:3], True, *_mask_state(attn_mask)):
         return hit[2][0]
     return None
 
@@ -148,7 +154,7 @@ def classify_mask(attn_mask: Tensor | None, causal: bool, Z: int, H: int, N: int
         return _lib.MaskSpec(_lib.MASK_NONE), 0, None
     if not MASK_MEMO_ENABLED:
         return _classify_mask_tensor(attn_mask, Z, H, N, verify)
-    key = (Z, H, N, verify, _unwrap(attn_mask)._version)
+    key = (Z, H, N, verify, *_mask_state(_unwrap(attn_mask)))
     hit = _MASK_MEMO.get(id(attn_mask))
     if hit is not None and hit[0]() is attn_mask and hit[1] == key:
         spec, mask_type = hit[2]

@@ -74,3 +74,18 @@ def test_a_remembered_mask_does_not_let_host_tensors_past_the_checks(cpu_kernels
     monkeypatch.setattr(ja, "_require_cuda", require_cuda)
     with pytest.raises(RuntimeError, match="runs only on CUDA tensors"):
         ja.attention(q, k, v, attn_mask=mask)
+
+
+@pytest.mark.parametrize("kind", ["bias", "bool", "transposed"])
+def test_a_mask_whose_data_is_replaced_is_another_mask(cpu_kernels, kind):  # noqa: F811
+    """An assignment to ``.data`` leaves object and version counter as they are."""
+    q, k, v, *_ = _inputs(17)
+    g = torch.Generator().manual_seed(17)
+    masks = [torch.randn(1, 2, 32, 32, generator=g, dtype=torch.float64) for _ in range(2)]
+    if kind == "bool":
+        masks = [(m > 0) | torch.eye(32, dtype=torch.bool) for m in masks]
+    mask = masks[0].clone()
+    ja.attention(q, k, v, attn_mask=mask)
+    mask.data = mask.data.transpose(2, 3) if kind == "transposed" else masks[1]
+    got = ja.attention(q, k, v, attn_mask=mask)
+    assert torch.equal(got, ja.attention(q, k, v, attn_mask=mask.clone()))
