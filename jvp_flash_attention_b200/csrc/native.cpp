@@ -612,13 +612,15 @@ std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tens
 }
 
 // attention (dual = false) or fwd_dual (true).  None: not a case for this path (bad arguments, dual inputs of a
-// primal-only call, functorch transforms other than a lone torch.func.jvp); the caller takes its general route.
-py::object attend(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const MaskPtr& mask, std::optional<double> scale,
-                  bool tf32, bool dual, bool strict_length) {
+// primal-only call, a mask's tangent alone, functorch transforms other than a lone torch.func.jvp); the caller takes its
+// general route.  `mask_in`: the caller's mask tensor.
+py::object attend(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, const std::optional<Tensor>& mask_in, const MaskPtr& mask,
+                  std::optional<double> scale, bool tf32, bool dual, bool strict_length) {
   const auto& stack = at::functorch::getDynamicLayerStack();
   Tensor q = q_in, k = k_in, v = v_in, tq = q._fw_grad(0), tk = k._fw_grad(0), tv = v._fw_grad(0);
   const bool any_tangent = tq.defined() || tk.defined() || tv.defined();
   if (!dual && any_tangent) return py::none();
+  if (mask_in && !any_tangent && mask_in->_fw_grad(0).defined()) return py::none();
   int64_t level = -1;
   if (!stack.empty()) {
     // Primals and tangents are taken off the transform's wrappers, the call runs one level down on plain tensors, and

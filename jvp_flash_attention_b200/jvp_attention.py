@@ -674,15 +674,16 @@ def _attend(q, k, v, attn_mask, causal, sm_scale, dual):
         if attn_mask is None:
             spec = _CAUSAL if causal else _NO_MASK
         else:
-            if interp is not None and _functorch.is_functorch_wrapped_tensor(attn_mask):
-                attn_mask = _functorch._unwrap_for_grad(attn_mask, 1)
-            spec = None if causal else _remembered_mask(attn_mask, q.shape)
+            mask = attn_mask
+            if interp is not None and _functorch.is_functorch_wrapped_tensor(mask):
+                mask = _functorch._unwrap_for_grad(mask, 1)
+            spec = None if causal else _remembered_mask(mask, q.shape)
         if spec is None or not q.is_cuda:  # (the native layer checks CUDA tensors itself, for a mask that is known to fit)
             _check_args(q, k, v, None, None, None, attn_mask, causal)
             if spec is None:
                 with native.NoFunctorch():  # the mask is a plain tensor, and so is what is found out about it
-                    spec = classify_mask(attn_mask, causal, *q.shape[:3], q.dtype, True)[0]
-        out = native.attend(q, k, v, spec.native(), sm_scale, _lib.FP32_PRECISION == "tf32", dual, STRICT_SEQUENCE_LENGTH)
+                    spec = classify_mask(mask, causal, *q.shape[:3], q.dtype, True)[0]
+        out = native.attend(q, k, v, attn_mask, spec.native(), sm_scale, _lib.FP32_PRECISION == "tf32", dual, STRICT_SEQUENCE_LENGTH)
         if out is not None:
             return out
     q_t, k_t, v_t = (fwAD.unpack_dual(x).tangent for x in (q, k, v)) if dual else (None, None, None)

@@ -89,3 +89,19 @@ def test_a_mask_whose_data_is_replaced_is_another_mask(cpu_kernels, kind):  # no
     mask.data = mask.data.transpose(2, 3) if kind == "transposed" else masks[1]
     got = ja.attention(q, k, v, attn_mask=mask)
     assert torch.equal(got, ja.attention(q, k, v, attn_mask=mask.clone()))
+
+
+@pytest.mark.parametrize("call", [ja.attention, ja.JVPAttn.fwd_dual])
+@pytest.mark.parametrize("route", ["func_jvp", "fwad"])
+def test_a_tangent_of_the_mask_alone_is_refused(cpu_kernels, call, route):  # noqa: F811
+    """There is no derivative with respect to a bias: a call that is differentiated along the bias alone says so, and does
+    not answer with a tangent of zero."""
+    q, k, v, *_ = _inputs(18)
+    g = torch.Generator().manual_seed(18)
+    mask, t = (torch.randn(1, 2, 32, 32, generator=g, dtype=torch.float64) for _ in range(2))
+    with pytest.raises(RuntimeError, match="needs tangents at forward time"):
+        if route == "fwad":
+            with fwAD.dual_level():
+                call(q, k, v, attn_mask=fwAD.make_dual(mask, t))
+        else:
+            torch.func.jvp(lambda m: call(q, k, v, attn_mask=m), (mask,), (t,))
