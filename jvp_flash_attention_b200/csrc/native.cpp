@@ -482,15 +482,15 @@ Grads backward_through_o(const Tensor& q, const Tensor& k, const Tensor& v, cons
   return g;
 }
 
-// The node of a call: outputs O (0) and, with tangents, tO (1); edges to q, k, v and the three tangents.
+// The node of a call: outputs O (0) and, with tangents, tO (1); edges to q, k, v, with tangents to these, and to a mask that
+// requires a gradient (which is undefined: O is part of the mask's graph, and the mask's gradient stays None).
 struct AttnNode : public Node {
   Call call;
-  bool dual = false;
   SavedVariable q, k, v, tq, tk, tv, o, to, lse, mu;
 
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
-    variable_list out(dual ? 6 : 3);
+    variable_list out(num_outputs());
     const Tensor go = primal_of(grads[0]);
     const Tensor gto = grads.size() > 1 ? primal_of(grads[1]) : Tensor();
     if (!go.defined() && !gto.defined()) return out;
@@ -569,7 +569,8 @@ struct Outputs {
 
 // The call itself on plain tensors; tangents all undefined or all given.  nullopt: not a case for this path.
 std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, Tensor tk, Tensor tv,
-                                    const MaskPtr& mask, std::optional<double> scale, bool tf32, bool strict_length) {
+                                    const Tensor& mask_tensor, const MaskPtr& mask, std::optional<double> scale, bool tf32,
+                                    bool strict_length) {
   for (const Tensor* t : std::initializer_list<const Tensor*>{&q, &k, &v, &tq, &tk, &tv})
     if (t->defined() && is_wrapped(*t)) return std::nullopt;
   if (!acceptable(q, k, v, strict_length)) return std::nullopt;
@@ -580,24 +581,26 @@ std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tens
     tq = tangent(tq, q), tk = tangent(tk, q), tv = tangent(tv, q);
   }
   Call call{mask, scale ? *scale : 1.0 / std::sqrt((double)q.size(3)), tf32};
-  const bool grad_primals = torch::autograd::compute_requires_grad(q, k, v);
-  const bool backward = grad_primals || torch::autograd::compute_requires_grad(tq, tk, tv);
+  const bool grad_qkv = torch::autograd::compute_requires_grad(q, k, v), grad_mask = torch::autograd::compute_requires_grad(mask_tensor);
+  const bool backward = grad_qkv || torch::autograd::compute_requires_grad(tq, tk, tv);
   prepare_mask(call, q, backward);
   FwdResult r = launch_fwd(q, k, v, tq, tk, tv, call);
-  if (backward) {
+  if (backward || grad_mask) {
     auto node = std::shared_ptr<AttnNode>(new AttnNode(), torch::autograd::deleteNode);
     node->call = call;
-    node->dual = dual;
-    node->set_next_edges(dual ? torch::autograd::collect_next_edges(q, k, v, tq, tk, tv)
-                              : torch::autograd::collect_next_edges(q, k, v));
+    torch::autograd::edge_list edges =
+        dual ? torch::autograd::collect_next_edges(q, k, v, tq, tk, tv) : torch::autograd::collect_next_edges(q, k, v);
+    if (grad_mask) edges.push_back(torch::autograd::impl::gradient_edge(mask_tensor));
+    node->set_next_edges(std::move(edges));
     node->q = SavedVariable(q, false);
     node->k = SavedVariable(k, false);
     node->v = SavedVariable(v, false);
-    if (grad_primals)
+    const bool grad_o = grad_qkv || grad_mask;
+    if (grad_o)
       torch::autograd::set_history(r.o, node);
     else
       node->add_input_metadata(Node::undefined_input());
-    if (dual) {
+    if (dual && backward) {
       torch::autograd::set_history(r.to, node);
       node->tq = SavedVariable(tq, false);
       node->tk = SavedVariable(tk, false);
@@ -605,7 +608,7 @@ std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tens
       node->to = SavedVariable(r.to, true);
       node->mu = SavedVariable(r.mu, false);
     }
-    node->o = SavedVariable(r.o, grad_primals);
+    node->o = SavedVariable(r.o, grad_o);
     node->lse = SavedVariable(r.lse, false);
   }
   return Outputs{r.o, r.to};
@@ -632,7 +635,7 @@ py::object attend(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, co
       if (w && w->level() == level) *t = Tensor(w->value());
     }
   }
-  auto out = attend_plain(q, k, v, tq, tk, tv, mask, scale, tf32, strict_length);
+  auto out = attend_plain(q, k, v, tq, tk, tv, mask_in ? unwrap(*mask_in) : Tensor(), mask, scale, tf32, strict_length);
   if (!out) return py::none();
   if (!out->to.defined()) return py::cast(out->o);
   Tensor o = out->o, to = out->to;

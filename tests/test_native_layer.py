@@ -105,3 +105,29 @@ def test_a_tangent_of_the_mask_alone_is_refused(cpu_kernels, call, route):  # no
                 call(q, k, v, attn_mask=fwAD.make_dual(mask, t))
         else:
             torch.func.jvp(lambda m: call(q, k, v, attn_mask=m), (mask,), (t,))
+
+
+@pytest.mark.parametrize("leaf", ["mask", "mask and q"])
+@pytest.mark.parametrize("route", ["attention", "fwad", "func_jvp"])
+def test_a_mask_that_requires_a_gradient_is_part_of_the_graph(cpu_kernels, leaf, route):  # noqa: F811
+    """A learned bias gets no gradient, but a backward from a call that has one works, whether q needs one or not."""
+    q, k, v, tq, tk, tv, w, _ = _inputs(19)
+    mask = torch.randn(1, 2, 32, 32, dtype=torch.float64, requires_grad=True)
+    q.requires_grad_("q" in leaf)
+    if route == "attention":
+        o, to = ja.attention(q, k, v, attn_mask=mask), None
+    elif route == "fwad":
+        with fwAD.dual_level():
+            o, to = fwAD.unpack_dual(ja.JVPAttn.fwd_dual(*map(fwAD.make_dual, (q, k, v), (tq, tk, tv)), attn_mask=mask))
+    else:
+        o, to = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, attn_mask=mask), (q, k, v), (tq, tk, tv))
+    assert o.requires_grad and (to is None or to.requires_grad == q.requires_grad)
+    (o * w).sum().backward(retain_graph=True)
+    ro, rto, rdq, _, _ = orc.grads_through_both(q, k, v, tq, tk, tv, w, None, attn_mask=mask.detach())
+    assert mask.grad is None and orc.max_abs_err(o, ro) < 1e-10
+    if "q" in leaf:
+        assert orc.max_abs_err(q.grad, rdq) < 1e-9
+        if to is not None:
+            (to * w).sum().backward()
+    else:
+        assert q.grad is None
