@@ -424,6 +424,15 @@ Tensor primal_of(const Tensor& x) {  // inside a forward-AD level the saved tens
   return x.defined() && x._fw_grad(0).defined() ? x._fw_primal(0) : x;
 }
 
+// A tensor of the forward's own as the kernels read it, under functorch's wrappers.  Hooks on saved tensors may hand back
+// another layout than the row-major one it was allocated with; upstream refuses such an output in its backward
+// (jvp_attention.py:2858-2877).
+Tensor saved_output(const Tensor& x, const char* name) {
+  const Tensor t = unwrap(x);
+  TORCH_CHECK_VALUE(t.is_contiguous(), "JVPAttn expected ", name, " to be contiguous; got ", name, ".is_contiguous()=False");
+  return t;
+}
+
 // (dq, dk, dv) = d<do, O>/d(q, k, v), as a node that can be differentiated once more.  With u the incoming gradients of
 // (dq, dk, dv):  d<(dq,dk,dv), u>/d(q,k,v) = d<tO(q,k,v; u), do>/d(q,k,v)  and  d<...>/d(do) = tO(q,k,v; u), so a
 // Hessian-vector product is one primal + tangent forward with tangents u and one backward through the tangent output.
@@ -496,7 +505,7 @@ struct AttnNode : public Node {
     if (!go.defined() && !gto.defined()) return out;
     const auto self = shared_from_this();
     const Tensor q_ = primal_of(q.unpack()), k_ = primal_of(k.unpack()), v_ = primal_of(v.unpack());
-    const Tensor o_ = unwrap(o.unpack(self)), lse_ = lse.unpack();
+    const Tensor o_ = saved_output(o.unpack(self), "o"), lse_ = saved_output(lse.unpack(), "lse");
     const int skip = unused_gradients(task_should_compute_output(0), task_should_compute_output(1) || task_should_compute_output(2));
     const bool need_primals = skip != (JVPFA_SKIP_DQ | JVPFA_SKIP_DKDV);
     if (!gto.defined()) {
@@ -507,7 +516,7 @@ struct AttnNode : public Node {
       return out;
     }
     const Tensor tq_ = tq.unpack(), tk_ = tk.unpack(), tv_ = tv.unpack();
-    const Tensor to_ = unwrap(to.unpack(self)), mu_ = mu.unpack();
+    const Tensor to_ = saved_output(to.unpack(self), "to"), mu_ = saved_output(mu.unpack(), "mu");
     const Tensor qp = unwrap(q_), kp = unwrap(k_), vp = unwrap(v_), tqp = unwrap(tq_), tkp = unwrap(tk_), tvp = unwrap(tv_);
     static constexpr const char* kOnce = "the gradient through the tangent output of JVPAttn cannot be differentiated a second time";
     if (need_primals) {

@@ -131,3 +131,42 @@ def test_a_mask_that_requires_a_gradient_is_part_of_the_graph(cpu_kernels, leaf,
             (to * w).sum().backward()
     else:
         assert q.grad is None
+
+
+def _strided(x):  # the same values, not row-major
+    return x.transpose(1, 2).contiguous().transpose(1, 2)
+
+
+@pytest.mark.parametrize("which", ["all", "o", "to", "lse", "mu", "inputs"])
+def test_hooks_on_saved_tensors_that_change_the_layout(cpu_kernels, which):  # noqa: F811
+    """q, k, v and their tangents may come back in any layout; what the forward allocated is refused unless row-major."""
+    q, k, v, tq, tk, tv, w1, w2 = _inputs(20)
+    a = [x.clone().requires_grad_() for x in (q, k, v)]
+    packed = []
+
+    def pack(x):
+        packed.append(x.detach().clone())
+        return len(packed) - 1, x
+
+    def unpack(handle):
+        n, x = handle
+        own = {k_: any(torch.equal(packed[n], y) for y in ys) for k_, ys in outputs.items() if ys and ys[0].shape == x.shape}
+        name = next((k_ for k_, same in own.items() if same), "inputs" if x.dim() == 4 else None)
+        if name is None:  # lse and mu: told apart by what is known of lse
+            name = "lse" if n == rows[0] else "mu"
+        return _strided(x) if which in ("all", name) else x
+
+    outputs = {"o": [], "to": []}
+    with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+        o, to = torch.func.jvp(ja.JVPAttn.fwd_dual, tuple(a), (tq, tk, tv))
+    outputs["o"].append(o.detach()), outputs["to"].append(to.detach())
+    lse = torch.logsumexp(q @ k.transpose(-1, -2) * 32**-0.5, -1) / 0.6931471805599453
+    rows = [n for n, x in enumerate(packed) if x.dim() == 3 and torch.allclose(x, lse)]
+    assert len(rows) == 1
+    if which == "inputs":
+        g = torch.autograd.grad((o * w1).sum() + (to * w2).sum(), a)
+        for x, y in zip(g, orc.grads_through_both(q, k, v, tq, tk, tv, w1, w2)[2:]):
+            assert orc.max_abs_err(x, y) < 1e-9
+    else:
+        with pytest.raises(ValueError, match="to be contiguous"):
+            torch.autograd.grad((o * w1).sum() + (to * w2).sum(), a)
