@@ -477,6 +477,11 @@ struct AttnBwdNode : public Node {
 
 Grads backward_through_o(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& go,
                          const Call& call, int skip) {
+  if (is_wrapped(go)) {  // the cotangent belongs to a functorch transform: a Function, which the transform differentiates or refuses
+    py::gil_scoped_acquire gil;
+    py::tuple g = python_module().attr("_backward_under_functorch")(q, k, v, o, lse, go, *call.mask->spec, call.scale, call.tf32);
+    return {g[0].cast<Tensor>(), g[1].cast<Tensor>(), g[2].cast<Tensor>()};
+  }
   Grads g = launch_bwd(unwrap(q), unwrap(k), unwrap(v), Tensor(), Tensor(), Tensor(), o, Tensor(), lse, Tensor(), go, Tensor(), call, skip);
   if (torch::autograd::compute_requires_grad(q, k, v, go)) {  // create_graph: a second differentiation was asked for
     auto node = std::shared_ptr<AttnBwdNode>(new AttnBwdNode(), torch::autograd::deleteNode);

@@ -170,3 +170,38 @@ def test_hooks_on_saved_tensors_that_change_the_layout(cpu_kernels, which):  # n
     else:
         with pytest.raises(ValueError, match="to be contiguous"):
             torch.autograd.grad((o * w1).sum() + (to * w2).sum(), a)
+
+
+@pytest.fixture()
+def unwrapping_cpu_kernels(cpu_kernels, monkeypatch):  # noqa: F811
+    """The stand-ins on plain tensors, as the package's own launch helpers run."""
+    def plain(launch):
+        def run(*args):
+            with torch.no_grad(), _lib.native().NoFunctorch():
+                return launch(*(ja._unwrap(x).detach() if isinstance(x, torch.Tensor) else x for x in args))
+        return run
+
+    monkeypatch.setattr(ja, "_launch_fwd", plain(stand_in.launch_fwd))
+    monkeypatch.setattr(ja, "_launch_bwd", plain(stand_in.launch_bwd))
+
+
+@pytest.mark.parametrize("outputs", ["o", "both"])
+def test_a_functorch_transform_of_the_cotangent(unwrapping_cpu_kernels, outputs):
+    """d/dw <dq(w), u> of a graph built outside the transform is the tangent of O along u; vmap over w is refused."""
+    q, k, v, tq, tk, tv, w, u = _inputs(21)
+    a = [x.clone().requires_grad_() for x in (q, k, v)]
+    if outputs == "o":
+        o, to = ja.attention(*a), None
+    else:
+        o, to = torch.func.jvp(ja.JVPAttn.fwd_dual, tuple(a), (tq, tk, tv))
+
+    def vjp(x):
+        outs, cots = ((o,), (x,)) if to is None else ((o, to), (x, w))
+        return torch.autograd.grad(outs, a[0], cots, retain_graph=True, create_graph=True)[0]
+
+    got = torch.func.grad(lambda x: (vjp(x) * u).sum())(w)
+    z = torch.zeros_like(q)
+    assert orc.max_abs_err(got, orc.sdpa_jvp(q, k, v, u, z, z)[1]) < 1e-9
+    if to is None:
+        with pytest.raises(RuntimeError, match="vmap"):
+            torch.func.vmap(vjp)(torch.stack([w, u]))
