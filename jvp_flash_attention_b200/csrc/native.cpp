@@ -80,19 +80,11 @@ struct Call {
   MaskPtr mask;
   double scale;
   bool tf32;  // fp32 tensors: one TF32 product instead of three, recorded so that the backward recomputes what the forward saw
-  // The mask's entries in the form the 16-bit tensor-core kernels read best, made by this call for its forward and
-  // backward (prepare_mask): a boolean mask as bits, by rows and transposed, a ragged bias with its rows padded.
-  Tensor bits, bits_t, padded;
+  // A boolean mask as bits, by rows and transposed: the form the 16-bit tensor-core kernels read best, made by this call for
+  // its forward and backward (pack_mask).
+  Tensor bits, bits_t;
 
-  jvpfa_mask c_mask() const {
-    jvpfa_mask m = mask->c;
-    if (padded.defined()) {
-      m.ptr = padded.const_data_ptr();
-      for (int d = 0; d < 4; ++d) m.stride[d] = padded.size(d) == 1 ? 0 : padded.stride(d);
-    }
-    return m;
-  }
-  void drop_tensors() { bits = bits_t = padded = Tensor(); }
+  void drop_tensors() { bits = bits_t = Tensor(); }
 };
 
 bool is_wrapped(const Tensor& x) {
@@ -189,6 +181,89 @@ struct Inputs {
   }
 };
 
+// ---- masks -----------------------------------------------------------------------------------------------------------
+// Whether the launches of a call may take the forms that only the 16-bit tensor-core kernels read.
+bool takes_16_bit_forms(const Tensor& q) { return q.is_cuda() && q.scalar_type() != at::kFloat && g_impl != JVPFA_IMPL_GENERIC; }
+
+// A ragged bias of the tensors' type with its rows padded to whole 16-byte pieces, the form in which the tensor-core kernels
+// take a bias (what lies beyond the row's end is not looked at); undefined for every other mask.  Up to one tile of keys a
+// bias is read element by element, whatever its layout.  Dimensions that broadcast are not written out, and the copy lives
+// for one launch: layers that share a bias do not hold a copy each until their backward.  Where there is no memory for it the
+// bias is read in place, by the register-tiled kernels.
+Tensor padded_bias(const MaskDesc& m, const Tensor& q) {
+  if (m.c.kind != JVPFA_MASK_BIAS || !takes_16_bit_forms(q) || m.tensor.scalar_type() != q.scalar_type() || m.c.stride[2] == 0) return {};
+  const int64_t L = q.size(2), step = 16 / m.tensor.element_size();
+  if (L <= 64 || L % step == 0) return {};
+  NoFunctorch nf;
+  at::AutoDispatchBelowADInplaceOrView below;
+  Tensor own = m.tensor;
+  for (int d = 0; d < 2; ++d)
+    if (m.c.stride[d] == 0) own = own.narrow(d, 0, 1);
+  Tensor padded;
+  try {
+    padded = empty({own.size(0), own.size(1), L, (L + step - 1) / step * step}, own.scalar_type(), own.device());
+  } catch (const c10::OutOfMemoryError&) {
+    return {};
+  }
+  padded = padded.narrow(3, 0, L);
+  padded.copy_(own);
+  return padded;
+}
+
+jvpfa_mask c_mask(const MaskDesc& m, const Tensor& padded) {
+  jvpfa_mask c = m.c;
+  if (padded.defined()) {
+    c.ptr = padded.const_data_ptr();
+    for (int d = 0; d < 4; ++d) c.stride[d] = padded.size(d) == 1 ? 0 : padded.stride(d);
+  }
+  return c;
+}
+
+// Whether the mask's own entries can be read as 16-byte pieces of its rows.
+bool whole_pieces(const MaskDesc& m, int64_t L) {
+  const int64_t esz = m.tensor.element_size();
+  bool ok = m.c.stride[3] == 1 && (reinterpret_cast<uintptr_t>(m.c.ptr) & 15u) == 0 && L % 16 == 0;
+  for (int d = 0; d < 3; ++d) ok = ok && m.c.stride[d] * esz % 16 == 0;
+  return ok;
+}
+
+// Packs a call's boolean mask.  Bits are made anew by every call and not kept with the mask's description: the entries that
+// the kernels read are then those that the mask holds when they run, also where it was written behind torch's version
+// counter (a replayed graph, a foreign kernel, `.data`).
+//
+// Packing reads the mask once (HBM bound) and saves a kernel that reads it one 16-byte piece per row and sub-tile.
+// B2 H12 L2048 D64, 100 MB of mask: packing 32 us; forward with tangents 168 -> 151 us, backward through tO 239 -> 186.
+// So it pays with a backward, for a mask that several heads share, and where the bytes' layout would send the call to
+// the register-tiled kernels.  Where there is no memory for the bits the kernels read the bytes.
+void pack_mask(Call& call, const Tensor& q, bool backward) {
+  const MaskDesc& m = *call.mask;
+  if (m.c.kind != JVPFA_MASK_BOOL || !takes_16_bit_forms(q)) return;
+  const int64_t L = q.size(2);
+  const int64_t n_b = m.c.stride[0] ? m.tensor.size(0) : 1, n_h = m.c.stride[1] ? m.tensor.size(1) : 1;
+  const int64_t n_rows = m.c.stride[2] ? L : 1;
+  if (!backward && whole_pieces(m, L) && 4 * n_b * n_h > q.size(0) * q.size(1)) return;
+  c10::cuda::OptionalCUDAGuard guard;
+  if (q.get_device() != c10::cuda::current_device()) guard.set_index(q.get_device());
+  const int64_t w = (L + 63) / 64 * 2;
+  jvpfa_mask_tiles_args a{};
+  a.struct_size = sizeof(a);
+  a.n_b = (int)n_b, a.n_h = (int)n_h, a.n_rows = (int)n_rows, a.L = (int)L;
+  a.mask = m.c;
+  Tensor bits, bits_t;
+  try {
+    bits = empty({n_b * n_h * n_rows * w}, at::kInt, q.device());
+    if (backward) bits_t = empty({n_b * n_h * L * (n_rows > 1 ? w : 1)}, at::kInt, q.device());
+  } catch (const c10::OutOfMemoryError&) {
+    return;
+  }
+  a.bits = bits.data_ptr();
+  if (backward) a.bits_t = bits_t.data_ptr();
+  const int rc = jvpfa_mask_tiles(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream());
+  if (rc == JVPFA_ERR_TOO_LARGE) return;  // the kernels read the bytes
+  check_status(rc, "jvpfa_mask_tiles");
+  call.bits = bits, call.bits_t = bits_t;
+}
+
 // ---- launches ------------------------------------------------------------------------------------------------------
 py::object or_none(const Tensor& t) { return t.defined() ? py::cast(t) : py::object(py::none()); }
 
@@ -219,6 +294,7 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     r.to = empty(sizes, q.scalar_type(), q.device());
     r.mu = empty(sizes.slice(0, 3), at::kFloat, q.device());
   }
+  const Tensor padded = padded_bias(*call.mask, q);
   jvpfa_fwd_args a{};
   a.struct_size = sizeof(a);
   a.dtype = dtype_of(q, call.tf32);
@@ -229,7 +305,7 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   a.lse = static_cast<float*>(r.lse.data_ptr());
   a.to = dual ? r.to.data_ptr() : nullptr;
   a.mu = dual ? static_cast<float*>(r.mu.data_ptr()) : nullptr;
-  a.mask = call.c_mask();
+  a.mask = c_mask(*call.mask, padded);
   a.mask_tile_live = data(call.mask->tile_live);
   a.mask_bits = data(call.bits);
   a.flags = dual && !tk.defined() ? JVPFA_ZERO_TKV : 0;
@@ -245,60 +321,6 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     }
     check_status(rc, "jvpfa_fwd");
     return r;
-  }
-}
-
-// Whether the mask's own entries can be read as 16-byte pieces of its rows.
-bool whole_pieces(const MaskDesc& m, int64_t L) {
-  const int64_t esz = m.tensor.element_size();
-  bool ok = m.c.stride[3] == 1 && (reinterpret_cast<uintptr_t>(m.c.ptr) & 15u) == 0 && L % 16 == 0;
-  for (int d = 0; d < 3; ++d) ok = ok && m.c.stride[d] * esz % 16 == 0;
-  return ok;
-}
-
-// Fills in the call's forms of its mask.  They are made anew by every call and not kept with the mask's description: what
-// the kernels read is then what the mask holds when they run, also where it was written behind torch's version counter
-// (a replayed graph, a foreign kernel, `.data`).
-//
-// Packing reads the mask once (HBM bound) and saves a kernel that reads it one 16-byte piece per row and sub-tile.
-// B2 H12 L2048 D64, 100 MB of mask: packing 32 us; forward with tangents 168 -> 151 us, backward through tO 239 -> 186.
-// So it pays with a backward, for a mask that several heads share, and where the bytes' layout would send the call to
-// the register-tiled kernels.
-void prepare_mask(Call& call, const Tensor& q, bool backward) {
-  const MaskDesc& m = *call.mask;
-  if (!q.is_cuda() || q.scalar_type() == at::kFloat || g_impl == JVPFA_IMPL_GENERIC) return;
-  const int64_t L = q.size(2), esz = m.tensor.defined() ? m.tensor.element_size() : 0;
-  if (m.c.kind == JVPFA_MASK_BOOL) {
-    const int64_t n_b = m.c.stride[0] ? m.tensor.size(0) : 1, n_h = m.c.stride[1] ? m.tensor.size(1) : 1;
-    const int64_t n_rows = m.c.stride[2] ? L : 1;
-    if (!backward && whole_pieces(m, L) && 4 * n_b * n_h > q.size(0) * q.size(1)) return;
-    c10::cuda::OptionalCUDAGuard guard;
-    if (q.get_device() != c10::cuda::current_device()) guard.set_index(q.get_device());
-    const int64_t w = (L + 63) / 64 * 2;
-    jvpfa_mask_tiles_args a{};
-    a.struct_size = sizeof(a);
-    a.n_b = (int)n_b, a.n_h = (int)n_h, a.n_rows = (int)n_rows, a.L = (int)L;
-    a.mask = m.c;
-    Tensor bits = empty({n_b * n_h * n_rows * w}, at::kInt, q.device()), bits_t;
-    a.bits = bits.data_ptr();
-    if (backward) {
-      bits_t = empty({n_b * n_h * L * (n_rows > 1 ? w : 1)}, at::kInt, q.device());
-      a.bits_t = bits_t.data_ptr();
-    }
-    const int rc = jvpfa_mask_tiles(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream());
-    if (rc == JVPFA_ERR_TOO_LARGE) return;  // the kernels read the bytes
-    check_status(rc, "jvpfa_mask_tiles");
-    call.bits = bits, call.bits_t = bits_t;
-  } else if (m.c.kind == JVPFA_MASK_BIAS && m.tensor.scalar_type() == q.scalar_type() && m.c.stride[2] != 0 && L > 64 && L * esz % 16 != 0) {
-    // rows padded to whole 16-byte pieces, the form in which those kernels take a bias (what lies beyond the row's end is
-    // not looked at); up to one tile of keys it is read element by element, whatever its layout
-    NoFunctorch nf;
-    at::AutoDispatchBelowADInplaceOrView below;
-    c10::cuda::OptionalCUDAGuard guard(q.device());
-    const int64_t step = 16 / esz;
-    const auto s = m.tensor.sizes();
-    call.padded = at::empty({s[0], s[1], s[2], (L + step - 1) / step * step}, m.tensor.options()).narrow(3, 0, L);
-    call.padded.copy_(m.tensor);
   }
 }
 
@@ -358,6 +380,7 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   if (!(skip & JVPFA_SKIP_DQ)) g[0] = empty(sizes, q.scalar_type(), q.device());
   if (!(skip & JVPFA_SKIP_DKDV))
     for (int i = 1; i < 3; ++i) g[i] = empty(sizes, q.scalar_type(), q.device());
+  const Tensor padded = padded_bias(m, q);
   jvpfa_bwd_args a{};
   a.struct_size = sizeof(a);
   a.dtype = p.dtype;
@@ -371,7 +394,7 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.flags = skip | (single ? JVPFA_DQ_ACCUM_IS_ZERO : 0) | (tq.defined() && !tk.defined() ? JVPFA_ZERO_TKV : 0);
   if (g[0].defined()) a.dq = g[0].data_ptr();
   if (g[1].defined()) a.dk = g[1].data_ptr(), a.dv = g[2].data_ptr();
-  a.mask = call.c_mask();
+  a.mask = c_mask(*call.mask, padded);
   if (m.tile_live.defined() && m.tile_live_t.defined() && a.L <= 8192) {
     a.mask_tile_live = data(m.tile_live);
     a.mask_tile_live_t = data(m.tile_live_t);
@@ -597,7 +620,7 @@ std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tens
   Call call{mask, scale ? *scale : 1.0 / std::sqrt((double)q.size(3)), tf32};
   const bool grad_qkv = torch::autograd::compute_requires_grad(q, k, v), grad_mask = torch::autograd::compute_requires_grad(mask_tensor);
   const bool backward = grad_qkv || torch::autograd::compute_requires_grad(tq, tk, tv);
-  prepare_mask(call, q, backward);
+  pack_mask(call, q, backward);
   FwdResult r = launch_fwd(q, k, v, tq, tk, tv, call);
   if (backward || grad_mask) {
     auto node = std::shared_ptr<AttnNode>(new AttnNode(), torch::autograd::deleteNode);

@@ -318,3 +318,66 @@ def test_a_trace_is_refused_rather_than_recorded_as_a_constant(kind):
     ja.attention(q, k, v, attn_mask=mask)
     with pytest.raises(AssertionError, match="HEAD_DIM"):
         torch.jit.trace(lambda x: ja.attention(x, k, v, attn_mask=mask), (q,), check_trace=False)
+
+
+def _peak(run):
+    """Outputs of a call, its peak of allocated bytes, and what it leaves allocated, both over what was there before."""
+    out = run()  # the mask's verification, kernels' first use
+    del out
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    out = run()
+    return out, torch.cuda.max_memory_allocated() - before, torch.cuda.memory_allocated() - before
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dims", [(1, 1), (8, 1), (1, 16)])
+def test_a_ragged_bias_that_broadcasts_is_not_written_out(D, dims):
+    """Rows of 250 elements are padded to 256 for the tensor-core kernels: what the copy takes is the bias's own extents, a
+    view that expands costs no more than the tensor it is a view of (and what the allocator's blocks are larger, up to 1 MiB).
+    Written out it would be 16 MB."""
+    B, H, L = 8, 16, 250
+    q, k, v, *_ = (x.to(DEV) for x in _inputs(B, H, L, D, torch.bfloat16, D))
+    own = _mask("bias", *dims, L, torch.bfloat16, 1).to(DEV)
+    view = own.expand(B, H, L, L)
+    assert 0 in view.stride()
+    with torch.no_grad():
+        got, peak, _ = _peak(lambda: ja.attention(q, k, v, attn_mask=view))
+        _, plain, _ = _peak(lambda: ja.attention(q, k, v))
+        want = ja.attention(q, k, v, attn_mask=view.contiguous())
+    assert torch.equal(got, want)
+    assert peak - plain <= dims[0] * dims[1] * L * 256 * 2 + (1 << 20)
+
+
+def test_the_copy_of_a_ragged_bias_does_not_wait_for_the_backward():
+    B, H, L, D = 4, 8, 506, 64
+    q, k, v, _, _, _, go, _ = (x.to(DEV) for x in _inputs(B, H, L, D, torch.bfloat16, 3))
+    bias = _mask("bias", B, H, L, torch.bfloat16, 1).to(DEV)
+    a = [x.clone().requires_grad_() for x in (q, k, v)]
+    o, _, held = _peak(lambda: ja.attention(*a, attn_mask=bias))
+    _, _, plain = _peak(lambda: ja.attention(*a))
+    assert held <= plain + (1 << 20)  # blocks may be that much larger than what is asked for; the copy takes 16.6 MB
+    ref = orc.grads_through_both(*(x.cpu() for x in (q, k, v)), *(torch.zeros(B, H, L, D) for _ in range(3)), go.cpu(), None, attn_mask=bias.cpu())
+    for x, r in zip(torch.autograd.grad(o, a, go), ref[2:]):
+        assert orc.max_abs_err(x, r) <= 2e-2 * max(1.0, r.abs().max().item())
+
+
+@pytest.mark.parametrize("kind", ["bias", "bool"])
+def test_a_mask_whose_copy_does_not_fit_is_read_in_place(kind):
+    """With room for the results but not for another form of the mask, the call runs as it did without one."""
+    B, H, L, D = 2, 24, 2050, 64
+    q, k, v, *_ = (x.to(DEV) for x in _inputs(B, H, L, D, torch.bfloat16, 4))
+    mask = _mask("bias", B, H, L, torch.bfloat16, 1).to(DEV) if kind == "bias" else (torch.rand(B, H, L, L, device=DEV) > 0.5)
+    torch.cuda.empty_cache()  # the results get memory of their own, not a part of what the mask was made in
+    with torch.no_grad():
+        want = ja.attention(q, k, v, attn_mask=mask)
+        torch.cuda.empty_cache()
+        room = torch.cuda.memory_reserved() + (20 << 20)  # O and its row statistics take 13 MB, the bits of `bool` 26 MB
+        try:
+            torch.cuda.set_per_process_memory_fraction(room / torch.cuda.get_device_properties(0).total_memory)
+            got = ja.attention(q, k, v, attn_mask=mask)
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+    assert (got.float() - want.float()).abs().max().item() <= 2e-2 * max(1.0, want.abs().max().item())
+    assert _lib.device_status() == 0
