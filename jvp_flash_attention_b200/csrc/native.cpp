@@ -620,8 +620,14 @@ std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tens
   Call call{mask, scale ? *scale : 1.0 / std::sqrt((double)q.size(3)), tf32};
   const bool grad_qkv = torch::autograd::compute_requires_grad(q, k, v), grad_mask = torch::autograd::compute_requires_grad(mask_tensor);
   const bool backward = grad_qkv || torch::autograd::compute_requires_grad(tq, tk, tv);
-  pack_mask(call, q, backward);
-  FwdResult r = launch_fwd(q, k, v, tq, tk, tv, call);
+  FwdResult r;
+  {
+    // A launch waits while the queue of launches is full: other Python threads run meanwhile.
+    std::optional<py::gil_scoped_release> no_gil;
+    if (q.is_cuda()) no_gil.emplace();
+    pack_mask(call, q, backward);
+    r = launch_fwd(q, k, v, tq, tk, tv, call);
+  }
   if (backward || grad_mask) {
     auto node = std::shared_ptr<AttnNode>(new AttnNode(), torch::autograd::deleteNode);
     node->call = call;

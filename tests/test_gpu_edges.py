@@ -1,5 +1,8 @@
 """GPU tests at the edges of the dispatch: head dimension 32 on the D = 64 tensor-core kernels, masks whose rows do not
 fill 16-byte pieces, the row / key splits of the register-tiled kernels, and gradients that nobody asked for."""
+import threading
+import time
+
 import pytest
 import torch
 
@@ -381,3 +384,35 @@ def test_a_mask_whose_copy_does_not_fit_is_read_in_place(kind):
             torch.cuda.set_per_process_memory_fraction(1.0)
     assert (got.float() - want.float()).abs().max().item() <= 2e-2 * max(1.0, want.abs().max().item())
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["none", "bool"])
+def test_other_threads_run_while_the_launch_queue_is_full(kind):
+    """Launches behind half a second of device time: more than the queue holds, so the launching thread waits.  Another
+    thread's largest pause stays far below that wait."""
+    q, *_ = (x.to(DEV) for x in _inputs(1, 2, 66, 64, torch.bfloat16, 5))
+    mask = None if kind == "none" else _mask(kind, 1, 2, 66, torch.bfloat16, 1).to(DEV)
+    pauses, stop = [], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            pauses.append(now - last)
+            last = now
+
+    with torch.no_grad():
+        ja.attention(q, q, q, attn_mask=mask)
+        torch.cuda.synchronize()
+        other = threading.Thread(target=tick)
+        other.start()
+        torch.cuda._sleep(1_000_000_000)  # clock cycles
+        begin = time.perf_counter()
+        for _ in range(4000):
+            ja.attention(q, q, q, attn_mask=mask)
+        waited = time.perf_counter() - begin
+        torch.cuda.synchronize()
+        stop.set()
+        other.join()
+    assert waited > 0.2 and max(pauses) < waited / 4, (waited, max(pauses))
