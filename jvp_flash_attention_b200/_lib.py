@@ -351,13 +351,6 @@ def _stream(t: torch.Tensor) -> int:
     return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
-ERR_UNSUPPORTED = -9
-
-
-class Unsupported(RuntimeError):
-    """The library understood the request but this build cannot serve it (JVPFA_ERR_UNSUPPORTED)."""
-
-
 def common_strides(*ts) -> tuple[int, int, int] | None:
     """(batch, head, row) element strides shared by the given (B,H,L,D) tensors, or None when they are all
     row-major.  Raises ValueError when the tensors disagree or the layout cannot be described that way
@@ -391,10 +384,7 @@ def fwd(q, k, v, tq, tk, tv, o, to, lse, mu, mask: MaskSpec, sm_scale: float, im
     a.mask_tile_live = ptr(mask.tile_live)
     if in_stride is not None:
         a.in_stride[0], a.in_stride[1], a.in_stride[2] = in_stride
-    rc = _launch(q, lib.jvpfa_fwd, a)
-    if rc == ERR_UNSUPPORTED and in_stride is not None:
-        raise Unsupported("jvpfa_fwd cannot read this layout in place")
-    check(rc, "jvpfa_fwd")
+    check(_launch(q, lib.jvpfa_fwd, a), "jvpfa_fwd")
 
 
 def mask_check(mask: "MaskSpec", shape) -> tuple[bool, bool]:
@@ -439,8 +429,7 @@ def mask_tiles(mask: "MaskSpec", L: int):
     a.tile_live = tile_live.data_ptr()
     a.head_live = head_live.data_ptr()
     a.tile_live_t = tile_live_t.data_ptr()
-    rc = _launch(t, lib.jvpfa_mask_tiles, a)
-    check(rc, "jvpfa_mask_tiles")
+    check(_launch(t, lib.jvpfa_mask_tiles, a), "jvpfa_mask_tiles")
     return tile_live, head_live, tile_live_t
 
 
@@ -482,10 +471,7 @@ def bwd(q, k, v, tq, tk, tv, go, gto, lse, mu, delta, eps, cterm, dq, dk, dv, ma
     if in_stride is not None:
         a.in_stride[0], a.in_stride[1], a.in_stride[2] = in_stride
     a.dq_accum = ptr(dq_accum)
-    rc = _launch(q, lib.jvpfa_bwd, a)
-    if rc == ERR_UNSUPPORTED and in_stride is not None:
-        raise Unsupported("jvpfa_bwd cannot read this layout in place")
-    check(rc, "jvpfa_bwd")
+    check(_launch(q, lib.jvpfa_bwd, a), "jvpfa_bwd")
 
 
 def bwd_noalloc(q, k, v, tq, tk, tv, o, to, go, gto, lse, mu, dq, dk, dv, mask: MaskSpec, sm_scale: float,

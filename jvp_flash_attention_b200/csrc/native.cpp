@@ -171,7 +171,6 @@ struct Inputs {
       : q(q_), k(k_), v(v_), tq(tq_), tk(tk_), tv(tv_) {
     if (!common_layout({&q, &k, &v, &tq, &tk, &tv}, st)) make_dense();
   }
-  bool strided() const { return st[0] != 0; }
   void make_dense() {
     NoFunctorch nf;
     at::AutoDispatchBelowADInplaceOrView below;
@@ -309,19 +308,11 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   a.mask_tile_live = data(call.mask->tile_live);
   a.mask_bits = data(call.bits);
   a.flags = dual && !tk.defined() ? JVPFA_ZERO_TKV : 0;
-  void* stream = c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
-  for (;;) {
-    a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
-    a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
-    for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
-    const int rc = jvpfa_fwd(&a, stream);
-    if (rc == JVPFA_ERR_UNSUPPORTED && in.strided()) {  // this kernel family wants row-major inputs
-      in.make_dense();
-      continue;
-    }
-    check_status(rc, "jvpfa_fwd");
-    return r;
-  }
+  a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
+  a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
+  for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
+  check_status(jvpfa_fwd(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "jvpfa_fwd");
+  return r;
 }
 
 // Gradients of <go, O> + <gto, tO> with respect to q, k, v; those named in `skip` (JVPFA_SKIP_*) stay undefined.
@@ -402,18 +393,11 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.dq_accum = p.dq_accum;
   a.mask_bits = data(call.bits);
   a.mask_bits_t = data(call.bits_t);
-  for (;;) {
-    a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
-    a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
-    for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
-    const int rc = jvpfa_bwd(&a, stream);
-    if (rc == JVPFA_ERR_UNSUPPORTED && in.strided()) {
-      in.make_dense();
-      continue;
-    }
-    check_status(rc, "jvpfa_bwd");
-    return g;
-  }
+  a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
+  a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
+  for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
+  check_status(jvpfa_bwd(&a, stream), "jvpfa_bwd");
+  return g;
 }
 
 // What autograd will not use of a node's gradients with respect to q, k, v (its first three outputs).

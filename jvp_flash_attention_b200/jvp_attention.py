@@ -208,15 +208,12 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, verify: boo
             # One pass answers upstream's check and says which 128 x 64 tiles have a True at all; forward and
             # backward step over the others.  (Without verification the mask is not looked at beforehand, so
             # there is no block skipping either: whether it would pay is known only from the pass's counts.)
-            try:
-                spec.tile_live, head_live, spec.tile_live_t = _lib.mask_tiles(spec, N)
-                *heads, n_live = head_live.tolist()  # the one read-back
-                every_head_live = all(heads)
-                n_entries = spec.tile_live.numel() // (((N + 63) // 64 + 63) // 64)
-                if n_live > 0.85 * n_entries * ((N + 63) // 64):
-                    spec.tile_live = spec.tile_live_t = None  # (nearly) every tile is live: the plain loops are quicker
-            except _lib.Unsupported:  # no summary of this mask: no skipping, element-wise check
-                every_head_live = _lib.mask_check(spec, m8.shape)[0]
+            spec.tile_live, head_live, spec.tile_live_t = _lib.mask_tiles(spec, N)
+            *heads, n_live = head_live.tolist()  # the one read-back
+            every_head_live = all(heads)
+            n_entries = spec.tile_live.numel() // (((N + 63) // 64 + 63) // 64)
+            if n_live > 0.85 * n_entries * ((N + 63) // 64):
+                spec.tile_live = spec.tile_live_t = None  # (nearly) every tile is live: the plain loops are quicker
         assert every_head_live, "The attention mask cannot be all False for any head."
         return spec, 1, attn_mask
 
@@ -251,13 +248,7 @@ def _launch_fwd(q, k, v, tq, tk, tv, spec: _lib.MaskSpec, sm_scale: float):
     dual = ins[3] is not None
     to = torch.empty_like(o) if dual else None
     mu = torch.empty_like(lse) if dual else None
-    if st is not None:
-        try:
-            _lib.fwd(*ins, o, to, lse, mu, spec, sm_scale, KERNEL_IMPL, in_stride=st)
-            return o, to, lse, mu
-        except _lib.Unsupported:  # this kernel family wants row-major inputs
-            ins = [None if t is None else t.contiguous() for t in ins]
-    _lib.fwd(*ins, o, to, lse, mu, spec, sm_scale, KERNEL_IMPL)
+    _lib.fwd(*ins, o, to, lse, mu, spec, sm_scale, KERNEL_IMPL, in_stride=st)
     return o, to, lse, mu
 
 
@@ -286,14 +277,7 @@ def _launch_bwd(q, k, v, tq, tk, tv, o, to, lse, mu, go, gto, spec: _lib.MaskSpe
     if SINGLE_PASS_BACKWARD and q.shape[-1] == 64 and q.dtype != torch.float32 and (
             spec.kind in _lib.INDEX_MASKS or dense_bool or bias_o):
         acc = torch.empty(q.shape, device=q.device, dtype=torch.float32)
-    if st is not None:
-        try:
-            _lib.bwd(*ins, go, gto, lse, mu, delta, eps, cterm, dq, dk, dv, spec, sm_scale, KERNEL_IMPL, in_stride=st,
-                     dq_accum=acc)
-            return dq, dk, dv
-        except _lib.Unsupported:
-            ins = [None if t is None else t.contiguous() for t in ins]
-    _lib.bwd(*ins, go, gto, lse, mu, delta, eps, cterm, dq, dk, dv, spec, sm_scale, KERNEL_IMPL, dq_accum=acc)
+    _lib.bwd(*ins, go, gto, lse, mu, delta, eps, cterm, dq, dk, dv, spec, sm_scale, KERNEL_IMPL, in_stride=st, dq_accum=acc)
     return dq, dk, dv
 
 

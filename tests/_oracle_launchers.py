@@ -50,5 +50,23 @@ def mask_check(spec, shape):
 
 
 def mask_tiles(spec, L):
-    """Stand-in for jvpfa_mask_tiles: no tile bitmap on the host, so the caller takes its element-wise route."""
-    raise _lib.Unsupported("no tile bitmap without the device pass")
+    """Stand-in for the device pass jvpfa_mask_tiles: the same bitmaps, flags and count, from eager reductions."""
+    t = spec.tensor.bool()
+    for d in range(3):
+        if spec.strides[d] == 0:
+            t = t.narrow(d, 0, 1)
+    n_rows = t.shape[2]
+    t = t.reshape(-1, n_rows, L)
+    n_qt, n_kt = (1 if n_rows == 1 else -(-L // 128)), -(-L // 64)
+    padded = torch.zeros(t.shape[0], n_qt * (1 if n_rows == 1 else 128), n_kt * 64, dtype=torch.bool)
+    padded[:, :n_rows, :L] = t
+    live = padded.reshape(t.shape[0], n_qt, -1, n_kt, 64).any(dim=4).any(dim=2)  # [head][query tile][64-key tile]
+    wide = torch.nn.functional.pad(live, (0, n_kt % 2)).reshape(t.shape[0], n_qt, -1, 2).any(dim=3)  # of 128 keys
+    heads = torch.cat([live.any(dim=2).any(dim=1).to(torch.int32), live.sum().reshape(1).to(torch.int32)])
+    return _words(live), heads, _words(wide.transpose(1, 2))
+
+
+def _words(bits):
+    """Bit (n % 64) of int64 word n / 64 of every row."""
+    bits = torch.nn.functional.pad(bits, (0, -bits.shape[-1] % 64)).reshape(-1, 64)
+    return (bits.to(torch.int64) << torch.arange(64)).sum(dim=1)

@@ -9,6 +9,7 @@ import torch
 import jvp_flash_attention_b200.jvp_attention as ja
 from jvp_flash_attention_b200 import _lib
 from oracle import jvp_attention_oracle as orc
+from tests import _oracle_launchers as stand_in
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -416,3 +417,23 @@ def test_other_threads_run_while_the_launch_queue_is_full(kind):
         stop.set()
         other.join()
     assert waited > 0.2 and max(pauses) < waited / 4, (waited, max(pauses))
+
+
+@pytest.mark.parametrize("L", [34, 130, 1000, 4200])
+@pytest.mark.parametrize("layout", ["rows", "keys", "one row", "expanded"])
+def test_tile_bitmaps_are_those_of_the_host_stand_in(L, layout):
+    """jvpfa_mask_tiles against the eager reductions that stand in for it in the CPU tests, ragged and in other strides."""
+    g = torch.Generator().manual_seed(L)
+    m = torch.rand(2, 1 if L > 1000 else 3, 1 if layout == "one row" else L, L, generator=g) > 1 - 2 / (128 * 64)
+    m[:, :, 0, L // 3] = True
+    if layout == "keys":
+        m = m.transpose(2, 3)
+    if layout == "expanded":
+        m = m[:1].expand(2, -1, -1, -1)
+
+    def spec(t):
+        return _lib.MaskSpec(_lib.MASK_BOOL, t.view(torch.uint8), tuple(0 if n == 1 else s for n, s in zip(t.shape, t.stride())))
+
+    dev = torch.empty_strided(m.shape, m.stride(), dtype=torch.bool, device=DEV).copy_(m) if layout != "expanded" else m[:1].to(DEV).expand(2, -1, -1, -1)
+    for x, y in zip(_lib.mask_tiles(spec(dev), L), stand_in.mask_tiles(spec(m), L)):
+        assert torch.equal(x.cpu(), y.to(x.dtype))
