@@ -4,7 +4,8 @@ Usage: ``python -m jvp_flash_attention_b200.build [--force] [--verbose]``.
 Each ``csrc/*.cu`` is compiled to an object file under ``csrc/_obj`` (in parallel) and the
 objects are linked into ``jvp_flash_attention_b200/libjvpfa.so``.  A translation unit is rebuilt
 only when it or a header is newer than its object.  ``csrc/native.cpp``, the host side of a call
-(``_native.so``, a Python extension module linked against torch and libjvpfa.so), is built with g++.
+(``_native.so``, a Python extension module linked against torch and libjvpfa.so), is built with g++, again also when
+the command or the version of torch is another one than it was built with.
 """
 from __future__ import annotations
 
@@ -21,6 +22,7 @@ CSRC = PKG_DIR / "csrc"
 OBJ = CSRC / "_obj"
 LIB = PKG_DIR / "libjvpfa.so"
 NATIVE = PKG_DIR / "_native.so"
+NATIVE_STAMP = OBJ / "native.stamp"  # what the present _native.so was built with
 INCLUDE = PKG_DIR.parent / "include"
 
 NVCC_FLAGS = [
@@ -64,6 +66,19 @@ def _native_cmd() -> list[str]:
     ]
 
 
+def _native_with() -> str:
+    import torch
+
+    return "\n".join([f"torch {torch.__version__}", f"python {sys.version}", *_native_cmd()])
+
+
+def _native_stale() -> bool:
+    sources = [CSRC / "native.cpp", INCLUDE / "jvpfa.h", *(CSRC / "compat").rglob("*.hpp")]
+    if not NATIVE.exists() or NATIVE.stat().st_mtime < max(f.stat().st_mtime for f in sources):
+        return True
+    return not NATIVE_STAMP.exists() or NATIVE_STAMP.read_text() != _native_with()
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     """Compile every CUDA source for sm_100a and link the shared library; returns its path."""
     OBJ.mkdir(exist_ok=True)
@@ -98,12 +113,12 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
-    src = CSRC / "native.cpp"
-    if force or not NATIVE.exists() or NATIVE.stat().st_mtime < max(src.stat().st_mtime, (INCLUDE / "jvpfa.h").stat().st_mtime):
+    if force or _native_stale():
         r = subprocess.run(_native_cmd(), capture_output=True, text=True)
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("g++ failed for native.cpp")
+        NATIVE_STAMP.write_text(_native_with())
     return LIB
 
 

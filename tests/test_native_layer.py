@@ -5,7 +5,7 @@ import torch
 import torch.autograd.forward_ad as fwAD
 
 import jvp_flash_attention_b200.jvp_attention as ja
-from jvp_flash_attention_b200 import _lib
+from jvp_flash_attention_b200 import _lib, build
 from oracle import jvp_attention_oracle as orc
 from tests import _oracle_launchers as stand_in
 from tests.test_autograd_wiring import _inputs, cpu_kernels  # noqa: F401
@@ -205,3 +205,15 @@ def test_a_functorch_transform_of_the_cotangent(unwrapping_cpu_kernels, outputs)
     if to is None:
         with pytest.raises(RuntimeError, match="vmap"):
             torch.func.vmap(vjp)(torch.stack([w, u]))
+
+
+def test_another_torch_has_the_call_layer_built_again(monkeypatch, tmp_path):
+    monkeypatch.setattr(build, "NATIVE", tmp_path / "_native.so")
+    monkeypatch.setattr(build, "NATIVE_STAMP", tmp_path / "native.stamp")
+    assert build._native_stale()
+    build.NATIVE.touch()
+    assert build._native_stale()  # built with nobody knows what
+    build.NATIVE_STAMP.write_text(build._native_with())
+    assert not build._native_stale()
+    monkeypatch.setattr(torch, "__version__", "0.0")
+    assert build._native_stale()
