@@ -38,7 +38,7 @@ typedef enum {
   JVPFA_ERR_ARCH = -5,        /* current device is not compute capability 10.x      */
   JVPFA_ERR_CUDA = -6,        /* a CUDA runtime/driver call failed                  */
   JVPFA_ERR_STRUCT = -7,      /* struct_size does not match this library            */
-  JVPFA_ERR_ALIGN = -8,       /* a tensor base pointer is not 16-byte aligned       */
+  JVPFA_ERR_ALIGN = -8,       /* a tensor base pointer is not 16-byte aligned (a tile bitmap: 8 bytes) */
   JVPFA_ERR_UNSUPPORTED = -9, /* valid request that this build cannot serve         */
   JVPFA_ERR_TOO_LARGE = -10,  /* problem exceeds a fixed internal capacity          */
   JVPFA_ERR_DEVICE_STATUS = -11 /* an earlier tcgen05 launch gave up a bounded wait; see jvpfa_device_status */

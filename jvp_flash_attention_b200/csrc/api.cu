@@ -53,6 +53,13 @@ static int check_arch() {
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// The forms of a boolean mask that jvpfa_mask_tiles makes: kernels read and write bits 8 bytes at a time, and the words of
+// the tile bitmaps are 8 bytes.
+static bool mask_forms_aligned(const void* tile_live, const void* tile_live_t, const void* bits, const void* bits_t) {
+  const uintptr_t words = reinterpret_cast<uintptr_t>(tile_live) | reinterpret_cast<uintptr_t>(tile_live_t);
+  return (words & 7u) == 0 && aligned16(bits) && aligned16(bits_t);
+}
+
 static int check_shape(int dtype, int B, int H, int L, int D) {
   if (dtype != JVPFA_BF16 && dtype != JVPFA_FP16 && dtype != JVPFA_FP32 && dtype != JVPFA_FP32_TF32) return JVPFA_ERR_DTYPE;
   if (B < 1 || H < 1 || L < 1) return JVPFA_ERR_SHAPE;
@@ -104,6 +111,7 @@ static int validate_fwd(const jvpfa_fwd_args* a) {
   const void* ptrs[] = {a->q, a->k, a->v, a->tq, a->tk, a->tv, a->o, a->to};
   for (const void* p : ptrs)
     if (p && !aligned16(p)) return JVPFA_ERR_ALIGN;
+  if (!mask_forms_aligned(a->mask_tile_live, nullptr, a->mask_bits, nullptr)) return JVPFA_ERR_ALIGN;
   if (a->impl < JVPFA_IMPL_AUTO || a->impl > JVPFA_IMPL_TCGEN05) return JVPFA_ERR_UNSUPPORTED;
   rc = check_strides(a->in_stride);
   if (rc) return rc;
@@ -131,6 +139,7 @@ static int validate_bwd(const jvpfa_bwd_args* a) {
   for (const void* p : ptrs)
     if (p && !aligned16(p)) return JVPFA_ERR_ALIGN;
   if (a->dq_accum && !aligned16(a->dq_accum)) return JVPFA_ERR_ALIGN;
+  if (!mask_forms_aligned(a->mask_tile_live, a->mask_tile_live_t, a->mask_bits, a->mask_bits_t)) return JVPFA_ERR_ALIGN;
   if (a->impl < JVPFA_IMPL_AUTO || a->impl > JVPFA_IMPL_TCGEN05) return JVPFA_ERR_UNSUPPORTED;
   rc = check_strides(a->in_stride);
   if (rc) return rc;
@@ -269,6 +278,7 @@ int jvpfa_mask_tiles(const jvpfa_mask_tiles_args* args, void* stream) {
   if (a->n_b < 1 || a->n_h < 1 || a->L < 1 || (a->n_rows != 1 && a->n_rows != a->L)) return JVPFA_ERR_SHAPE;
   if ((long long)a->n_b * a->n_h > 65535LL || (a->L + 127) / 128 > 65535) return JVPFA_ERR_TOO_LARGE;  // grid limits
   if (!a->tile_live && (!(a->bits || a->bits_t) || a->head_live || a->tile_live_t)) return JVPFA_ERR_NULL;
+  if (!mask_forms_aligned(a->tile_live, a->tile_live_t, a->bits, a->bits_t)) return JVPFA_ERR_ALIGN;
   if (a->mask.kind != JVPFA_MASK_BOOL || !a->mask.ptr) return JVPFA_ERR_MASK;
   for (int d = 0; d < 4; ++d)
     if (a->mask.stride[d] < 0) return JVPFA_ERR_MASK;
@@ -307,7 +317,7 @@ const char* jvpfa_strerror(int status) {
     case JVPFA_ERR_STRUCT:
       return "struct_size mismatch between caller and library";
     case JVPFA_ERR_ALIGN:
-      return "tensor base pointer is not 16-byte aligned";
+      return "tensor base pointer is not 16-byte aligned (a tile bitmap: 8 bytes)";
     case JVPFA_ERR_UNSUPPORTED:
       return "request not supported by the selected kernel family";
     case JVPFA_ERR_TOO_LARGE:

@@ -1,5 +1,7 @@
 """CPU tests of the native call layer (csrc/native.cpp): what the existing wiring tests do not reach.  Launches go to
 the float64 stand-ins of tests/_oracle_launchers.py."""
+import ctypes
+
 import pytest
 import torch
 import torch.autograd.forward_ad as fwAD
@@ -217,3 +219,34 @@ def test_another_torch_has_the_call_layer_built_again(monkeypatch, tmp_path):
     assert not build._native_stale()
     monkeypatch.setattr(torch, "__version__", "0.0")
     assert build._native_stale()
+
+
+def test_misaligned_forms_of_a_mask_are_refused_by_the_library():
+    """Checked on the host before anything is launched: the kernels read the bits 8 bytes at a time."""
+    lib = _lib.load()
+    x = 1 << 20  # an address that is never followed: the kind of the mask is refused as well
+    refused = 99
+
+    def fwd(**fields):
+        a = _lib.FwdArgs(struct_size=ctypes.sizeof(_lib.FwdArgs), dtype=_lib.BF16, B=1, H=1, L=64, D=64, sm_scale=0.125, q=x, k=x, v=x, o=x,
+                         lse=x, **fields)
+        a.mask.kind = refused
+        return lib.jvpfa_fwd(ctypes.byref(a), None)
+
+    def bwd(**fields):
+        a = _lib.BwdArgs(struct_size=ctypes.sizeof(_lib.BwdArgs), dtype=_lib.BF16, B=1, H=1, L=64, D=64, sm_scale=0.125, q=x, k=x, v=x, go=x,
+                         lse=x, delta=x, dq=x, dk=x, dv=x, **fields)
+        a.mask.kind = refused
+        return lib.jvpfa_bwd(ctypes.byref(a), None)
+
+    def tiles(**fields):
+        a = _lib.MaskTilesArgs(struct_size=ctypes.sizeof(_lib.MaskTilesArgs), n_b=1, n_h=1, n_rows=64, L=64, **fields)
+        a.mask.kind = refused
+        return lib.jvpfa_mask_tiles(ctypes.byref(a), None)
+
+    misaligned = -8
+    for call, fields in ((fwd, ("mask_bits", "mask_tile_live")), (bwd, ("mask_bits", "mask_bits_t", "mask_tile_live", "mask_tile_live_t")),
+                         (tiles, ("bits", "bits_t", "tile_live_t"))):
+        for field in fields:
+            extra = {"tile_live": x} if call is tiles else {}
+            assert call(**extra, **{field: x + 4}) == misaligned, (call.__name__, field)
