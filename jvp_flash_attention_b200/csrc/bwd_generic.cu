@@ -158,17 +158,6 @@ struct BwdCfg {
   }
 };
 
-template <int N>
-__device__ __forceinline__ void zero_acc(float (*x)[4]) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    x[i][0] = 0.f;
-    x[i][1] = 0.f;
-    x[i][2] = 0.f;
-    x[i][3] = 0.f;
-  }
-}
-
 // x += A0 B0^T and, where asked for, y += A1 B0^T (HAS_Y1) + A0 B1^T (HAS_Y2); rows r0.. of A0 / A1, all operands D-contiguous.
 // {S, tS} with (Q, tQ; K, tK), {E, F + dP} with (V, tV; G, gO) of the side in question.
 // TF32: the two products of y have an accumulator each and are added once, rounded (see gemm_out): in a single one the larger
@@ -257,39 +246,16 @@ __device__ __forceinline__ void gemm_out(float (*out)[4], const float (*at0)[4],
   }
 }
 
-// Writes a warp's 16 x D accumulator strip (scaled) into a padded smem tile as T.
-template <typename T, int D>
-__device__ __forceinline__ void acc_to_smem(T* s, int ld, int r0, int lane, const float (*acc)[4], float scale) {
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int dt = 0; dt < D / 8; ++dt) {
-    T* lo = s + (r0 + g) * ld + dt * 8 + 2 * t;
-    T* hi = lo + 8 * ld;
-    lo[0] = Elem<T>::from_float(acc[dt][0] * scale);
-    lo[1] = Elem<T>::from_float(acc[dt][1] * scale);
-    hi[0] = Elem<T>::from_float(acc[dt][2] * scale);
-    hi[1] = Elem<T>::from_float(acc[dt][3] * scale);
-  }
-}
-
-template <typename T, int ROWS, int D, int NTHREADS>
-__device__ __forceinline__ void smem_tile_to_global(T* ghead, const T* s, int ld, int row0, int L, int tid) {
-  constexpr int VEC = 16 / (int)sizeof(T);
-  constexpr int VPR = D / VEC;
-  for (int idx = tid; idx < ROWS * VPR; idx += NTHREADS) {
-    const int r = idx / VPR, c = (idx - r * VPR) * VEC;
-    const int row = row0 + r;
-    if (row < L)
-      *reinterpret_cast<uint4*>(ghead + (size_t)row * D + c) = *reinterpret_cast<const uint4*>(s + r * ld + c);
-  }
-}
-
 // ---- dK, dV: CTA owns 64 keys, loops over query tiles.  Tiles are held transposed
 // (rows = keys, columns = queries) so that P^T etc. feed the second MMAs from registers. ----
+// fp32 (and TF32) at head dimension 32 with tangents: 128 registers, for two CTAs of 64 rows on an SM; the compiler would take
+// up to 163 (B2 H8 L2048, dQ through tO 1025 -> 839 us with what then spills).
+template <typename T, int D, bool HAS_GT, int RG>
+constexpr bool kTwoOnAnSm = !Elem<T>::k16 && D == 32 && HAS_GT && RG == 4;
+
 // TKV: K and V have tangents (JVPFA_ZERO_TKV leaves out what they would be multiplied by; it comes without gO).
-// (Head dimension 32 with 64-row tiles: 128 registers for two CTAs on an SM; the compiler would take 163.)
 template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
-__global__ void __launch_bounds__(32 * RG * KG, !Elem<T>::k16 && D == 32 && HAS_GT && RG == 4 ? 2 : 0) bwd_dkdv_kernel(const jvpfa_bwd_args a) {
+__global__ void __launch_bounds__(32 * RG * KG, kTwoOnAnSm<T, D, HAS_GT, RG> ? 2 : 0) bwd_dkdv_kernel(const jvpfa_bwd_args a) {
   using C = BwdCfg<T, D, RG, KG>;
   constexpr int BN = C::OWN, BM = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES, LW = C::LW;
   constexpr int NQ = LW / 8;
@@ -469,7 +435,7 @@ __global__ void __launch_bounds__(32 * RG * KG, !Elem<T>::k16 && D == 32 && HAS_
 
 // ---- dQ: CTA owns 64 queries, loops over key tiles (rows = queries, columns = keys). ----
 template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
-__global__ void __launch_bounds__(32 * RG * KG) bwd_dq_kernel(const jvpfa_bwd_args a) {
+__global__ void __launch_bounds__(32 * RG * KG, kTwoOnAnSm<T, D, HAS_GT, RG> ? 2 : 0) bwd_dq_kernel(const jvpfa_bwd_args a) {
   using C = BwdCfg<T, D, RG, KG>;
   constexpr int BM = C::OWN, BN = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES, LW = C::LW;
   constexpr int NK = LW / 8;
@@ -663,8 +629,9 @@ static int launch_bwd_split(const jvpfa_bwd_args& a, cudaStream_t s) {
 // Rows x loop parts of a CTA, by the same rule as in the forward.
 template <typename T, int D>
 static int launch_bwd_d(const jvpfa_bwd_args& a, cudaStream_t s) {
+  const long long rows16 = tiles16(a.B, a.H, a.L);
+  if (rows16 >= kBwdRowsFrom<T, D> && (!a.gto || kBwdRowsDual<T, D>)) return launch_bwd_rows(a, s);  // (JVPFA_ZERO_TKV: fp32 with gto)
   if constexpr (!Elem<T>::k16) {
-    const long long rows16 = (long long)((a.L + 15) / 16) * a.B * a.H;
     if (rows16 < 2 * 148) return launch_bwd_split<T, D, 1, 8>(a, s);
     if (rows16 < 4 * 148) return launch_bwd_split<T, D, 2, 4>(a, s);
   }

@@ -25,6 +25,7 @@ struct Elem;
 template <>
 struct Elem<__nv_bfloat16> {
   static constexpr bool k16 = true;
+  static constexpr bool kSplit = false;
   static constexpr int kPad = 8;  // smem row padding in elements (keeps 16-byte rows, spreads banks)
   static constexpr int kKStep = 16;
   __device__ static __forceinline__ uint32_t pack(float lo, float hi) {
@@ -38,6 +39,7 @@ struct Elem<__nv_bfloat16> {
 template <>
 struct Elem<__half> {
   static constexpr bool k16 = true;
+  static constexpr bool kSplit = false;
   static constexpr int kPad = 8;
   static constexpr int kKStep = 16;
   __device__ static __forceinline__ uint32_t pack(float lo, float hi) {
@@ -433,14 +435,77 @@ __device__ __forceinline__ void merge_parts(float4* buf, float (*x)[4], int rg, 
   }
 }
 
+template <int N>
+__device__ __forceinline__ void zero_acc(float (*x)[4]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    x[i][0] = 0.f;
+    x[i][1] = 0.f;
+    x[i][2] = 0.f;
+    x[i][3] = 0.f;
+  }
+}
+
+// Writes a warp's 16 x D accumulator strip (scaled) into a padded smem tile as T.
+template <typename T, int D>
+__device__ __forceinline__ void acc_to_smem(T* s, int ld, int r0, int lane, const float (*acc)[4], float scale) {
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int dt = 0; dt < D / 8; ++dt) {
+    T* lo = s + (r0 + g) * ld + dt * 8 + 2 * t;
+    T* hi = lo + 8 * ld;
+    lo[0] = Elem<T>::from_float(acc[dt][0] * scale);
+    lo[1] = Elem<T>::from_float(acc[dt][1] * scale);
+    hi[0] = Elem<T>::from_float(acc[dt][2] * scale);
+    hi[1] = Elem<T>::from_float(acc[dt][3] * scale);
+  }
+}
+
+template <typename T, int ROWS, int D, int NTHREADS>
+__device__ __forceinline__ void smem_tile_to_global(T* ghead, const T* s, int ld, int row0, int L, int tid) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  constexpr int VPR = D / VEC;
+  for (int idx = tid; idx < ROWS * VPR; idx += NTHREADS) {
+    const int r = idx / VPR, c = (idx - r * VPR) * VEC;
+    const int row = row0 + r;
+    if (row < L)
+      *reinterpret_cast<uint4*>(ghead + (size_t)row * D + c) = *reinterpret_cast<const uint4*>(s + r * ld + c);
+  }
+}
+
 // Raises a kernel's dynamic shared-memory limit once per device (the call costs about a microsecond of host time).
 struct SmemOptIn {
   unsigned long long done = 0;  // bit per device; setting it twice does no harm
   bool ensure(const void* kernel, size_t bytes);
 };
 
+// The register-tiled kernels have two forms: a row group's loop split among several warps (fwd_generic.cu, bwd_generic.cu), and
+// one warp for each 16 rows with little in registers (fwd_rows.cu, bwd_rows.cu).  The first fills the GPU from fewer rows, the
+// second hides more latency once there are enough of them: n16 = 16-row tiles of the call.  Measured on a B200 at n16 = 32,
+// 256, 512, 1008, 2048 and 8192 (split form / one warp form):
+//   forward, O alone     16 bit D64 0.66 at 512, 1.15 at 2048   TF32 D64 0.83 at 1008, 1.29 at 2048   fp32 D64 0.97, 1.30
+//   forward, tangents    16 bit D64 0.93 at 1008, 1.29 at 2048, D32 0.88 at 2048   TF32 D64 1.05, 1.24   fp32 D64 0.97, 1.04, D128 0.80
+//   backward through O   16 bit D64 0.93 at 512, 1.36 at 1008   TF32 D64 0.98 at 512, 1.44 at 1008   fp32 D64 0.71, 1.16
+//   backward, tangents   16 bit D64 0.78 at 512, 1.25 at 1008, D128 0.86   TF32 D32 1.18 at 1008, D64 0.89   fp32 D32 0.99, D64 0.57
+// The lines lie between the sizes of either side, at four (backward) and eight (forward) 16-row tiles for each of the 148 SMs;
+// TF32 at D = 128 gains least from the split (tangents 0.79 at 256, 1.08 at 512) and leaves it at two.  Variants of the second
+// form that are never the better one are not compiled.
+inline long long tiles16(int B, int H, int L) { return (long long)((L + 15) / 16) * B * H; }
+template <typename T, int D>
+constexpr bool kTf32AtD128 = !Elem<T>::k16 && !Elem<T>::kSplit && D == 128;
+template <typename T, int D>
+constexpr long long kFwdRowsFrom = kTf32AtD128<T, D> ? 2 * 148 : 8 * 148;
+template <typename T, int D>
+constexpr long long kBwdRowsFrom = kTf32AtD128<T, D> ? 2 * 148 : 4 * 148;
+template <typename T, int D>
+constexpr bool kFwdRowsDual = Elem<T>::k16 ? D > 32 : Elem<T>::kSplit ? D == 64 : true;
+template <typename T, int D>
+constexpr bool kBwdRowsDual = Elem<T>::k16 ? D <= 64 : !Elem<T>::kSplit && D == 32;
+
 // Host-side launch helpers implemented by each kernel translation unit.
 int launch_fwd_generic(const jvpfa_fwd_args& a, cudaStream_t stream);
+int launch_fwd_rows(const jvpfa_fwd_args& a, cudaStream_t stream);
+int launch_bwd_rows(const jvpfa_bwd_args& a, cudaStream_t stream);
 int launch_pre(const jvpfa_pre_args& a, cudaStream_t stream);
 int launch_bwd_generic(const jvpfa_bwd_args& a, cudaStream_t stream);
 int launch_mask_check(const jvpfa_mask_check_args& a, cudaStream_t stream);

@@ -438,8 +438,9 @@ static int launch_split(const jvpfa_fwd_args& a, cudaStream_t s) {
 // each of the 148 SMs a CTA; below that shorter row tiles (whose warps share out the keys) put more SMs to work.
 template <typename T, int D>
 static int launch_d(const jvpfa_fwd_args& a, cudaStream_t s) {
+  const long long rows16 = tiles16(a.B, a.H, a.L);
+  if (rows16 >= kFwdRowsFrom<T, D> && !(a.flags & JVPFA_ZERO_TKV) && (!a.tq || kFwdRowsDual<T, D>)) return launch_fwd_rows(a, s);
   if constexpr (!Elem<T>::k16) {
-    const long long rows16 = (long long)((a.L + 15) / 16) * a.B * a.H;
     if (rows16 < 2 * 148) return launch_split<T, D, 1, 8>(a, s);
     if (rows16 < 4 * 148) return launch_split<T, D, 2, 4>(a, s);
   }
