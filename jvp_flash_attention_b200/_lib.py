@@ -24,7 +24,7 @@ DTYPE_ENUM = {torch.bfloat16: BF16, torch.float16: FP16, torch.float32: FP32}
 FP32_TF32 = 3  # JVPFA_FP32_TF32: fp32 tensors, products as one TF32 MMA
 
 # How fp32 inputs are multiplied: "3xtf32" (default; error ~1e-6 relative) or "tf32" (one TF32 MMA per product, the
-# precision of upstream's fp32 path; error ~5e-4, about 2.5x faster).  Set through jvp_attention.set_fp32_precision.
+# precision of upstream's fp32 path; error ~5e-4, about twice as fast).  Set through jvp_attention.set_fp32_precision.
 FP32_PRECISION = "3xtf32"
 
 

@@ -1,4 +1,4 @@
-// Persistent, pipelined tcgen05 backward for head dimension 64 (bf16 / fp16; none, causal, key
+// Persistent, pipelined tcgen05 backward for head dimension 64, and 32 on half-filled tiles (bf16 / fp16; none, causal, key
 // padding).
 //
 // Same mathematics and the same two launches as bwd_tc5.cu (own 128 keys -> dK, dV; own 128

@@ -13,6 +13,8 @@
 // is applied as scale*QK^T + bias (SDPA semantics; upstream scales the bias too,
 // jvp_attention.py:247-251), and boolean masking uses -inf rather than adding -100.
 //
+// It serves fp32 and what the tcgen05 kernels do not take of the 16-bit types; with many rows, and where that is faster, the
+// form with one warp for each 16 rows does instead (fwd_rows.cu; common.cuh says where the lines lie).
 // What bounds it: mma.sync, at 512 (TF32) or 1024 (16-bit) multiply-adds per clock and SM, measured; an fp32 product is
 // three TF32 instructions.  One instruction occupies its quarter of the SM for 8 cycles and returns after 21, and the
 // fp32 products of one accumulator are a chain, so the split matters: 64 rows x D=128 fp32 fill the shared memory of an

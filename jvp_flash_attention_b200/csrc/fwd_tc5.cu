@@ -112,10 +112,11 @@ bool encode_map4d_f32(CUtensorMap* m, const void* ptr, int D, int L, int H, int 
 
 }  // namespace tc5
 
-// Head dimension 32 runs on the D = 64 kernels: the tensor maps end at column 32, so TMA fills the other half of every
-// tile with zeros and clips what is stored, and the contractions over D stop half-way.  An MMA costs the same for 32
-// output columns as for 64, so little is wasted (B4 H8 L1000, bf16: forward with tangents 144 -> 33 us, backward through both
-// outputs 302 -> 69 us against the register-tiled kernels).  Up to one 64-row tile the register-tiled kernels stay: a 256-row pair of query tiles would be mostly padding.
+// Head dimension 32 runs on the D = 64 kernels (the backward on the two launches of bwd_tc5_d64.cu): the tensor maps end at
+// column 32, so TMA fills the other half of every tile with zeros and clips what is stored, and the contractions over D stop
+// half-way.  An MMA costs the same for 32 output columns as for 64, so little is wasted (B4 H8 L1000, bf16: forward with tangents
+// 150 -> 46 us, backward through both outputs 325 -> 99 us against the register-tiled kernels).  Up to one 64-row tile the
+// register-tiled kernels stay: a 256-row pair of query tiles would be mostly padding.
 bool tc5_head_dim(int D, int L) { return D == 64 || D == 128 || (D == 32 && L > 64); }
 
 bool fwd_tc5_eligible(const jvpfa_fwd_args& a) {
@@ -145,7 +146,8 @@ bool tc5_mask_layout(const jvpfa_mask& m, int dtype, int L) {
 // with a reference up to 2^8 below it (lazy rescaling) it is rounded like the others.  At a few hundred keys that is a part
 // of the error that shows: O against 64 bits, B2 H4 D32, L512 fp16 with bias 2.56e-4 -> 2.90e-4, L1000 bf16 2.21e-3 ->
 // 2.33e-3.  What the register-tiled kernels (exact) served before these kernels could, keeps their error: head dimension
-// 32, and masks and bias that cannot be read in place as whole 16-byte pieces of rows.
+// 32, and masks and bias that cannot be read in place as whole 16-byte pieces of rows (B4 H8 L1000 D32: forward with tangents
+// 40 -> 46 us; B2 H12 L1330 D64 with bias 183 -> 191 us).
 static bool exact_row_max(const jvpfa_fwd_args& a) {
   if (a.D == 32) return true;
   const bool by_element = a.mask.kind == JVPFA_MASK_BOOL || a.mask.kind == JVPFA_MASK_BIAS;

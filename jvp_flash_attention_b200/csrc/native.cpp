@@ -2,9 +2,10 @@
 // autograd graph around them, behind one Python entry point (`attend`).
 //
 // What bounds the calls it serves is host time, not the GPU: up to a few hundred microseconds of kernels, the pass of a
-// program was the Python layer's.  Measured on a B200 machine before and after (a pass through the public API, kernels
-// excluded): attention() 55 -> 9 us, fwd_dual + gradients through both outputs on forward-AD dual tensors about 400 -> 90 us,
-// under torch.func.jvp about 600 -> 250 us (of which torch.func.jvp itself takes some 150).
+// program was the Python layer's.  Measured on a B200 machine before and after, whole passes through the public API:
+// attention() at B2 H12 L32 D64 43 -> 9 us, fwd_dual on forward-AD dual tensors at L256 96 -> 28 us, fwd_dual and the
+// gradients through both outputs under torch.func.jvp (fp32, B2 H4 L256 D64) 493 -> 207 us, of which torch.func.jvp itself
+// takes some 150.
 //
 // Graph: one node with two outputs, O and tO.  Autograd hands it both cotangents at once, so a loss on both outputs is
 // one backward launch.  Under create_graph the gradient through O is a node that can be differentiated once more (the
@@ -12,7 +13,9 @@
 // The tangent rides on O as its forward-mode gradient, set directly instead of through make_dual's view.
 //
 // CUDA tensors go straight to the library.  For tensors of another device the launch is handed back to the Python
-// module's _launch_fwd / _launch_bwd (the CPU suite puts its oracle there), so there is one graph, not two.
+// module's _launch_fwd / _launch_bwd (the CPU suite puts its oracle there), so that its tests run this graph.
+// The Functions of the Python module serve what this layer declines: nested functorch transforms, cotangents that belong to
+// one, JVPAttn.apply, and calls that are refused.
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/functorch/DynamicLayer.h>
@@ -228,7 +231,8 @@ bool whole_pieces(const MaskDesc& m, int64_t L) {
 
 // Packs a call's boolean mask.  Bits are made anew by every call and not kept with the mask's description: the entries that
 // the kernels read are then those that the mask holds when they run, also where it was written behind torch's version
-// counter (a replayed graph, a foreign kernel, `.data`).
+// counter (a replayed graph, a foreign kernel).  Which tiles are stepped over, and the lengths of a key-padding mask, are
+// those of its verification.
 //
 // Packing reads the mask once (HBM bound) and saves a kernel that reads it one 16-byte piece per row and sub-tile.
 // B2 H12 L2048 D64, 100 MB of mask: packing 32 us; forward with tangents 168 -> 151 us, backward through tO 239 -> 186.

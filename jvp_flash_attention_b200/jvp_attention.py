@@ -107,7 +107,8 @@ def set_fp32_precision(mode: str) -> str:
 
     ``"3xtf32"`` (default): every product as three TF32 MMAs on a hi/lo split, about 1e-6 relative error.
     ``"tf32"``: one TF32 MMA per product, about 5e-4 -- what upstream's fp32 path computes (its ``tl.dot`` calls
-    run on TF32 tensor cores, jvp_attention.py:233-236; its fp32 tolerance is 2.35e-2), about 2.5x faster.
+    run on TF32 tensor cores, jvp_attention.py:233-236; its fp32 tolerance is 2.35e-2), 1.7 to 2.2 times
+    as fast (B2 H8 L2048 D64: O 479 -> 241 us, its backward 1885 -> 988, fwd_dual 1280 -> 605).
     A call's backward (and double backward) runs at the precision its forward ran at: the mode is recorded with the
     call, so changing it in between affects later forwards only."""
     if mode not in ("3xtf32", "tf32"):
@@ -118,10 +119,12 @@ def set_fp32_precision(mode: str) -> str:
 
 # What classify_mask found out about a mask tensor, kept while the same tensor object is passed again unmodified
 # (same Python object, same version counter, which every in-place operation of torch bumps, and still the same memory and
-# layout, which an assignment to `.data` changes).  A mask is typically
-# built once and used by every layer and step; its verification is a pass over B*H*L*L elements and a read-back.
-# Writes that bypass torch (a foreign kernel writing through the raw pointer) are not seen; MASK_MEMO_ENABLED = False
-# turns the memo off.
+# layout, which an assignment to `.data` changes).  A mask is typically built once and used by every layer and step; its
+# verification is a pass over B*H*L*L elements and a read-back.
+# What is kept: that the mask is a valid one, which tiles of a boolean mask are stepped over, and the lengths of a
+# key-padding mask.  Writes that bypass torch's counter (a foreign kernel, a captured graph that is replayed after the mask
+# was changed) are not seen by these; the entries themselves are read by every launch.  MASK_MEMO_ENABLED = False turns the
+# memo off.
 MASK_MEMO_ENABLED = True
 _MASK_MEMO: dict = {}
 _MASK_MEMO_MAX = 16
@@ -695,8 +698,8 @@ class _Box:
 
 class _Attn(Function):
     """The general route of ``JVPAttn.fwd`` and ``JVPAttn.fwd_dual`` (functorch transforms other than a lone
-    ``torch.func.jvp``): the same forward, jvp and backward as ``JVPAttn``, whose second output is one opaque holder of (o_t, M, mu, mask description, scale) instead of upstream's nested
-    NamedTuples.  Under ``torch.func.jvp`` every output of a custom Function is wrapped and unwrapped as a pytree once
+    ``torch.func.jvp``): the same forward, jvp and backward as ``JVPAttn``, whose second output is one opaque holder of
+    (o_t, M, mu, mask description, scale) instead of upstream's nested NamedTuples.  Under ``torch.func.jvp`` every output of a custom Function is wrapped and unwrapped as a pytree once
     per transform level; the NamedTuples (some twenty leaves) made that the larger part of a call's host time.
     ``JVPAttn.apply`` keeps upstream's output structure for callers that use it directly."""
 

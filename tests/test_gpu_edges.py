@@ -1,5 +1,6 @@
 """GPU tests at the edges of the dispatch: head dimension 32 on the D = 64 tensor-core kernels, masks whose rows do not
-fill 16-byte pieces, the row / key splits of the register-tiled kernels, and gradients that nobody asked for."""
+fill 16-byte pieces, the forms of the register-tiled kernels, the range of fp32, gradients that nobody asked for, and what a
+call takes of memory and of the interpreter."""
 import threading
 import time
 
@@ -86,7 +87,7 @@ def test_masks_whose_rows_do_not_fill_16_byte_pieces(D, dt, L, kind, cot):
     (2, 12, 450, "bias", "both"),
 ])
 def test_row_and_key_splits_of_the_register_tiled_kernels(D, B, H, L, kind, cot):
-    """16-row tiles below 296 of them run as 1 x 8 warps, below 592 as 2 x 4, above as 4 x 2."""
+    """16-row tiles below 296 of them run as 1 x 8 warps, below 592 as 2 x 4, above as 4 x 2 (through O alone: one warp each)."""
     _check(B, H, L, D, "fp32", kind, cot)
 
 
@@ -115,7 +116,8 @@ def test_gradients_nobody_asked_for_are_left_out(dt, D, want):
 @pytest.mark.parametrize("how", ["data", "graph"])
 def test_a_mask_written_behind_the_version_counter_is_read_as_it_is(kind, L, D, how):
     """Neither a write through ``.data`` nor one between two replays of a graph moves the counter that the mask's
-    verification is remembered by; what the kernels read has to be the new entries all the same."""
+    verification is remembered by; what the kernels read has to be the new entries all the same.  (Dense masks and bias:
+    which tiles are stepped over, and key lengths, are those of the verification.)"""
     q, k, v, tq, tk, tv, _, _ = (x.to(DEV) for x in _inputs(2, 3, L, D, torch.bfloat16, 6))
     first, second = (_mask(kind, 2, 3, L, torch.bfloat16, s).to(DEV) for s in (1, 2))
     a = [x.clone().requires_grad_() for x in (q, k, v)]
