@@ -27,7 +27,7 @@
 extern "C" {
 #endif
 
-#define JVPFA_VERSION 101 /* major*100 + minor; 101: fields after the last of 100 in four structs, see struct_size there */
+#define JVPFA_VERSION 102 /* major*100 + minor; 101: fields after the last of 100 in four structs; 102: workspace in two */
 
 typedef enum {
   JVPFA_OK = 0,
@@ -123,9 +123,19 @@ typedef struct {
   const void* mask_bits;
   /* 0 or JVPFA_ZERO_TKV.  (struct_size up to mask_tile_live: 0.) */
   int32_t flags;
+  /* Optional caller-owned scratch of the call, JVPFA_FP32 only: jvpfa_fwd_workspace() bytes, 16-byte aligned, contents
+   * irrelevant.  With it the call runs on the tcgen05 tensor cores, which multiply three bf16 parts of every entry; the
+   * parts are made there first.  NULL or too small: the register-tiled kernels.  (struct_size up to flags: NULL.) */
+  void* workspace;
+  int64_t workspace_bytes;
 } jvpfa_fwd_args;
 
 int jvpfa_fwd(const jvpfa_fwd_args* args, void* stream);
+
+/* Bytes of jvpfa_fwd_args.workspace with which this call (workspace itself not looked at) runs on the tcgen05 kernels;
+ * 0 if it gains nothing from one, or for arguments that jvpfa_fwd refuses.  impl JVPFA_IMPL_TCGEN05: whether it gains or not.
+ * Pure host logic. */
+int64_t jvpfa_fwd_workspace(const jvpfa_fwd_args* args);
 
 /*
  * jvpfa_bwd_preprocess -- per-row reductions needed by jvpfa_bwd.
@@ -200,7 +210,16 @@ typedef struct {
   /* Optional, JVPFA_MASK_BOOL only, both or neither: `bits` and `bits_t` of jvpfa_mask_tiles, as in jvpfa_fwd_args. */
   const void* mask_bits;
   const void* mask_bits_t;
+  /* Optional caller-owned scratch of the call, as in jvpfa_fwd_args: jvpfa_bwd_workspace() bytes.  (struct_size up to
+   * mask_bits_t: NULL.) */
+  void* workspace;
+  int64_t workspace_bytes;
 } jvpfa_bwd_args;
+
+/* As jvpfa_fwd_workspace.  Non-zero for JVPFA_FP32 through O, and for dQ alone (JVPFA_SKIP_DKDV) through tO with
+ * JVPFA_ZERO_TKV.  These recompute the scores as jvpfa_fwd with its workspace forms them, the other kernels as jvpfa_fwd without:
+ * lse and mu fit the scores to the last bit when both calls of a pair are given a workspace, or neither. */
+int64_t jvpfa_bwd_workspace(const jvpfa_bwd_args* args);
 
 #define JVPFA_SKIP_DQ 1
 #define JVPFA_SKIP_DKDV 2

@@ -38,8 +38,10 @@ def compute_enum(t: torch.Tensor, fp32_mode: str | None = None) -> int:
 
 EXPORTS = (
     "jvpfa_fwd",
+    "jvpfa_fwd_workspace",
     "jvpfa_bwd_preprocess",
     "jvpfa_bwd",
+    "jvpfa_bwd_workspace",
     "jvpfa_strerror",
     "jvpfa_version",
     "jvpfa_last_cuda_error",
@@ -90,6 +92,8 @@ class FwdArgs(C.Structure):
         ("mask_tile_live", C.c_void_p),
         ("mask_bits", C.c_void_p),
         ("flags", C.c_int32),
+        ("workspace", C.c_void_p),
+        ("workspace_bytes", C.c_int64),
     ]
 
 
@@ -146,6 +150,8 @@ class BwdArgs(C.Structure):
         ("flags", C.c_int32),
         ("mask_bits", C.c_void_p),
         ("mask_bits_t", C.c_void_p),
+        ("workspace", C.c_void_p),
+        ("workspace_bytes", C.c_int64),
     ]
 
 
@@ -222,10 +228,14 @@ def load() -> C.CDLL:
     lib = C.CDLL(str(LIB_PATH))
     lib.jvpfa_fwd.argtypes = [C.POINTER(FwdArgs), C.c_void_p]
     lib.jvpfa_fwd.restype = C.c_int
+    lib.jvpfa_fwd_workspace.argtypes = [C.POINTER(FwdArgs)]
+    lib.jvpfa_fwd_workspace.restype = C.c_int64
     lib.jvpfa_bwd_preprocess.argtypes = [C.POINTER(PreArgs), C.c_void_p]
     lib.jvpfa_bwd_preprocess.restype = C.c_int
     lib.jvpfa_bwd.argtypes = [C.POINTER(BwdArgs), C.c_void_p]
     lib.jvpfa_bwd.restype = C.c_int
+    lib.jvpfa_bwd_workspace.argtypes = [C.POINTER(BwdArgs)]
+    lib.jvpfa_bwd_workspace.restype = C.c_int64
     lib.jvpfa_strerror.argtypes = [C.c_int]
     lib.jvpfa_strerror.restype = C.c_char_p
     lib.jvpfa_version.argtypes = []
@@ -303,7 +313,7 @@ class MaskSpec:
     bias, or int32 kv_len) and ``strides`` are the broadcast element strides of a (B,H,L,L) view.
     """
 
-    __slots__ = ("kind", "tensor", "strides", "bias_dtype", "tile_live", "tile_live_t", "fp32_mode", "_native")
+    __slots__ = ("kind", "tensor", "strides", "bias_dtype", "tile_live", "tile_live_t", "fp32_mode", "fp32_parts", "_native")
 
     def __init__(self, kind=MASK_NONE, tensor=None, strides=(0, 0, 0, 0), bias_dtype=FP32):
         self.kind = kind
@@ -313,6 +323,7 @@ class MaskSpec:
         self.tile_live = None  # MASK_BOOL: bitmap from mask_tiles(), lets the forward step over dead tiles
         self.tile_live_t = None  # ... and its transpose (per 128-key tile), for the backward launch that owns keys
         self._native = None  # the native layer's form of this description, made on first use
+        self.fp32_parts = False  # the forward of this call ran on the fp32 tcgen05 kernels: so does a backward through O
         self.fp32_mode = None  # fp32 precision the forward of this call ran under ("3xtf32" / "tf32"); None = current
 
     def native(self):
@@ -471,6 +482,10 @@ def bwd(q, k, v, tq, tk, tv, go, gto, lse, mu, delta, eps, cterm, dq, dk, dv, ma
     if in_stride is not None:
         a.in_stride[0], a.in_stride[1], a.in_stride[2] = in_stride
     a.dq_accum = ptr(dq_accum)
+    workspace = None
+    if mask.fp32_parts and (n := lib.jvpfa_bwd_workspace(C.byref(a))):
+        workspace = torch.empty(n, device=q.device, dtype=torch.uint8)
+        a.workspace, a.workspace_bytes = ptr(workspace), n
     check(_launch(q, lib.jvpfa_bwd, a), "jvpfa_bwd")
 
 

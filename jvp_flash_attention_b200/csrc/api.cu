@@ -146,17 +146,22 @@ static int validate_bwd(const jvpfa_bwd_args* a) {
   return check_mask(a->mask);
 }
 
-// The arguments as this build knows them: a caller built before the last field was added passes a shorter struct.
-template <typename Args>
-static const Args* current_args(const Args* a, Args* full, size_t size_before) {
-  if (!a || a->struct_size != (int32_t)size_before) return a;
+// The arguments as this build knows them: a caller built before the last fields were added passes a shorter struct, of one
+// of the sizes that earlier versions had.
+template <typename Args, typename... Sizes>
+static const Args* current_args(const Args* a, Args* full, Sizes... earlier) {
+  if (!a || !((a->struct_size == (int32_t)earlier) || ...)) return a;
+  const size_t size = (size_t)a->struct_size;
   *full = Args{};
-  memcpy(full, a, size_before);
+  memcpy(full, a, size);
   full->struct_size = (int32_t)sizeof(Args);
   return full;
 }
+static const jvpfa_fwd_args* current_fwd_args(const jvpfa_fwd_args* a, jvpfa_fwd_args* full) {
+  return current_args(a, full, offsetof(jvpfa_fwd_args, mask_bits), offsetof(jvpfa_fwd_args, workspace));
+}
 static const jvpfa_bwd_args* current_bwd_args(const jvpfa_bwd_args* a, jvpfa_bwd_args* full) {
-  return current_args(a, full, offsetof(jvpfa_bwd_args, flags));
+  return current_args(a, full, offsetof(jvpfa_bwd_args, flags), offsetof(jvpfa_bwd_args, workspace));
 }
 
 static int validate_pre(const jvpfa_pre_args* a) {
@@ -185,7 +190,7 @@ int check_bwd_request(const jvpfa_bwd_args* a) {
   if (rc) return rc;
   rc = check_arch();
   if (rc) return rc;
-  const bool tc5 = bwd_tc5_eligible(*a);
+  const bool tc5 = bwd_tc5_eligible(*a) || bwd_f32_tc5_eligible(*a);
   const int fam = impl_family(a->impl);
   if (fam == JVPFA_IMPL_TCGEN05 && !tc5) return JVPFA_ERR_UNSUPPORTED;
   return JVPFA_OK;
@@ -199,10 +204,16 @@ extern "C" {
 
 int jvpfa_fwd_uses_tcgen05(const jvpfa_fwd_args* args) {
   jvpfa_fwd_args full;
-  const jvpfa_fwd_args* a = current_args(args, &full, offsetof(jvpfa_fwd_args, mask_bits));
+  const jvpfa_fwd_args* a = current_fwd_args(args, &full);
   if (validate_fwd(a) != JVPFA_OK) return 0;
   if (a->impl == JVPFA_IMPL_GENERIC) return 0;
-  return fwd_tc5_eligible(*a) ? 1 : 0;
+  return fwd_tc5_eligible(*a) || fwd_f32_tc5_eligible(*a) ? 1 : 0;
+}
+
+int64_t jvpfa_fwd_workspace(const jvpfa_fwd_args* args) {
+  jvpfa_fwd_args full;
+  const jvpfa_fwd_args* a = current_fwd_args(args, &full);
+  return validate_fwd(a) == JVPFA_OK ? fwd_f32_tc5_workspace(*a) : 0;
 }
 
 int jvpfa_bwd_uses_tcgen05(const jvpfa_bwd_args* args) {
@@ -210,23 +221,33 @@ int jvpfa_bwd_uses_tcgen05(const jvpfa_bwd_args* args) {
   const jvpfa_bwd_args* a = current_bwd_args(args, &full);
   if (validate_bwd(a) != JVPFA_OK) return 0;
   if (impl_family(a->impl) == JVPFA_IMPL_GENERIC) return 0;
-  return bwd_tc5_eligible(*a) ? 1 : 0;
+  return bwd_tc5_eligible(*a) || bwd_f32_tc5_eligible(*a) ? 1 : 0;
+}
+
+int64_t jvpfa_bwd_workspace(const jvpfa_bwd_args* args) {
+  jvpfa_bwd_args full;
+  const jvpfa_bwd_args* a = current_bwd_args(args, &full);
+  return validate_bwd(a) == JVPFA_OK ? bwd_f32_tc5_workspace(*a) : 0;
 }
 
 int jvpfa_fwd(const jvpfa_fwd_args* args, void* stream) {
   jvpfa_fwd_args full;
-  const jvpfa_fwd_args* a = current_args(args, &full, offsetof(jvpfa_fwd_args, mask_bits));
+  const jvpfa_fwd_args* a = current_fwd_args(args, &full);
   int rc = validate_fwd(a);
   if (rc) return rc;
   rc = check_arch();
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const bool tc5 = fwd_tc5_eligible(*a);
-  if (a->impl == JVPFA_IMPL_TCGEN05 && !tc5) return JVPFA_ERR_UNSUPPORTED;
+  const bool tc5 = fwd_tc5_eligible(*a), f32 = fwd_f32_tc5_eligible(*a);
+  if (a->impl == JVPFA_IMPL_TCGEN05 && !tc5 && !f32) return JVPFA_ERR_UNSUPPORTED;
   // strided inputs are read in place by both kernel families (tensor maps or plain row strides)
   if (tc5 && a->impl != JVPFA_IMPL_GENERIC) {
     if (tc5_status_peek() != 0) return JVPFA_ERR_DEVICE_STATUS;
     return launch_fwd_tc5(*a, s);
+  }
+  if (f32) {
+    if (tc5_status_peek() == 0) return launch_fwd_f32_tc5(*a, s);
+    if (a->impl == JVPFA_IMPL_TCGEN05) return JVPFA_ERR_DEVICE_STATUS;  // else: fp32 is served whatever a tcgen05 launch left
   }
   return launch_fwd_generic(*a, s);
 }
@@ -250,6 +271,10 @@ int jvpfa_bwd(const jvpfa_bwd_args* args, void* stream) {
   if (tc5 && fam != JVPFA_IMPL_GENERIC) {
     if (tc5_status_peek() != 0) return JVPFA_ERR_DEVICE_STATUS;
     return launch_bwd_tc5(*a, s);
+  }
+  if (bwd_f32_tc5_eligible(*a)) {
+    if (tc5_status_peek() == 0) return launch_bwd_f32_tc5(*a, s);
+    if (fam == JVPFA_IMPL_TCGEN05) return JVPFA_ERR_DEVICE_STATUS;
   }
   return launch_bwd_generic(*a, s);
 }

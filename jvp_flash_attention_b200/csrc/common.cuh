@@ -527,6 +527,12 @@ int launch_fwd_tc5_pipe128(const jvpfa_fwd_args& a, cudaStream_t stream);
 bool bwd_tc5_pipe128_eligible(const jvpfa_bwd_args& a);
 int launch_bwd_tc5_pipe128(const jvpfa_bwd_args& a, cudaStream_t stream);
 bool bwd_tc5_eligible(const jvpfa_bwd_args& a);
+long long fwd_f32_tc5_workspace(const jvpfa_fwd_args& a);
+bool fwd_f32_tc5_eligible(const jvpfa_fwd_args& a);
+int launch_fwd_f32_tc5(const jvpfa_fwd_args& a, cudaStream_t stream);
+long long bwd_f32_tc5_workspace(const jvpfa_bwd_args& a);
+bool bwd_f32_tc5_eligible(const jvpfa_bwd_args& a);
+int launch_bwd_f32_tc5(const jvpfa_bwd_args& a, cudaStream_t stream);
 void set_last_cuda_error(cudaError_t e, const char* where);
 int check_pre_request(const jvpfa_pre_args* a);
 int check_bwd_request(const jvpfa_bwd_args* a);

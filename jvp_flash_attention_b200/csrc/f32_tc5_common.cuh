@@ -1,0 +1,131 @@
+// fp32 on the 16-bit tensor cores, without loss: what the kernels of fwd_f32_tc5.cu share.
+//
+// An fp32 number x is the sum of three bf16 numbers, hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid (24 significant bits
+// are 8 + 8 + 8, the differences are exact), and bf16 has fp32's range of exponents, so every entry keeps its precision
+// whatever else its row or column holds.  A product is the six MMAs hi*hi, hi*mid, mid*hi, mid*mid, hi*lo, lo*hi; what is left
+// out (mid*lo, lo*mid, lo*lo) is below 2^-26 of it.
+//
+// The inputs are split once per call into a caller-owned workspace: three row-major (B*H, L, D) planes of bf16 per tensor,
+// all of them one tensor map (D, L, B*H, planes).
+#pragma once
+
+#include "tc5_common.cuh"
+
+namespace jvpfa {
+namespace tc5 {
+
+constexpr int kF32MaxSlots = 6;
+
+struct SplitArgs {
+  const float* src[kF32MaxSlots];
+  long long st[kF32MaxSlots][3];  // batch, head, row strides in elements
+  __nv_bfloat16* dst;             // [slot][part][B*H][L][D]
+  long long plane;                // B*H*L*D
+  int H, L, D;
+  void set(int slot, const void* p, const int64_t* in_stride) {  // in_stride all zero or null: row-major
+    src[slot] = static_cast<const float*>(p);
+    const bool strided = in_stride && (in_stride[0] | in_stride[1] | in_stride[2]) != 0;
+    st[slot][0] = strided ? in_stride[0] : (long long)H * L * D;
+    st[slot][1] = strided ? in_stride[1] : (long long)L * D;
+    st[slot][2] = strided ? in_stride[2] : D;
+  }
+};
+
+// One value as three bf16 parts.  A value that rounds beyond bf16's range is cut instead; Inf and NaN make all that they enter NaN.
+__device__ __forceinline__ void split3(float x, float& h, float& m, float& l) {
+  uint32_t hb = __float_as_uint(__bfloat162float(__float2bfloat16_rn(x)));
+  if ((hb & 0x7fffffffu) == 0x7f800000u) hb = __float_as_uint(x) & 0xffff0000u;
+  h = __uint_as_float(hb);
+  const float r = x - h;
+  m = __bfloat162float(__float2bfloat16_rn(r));
+  l = r - m;
+}
+// Two values, packed: the form in which they are stored or handed to the tensor cores.
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
+__device__ __forceinline__ void split3_pair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+  h = pack_bf16(a, b);
+  const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
+  m = pack_bf16(ra, rb);
+  l = pack_bf16(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
+}
+
+// What a thread reads of the mask: 32 neighbouring keys of its query row i at a time.
+// MK: 0 = none / causal / key padding; 1 = boolean mask (bits, or bytes of any strides); 2 = additive bias (any type and
+// strides).
+template <int MK>
+struct F32RowMask {
+  MaskView mv;
+  const unsigned char* row;
+  const uint32_t* bits;
+  int L, i, esz;
+  bool vec;  // the row can be read 16 bytes at a time
+
+  __device__ __forceinline__ F32RowMask(const jvpfa_mask& m, const void* mask_bits, int b, int h, int H, int i_, int L_)
+      : mv(make_mask_view(m, b, h, L_)), row(nullptr), bits(nullptr), L(L_), i(min(i_, L_ - 1)), esz(1), vec(false) {
+    if constexpr (MK != 0) {
+      if (MK == 2) esz = m.bias_dtype == JVPFA_FP32 ? 4 : 2;
+      row = reinterpret_cast<const unsigned char*>(mv.base) + (long long)i * mv.si * esz;
+      vec = mv.sj == 1 && (reinterpret_cast<uintptr_t>(row) & 15u) == 0;
+      if (MK == 1 && mask_bits != nullptr) bits = mask_bit_row(mask_bits, m, mask_head(m, b, h, H), i, L);
+    }
+  }
+  // Keys n0 .. n0 + 31: a bit for each that the mask lets the row attend, of those in `live`; the bias.
+  __device__ __forceinline__ uint32_t fetch(int n0, uint32_t live, float* bias) const {
+    if constexpr (MK == 1) {
+      uint32_t r = 0u;
+      if (bits != nullptr) {
+        r = n0 < L ? ldg_nc_u32(bits + (n0 >> 5)) : 0u;
+      } else if (vec && n0 + 32 <= L) {
+        const uint4 r0 = ldg_nc_v4(row + n0), r1 = ldg_nc_v4(row + n0 + 16);
+        r = bits_of_bytes(r0.x) | bits_of_bytes(r0.y) << 4 | bits_of_bytes(r0.z) << 8 | bits_of_bytes(r0.w) << 12 |
+            bits_of_bytes(r1.x) << 16 | bits_of_bytes(r1.y) << 20 | bits_of_bytes(r1.z) << 24 | bits_of_bytes(r1.w) << 28;
+      } else {
+#pragma unroll 8
+        for (int c = 0; c < 32; ++c) r |= (ldg_nc_u8(row + (long long)min(n0 + c, L - 1) * mv.sj) != 0u ? 1u : 0u) << c;
+      }
+      live &= r;
+    }
+    if constexpr (MK == 2) {
+      // (the piece of two 64-key tiles on is brought into L2 meanwhile: a row's pieces lie in DRAM pages of their own)
+      if (mv.sj == 1 && n0 + 128 < L) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + (size_t)(n0 + 128) * esz));
+      if (vec && n0 + 32 <= L && esz == 4) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const uint4 r = ldg_nc_v4(row + (size_t)(n0 + 4 * c) * 4);
+          bias[4 * c] = __uint_as_float(r.x), bias[4 * c + 1] = __uint_as_float(r.y);
+          bias[4 * c + 2] = __uint_as_float(r.z), bias[4 * c + 3] = __uint_as_float(r.w);
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) bias[c] = mv.bias(i, min(n0 + c, L - 1));
+      }
+    }
+    return live;
+  }
+};
+
+// From how many rows on the register-tiled kernels, which fill the GPU from fewer, are the slower ones.  Measured on a B200,
+// us, register-tiled / here, for O alone and with tangents; n16 = 16-row tiles of the call:
+//   D = 128  n16 256 (L2048) 249/101 469/249, causal 137/101 250/251; n16 288 (L130) 33/26 55/48; n16 416 (L200) 45/32 96/60;
+//            n16 1024 (L1024) 297/73 679/169; 64-row sequences, n16 1024: 33/36 63/62
+//   D = 64   n16 256 (L512) 34/30 71/46, bias 36/42 74/65; n16 384 (L500) 59/30 121/50, bias 59/38 123/71; n16 1024 (L1024) 169/48
+//            338/89; 64-row sequences, n16 1024: 21/26 35/38
+//   D = 32   n16 528 (L700) 50/34 82/50, bias 49/48 82/87; n16 1152 (L130) 27/30 49/42; n16 1024 (L1024) 84/42 169/71, bias 99/71
+//            183/114; n16 1664 (L200) 45/34 80/54
+inline bool f32_rows_enough(int B, int H, int L, int D) {
+  const long long n16 = tiles16(B, H, L);
+  if (D == 128) return L > 64 && n16 >= 320;
+  if (D == 64) return L > 64 && n16 >= 384;
+  return L >= 192 && n16 >= 1024;
+}
+
+// Host: the splitting launch, and the tensor map of its result (boxes of 64 columns x 64 rows of one plane).
+int launch_split3(const SplitArgs& s, int slots, cudaStream_t stream);
+bool encode_map_parts(CUtensorMap* m, const void* ptr, int D, int L, int BH, int planes);
+
+}  // namespace tc5
+}  // namespace jvpfa

@@ -110,6 +110,10 @@ bool encode_map4d_f32(CUtensorMap* m, const void* ptr, int D, int L, int H, int 
   return r == CUDA_SUCCESS;
 }
 
+bool encode_map_parts(CUtensorMap* m, const void* ptr, int D, int L, int BH, int planes) {
+  return encode_map4d(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, ptr, D, L, BH, planes, nullptr, 64);
+}
+
 }  // namespace tc5
 
 // Head dimension 32 runs on the D = 64 kernels (the backward on the two launches of bwd_tc5_d64.cu): the tensor maps end at

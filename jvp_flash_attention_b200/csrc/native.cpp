@@ -83,6 +83,10 @@ struct Call {
   MaskPtr mask;
   double scale;
   bool tf32;  // fp32 tensors: one TF32 product instead of three, recorded so that the backward recomputes what the forward saw
+  // fp32: whatever is asked of the call's backward, the tcgen05 kernels form it, which recompute the scores as the tcgen05
+  // forward forms them.  (A backward of the register-tiled kernels, whose scores are off in their own way, keeps the forward
+  // whose lse is off in the same.)
+  bool parts = false;
   // A boolean mask as bits, by rows and transposed: the form the 16-bit tensor-core kernels read best, made by this call for
   // its forward and backward (pack_mask).
   Tensor bits, bits_t;
@@ -229,6 +233,32 @@ bool whole_pieces(const MaskDesc& m, int64_t L) {
   return ok;
 }
 
+// Bits by rows and, if asked for, transposed; both stay undefined where there is no memory or the mask is too large.
+void pack(const MaskDesc& m, const Tensor& q, Tensor& bits_out, Tensor* bits_t_out) {
+  const int64_t L = q.size(2);
+  const int64_t n_b = m.c.stride[0] ? m.tensor.size(0) : 1, n_h = m.c.stride[1] ? m.tensor.size(1) : 1;
+  const int64_t n_rows = m.c.stride[2] ? L : 1;
+  const int64_t w = (L + 63) / 64 * 2;
+  jvpfa_mask_tiles_args a{};
+  a.struct_size = sizeof(a);
+  a.n_b = (int)n_b, a.n_h = (int)n_h, a.n_rows = (int)n_rows, a.L = (int)L;
+  a.mask = m.c;
+  Tensor bits, bits_t;
+  try {
+    bits = empty({n_b * n_h * n_rows * w}, at::kInt, q.device());
+    if (bits_t_out) bits_t = empty({n_b * n_h * L * (n_rows > 1 ? w : 1)}, at::kInt, q.device());
+  } catch (const c10::OutOfMemoryError&) {
+    return;
+  }
+  a.bits = bits.data_ptr();
+  if (bits_t_out) a.bits_t = bits_t.data_ptr();
+  const int rc = jvpfa_mask_tiles(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream());
+  if (rc == JVPFA_ERR_TOO_LARGE) return;  // the kernels read the bytes
+  check_status(rc, "jvpfa_mask_tiles");
+  bits_out = bits;
+  if (bits_t_out) *bits_t_out = bits_t;
+}
+
 // Packs a call's boolean mask.  Bits are made anew by every call and not kept with the mask's description: the entries that
 // the kernels read are then those that the mask holds when they run, also where it was written behind torch's version
 // counter (a replayed graph, a foreign kernel).  Which tiles are stepped over, and the lengths of a key-padding mask, are
@@ -241,34 +271,40 @@ bool whole_pieces(const MaskDesc& m, int64_t L) {
 void pack_mask(Call& call, const Tensor& q, bool backward) {
   const MaskDesc& m = *call.mask;
   if (m.c.kind != JVPFA_MASK_BOOL || !takes_16_bit_forms(q)) return;
-  const int64_t L = q.size(2);
   const int64_t n_b = m.c.stride[0] ? m.tensor.size(0) : 1, n_h = m.c.stride[1] ? m.tensor.size(1) : 1;
-  const int64_t n_rows = m.c.stride[2] ? L : 1;
-  if (!backward && whole_pieces(m, L) && 4 * n_b * n_h > q.size(0) * q.size(1)) return;
+  if (!backward && whole_pieces(m, q.size(2)) && 4 * n_b * n_h > q.size(0) * q.size(1)) return;
   c10::cuda::OptionalCUDAGuard guard;
   if (q.get_device() != c10::cuda::current_device()) guard.set_index(q.get_device());
-  const int64_t w = (L + 63) / 64 * 2;
-  jvpfa_mask_tiles_args a{};
-  a.struct_size = sizeof(a);
-  a.n_b = (int)n_b, a.n_h = (int)n_h, a.n_rows = (int)n_rows, a.L = (int)L;
-  a.mask = m.c;
-  Tensor bits, bits_t;
-  try {
-    bits = empty({n_b * n_h * n_rows * w}, at::kInt, q.device());
-    if (backward) bits_t = empty({n_b * n_h * L * (n_rows > 1 ? w : 1)}, at::kInt, q.device());
-  } catch (const c10::OutOfMemoryError&) {
-    return;
-  }
-  a.bits = bits.data_ptr();
-  if (backward) a.bits_t = bits_t.data_ptr();
-  const int rc = jvpfa_mask_tiles(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream());
-  if (rc == JVPFA_ERR_TOO_LARGE) return;  // the kernels read the bytes
-  check_status(rc, "jvpfa_mask_tiles");
-  call.bits = bits, call.bits_t = bits_t;
+  pack(m, q, call.bits, backward ? &call.bits_t : nullptr);
 }
 
 // ---- launches ------------------------------------------------------------------------------------------------------
+// The workspace of a launch, which its kernels on the call's stream are the last to use; undefined for 0 bytes, and where
+// there is no memory for it (the kernels that need none serve the call then).
+Tensor workspace_of(int64_t bytes, const Tensor& q) {
+  if (bytes <= 0) return {};
+  try {
+    return empty({bytes}, at::kByte, q.device());
+  } catch (const c10::OutOfMemoryError&) {
+    return {};
+  }
+}
+
 py::object or_none(const Tensor& t) { return t.defined() ? py::cast(t) : py::object(py::none()); }
+
+// Gives an fp32 launch its workspace, and a boolean mask whose rows cannot be read 16 bytes at a time as bits (returned: they
+// live as long as the launch is being issued).
+template <typename Args>
+Tensor use_workspace(Args& a, const Tensor& workspace, const Call& call, const Tensor& q) {
+  Tensor bits;
+  if (!workspace.defined()) return bits;
+  a.workspace = workspace.data_ptr(), a.workspace_bytes = workspace.numel();
+  if (a.mask.kind == JVPFA_MASK_BOOL && !whole_pieces(*call.mask, q.size(2))) {
+    pack(*call.mask, q, bits, nullptr);
+    a.mask_bits = data(bits);
+  }
+  return bits;
+}
 
 // tq without tk and tv: JVPFA_ZERO_TKV.
 FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& tq, const Tensor& tk, const Tensor& tv,
@@ -315,6 +351,8 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
   a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
   for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
+  const Tensor workspace = workspace_of(call.parts ? jvpfa_fwd_workspace(&a) : 0, q);
+  const Tensor bits = use_workspace(a, workspace, call, q);
   check_status(jvpfa_fwd(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "jvpfa_fwd");
   return r;
 }
@@ -400,6 +438,8 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
   a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
   for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
+  const Tensor workspace = workspace_of(call.parts ? jvpfa_bwd_workspace(&a) : 0, q);
+  const Tensor bits = use_workspace(a, workspace, call, q);
   check_status(jvpfa_bwd(&a, stream), "jvpfa_bwd");
   return g;
 }
@@ -466,10 +506,13 @@ struct AttnBwdNode : public Node {
       at::AutoDispatchBelowADInplaceOrView below;
       for (int i = 0; i < (zero_tkv ? 1 : 3); ++i) t[i] = u[i].defined() ? unwrap(u[i]).contiguous() : at::zeros_like(qp, at::MemoryFormat::Contiguous);
     }
-    FwdResult f = launch_fwd(qp, kp, vp, t[0], t[1], t[2], call);
     const int skip = unused_gradients(task_should_compute_output(0), task_should_compute_output(1) || task_should_compute_output(2));
-    if (skip != (JVPFA_SKIP_DQ | JVPFA_SKIP_DKDV)) {
-      Grads h = launch_bwd(qp, kp, vp, t[0], t[1], t[2], f.o, f.to, f.lse, f.mu, Tensor(), gop, call, skip);
+    const bool again = skip != (JVPFA_SKIP_DQ | JVPFA_SKIP_DKDV);
+    Call c = call;
+    c.parts = !again || (zero_tkv && (skip & JVPFA_SKIP_DKDV));
+    FwdResult f = launch_fwd(qp, kp, vp, t[0], t[1], t[2], c);
+    if (again) {
+      Grads h = launch_bwd(qp, kp, vp, t[0], t[1], t[2], f.o, f.to, f.lse, f.mu, Tensor(), gop, c, skip);
       for (int i = 0; i < 3; ++i) out[i] = h[i];
     }
     if (task_should_compute_output(3)) out[3] = f.to;
@@ -490,7 +533,7 @@ Grads backward_through_o(const Tensor& q, const Tensor& k, const Tensor& v, cons
                          const Call& call, int skip) {
   if (is_wrapped(go)) {  // the cotangent belongs to a functorch transform: a Function, which the transform differentiates or refuses
     py::gil_scoped_acquire gil;
-    py::tuple g = python_module().attr("_backward_under_functorch")(q, k, v, o, lse, go, *call.mask->spec, call.scale, call.tf32);
+    py::tuple g = python_module().attr("_backward_under_functorch")(q, k, v, o, lse, go, *call.mask->spec, call.scale, call.tf32, call.parts);
     return {g[0].cast<Tensor>(), g[1].cast<Tensor>(), g[2].cast<Tensor>()};
   }
   Grads g = launch_bwd(unwrap(q), unwrap(k), unwrap(v), Tensor(), Tensor(), Tensor(), o, Tensor(), lse, Tensor(), go, Tensor(), call, skip);
@@ -608,6 +651,7 @@ std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tens
   Call call{mask, scale ? *scale : 1.0 / std::sqrt((double)q.size(3)), tf32};
   const bool grad_qkv = torch::autograd::compute_requires_grad(q, k, v), grad_mask = torch::autograd::compute_requires_grad(mask_tensor);
   const bool backward = grad_qkv || torch::autograd::compute_requires_grad(tq, tk, tv);
+  call.parts = !dual || !grad_qkv;  // (with respect to the tangents tO is an ordinary attention output)
   FwdResult r;
   {
     // A launch waits while the queue of launches is full: other Python threads run meanwhile.

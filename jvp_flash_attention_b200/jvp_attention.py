@@ -642,11 +642,11 @@ def _backward_impl(ctx, do):
     return _AttnBwd.apply(q, k, v, o.detach(), M, fwAD.unpack_dual(do).primal, ctx.mask_spec, ctx.sm_scale)
 
 
-def _backward_under_functorch(q, k, v, o, M, do, spec, sm_scale, tf32):
+def _backward_under_functorch(q, k, v, o, M, do, spec, sm_scale, tf32, parts):
     """The native layer's backward through O where the cotangent is a tensor of a functorch transform (``torch.func.grad``
     over a vector-Jacobian product, say): ``_AttnBwd`` takes part in it."""
     spec = copy.copy(spec)
-    spec.fp32_mode = "tf32" if tf32 else "3xtf32"
+    spec.fp32_mode, spec.fp32_parts = "tf32" if tf32 else "3xtf32", parts
     return _AttnBwd.apply(q, k, v, o, M, do, spec, sm_scale)
 
 

@@ -1,0 +1,248 @@
+"""fp32 on the tcgen05 kernels (three bf16 parts of every entry): at the edges of their tiles, in every form of mask and layout
+that the register-tiled kernels take, against the float64 oracle and against those kernels; and where the dispatch begins."""
+import ctypes
+import math
+
+import pytest
+import torch
+
+from jvp_flash_attention_b200 import _lib
+from oracle import jvp_attention_oracle as orc
+
+DEV = "cuda:0"
+
+
+def _fwd_args(ts, tangents, mask, out, impl, strides=None):
+    """jvpfa_fwd_args on tensors (or, for the host logic alone, on addresses that nothing follows)."""
+    at = lambda x: None if x is None else x if isinstance(x, int) else x.data_ptr()  # noqa: E731
+    B, H, L, D = ts[0].shape
+    a = _lib.FwdArgs(struct_size=ctypes.sizeof(_lib.FwdArgs), dtype=_lib.FP32, B=B, H=H, L=L, D=D, impl=impl, sm_scale=D**-0.5)
+    a.q, a.k, a.v = (at(x) for x in ts)
+    a.tq, a.tk, a.tv = (at(x) for x in (*tangents, None, None, None)[:3])
+    a.o, a.to, a.lse, a.mu = (at(x) for x in out)
+    a.flags = 8 if len(tangents) == 1 else 0  # JVPFA_ZERO_TKV
+    a.mask = mask
+    if strides:
+        a.in_stride[0], a.in_stride[1], a.in_stride[2] = strides
+    return a
+
+
+def _mask(kind, B, H, L, g):
+    """(kernel-side description, what keeps it alive, the oracle's mask, causal)"""
+    m = _lib.Mask(kind=_lib.MASK_NONE)
+    if kind == "none":
+        return m, None, None, False
+    if kind == "causal":
+        m.kind = _lib.MASK_CAUSAL
+        return m, None, None, True
+    if kind == "keys":
+        lens = torch.randint(0, L + 1, (B,), generator=g)
+        lens[0] = L  # (and one sequence may be empty)
+        t = lens.to(DEV, torch.int32)
+        m.kind, m.kv_len = _lib.MASK_KVLEN, t.data_ptr()
+        return m, t, (torch.arange(L)[None] < lens[:, None])[:, None, None], False
+    if kind.startswith("bool"):
+        x = torch.rand(B, 1 if kind == "bool_shared" else H, L, L, generator=g) > 0.5
+        x[:, :, L // 2] = False  # a row without a key
+        t = x.to(DEV)
+        if kind == "bool_transposed":  # keys are not the contiguous dimension
+            t = t.transpose(2, 3).contiguous().transpose(2, 3)
+        m.kind = _lib.MASK_BOOL
+    else:
+        dt = {"bias": torch.float32, "bias_bf16": torch.bfloat16, "bias_odd": torch.float32, "bias_row": torch.float16}[kind]
+        x = torch.randn(B, H, 1 if kind == "bias_row" else L, L, generator=g).to(dt)
+        t = x.to(DEV)
+        if kind == "bias_odd":  # rows that begin 4 bytes off a 16-byte boundary
+            t = torch.nn.functional.pad(t, (1, 0))[..., 1:]
+        m.kind, m.bias_dtype = _lib.MASK_BIAS, _lib.DTYPE_ENUM[dt]
+    m.ptr = t.data_ptr()
+    for d in range(4):
+        m.stride[d] = t.stride(d) if t.size(d) > 1 else 0
+    if t.size(3) == 1:
+        m.stride[3] = 1
+    return m, t, x, False
+
+
+def _run_fwd(ts, tangents, mask, impl, strides=None):
+    B, H, L, D = ts[0].shape
+    nan = lambda *s: torch.full(s, math.nan, device=DEV)  # noqa: E731
+    out = [nan(B, H, L, D), nan(B, H, L, D) if tangents else None, nan(B, H, L), nan(B, H, L) if tangents else None]
+    a = _fwd_args(ts, tangents, mask, out, impl, strides)
+    lib = _lib.load()
+    if impl == _lib.IMPL_TCGEN05:
+        ws = torch.full((lib.jvpfa_fwd_workspace(ctypes.byref(a)),), 0x7F, dtype=torch.uint8, device=DEV)
+        assert ws.numel() > 0
+        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    _lib.check(lib.jvpfa_fwd(ctypes.byref(a), torch.cuda.current_stream().cuda_stream), "jvpfa_fwd")
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    return out
+
+
+def _rel(x, r):
+    return ((x.cpu().double() - r).norm() / r.norm().clamp(min=1e-30)).item()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("L,kind,n_tangents", [
+    (1, "none", 3), (34, "causal", 3), (63, "bias", 0), (65, "bool", 1), (128, "none", 0), (129, "causal", 1), (130, "bias_odd", 3),
+    (192, "bool_transposed", 3), (200, "keys", 3), (257, "bias_bf16", 1), (300, "bool_shared", 0), (384, "keys", 1), (500, "bias", 3),
+    (333, "bias_row", 3),
+])
+def test_forward_on_three_bf16_parts(D, L, kind, n_tangents):
+    """A product is exact to 2^-26 of its operands and an accumulator takes 24 instructions a key tile, truncated at 2^-24 of
+    it or of its small parts: 1e-5 of the largest entry, the fp32 bound of the parity tests, and no further from 64 bits than
+    the register-tiled kernels (1.2 times, for the luck of a few rows)."""
+    B, H = 2, 3
+    g = torch.Generator().manual_seed(L + D)
+    ts = [torch.randn(B, H, L, D, generator=g) for _ in range(3)]
+    tg = [torch.randn(B, H, L, D, generator=g) for _ in range(n_tangents)]
+    mask, alive, attn_mask, causal = _mask(kind, B, H, L, g)
+    zero = torch.zeros(B, H, L, D)
+    if attn_mask is not None and attn_mask.dtype == torch.bool:
+        attn_mask = attn_mask.expand(B, H, L, L)
+    elif attn_mask is not None:
+        attn_mask = attn_mask.double()
+    ref = orc.sdpa_jvp(*ts, *(*tg, zero, zero, zero)[:3], attn_mask, causal)
+    # the (B, H, L, D) view of (B, L, H, D) tensors, read in place
+    dev = [x.transpose(1, 2).contiguous().to(DEV).transpose(1, 2) for x in (*ts, *tg)]
+    runs = {}
+    for impl in (_lib.IMPL_GENERIC, _lib.IMPL_TCGEN05):
+        runs[impl] = _run_fwd(dev[:3], dev[3:], mask, impl, (L * H * D, D, H * D))
+    old, new = runs[_lib.IMPL_GENERIC], runs[_lib.IMPL_TCGEN05]
+    for n, r in enumerate(ref if n_tangents else ref[:1]):
+        assert orc.max_abs_err(new[n], r) <= 1e-5 * max(r.abs().max().item(), 1e-30), n
+        assert _rel(new[n], r) <= max(1.2 * _rel(old[n], r), 2**-22), n
+    for n in (2, 3):  # lse (+inf where no key attends) and mu
+        if new[n] is not None:
+            same = torch.isfinite(old[n])
+            assert torch.equal(same, torch.isfinite(new[n])) and torch.equal(old[n][~same], new[n][~same])
+            if same.any():
+                assert (new[n] - old[n])[same].abs().max().item() <= 1e-5 * max(1.0, old[n][same].abs().max().item())
+    dense = _run_fwd([x.contiguous() for x in dev[:3]], [x.contiguous() for x in dev[3:]], mask, _lib.IMPL_TCGEN05)
+    for x, y in zip(dense, new):
+        assert x is None or torch.equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("through", ["o", "t"])
+@pytest.mark.parametrize("L,kind", [
+    (1, "none"), (34, "causal"), (63, "bias"), (65, "bool"), (128, "none"), (129, "causal"), (130, "bias_odd"),
+    (192, "bool_transposed"), (200, "keys"), (257, "bias_bf16"), (300, "bool_shared"), (500, "bias"), (333, "bias_row"),
+])
+def test_backward_on_three_bf16_parts(D, through, L, kind):
+    """Through O, and dQ through tO with no tangents of K and V, from the lse and mu of the forward on the same kernels: 1e-5 of
+    the largest entry, and no further from 64 bits than the register-tiled pair (1.2 times).  dQ alone is dQ of the full call.
+    A single key shows how S was formed (its P is 1): by the forward and, with the operands exchanged, by the launch that owns
+    keys.  Either is truncated by up to 16 instructions at 2^-24 of it, half of that on average, and S is about 1: 2^-21."""
+    B, H = 2, 3
+    g = torch.Generator().manual_seed(L + D)
+    q, k, v, tq, cot = (torch.randn(B, H, L, D, generator=g) for _ in range(5))
+    mask, alive, attn_mask, causal = _mask(kind, B, H, L, g)
+    zero = torch.zeros(B, H, L, D)
+    if attn_mask is not None:
+        attn_mask = attn_mask.expand(B, H, L, L) if attn_mask.dtype == torch.bool else attn_mask.double()
+    ref = orc.grads_through_both(q, k, v, tq, zero, zero, cot if through == "o" else None, cot if through == "t" else None, attn_mask, causal)[2:]
+    strides = (L * H * D, D, H * D)
+    dq_, dk_, dv_, dtq_ = (x.transpose(1, 2).contiguous().to(DEV).transpose(1, 2) for x in (q, k, v, tq))
+    cot = cot.to(DEV)
+    lib, got = _lib.load(), {}
+    full = 0 if through == "o" else 2  # JVPFA_SKIP_DKDV
+    for impl, skip in ((_lib.IMPL_GENERIC, full), (_lib.IMPL_TCGEN05, 2), (_lib.IMPL_TCGEN05, full)):
+        o, to, lse, mu = _run_fwd([dq_, dk_, dv_], [dtq_] if through == "t" else [], mask, impl, strides)
+        stats = torch.empty(3, B, H, L, device=DEV)
+        _lib.bwd_preprocess(o, to, *((cot, None) if through == "o" else (None, cot)), mu, *stats)
+        grads = [torch.full((B, H, L, D), math.nan, device=DEV) for _ in range(3)]
+        a = _lib.BwdArgs(struct_size=ctypes.sizeof(_lib.BwdArgs), dtype=_lib.FP32, B=B, H=H, L=L, D=D, impl=impl, sm_scale=D**-0.5)
+        a.q, a.k, a.v = dq_.data_ptr(), dk_.data_ptr(), dv_.data_ptr()
+        a.lse, a.delta, a.eps, a.cterm = lse.data_ptr(), *(x.data_ptr() for x in stats)
+        a.dq, a.flags, a.mask = grads[0].data_ptr(), skip, mask
+        if not skip:
+            a.dk, a.dv = (x.data_ptr() for x in grads[1:])
+        if through == "t":
+            a.tq, a.gto, a.mu, a.flags = dtq_.data_ptr(), cot.data_ptr(), mu.data_ptr(), 2 | 8
+        else:
+            a.go = cot.data_ptr()
+        a.in_stride[0], a.in_stride[1], a.in_stride[2] = strides
+        if impl == _lib.IMPL_TCGEN05:
+            ws = torch.full((lib.jvpfa_bwd_workspace(ctypes.byref(a)),), 0x7F, dtype=torch.uint8, device=DEV)
+            a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+        _lib.check(lib.jvpfa_bwd(ctypes.byref(a), torch.cuda.current_stream().cuda_stream), "jvpfa_bwd")
+        torch.cuda.synchronize()
+        assert _lib.device_status() == 0
+        got.setdefault(impl, []).append(grads)
+    (old,), (alone, new) = got[_lib.IMPL_GENERIC], got[_lib.IMPL_TCGEN05]
+    assert torch.equal(alone[0], new[0])
+    for n, r in enumerate(ref if through == "o" else ref[:1]):
+        if L == 1 and n < 2:  # (one key: no gradient of q and k)
+            assert new[n].abs().max().item() <= 1e-5
+            continue
+        assert orc.max_abs_err(new[n], r) <= 1e-5 * r.abs().max().item(), n
+        assert _rel(new[n], r) <= max(1.2 * _rel(old[n], r), 2**-21 if L == 1 else 2**-22), n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,L,kind", [(64, 514, "bool"), (128, 500, "bias"), (128, 334, "bool"), (32, 1410, "causal"), (64, 1024, "none")])
+def test_what_is_asked_of_a_call_decides_the_kernels(D, L, kind):
+    """A Hessian-vector product along q runs on the tcgen05 kernels; one that k and v take part in differentiates through tO with
+    tangents of all three, which the register-tiled kernels do.  All against the float64 oracle."""
+    from jvp_flash_attention_b200 import jvp_attention as ja
+
+    B, H = 2, 6
+    g = torch.Generator().manual_seed(L)
+    q, k, v, w, u = (torch.randn(B, H, L, D, generator=g) for _ in range(5))
+    mask = None
+    if kind == "bool":
+        mask = (torch.rand(B, 1, L, L, generator=g) > 0.7) | torch.eye(L, dtype=torch.bool)
+    elif kind == "bias":
+        mask = torch.randn(B, H, L, L, generator=g)
+    causal = kind == "causal"
+    m = None if mask is None else mask.to(DEV)
+    ref = orc.hvp_q(q, k, v, w, u, mask, causal)
+    errors = {}
+    for leaves in ("q", "qkv"):
+        a = [x.to(DEV).requires_grad_(n in leaves) for n, x in zip("qkv", (q, k, v))]
+        o = ja.attention(*a, attn_mask=m, causal=causal)
+        (dq,) = torch.autograd.grad(o, a[0], w.to(DEV), create_graph=True)
+        hq = torch.autograd.grad(dq, [x for x in a if x.requires_grad], u.to(DEV))[0]
+        for name, x, r in zip(("O", "dq", "hq"), (o, dq, hq), ref):
+            assert orc.max_abs_err(x, r) <= 1e-5 * r.abs().max().item(), (leaves, name)
+            errors[leaves, name] = _rel(x.detach(), r)
+    for name in ("O", "dq", "hq"):
+        assert errors["q", name] <= max(1.2 * errors["qkv", name], 2**-22), (name, errors)
+    assert _lib.device_status() == 0
+
+
+def _workspace(B, H, L, D, tangents=0, impl=_lib.IMPL_AUTO, dtype=_lib.FP32, **fields):
+    class At(int):
+        shape = (B, H, L, D)
+    x = At(1 << 20)
+    a = _fwd_args([x] * 3, [x] * tangents, _lib.Mask(kind=_lib.MASK_NONE), [x, x if tangents else None, x, x if tangents else None], impl)
+    a.dtype = dtype
+    for k, v in fields.items():
+        setattr(a, k, v)
+    lib = _lib.load()
+    return lib.jvpfa_fwd_workspace(ctypes.byref(a)), lib.jvpfa_fwd_uses_tcgen05(ctypes.byref(a))
+
+
+def test_where_fp32_takes_the_tcgen05_kernels():
+    """Host logic.  From 384 16-row tiles on at D = 64 (320 at 128, 1024 at 32), and not for one 64-row tile; 18, 24 or 36 bytes
+    an element (three, four or six tensors); with a workspace that is large enough and aligned."""
+    assert _workspace(2, 6, 512, 64) == (18 * 2 * 6 * 512 * 64, 0)  # (no workspace given: the register-tiled kernels)
+    assert _workspace(2, 6, 512, 64, 1)[0] == 24 * 2 * 6 * 512 * 64
+    assert _workspace(2, 6, 512, 64, 3)[0] == 36 * 2 * 6 * 512 * 64
+    assert _workspace(2, 6, 496, 64)[0] == 0 and _workspace(16, 16, 64, 64)[0] == 0
+    assert _workspace(2, 5, 512, 128)[0] > 0 and _workspace(2, 5, 480, 128)[0] == 0
+    assert _workspace(4, 16, 256, 32)[0] > 0 and _workspace(4, 16, 128, 32)[0] == 0 and _workspace(2, 16, 448, 32)[0] == 0
+    assert _workspace(1, 1, 32, 64, impl=_lib.IMPL_TCGEN05)[0] > 0
+    for dtype in (_lib.BF16, _lib.FP16, _lib.FP32_TF32):
+        assert _workspace(2, 6, 512, 64, dtype=dtype)[0] == 0
+    assert _workspace(2, 6, 512, 64, impl=_lib.IMPL_GENERIC)[0] == 0
+    need = 18 * 2 * 6 * 512 * 64
+    assert _workspace(2, 6, 512, 64, workspace=1 << 20, workspace_bytes=need)[1] == 1
+    assert _workspace(2, 6, 512, 64, workspace=1 << 20, workspace_bytes=need - 1)[1] == 0
+    assert _workspace(2, 6, 512, 64, workspace=(1 << 20) + 8, workspace_bytes=need)[1] == 0
+    assert _workspace(2, 6, 512, 64, workspace=1 << 20, workspace_bytes=need, struct_size=_lib.FwdArgs.workspace.offset)[1] == 0
+    assert _workspace(2, 6, 512, 64, struct_size=_lib.FwdArgs.workspace.offset + 8) == (0, 0)
