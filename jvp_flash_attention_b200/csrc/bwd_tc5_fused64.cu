@@ -154,7 +154,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* rb_ok = reinterpret_cast<volatile int*>(tmem_slot + 2);  // the read-back group's poller tells the rest
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int L = a.L;
   const int BH = a.B * a.H;
   const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL;
@@ -247,14 +247,11 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
   // Registers: the elementwise threads hold four 32-column accumulator slices; everybody else needs few.
   // (setmaxnreg.inc draws on what setmaxnreg.dec of the same CTA has released and blocks until it is there: 256
   // threads x 56 registers up equals 256 threads x 56 registers down from the 128 the kernel is launched with.)
-  if (warp < 4 || warp >= 12) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-  } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
-  }
-
   // Phase counters kept alike by all roles: g counts the sub-tiles of this CTA (ring stage g % STAGES, dQ buffer
   // g & 1; s_full, s_free complete once per sub-tile, p_full and out_free of buffer g & 1 every other one), kact the items that have sub-tiles.
+  // (setmaxnreg stands in the branches of the roles: ptxas holds code behind a join of the two to the smaller number.)
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer + per-query statistics
     if (lane == 0) {
@@ -334,8 +331,9 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       }
       ++kact;
     }
-  } else if (warp <= 3) {
-    if (lane == 0) {
+  } else {
+    // The issuing warps stay converged and let one lane issue (mbar_wait_warp).
+    {
       constexpr uint32_t idesc_sc = make_idesc(Fmt<T>::kIdesc, OWN, BL, 0, 0);       // 128 x 64 scores
       constexpr uint32_t idesc_sc2 = make_idesc(Fmt<T>::kIdesc, OWN, 2 * BL, 0, 0);  // 128 x 128: [S | tS]
       constexpr uint32_t idesc_kv = make_idesc(Fmt<T>::kIdesc, OWN, D, 0, 1);        // dK, dV: 128 x 64, B MN-major
@@ -369,17 +367,18 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
         for (int k = 0; ok && k < k_max; ++k) {
           if (!get_item(k, it) || it.n_sub == 0) continue;
           const int oset = kact % C::OWN_BUFS;
-          if (!mbar_wait(own_full + oset, (kact / C::OWN_BUFS) & 1, ab, kAbortBwdOwn)) break;
+          if (!mbar_wait_warp(own_full + oset, (kact / C::OWN_BUFS) & 1, ab, kAbortBwdOwn)) break;
           own_k = own_k0 + oset * OWNSET16;
           for (int s = 0; s < it.n_sub; ++s, ++g) {
             const int st = g % STAGES;
-            if (!mbar_wait(loop_full + st, (g / STAGES) & 1, ab, kAbortBwdLoopFull) ||
-                (g > 0 && !mbar_wait(s_free, (g - 1) & 1, ab, kAbortBwdSFull))) {
+            if (!mbar_wait_warp(loop_full + st, (g / STAGES) & 1, ab, kAbortBwdLoopFull) ||
+                (g > 0 && !mbar_wait_warp(s_free, (g - 1) & 1, ab, kAbortBwdSFull))) {
               ok = false;
               break;
             }
             tc_fence_after();
             const uint32_t lp = ring_k + st * STAGE16;
+            if (elect_one()) {
             if constexpr (HAS_GT) {
               score(C::COL_S, C::SLOT_K, lp + C::SLOT_Q * LOOP16, idesc_sc2, true);    // [S | tS] = K [Q ; tQ]^T
               score(C::COL_TS, C::SLOT_TK, lp + C::SLOT_Q * LOOP16, idesc_sc, false);  // tS += tK Q^T
@@ -392,9 +391,10 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             }
             tc_commit(s_full);
             tc_commit(loop_empty + st);
+            if (s == it.n_sub - 1) tc_commit(own_free + oset);
+            }
           }
           if (!ok) break;
-          tc_commit(own_free + oset);
           ++kact;
         }
       } else if (warp == 2) {
@@ -417,8 +417,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           if (!get_item(k, it) || it.n_sub == 0) continue;
           for (int s = 0; s < it.n_sub; ++s, ++g) {
             const int st = g % STAGES;
-            if (!mbar_wait(p_full + (g & 1), (g >> 1) & 1, ab, kAbortBwdPFull) ||
-                (s == 0 && kact > 0 && !mbar_wait(acc_free, (kact - 1) & 1, ab, kAbortBwdDone))) {
+            if (!mbar_wait_warp(p_full + (g & 1), (g >> 1) & 1, ab, kAbortBwdPFull) ||
+                (s == 0 && kact > 0 && !mbar_wait_warp(acc_free, (kact - 1) & 1, ab, kAbortBwdDone))) {
               ok = false;
               break;
             }
@@ -427,6 +427,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             ob16 = ob * (C::OBUF_BYTES >> 4);
             const uint32_t lp = ring_mn + st * STAGE16;
             const uint32_t acc = s > 0;
+            if (elect_one()) {
             outer(C::COL_DK, C::OUT_GS, lp + C::SLOT_Q * LOOP16, acc);  // dK += gS^T Q
             if constexpr (HAS_GT) {
               outer(C::COL_DK, C::OUT_GT, lp + C::SLOT_TQ * LOOP16, 1);  // dK += gtS^T tQ
@@ -438,9 +439,10 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             tc_commit(loop_empty + st);
             tc_commit(out_free + ob);
             tc_commit(av_free);
+            if (s == it.n_sub - 1) tc_commit(done);
+            }
           }
           if (!ok) break;
-          tc_commit(done);
           ++kact;
         }
       } else {
@@ -461,8 +463,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           if (!get_item(k, it) || it.n_sub == 0) continue;
           own_mn = own_mn0 + (kact % C::OWN_BUFS) * OWNSET16;
           for (int s = 0; s < it.n_sub; ++s, ++g) {
-            if (!mbar_wait(p_full + (g & 1), (g >> 1) & 1, ab, kAbortBwdPFull) ||
-                (g >= 1 && !mbar_wait(dq_free, (g - 1) & 1, ab, kAbortBwdDone))) {
+            if (!mbar_wait_warp(p_full + (g & 1), (g >> 1) & 1, ab, kAbortBwdPFull) ||
+                (g >= 1 && !mbar_wait_warp(dq_free, (g - 1) & 1, ab, kAbortBwdDone))) {
               ok = false;
               break;
             }
@@ -470,18 +472,22 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             const int ob = g % C::N_OBUF;
             ob16 = ob * (C::OBUF_BYTES >> 4);
             const uint32_t col = C::COL_DQ;
+            if (elect_one()) {
             inner(col, C::OUT_GS, C::SLOT_K, true);                       // dQ = gS K
             if constexpr (HAS_GT) inner(col, C::OUT_GT, C::SLOT_TK, false);  // dQ += gtS tK
             tc_commit(dq_full);
             tc_commit(out_free + ob);
+            if (s == it.n_sub - 1) tc_commit(own_free + kact % C::OWN_BUFS);
+            }
           }
           if (!ok) break;
-          tc_commit(own_free + kact % C::OWN_BUFS);
           ++kact;
         }
       }
     }
+  }
   } else if (warp < 12) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
     // ------------------------------------------------------------------ elementwise warpgroups
     const int wg = (warp - 4) >> 2;  // 0 / 1: query columns [32 wg, 32 wg + 32) of every sub-tile
     const int quarter = warp & 3;
@@ -674,6 +680,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       ++kact;
     }
   } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     // ------------------------------------------------------------------ dQ read-back
     const int quarter = warp & 3;
     const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + C::COL_DQ;
