@@ -163,7 +163,7 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stat_full + STAGES);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int L = a.L;
   const int BH = a.B * a.H;
   const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL;
@@ -442,9 +442,8 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
     }
   } else if (warp <= 3 || warp >= 12) {
     // ------------------------------------------------------------------ MMA issuers
-    // Each of these warps works with one thread.  Such a thread pays ~75 cycles per MMA and a few
-    // hundred cycles of waits and bookkeeping per sub-tile, and the time a sub-tile's scores take to
-    // issue is part of the latency that the three buffers in flight have to cover.  So the scores of
+    // Converged warps with one elected lane each (mbar_wait_warp).  The time a sub-tile's scores take to
+    // issue is part of the latency that the three buffers in flight have to cover, so the scores of
     // the even sub-tiles belong to warps 1 and 13, those of the odd sub-tiles to warps 2 and 14:
     //   own keys   : warps 1, 2: [S|TS] = K [Q;tQ]^T, TS += tK Q^T ; warps 13, 14: E = V G^T, FP = tV G^T (+ V gO^T)
     //   own queries: warps 1, 2: [S|TS] = Q [K;tK]^T, TS += tQ K^T ; warps 13, 14: [E|FP] = G [V;tV]^T (+ FP += gO V^T)
@@ -476,7 +475,7 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
     const uint32_t bar_s_full = smem_u32(s_full), bar_p_full = smem_u32(p_full);
     const uint32_t ring_lo = kDescLo | (smem_u32(sLoop) >> 4);
 
-    if (lane == 0 && (warp == 1 || warp == 2 || warp >= 13)) {
+    if ((warp == 1 || warp == 2 || warp >= 13)) {
       // ---------------- scores of the sub-tiles g = r, r + 2, r + 4, ...
       const bool part_b = warp >= 13;  // which accumulators
       const uint32_t r = part_b ? warp - 13 : warp - 1;
@@ -510,7 +509,7 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
         const int g_end = gbase + it.n_sub;
         // This item's own operands: its staging half.  Waited for even when none of the item's sub-tiles
         // is this thread's: a parity wait is only safe for a thread that sees every phase of the barrier.
-        ok = mbar_wait(own_staged + (kact & 1), (kact >> 1) & 1, ab, kAbortBwdOwn);
+        ok = mbar_wait_warp(own_staged + (kact & 1), (kact >> 1) & 1, ab, kAbortBwdOwn);
         if (!ok) break;
         tc_fence_after();
         own_lo = kDescLo | (smem_u32(sOwn + (kact & 1) * C::STAGING_HALF) >> 4);
@@ -519,19 +518,20 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
           // The buffer may be overwritten once every second-stage chain of sub-tile g - NBUF has read
           // it: that is what loop_empty[its stage] records (one arrival per second-stage issuer).
           if (g >= NBUF) {
-            if (!mbar_wait_u32(bar_loop_empty + cf.st_bar, cf.st_par, ab, kAbortAux)) {
+            if (!mbar_wait_warp_u32(bar_loop_empty + cf.st_bar, cf.st_par, ab, kAbortAux)) {
               ok = false;
               break;
             }
             cf.advance(2);
           }
-          if (!mbar_wait_u32(bar_loop_full + cs.st_bar, cs.st_par, ab, kAbortBwdLoopFull)) {
+          if (!mbar_wait_warp_u32(bar_loop_full + cs.st_bar, cs.st_par, ab, kAbortBwdLoopFull)) {
             ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t lp = ring_lo + cs.st_tile;  // tile slot 0 of the stage
           const uint32_t acc = tmem + cs.buf_col;
+          if (elect_one()) {
           if (!part_b) {
             if constexpr (OWN_KEYS) {
               if constexpr (HAS_GT) {
@@ -567,16 +567,17 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
             }
           }
           tc_commit_u32(bar_s_full + cs.sf_bar);
+          }
           cs.advance(2);
         }
         if (!ok) break;
         // "This thread is through with the item": the staging half is not refilled before, so its
         // barrier cannot run more than one phase ahead of this thread.
-        mbar_arrive(own_free + (kact & 1));
+        if (elect_one()) mbar_arrive(own_free + (kact & 1));
         gbase = g_end;
         ++kact;
       }
-    } else if (lane == 0 && (warp == 3 || (OWN_KEYS && warp == 12))) {
+    } else if ((warp == 3 || (OWN_KEYS && warp == 12))) {
       // ---------------- second stage: one output accumulator through all sub-tiles
       const bool second = warp == 12;  // dV
       Cursor co(0);
@@ -593,14 +594,14 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
         if (it.n_sub == 0) continue;
 #pragma unroll 1
         for (int s = 0; s < it.n_sub; ++s, ++g) {
-          if (!mbar_wait_u32(bar_p_full + co.buf_bar, co.buf_par, ab, kAbortBwdPFull)) {
+          if (!mbar_wait_warp_u32(bar_p_full + co.buf_bar, co.buf_par, ab, kAbortBwdPFull)) {
             ok = false;
             break;
           }
           // The first sub-tile overwrites the output accumulators: the epilogue of the item that used
           // them last must have read them.
           if (s == 0 && kact >= C::N_OUT_BUF &&
-              !mbar_wait(out_free + kact % C::N_OUT_BUF, (kact / C::N_OUT_BUF - 1) & 1, ab, kAbortBwdDone)) {
+              !mbar_wait_warp(out_free + kact % C::N_OUT_BUF, (kact / C::N_OUT_BUF - 1) & 1, ab, kAbortBwdDone)) {
             ok = false;
             break;
           }
@@ -608,6 +609,7 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
           const uint32_t lp = ring_lo + co.st_tile;
           const uint32_t opnd = tmem + co.buf_col;
           const uint32_t acc = s > 0;
+          if (elect_one()) {
           if constexpr (OWN_KEYS) {
             if (!second) {
               outer(C::COL_OUT0, opnd + C::OFF_FP, lp + C::SLOT_Q * LOOP16, acc);                        // dK += gS^T Q
@@ -624,9 +626,10 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
             if constexpr (HAS_GT) outer(oc, opnd + C::OFF_E, lp + C::SLOT_TK * LOOP16, 1);              // dQ += gtS tK
           }
           tc_commit_u32(bar_loop_empty + co.st_bar);
+          }
           co.advance(1);
         }
-        if (ok) tc_commit(done + kact % C::N_OUT_BUF);
+        if (ok && elect_one()) tc_commit(done + kact % C::N_OUT_BUF);
         ++kact;
       }
     }

@@ -149,7 +149,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* n_live = reinterpret_cast<int*>(tmem_slot + 2);  // MK == 3: live loop tiles of this CTA
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int L = a.L;
   const int bh = blockIdx.y;
   const int tma_b = bh / a.H, tma_h = bh - tma_b * a.H;  // coordinates in the (D, L, H, B) tensor maps
@@ -340,13 +340,12 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
     }
   } else if (warp == 1 || warp == C::WARP_ISSUER2) {
     // ------------------------------------------------------------------ MMA issuers
-    // One thread cannot issue an MMA more often than about every 58 cycles, whatever its shape; two threads together
-    // can.  The first issuer forms [S | TS] and, after the elementwise threads, the outputs; the second forms [E | FP].
+    // Two converged warps, one elected lane each (mbar_wait_warp).  The first issuer forms [S | TS] and, after the elementwise threads, the outputs; the second forms [E | FP].
     // Everything that reads what the elementwise threads write (they write over S and TS only) is issued by the first
     // thread, after that thread's own scores into the same buffer two tiles earlier and before its next ones: the
     // tensor pipe keeps one thread's instructions in order, so no barrier between the two issuers is needed.  The
     // second thread waits for p_full(t) only to know that E and FP of tile t have been read before it overwrites them.
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0) {
       const bool second = warp != 1;
       constexpr uint32_t idesc_n1 = make_idesc(Fmt<T>::kIdesc, OWN, BL, 0, 0);      // one 128 x BL accumulator
       constexpr uint32_t idesc_n2 = make_idesc(Fmt<T>::kIdesc, OWN, 2 * BL, 0, 0);  // two adjacent accumulators
@@ -366,11 +365,12 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
       // first issuer: [S | TS] = own0 [loop0 | loop1]^T, TS += own1 loop0^T
       auto issue_s = [&](int t) -> bool {
         const int st = t % STAGES;
-        if (!mbar_wait(loop_full + st, (t / STAGES) & 1, ab, kAbortBwdLoopFull)) return false;
+        if (!mbar_wait_warp(loop_full + st, (t / STAGES) & 1, ab, kAbortBwdLoopFull)) return false;
         tc_fence_after();
         const uint32_t lx = kDescLo | (smem_u32(sX + st * C::X_STAGE) >> 4);
         const uint32_t sc = tmem + (t & 1) * C::SC_COLS;
         constexpr uint32_t id = HAS_GT ? idesc_n2 : idesc_n1;
+        if (elect_one()) {
         umma_ss_lo<false>(sc + C::COL_S, a_lo0 + a_off(0, 0), lx + b_off(C::X_HALF, 0, 0), id);
 #pragma unroll
         for (int ks = 1; ks < 8; ++ks)
@@ -381,6 +381,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
             umma_ss_lo<true>(sc + C::COL_TS, a_lo0 + a_off(1, ks), lx + b_off(C::X_HALF, 0, ks), idesc_n1);
         }
         tc_commit(s_full + (t & 1));
+        }
         return true;
       };
       // second issuer: [E | FP] = own2 [loop2 | loop3]^T, FP += own3 loop2^T; loop tensors 2 and 3 are slots 2, 3 of the
@@ -389,15 +390,16 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
         uint32_t l2;
         if constexpr (OWN_KEYS) {
           const int st = t % STAGES;
-          if (!mbar_wait(loop_full + st, (t / STAGES) & 1, ab, kAbortBwdLoopFull)) return false;
+          if (!mbar_wait_warp(loop_full + st, (t / STAGES) & 1, ab, kAbortBwdLoopFull)) return false;
           l2 = (kDescLo | (smem_u32(sX + st * C::X_STAGE) >> 4)) + ((2 * C::LQ_BYTES) >> 4);
         } else {
-          if (!mbar_wait(y_full, t & 1, ab, kAbortBwdLoopFull)) return false;
+          if (!mbar_wait_warp(y_full, t & 1, ab, kAbortBwdLoopFull)) return false;
           l2 = kDescLo | (smem_u32(sY) >> 4);
         }
         tc_fence_after();
         constexpr uint32_t h2 = OWN_KEYS ? C::X_HALF : C::Y_HALF;
         const uint32_t sc = tmem + (t & 1) * C::SC_COLS;
+        if (elect_one()) {
         if constexpr (HAS_GT) {
           constexpr bool wide = !OWN_KEYS || HAS_GO;  // [E | FP] in one instruction
           umma_ss_lo<false>(sc + C::COL_E, a_lo0 + a_off(2, 0), l2 + b_off(h2, 0, 0), wide ? idesc_n2 : idesc_n1);
@@ -420,25 +422,27 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
         }
         if constexpr (OWN_KEYS) tc_commit(loop_empty + (t % STAGES)); else tc_commit(y_empty);
         tc_commit(s_full + (t & 1));
+        }
         return true;
       };
-      bool ok = mbar_wait(own_full, 0, ab, kAbortBwdOwn);
+      bool ok = mbar_wait_warp(own_full, 0, ab, kAbortBwdOwn);
       if (second) {
         if (ok) ok = issue_e(0);
         for (int t = 0; ok && t + 1 < n_tiles; ++t) {
           if (!issue_e(t + 1)) break;
-          if (!mbar_wait(p_full + (t & 1), (t >> 1) & 1, ab, kAbortBwdPFull)) break;
+          if (!mbar_wait_warp(p_full + (t & 1), (t >> 1) & 1, ab, kAbortBwdPFull)) break;
         }
       } else {
         if (ok) ok = issue_s(0);
         for (int t = 0; ok && t < n_tiles; ++t) {
           if (t + 1 < n_tiles && !issue_s(t + 1)) break;
-          if (!mbar_wait(p_full + (t & 1), (t >> 1) & 1, ab, kAbortBwdPFull)) break;
+          if (!mbar_wait_warp(p_full + (t & 1), (t >> 1) & 1, ab, kAbortBwdPFull)) break;
           tc_fence_after();
           const int st = t % STAGES;
           const uint32_t mx = kMnLo | (smem_u32(sX + st * C::X_STAGE) >> 4);
           const uint32_t sc = tmem + (t & 1) * C::SC_COLS;
           const uint32_t acc = t > 0;
+          if (elect_one()) {
           // Contraction step kk = NP * term + piece: rows 16 * piece .. of X tile (slot + term), operand piece at
           // column 16 * piece + 8 * term of the accumulator it was written over.
           // dK or dQ += gS x0 + gtS x1
@@ -464,8 +468,9 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
             }
           }
           tc_commit(loop_empty + st);
+          }
         }
-        tc_commit(done);
+        if (elect_one()) tc_commit(done);
       }
     }
   } else {

@@ -149,7 +149,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wg_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int L = a.L;
   const int BH = a.B * a.H;
   const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL;
@@ -258,12 +258,10 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
   // Phase counters, kept alike by every role: g counts the key tiles loaded by this CTA (ring stage g % STAGES),
   // kact the items that load anything (q_full / q_empty), t[X] the key tiles query tile X has used (s_full,
   // s_free, p_full, pv_done of X complete once per such tile), kx[X] the items in which X used a tile (o_free).
-  // The four warps of warpgroup 0 need few registers; the softmax threads hold two score tiles each.
+  // The four warps of warpgroup 0 need few registers; the softmax threads hold two score tiles each.  (In the branches of the
+  // roles: ptxas holds code behind a join of the two to the smaller number.)
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
-  } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
-  }
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
@@ -305,10 +303,10 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
     }
   } else if (warp <= 2) {
     // ------------------------------------------------------------------ issuer of query tile X
-    // One thread.  Whatever it executes between two MMAs is pure latency for the tensor pipe, so stage and
-    // barrier cursors, parities and the low words of the operand descriptors live in registers and advance by
+    // A converged warp, one elected lane (mbar_wait_warp).  Whatever it executes between two MMAs is pure latency for the tensor
+    // pipe, so stage and barrier cursors, parities and the low words of the operand descriptors live in registers and advance by
     // additions (descriptor = constant high word kDescHi + (byte address >> 4) in the low word).
-    if (lane == 0) {
+    {
       const int X = warp - 1;
       constexpr uint32_t idesc_s = make_idesc(Fmt<T>::kIdesc, BM, BN, 0, 0);       // 128 x 64
       constexpr uint32_t idesc_s2 = make_idesc(Fmt<T>::kIdesc, BM, 2 * BN, 0, 0);  // 128 x 128: [S | tS]
@@ -334,11 +332,12 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
 
       // [O | tO'] (+)= P [V | tV] ; tO' += W V for the tile in ring stage pst, whose phases have parity ppar
       auto issue_pv = [&](uint32_t pst, uint32_t ppar, bool first) -> bool {
-        if (!mbar_wait_u32(bar_p_full, ppar, ab, kAbortPFull)) return false;
+        if (!mbar_wait_warp_u32(bar_p_full, ppar, ab, kAbortPFull)) return false;
         // The item's first tile overwrites O / tO': the previous item's epilogue must have read them.
-        if (first && kx > 0 && !mbar_wait_u32(bar_o_free, (kx - 1) & 1, ab, kAbortOFull)) return false;
+        if (first && kx > 0 && !mbar_wait_warp_u32(bar_o_free, (kx - 1) & 1, ab, kAbortOFull)) return false;
         tc_fence_after();
         const uint32_t v_lo = v_lo0 + pst * STAGE16;
+        if (elect_one()) {
         if constexpr (DUAL) {
           umma_ss_lo_dyn(tq + C::COL_O, p_lo, v_lo, idesc_o2, first ? 0u : 1u);
 #pragma unroll
@@ -352,13 +351,14 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         }
         tc_commit_u32(bar_kv_empty + 8 * pst);
         tc_commit_u32(bar_pv_done);
+        }
         return true;
       };
 
       for (int k = 0; ok && k < k_max; ++k) {
         if (!get_item(k, it) || it.n_load == 0) continue;
         // waited for by both issuers in every item, used or not: a parity wait must see every phase
-        if (!mbar_wait(q_full, kact & 1, ab, kAbortQFull)) break;
+        if (!mbar_wait_warp(q_full, kact & 1, ab, kAbortQFull)) break;
         const int my_last = it.last(X);
         bool pend = false, pend_first = false, first = true;
         uint32_t pend_st = 0, pend_par = 0;
@@ -366,18 +366,19 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         for (int j = 0; j < it.n_load; ++j) {
           const int m = use(j);
           if (m == 0) continue;
-          if (!mbar_wait_u32(bar_kv_full + 8 * st, st_par, ab, kAbortKvFull)) {
+          if (!mbar_wait_warp_u32(bar_kv_full + 8 * st, st_par, ab, kAbortKvFull)) {
             ok = false;
             break;
           }
           if (m & (1 << X)) {
             // S / tS of the previous tile (of this item or the one before) must be in the softmax threads' registers
-            if (any_t && !mbar_wait_u32(bar_s_free, tpar ^ 1, ab, kAbortSFull)) {
+            if (any_t && !mbar_wait_warp_u32(bar_s_free, tpar ^ 1, ab, kAbortSFull)) {
               ok = false;
               break;
             }
             tc_fence_after();
             const uint32_t k_lo = k_lo0 + st * STAGE16;
+            if (elect_one()) {
             if constexpr (DUAL) {
               umma_ss_lo<false>(tq + C::COL_S, q_lo, k_lo, idesc_s2);  // [S | tS] = Q [K ; tK]^T
 #pragma unroll
@@ -394,6 +395,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
             }
             tc_commit_u32(bar_s_full);
             if (j == my_last) tc_commit_u32(bar_q_empty);  // arrives when the item's last scores are complete
+            }
             if (pend && !issue_pv(pend_st, pend_par, pend_first)) {
               ok = false;
               break;
@@ -410,7 +412,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
               }
               pend = false;
             }
-            mbar_arrive(kv_empty + st);
+            if (elect_one()) mbar_arrive(kv_empty + st);
           }
           if (++st == STAGES) st = 0, st_par ^= 1;
         }
@@ -418,12 +420,14 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         if (pend && !issue_pv(pend_st, pend_par, pend_first)) break;
         if (!first)
           ++kx;  // this query tile used key tiles in the item (its q_empty arrival went out with the last scores)
-        else
+        else if (elect_one())
           mbar_arrive(q_empty);
         ++kact;
       }
     }
-  } else if (warp >= 4) {
+  }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     // ------------------------------------------------------------------ softmax + epilogue of query tile X
     const int X = (warp - 4) >> 2;
     const int quarter = warp & 3;  // the TMEM lane quarter this warp may access

@@ -272,29 +272,36 @@ static __device__ __noinline__ bool mbar_wait_slow_u32(uint32_t bar, uint32_t pa
   }
 }
 
-// The wait of an issuing warp, by all of its lanes with one outcome for them (the vote tells the compiler so).  A warp
-// that stays converged keeps descriptors and loop counters in uniform registers, where tcgen05.mma takes its operands from, and
-// only the instructions themselves are one lane's (`elect_one`).  Issued from a branch of lane 0 every operand is moved there
-// first: measured on a B200, cycles per M = 128 instruction with such a branch / a converged warp: N = 64 with A in TMEM
-// 45-54 / 32, both operands in shared memory 48-57 / 48 (what the port delivers), N = 32 45 / 40, N = 128 64 / 64.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const AbortState& ab, int code) {
-  const uint32_t addr = smem_u32(bar);
-  if (__all_sync(0xffffffffu, mbar_try_wait_u32(addr, parity))) return true;
-  const long long t0 = clock64();
-  int polls = 0;
-  while (true) {
-    if (__all_sync(0xffffffffu, mbar_try_wait_u32(addr, parity))) return true;
-    if ((++polls & 63) == 0) {
-      if (__any_sync(0xffffffffu, *ab.cta_flag != 0)) return false;
-      if (__any_sync(0xffffffffu, clock64() - t0 > kWaitBudgetCycles)) {
-        if ((threadIdx.x & 31) == 0) {
+// The wait of an issuing warp, by all of its lanes with one outcome for them (a lane that gave up takes the others along: what
+// follows needs all of them).  A warp that stays converged keeps descriptors and loop counters in uniform registers, where
+// tcgen05.mma takes its operands from, and only the instructions themselves are one lane's (`elect_one`).  Issued from a branch of
+// lane 0 every operand is moved there first: measured on a B200, cycles per M = 128 instruction with such a branch / a converged
+// warp: N = 64 with A in TMEM 45-54 / 32, both operands in shared memory 48-57 / 48 (what the port delivers), N = 32 45 / 40,
+// N = 128 64 / 64.
+__device__ __forceinline__ bool mbar_wait_warp_u32(uint32_t addr, uint32_t parity, const AbortState& ab, int code) {
+  bool ok = true;
+  if (!mbar_try_wait_u32(addr, parity)) {
+    const long long t0 = clock64();
+    int polls = 0;
+    while (!mbar_try_wait_u32(addr, parity)) {
+      if ((++polls & 63) == 0) {
+        if (*ab.cta_flag != 0) {
+          ok = false;
+          break;
+        }
+        if (clock64() - t0 > kWaitBudgetCycles) {
           *ab.cta_flag = code;
           publish_abort(ab.global_status, code);
+          ok = false;
+          break;
         }
-        return false;
       }
     }
   }
+  return __all_sync(0xffffffffu, ok);
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const AbortState& ab, int code) {
+  return mbar_wait_warp_u32(smem_u32(bar), parity, ab, code);
 }
 // One lane of the converged warp, always the same.
 __device__ __forceinline__ bool elect_one() {
