@@ -198,7 +198,7 @@ typedef struct {
   const void* mask_tile_live_t;
   /* Optional caller-owned scratch: B*H*L*D floats, 16-byte aligned, contents irrelevant on entry.  With it (D = 64,
    * 16-bit types, mask kinds NONE / CAUSAL / KVLEN, and with key stride 1, 16-byte aligned rows and L % 16 == 0 also
-   * BOOL without the two bitmaps above, or - through O alone - BIAS of the tensors' type) the backward runs as ONE pass that forms every score tile once:
+   * BOOL without the two bitmaps above, or - through O alone; through tO see jvpfa_bwd_workspace - BIAS of the tensors' type) the backward runs as ONE pass that forms every score tile once:
    * dK and dV accumulate on chip, dQ is summed into this buffer with floating-point reductions and converted at the
    * end, so dQ is reproducible to rounding but not bitwise from run to run.  NULL: the two-launch kernels, which
    * recompute the score tiles for dQ (as upstream does, jvp_attention.py:1415-1707) and are bitwise reproducible. */
@@ -217,7 +217,9 @@ typedef struct {
 } jvpfa_bwd_args;
 
 /* As jvpfa_fwd_workspace.  Non-zero for JVPFA_FP32 through O, and for dQ alone (JVPFA_SKIP_DKDV) through tO with
- * JVPFA_ZERO_TKV.  These recompute the scores as jvpfa_fwd with its workspace forms them, the other kernels as jvpfa_fwd without:
+ * JVPFA_ZERO_TKV; and for 16-bit types at D = 64 through tO with a BIAS of their type (key stride 1, 16-byte aligned rows,
+ * L % 16 == 0), where the backward then is one pass, bitwise reproducible, that leaves a share of dQ for each 128 keys there.
+ * The fp32 ones recompute the scores as jvpfa_fwd with its workspace forms them, the other kernels as jvpfa_fwd without:
  * lse and mu fit the scores to the last bit when both calls of a pair are given a workspace, or neither. */
 int64_t jvpfa_bwd_workspace(const jvpfa_bwd_args* args);
 

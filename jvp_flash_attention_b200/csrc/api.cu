@@ -227,7 +227,8 @@ int jvpfa_bwd_uses_tcgen05(const jvpfa_bwd_args* args) {
 int64_t jvpfa_bwd_workspace(const jvpfa_bwd_args* args) {
   jvpfa_bwd_args full;
   const jvpfa_bwd_args* a = current_bwd_args(args, &full);
-  return validate_bwd(a) == JVPFA_OK ? bwd_f32_tc5_workspace(*a) : 0;
+  if (validate_bwd(a) != JVPFA_OK) return 0;
+  return a->dtype == JVPFA_FP32 ? bwd_f32_tc5_workspace(*a) : bwd_bias_workspace(*a);
 }
 
 int jvpfa_fwd(const jvpfa_fwd_args* args, void* stream) {

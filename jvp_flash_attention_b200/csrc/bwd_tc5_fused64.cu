@@ -1,4 +1,4 @@
-// Single-pass tcgen05 backward for head dimension 64 (bf16 / fp16; none, causal, key padding): the score
+// Single-pass tcgen05 backward for head dimension 64 (bf16 / fp16): the score
 // tiles S, tS, E, FP are formed ONCE per (128 keys x 64 queries) sub-tile and feed all three gradients.
 //
 // The two-launch backward (bwd_tc5_d64.cu, like upstream's _attn_bwd_dkdv / _attn_bwd_dq,
@@ -14,9 +14,14 @@
 // shared memory also frees the score accumulators as soon as the elementwise threads hold them in
 // registers, so the scores of sub-tile g+1 are formed while sub-tile g is still being worked on.
 // A dQ sub-tile is read back by a fourth warpgroup (an M = 64 accumulator sits in lanes 0..15 of each
-// 32-lane quarter) and added to an fp32 accumulation buffer in global memory with vector reductions
-// (red.global.add.v4.f32); a small kernel converts that buffer to the output type at the end.  The order of
-// those additions varies from run to run, so dQ is reproducible to rounding, not bitwise.
+// 32-lane quarter) and added to an fp32 accumulation buffer in global memory with TMA reductions; a small kernel converts that
+// buffer to the output type at the end.  The order of those additions varies from run to run, so dQ is reproducible to
+// rounding, not bitwise.  (With a bias and through tO a key tile's share is stored instead, see kDqParts.)
+//
+// Measured on a B200, cycles of a sub-tile with every SM at work (37 heads, L2048): through O 1960, through tO 2760-2800, both
+// 3500 (4030 with one ring of two stages for all four streamed tiles); the tensor pipe's own time is 1024, 1860 and 2050.  What
+// bounds it: the elementwise threads are busy four fifths of the time (two warps for a scheduler, so their latencies show), beside
+// a shared-memory port that MMA operands, statistics and result tiles fill to nine tenths.
 //
 // Warps: 0 TMA producer (+ per-query statistics), 1 score issuer, 2 dK/dV issuer, 3 dQ issuer,
 // 4..11 two elementwise warpgroups (thread <-> key row; group w takes query columns [32w, 32w+32) of every
@@ -41,6 +46,12 @@ __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* map, uint32
                "r"(smem_src), "r"(x), "r"(y), "r"(z), "r"(w)
                : "memory");
 }
+// The same as a plain store.
+__device__ __forceinline__ void tma_store_part_4d(const CUtensorMap* map, uint32_t smem_src, int x, int y, int z, int w) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(map), "r"(smem_src),
+               "r"(x), "r"(y), "r"(z), "r"(w)
+               : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
@@ -50,7 +61,12 @@ struct BwdFCfg {
   static constexpr int D = 64;
   static constexpr int OWN = 128;
   static constexpr int BL = 64;
-  static constexpr int STAGES = (HAS_GO && HAS_GT) ? 2 : 3;
+  // The streamed tiles go through one ring, or, where three stages of all four would not fit, through two: Q and tQ three
+  // stages deep, G and gO two.  With two stages of everything the scores of sub-tile g + 2 waited for the outputs of g and then
+  // for the loads (half of the score issuer's time).
+  static constexpr bool TWO_RINGS = HAS_GO && HAS_GT;
+  static constexpr int STAGES = 3;
+  static constexpr int GSTAGES = TWO_RINGS ? 2 : STAGES;  // (also the stages of the statistics)
   // The shared-memory result tiles (gS, gtS) exist twice, so that the elementwise threads can write sub-tile g + 1
   // while the products of sub-tile g still read theirs.
   static constexpr int N_OBUF = 2;
@@ -61,7 +77,8 @@ struct BwdFCfg {
   static constexpr int OWN_BYTES = OWN * D * 2;   // 16 KiB
   static constexpr int LOOP_BYTES = BL * D * 2;   // 8 KiB
   static constexpr int OUT_BYTES = OWN * BL * 2;  // 16 KiB: [128 keys][64 queries]
-  static constexpr int STAGE_BYTES = N_LOOP * LOOP_BYTES;
+  static constexpr int STAGE_BYTES = (TWO_RINGS ? 2 : N_LOOP) * LOOP_BYTES;
+  static constexpr int G_STAGE_BYTES = TWO_RINGS ? 2 * LOOP_BYTES : 0;
   static constexpr int STAT_STAGE_BYTES = (BL / 2) * 32;  // per query pair two float4
   // Two sets of own tiles where shared memory allows it (backward through O alone: K and V only): the next item's
   // are then loaded while this item's last sub-tiles run.  With one set the item boundary is exposed - the next
@@ -70,20 +87,21 @@ struct BwdFCfg {
   static constexpr int OWN_SET_BYTES = N_OWN * OWN_BYTES;
   static constexpr int OFF_OWN = 0;
   static constexpr int OFF_RING = OWN_BUFS * OWN_SET_BYTES;
-  static constexpr int OFF_OUT = OFF_RING + STAGES * STAGE_BYTES;
+  static constexpr int OFF_GRING = OFF_RING + STAGES * STAGE_BYTES;
+  static constexpr int OFF_OUT = OFF_GRING + GSTAGES * G_STAGE_BYTES;
   static constexpr int OBUF_BYTES = N_OUT * OUT_BYTES;
   static constexpr int OFF_STAT = OFF_OUT + N_OBUF * OBUF_BYTES;
   // dQ of a sub-tile on its way out: fp32 [64 queries][64 columns] as two 128-byte-swizzled halves of 32 columns
-  static constexpr int OFF_DQS = OFF_STAT + STAGES * STAT_STAGE_BYTES;
+  static constexpr int OFF_DQS = OFF_STAT + GSTAGES * STAT_STAGE_BYTES;
   static constexpr int DQS_BYTES = BL * D * 4;
   static_assert(OFF_DQS % 1024 == 0, "swizzled staging tile alignment");
   static constexpr int TILE_BYTES = OFF_DQS + DQS_BYTES;
-  static constexpr int SMEM_NEEDED = TILE_BYTES + 512 + 1024;
+  static constexpr int SMEM_NEEDED = TILE_BYTES + 512;
   // At least 120 KiB so that a second CTA can never share the SM (the CTA allocates all of TMEM).
   static constexpr int SMEM_BYTES = SMEM_NEEDED > 120 * 1024 ? SMEM_NEEDED : 120 * 1024;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
   static constexpr int SLOT_K = 0, SLOT_TK = 1, SLOT_V = HAS_GT ? 2 : 1, SLOT_TV = 3;
-  static constexpr int SLOT_Q = 0, SLOT_TQ = 1, SLOT_G = 2, SLOT_GO = HAS_GT ? 3 : 1;
+  static constexpr int SLOT_Q = 0, SLOT_TQ = 1, SLOT_G = TWO_RINGS ? 0 : 2, SLOT_GO = HAS_GT ? SLOT_G + 1 : 1;
   static constexpr int OUT_GS = 0, OUT_GT = 1;
   static constexpr int COL_S = 0, COL_TS = 64, COL_E = 128, COL_FP = HAS_GT ? 192 : 64;
   static constexpr int COL_DK = 256, COL_DV = 320, COL_DQ = 384;
@@ -115,29 +133,37 @@ struct FItem {
 
 // MK: 0 = none / causal / key padding (index comparisons); 1 = uint8 mask with any strides (each elementwise thread
 // reads the 32 mask bytes of its key row and the sub-tile's queries before it waits for the scores); 2 = additive bias of
-// the element type, read the same way (HAS_GT == false only).
+// the element type, read the same way.
+//
+// dQ of a bias call through tO is summed in a fixed order, as the two launches that served it sum it: a key tile's share goes to
+// a buffer of its own (dq_acc: [key tile][B*H][L][D] floats) and dq_sum_kernel adds them up.  Measured on a B200, the two
+// launches / this with the sum, us, bf16 through both outputs: B2 H12 L512 42 / 38, L1024 134 / 105, L2048 353 / 290, H4 L4096
+// 229 / 187; with 48 key tiles (B2 H12 L256) 22 / 28, with 32 (H1 L4096) 124 / 173.
+template <bool HAS_GT, int MK>
+constexpr bool kDqParts = HAS_GT && MK == 2;
 template <typename T, bool HAS_GO, bool HAS_GT, int MK>
 __global__ void __launch_bounds__(512, 1)
 bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps maps, float* dq_acc, int* status) {
   using C = BwdFCfg<HAS_GO, HAS_GT>;
-  constexpr int D = 64, OWN = C::OWN, BL = C::BL, STAGES = C::STAGES;
+  constexpr int D = 64, OWN = C::OWN, BL = C::BL, STAGES = C::STAGES, GSTAGES = C::GSTAGES;
 
   const bool dead_on_entry = *(volatile int*)status != 0;  // an earlier bounded wait gave up
 
-  extern __shared__ unsigned char smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
-  unsigned char* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
+  extern __shared__ __align__(1024) unsigned char smem[];  // (the tiles' swizzle repeats every 1024 bytes)
   unsigned char* sOwn = smem + C::OFF_OWN;
   unsigned char* sRing = smem + C::OFF_RING;
   unsigned char* sOut = smem + C::OFF_OUT;
-  float4* sStat = reinterpret_cast<float4*>(smem + C::OFF_STAT);  // [STAGES][BL/2][2]
+  unsigned char* sG = smem + C::OFF_GRING;
+  float4* sStat = reinterpret_cast<float4*>(smem + C::OFF_STAT);  // [GSTAGES][BL/2][2]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::TILE_BYTES);
   uint64_t* own_full = bars + 0;             // [2] per set of own tiles (item kact uses set kact % OWN_BUFS)
   uint64_t* own_free = bars + 2;             // [2] score issuer + dQ issuer are through with the set
   uint64_t* loop_full = bars + 4;            // [STAGES]
   uint64_t* loop_empty = loop_full + STAGES;  // [STAGES]: score issuer + dK/dV issuer
-  uint64_t* stat_full = loop_empty + STAGES;  // [STAGES]
-  uint64_t* s_full = stat_full + STAGES;
+  uint64_t* g_full = loop_empty + STAGES;     // [2] TWO_RINGS: the same of G and gO
+  uint64_t* g_empty = g_full + 2;             // [2]
+  uint64_t* stat_full = g_empty + 2;          // [GSTAGES]
+  uint64_t* s_full = stat_full + GSTAGES;
   uint64_t* s_free = s_full + 1;    // 256 elementwise threads hold the scores in registers
   // [2] by g & 1, 256 each: gS, gtS, A, P of the sub-tile are in shared memory. A pair, because the elementwise
   // threads can finish sub-tile g + 1 before the dQ issuer has looked at g (sub-tile g + 1 needs the dV products of
@@ -201,10 +227,15 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       if (tid < OWN && i < L) {
         poison_row<T>(a.dk, (size_t)it.bh * L + i, D);
         poison_row<T>(a.dv, (size_t)it.bh * L + i, D);
-        dq_acc[((size_t)it.bh * L + i) * D] = poison_f32();
+        dq_acc[((kDqParts<HAS_GT, MK> ? (size_t)(it.own0 / OWN) * BH * L : 0) + (size_t)it.bh * L + i) * D] = poison_f32();
       }
     }
   };
+  if ((smem_u32(smem) & 1023u) != 0) {  // (does not happen: the array is declared so)
+    if (tid == 0) publish_abort(status, kAbortAux);
+    poison();
+    return;
+  }
   if (dead_on_entry) {
     poison();
     return;
@@ -218,7 +249,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(loop_full + s, 1);
       mbar_init(loop_empty + s, 2);
-      mbar_init(stat_full + s, 1);
+      if (s < 2) mbar_init(g_full + s, 1), mbar_init(g_empty + s, 2);
+      if (s < GSTAGES) mbar_init(stat_full + s, 1);
     }
     mbar_init(s_full, 1);
     mbar_init(s_free, 256);
@@ -246,12 +278,13 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 
   // Registers: the elementwise threads hold four 32-column accumulator slices; everybody else needs few.
   // (setmaxnreg.inc draws on what setmaxnreg.dec of the same CTA has released and blocks until it is there: 256
-  // threads x 56 registers up equals 256 threads x 56 registers down from the 128 the kernel is launched with.)
+  // threads x 48 registers up equals 256 threads x 48 registers down from the 128 the kernel is launched with.  At 72 the
+  // read-back threads, which hold 64 of a row, and the issuers spilled: through tO at B4 H16 L2048 causal 204 us against 193.)
+  // (It stands in the branches of the roles: ptxas holds code behind a join of the two to the smaller number.)
   // Phase counters kept alike by all roles: g counts the sub-tiles of this CTA (ring stage g % STAGES, dQ buffer
   // g & 1; s_full, s_free complete once per sub-tile, p_full and out_free of buffer g & 1 every other one), kact the items that have sub-tiles.
-  // (setmaxnreg stands in the branches of the roles: ptxas holds code behind a join of the two to the smaller number.)
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer + per-query statistics
     if (lane == 0) {
@@ -299,35 +332,49 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           }
         }
       };
-      Stat cur, nxt;
-      load_stats(0, cur);
-      for (int s = 0; s < it.n_sub; ++s, ++g) {
+      // One sub-tile: its tiles, the loads of the next one's statistics, and its own, which arrived meanwhile.  (Two names that
+      // take turns: a copy from one to the other would wait for the loads, and the next tiles with it.)
+      auto sub_tile = [&](int s, const Stat& cur, Stat& nxt) -> bool {
         const int st = g % STAGES;
-        if (!mbar_wait_backoff(loop_empty + st, ((g / STAGES) & 1) ^ 1, ab, kAbortBwdLoopEmpty)) {
-          ok = false;
-          break;
-        }
+        if (!mbar_wait_backoff<32>(loop_empty + st, ((g / STAGES) & 1) ^ 1, ab, kAbortBwdLoopEmpty)) return false;
         const int l0 = it.loop_begin + s * BL;
         if (lane == 0) {
           unsigned char* base = sRing + st * C::STAGE_BYTES;
           mbar_expect_tx(loop_full + st, C::STAGE_BYTES);
           tma_load_4d(base + C::SLOT_Q * C::LOOP_BYTES, &maps.q, loop_full + st, 0, l0, it.h, it.b);
-          if constexpr (HAS_GO) tma_load_4d(base + C::SLOT_GO * C::LOOP_BYTES, &maps.go, loop_full + st, 0, l0, it.h, it.b);
-          if constexpr (HAS_GT) {
-            tma_load_4d(base + C::SLOT_TQ * C::LOOP_BYTES, &maps.tq, loop_full + st, 0, l0, it.h, it.b);
-            tma_load_4d(base + C::SLOT_G * C::LOOP_BYTES, &maps.g, loop_full + st, 0, l0, it.h, it.b);
+          if constexpr (HAS_GT) tma_load_4d(base + C::SLOT_TQ * C::LOOP_BYTES, &maps.tq, loop_full + st, 0, l0, it.h, it.b);
+          if constexpr (!C::TWO_RINGS) {
+            if constexpr (HAS_GO) tma_load_4d(base + C::SLOT_GO * C::LOOP_BYTES, &maps.go, loop_full + st, 0, l0, it.h, it.b);
+            if constexpr (HAS_GT) tma_load_4d(base + C::SLOT_G * C::LOOP_BYTES, &maps.g, loop_full + st, 0, l0, it.h, it.b);
+          }
+        }
+        const int gst = g % GSTAGES;
+        if constexpr (C::TWO_RINGS) {
+          if (!mbar_wait_backoff<32>(g_empty + gst, ((g / GSTAGES) & 1) ^ 1, ab, kAbortBwdLoopEmpty)) return false;
+          if (lane == 0) {
+            unsigned char* base = sG + gst * C::G_STAGE_BYTES;
+            mbar_expect_tx(g_full + gst, C::G_STAGE_BYTES);
+            tma_load_4d(base + C::SLOT_G * C::LOOP_BYTES, &maps.g, g_full + gst, 0, l0, it.h, it.b);
+            tma_load_4d(base + C::SLOT_GO * C::LOOP_BYTES, &maps.go, g_full + gst, 0, l0, it.h, it.b);
           }
         }
         load_stats(s + 1, nxt);
         // negated and stored pairwise for the packed arithmetic:
         //   float4 A = (-lse0, -lse1, -mu0, -mu1), float4 B = (-eps0, -eps1, -sub0, -sub1)
-        float4* dst = sStat + (st * (BL / 2) + lane) * 2;
+        float4* dst = sStat + (gst * (BL / 2) + lane) * 2;
         dst[0] = make_float4(-cur.lse[0], -cur.lse[1], -cur.mu[0], -cur.mu[1]);
         dst[1] = make_float4(-cur.eps[0], -cur.eps[1], -(cur.delta[0] + cur.cterm[0] + cur.eps[0] * cur.mu[0]),
                              -(cur.delta[1] + cur.cterm[1] + cur.eps[1] * cur.mu[1]));
         __syncwarp();
-        if (lane == 0) mbar_arrive(stat_full + st);
-        cur = nxt;
+        if (lane == 0) mbar_arrive(stat_full + gst);
+        ++g;
+        return true;
+      };
+      Stat s0, s1;
+      load_stats(0, s0);
+      for (int s = 0; ok && s < it.n_sub; s += 2) {
+        ok = sub_tile(s, s0, s1);
+        if (ok && s + 1 < it.n_sub) ok = sub_tile(s + 1, s1, s0);
       }
       ++kact;
     }
@@ -347,6 +394,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       constexpr uint32_t OWNSET16 = C::OWN_SET_BYTES >> 4;
       const uint32_t ring_k = kDescLo | (smem_u32(sRing) >> 4);  // streamed tiles as K-major B operands (scores)
       const uint32_t ring_mn = kLoMN | (smem_u32(sRing) >> 4);   // ... as MN-major B operands (dK, dV)
+      constexpr uint32_t GSTAGE16 = C::G_STAGE_BYTES >> 4;       // G and gO: a ring of their own, or beside Q
+      const uint32_t gring_k = kDescLo | (smem_u32(sG) >> 4), gring_mn = kLoMN | (smem_u32(sG) >> 4);
       const uint32_t out_k = kDescLo | (smem_u32(sOut) >> 4);    // elementwise results as K-major A operands (dK, dV)
       const uint32_t out_mn = kLoMN | (smem_u32(sOut) >> 4);     // ... as MN-major A operands (dQ)
       int g = 0, kact = 0;
@@ -378,20 +427,40 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             }
             tc_fence_after();
             const uint32_t lp = ring_k + st * STAGE16;
-            if (elect_one()) {
-            if constexpr (HAS_GT) {
-              score(C::COL_S, C::SLOT_K, lp + C::SLOT_Q * LOOP16, idesc_sc2, true);    // [S | tS] = K [Q ; tQ]^T
-              score(C::COL_TS, C::SLOT_TK, lp + C::SLOT_Q * LOOP16, idesc_sc, false);  // tS += tK Q^T
-              score(C::COL_E, C::SLOT_V, lp + C::SLOT_G * LOOP16, idesc_sc, true);     // E = V G^T
-              score(C::COL_FP, C::SLOT_TV, lp + C::SLOT_G * LOOP16, idesc_sc, true);   // FP = tV G^T
-              if constexpr (HAS_GO) score(C::COL_FP, C::SLOT_V, lp + C::SLOT_GO * LOOP16, idesc_sc, false);  // + V gO^T
-            } else {
-              score(C::COL_S, C::SLOT_K, lp + C::SLOT_Q * LOOP16, idesc_sc, true);    // S = K Q^T
-              score(C::COL_FP, C::SLOT_V, lp + C::SLOT_GO * LOOP16, idesc_sc, true);  // FP = V gO^T
-            }
-            tc_commit(s_full);
-            tc_commit(loop_empty + st);
-            if (s == it.n_sub - 1) tc_commit(own_free + oset);
+            const uint32_t lg = C::TWO_RINGS ? gring_k + (g % GSTAGES) * GSTAGE16 : lp;
+            auto from_q = [&]() {
+              if constexpr (HAS_GT) {
+                score(C::COL_S, C::SLOT_K, lp + C::SLOT_Q * LOOP16, idesc_sc2, true);    // [S | tS] = K [Q ; tQ]^T
+                score(C::COL_TS, C::SLOT_TK, lp + C::SLOT_Q * LOOP16, idesc_sc, false);  // tS += tK Q^T
+              } else {
+                score(C::COL_S, C::SLOT_K, lp + C::SLOT_Q * LOOP16, idesc_sc, true);  // S = K Q^T
+              }
+            };
+            auto from_g = [&]() {
+              if constexpr (HAS_GT) {
+                score(C::COL_E, C::SLOT_V, lg + C::SLOT_G * LOOP16, HAS_GO ? idesc_sc2 : idesc_sc, true);  // E = V G^T; [E | FP] = V [G ; gO]^T
+                score(C::COL_FP, C::SLOT_TV, lg + C::SLOT_G * LOOP16, idesc_sc, !HAS_GO);                  // FP (+)= tV G^T
+              } else {
+                score(C::COL_FP, C::SLOT_V, lg + C::SLOT_GO * LOOP16, idesc_sc, true);  // FP = V gO^T
+              }
+              tc_commit(s_full);
+              tc_commit(C::TWO_RINGS ? g_empty + g % GSTAGES : loop_empty + st);
+              if (s == it.n_sub - 1) tc_commit(own_free + oset);
+            };
+            if constexpr (C::TWO_RINGS) {
+              if (elect_one()) {
+                from_q();
+                tc_commit(loop_empty + st);
+              }
+              if (!mbar_wait_warp(g_full + g % GSTAGES, (g / GSTAGES) & 1, ab, kAbortBwdLoopFull)) {
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+              if (elect_one()) from_g();
+            } else if (elect_one()) {
+              from_q();
+              from_g();
             }
           }
           if (!ok) break;
@@ -426,17 +495,19 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             const int ob = g % C::N_OBUF;
             ob16 = ob * (C::OBUF_BYTES >> 4);
             const uint32_t lp = ring_mn + st * STAGE16;
+            const uint32_t lg = C::TWO_RINGS ? gring_mn + (g % GSTAGES) * GSTAGE16 : lp;
             const uint32_t acc = s > 0;
             if (elect_one()) {
             outer(C::COL_DK, C::OUT_GS, lp + C::SLOT_Q * LOOP16, acc);  // dK += gS^T Q
             if constexpr (HAS_GT) {
               outer(C::COL_DK, C::OUT_GT, lp + C::SLOT_TQ * LOOP16, 1);  // dK += gtS^T tQ
-              outer_t(C::COL_DV, C::COL_AV, lp + C::SLOT_G * LOOP16, acc);  // dV += A^T G
-              if constexpr (HAS_GO) outer_t(C::COL_DV, C::COL_P, lp + C::SLOT_GO * LOOP16, 1);  // dV += P^T gO
+              if constexpr (C::TWO_RINGS) tc_commit(loop_empty + st);
+              outer_t(C::COL_DV, C::COL_AV, lg + C::SLOT_G * LOOP16, acc);  // dV += A^T G
+              if constexpr (HAS_GO) outer_t(C::COL_DV, C::COL_P, lg + C::SLOT_GO * LOOP16, 1);  // dV += P^T gO
             } else {
-              outer_t(C::COL_DV, C::COL_P, lp + C::SLOT_GO * LOOP16, acc);  // dV += P^T gO
+              outer_t(C::COL_DV, C::COL_P, lg + C::SLOT_GO * LOOP16, acc);  // dV += P^T gO
             }
-            tc_commit(loop_empty + st);
+            tc_commit(C::TWO_RINGS ? g_empty + g % GSTAGES : loop_empty + st);
             tc_commit(out_free + ob);
             tc_commit(av_free);
             if (s == it.n_sub - 1) tc_commit(done);
@@ -487,7 +558,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
     }
   }
   } else if (warp < 12) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");
     // ------------------------------------------------------------------ elementwise warpgroups
     const int wg = (warp - 4) >> 2;  // 0 / 1: query columns [32 wg, 32 wg + 32) of every sub-tile
     const int quarter = warp & 3;
@@ -536,40 +607,49 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       const uint32_t* bcol = nullptr;  // packed boolean mask: this key's bits over the queries
       if (MK == 1 && a.mask_bits_t != nullptr)
         bcol = mask_bit_col(a.mask_bits_t, a.mask, mask_head(a.mask, it.b, it.h, a.H), min(own_idx, L - 1), L);
-      for (int s = 0; s < it.n_sub; ++s, ++g) {
-        const int st = g % STAGES;
-        const int l0 = it.loop_begin + s * BL + 32 * wg;  // first query of this group's columns
-        // MK = 1: this key's mask bits for the 32 queries, requested before the waits (packed: one word; else byte by
-        // byte, indices clamped into the tensor; what lies outside is switched off by col_hi and by lse = +inf of the
-        // padding queries)
-        // MK = 2 (backward through O alone: the variants with tangents have no registers to spare): the bias elements
-        // of the same positions, 16 bit each, of the tensors' type.
-        uint32_t live = 0xffffffffu;  // MK = 1: bit col = the mask lets query l0 + col attend this key
-        uint32_t mraw[MK == 2 ? 32 : 1];
+      // What the mask holds for this key and the 32 queries from l0 on (MK = 1: a bit each, packed one word, else byte by byte;
+      // MK = 2: the bias elements, 16 bit each, of the tensors' type).  Requested a sub-tile ahead, when the scores of this one have
+      // left their registers: behind that the scores of the next are long there, and the loads would be waited for.  Indices are
+      // clamped into the tensor; what lies outside is switched off by col_hi and by lse = +inf of the padding queries.
+      uint32_t next_live = 0xffffffffu, braw[MK == 2 ? 32 : 1];
+      auto fetch_mask = [&](int l0) {
         if (MK == 1 && bcol != nullptr) {
-          live = l0 < L ? ldg_nc_u32(bcol + (a.mask.stride[2] ? l0 >> 5 : 0)) : 0u;
+          next_live = l0 < L ? ldg_nc_u32(bcol + (a.mask.stride[2] ? l0 >> 5 : 0)) : 0u;
         } else if constexpr (MK != 0) {
           constexpr int MESZ = MK == 1 ? 1 : 2;
-          const unsigned char* pm = reinterpret_cast<const unsigned char*>(a.mask.ptr) +
+          const long long step = a.mask.stride[2] * MESZ;  // to the next query; the last one's element stands for those beyond
+          const unsigned char* el = reinterpret_cast<const unsigned char*>(a.mask.ptr) +
                                     ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] +
-                                     (long long)min(own_idx, L - 1) * a.mask.stride[3]) * MESZ;
+                                     (long long)min(own_idx, L - 1) * a.mask.stride[3]) * MESZ + min(l0, L - 1) * step;
+          const int left = L - 1 - l0;
 #pragma unroll
           for (int col = 0; col < 32; ++col) {
-            const unsigned char* el = pm + (long long)min(l0 + col, L - 1) * a.mask.stride[2] * MESZ;
             if constexpr (MK == 1) {
-              if (col == 0) live = 0u;
-              live |= (ldg_nc_u8(el) != 0u ? 1u : 0u) << col;
+              if (col == 0) next_live = 0u;
+              next_live |= (ldg_nc_u8(el) != 0u ? 1u : 0u) << col;
             } else {
-              mraw[col] = ldg_nc_u16(el);
+              braw[col] = ldg_nc_u16(el);
             }
+            if (col < left) el += step;
           }
         }
-        if (!mbar_wait(stat_full + st, (g / STAGES) & 1, ab, kAbortBwdLoopFull) ||
+      };
+      if constexpr (MK != 0) fetch_mask(it.loop_begin + 32 * wg);
+      for (int s = 0; s < it.n_sub; ++s, ++g) {
+        const int st = g % GSTAGES;  // of the statistics
+        const int l0 = it.loop_begin + s * BL + 32 * wg;  // first query of this group's columns
+        uint32_t live = next_live;  // MK = 1: bit col = the mask lets query l0 + col attend this key
+        if (!mbar_wait(stat_full + st, (g / GSTAGES) & 1, ab, kAbortBwdLoopFull) ||
             !mbar_wait(s_full, g & 1, ab, kAbortBwdSFull)) {
           alive = false;
           break;
         }
         tc_fence_after();
+        uint32_t bias[MK == 2 ? 16 : 1];
+        if constexpr (MK == 2) {  // in pairs before the scores come: 16 registers beside their 128
+#pragma unroll
+          for (int x = 0; x < 16; ++x) bias[x] = braw[2 * x] | (braw[2 * x + 1] << 16);
+        }
         uint32_t sv[32], fp[32], ts[HAS_GT ? 32 : 1], ev[HAS_GT ? 32 : 1];
         tmem_ld32(tbase + C::COL_S, sv);
         tmem_ld32(tbase + C::COL_FP, fp);
@@ -597,7 +677,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           const float2 neps = make_float2(sb.x, sb.y), nsub = make_float2(sb.z, sb.w);
           float2 xs = __ffma2_rn(ff(sv[2 * x], sv[2 * x + 1]), c2, nl);
           if constexpr (MK == 2)  // scores are in log2 units: + bias * log2(e)
-            xs = __ffma2_rn(unpack2<T>(mraw[2 * x] | (mraw[2 * x + 1] << 16)), make_float2(kLog2e, kLog2e), xs);
+            xs = __ffma2_rn(unpack2<T>(bias[x]), make_float2(kLog2e, kLog2e), xs);
           float2 p = make_float2(fast_exp2(xs.x), fast_exp2(xs.y));
           if constexpr (MASKED) {
             if constexpr (MK == 1) {
@@ -635,6 +715,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 #pragma unroll
           for (int x = 0; x < 16; ++x) pair(x, IntC<0>{});
         }
+        if constexpr (MK != 0) fetch_mask(l0 + BL);  // (behind the last one too: else this one's would have to be kept)
         // The products of the sub-tile that used this result buffer last must have read it.
         const int ob = g % C::N_OBUF, use = g / C::N_OBUF;
         if (use > 0 && !mbar_wait(out_free + ob, (use - 1) & 1, ab, kAbortBwdPFull)) {
@@ -680,7 +761,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       ++kact;
     }
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
     // ------------------------------------------------------------------ dQ read-back
     const int quarter = warp & 3;
     const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + C::COL_DQ;
@@ -729,8 +810,13 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
         rb_meet();
         if (tid == 384) {
           const int i0 = it.loop_begin + s * BL;
-          tma_reduce_add_4d(&maps.dq, dqs, 0, i0, it.h, it.b);
-          tma_reduce_add_4d(&maps.dq, dqs + 8192, 32, i0, it.h, it.b);
+          if constexpr (kDqParts<HAS_GT, MK>) {
+            tma_store_part_4d(&maps.dq, dqs, 0, i0, it.bh, it.own0 / OWN);
+            tma_store_part_4d(&maps.dq, dqs + 8192, 32, i0, it.bh, it.own0 / OWN);
+          } else {
+            tma_reduce_add_4d(&maps.dq, dqs, 0, i0, it.h, it.b);
+            tma_reduce_add_4d(&maps.dq, dqs + 8192, 32, i0, it.h, it.b);
+          }
           bulk_commit();
         }
       }
@@ -764,6 +850,22 @@ __global__ void dq_convert_kernel(const float* __restrict__ acc, T* __restrict__
                                                Elem<T>::pack(hi.x * scale, hi.y * scale), Elem<T>::pack(hi.z * scale, hi.w * scale));
 }
 
+// dq = T(scale * sum of the n_parts key tiles' shares, in their order), 4 elements per thread.  Bound by reading them (B2 H12 L1024:
+// 50 MB, most of it still in L2).
+template <typename T>
+__global__ void __launch_bounds__(256) dq_sum_kernel(const float* __restrict__ parts, T* __restrict__ dq, long long n4, int n_parts, float scale) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n4) return;
+  const float4* p = reinterpret_cast<const float4*>(parts) + i;
+  float4 s = __ldcs(p);
+#pragma unroll 8
+  for (int k = 1; k < n_parts; ++k) {
+    const float4 x = __ldcs(p + k * n4);
+    s.x += x.x, s.y += x.y, s.z += x.z, s.w += x.w;
+  }
+  reinterpret_cast<uint2*>(dq)[i] = make_uint2(Elem<T>::pack(s.x * scale, s.y * scale), Elem<T>::pack(s.z * scale, s.w * scale));
+}
+
 static int fused_sm_count() {
   static int cache[64] = {};
   int dev = 0;
@@ -795,7 +897,11 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
   if (HAS_GT)
     ok = ok && encode_map4d(&m.tk, dt, a.tk, C::D, a.L, a.H, a.B, st, C::OWN) && encode_map4d(&m.tv, dt, a.tv, C::D, a.L, a.H, a.B, st, C::OWN) &&
          encode_map4d(&m.tq, dt, a.tq, C::D, a.L, a.H, a.B, st, C::BL) && encode_map4d(&m.g, dt, a.gto, C::D, a.L, a.H, a.B, nullptr, C::BL);
-  ok = ok && encode_map4d_f32(&m.dq, a.dq_accum, C::D, a.L, a.H, a.B, C::BL);
+  constexpr bool parts = kDqParts<HAS_GT, MK>;
+  float* dq_acc = parts ? static_cast<float*>(a.workspace) : a.dq_accum;
+  const int n_key_tiles = (a.L + C::OWN - 1) / C::OWN;
+  ok = ok && (parts ? encode_map4d_f32(&m.dq, dq_acc, C::D, a.L, a.B * a.H, n_key_tiles, C::BL)
+                    : encode_map4d_f32(&m.dq, dq_acc, C::D, a.L, a.H, a.B, C::BL));
   if (!ok) {
     set_last_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled(bwd fused64)");
     return JVPFA_ERR_CUDA;
@@ -807,7 +913,7 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
   }
   const size_t n = (size_t)a.B * a.H * a.L * C::D;
   cudaError_t e = cudaSuccess;
-  if (!(a.flags & JVPFA_DQ_ACCUM_IS_ZERO)) e = cudaMemsetAsync(a.dq_accum, 0, n * sizeof(float), stream);
+  if (!parts && !(a.flags & JVPFA_DQ_ACCUM_IS_ZERO)) e = cudaMemsetAsync(a.dq_accum, 0, n * sizeof(float), stream);
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "cudaMemsetAsync(dq_accum)");
     return JVPFA_ERR_CUDA;
@@ -815,9 +921,9 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
   auto kern = bwd_tc5_fused64_kernel<T, HAS_GO, HAS_GT, MK>;
   static SmemOptIn opt_in;
   if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return JVPFA_ERR_CUDA;
-  const long long n_items = (long long)((a.L + C::OWN - 1) / C::OWN) * a.B * a.H;
+  const long long n_items = (long long)n_key_tiles * a.B * a.H;
   const int grid = (int)(n_items < sms ? n_items : sms);
-  kern<<<grid, C::NTHREADS, C::SMEM_BYTES, stream>>>(a, m, a.dq_accum, status);
+  kern<<<grid, C::NTHREADS, C::SMEM_BYTES, stream>>>(a, m, dq_acc, status);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch bwd_tc5_fused64");
@@ -825,7 +931,10 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
   }
   const long long n8 = (long long)(n / 8);
   if (a.flags & JVPFA_SKIP_DQ) return JVPFA_OK;
-  dq_convert_kernel<T><<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(a.dq_accum, reinterpret_cast<T*>(a.dq), n8, a.sm_scale);
+  if (parts)
+    dq_sum_kernel<T><<<(unsigned)((2 * n8 + 255) / 256), 256, 0, stream>>>(dq_acc, reinterpret_cast<T*>(a.dq), 2 * n8, n_key_tiles, a.sm_scale);
+  else
+    dq_convert_kernel<T><<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(dq_acc, reinterpret_cast<T*>(a.dq), n8, a.sm_scale);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch dq_convert");
@@ -837,7 +946,11 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
 template <typename T>
 static int launch_fused64_t(const jvpfa_bwd_args& a, cudaStream_t s) {
   const bool go = a.go != nullptr, gt = a.gto != nullptr;
-  if (a.mask.kind == JVPFA_MASK_BIAS) return launch_fused64<T, true, false, 2>(a, s);  // eligible only through O alone
+  if (a.mask.kind == JVPFA_MASK_BIAS) {
+    if (go && gt) return launch_fused64<T, true, true, 2>(a, s);
+    if (gt) return launch_fused64<T, false, true, 2>(a, s);
+    return launch_fused64<T, true, false, 2>(a, s);
+  }
   if (a.mask.kind == JVPFA_MASK_BOOL) {
     if (go && gt) return launch_fused64<T, true, true, 1>(a, s);
     if (gt) return launch_fused64<T, false, true, 1>(a, s);
@@ -851,20 +964,36 @@ static int launch_fused64_t(const jvpfa_bwd_args& a, cudaStream_t s) {
 }  // namespace tc5
 
 // The single-pass kernel serves D = 64 with index masks (none, causal, key padding), boolean masks that come without tile
-// bitmaps, and through O alone a bias of the tensors' type, when the caller provides the fp32 accumulation buffer for dQ.
-// What it sums there in no fixed order, so it takes only what callers know to be summed so: not head dimension 32, nor masks
-// and bias whose rows are not whole 16-byte pieces, which the kernels of a fixed order have always served (B4 H8 L1000 D32,
-// both outputs: 85 us here, 99 us there; a whole step: 209 us with either).
+// bitmaps, and a bias of the tensors' type, when the caller provides the fp32 buffer for dQ: dq_accum, or for a bias through tO
+// the workspace, in which dQ is summed in a fixed order.
+// What dq_accum takes is summed in no fixed order, so only what callers know to be summed so goes there: not head dimension 32,
+// nor masks and bias whose rows are not whole 16-byte pieces, which the kernels of a fixed order have always served (B4 H8 L1000
+// D32, both outputs: 85 us here, 99 us there; a whole step: 209 us with either).
 bool bwd_tc5_fused64_eligible(const jvpfa_bwd_args& a) {
-  if (a.D != 64 || a.dq_accum == nullptr) return false;
-  if ((reinterpret_cast<uintptr_t>(a.dq_accum) & 15u) != 0) return false;
+  if (a.D != 64) return false;
   const int k = a.mask.kind;
+  if (k == JVPFA_MASK_BIAS && a.gto != nullptr) {
+    const long long need = bwd_bias_workspace(a);
+    return need > 0 && a.workspace != nullptr && a.workspace_bytes >= need && (reinterpret_cast<uintptr_t>(a.workspace) & 15u) == 0;
+  }
+  if (a.dq_accum == nullptr || (reinterpret_cast<uintptr_t>(a.dq_accum) & 15u) != 0) return false;
   if (k == JVPFA_MASK_NONE || k == JVPFA_MASK_CAUSAL || k == JVPFA_MASK_KVLEN) return true;
   if ((a.L & 15) != 0 || !tc5_mask_layout(a.mask, a.dtype, a.L)) return false;
   // A boolean mask without tile bitmaps (dense, or not looked at beforehand): with them the two-launch kernels, which
   // step over dead tiles, are the better choice.
-  if (k == JVPFA_MASK_BOOL) return a.mask_tile_live == nullptr && a.mask_tile_live_t == nullptr;
-  return a.gto == nullptr;  // a bias: only the backward through O alone has the registers for it
+  return k != JVPFA_MASK_BOOL || (a.mask_tile_live == nullptr && a.mask_tile_live_t == nullptr);
+}
+
+// Floats for a key tile's share of dQ, of every key tile: as many bytes as the (B, H, L, L) bias itself has, up to half a GiB.
+// From 96 key tiles on: with fewer the two launches, of as many CTAs each, fill more of the 148 SMs.
+long long bwd_bias_workspace(const jvpfa_bwd_args& a) {
+  if ((a.dtype != JVPFA_BF16 && a.dtype != JVPFA_FP16) || a.impl == JVPFA_IMPL_GENERIC || a.D != 64) return 0;
+  if (a.mask.kind != JVPFA_MASK_BIAS || a.gto == nullptr || (a.flags & JVPFA_SKIP_DKDV)) return 0;
+  if ((a.L & 15) != 0 || !tc5_mask_layout(a.mask, a.dtype, a.L)) return 0;
+  const long long key_tiles = (long long)((a.L + 127) / 128) * a.B * a.H;
+  if (key_tiles < 96) return 0;
+  const long long bytes = key_tiles * a.L * a.D * 4;
+  return bytes <= (1ll << 29) ? bytes : 0;
 }
 
 int launch_bwd_tc5_fused64(const jvpfa_bwd_args& a, cudaStream_t s) {

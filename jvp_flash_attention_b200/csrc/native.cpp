@@ -438,7 +438,7 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
   a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
   for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
-  const Tensor workspace = workspace_of(call.parts ? jvpfa_bwd_workspace(&a) : 0, q);
+  const Tensor workspace = workspace_of((q.scalar_type() == at::kFloat ? call.parts : g_single_pass.load()) ? jvpfa_bwd_workspace(&a) : 0, q);
   const Tensor bits = use_workspace(a, workspace, call, q);
   check_status(jvpfa_bwd(&a, stream), "jvpfa_bwd");
   return g;

@@ -50,16 +50,20 @@ def in_order(w, gen):
         yield x
 
 
-def run_fused64(n_subs, stages, seed, single_p_full=False, slow_dq=0.0, own_bufs=1):
+def run_fused64(n_subs, stages, seed, single_p_full=False, slow_dq=0.0, own_bufs=1, g_stages=0):
     """One random interleaving for a CTA whose item k has n_subs[k] sub-tiles (0: an item of padding only, which every
     role skips).  slow_dq: probability with which the dQ issuer lets a turn pass without doing anything.  own_bufs: sets
-    of own tiles (2 in the variant without tangents: the next item's are loaded while this item still runs)."""
+    of own tiles (2 in the variant without tangents: the next item's are loaded while this item still runs).  g_stages: with
+    it G and gO have a ring of their own, and the statistics go by its stages (the variant through both outputs)."""
     w = World(seed)
     own_full = [w.bar(1) for _ in range(own_bufs)]
     own_free = [w.bar(2) for _ in range(own_bufs)]
     loop_full = [w.bar(1) for _ in range(stages)]
     loop_empty = [w.bar(2) for _ in range(stages)]
-    stat_full = [w.bar(1) for _ in range(stages)]
+    g_full = [w.bar(1) for _ in range(g_stages)]
+    g_empty = [w.bar(2) for _ in range(g_stages)]
+    n_stat = g_stages or stages
+    stat_full = [w.bar(1) for _ in range(n_stat)]
     s_full, s_free = w.bar(1), w.bar(GROUPS)
     p_full = [w.bar(GROUPS)] if single_p_full else [w.bar(GROUPS), w.bar(GROUPS)]
     out_free = [w.bar(2), w.bar(2)]
@@ -83,10 +87,14 @@ def run_fused64(n_subs, stages, seed, single_p_full=False, slow_dq=0.0, own_bufs
                 st = g % stages
                 yield from w.wait(loop_empty[st], ((g // stages) & 1) ^ 1, ("ring_free", g - stages) if g >= stages else None)
                 w.later(lambda g=g, st=st: (w.events.add(("loop", g)), loop_full[st].arrive()))
+                if g_stages:
+                    gs = g % g_stages
+                    yield from w.wait(g_empty[gs], ((g // g_stages) & 1) ^ 1, ("g_free", g - g_stages) if g >= g_stages else None)
+                    w.later(lambda g=g, gs=gs: (w.events.add(("gloop", g)), g_full[gs].arrive()))
                 # the statistics of the stage are overwritten here: their readers must be through
-                assert g < stages or ("operands", g - stages) in w.events
+                assert g < n_stat or ("operands", g - n_stat) in w.events
                 w.events.add(("stat", g))
-                stat_full[st].arrive()
+                stat_full[g % n_stat].arrive()
                 g += 1
                 yield
 
@@ -99,8 +107,15 @@ def run_fused64(n_subs, stages, seed, single_p_full=False, slow_dq=0.0, own_bufs
                 yield from w.wait(loop_full[st], (g // stages) & 1, ("loop", g))
                 if g > 0:
                     yield from w.wait(s_free, (g - 1) & 1, ("scores_read", g - 1))
-                w.later(lambda g=g, st=st: (w.events.add(("scores", g)), s_full.arrive(),
-                                            w.tally(("rf", g), 2, ("ring_free", g)), loop_empty[st].arrive()))
+                if g_stages:
+                    w.later(lambda g=g, st=st: (w.tally(("rf", g), 2, ("ring_free", g)), loop_empty[st].arrive()))
+                    gs = g % g_stages
+                    yield from w.wait(g_full[gs], (g // g_stages) & 1, ("gloop", g))
+                    w.later(lambda g=g, gs=gs: (w.events.add(("scores", g)), s_full.arrive(),
+                                                w.tally(("gf", g), 2, ("g_free", g)), g_empty[gs].arrive()))
+                else:
+                    w.later(lambda g=g, st=st: (w.events.add(("scores", g)), s_full.arrive(),
+                                                w.tally(("rf", g), 2, ("ring_free", g)), loop_empty[st].arrive()))
                 g += 1
                 yield
             w.later(lambda kact=kact: (w.tally(("or", kact), 2, ("own_released", kact)), own_free[kact % own_bufs].arrive()))
@@ -113,6 +128,9 @@ def run_fused64(n_subs, stages, seed, single_p_full=False, slow_dq=0.0, own_bufs
                 yield from wait_p_full(g)
                 if s == 0 and kact > 0:
                     yield from w.wait(acc_free, (kact - 1) & 1, ("acc_read", kact - 1))
+                if g_stages:
+                    gs = g % g_stages
+                    w.later(lambda g=g, gs=gs: (w.tally(("gf", g), 2, ("g_free", g)), g_empty[gs].arrive()))
                 w.later(lambda g=g, st=st, ob=ob: (w.tally(("rf", g), 2, ("ring_free", g)), loop_empty[st].arrive(),
                                                    w.tally(("of", g), 2, ("out_read", g)), out_free[ob].arrive(),
                                                    w.events.add(("av_read", g)), av_free.arrive()))
@@ -140,8 +158,8 @@ def run_fused64(n_subs, stages, seed, single_p_full=False, slow_dq=0.0, own_bufs
         g = 0
         for kact, (k, n) in enumerate(items):
             for _ in range(n):
-                st, ob, use = g % stages, g & 1, g >> 1
-                yield from w.wait(stat_full[st], (g // stages) & 1, ("stat", g))
+                st, ob, use = g % n_stat, g & 1, g >> 1
+                yield from w.wait(stat_full[st], (g // n_stat) & 1, ("stat", g))
                 yield from w.wait(s_full, g & 1, ("scores", g))
                 w.tally(("sr", g), GROUPS, ("scores_read", g))
                 s_free.arrive()
@@ -183,6 +201,13 @@ def test_fused64_protocol_has_no_deadlock_and_no_premature_pass(n_subs, stages):
         assert run_fused64(n_subs, stages, seed, slow_dq=0.9) == "ok", (n_subs, stages, seed, "slow dQ issuer")
         assert run_fused64(n_subs, stages, seed, own_bufs=2) == "ok", (n_subs, stages, seed, "two sets of own tiles")
         assert run_fused64(n_subs, stages, seed, slow_dq=0.9, own_bufs=2) == "ok", (n_subs, stages, seed, "two sets, slow dQ")
+
+
+@pytest.mark.parametrize("n_subs", [[1], [2], [5], [1, 1, 1], [3, 0, 4], [16, 8, 1], [32]], ids=str)
+def test_fused64_protocol_with_a_ring_for_the_cotangents(n_subs):
+    for seed in range(8):
+        assert run_fused64(n_subs, 3, seed, g_stages=2) == "ok", (n_subs, seed)
+        assert run_fused64(n_subs, 3, seed, slow_dq=0.9, g_stages=2) == "ok", (n_subs, seed, "slow dQ issuer")
 
 
 def test_fused64_model_shows_the_stall_of_a_single_p_full_barrier():
