@@ -542,9 +542,6 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
       constexpr bool BOOLM = MK == 1 || MK == 3;
       constexpr int MESZ = BOOLM ? 1 : 2;       // bytes per mask element
       constexpr int MW = MK == 2 ? 32 : 1;      // 32-bit words per row of a 64-key tile of bias elements
-      // The tangent scores are fetched together with the scores, so that the accumulators are free at once,
-      // where the registers allow it (no bias elements to hold).
-      constexpr bool EARLY_TS = DUAL && MK != 2;
       const unsigned char* mrow = nullptr;
       const uint32_t* brow = nullptr;  // packed boolean mask
       if constexpr (BOOLM) {
@@ -555,22 +552,21 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         mrow = reinterpret_cast<const unsigned char*>(a.mask.ptr) +
                ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] +
                 (long long)min(i, L - 1) * a.mask.stride[2]) * MESZ;
-      TileUse<MK> use(it);
-      bool first = true;  // the item's first tile used by this query tile
-      for (int j = 0; j < it.n_load; ++j) {
-        if (!(use(j) & (1 << X))) continue;
-        const int n0 = j * BN;
-        uint32_t mw[MW];
-        uint2 keys = make_uint2(~0u, ~0u);  // BOOLM: bit c of (x, y) = the mask lets this row attend key n0 + c
+      // The mask's piece of a tile.  Where the next tile is known it is requested when the registers of this one's are free
+      // again: behind its own tile's beginning the scores are there already, and the loads would be waited for.  (Without a
+      // condition, zeros beyond the last tile: else this tile's piece would have to be kept.)
+      uint32_t mw[MW];
+      uint2 next_keys = make_uint2(~0u, ~0u);
+      auto fetch_mask = [&](int n0) {
         if constexpr (BOOLM) {
           if (brow != nullptr) {
-            keys = ldg_nc_v2(brow + (n0 >> 5));
+            next_keys = n0 < L ? ldg_nc_v2(brow + (n0 >> 5)) : make_uint2(0u, 0u);
           } else {
-            keys.x = mask_piece_bits(mrow + n0, n0, L) | mask_piece_bits(mrow + n0 + 16, n0 + 16, L) << 16;
-            keys.y = mask_piece_bits(mrow + n0 + 32, n0 + 32, L) | mask_piece_bits(mrow + n0 + 48, n0 + 48, L) << 16;
+            next_keys.x = mask_piece_bits(mrow + n0, n0, L) | mask_piece_bits(mrow + n0 + 16, n0 + 16, L) << 16;
+            next_keys.y = mask_piece_bits(mrow + n0 + 32, n0 + 32, L) | mask_piece_bits(mrow + n0 + 48, n0 + 48, L) << 16;
           }
         }
-        if constexpr (MK == 2) {  // issued before the wait: the loads fly while the scores are formed
+        if constexpr (MK == 2) {
 #pragma unroll
           for (int q4 = 0; q4 < MW / 4; ++q4) {
             uint4 r = make_uint4(0u, 0u, 0u, 0u);
@@ -578,21 +574,33 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
             mw[4 * q4] = r.x, mw[4 * q4 + 1] = r.y, mw[4 * q4 + 2] = r.z, mw[4 * q4 + 3] = r.w;
           }
         }
+      };
+      constexpr bool AHEAD = MK == 1 || MK == 2;
+      if constexpr (AHEAD) fetch_mask(0);
+      TileUse<MK> use(it);
+      bool first = true;  // the item's first tile used by this query tile
+      for (int j = 0; j < it.n_load; ++j) {
+        if (!(use(j) & (1 << X))) continue;
+        const int n0 = j * BN;
+        if constexpr (BOOLM && !AHEAD) fetch_mask(n0);
+        uint2 keys = next_keys;  // BOOLM: bit c of (x, y) = the mask lets this row attend key n0 + c
         if (!mbar_wait(s_full + X, t & 1, ab, kAbortSFull)) {
           alive = false;
           break;
         }
         tc_fence_after();
         uint32_t x0[32], x1[32];
-        uint32_t t0[EARLY_TS ? 32 : 1], t1[EARLY_TS ? 32 : 1];
+        uint32_t t0[DUAL ? 32 : 1], t1[DUAL ? 32 : 1];
         tmem_ld32(tS, x0);
         tmem_ld32(tS + 32, x1);
-        if constexpr (EARLY_TS) {
+        // (the tangent scores together with the scores, beside a bias when it has been added)
+        constexpr bool TS_LATER = DUAL && MK == 2;
+        if constexpr (DUAL && !TS_LATER) {
           tmem_ld32(tTS, t0);
           tmem_ld32(tTS + 32, t1);
         }
         tmem_wait_ld();
-        if constexpr (EARLY_TS || !DUAL) {
+        if constexpr (!TS_LATER) {
           tc_fence_before();
           mbar_arrive(s_free + X);
         }
@@ -654,6 +662,14 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
           }
           mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
         }
+        if constexpr (MK == 1) fetch_mask(n0 + BN);
+        if constexpr (TS_LATER) {
+          tmem_ld32(tTS, t0);
+          tmem_ld32(tTS + 32, t1);
+          tmem_wait_ld();
+          tc_fence_before();
+          mbar_arrive(s_free + X);
+        }
         // Lazy running max: keep the old reference while the new maximum is at most 2^8 above it (kExactRowMax: never).
         const bool grow = mx > m_used + slack;
         float alpha = 1.f;
@@ -704,16 +720,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           uint32_t* xs = hh ? x1 : x0;
-          uint32_t tt[(DUAL && !EARLY_TS) ? 32 : 1];
-          if constexpr (DUAL && !EARLY_TS) {
-            tmem_ld32(tTS + 32 * hh, tt);
-            tmem_wait_ld();
-            if (hh == 1) {
-              tc_fence_before();
-              mbar_arrive(s_free + X);  // both score accumulators are in registers now
-            }
-          }
-          const uint32_t* ts = EARLY_TS ? (hh ? t1 : t0) : tt;
+          const uint32_t* ts = hh ? t1 : t0;
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
             float2 e;
@@ -731,6 +738,8 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
             }
           }
         }
+
+        if constexpr (MK == 2) fetch_mask(n0 + BN);
         l_run = l_run * alpha + (ls2.x + ls2.y);
         if constexpr (DUAL) mu_run = mu_run * alpha + (ms2.x + ms2.y);
         // The P / W tiles are single-buffered: the previous tile's output MMAs must have read them.
