@@ -18,8 +18,8 @@
 // buffer to the output type at the end.  The order of those additions varies from run to run, so dQ is reproducible to
 // rounding, not bitwise.  (With a bias and through tO a key tile's share is stored instead, see kDqParts.)
 //
-// Measured on a B200, cycles of a sub-tile with every SM at work (37 heads, L2048): through O 1960, through tO 2760-2800, both
-// 3500 (4030 with one ring of two stages for all four streamed tiles); the tensor pipe's own time is 1024, 1860 and 2050.  What
+// Measured on a B200, cycles of a sub-tile with every SM at work (37 heads, L2048): through O 1830, through tO 2730, both 3410
+// (4030 with one ring of two stages for all four streamed tiles); the tensor pipe's own time is 1024, 1860 and 2050.  What
 // bounds it: the elementwise threads are busy four fifths of the time (two warps for a scheduler, so their latencies show), beside
 // a shared-memory port that MMA operands, statistics and result tiles fill to nine tenths.
 //
@@ -278,13 +278,13 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 
   // Registers: the elementwise threads hold four 32-column accumulator slices; everybody else needs few.
   // (setmaxnreg.inc draws on what setmaxnreg.dec of the same CTA has released and blocks until it is there: 256
-  // threads x 48 registers up equals 256 threads x 48 registers down from the 128 the kernel is launched with.  At 72 the
-  // read-back threads, which hold 64 of a row, and the issuers spilled: through tO at B4 H16 L2048 causal 204 us against 193.)
+  // threads x 48 registers up equal 128 x 64 and 128 x 32 down from the 128 the kernel is launched with.  The read-back threads
+  // hold 64 of a row and spilled at 72 and at 80: through tO at B4 H16 L2048 causal 204 and 195 us against 192.)
   // (It stands in the branches of the roles: ptxas holds code behind a join of the two to the smaller number.)
   // Phase counters kept alike by all roles: g counts the sub-tiles of this CTA (ring stage g % STAGES, dQ buffer
   // g & 1; s_full, s_free complete once per sub-tile, p_full and out_free of buffer g & 1 every other one), kact the items that have sub-tiles.
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer + per-query statistics
     if (lane == 0) {
@@ -379,7 +379,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       ++kact;
     }
   } else {
-    // The issuing warps stay converged and let one lane issue (mbar_wait_warp).
+    // The issuing warps stay converged and let one lane issue (mbar_wait_warp), at most twelve instructions in a row: the operands
+    // of sixteen are computed ahead, and those uniform registers spill.
     {
       constexpr uint32_t idesc_sc = make_idesc(Fmt<T>::kIdesc, OWN, BL, 0, 0);       // 128 x 64 scores
       constexpr uint32_t idesc_sc2 = make_idesc(Fmt<T>::kIdesc, OWN, 2 * BL, 0, 0);  // 128 x 128: [S | tS]
@@ -458,9 +459,9 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
               }
               tc_fence_after();
               if (elect_one()) from_g();
-            } else if (elect_one()) {
-              from_q();
-              from_g();
+            } else {
+              if (elect_one()) from_q();
+              if (elect_one()) from_g();
             }
           }
           if (!ok) break;
@@ -498,10 +499,12 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             const uint32_t lg = C::TWO_RINGS ? gring_mn + (g % GSTAGES) * GSTAGE16 : lp;
             const uint32_t acc = s > 0;
             if (elect_one()) {
-            outer(C::COL_DK, C::OUT_GS, lp + C::SLOT_Q * LOOP16, acc);  // dK += gS^T Q
+            outer(C::COL_DK, C::OUT_GS, lp + C::SLOT_Q * LOOP16, acc);                        // dK += gS^T Q
+            if constexpr (HAS_GT) outer(C::COL_DK, C::OUT_GT, lp + C::SLOT_TQ * LOOP16, 1);  // dK += gtS^T tQ
+            if constexpr (C::TWO_RINGS) tc_commit(loop_empty + st);
+            }
+            if (elect_one()) {
             if constexpr (HAS_GT) {
-              outer(C::COL_DK, C::OUT_GT, lp + C::SLOT_TQ * LOOP16, 1);  // dK += gtS^T tQ
-              if constexpr (C::TWO_RINGS) tc_commit(loop_empty + st);
               outer_t(C::COL_DV, C::COL_AV, lg + C::SLOT_G * LOOP16, acc);  // dV += A^T G
               if constexpr (HAS_GO) outer_t(C::COL_DV, C::COL_P, lg + C::SLOT_GO * LOOP16, 1);  // dV += P^T gO
             } else {
@@ -545,6 +548,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             const uint32_t col = C::COL_DQ;
             if (elect_one()) {
             inner(col, C::OUT_GS, C::SLOT_K, true);                       // dQ = gS K
+            }
+            if (elect_one()) {
             if constexpr (HAS_GT) inner(col, C::OUT_GT, C::SLOT_TK, false);  // dQ += gtS tK
             tc_commit(dq_full);
             tc_commit(out_free + ob);
@@ -761,7 +766,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       ++kact;
     }
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
     // ------------------------------------------------------------------ dQ read-back
     const int quarter = warp & 3;
     const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + C::COL_DQ;
