@@ -188,6 +188,12 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
   const int n_items = n_own_tiles * BH;
   const int G = (int)gridDim.x, cta = (int)blockIdx.x;
   const int k_max = (n_items + G - 1) / G;
+  unsigned char* order = smem + C::TILE_BYTES + 256;  // behind the barriers
+  const bool sorted = a.mask.kind == JVPFA_MASK_KVLEN && a.B <= kMaxSortedBatch && n_items > G;
+  if (sorted) {
+    sort_batch(a.mask, a.B, order);
+    __syncthreads();
+  }
 
   // Item k of this CTA: ranked heaviest first (causal: the first key tile sees every query), dealt in serpentine order.
   auto get_item = [&](int k, FItem& it) -> bool {
@@ -197,6 +203,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
     it.bh = w - rank * BH;
     it.b = it.bh / a.H;
     it.h = it.bh - it.b * a.H;
+    if (sorted) it.b = order[it.b], it.bh = it.b * a.H + it.h;
     int n_valid = L;
     if (a.mask.kind == JVPFA_MASK_KVLEN) {
       const int n = a.mask.kv_len[it.b];
@@ -379,7 +386,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       ++kact;
     }
   } else {
-    // The issuing warps stay converged and let one lane issue (mbar_wait_warp), at most twelve instructions in a row: the operands
+    // The issuing warps stay converged and let one lane issue (mbar_wait_warp), at most eight instructions in a row: the operands
     // of sixteen are computed ahead, and those uniform registers spill.
     {
       constexpr uint32_t idesc_sc = make_idesc(Fmt<T>::kIdesc, OWN, BL, 0, 0);       // 128 x 64 scores

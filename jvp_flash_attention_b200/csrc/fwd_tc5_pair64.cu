@@ -52,7 +52,8 @@ struct FwdPairCfg {
   static constexpr int OFF_KV = NQ * N_QT * Q_BYTES;
   static constexpr int OFF_P = OFF_KV + STAGES * STAGE_BYTES;
   static constexpr int TILE_BYTES = OFF_P + NQ * N_P * P_BYTES;
-  static constexpr int SMEM_BYTES = TILE_BYTES + 256 + 1024;
+  static constexpr int OFF_ORDER = TILE_BYTES + 256;  // behind the barriers
+  static constexpr int SMEM_BYTES = OFF_ORDER + kMaxSortedBatch + 1024;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
   static constexpr int COL_S = 0;
   static constexpr int COL_TS = 64;
@@ -158,6 +159,12 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
   const int n_items = n_pairs * BH;
   const int G = (int)gridDim.x, cta = (int)blockIdx.x;
   const int k_max = (n_items + G - 1) / G;
+  unsigned char* order = smem + C::OFF_ORDER;
+  const bool sorted = a.mask.kind == JVPFA_MASK_KVLEN && a.B <= kMaxSortedBatch && n_items > G;
+  if (sorted) {
+    sort_batch(a.mask, a.B, order);
+    __syncthreads();
+  }
 
   // Item k of this CTA: items are ranked heaviest first (for causal masks the last pair is the longest) and
   // dealt in serpentine order.
@@ -176,6 +183,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
     it.m0 = pair * (2 * BM);
     it.b = it.bh / a.H;
     it.h = it.bh - it.b * a.H;
+    if (sorted) it.b = order[it.b], it.bh = it.b * a.H + it.h;
     it.n_valid = L;
     if (a.mask.kind == JVPFA_MASK_KVLEN) {
       const int n = a.mask.kv_len[it.b];

@@ -310,6 +310,24 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
+// ---- Key padding: the batch entries, longest first ----------------------------------------
+// Persistent kernels deal their items in one order to all CTAs; with the entries' lengths mixed some CTAs got the long ones twice
+// (B8 H12 L1024, lengths in [L/2, L], 148 CTAs: 39-48 key tiles in the forward against 32-40 for the longest first, mean 28-34;
+// in the backward 6 key tiles of 128 against 5).  Up to this many entries, and where a CTA has more than one item.
+constexpr int kMaxSortedBatch = 64;
+// By all threads of the CTA, before they meet: order[r] = the r-th longest entry.
+__device__ __forceinline__ void sort_batch(const jvpfa_mask& m, int B, unsigned char* order) {
+  if ((int)threadIdx.x < B) {
+    const int mine = m.kv_len[threadIdx.x];
+    int r = 0;
+    for (int x = 0; x < B; ++x) {
+      const int n = m.kv_len[x];
+      r += n > mine || (n == mine && x < (int)threadIdx.x);
+    }
+    order[r] = (unsigned char)threadIdx.x;
+  }
+}
+
 // ---- TMA -----------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y,
                                             int z, int w) {
