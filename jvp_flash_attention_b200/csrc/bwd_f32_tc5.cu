@@ -695,23 +695,29 @@ bwd_f32_dkdv_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap 
     for (int x = 0; x < C::W_OUT; ++x) acc_k[x] = acc_v[x] = 0.f;
     int piece = 0;
     bool alive = true;
-    for (int t = 0; alive && t < n_tiles; ++t) {
-      const int i0 = i_begin + t * BN + 32 * w;  // this thread's first query
-      const uint32_t tS = tmem + lane_off + (t & 1) * C::SC + 32 * w, tLO = tmem + lane_off + C::COL_LO + 32 * w;
-      uint32_t live = j < n_valid ? first_columns(L - i0) : 0u;  // queries that attend this key, a bit each
-      if (causal) live &= ~first_columns(j - i0);
-      float bias[MK == 2 ? 32 : 1];
-      if constexpr (MK == 1) {  // (neighbouring lanes read neighbouring keys)
+    // What the mask holds for a tile's queries (neighbouring lanes read neighbouring keys), requested a tile ahead as in the forward.
+    float bias[MK == 2 ? 32 : 1];
+    uint32_t next_live = 0u;
+    auto fetch_mask = [&](int t) {
+      const int i0 = i_begin + min(t, n_tiles - 1) * BN + 32 * w;
+      next_live = j < n_valid ? first_columns(L - i0) : 0u;  // queries that attend this key, a bit each
+      if (causal) next_live &= ~first_columns(j - i0);
+      if constexpr (MK == 1) {
         uint32_t r = 0u;
 #pragma unroll 8
         for (int c = 0; c < 32; ++c)
           r |= (ldg_nc_u8(reinterpret_cast<const unsigned char*>(mv.base) + (long long)min(i0 + c, L - 1) * mv.si + jo) != 0u ? 1u : 0u) << c;
-        live &= r;
+        next_live &= r;
       }
       if constexpr (MK == 2) {
 #pragma unroll
         for (int c = 0; c < 32; ++c) bias[c] = mv.bias(min(i0 + c, L - 1), min(j, L - 1));
       }
+    };
+    if (n_tiles > 0) fetch_mask(0);
+    for (int t = 0; alive && t < n_tiles; ++t) {
+      const uint32_t tS = tmem + lane_off + (t & 1) * C::SC + 32 * w, tLO = tmem + lane_off + C::COL_LO + 32 * w;
+      const uint32_t live = next_live;
       if (!mbar_wait(stat_full + (t & 1), (t >> 1) & 1, ab, kAbortBwdLoopFull) ||
           !mbar_wait(s_full + (t & 1), (t >> 1) & 1, ab, kAbortBwdSFull)) {
         alive = false;
@@ -752,6 +758,7 @@ bwd_f32_dkdv_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap 
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(p_full + (t & 1));
+      fetch_mask(t + 1);
 #pragma unroll
       for (int pc = 0; pc < C::PIECES; ++pc) {
         if (!mbar_wait(acc_full, piece & 1, ab, kAbortBwdDone)) {

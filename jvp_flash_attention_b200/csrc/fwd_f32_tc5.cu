@@ -362,15 +362,21 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
     float m_used = -INFINITY, l_run = 0.f, mu_run = 0.f;
     int piece = 0;
     bool alive = true;
+    // What the mask holds for a tile's keys.  Requested a tile ahead, once this one's probabilities are written: it arrives under
+    // the output products.  (Behind the last tile that tile's again: under a condition this one's would have to be kept.)
+    float bias[MK == 2 ? 32 : 1];
+    uint32_t next_live = 0u;
+    auto fetch_mask = [&](int t) {
+      const int n0 = min(t, n_tiles - 1) * BN + 32 * w;
+      int hi = min(32, n_valid - n0);  // live keys of this row among the 32: a bit each
+      if (causal) hi = min(hi, i - n0 + 1);
+      next_live = rm.fetch(n0, first_columns(hi), bias);
+    };
+    if (n_tiles > 0) fetch_mask(0);
     for (int t = 0; alive && t < n_tiles; ++t) {
-      const int n0 = t * BN + 32 * w;  // this thread's first key
       const uint32_t tS = tmem + lane_off + (t & 1) * C::SC + 32 * w, tTS = tS + 64;
       const uint32_t tLO = tmem + lane_off + C::COL_LO + 32 * w;
-      // live keys of this row among the 32: a bit each
-      int hi = min(32, n_valid - n0);
-      if (causal) hi = min(hi, i - n0 + 1);
-      float bias[MK == 2 ? 32 : 1];
-      const uint32_t live = rm.fetch(n0, first_columns(hi), bias);
+      const uint32_t live = next_live;
       if (!mbar_wait(s_full + (t & 1), (t >> 1) & 1, ab, kAbortSFull)) {
         alive = false;
         break;
@@ -443,6 +449,7 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(p_full + (t & 1));
+      fetch_mask(t + 1);
       // The tile's outputs: read back, rescaled and added with rounding.
 #pragma unroll
       for (int pc = 0; pc < C::PIECES; ++pc) {
