@@ -312,13 +312,22 @@ bwd_f32_dq_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap ma
 #pragma unroll
     for (int x = 0; x < C::W_OUT; ++x) acc[x] = 0.f;
     bool alive = true;
-    for (int t = 0; t < n_tiles; ++t) {
-      const int n0 = t * BN + 32 * w;  // this thread's first key
-      const uint32_t tS = tmem + lane_off + (t % NBUF) * C::SC + 32 * w;
+    // What the mask holds for a tile's keys, requested a tile ahead as in the forward.  (D = 128: at the tile's own beginning, where
+    // the scores of one buffer are still being formed; 144 us through tO at B2 H8 L1024 with a bias, 158 ahead.)
+    constexpr bool AHEAD = D < 128;
+    float bias[MK == 2 ? 32 : 1];
+    uint32_t live = 0u;
+    auto fetch_mask = [&](int t) -> uint32_t {
+      const int n0 = min(t, n_tiles - 1) * BN + 32 * w;
       int hi = min(32, n_valid - n0);  // live keys of this row among the 32: a bit each
       if (causal) hi = min(hi, i - n0 + 1);
-      float bias[MK == 2 ? 32 : 1];
-      const uint32_t live = rm.fetch(n0, first_columns(hi), bias);
+      return rm.fetch(n0, first_columns(hi), bias);
+    };
+    uint32_t next_live = 0u;
+    if (AHEAD && n_tiles > 0) next_live = fetch_mask(0);
+    for (int t = 0; t < n_tiles; ++t) {
+      const uint32_t tS = tmem + lane_off + (t % NBUF) * C::SC + 32 * w;
+      live = AHEAD ? next_live : fetch_mask(t);
       if (!mbar_wait(s_full + t % NBUF, (t / NBUF) & 1, ab, kAbortBwdSFull)) {
         alive = false;
         break;
@@ -356,6 +365,7 @@ bwd_f32_dq_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap ma
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(p_full + t % NBUF);
+      if constexpr (AHEAD) next_live = fetch_mask(t + 1);
       if (!mbar_wait(acc_full, t & 1, ab, kAbortBwdDone)) {
         alive = false;
         break;
