@@ -136,7 +136,7 @@ __device__ __forceinline__ void transpose_bytes(uint32_t a, uint32_t b, uint32_t
   w[2] = __byte_perm(ab2, cd2, 0x5410), w[3] = __byte_perm(ab2, cd2, 0x7632);
 }
 
-__global__ void __launch_bounds__(256) mask_pack_kernel(const jvpfa_mask m, int n_h, int n_rows, int L, int n_qt, int n_words,
+__global__ void __launch_bounds__(256, 4) mask_pack_kernel(const jvpfa_mask m, int n_h, int n_rows, int L, int n_qt, int n_words,
                                                         unsigned char* tile_live, int32_t* head_live,
                                                         unsigned long long* tile_live_t, int n_kt128, int n_words_t,
                                                         uint32_t* bits, uint32_t* bits_t) {
@@ -154,17 +154,24 @@ __global__ void __launch_bounds__(256) mask_pack_kernel(const jvpfa_mask m, int 
   const unsigned char* p0 = base + (long long)row0 * rs + (long long)col * ks;
   uint32_t x[8];  // byte i of x[j]: row 4j + i, a bit per column
   if (vec) {
-    uint2 v[32];
+    // Sixteen rows in flight at a time, so that four CTAs fit an SM: one's loads run under another's arithmetic and stores
+    // (B2 H12 L2048 from DRAM: 41 us with all 32 rows and two or three CTAs, 36 so).  Volatile loads: the compiler would move the
+    // second half's before the first's arithmetic.
 #pragma unroll
-    for (int r = 0; r < 32; ++r) {
-      v[r] = make_uint2(0u, 0u);
-      if (row0 + r < n_rows) v[r] = __ldg(reinterpret_cast<const uint2*>(p0 + (long long)r * rs));
-    }
+    for (int half = 0; half < 2; ++half) {
+      uint2 v[16];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      x[j] = 0u;
+      for (int r = 0; r < 16; ++r) {
+        v[r] = make_uint2(0u, 0u);
+        if (row0 + 16 * half + r < n_rows)
+          asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(v[r].x), "=r"(v[r].y) : "l"(p0 + (long long)(16 * half + r) * rs));
+      }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) x[j] |= (nonzero_bits(v[4 * j + i].x) | nonzero_bits(v[4 * j + i].y) << 4) << (8 * i);
+      for (int j = 0; j < 4; ++j) {
+        x[4 * half + j] = 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[4 * half + j] |= (nonzero_bits(v[4 * j + i].x) | nonzero_bits(v[4 * j + i].y) << 4) << (8 * i);
+      }
     }
   } else {
     const int n = min(8, L - col);  // <= 0: beyond the end
