@@ -560,9 +560,10 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         mrow = reinterpret_cast<const unsigned char*>(a.mask.ptr) +
                ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] +
                 (long long)min(i, L - 1) * a.mask.stride[2]) * MESZ;
-      // The mask's piece of a tile.  Where the next tile is known it is requested when the registers of this one's are free
-      // again: behind its own tile's beginning the scores are there already, and the loads would be waited for.  (Without a
-      // condition, zeros beyond the last tile: else this tile's piece would have to be kept.)
+      // The mask's piece of a tile.  Where the next tile is known that of a boolean mask is requested as soon as this one's has been
+      // used: at its own tile's beginning the scores are there already, and the loads would be waited for.  (Without a condition,
+      // zeros beyond the last tile: else this tile's piece would have to be kept.)  A bias is requested at its own tile's
+      // beginning: a tile ahead its 32 registers are in the way (forward with tangents B2 H12 L1024 50 -> 52 us, B8 H6 L1056 3 % more).
       uint32_t mw[MW];
       uint2 next_keys = make_uint2(~0u, ~0u);
       auto fetch_mask = [&](int n0) {
@@ -583,14 +584,14 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
           }
         }
       };
-      constexpr bool AHEAD = MK == 1 || MK == 2;
+      constexpr bool AHEAD = MK == 1;
       if constexpr (AHEAD) fetch_mask(0);
       TileUse<MK> use(it);
       bool first = true;  // the item's first tile used by this query tile
       for (int j = 0; j < it.n_load; ++j) {
         if (!(use(j) & (1 << X))) continue;
         const int n0 = j * BN;
-        if constexpr (BOOLM && !AHEAD) fetch_mask(n0);
+        if constexpr (MK != 0 && !AHEAD) fetch_mask(n0);
         uint2 keys = next_keys;  // BOOLM: bit c of (x, y) = the mask lets this row attend key n0 + c
         if (!mbar_wait(s_full + X, t & 1, ab, kAbortSFull)) {
           alive = false;
@@ -598,10 +599,10 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         }
         tc_fence_after();
         uint32_t x0[32], x1[32];
-        uint32_t t0[DUAL ? 32 : 1], t1[DUAL ? 32 : 1];
+        uint32_t t0[DUAL && MK != 2 ? 32 : 1], t1[DUAL && MK != 2 ? 32 : 1];
         tmem_ld32(tS, x0);
         tmem_ld32(tS + 32, x1);
-        // (the tangent scores together with the scores, beside a bias when it has been added)
+        // (the tangent scores together with the scores; beside a bias half a tile at a time, when it has been added)
         constexpr bool TS_LATER = DUAL && MK == 2;
         if constexpr (DUAL && !TS_LATER) {
           tmem_ld32(tTS, t0);
@@ -671,13 +672,6 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
           mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
         }
         if constexpr (MK == 1) fetch_mask(n0 + BN);
-        if constexpr (TS_LATER) {
-          tmem_ld32(tTS, t0);
-          tmem_ld32(tTS + 32, t1);
-          tmem_wait_ld();
-          tc_fence_before();
-          mbar_arrive(s_free + X);
-        }
         // Lazy running max: keep the old reference while the new maximum is at most 2^8 above it (kExactRowMax: never).
         const bool grow = mx > m_used + slack;
         float alpha = 1.f;
@@ -728,7 +722,16 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           uint32_t* xs = hh ? x1 : x0;
-          const uint32_t* ts = hh ? t1 : t0;
+          uint32_t tt[TS_LATER ? 32 : 1];
+          if constexpr (TS_LATER) {
+            tmem_ld32(tTS + 32 * hh, tt);
+            tmem_wait_ld();
+            if (hh == 1) {
+              tc_fence_before();
+              mbar_arrive(s_free + X);  // both score accumulators are in registers now
+            }
+          }
+          const uint32_t* ts = TS_LATER ? tt : hh ? t1 : t0;
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
             float2 e;
@@ -747,7 +750,6 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
           }
         }
 
-        if constexpr (MK == 2) fetch_mask(n0 + BN);
         l_run = l_run * alpha + (ls2.x + ls2.y);
         if constexpr (DUAL) mu_run = mu_run * alpha + (ms2.x + ms2.y);
         // The P / W tiles are single-buffered: the previous tile's output MMAs must have read them.
