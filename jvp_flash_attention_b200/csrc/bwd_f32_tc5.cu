@@ -885,6 +885,7 @@ int launch_bwd_f32_tc5(const jvpfa_bwd_args& a, cudaStream_t stream) {
   s.dst = static_cast<__nv_bfloat16*>(a.workspace);
   s.plane = (long long)a.B * a.H * a.L * a.D;
   s.H = a.H, s.L = a.L, s.D = a.D;
+  if (a.mask.kind == JVPFA_MASK_KVLEN) s.kv_len = a.mask.kv_len, s.padded = 1u << kDqSlotK | 1u << kDqSlotV;
   s.set(kDqSlotQ, a.q, a.in_stride), s.set(kDqSlotK, a.k, a.in_stride), s.set(kDqSlotV, a.v, a.in_stride);
   if (a.gto) {
     s.set(kDqSlotA, a.tq, a.in_stride), s.set(kDqSlotB, a.gto, nullptr);

@@ -22,6 +22,10 @@ struct SplitArgs {
   __nv_bfloat16* dst;             // [slot][part][B*H][L][D]
   long long plane;                // B*H*L*D
   int H, L, D;
+  // Key padding: what `padded` (a bit per slot) holds of keys that no query attends is written as zeros.  A tile of 64 keys goes
+  // into the products whole, and an Inf or a NaN there would reach every row through its probability of 0.
+  const int32_t* kv_len;
+  unsigned padded;
   void set(int slot, const void* p, const int64_t* in_stride) {  // in_stride all zero or null: row-major
     src[slot] = static_cast<const float*>(p);
     const bool strided = in_stride && (in_stride[0] | in_stride[1] | in_stride[2]) != 0;

@@ -548,9 +548,12 @@ __global__ void __launch_bounds__(256) split3_kernel(const SplitArgs s) {
   const int col = (int)(e - row * s.D);
   const long long bh = row / s.L;
   const int i = (int)(row - bh * s.L);
-  const float4* src = reinterpret_cast<const float4*>(s.src[slot] + (bh / s.H) * s.st[slot][0] + (bh % s.H) * s.st[slot][1] +
-                                                      (long long)i * s.st[slot][2] + col);
-  const float4 x0 = __ldg(src), x1 = __ldg(src + 1);
+  float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
+  if (s.kv_len == nullptr || !((s.padded >> slot) & 1u) || i < s.kv_len[bh / s.H]) {
+    const float4* src = reinterpret_cast<const float4*>(s.src[slot] + (bh / s.H) * s.st[slot][0] + (bh % s.H) * s.st[slot][1] +
+                                                        (long long)i * s.st[slot][2] + col);
+    x0 = __ldg(src), x1 = __ldg(src + 1);
+  }
   const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
   uint32_t r[3][4];
 #pragma unroll
@@ -633,6 +636,10 @@ int launch_fwd_f32_tc5(const jvpfa_fwd_args& a, cudaStream_t stream) {
   s.dst = static_cast<__nv_bfloat16*>(a.workspace);
   s.plane = (long long)a.B * a.H * a.L * a.D;
   s.H = a.H, s.L = a.L, s.D = a.D;
+  if (a.mask.kind == JVPFA_MASK_KVLEN) {
+    s.kv_len = a.mask.kv_len;
+    s.padded = 1u << kSlotK | 1u << kSlotV | 1u << kSlotTK | 1u << kSlotTV;
+  }
   const void* src[kF32MaxSlots] = {a.q, a.k, a.v, a.tq, a.tk, a.tv};
   for (int n = 0; n < slots; ++n) s.set(n, src[n], a.in_stride);
   CUtensorMap map;

@@ -215,6 +215,37 @@ def test_what_is_asked_of_a_call_decides_the_kernels(D, L, kind):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("rest", [math.nan, math.inf])
+def test_what_padded_keys_hold_does_not_matter(D, rest):
+    """Lengths that end inside a 64-key tile; K, V and their tangents hold NaN or Inf from there on: all results are what they are
+    with zeros there."""
+    from jvp_flash_attention_b200 import jvp_attention as ja
+
+    B, H, L = 4, 16, 512
+    lens = torch.tensor([512, 96, 161, 352])
+    live = torch.arange(L)[None] < lens[:, None]
+    m = live[:, None, None].to(DEV)
+    g = torch.Generator().manual_seed(D)
+    q, k, v, tq, tk, tv, go = (torch.randn(B, H, L, D, generator=g).to(DEV) for _ in range(7))
+    u = torch.randn(B, H, L, D, generator=g).to(DEV)
+    keys = live[:, None, :, None].to(DEV)
+
+    def run(fill):
+        kk, vv, tkk, tvv = (x.masked_fill(~keys, fill) for x in (k, v, tk, tv))
+        a = [x.clone().requires_grad_() for x in (q, kk, vv)]
+        o = ja.attention(*a, attn_mask=m)
+        o_grads = torch.autograd.grad(o, a, go, create_graph=False)
+        dual = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, attn_mask=m), (q, kk, vv), (tq, tkk, tvv))
+        along_q = q.clone().requires_grad_()
+        (dq,) = torch.autograd.grad(ja.attention(along_q, kk, vv, attn_mask=m), along_q, go, create_graph=True)
+        return o, *o_grads, *dual, dq, torch.autograd.grad(dq, along_q, u)[0]
+
+    for n, (x, y) in enumerate(zip(run(rest), run(0.0))):
+        assert torch.isfinite(x).all() and torch.equal(x, y), n
+
+
 def _workspace(B, H, L, D, tangents=0, impl=_lib.IMPL_AUTO, dtype=_lib.FP32, **fields):
     class At(int):
         shape = (B, H, L, D)
