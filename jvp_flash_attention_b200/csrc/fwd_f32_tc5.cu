@@ -405,9 +405,10 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
         break;
       }
       mx = fmaxf(mx, red[(w ^ 1) * BM + row]);
-      // Lazy reference: kept while the new maximum is at most 2^8 above it (P is fp32 in three parts: nothing is lost).
+      // The running maximum itself is the reference: P is at most 1, so nothing overflows before the result does.  (A reference up
+      // to 2^8 below it, as in the 16-bit kernels, saves nothing here: alpha goes into the additions below in any case.)
       float alpha = 1.f;
-      if (mx > m_used + 8.f) {
+      if (mx > m_used) {
         alpha = fast_exp2(m_used - mx);
         m_used = mx;
       }

@@ -246,6 +246,21 @@ def test_what_padded_keys_hold_does_not_matter(D, rest):
         assert torch.isfinite(x).all() and torch.equal(x, y), n
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_forward_up_to_the_end_of_the_range(D):
+    """All of V, and of its tangent, 3e36, and a key of the second tile 2^7.8 times as probable as the others: sums of a tile's P V
+    stay below 64 * 3e36 < FLT_MAX with probabilities of at most 1.  O and tO are 3e36, to 2^-20 for 512 terms."""
+    from jvp_flash_attention_b200 import jvp_attention as ja
+
+    q, k = torch.zeros(2, 32, 512, D, device=DEV), torch.zeros(2, 32, 512, D, device=DEV)
+    v = torch.full((2, 32, 512, D), 3e36, device=DEV)
+    q[..., 0], k[:, :, 100, 0] = 1.0, 5.4 * D**0.5
+    o, to = torch.func.jvp(ja.JVPAttn.fwd_dual, (q, k, v), (torch.zeros_like(q), torch.zeros_like(k), v))
+    for x in (o, to, ja.attention(q, k, v)):
+        assert ((x.double() - 3e36).abs().max() / 3e36).item() <= 2**-20
+
+
 def _workspace(B, H, L, D, tangents=0, impl=_lib.IMPL_AUTO, dtype=_lib.FP32, **fields):
     class At(int):
         shape = (B, H, L, D)
