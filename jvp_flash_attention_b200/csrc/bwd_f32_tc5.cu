@@ -17,7 +17,7 @@
 //
 // Bound by the tensor pipe as the forward.  Measured on a B200, B2 H8 L1024, us, the register-tiled kernels / here with the
 // splitting: dQ through O D128 353 / 103, D64 197 / 58, D32 125 / 44; dQ through tO 566 / 142, 298 / 73, 144 / 52; all three
-// gradients through O 853 / 255, 468 / 126, 282 / 101.
+// gradients through O 853 / 248, 468 / 125, 282 / 102.
 #include "f32_tc5_common.cuh"
 
 namespace jvpfa {
@@ -347,8 +347,7 @@ bwd_f32_dq_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap ma
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int n = 2 * c + e;
-            float v = __uint_as_float(x[n]) * scale_log2;
-            if constexpr (MK == 2) v += bias[16 * s + n] * kLog2e;
+            const float v = f32_score<MK>(__uint_as_float(x[n]), scale_log2, MK == 2 ? bias[16 * s + n] : 0.f);
             const float p = fast_exp2(v - lse);
             float u = __uint_as_float(y[n]);
             if constexpr (GT) {
@@ -412,6 +411,10 @@ bwd_f32_dq_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap ma
 // Shared memory: the parts of K and V (D = 128: the lo part of K in TMEM), and the ring: Q and gO for the scores, gO and Q once more
 // for dV and dK.  TMEM as in the forward: two score buffers [S | X = V gO^T], the parts of P over S and of gS over X, their lo
 // parts beside them, one accumulator of 128 columns ([dV | dK], D = 128: dV, then dK).
+// S has the forward's bits: its instructions come in the forward's order, for which all of a tile's Q stays in the ring until S is
+// formed.  With the small products ordered by the parts of Q, as those of X are by the parts of gO, P was off by what S had lost to
+// truncation in another way: dV of rows with one key 1.4e-6 from 64 bits at |S| of 50 (D = 128; 0 now), of dense rows 3.2e-6 (1.3e-6
+// now, 2.3e-6 on the register-tiled kernels).  us of this launch, B2 H8 L1024, so / now: D128 155 / 141, D64 72 / 71, D32 61 / 64.
 template <int D_>
 struct DkvF32Cfg {
   static constexpr int D = D_;
@@ -429,7 +432,7 @@ struct DkvF32Cfg {
   static constexpr int BUDGET = 227 * 1024 - 1024 - STAT_BYTES - 512;
   static constexpr int FIT = (BUDGET - OFF_RING) / TILE;
   static constexpr int STAGES = FIT > 16 ? 16 : FIT;
-  static_assert(STAGES >= 4, "ring");
+  static_assert(STAGES >= 3 * NSL + 2 && (STAGES & (STAGES - 1)) == 0, "a tile's Q stays until S is formed");
   static constexpr int OFF_STAT = OFF_RING + STAGES * TILE;
   static constexpr int OFF_BAR = OFF_STAT + STAT_BYTES;
   static constexpr int SMEM_NEEDED = OFF_BAR + 512 + 1024;
@@ -540,18 +543,24 @@ bwd_f32_dkdv_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap 
         int st = 0;
         uint32_t ph = 1;
         bool ok = true;
+        auto unit = [&](int t, int slot, int p, int s) {
+          if (!ok || !(ok = mbar_wait_backoff<64>(empty + st, ph, ab, kAbortBwdLoopEmpty))) return;
+          mbar_expect_tx(full + st, C::TILE);
+          load(smem + C::OFF_RING + st * C::TILE, full + st, slot, p, 64 * s, i_begin + t * BN);
+          if (++st == STAGES) st = 0, ph ^= 1;
+        };
         auto units = [&](int t, int slot) {  // one part and slice after another, the lo parts first
           for (int p = 2; p >= 0; --p)
-            for (int s = 0; s < NSL; ++s) {
-              if (!ok || !(ok = mbar_wait_backoff<64>(empty + st, ph, ab, kAbortBwdLoopEmpty))) return;
-              mbar_expect_tx(full + st, C::TILE);
-              load(smem + C::OFF_RING + st * C::TILE, full + st, slot, p, 64 * s, i_begin + t * BN);
-              if (++st == STAGES) st = 0, ph ^= 1;
-            }
+            for (int s = 0; s < NSL; ++s) unit(t, slot, p, s);
         };
-        units(0, kDqSlotQ), units(0, kDqSlotA);
+        auto scores = [&](int t) {
+          for (int s = 0; s < NSL; ++s)
+            for (int p = 0; p < 3; ++p) unit(t, kDqSlotQ, p, s);
+          units(t, kDqSlotA);
+        };
+        scores(0);
         for (int t = 0; ok && t < n_tiles; ++t) {
-          if (t + 1 < n_tiles) units(t + 1, kDqSlotQ), units(t + 1, kDqSlotA);
+          if (t + 1 < n_tiles) scores(t + 1);
           units(t, kDqSlotA), units(t, kDqSlotQ);
         }
       }
@@ -576,36 +585,72 @@ bwd_f32_dkdv_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap 
         auto next = [&]() {
           if (++st == STAGES) st = 0, ph ^= 1;
         };
+        auto stage = [&](int n) { return (st + n) & (STAGES - 1); };  // of the n-th unit from here
         auto scores = [&](int t) {
           const uint32_t sc = tmem + (t & 1) * C::SC;
+          // S = K Q^T in the forward's order: parts lo, mid, hi of K, and beside each the small parts of Q first.  Unit 3 s + p from
+          // here holds part p (hi, mid, lo) of slice s of Q; it is first used beside part 2 - p of K, and a slice's units are free
+          // after its last product.
 #pragma unroll
-          for (int side = 0; side < 2; ++side) {  // S = K Q^T, X = V gO^T
+          for (int p = 2; p >= 0; --p) {
 #pragma unroll
-            for (int p = 2; p >= 0; --p) {
+            for (int s = 0; s < NSL; ++s) {
+              if (!mbar_wait_warp(full + stage(3 * s + 2 - p), ph ^ (st + 3 * s + 2 - p >= STAGES), ab, kAbortBwdLoopFull)) {
+                ok = false;
+                return;
+              }
+              tc_fence_after();
+              if (elect_one()) {
 #pragma unroll
-              for (int s = 0; s < NSL; ++s) {
-                if (!acquire()) return;
-                const uint32_t bk = kDescLo | (ring16 + st * TILE16);
-                if (elect_one()) {
-                  const uint32_t col = sc + side * C::COL_X;
+                for (int pq = 2 - p; pq >= 0; --pq) {
+                  const uint32_t bk = kDescLo | (ring16 + stage(3 * s + pq) * TILE16);
 #pragma unroll
-                  for (int pa = 2 - p; pa >= 0; --pa) {  // small products first
-#pragma unroll
-                    for (int ks = 0; ks < KS; ++ks) {
-                      const uint32_t al = (side == 0 ? k_lo : v_lo) + (pa * NSL + s) * PART16 + ks * 2;
-                      if (C::KLO_TMEM && side == 0 && pa == 2)
-                        umma_ts_lo<true>(col, tmem + C::COL_KLO + s * 32 + ks * 8, bk + ks * 2, id64);
-                      else if (p == 2 && s == 0 && ks == 0)
-                        umma_ss_lo<false>(col, al, bk, id64);
+                  for (int ks = 0; ks < KS; ++ks) {
+                    const uint32_t al = k_lo + (p * NSL + s) * PART16 + ks * 2;
+                    const bool fresh = p == 2 && s == 0 && ks == 0;
+                    if (C::KLO_TMEM && p == 2) {
+                      if (fresh)
+                        umma_ts_lo<false>(sc, tmem + C::COL_KLO, bk, id64);
                       else
-                        umma_ss_lo<true>(col, al, bk + ks * 2, id64);
+                        umma_ts_lo<true>(sc, tmem + C::COL_KLO + s * 32 + ks * 8, bk + ks * 2, id64);
+                    } else if (fresh) {
+                      umma_ss_lo<false>(sc, al, bk, id64);
+                    } else {
+                      umma_ss_lo<true>(sc, al, bk + ks * 2, id64);
                     }
                   }
-                  tc_commit(empty + st);
-                  if (side == 1 && p == 0 && s == NSL - 1) tc_commit(s_full + (t & 1));
                 }
-                next();
+                if (p == 0) {
+#pragma unroll
+                  for (int x = 0; x < 3; ++x) tc_commit(empty + stage(3 * s + x));
+                }
               }
+            }
+          }
+          st += 3 * NSL;
+          if (st >= STAGES) st -= STAGES, ph ^= 1;
+          // X = V gO^T
+#pragma unroll
+          for (int p = 2; p >= 0; --p) {
+#pragma unroll
+            for (int s = 0; s < NSL; ++s) {
+              if (!acquire()) return;
+              const uint32_t bk = kDescLo | (ring16 + st * TILE16);
+              if (elect_one()) {
+#pragma unroll
+                for (int pa = 2 - p; pa >= 0; --pa) {  // small products first
+#pragma unroll
+                  for (int ks = 0; ks < KS; ++ks) {
+                    if (p == 2 && s == 0 && ks == 0)
+                      umma_ss_lo<false>(sc + C::COL_X, v_lo, bk, id64);
+                    else
+                      umma_ss_lo<true>(sc + C::COL_X, v_lo + (pa * NSL + s) * PART16 + ks * 2, bk + ks * 2, id64);
+                  }
+                }
+                tc_commit(empty + st);
+                if (p == 0 && s == NSL - 1) tc_commit(s_full + (t & 1));
+              }
+              next();
             }
           }
         };
@@ -749,8 +794,7 @@ bwd_f32_dkdv_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap 
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int n = 2 * c + e;
-            float v = __uint_as_float(x[n]) * scale_log2;
-            if constexpr (MK == 2) v += bias[16 * s + n] * kLog2e;
+            const float v = f32_score<MK>(__uint_as_float(x[n]), scale_log2, MK == 2 ? bias[16 * s + n] : 0.f);
             const bool ok = (live >> (16 * s + n)) & 1u;  // (nothing of a masked pair counts, whatever it is)
             p[e] = ok ? fast_exp2(v - (e ? q2.z : q2.x)) : 0.f;
             g[e] = ok ? p[e] * (__uint_as_float(y[n]) - (e ? q2.w : q2.y)) : 0.f;

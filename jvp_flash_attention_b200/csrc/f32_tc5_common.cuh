@@ -57,6 +57,15 @@ __device__ __forceinline__ void split3_pair(float a, float b, uint32_t& h, uint3
   l = pack_bf16(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
 }
 
+// A score in base-2 units, as every kernel rounds it: what the backward subtracts lse from is what the forward made lse of.  (A
+// product that goes unrounded into the subtraction, as the compiler would have it, is off by up to half a unit of the score: at
+// |S| of 50 the probability of a row's only key came out 1 + 1e-6.)
+template <int MK>
+__device__ __forceinline__ float f32_score(float s, float scale_log2, float bias) {
+  const float v = __fmul_rn(s, scale_log2);
+  return MK == 2 ? __fmaf_rn(bias, kLog2e, v) : v;
+}
+
 // What a thread reads of the mask: 32 neighbouring keys of its query row i at a time.
 // MK: 0 = none / causal / key padding; 1 = boolean mask (bits, or bytes of any strides); 2 = additive bias (any type and
 // strides).

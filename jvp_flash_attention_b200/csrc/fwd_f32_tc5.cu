@@ -389,8 +389,7 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
         tmem_wait_ld();
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
-          float v = __uint_as_float(x[c]) * scale_log2;
-          if constexpr (MK == 2) v += bias[c] * kLog2e;
+          float v = f32_score<MK>(__uint_as_float(x[c]), scale_log2, MK == 2 ? bias[c] : 0.f);
           if (!((live >> c) & 1u)) v = -INFINITY;
           x[c] = __float_as_uint(v);
           mx = fmaxf(mx, v);
