@@ -345,13 +345,14 @@ const char* jvpfa_last_cuda_error(void);
  * 0 = every bounded wait completed; otherwise the code of the first wait that gave up.  The
  * kernels then drained and exited early, the output rows of the affected CTAs (lse in the
  * forward; dq / dk / dv rows in the backward) hold NaN, and while the word stays non-zero every
- * later tcgen05 launch on the device writes NaN and returns at once.  clear != 0 resets the
- * word.  This call synchronises with the device (it copies the word): poll it where the caller
+ * later 16-bit tcgen05 launch on the device writes NaN and returns at once (an fp32 one does so only
+ * when the wait that gave up was of an fp32 launch).  clear != 0 resets the word.  This call synchronises with the device (it copies the word): poll it where the caller
  * synchronises anyway, not per launch.  A caller that never polls is still told: the thread that
  * gives up also writes the code to a host-visible mirror (pinned, mapped memory), and jvpfa_fwd,
  * jvpfa_bwd and jvpfa_bwd_noalloc look at that mirror (a host read, no synchronisation) before they
  * launch a tcgen05 kernel and return JVPFA_ERR_DEVICE_STATUS while it is non-zero, i.e. from the
- * first call after the failing kernel has run until jvpfa_device_status(.., 1) clears the word.
+ * first call after the failing kernel has run until jvpfa_device_status(.., 1) clears the word (fp32 calls
+ * of impl AUTO run on the register-tiled kernels meanwhile).
  * No upstream counterpart: Triton kernels have no such waits. */
 int jvpfa_device_status(int* status, int clear);
 

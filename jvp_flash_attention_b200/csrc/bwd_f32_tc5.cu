@@ -64,7 +64,7 @@ bwd_f32_dq_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap ma
   using C = DqF32Cfg<D_, GT_>;
   constexpr int D = C::D, BM = C::BM, BN = C::BN, STAGES = C::STAGES, NSL = C::NSL, KS = C::KS, NA = C::NA, NBUF = C::NBUF;
   constexpr bool GT = C::GT;
-  const bool dead_on_entry = *(volatile int*)status != 0;  // an earlier bounded wait gave up
+  const bool dead_on_entry = *(volatile int*)(status + kF32GaveUp) != 0;
 
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -391,7 +391,10 @@ bwd_f32_dq_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap ma
 
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag != 0) poison();
+  if (*abort_flag != 0) {
+    poison();
+    if (tid == 0) *(volatile int*)(status + kF32GaveUp) = *abort_flag;
+  }
   if (warp == 0) {
     if (*abort_flag != 0) {
       // Something gave up: give copies and MMAs that may still be in flight time to land before the TMEM
@@ -451,7 +454,7 @@ __global__ void __launch_bounds__(384, 1)
 bwd_f32_dkdv_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap map, const __nv_bfloat16* parts, int* status) {
   using C = DkvF32Cfg<D_>;
   constexpr int D = C::D, OWN = C::OWN, BN = C::BN, STAGES = C::STAGES, NSL = C::NSL, KS = C::KS;
-  const bool dead_on_entry = *(volatile int*)status != 0;  // an earlier bounded wait gave up
+  const bool dead_on_entry = *(volatile int*)(status + kF32GaveUp) != 0;
 
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -858,7 +861,10 @@ bwd_f32_dkdv_kernel(const jvpfa_bwd_args a, const __grid_constant__ CUtensorMap 
 
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag != 0) poison();
+  if (*abort_flag != 0) {
+    poison();
+    if (tid == 0) *(volatile int*)(status + kF32GaveUp) = *abort_flag;
+  }
   if (warp == 0) {
     if (*abort_flag != 0) {
       // Something gave up: give copies and MMAs that may still be in flight time to land before the TMEM

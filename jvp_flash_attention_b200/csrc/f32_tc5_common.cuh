@@ -16,6 +16,10 @@ namespace tc5 {
 
 constexpr int kF32MaxSlots = 6;
 
+// Beside the status word: a wait of an fp32 kernel gave up.  Only this ends a later one on entry: an fp32 call that is queued, or
+// replayed, behind a 16-bit launch that gave up is computed, as on the register-tiled kernels.
+constexpr int kF32GaveUp = 1;
+
 struct SplitArgs {
   const float* src[kF32MaxSlots];
   long long st[kF32MaxSlots][3];  // batch, head, row strides in elements

@@ -76,7 +76,7 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
   using C = FwdF32Cfg<D_, MODE>;
   constexpr int D = C::D, BM = C::BM, BN = C::BN, STAGES = C::STAGES, NSL = C::NSL, KS = C::KS;
   constexpr bool DUAL = C::DUAL, TKV = C::TKV;
-  const bool dead_on_entry = *(volatile int*)status != 0;  // an earlier bounded wait gave up
+  const bool dead_on_entry = *(volatile int*)(status + kF32GaveUp) != 0;
 
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -524,7 +524,10 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
 
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag != 0) poison();
+  if (*abort_flag != 0) {
+    poison();
+    if (tid == 0) *(volatile int*)(status + kF32GaveUp) = *abort_flag;
+  }
   if (warp == 0) {
     if (*abort_flag != 0) {
       // Something gave up: give copies and MMAs that may still be in flight time to land before the TMEM

@@ -7,7 +7,7 @@
 
 namespace jvpfa {
 
-// [0]: the status word.  [2], [3]: device address of its host-visible mirror (pinned, mapped host memory), written by
+// [0]: the status word.  [1]: kF32GaveUp.  [2], [3]: device address of its host-visible mirror (pinned, mapped host memory), written by
 // a thread that gives up a wait, so that the host can see a failure without synchronising.
 __device__ __align__(16) int g_tc5_status[4] = {0, 0, 0, 0};
 
@@ -178,8 +178,8 @@ int tc5_read_status(int* out, int clear) {
     return JVPFA_ERR_CUDA;
   }
   if (clear && v != 0) {
-    const int zero = 0;
-    e = cudaMemcpy(sl->dev, &zero, sizeof(int), cudaMemcpyHostToDevice);
+    const int zero[2] = {0, 0};
+    e = cudaMemcpy(sl->dev, zero, sizeof(zero), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
       set_last_cuda_error(e, "cudaMemcpy(status)");
       return JVPFA_ERR_CUDA;

@@ -288,6 +288,41 @@ def test_the_launch_that_owns_keys_forms_the_scores_of_the_forward(monkeypatch, 
     assert errors[_lib.IMPL_AUTO] <= max(1.2 * errors[_lib.IMPL_GENERIC], 2**-23), errors
 
 
+@pytest.mark.gpu
+def test_a_replayed_call_is_computed_behind_a_16_bit_launch_that_gave_up():
+    """The failure is made on the host, which sets the status word as a thread of a 16-bit kernel would."""
+    from jvp_flash_attention_b200 import jvp_attention as ja
+
+    g = torch.Generator().manual_seed(2)
+    q, k, v, go = (torch.randn(2, 16, 512, 64, generator=g).to(DEV) for _ in range(4))
+    a = [x.requires_grad_() for x in (q, k, v)]
+
+    def step():
+        o = ja.attention(*a)
+        return [x.detach() for x in (o, *torch.autograd.grad(o, a, go))]
+
+    side = torch.cuda.Stream()  # (the legacy stream's graph nodes cannot be captured)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        ref = step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step()
+    for code in (5, 0):
+        if code:
+            _lib.device_status_inject(code)
+        try:
+            for x in got:
+                x.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            for x, y in zip(got, ref):
+                assert torch.equal(x, y)
+        finally:
+            assert _lib.device_status(clear=True) == code
+
+
 def _workspace(B, H, L, D, tangents=0, impl=_lib.IMPL_AUTO, dtype=_lib.FP32, **fields):
     class At(int):
         shape = (B, H, L, D)
