@@ -484,8 +484,11 @@ def bwd(q, k, v, tq, tk, tv, go, gto, lse, mu, delta, eps, cterm, dq, dk, dv, ma
     a.dq_accum = ptr(dq_accum)
     workspace = None
     if mask.fp32_parts and (n := lib.jvpfa_bwd_workspace(C.byref(a))):
-        workspace = torch.empty(n, device=q.device, dtype=torch.uint8)
-        a.workspace, a.workspace_bytes = ptr(workspace), n
+        try:
+            workspace = torch.empty(n, device=q.device, dtype=torch.uint8)
+            a.workspace, a.workspace_bytes = ptr(workspace), n
+        except torch.OutOfMemoryError:
+            pass  # the register-tiled kernels, which need none
     check(_launch(q, lib.jvpfa_bwd, a), "jvpfa_bwd")
 
 

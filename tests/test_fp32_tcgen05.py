@@ -335,6 +335,27 @@ def _workspace(B, H, L, D, tangents=0, impl=_lib.IMPL_AUTO, dtype=_lib.FP32, **f
     return lib.jvpfa_fwd_workspace(ctypes.byref(a)), lib.jvpfa_fwd_uses_tcgen05(ctypes.byref(a))
 
 
+def test_a_backward_that_finds_no_memory_for_its_workspace_goes_without(monkeypatch):
+    """Host logic of the Python layer's launch, which a functorch transform of the cotangent takes: no memory, no workspace, no error."""
+    spec = _lib.MaskSpec(_lib.MASK_CAUSAL)
+    spec.fp32_parts = True
+    x, r = torch.zeros(2, 6, 512, 64), torch.zeros(2, 6, 512)
+    seen, empty = [], torch.empty
+
+    def launch(t, entry, a):
+        seen.append((a.workspace, a.workspace_bytes))
+        return 0
+
+    def no_memory(*args, **kw):
+        raise torch.OutOfMemoryError("made by this test")
+
+    monkeypatch.setattr(_lib, "_launch", launch)
+    for f in (empty, no_memory):
+        monkeypatch.setattr(torch, "empty", f)
+        _lib.bwd(x, x, x, None, None, None, x, None, r, None, r, r, r, x, x, x, spec, 0.125)
+    assert seen[0][0] and seen[0][1] == 24 * x.numel() and seen[1] == (None, 0)
+
+
 def test_where_fp32_takes_the_tcgen05_kernels():
     """Host logic.  From 384 16-row tiles on at D = 64 (320 at 128, 1024 at 32), and not for one 64-row tile; 18, 24 or 36 bytes
     an element (three, four or six tensors); with a workspace that is large enough and aligned."""
