@@ -323,7 +323,7 @@ class MaskSpec:
         self.tile_live = None  # MASK_BOOL: bitmap from mask_tiles(), lets the forward step over dead tiles
         self.tile_live_t = None  # ... and its transpose (per 128-key tile), for the backward launch that owns keys
         self._native = None  # the native layer's form of this description, made on first use
-        self.fp32_parts = False  # the forward of this call ran on the fp32 tcgen05 kernels: so does a backward through O
+        self.fp32_parts = False  # the forward of this call had a workspace for the fp32 tcgen05 kernels: so does a backward through O
         self.fp32_mode = None  # fp32 precision the forward of this call ran under ("3xtf32" / "tf32"); None = current
 
     def native(self):

@@ -83,9 +83,9 @@ struct Call {
   MaskPtr mask;
   double scale;
   bool tf32;  // fp32 tensors: one TF32 product instead of three, recorded so that the backward recomputes what the forward saw
-  // fp32: whatever is asked of the call's backward, the tcgen05 kernels form it, which recompute the scores as the tcgen05
-  // forward forms them.  (A backward of the register-tiled kernels, whose scores are off in their own way, keeps the forward
-  // whose lse is off in the same.)
+  // fp32: the tcgen05 kernels, which recompute the scores as the tcgen05 forward forms them.  Asked for where whatever may be asked
+  // of the call's backward is theirs, and kept for that backward if the forward ran on them.  (The register-tiled kernels, whose
+  // scores are off in their own way, keep the forward whose lse is off in the same.)
   bool parts = false;
   // A boolean mask as bits, by rows and transposed: the form the 16-bit tensor-core kernels read best, made by this call for
   // its forward and backward (pack_mask).
@@ -166,6 +166,7 @@ bool common_layout(std::initializer_list<const Tensor*> ts, int64_t* st) {
 
 struct FwdResult {
   Tensor o, to, lse, mu;
+  bool parts = false;  // fp32: there was a workspace for the tcgen05 kernels (Call::parts of a backward from this lse and mu)
 };
 using Grads = std::array<Tensor, 3>;
 
@@ -353,6 +354,7 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
   const Tensor workspace = workspace_of(call.parts ? jvpfa_fwd_workspace(&a) : 0, q);
   const Tensor bits = use_workspace(a, workspace, call, q);
+  r.parts = workspace.defined();
   check_status(jvpfa_fwd(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "jvpfa_fwd");
   return r;
 }
@@ -511,6 +513,7 @@ struct AttnBwdNode : public Node {
     Call c = call;
     c.parts = !again || (zero_tkv && (skip & JVPFA_SKIP_DKDV));
     FwdResult f = launch_fwd(qp, kp, vp, t[0], t[1], t[2], c);
+    c.parts = f.parts;
     if (again) {
       Grads h = launch_bwd(qp, kp, vp, t[0], t[1], t[2], f.o, f.to, f.lse, f.mu, Tensor(), gop, c, skip);
       for (int i = 0; i < 3; ++i) out[i] = h[i];
@@ -659,6 +662,7 @@ std::optional<Outputs> attend_plain(const Tensor& q, const Tensor& k, const Tens
     if (q.is_cuda()) no_gil.emplace();
     pack_mask(call, q, backward);
     r = launch_fwd(q, k, v, tq, tk, tv, call);
+    call.parts = r.parts;
   }
   if (backward || grad_mask) {
     auto node = std::shared_ptr<AttnNode>(new AttnNode(), torch::autograd::deleteNode);

@@ -323,6 +323,33 @@ def test_a_replayed_call_is_computed_behind_a_16_bit_launch_that_gave_up():
             assert _lib.device_status(clear=True) == code
 
 
+@pytest.mark.gpu
+def test_a_forward_without_memory_for_its_workspace_decides_for_the_backward(monkeypatch):
+    """Both run on the register-tiled kernels then, whose lse and scores belong together, also where the backward finds memory."""
+    from jvp_flash_attention_b200 import jvp_attention as ja
+
+    g = torch.Generator().manual_seed(4)
+    q, k, v, go = (torch.randn(2, 16, 2048, 64, generator=g).to(DEV) for _ in range(4))
+    a = [x.requires_grad_() for x in (q, k, v)]
+
+    def grads(o):
+        return [x.detach() for x in (o, *torch.autograd.grad(o, a, go))]
+
+    monkeypatch.setattr(ja, "KERNEL_IMPL", _lib.IMPL_GENERIC)
+    want = grads(ja.attention(*a))
+    monkeypatch.setattr(ja, "KERNEL_IMPL", _lib.IMPL_AUTO)
+    assert not torch.equal(want[0], ja.attention(*a).detach())
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (48 << 20)) / total)  # O needs 17 MB, the workspace 75
+    try:
+        o = ja.attention(*a)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for x, y in zip(grads(o), want):
+        assert torch.equal(x, y)
+
+
 def _workspace(B, H, L, D, tangents=0, impl=_lib.IMPL_AUTO, dtype=_lib.FP32, **fields):
     class At(int):
         shape = (B, H, L, D)
