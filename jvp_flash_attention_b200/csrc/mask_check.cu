@@ -102,8 +102,8 @@ __global__ void __launch_bounds__(kCheckThreads) mask_check_kernel(const jvpfa_m
 // HBM bound (1 byte read and 1/4 byte written per entry), if enough of it is in flight: a warp takes 32 rows x 256 keys and
 // a lane asks for its 8 bytes of all 32 rows at once.  Four lanes put a row's word together; eight rows at a time are
 // transposed as 8 x 8 bits, and the CTA's eight warps (256 rows) pass the transposed words through shared memory so that
-// they leave as 32-byte pieces.  B2 H12 L2048 (100 MB) 32 us, one head of L4096 (17 MB) 8
-// us; 16 bytes of up to eight rows at a time and a transposition bit by bit took 60 and 25 us.
+// they leave as 32-byte pieces.  B2 H12 L2048 (100 MB) 32 us, 36 where other kernels' lines leave L2 meanwhile; one head of L4096
+// (17 MB) 8 us; 16 bytes of up to eight rows at a time and a transposition bit by bit took 60 and 25 us.
 // With the packed mask, B2 H12 L2048 D64 and nine tenths random False: forward with tangents 168 -> 151 us, backward
 // through tO 239 -> 186 us.
 constexpr int kPackRows = 256, kPackKeys = 256;
@@ -174,14 +174,49 @@ __global__ void __launch_bounds__(256, 4) mask_pack_kernel(const jvpfa_mask m, i
       }
     }
   } else {
+    // Rows that begin anywhere: three aligned words hold eight bytes of a row, where all that a lane reads lies inside the mask.  Else
+    // byte by byte, in order of columns, so that all rows are in flight at once.  (From DRAM, us, row after row and byte after byte / so:
+    // 77 heads of L66 22 / 12, 43 of L130 27 / 12, 24 of L1330 57 / 35, of L2046 91 / 60.)
     const int n = min(8, L - col);  // <= 0: beyond the end
+    const int rows = min(32, n_rows - row0);
+    const unsigned char* first = reinterpret_cast<const unsigned char*>(m.ptr);
+    const unsigned char* end = first + (long long)(gridDim.z / n_h - 1) * m.stride[0] + (long long)(n_h - 1) * m.stride[1] +
+                               (long long)(n_rows - 1) * rs + (long long)(L - 1) * ks + 1;
+    const bool words = ks == 1 && rs >= 0 && m.stride[0] >= 0 && m.stride[1] >= 0 && n > 0 && rows > 0 &&
+                       p0 - (reinterpret_cast<uintptr_t>(p0) & 3u) >= first && p0 + (long long)(rows - 1) * rs + 12 <= end;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      x[j] = 0u;
-      for (int i = 0; i < 4; ++i) {
-        const unsigned char* p = p0 + (long long)(4 * j + i) * rs;
-        if (row0 + 4 * j + i < n_rows)
-          for (int c = 0; c < n; ++c) x[j] |= (p[c * ks] != 0 ? 1u : 0u) << (8 * i + c);
+    for (int j = 0; j < 8; ++j) x[j] = 0u;
+    if (words) {
+      const uint32_t cols = (1u << n) - 1u;
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        uint32_t v[8][3], shift[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const unsigned char* p = p0 + (long long)(4 * j + r) * rs;
+          shift[r] = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3u);
+#pragma unroll
+          for (int w = 0; w < 3; ++w) {
+            v[r][w] = 0u;
+            if (4 * j + r < rows) v[r][w] = __ldg(reinterpret_cast<const uint32_t*>(p - shift[r]) + w);
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const uint32_t lo = __funnelshift_r(v[r][0], v[r][1], 8 * shift[r]), hi = __funnelshift_r(v[r][1], v[r][2], 8 * shift[r]);
+          x[j + (r >> 2)] |= ((nonzero_bits(lo) | nonzero_bits(hi) << 4) & cols) << (8 * (r & 3));
+        }
+      }
+    } else {
+      for (int c = 0; c < n; ++c) {
+        uint32_t v[32];
+#pragma unroll
+        for (int r = 0; r < 32; ++r) {
+          v[r] = 0u;
+          if (r < rows) v[r] = __ldg(p0 + (long long)r * rs + (long long)c * ks);
+        }
+#pragma unroll
+        for (int r = 0; r < 32; ++r) x[r >> 2] |= (v[r] != 0u ? 1u : 0u) << (8 * (r & 3) + c);
       }
     }
   }

@@ -1,6 +1,7 @@
 """GPU tests at the edges of the dispatch: head dimension 32 on the D = 64 tensor-core kernels, masks whose rows do not
 fill 16-byte pieces, the forms of the register-tiled kernels, the range of fp32, gradients that nobody asked for, and what a
 call takes of memory and of the interpreter."""
+import ctypes
 import threading
 import time
 
@@ -439,6 +440,40 @@ def test_tile_bitmaps_are_those_of_the_host_stand_in(L, layout):
     dev = torch.empty_strided(m.shape, m.stride(), dtype=torch.bool, device=DEV).copy_(m) if layout != "expanded" else m[:1].to(DEV).expand(2, -1, -1, -1)
     for x, y in zip(_lib.mask_tiles(spec(dev), L), stand_in.mask_tiles(spec(m), L)):
         assert torch.equal(x.cpu(), y.to(x.dtype))
+
+
+@pytest.mark.parametrize("L", [33, 66, 130, 257, 520])
+@pytest.mark.parametrize("layout", ["rows", "offset", "padded", "keys", "one row", "expanded"])
+def test_packed_bits_are_the_mask(L, layout):
+    """Bits by rows and transposed, of rows that begin at any address: whole pieces, words that straddle them, and the mask's ends."""
+    g = torch.Generator().manual_seed(L)
+    heads, n_rows = (2, 3), 1 if layout == "one row" else L
+    m = torch.rand(*heads, n_rows, L, generator=g) > 0.5
+    dev = m.to(DEV)
+    if layout == "offset":  # the first entry one byte behind a 16-byte boundary, the last one at the end of its storage
+        dev = torch.cat([torch.ones(1, dtype=torch.bool, device=DEV), dev.flatten()])[1:].view(m.shape)
+    elif layout == "padded":
+        dev = torch.nn.functional.pad(dev, (3, 4), value=True)[..., 3:-4]
+    elif layout == "keys":
+        dev = dev.transpose(2, 3).contiguous().transpose(2, 3)
+    elif layout == "expanded":
+        m, dev = m[:, :1], dev[:, :1].contiguous().expand(2, 3, L, L)
+    n_h, w, wt = m.shape[1], (L + 63) // 64 * 2, (n_rows + 63) // 64 * 2 if n_rows > 1 else 1
+    a = _lib.MaskTilesArgs(struct_size=ctypes.sizeof(_lib.MaskTilesArgs), n_b=2, n_h=n_h, n_rows=n_rows, L=L)
+    a.mask = _lib.MaskSpec(_lib.MASK_BOOL, dev.view(torch.uint8), tuple(0 if n == 1 else s for n, s in zip(m.shape, dev.stride()))).to_c()
+    a.mask.stride[3] = dev.stride(3)
+    bits = torch.zeros(2 * n_h, n_rows, w, dtype=torch.int32, device=DEV)
+    bits_t = torch.zeros(2 * n_h, L, wt, dtype=torch.int32, device=DEV)
+    a.bits, a.bits_t = bits.data_ptr(), bits_t.data_ptr()
+    _lib.check(_lib.load().jvpfa_mask_tiles(ctypes.byref(a), torch.cuda.current_stream().cuda_stream), "jvpfa_mask_tiles")
+    one = torch.arange(32, dtype=torch.int32)
+
+    def unpack(x, n):
+        return (x.cpu()[..., None] >> one & 1).flatten(-2).bool()[..., :n]
+
+    m = m.reshape(-1, n_rows, L)
+    assert torch.equal(unpack(bits, L), m)
+    assert torch.equal(unpack(bits_t, n_rows), m.transpose(1, 2))
 
 
 @pytest.mark.parametrize("D", [32, 64, 128])
