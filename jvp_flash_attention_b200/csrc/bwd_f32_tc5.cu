@@ -914,7 +914,7 @@ static int launch_bwd_f32_d(const jvpfa_bwd_args& a, const CUtensorMap& map, int
 long long bwd_f32_tc5_workspace(const jvpfa_bwd_args& a) {
   if (a.dtype != JVPFA_FP32 || a.impl == JVPFA_IMPL_GENERIC) return 0;
   if (a.gto && (a.go || !(a.flags & JVPFA_ZERO_TKV) || !(a.flags & JVPFA_SKIP_DKDV))) return 0;
-  if (a.impl == JVPFA_IMPL_AUTO && !tc5::f32_rows_enough(a.B, a.H, a.L, a.D)) return 0;
+  if (a.impl == JVPFA_IMPL_AUTO && !tc5::f32_rows_enough(a.mask, a.B, a.H, a.L, a.D)) return 0;
   return (long long)(a.gto ? 5 : 4) * 3 * 2 * a.B * a.H * a.L * a.D;
 }
 

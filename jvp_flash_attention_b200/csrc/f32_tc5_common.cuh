@@ -125,19 +125,29 @@ struct F32RowMask {
   }
 };
 
-// From how many rows on the register-tiled kernels, which fill the GPU from fewer, are the slower ones.  Measured on a B200,
-// us, register-tiled / here, for O alone and with tangents; n16 = 16-row tiles of the call:
-//   D = 128  n16 256 (L2048) 249/101 469/249, causal 137/101 250/251; n16 288 (L130) 33/26 55/48; n16 416 (L200) 45/32 96/60;
-//            n16 1024 (L1024) 297/73 679/169; 64-row sequences, n16 1024: 33/36 63/62
-//   D = 64   n16 256 (L512) 34/30 71/46, bias 36/42 74/65; n16 384 (L500) 59/30 121/50, bias 59/38 123/71; n16 1024 (L1024) 169/48
-//            338/89; 64-row sequences, n16 1024: 21/26 35/38
-//   D = 32   n16 528 (L700) 50/34 82/50, bias 49/48 82/87; n16 1152 (L130) 27/30 49/42; n16 1024 (L1024) 84/42 169/71, bias 99/71
-//            183/114; n16 1664 (L200) 45/34 80/54
-inline bool f32_rows_enough(int B, int H, int L, int D) {
+// Whether a call has rows enough for these kernels, which work on 128-row tiles and split their inputs first, not to be slower than
+// the register-tiled ones, which fill the GPU from fewer.  n16: 16-row tiles of the call.  Measured on a B200, us of the device,
+// register-tiled / here: O alone, with tangents, O and its three gradients; 64-row sequences (one tile, half of it empty) lose.
+//   D = 64   L66  n16 385 16/16 31/25 53/49    bias 18/18 31/27 54/63   ragged boolean 18/29 33/37 55/74
+//            L96  n16 384 16/18 31/27 55/51    bias 18/23 33/29 57/68   n16 672 bias 29/25 49/33 100/72
+//            L130 n16 387 25/20 45/31 80/59    bias 25/25 45/33 79/76   ragged boolean 25/31 49/43 82/84, n16 774 43/41 72/61 145/121
+//            L192 n16 384 27/20 51/33 94/57    bias 29/22 55/33 94/70   L512 n16 256 34/30 71/46, bias 36/42 74/65
+//   D = 128  L66  n16 320 25/23 49/39 90/82    causal 25/23 41/39 78/82  bias 25/23 49/41 90/92   ragged boolean 25/33 51/57 92/106
+//            L96  n16 324 25/23 51/41 96/86    causal 23/22 41/41 80/88  bias 27/27 53/45 96/100, n16 642 43/31 86/53 176/111
+//            L112 n16 322 31/23 61/43 115/90   causal 29/23 47/43 96/90  bias 29/25 61/45 115/100
+//   D = 32   L192 n16 1032 22/29 41/43 84/86   causal 25/27 41/39 82/76  n16 4104 53/61 119/104 207/203  (64-row tiles fit, 128 do not)
+//            L200 n16 1027 35/31 66/47 119/96  bias 37/39 68/55 147/123; L208 n16 1027 bias 37/41, n16 1547 57/45
+//            L256 n16 1024 29/23 51/33 106/61  bias 33/27 55/37 150/80
+// Far above the lines nothing loses more than 3 % (D64 n16 12288: L66 244/188 610/330 917/631, L96 with bias 223/231 547/360
+// 1059/727).  Below them long sequences gain as well (D = 128 n16 256, L2048: 249/101 469/249), short ones do not.
+// `by_element`: a bias, and a boolean mask that is packed first because its rows are not whole 16-byte pieces.
+inline bool f32_rows_enough(const jvpfa_mask& m, int B, int H, int L, int D) {
   const long long n16 = tiles16(B, H, L);
-  if (D == 128) return L > 64 && n16 >= 320;
-  if (D == 64) return L > 64 && n16 >= 384;
-  return L >= 192 && n16 >= 1024;
+  const bool by_element =
+      m.kind == JVPFA_MASK_BIAS || (m.kind == JVPFA_MASK_BOOL && ((L & 15) != 0 || !tc5_mask_layout(m, JVPFA_FP32, L)));
+  if (D == 128) return L > 64 && n16 >= (L <= 96 && (by_element || m.kind == JVPFA_MASK_CAUSAL) ? 576 : 320);
+  if (D == 64) return L > 64 && n16 >= (L < 192 && by_element ? 640 : 384);
+  return L > 192 && n16 >= (L < 224 && by_element ? 1280 : 1024);
 }
 
 // Host: the splitting launch, and the tensor map of its result (boxes of 64 columns x 64 rows of one plane).

@@ -618,7 +618,7 @@ static int fwd_f32_slots(const jvpfa_fwd_args& a) { return !a.tq ? 3 : (a.flags 
 
 long long fwd_f32_tc5_workspace(const jvpfa_fwd_args& a) {
   if (a.dtype != JVPFA_FP32 || a.impl == JVPFA_IMPL_GENERIC) return 0;
-  if (a.impl == JVPFA_IMPL_AUTO && !tc5::f32_rows_enough(a.B, a.H, a.L, a.D)) return 0;
+  if (a.impl == JVPFA_IMPL_AUTO && !tc5::f32_rows_enough(a.mask, a.B, a.H, a.L, a.D)) return 0;
   return (long long)fwd_f32_slots(a) * 3 * 2 * a.B * a.H * a.L * a.D;
 }
 

@@ -384,15 +384,29 @@ def test_a_backward_that_finds_no_memory_for_its_workspace_goes_without(monkeypa
 
 
 def test_where_fp32_takes_the_tcgen05_kernels():
-    """Host logic.  From 384 16-row tiles on at D = 64 (320 at 128, 1024 at 32), and not for one 64-row tile; 18, 24 or 36 bytes
-    an element (three, four or six tensors); with a workspace that is large enough and aligned."""
+    """Host logic.  From 384 16-row tiles on at D = 64 (320 at 128, 1024 at 32), and not for one 64-row tile; later for short sequences
+    with a mask that is read by element, or at D = 128 a causal one; 18, 24 or 36 bytes an element (three, four or six tensors);
+    with a workspace that is large enough and aligned."""
     assert _workspace(2, 6, 512, 64) == (18 * 2 * 6 * 512 * 64, 0)  # (no workspace given: the register-tiled kernels)
     assert _workspace(2, 6, 512, 64, 1)[0] == 24 * 2 * 6 * 512 * 64
     assert _workspace(2, 6, 512, 64, 3)[0] == 36 * 2 * 6 * 512 * 64
     assert _workspace(2, 6, 496, 64)[0] == 0 and _workspace(16, 16, 64, 64)[0] == 0
     assert _workspace(2, 5, 512, 128)[0] > 0 and _workspace(2, 5, 480, 128)[0] == 0
     assert _workspace(4, 16, 256, 32)[0] > 0 and _workspace(4, 16, 128, 32)[0] == 0 and _workspace(2, 16, 448, 32)[0] == 0
+    assert _workspace(1, 200, 192, 32)[0] == 0 and _workspace(1, 200, 194, 32)[0] > 0
     assert _workspace(1, 1, 32, 64, impl=_lib.IMPL_TCGEN05)[0] > 0
+
+    def masked(kind, B, H, L, D, offset=0):
+        m = _lib.Mask(kind=kind, bias_dtype=_lib.FP32, ptr=(1 << 20) + offset)
+        m.stride[:] = [H * L * L, L * L, L, 1]
+        return _workspace(B, H, L, D, mask=m)[0] > 0
+
+    for kind, offset in ((_lib.MASK_BIAS, 0), (_lib.MASK_BOOL, 1)):
+        assert not masked(kind, 1, 63, 160, 64, offset) and masked(kind, 1, 64, 160, 64, offset) and masked(kind, 1, 32, 192, 64, offset)
+        assert not masked(kind, 1, 95, 96, 128, offset) and masked(kind, 1, 96, 96, 128, offset) and masked(kind, 1, 46, 112, 128, offset)
+        assert not masked(kind, 1, 98, 208, 32, offset) and masked(kind, 1, 99, 208, 32, offset) and masked(kind, 1, 74, 224, 32, offset)
+    assert masked(_lib.MASK_BOOL, 1, 39, 160, 64) and not masked(_lib.MASK_BOOL, 1, 55, 130, 64)
+    assert masked(_lib.MASK_CAUSAL, 1, 39, 160, 64) and not masked(_lib.MASK_CAUSAL, 1, 95, 96, 128) and masked(_lib.MASK_NONE, 1, 54, 96, 128)
     for dtype in (_lib.BF16, _lib.FP16, _lib.FP32_TF32):
         assert _workspace(2, 6, 512, 64, dtype=dtype)[0] == 0
     assert _workspace(2, 6, 512, 64, impl=_lib.IMPL_GENERIC)[0] == 0
