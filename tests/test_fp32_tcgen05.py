@@ -350,6 +350,96 @@ def test_a_forward_without_memory_for_its_workspace_decides_for_the_backward(mon
         assert torch.equal(x, y)
 
 
+def _all_results(q, k, v, tq, tk, tv, go, mask=None, **kw):
+    """O and its gradients, and O and tO of a call without gradients: the calls that the tcgen05 kernels serve as a whole."""
+    from jvp_flash_attention_b200 import jvp_attention as ja
+
+    dev = [x.to(DEV) for x in (q, k, v, tq, tk, tv)]
+    m = None if mask is None else mask.to(DEV)
+    o, to = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, attn_mask=m, **kw), tuple(dev[:3]), tuple(dev[3:]))
+    a = [x.requires_grad_() for x in dev[:3]]
+    o2 = ja.attention(*a, attn_mask=m, **kw)
+    assert torch.allclose(o, o2, 0.0, 0.0, equal_nan=True)
+    return [x.detach().cpu().double() for x in (o, to, *torch.autograd.grad(o2, a, go.to(DEV)))]
+
+
+def _range_inputs(D):
+    """Rows enough for the tcgen05 kernels at every head dimension, with or without a mask."""
+    B, H, L = 2, 24 if D == 32 else 14, 450
+    assert _workspace(B, H, L, D)[0] > 0
+    g = torch.Generator().manual_seed(D)
+    return (B, H, L), g, [torch.randn(B, H, L, D, generator=g) * (0.1 if n in (3, 4, 5) else 1.0) for n in range(7)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("big", [1e8, 1e15, 1e36, 3.4e38, math.inf, math.nan])
+def test_a_large_entry_costs_the_others_nothing(D, big):
+    """One entry of V (of gO for dV) that is very large (3.4e38: above bf16's largest number), Inf or NaN: the other columns are what
+    they are without it, to 2^-20 of P |V| (P^T |gO|): products are exact to 2^-24 and a column sums a few hundred.  That column is
+    P V, or not finite where V is not."""
+    (B, H, L), g, (q, k, v, tq, tk, tv, go) = _range_inputs(D)
+    rest = [c for c in range(D) if c != 5]
+    p = torch.softmax(q.double() @ k.double().transpose(-1, -2) * D**-0.5, -1)
+    ts = (tq.double() @ k.double().transpose(-1, -2) + q.double() @ tk.double().transpose(-1, -2)) * D**-0.5
+    w = p * (ts - (p * ts).sum(-1, keepdim=True))
+    v[:, :, L // 2, 5] = big
+    o, to, *_ = _all_results(q, k, v, tq, tk, tv, go)
+    vd, tvd = v.double()[..., rest], tv.double()[..., rest]
+    for x, r, top in ((o, p @ vd, p @ vd.abs()), (to, w @ vd + p @ tvd, (p * ts.abs().amax(-1, keepdim=True)) @ vd.abs() + p @ tvd.abs())):
+        assert ((x[..., rest] - r).abs() / top).max().item() <= 2**-20
+    if math.isfinite(big):
+        assert (o[..., 5] - (p @ v.double()[..., 5:6])[..., 0]).abs().max().item() <= 2**-20 * big
+    else:
+        assert not torch.isfinite(o[..., 5]).any()
+    v[:, :, L // 2, 5] = 1.0
+    go[:, :, L // 3, 5] = big
+    dv = _all_results(q, k, v, tq, tk, tv, go)[4][..., rest]
+    pt, god = p.transpose(-1, -2), go.double()[..., rest]
+    assert ((dv - pt @ god).abs() / (pt @ god.abs())).max().item() <= 2**-20
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_rows_and_channels_of_very_different_magnitude(D):
+    """Rows of V and its tangent up to a factor of 2^40 apart, masked-out keys that hold 1e15, and a channel of q a million times
+    larger where k is that much smaller: 1e-5 of P |V| for O, of the head's largest V for tO, of a gradient's largest entry."""
+    (B, H, L), g, (q, k, v, tq, tk, tv, go) = _range_inputs(D)
+    zoom = torch.exp2(torch.randint(-20, 21, (B, H, L, 1), generator=g).float())
+    v, tv = v * zoom, tv * zoom
+    s = torch.ones(D)
+    s[1], s[2] = 2.0**20, 2.0**-20
+    q, tq, k, tk = q * s, tq * s, k / s, tk / s
+    dead = torch.rand(B, 1, L, 1, generator=g) > 0.8
+    dead[:, :, 0] = False
+    mask = (torch.rand(B, 1, L, L, generator=g) > 0.3) & ~dead.transpose(2, 3)
+    mask[..., 0] = True
+    clean = [x.masked_fill(dead, 0.0) for x in (k, v, tk, tv)]
+    ro, rto = orc.sdpa_jvp(q, clean[0], clean[1], tq, clean[2], clean[3], mask.expand(B, H, L, L))[:2]
+    grads = orc.grads_through_both(q, clean[0], clean[1], tq, clean[2], clean[3], go, None, attn_mask=mask)[2:]
+    k, v, tk, tv = (x.masked_fill(dead, 1e15) for x in (k, v, tk, tv))
+    got = _all_results(q, k, v, tq, tk, tv, go, mask)
+    scores = (q.double() @ clean[0].double().transpose(-1, -2) * D**-0.5).masked_fill(~mask, -math.inf)
+    tops = [torch.softmax(scores, -1) @ clean[1].double().abs(), clean[1].double().abs().amax(dim=(2, 3), keepdim=True)]
+    scales = [1.0, 1.0, s.double(), 1 / s.double(), 1.0]
+    for n, (x, r) in enumerate(zip(got, (ro, rto, *grads))):
+        x, r = x * scales[n], r.double() * scales[n]
+        top = tops[n] if n < 2 else r.abs().amax(dim=(2, 3), keepdim=True)
+        assert torch.isfinite(x).all() and ((x - r).abs() / top.clamp(min=1e-30)).max().item() <= 1e-5, n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_a_negative_softmax_scale(D):
+    (B, H, L), g, ts = _range_inputs(D)
+    q, k, v, tq, tk, tv, go = ts
+    got = _all_results(*ts, causal=True, sm_scale=-0.2)
+    flip = [-q, k, v, -tq, tk, tv]  # the same scores at a positive one
+    ref = _all_results(*flip, go, causal=True, sm_scale=0.2)
+    for n, (x, r) in enumerate(zip(got, ref)):
+        assert torch.equal(x, -r if n == 2 else r), n
+
+
 def _workspace(B, H, L, D, tangents=0, impl=_lib.IMPL_AUTO, dtype=_lib.FP32, **fields):
     class At(int):
         shape = (B, H, L, D)

@@ -491,7 +491,10 @@ def test_register_tiled_kernels_with_one_warp_for_16_rows(monkeypatch, D, how, k
 
 @pytest.mark.parametrize("D", [32, 64, 128])
 @pytest.mark.parametrize("want", ["q", "kv"])
-def test_one_warp_for_16_rows_leaves_out_what_nobody_asked_for(D, want):
+@pytest.mark.parametrize("impl", [_lib.IMPL_GENERIC, _lib.IMPL_AUTO], ids=["one warp", "tcgen05"])
+def test_one_warp_for_16_rows_leaves_out_what_nobody_asked_for(monkeypatch, D, want, impl):
+    """Of the register-tiled kernels with one warp for 16 rows, and of the fp32 tcgen05 kernels, which serve such a call otherwise."""
+    monkeypatch.setattr(ja, "KERNEL_IMPL", impl)
     q, k, v, _, _, _, go, _ = (x.to(DEV) for x in _inputs(4, 10, 474, D, torch.float32, 5))
 
     def run(names):
