@@ -12,6 +12,7 @@ import pytest
 import torch
 
 from jvp_flash_attention_b200 import _lib
+from jvp_flash_attention_b200 import jvp_attention as ja
 
 pytestmark = pytest.mark.gpu
 
@@ -111,3 +112,41 @@ def test_repeated_launches_with_a_boolean_mask():
     _soak(lambda: _lib.bwd(d["q"], d["k"], d["v"], d["tq"], d["tk"], d["tv"], d["go"], d["gto"], lse, mu, stats[0],
                            stats[1], stats[2], dq, dk, dv, spec, D ** -0.5, _lib.IMPL_TCGEN05, dq_accum=acc),
           [dk, dv], close=[dq])
+
+
+def _into(outs, step):
+    def run():
+        for o, x in zip(outs, step()):
+            o.copy_(x)
+    return run
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("kind", ["none", "causal", "bias"])
+def test_repeated_fp32_calls_on_the_tcgen05_kernels(D, kind):
+    """Forward with tangents, gradients through O, and a Hessian-vector product along q (forward and dQ through tO)."""
+    B, H, L = 2, 16 if D == 32 else 6, 520
+    d = _tensors(B, H, L, D, torch.float32, seed=D)
+    kw = dict(causal=kind == "causal", attn_mask=torch.randn(B, H, L, L, device=DEV) if kind == "bias" else None)
+    a = [d[n].clone().requires_grad_() for n in "qkv"]
+
+    def step():
+        o, to = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, **kw), (d["q"], d["k"], d["v"]), (d["tq"], d["tk"], d["tv"]))
+        grads = torch.autograd.grad(ja.attention(*a, **kw), a, d["go"])
+        (dq,) = torch.autograd.grad(ja.attention(a[0], d["k"], d["v"], **kw), a[0], d["go"], create_graph=True)
+        return [x.detach() for x in (o, to, *grads, dq, *torch.autograd.grad(dq, a[0], d["gto"]))]
+
+    outs = [torch.empty_like(d["q"]) for _ in range(7)]
+    _soak(_into(outs, step), outs)
+
+
+@pytest.mark.parametrize("cot", ["both", "t"])
+def test_repeated_launches_with_a_bias_through_the_tangent(cot):
+    B, H, L, D = 2, 12, 1040, 64
+    d = _tensors(B, H, L, D, torch.bfloat16, seed=2)
+    mask = torch.randn(B, H, L, L, device=DEV, dtype=torch.bfloat16)
+    a = [d[n].clone().requires_grad_() for n in "qkv"]
+    o, to = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, attn_mask=mask), tuple(a), (d["tq"], d["tk"], d["tv"]))
+    asked = [(to, d["gto"])] + [(o, d["go"])] * (cot == "both")
+    outs = [torch.empty_like(d["q"]) for _ in range(3)]
+    _soak(_into(outs, lambda: torch.autograd.grad([x for x, _ in asked], a, [w for _, w in asked], retain_graph=True)), outs)
