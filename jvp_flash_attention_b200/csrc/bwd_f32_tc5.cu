@@ -7,9 +7,9 @@
 //     dQ = scale gS K
 // in two launches, one that owns queries (dQ) and one that owns keys (dK, dV), as the register-tiled kernels.
 //
-// The launch that owns queries: CTA = one 128-row query tile of one (batch, head), 384 threads with the roles of the forward (fwd_f32_tc5.cu): producer,
-// issuing warp, two elementwise warpgroups (thread <-> query row <-> TMEM lane; group w takes keys [32 w, 32 w + 32) of a 64-key
-// tile, and half of dQ's columns in its registers).
+// The launch that owns queries: CTA = one 128-row query tile of one (batch, head), 384 threads with the roles of the forward
+// (fwd_f32_tc5.cu): producer, issuing warp, two elementwise warpgroups (thread <-> query row <-> TMEM lane; group w takes keys
+// [32 w, 32 w + 32) of a 64-key tile, and half of dQ's columns in its registers).
 // Shared memory: the parts of the own operands (Q, gO | Q, tQ, G), and a ring of 8 KiB units: one part of 64 keys x 64 columns of
 // K, of V, and of K once more for dQ.  D = 128: the lo parts of the own operands are TMEM operands.
 // TMEM: the scores of a tile (two buffers where they fit: the next tile's are formed under this one's elementwise work); gS in

@@ -532,41 +532,41 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
           const uint32_t lp = ring_lo + cs.st_tile;  // tile slot 0 of the stage
           const uint32_t acc = tmem + cs.buf_col;
           if (elect_one()) {
-          if (!part_b) {
-            if constexpr (OWN_KEYS) {
-              if constexpr (HAS_GT) {
-                score(acc + C::OFF_S, IntC<C::SLOT_K>{}, lp + C::SLOT_Q * LOOP16, I1{}, I1{});    // [S|TS] = K [Q;tQ]^T
-                score(acc + C::OFF_TS, IntC<C::SLOT_TK>{}, lp + C::SLOT_Q * LOOP16, I0{}, I0{});  // TS += tK Q^T
+            if (!part_b) {
+              if constexpr (OWN_KEYS) {
+                if constexpr (HAS_GT) {
+                  score(acc + C::OFF_S, IntC<C::SLOT_K>{}, lp + C::SLOT_Q * LOOP16, I1{}, I1{});    // [S|TS] = K [Q;tQ]^T
+                  score(acc + C::OFF_TS, IntC<C::SLOT_TK>{}, lp + C::SLOT_Q * LOOP16, I0{}, I0{});  // TS += tK Q^T
+                } else {
+                  score(acc + C::OFF_S, IntC<C::SLOT_K>{}, lp + C::SLOT_Q * LOOP16, I1{}, I0{});    // S = K Q^T
+                }
               } else {
-                score(acc + C::OFF_S, IntC<C::SLOT_K>{}, lp + C::SLOT_Q * LOOP16, I1{}, I0{});    // S = K Q^T
+                if constexpr (HAS_GT) {
+                  score(acc + C::OFF_S, IntC<C::SLOT_Q>{}, lp + C::SLOT_K * LOOP16, I1{}, I1{});    // [S|TS] = Q [K;tK]^T
+                  score(acc + C::OFF_TS, IntC<C::SLOT_TQ>{}, lp + C::SLOT_K * LOOP16, I0{}, I0{});  // TS += tQ K^T
+                } else {
+                  score(acc + C::OFF_S, IntC<C::SLOT_Q>{}, lp + C::SLOT_K * LOOP16, I1{}, I0{});    // S = Q K^T
+                }
               }
             } else {
-              if constexpr (HAS_GT) {
-                score(acc + C::OFF_S, IntC<C::SLOT_Q>{}, lp + C::SLOT_K * LOOP16, I1{}, I1{});    // [S|TS] = Q [K;tK]^T
-                score(acc + C::OFF_TS, IntC<C::SLOT_TQ>{}, lp + C::SLOT_K * LOOP16, I0{}, I0{});  // TS += tQ K^T
+              if constexpr (OWN_KEYS) {
+                if constexpr (HAS_GT) {
+                  score(acc + C::OFF_E, IntC<C::SLOT_V>{}, lp + C::SLOT_G * LOOP16, I1{}, I0{});    // E = V G^T
+                  score(acc + C::OFF_FP, IntC<C::SLOT_TV>{}, lp + C::SLOT_G * LOOP16, I1{}, I0{});  // FP = tV G^T
+                  if constexpr (HAS_GO) score(acc + C::OFF_FP, IntC<C::SLOT_V>{}, lp + C::SLOT_GO * LOOP16, I0{}, I0{});
+                } else {
+                  score(acc + C::OFF_FP, IntC<C::SLOT_V>{}, lp + C::SLOT_GO * LOOP16, I1{}, I0{});  // FP = V gO^T
+                }
               } else {
-                score(acc + C::OFF_S, IntC<C::SLOT_Q>{}, lp + C::SLOT_K * LOOP16, I1{}, I0{});    // S = Q K^T
+                if constexpr (HAS_GT) {
+                  score(acc + C::OFF_E, IntC<C::SLOT_G>{}, lp + C::SLOT_V * LOOP16, I1{}, I1{});    // [E|FP] = G [V;tV]^T
+                  if constexpr (HAS_GO) score(acc + C::OFF_FP, IntC<C::SLOT_GO>{}, lp + C::SLOT_V * LOOP16, I0{}, I0{});
+                } else {
+                  score(acc + C::OFF_FP, IntC<C::SLOT_GO>{}, lp + C::SLOT_V * LOOP16, I1{}, I0{});  // FP = gO V^T
+                }
               }
             }
-          } else {
-            if constexpr (OWN_KEYS) {
-              if constexpr (HAS_GT) {
-                score(acc + C::OFF_E, IntC<C::SLOT_V>{}, lp + C::SLOT_G * LOOP16, I1{}, I0{});    // E = V G^T
-                score(acc + C::OFF_FP, IntC<C::SLOT_TV>{}, lp + C::SLOT_G * LOOP16, I1{}, I0{});  // FP = tV G^T
-                if constexpr (HAS_GO) score(acc + C::OFF_FP, IntC<C::SLOT_V>{}, lp + C::SLOT_GO * LOOP16, I0{}, I0{});
-              } else {
-                score(acc + C::OFF_FP, IntC<C::SLOT_V>{}, lp + C::SLOT_GO * LOOP16, I1{}, I0{});  // FP = V gO^T
-              }
-            } else {
-              if constexpr (HAS_GT) {
-                score(acc + C::OFF_E, IntC<C::SLOT_G>{}, lp + C::SLOT_V * LOOP16, I1{}, I1{});    // [E|FP] = G [V;tV]^T
-                if constexpr (HAS_GO) score(acc + C::OFF_FP, IntC<C::SLOT_GO>{}, lp + C::SLOT_V * LOOP16, I0{}, I0{});
-              } else {
-                score(acc + C::OFF_FP, IntC<C::SLOT_GO>{}, lp + C::SLOT_V * LOOP16, I1{}, I0{});  // FP = gO V^T
-              }
-            }
-          }
-          tc_commit_u32(bar_s_full + cs.sf_bar);
+            tc_commit_u32(bar_s_full + cs.sf_bar);
           }
           cs.advance(2);
         }
@@ -610,22 +610,22 @@ bwd_tc5_d64_kernel(const jvpfa_bwd_args a, const __grid_constant__ Bwd64Maps map
           const uint32_t opnd = tmem + co.buf_col;
           const uint32_t acc = s > 0;
           if (elect_one()) {
-          if constexpr (OWN_KEYS) {
-            if (!second) {
-              outer(C::COL_OUT0, opnd + C::OFF_FP, lp + C::SLOT_Q * LOOP16, acc);                        // dK += gS^T Q
-              if constexpr (HAS_GT) outer(C::COL_OUT0, opnd + C::OFF_E, lp + C::SLOT_TQ * LOOP16, 1);   // dK += gtS^T tQ
-            } else if constexpr (HAS_GT) {
-              outer(C::COL_OUT1, opnd + C::OFF_TS, lp + C::SLOT_G * LOOP16, acc);                        // dV += A^T G
-              if constexpr (HAS_GO) outer(C::COL_OUT1, opnd + C::OFF_S, lp + C::SLOT_GO * LOOP16, 1);   // dV += P^T gO
+            if constexpr (OWN_KEYS) {
+              if (!second) {
+                outer(C::COL_OUT0, opnd + C::OFF_FP, lp + C::SLOT_Q * LOOP16, acc);                        // dK += gS^T Q
+                if constexpr (HAS_GT) outer(C::COL_OUT0, opnd + C::OFF_E, lp + C::SLOT_TQ * LOOP16, 1);   // dK += gtS^T tQ
+              } else if constexpr (HAS_GT) {
+                outer(C::COL_OUT1, opnd + C::OFF_TS, lp + C::SLOT_G * LOOP16, acc);                        // dV += A^T G
+                if constexpr (HAS_GO) outer(C::COL_OUT1, opnd + C::OFF_S, lp + C::SLOT_GO * LOOP16, 1);   // dV += P^T gO
+              } else {
+                outer(C::COL_OUT1, opnd + C::OFF_S, lp + C::SLOT_GO * LOOP16, acc);                        // dV += P^T gO
+              }
             } else {
-              outer(C::COL_OUT1, opnd + C::OFF_S, lp + C::SLOT_GO * LOOP16, acc);                        // dV += P^T gO
+              const uint32_t oc = C::COL_OUT0 + 64 * (kact & 1);
+              outer(oc, opnd + C::OFF_FP, lp + C::SLOT_K * LOOP16, acc);                                   // dQ += gS K
+              if constexpr (HAS_GT) outer(oc, opnd + C::OFF_E, lp + C::SLOT_TK * LOOP16, 1);              // dQ += gtS tK
             }
-          } else {
-            const uint32_t oc = C::COL_OUT0 + 64 * (kact & 1);
-            outer(oc, opnd + C::OFF_FP, lp + C::SLOT_K * LOOP16, acc);                                   // dQ += gS K
-            if constexpr (HAS_GT) outer(oc, opnd + C::OFF_E, lp + C::SLOT_TK * LOOP16, 1);              // dQ += gtS tK
-          }
-          tc_commit_u32(bar_loop_empty + co.st_bar);
+            tc_commit_u32(bar_loop_empty + co.st_bar);
           }
           co.advance(1);
         }

@@ -114,9 +114,6 @@ __device__ __forceinline__ void sts_v4(uint32_t addr, uint32_t a, uint32_t b, ui
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
 // D[tmem] (+)= A[smem] * B[smem]; descriptor low words as in umma_ss_lo, accumulate flag known at run time.
 __device__ __forceinline__ void mma_ss_dyn(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -131,9 +128,9 @@ struct FItem {
   int bh, b, h, own0, loop_begin, n_sub;
 };
 
-// MK: 0 = none / causal / key padding (index comparisons); 1 = uint8 mask with any strides (each elementwise thread
-// reads the 32 mask bytes of its key row and the sub-tile's queries before it waits for the scores); 2 = additive bias of
-// the element type, read the same way.
+// MK: 0 = none / causal / key padding (index comparisons); 1 = boolean mask, as bits or as bytes of any strides (each elementwise
+// thread requests the next sub-tile's 32 entries of its key when the scores of this one have left its registers); 2 = additive
+// bias of the element type, requested the same way.
 //
 // dQ of a bias call through tO is summed in a fixed order, as the two launches that served it sum it: a key tile's share goes to
 // a buffer of its own (dq_acc: [key tile][B*H][L][D] floats) and dq_sum_kernel adds them up.  Measured on a B200, the two
@@ -291,284 +288,284 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
   // Phase counters kept alike by all roles: g counts the sub-tiles of this CTA (ring stage g % STAGES, dQ buffer
   // g & 1; s_full, s_free complete once per sub-tile, p_full and out_free of buffer g & 1 every other one), kact the items that have sub-tiles.
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer + per-query statistics
-    if (lane == 0) {
-      prefetch_tmap(&maps.k), prefetch_tmap(&maps.v), prefetch_tmap(&maps.q);
-      if constexpr (HAS_GO) prefetch_tmap(&maps.go);
-      if constexpr (HAS_GT) prefetch_tmap(&maps.tk), prefetch_tmap(&maps.tv), prefetch_tmap(&maps.tq), prefetch_tmap(&maps.g);
-    }
-    struct Stat {
-      float lse[2], delta[2], mu[2], eps[2], cterm[2];
-    };
-    int g = 0, kact = 0;
-    bool ok = true;
-    FItem it;
-    for (int k = 0; ok && k < k_max; ++k) {
-      if (!get_item(k, it) || it.n_sub == 0) continue;
-      // The own tiles are single-buffered: every MMA that reads the previous item's must be complete.
-      const int oset = kact % C::OWN_BUFS, ouse = kact / C::OWN_BUFS;  // set of own tiles and how often it was used
-      if (ouse > 0 && !mbar_wait_backoff(own_free + oset, (ouse - 1) & 1, ab, kAbortBwdOwn)) break;
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    if (warp == 0) {
+      // ------------------------------------------------------------------ TMA producer + per-query statistics
       if (lane == 0) {
-        unsigned char* dst = sOwn + oset * C::OWN_SET_BYTES;
-        uint64_t* full = own_full + oset;
-        mbar_expect_tx(full, C::N_OWN * C::OWN_BYTES);
-        tma_load_4d(dst + C::SLOT_K * C::OWN_BYTES, &maps.k, full, 0, it.own0, it.h, it.b);
-        tma_load_4d(dst + C::SLOT_V * C::OWN_BYTES, &maps.v, full, 0, it.own0, it.h, it.b);
-        if constexpr (HAS_GT) {
-          tma_load_4d(dst + C::SLOT_TK * C::OWN_BYTES, &maps.tk, full, 0, it.own0, it.h, it.b);
-          tma_load_4d(dst + C::SLOT_TV * C::OWN_BYTES, &maps.tv, full, 0, it.own0, it.h, it.b);
-        }
+        prefetch_tmap(&maps.k), prefetch_tmap(&maps.v), prefetch_tmap(&maps.q);
+        if constexpr (HAS_GO) prefetch_tmap(&maps.go);
+        if constexpr (HAS_GT) prefetch_tmap(&maps.tk), prefetch_tmap(&maps.tv), prefetch_tmap(&maps.tq), prefetch_tmap(&maps.g);
       }
-      const size_t stat_off = (size_t)it.bh * L;
-      // lane l holds the statistics of queries 2l, 2l+1 of a sub-tile; fetched one sub-tile ahead of their use
-      auto load_stats = [&](int s, Stat& r) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          r.lse[e] = INFINITY, r.delta[e] = r.mu[e] = r.eps[e] = r.cterm[e] = 0.f;
-          const int i = it.loop_begin + s * BL + 2 * lane + e;
-          if (s < it.n_sub && i < L) {
-            r.lse[e] = a.lse[stat_off + i];
-            r.delta[e] = a.delta[stat_off + i];
-            if constexpr (HAS_GT) {
-              r.mu[e] = a.mu[stat_off + i];
-              r.eps[e] = a.eps[stat_off + i];
-              r.cterm[e] = a.cterm[stat_off + i];
-            }
-          }
-        }
+      struct Stat {
+        float lse[2], delta[2], mu[2], eps[2], cterm[2];
       };
-      // One sub-tile: its tiles, the loads of the next one's statistics, and its own, which arrived meanwhile.  (Two names that
-      // take turns: a copy from one to the other would wait for the loads, and the next tiles with it.)
-      auto sub_tile = [&](int s, const Stat& cur, Stat& nxt) -> bool {
-        const int st = g % STAGES;
-        if (!mbar_wait_backoff<32>(loop_empty + st, ((g / STAGES) & 1) ^ 1, ab, kAbortBwdLoopEmpty)) return false;
-        const int l0 = it.loop_begin + s * BL;
-        if (lane == 0) {
-          unsigned char* base = sRing + st * C::STAGE_BYTES;
-          mbar_expect_tx(loop_full + st, C::STAGE_BYTES);
-          tma_load_4d(base + C::SLOT_Q * C::LOOP_BYTES, &maps.q, loop_full + st, 0, l0, it.h, it.b);
-          if constexpr (HAS_GT) tma_load_4d(base + C::SLOT_TQ * C::LOOP_BYTES, &maps.tq, loop_full + st, 0, l0, it.h, it.b);
-          if constexpr (!C::TWO_RINGS) {
-            if constexpr (HAS_GO) tma_load_4d(base + C::SLOT_GO * C::LOOP_BYTES, &maps.go, loop_full + st, 0, l0, it.h, it.b);
-            if constexpr (HAS_GT) tma_load_4d(base + C::SLOT_G * C::LOOP_BYTES, &maps.g, loop_full + st, 0, l0, it.h, it.b);
-          }
-        }
-        const int gst = g % GSTAGES;
-        if constexpr (C::TWO_RINGS) {
-          if (!mbar_wait_backoff<32>(g_empty + gst, ((g / GSTAGES) & 1) ^ 1, ab, kAbortBwdLoopEmpty)) return false;
-          if (lane == 0) {
-            unsigned char* base = sG + gst * C::G_STAGE_BYTES;
-            mbar_expect_tx(g_full + gst, C::G_STAGE_BYTES);
-            tma_load_4d(base + C::SLOT_G * C::LOOP_BYTES, &maps.g, g_full + gst, 0, l0, it.h, it.b);
-            tma_load_4d(base + C::SLOT_GO * C::LOOP_BYTES, &maps.go, g_full + gst, 0, l0, it.h, it.b);
-          }
-        }
-        load_stats(s + 1, nxt);
-        // negated and stored pairwise for the packed arithmetic:
-        //   float4 A = (-lse0, -lse1, -mu0, -mu1), float4 B = (-eps0, -eps1, -sub0, -sub1)
-        float4* dst = sStat + (gst * (BL / 2) + lane) * 2;
-        dst[0] = make_float4(-cur.lse[0], -cur.lse[1], -cur.mu[0], -cur.mu[1]);
-        dst[1] = make_float4(-cur.eps[0], -cur.eps[1], -(cur.delta[0] + cur.cterm[0] + cur.eps[0] * cur.mu[0]),
-                             -(cur.delta[1] + cur.cterm[1] + cur.eps[1] * cur.mu[1]));
-        __syncwarp();
-        if (lane == 0) mbar_arrive(stat_full + gst);
-        ++g;
-        return true;
-      };
-      Stat s0, s1;
-      load_stats(0, s0);
-      for (int s = 0; ok && s < it.n_sub; s += 2) {
-        ok = sub_tile(s, s0, s1);
-        if (ok && s + 1 < it.n_sub) ok = sub_tile(s + 1, s1, s0);
-      }
-      ++kact;
-    }
-  } else {
-    // The issuing warps stay converged and let one lane issue (mbar_wait_warp), at most eight instructions in a row: the operands
-    // of sixteen are computed ahead, and those uniform registers spill.
-    {
-      constexpr uint32_t idesc_sc = make_idesc(Fmt<T>::kIdesc, OWN, BL, 0, 0);       // 128 x 64 scores
-      constexpr uint32_t idesc_sc2 = make_idesc(Fmt<T>::kIdesc, OWN, 2 * BL, 0, 0);  // 128 x 128: [S | tS]
-      constexpr uint32_t idesc_kv = make_idesc(Fmt<T>::kIdesc, OWN, D, 0, 1);        // dK, dV: 128 x 64, B MN-major
-      constexpr uint32_t idesc_dq = make_idesc(Fmt<T>::kIdesc, BL, D, 1, 1);         // dQ: 64 x 64, A and B MN-major
-      // MN-major operands made of one 64-element chunk: the leading offset is not used (any value), 8-row groups 1024 B
-      constexpr uint32_t kLoMN = (uint32_t)(8192 >> 4) << 16;
-      constexpr uint32_t OWN16 = C::OWN_BYTES >> 4, LOOP16 = C::LOOP_BYTES >> 4, OUT16 = C::OUT_BYTES >> 4,
-                         STAGE16 = C::STAGE_BYTES >> 4;
-      const uint32_t own_k0 = kDescLo | (smem_u32(sOwn) >> 4);    // own tiles (first set) as K-major A operands
-      const uint32_t own_mn0 = kLoMN | (smem_u32(sOwn) >> 4);     // ... as MN-major B operands (dQ)
-      constexpr uint32_t OWNSET16 = C::OWN_SET_BYTES >> 4;
-      const uint32_t ring_k = kDescLo | (smem_u32(sRing) >> 4);  // streamed tiles as K-major B operands (scores)
-      const uint32_t ring_mn = kLoMN | (smem_u32(sRing) >> 4);   // ... as MN-major B operands (dK, dV)
-      constexpr uint32_t GSTAGE16 = C::G_STAGE_BYTES >> 4;       // G and gO: a ring of their own, or beside Q
-      const uint32_t gring_k = kDescLo | (smem_u32(sG) >> 4), gring_mn = kLoMN | (smem_u32(sG) >> 4);
-      const uint32_t out_k = kDescLo | (smem_u32(sOut) >> 4);    // elementwise results as K-major A operands (dK, dV)
-      const uint32_t out_mn = kLoMN | (smem_u32(sOut) >> 4);     // ... as MN-major A operands (dQ)
       int g = 0, kact = 0;
       bool ok = true;
       FItem it;
-      if (warp == 1) {
-        // ---------------------------------------------------------------- scores
-        uint32_t own_k = own_k0;  // this item's set
-        auto score = [&](uint32_t col, uint32_t own_slot, uint32_t b_lo, uint32_t id, bool first) {
-          const uint32_t a_lo = own_k + own_slot * OWN16;
-          if (first)
-            umma_ss_lo<false>(tmem + col, a_lo, b_lo, id);
-          else
-            umma_ss_lo<true>(tmem + col, a_lo, b_lo, id);
+      for (int k = 0; ok && k < k_max; ++k) {
+        if (!get_item(k, it) || it.n_sub == 0) continue;
+        // The own tiles are single-buffered: every MMA that reads the previous item's must be complete.
+        const int oset = kact % C::OWN_BUFS, ouse = kact / C::OWN_BUFS;  // set of own tiles and how often it was used
+        if (ouse > 0 && !mbar_wait_backoff(own_free + oset, (ouse - 1) & 1, ab, kAbortBwdOwn)) break;
+        if (lane == 0) {
+          unsigned char* dst = sOwn + oset * C::OWN_SET_BYTES;
+          uint64_t* full = own_full + oset;
+          mbar_expect_tx(full, C::N_OWN * C::OWN_BYTES);
+          tma_load_4d(dst + C::SLOT_K * C::OWN_BYTES, &maps.k, full, 0, it.own0, it.h, it.b);
+          tma_load_4d(dst + C::SLOT_V * C::OWN_BYTES, &maps.v, full, 0, it.own0, it.h, it.b);
+          if constexpr (HAS_GT) {
+            tma_load_4d(dst + C::SLOT_TK * C::OWN_BYTES, &maps.tk, full, 0, it.own0, it.h, it.b);
+            tma_load_4d(dst + C::SLOT_TV * C::OWN_BYTES, &maps.tv, full, 0, it.own0, it.h, it.b);
+          }
+        }
+        const size_t stat_off = (size_t)it.bh * L;
+        // lane l holds the statistics of queries 2l, 2l+1 of a sub-tile; fetched one sub-tile ahead of their use
+        auto load_stats = [&](int s, Stat& r) {
 #pragma unroll
-          for (int ks = 1; ks < D / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 2, id);
-        };
-        for (int k = 0; ok && k < k_max; ++k) {
-          if (!get_item(k, it) || it.n_sub == 0) continue;
-          const int oset = kact % C::OWN_BUFS;
-          if (!mbar_wait_warp(own_full + oset, (kact / C::OWN_BUFS) & 1, ab, kAbortBwdOwn)) break;
-          own_k = own_k0 + oset * OWNSET16;
-          for (int s = 0; s < it.n_sub; ++s, ++g) {
-            const int st = g % STAGES;
-            if (!mbar_wait_warp(loop_full + st, (g / STAGES) & 1, ab, kAbortBwdLoopFull) ||
-                (g > 0 && !mbar_wait_warp(s_free, (g - 1) & 1, ab, kAbortBwdSFull))) {
-              ok = false;
-              break;
+          for (int e = 0; e < 2; ++e) {
+            r.lse[e] = INFINITY, r.delta[e] = r.mu[e] = r.eps[e] = r.cterm[e] = 0.f;
+            const int i = it.loop_begin + s * BL + 2 * lane + e;
+            if (s < it.n_sub && i < L) {
+              r.lse[e] = a.lse[stat_off + i];
+              r.delta[e] = a.delta[stat_off + i];
+              if constexpr (HAS_GT) {
+                r.mu[e] = a.mu[stat_off + i];
+                r.eps[e] = a.eps[stat_off + i];
+                r.cterm[e] = a.cterm[stat_off + i];
+              }
             }
-            tc_fence_after();
-            const uint32_t lp = ring_k + st * STAGE16;
-            const uint32_t lg = C::TWO_RINGS ? gring_k + (g % GSTAGES) * GSTAGE16 : lp;
-            auto from_q = [&]() {
-              if constexpr (HAS_GT) {
-                score(C::COL_S, C::SLOT_K, lp + C::SLOT_Q * LOOP16, idesc_sc2, true);    // [S | tS] = K [Q ; tQ]^T
-                score(C::COL_TS, C::SLOT_TK, lp + C::SLOT_Q * LOOP16, idesc_sc, false);  // tS += tK Q^T
-              } else {
-                score(C::COL_S, C::SLOT_K, lp + C::SLOT_Q * LOOP16, idesc_sc, true);  // S = K Q^T
-              }
-            };
-            auto from_g = [&]() {
-              if constexpr (HAS_GT) {
-                score(C::COL_E, C::SLOT_V, lg + C::SLOT_G * LOOP16, HAS_GO ? idesc_sc2 : idesc_sc, true);  // E = V G^T; [E | FP] = V [G ; gO]^T
-                score(C::COL_FP, C::SLOT_TV, lg + C::SLOT_G * LOOP16, idesc_sc, !HAS_GO);                  // FP (+)= tV G^T
-              } else {
-                score(C::COL_FP, C::SLOT_V, lg + C::SLOT_GO * LOOP16, idesc_sc, true);  // FP = V gO^T
-              }
-              tc_commit(s_full);
-              tc_commit(C::TWO_RINGS ? g_empty + g % GSTAGES : loop_empty + st);
-              if (s == it.n_sub - 1) tc_commit(own_free + oset);
-            };
-            if constexpr (C::TWO_RINGS) {
-              if (elect_one()) {
-                from_q();
-                tc_commit(loop_empty + st);
-              }
-              if (!mbar_wait_warp(g_full + g % GSTAGES, (g / GSTAGES) & 1, ab, kAbortBwdLoopFull)) {
+          }
+        };
+        // One sub-tile: its tiles, the loads of the next one's statistics, and its own, which arrived meanwhile.  (Two names that
+        // take turns: a copy from one to the other would wait for the loads, and the next tiles with it.)
+        auto sub_tile = [&](int s, const Stat& cur, Stat& nxt) -> bool {
+          const int st = g % STAGES;
+          if (!mbar_wait_backoff<32>(loop_empty + st, ((g / STAGES) & 1) ^ 1, ab, kAbortBwdLoopEmpty)) return false;
+          const int l0 = it.loop_begin + s * BL;
+          if (lane == 0) {
+            unsigned char* base = sRing + st * C::STAGE_BYTES;
+            mbar_expect_tx(loop_full + st, C::STAGE_BYTES);
+            tma_load_4d(base + C::SLOT_Q * C::LOOP_BYTES, &maps.q, loop_full + st, 0, l0, it.h, it.b);
+            if constexpr (HAS_GT) tma_load_4d(base + C::SLOT_TQ * C::LOOP_BYTES, &maps.tq, loop_full + st, 0, l0, it.h, it.b);
+            if constexpr (!C::TWO_RINGS) {
+              if constexpr (HAS_GO) tma_load_4d(base + C::SLOT_GO * C::LOOP_BYTES, &maps.go, loop_full + st, 0, l0, it.h, it.b);
+              if constexpr (HAS_GT) tma_load_4d(base + C::SLOT_G * C::LOOP_BYTES, &maps.g, loop_full + st, 0, l0, it.h, it.b);
+            }
+          }
+          const int gst = g % GSTAGES;
+          if constexpr (C::TWO_RINGS) {
+            if (!mbar_wait_backoff<32>(g_empty + gst, ((g / GSTAGES) & 1) ^ 1, ab, kAbortBwdLoopEmpty)) return false;
+            if (lane == 0) {
+              unsigned char* base = sG + gst * C::G_STAGE_BYTES;
+              mbar_expect_tx(g_full + gst, C::G_STAGE_BYTES);
+              tma_load_4d(base + C::SLOT_G * C::LOOP_BYTES, &maps.g, g_full + gst, 0, l0, it.h, it.b);
+              tma_load_4d(base + C::SLOT_GO * C::LOOP_BYTES, &maps.go, g_full + gst, 0, l0, it.h, it.b);
+            }
+          }
+          load_stats(s + 1, nxt);
+          // negated and stored pairwise for the packed arithmetic:
+          //   float4 A = (-lse0, -lse1, -mu0, -mu1), float4 B = (-eps0, -eps1, -sub0, -sub1)
+          float4* dst = sStat + (gst * (BL / 2) + lane) * 2;
+          dst[0] = make_float4(-cur.lse[0], -cur.lse[1], -cur.mu[0], -cur.mu[1]);
+          dst[1] = make_float4(-cur.eps[0], -cur.eps[1], -(cur.delta[0] + cur.cterm[0] + cur.eps[0] * cur.mu[0]),
+                               -(cur.delta[1] + cur.cterm[1] + cur.eps[1] * cur.mu[1]));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(stat_full + gst);
+          ++g;
+          return true;
+        };
+        Stat s0, s1;
+        load_stats(0, s0);
+        for (int s = 0; ok && s < it.n_sub; s += 2) {
+          ok = sub_tile(s, s0, s1);
+          if (ok && s + 1 < it.n_sub) ok = sub_tile(s + 1, s1, s0);
+        }
+        ++kact;
+      }
+    } else {
+      // The issuing warps stay converged and let one lane issue (mbar_wait_warp), at most eight instructions in a row: the operands
+      // of sixteen are computed ahead, and those uniform registers spill.
+      {
+        constexpr uint32_t idesc_sc = make_idesc(Fmt<T>::kIdesc, OWN, BL, 0, 0);       // 128 x 64 scores
+        constexpr uint32_t idesc_sc2 = make_idesc(Fmt<T>::kIdesc, OWN, 2 * BL, 0, 0);  // 128 x 128: [S | tS]
+        constexpr uint32_t idesc_kv = make_idesc(Fmt<T>::kIdesc, OWN, D, 0, 1);        // dK, dV: 128 x 64, B MN-major
+        constexpr uint32_t idesc_dq = make_idesc(Fmt<T>::kIdesc, BL, D, 1, 1);         // dQ: 64 x 64, A and B MN-major
+        // MN-major operands made of one 64-element chunk: the leading offset is not used (any value), 8-row groups 1024 B
+        constexpr uint32_t kLoMN = (uint32_t)(8192 >> 4) << 16;
+        constexpr uint32_t OWN16 = C::OWN_BYTES >> 4, LOOP16 = C::LOOP_BYTES >> 4, OUT16 = C::OUT_BYTES >> 4,
+                           STAGE16 = C::STAGE_BYTES >> 4;
+        const uint32_t own_k0 = kDescLo | (smem_u32(sOwn) >> 4);    // own tiles (first set) as K-major A operands
+        const uint32_t own_mn0 = kLoMN | (smem_u32(sOwn) >> 4);     // ... as MN-major B operands (dQ)
+        constexpr uint32_t OWNSET16 = C::OWN_SET_BYTES >> 4;
+        const uint32_t ring_k = kDescLo | (smem_u32(sRing) >> 4);  // streamed tiles as K-major B operands (scores)
+        const uint32_t ring_mn = kLoMN | (smem_u32(sRing) >> 4);   // ... as MN-major B operands (dK, dV)
+        constexpr uint32_t GSTAGE16 = C::G_STAGE_BYTES >> 4;       // G and gO: a ring of their own, or beside Q
+        const uint32_t gring_k = kDescLo | (smem_u32(sG) >> 4), gring_mn = kLoMN | (smem_u32(sG) >> 4);
+        const uint32_t out_k = kDescLo | (smem_u32(sOut) >> 4);    // elementwise results as K-major A operands (dK, dV)
+        const uint32_t out_mn = kLoMN | (smem_u32(sOut) >> 4);     // ... as MN-major A operands (dQ)
+        int g = 0, kact = 0;
+        bool ok = true;
+        FItem it;
+        if (warp == 1) {
+          // ---------------------------------------------------------------- scores
+          uint32_t own_k = own_k0;  // this item's set
+          auto score = [&](uint32_t col, uint32_t own_slot, uint32_t b_lo, uint32_t id, bool first) {
+            const uint32_t a_lo = own_k + own_slot * OWN16;
+            if (first)
+              umma_ss_lo<false>(tmem + col, a_lo, b_lo, id);
+            else
+              umma_ss_lo<true>(tmem + col, a_lo, b_lo, id);
+#pragma unroll
+            for (int ks = 1; ks < D / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 2, id);
+          };
+          for (int k = 0; ok && k < k_max; ++k) {
+            if (!get_item(k, it) || it.n_sub == 0) continue;
+            const int oset = kact % C::OWN_BUFS;
+            if (!mbar_wait_warp(own_full + oset, (kact / C::OWN_BUFS) & 1, ab, kAbortBwdOwn)) break;
+            own_k = own_k0 + oset * OWNSET16;
+            for (int s = 0; s < it.n_sub; ++s, ++g) {
+              const int st = g % STAGES;
+              if (!mbar_wait_warp(loop_full + st, (g / STAGES) & 1, ab, kAbortBwdLoopFull) ||
+                  (g > 0 && !mbar_wait_warp(s_free, (g - 1) & 1, ab, kAbortBwdSFull))) {
                 ok = false;
                 break;
               }
               tc_fence_after();
-              if (elect_one()) from_g();
-            } else {
-              if (elect_one()) from_q();
-              if (elect_one()) from_g();
+              const uint32_t lp = ring_k + st * STAGE16;
+              const uint32_t lg = C::TWO_RINGS ? gring_k + (g % GSTAGES) * GSTAGE16 : lp;
+              auto from_q = [&]() {
+                if constexpr (HAS_GT) {
+                  score(C::COL_S, C::SLOT_K, lp + C::SLOT_Q * LOOP16, idesc_sc2, true);    // [S | tS] = K [Q ; tQ]^T
+                  score(C::COL_TS, C::SLOT_TK, lp + C::SLOT_Q * LOOP16, idesc_sc, false);  // tS += tK Q^T
+                } else {
+                  score(C::COL_S, C::SLOT_K, lp + C::SLOT_Q * LOOP16, idesc_sc, true);  // S = K Q^T
+                }
+              };
+              auto from_g = [&]() {
+                if constexpr (HAS_GT) {
+                  score(C::COL_E, C::SLOT_V, lg + C::SLOT_G * LOOP16, HAS_GO ? idesc_sc2 : idesc_sc, true);  // E = V G^T; [E | FP] = V [G ; gO]^T
+                  score(C::COL_FP, C::SLOT_TV, lg + C::SLOT_G * LOOP16, idesc_sc, !HAS_GO);                  // FP (+)= tV G^T
+                } else {
+                  score(C::COL_FP, C::SLOT_V, lg + C::SLOT_GO * LOOP16, idesc_sc, true);  // FP = V gO^T
+                }
+                tc_commit(s_full);
+                tc_commit(C::TWO_RINGS ? g_empty + g % GSTAGES : loop_empty + st);
+                if (s == it.n_sub - 1) tc_commit(own_free + oset);
+              };
+              if constexpr (C::TWO_RINGS) {
+                if (elect_one()) {
+                  from_q();
+                  tc_commit(loop_empty + st);
+                }
+                if (!mbar_wait_warp(g_full + g % GSTAGES, (g / GSTAGES) & 1, ab, kAbortBwdLoopFull)) {
+                  ok = false;
+                  break;
+                }
+                tc_fence_after();
+                if (elect_one()) from_g();
+              } else {
+                if (elect_one()) from_q();
+                if (elect_one()) from_g();
+              }
             }
+            if (!ok) break;
+            ++kact;
           }
-          if (!ok) break;
-          ++kact;
-        }
-      } else if (warp == 2) {
-        // ---------------------------------------------------------------- dK, dV
-        // out (+)= result tile (A, K-major: 128 keys x 64 queries) x streamed tile (B, MN-major: 64 queries x 64)
-        uint32_t ob16 = 0;  // result buffer of the sub-tile, in 16-byte units
-        auto outer = [&](uint32_t col, uint32_t out_slot, uint32_t b_lo, uint32_t accumulate) {
-          const uint32_t a_lo = out_k + ob16 + out_slot * OUT16;
-          mma_ss_dyn(tmem + col, a_lo, b_lo, idesc_kv, accumulate);
+        } else if (warp == 2) {
+          // ---------------------------------------------------------------- dK, dV
+          // out (+)= result tile (A, K-major: 128 keys x 64 queries) x streamed tile (B, MN-major: 64 queries x 64)
+          uint32_t ob16 = 0;  // result buffer of the sub-tile, in 16-byte units
+          auto outer = [&](uint32_t col, uint32_t out_slot, uint32_t b_lo, uint32_t accumulate) {
+            const uint32_t a_lo = out_k + ob16 + out_slot * OUT16;
+            mma_ss_dyn(tmem + col, a_lo, b_lo, idesc_kv, accumulate);
 #pragma unroll
-          for (int ks = 1; ks < BL / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 128, idesc_kv);
-        };
-        // out (+)= packed operand (A, TMEM: 8 columns per 16 queries) x streamed tile (B, MN-major)
-        auto outer_t = [&](uint32_t col, uint32_t a_col, uint32_t b_lo, uint32_t accumulate) {
-          umma_ts_lo_dyn(tmem + col, tmem + a_col, b_lo, idesc_kv, accumulate);
+            for (int ks = 1; ks < BL / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 128, idesc_kv);
+          };
+          // out (+)= packed operand (A, TMEM: 8 columns per 16 queries) x streamed tile (B, MN-major)
+          auto outer_t = [&](uint32_t col, uint32_t a_col, uint32_t b_lo, uint32_t accumulate) {
+            umma_ts_lo_dyn(tmem + col, tmem + a_col, b_lo, idesc_kv, accumulate);
 #pragma unroll
-          for (int ks = 1; ks < BL / 16; ++ks) umma_ts_lo<true>(tmem + col, tmem + a_col + ks * 8, b_lo + ks * 128, idesc_kv);
-        };
-        for (int k = 0; ok && k < k_max; ++k) {
-          if (!get_item(k, it) || it.n_sub == 0) continue;
-          for (int s = 0; s < it.n_sub; ++s, ++g) {
-            const int st = g % STAGES;
-            if (!mbar_wait_warp(p_full + (g & 1), (g >> 1) & 1, ab, kAbortBwdPFull) ||
-                (s == 0 && kact > 0 && !mbar_wait_warp(acc_free, (kact - 1) & 1, ab, kAbortBwdDone))) {
-              ok = false;
-              break;
+            for (int ks = 1; ks < BL / 16; ++ks) umma_ts_lo<true>(tmem + col, tmem + a_col + ks * 8, b_lo + ks * 128, idesc_kv);
+          };
+          for (int k = 0; ok && k < k_max; ++k) {
+            if (!get_item(k, it) || it.n_sub == 0) continue;
+            for (int s = 0; s < it.n_sub; ++s, ++g) {
+              const int st = g % STAGES;
+              if (!mbar_wait_warp(p_full + (g & 1), (g >> 1) & 1, ab, kAbortBwdPFull) ||
+                  (s == 0 && kact > 0 && !mbar_wait_warp(acc_free, (kact - 1) & 1, ab, kAbortBwdDone))) {
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+              const int ob = g % C::N_OBUF;
+              ob16 = ob * (C::OBUF_BYTES >> 4);
+              const uint32_t lp = ring_mn + st * STAGE16;
+              const uint32_t lg = C::TWO_RINGS ? gring_mn + (g % GSTAGES) * GSTAGE16 : lp;
+              const uint32_t acc = s > 0;
+              if (elect_one()) {
+                outer(C::COL_DK, C::OUT_GS, lp + C::SLOT_Q * LOOP16, acc);                        // dK += gS^T Q
+                if constexpr (HAS_GT) outer(C::COL_DK, C::OUT_GT, lp + C::SLOT_TQ * LOOP16, 1);  // dK += gtS^T tQ
+                if constexpr (C::TWO_RINGS) tc_commit(loop_empty + st);
+              }
+              if (elect_one()) {
+                if constexpr (HAS_GT) {
+                  outer_t(C::COL_DV, C::COL_AV, lg + C::SLOT_G * LOOP16, acc);  // dV += A^T G
+                  if constexpr (HAS_GO) outer_t(C::COL_DV, C::COL_P, lg + C::SLOT_GO * LOOP16, 1);  // dV += P^T gO
+                } else {
+                  outer_t(C::COL_DV, C::COL_P, lg + C::SLOT_GO * LOOP16, acc);  // dV += P^T gO
+                }
+                tc_commit(C::TWO_RINGS ? g_empty + g % GSTAGES : loop_empty + st);
+                tc_commit(out_free + ob);
+                tc_commit(av_free);
+                if (s == it.n_sub - 1) tc_commit(done);
+              }
             }
-            tc_fence_after();
-            const int ob = g % C::N_OBUF;
-            ob16 = ob * (C::OBUF_BYTES >> 4);
-            const uint32_t lp = ring_mn + st * STAGE16;
-            const uint32_t lg = C::TWO_RINGS ? gring_mn + (g % GSTAGES) * GSTAGE16 : lp;
-            const uint32_t acc = s > 0;
-            if (elect_one()) {
-            outer(C::COL_DK, C::OUT_GS, lp + C::SLOT_Q * LOOP16, acc);                        // dK += gS^T Q
-            if constexpr (HAS_GT) outer(C::COL_DK, C::OUT_GT, lp + C::SLOT_TQ * LOOP16, 1);  // dK += gtS^T tQ
-            if constexpr (C::TWO_RINGS) tc_commit(loop_empty + st);
-            }
-            if (elect_one()) {
-            if constexpr (HAS_GT) {
-              outer_t(C::COL_DV, C::COL_AV, lg + C::SLOT_G * LOOP16, acc);  // dV += A^T G
-              if constexpr (HAS_GO) outer_t(C::COL_DV, C::COL_P, lg + C::SLOT_GO * LOOP16, 1);  // dV += P^T gO
-            } else {
-              outer_t(C::COL_DV, C::COL_P, lg + C::SLOT_GO * LOOP16, acc);  // dV += P^T gO
-            }
-            tc_commit(C::TWO_RINGS ? g_empty + g % GSTAGES : loop_empty + st);
-            tc_commit(out_free + ob);
-            tc_commit(av_free);
-            if (s == it.n_sub - 1) tc_commit(done);
-            }
+            if (!ok) break;
+            ++kact;
           }
-          if (!ok) break;
-          ++kact;
-        }
-      } else {
-        // ---------------------------------------------------------------- dQ of the sub-tile
-        // dQ (+)= result tile (A, MN-major: 64 queries x 128 keys) x own tile (B, MN-major: 128 keys x 64)
-        uint32_t ob16 = 0;
-        uint32_t own_mn = own_mn0;  // this item's set
-        auto inner = [&](uint32_t col, uint32_t out_slot, uint32_t own_slot, bool first) {
-          const uint32_t a_lo = out_mn + ob16 + out_slot * OUT16, b_lo = own_mn + own_slot * OWN16;
-          if (first)
-            umma_ss_lo<false>(tmem + col, a_lo, b_lo, idesc_dq);
-          else
-            umma_ss_lo<true>(tmem + col, a_lo, b_lo, idesc_dq);
+        } else {
+          // ---------------------------------------------------------------- dQ of the sub-tile
+          // dQ (+)= result tile (A, MN-major: 64 queries x 128 keys) x own tile (B, MN-major: 128 keys x 64)
+          uint32_t ob16 = 0;
+          uint32_t own_mn = own_mn0;  // this item's set
+          auto inner = [&](uint32_t col, uint32_t out_slot, uint32_t own_slot, bool first) {
+            const uint32_t a_lo = out_mn + ob16 + out_slot * OUT16, b_lo = own_mn + own_slot * OWN16;
+            if (first)
+              umma_ss_lo<false>(tmem + col, a_lo, b_lo, idesc_dq);
+            else
+              umma_ss_lo<true>(tmem + col, a_lo, b_lo, idesc_dq);
 #pragma unroll
-          for (int ks = 1; ks < OWN / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 128, b_lo + ks * 128, idesc_dq);
-        };
-        for (int k = 0; ok && k < k_max; ++k) {
-          if (!get_item(k, it) || it.n_sub == 0) continue;
-          own_mn = own_mn0 + (kact % C::OWN_BUFS) * OWNSET16;
-          for (int s = 0; s < it.n_sub; ++s, ++g) {
-            if (!mbar_wait_warp(p_full + (g & 1), (g >> 1) & 1, ab, kAbortBwdPFull) ||
-                (g >= 1 && !mbar_wait_warp(dq_free, (g - 1) & 1, ab, kAbortBwdDone))) {
-              ok = false;
-              break;
+            for (int ks = 1; ks < OWN / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 128, b_lo + ks * 128, idesc_dq);
+          };
+          for (int k = 0; ok && k < k_max; ++k) {
+            if (!get_item(k, it) || it.n_sub == 0) continue;
+            own_mn = own_mn0 + (kact % C::OWN_BUFS) * OWNSET16;
+            for (int s = 0; s < it.n_sub; ++s, ++g) {
+              if (!mbar_wait_warp(p_full + (g & 1), (g >> 1) & 1, ab, kAbortBwdPFull) ||
+                  (g >= 1 && !mbar_wait_warp(dq_free, (g - 1) & 1, ab, kAbortBwdDone))) {
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+              const int ob = g % C::N_OBUF;
+              ob16 = ob * (C::OBUF_BYTES >> 4);
+              const uint32_t col = C::COL_DQ;
+              if (elect_one()) {
+                inner(col, C::OUT_GS, C::SLOT_K, true);                       // dQ = gS K
+              }
+              if (elect_one()) {
+                if constexpr (HAS_GT) inner(col, C::OUT_GT, C::SLOT_TK, false);  // dQ += gtS tK
+                tc_commit(dq_full);
+                tc_commit(out_free + ob);
+                if (s == it.n_sub - 1) tc_commit(own_free + kact % C::OWN_BUFS);
+              }
             }
-            tc_fence_after();
-            const int ob = g % C::N_OBUF;
-            ob16 = ob * (C::OBUF_BYTES >> 4);
-            const uint32_t col = C::COL_DQ;
-            if (elect_one()) {
-            inner(col, C::OUT_GS, C::SLOT_K, true);                       // dQ = gS K
-            }
-            if (elect_one()) {
-            if constexpr (HAS_GT) inner(col, C::OUT_GT, C::SLOT_TK, false);  // dQ += gtS tK
-            tc_commit(dq_full);
-            tc_commit(out_free + ob);
-            if (s == it.n_sub - 1) tc_commit(own_free + kact % C::OWN_BUFS);
-            }
+            if (!ok) break;
+            ++kact;
           }
-          if (!ok) break;
-          ++kact;
         }
       }
     }
-  }
   } else if (warp < 12) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");
     // ------------------------------------------------------------------ elementwise warpgroups

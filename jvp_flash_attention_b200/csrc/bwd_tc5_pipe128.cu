@@ -40,8 +40,8 @@ template <bool OWN_KEYS, bool HAS_GO, bool HAS_GT>
 struct BwdPipeCfg {
   static constexpr int D = 128;
   static constexpr int OWN = 128;
-  // Rows of a loop tile.  An MMA instruction costs about 58 cycles whatever its N up to 64, so wider tiles mean fewer
-  // instructions per column.  Own keys: dK | dV take 256 TMEM columns, which leaves two score buffers of 4 x 32; own
+  // Rows of a loop tile.  An MMA instruction of N = 32 costs 40 cycles and one of N = 64 48 (mbar_wait_warp's comment), so wider tiles
+  // cost less per column.  Own keys: dK | dV take 256 TMEM columns, which leaves two score buffers of 4 x 32; own
   // queries: dQ takes 128, which leaves two buffers of 4 x 48.
   static constexpr int BL = OWN_KEYS ? 32 : 48;
   static constexpr int NP = BL / 16;                // 16-column pieces = elementwise warpgroups
@@ -340,7 +340,8 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
     }
   } else if (warp == 1 || warp == C::WARP_ISSUER2) {
     // ------------------------------------------------------------------ MMA issuers
-    // Two converged warps, one elected lane each (mbar_wait_warp).  The first issuer forms [S | TS] and, after the elementwise threads, the outputs; the second forms [E | FP].
+    // Two converged warps, one elected lane each (mbar_wait_warp).  The first issuer forms [S | TS] and, after the elementwise
+    // threads, the outputs; the second forms [E | FP].
     // Everything that reads what the elementwise threads write (they write over S and TS only) is issued by the first
     // thread, after that thread's own scores into the same buffer two tiles earlier and before its next ones: the
     // tensor pipe keeps one thread's instructions in order, so no barrier between the two issuers is needed.  The
@@ -371,16 +372,16 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
         const uint32_t sc = tmem + (t & 1) * C::SC_COLS;
         constexpr uint32_t id = HAS_GT ? idesc_n2 : idesc_n1;
         if (elect_one()) {
-        umma_ss_lo<false>(sc + C::COL_S, a_lo0 + a_off(0, 0), lx + b_off(C::X_HALF, 0, 0), id);
+          umma_ss_lo<false>(sc + C::COL_S, a_lo0 + a_off(0, 0), lx + b_off(C::X_HALF, 0, 0), id);
 #pragma unroll
-        for (int ks = 1; ks < 8; ++ks)
-          umma_ss_lo<true>(sc + C::COL_S, a_lo0 + a_off(0, ks), lx + b_off(C::X_HALF, 0, ks), id);
-        if constexpr (HAS_GT) {
+          for (int ks = 1; ks < 8; ++ks)
+            umma_ss_lo<true>(sc + C::COL_S, a_lo0 + a_off(0, ks), lx + b_off(C::X_HALF, 0, ks), id);
+          if constexpr (HAS_GT) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks)
-            umma_ss_lo<true>(sc + C::COL_TS, a_lo0 + a_off(1, ks), lx + b_off(C::X_HALF, 0, ks), idesc_n1);
-        }
-        tc_commit(s_full + (t & 1));
+            for (int ks = 0; ks < 8; ++ks)
+              umma_ss_lo<true>(sc + C::COL_TS, a_lo0 + a_off(1, ks), lx + b_off(C::X_HALF, 0, ks), idesc_n1);
+          }
+          tc_commit(s_full + (t & 1));
         }
         return true;
       };
@@ -400,28 +401,28 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
         constexpr uint32_t h2 = OWN_KEYS ? C::X_HALF : C::Y_HALF;
         const uint32_t sc = tmem + (t & 1) * C::SC_COLS;
         if (elect_one()) {
-        if constexpr (HAS_GT) {
-          constexpr bool wide = !OWN_KEYS || HAS_GO;  // [E | FP] in one instruction
-          umma_ss_lo<false>(sc + C::COL_E, a_lo0 + a_off(2, 0), l2 + b_off(h2, 0, 0), wide ? idesc_n2 : idesc_n1);
-#pragma unroll
-          for (int ks = 1; ks < 8; ++ks)
-            umma_ss_lo<true>(sc + C::COL_E, a_lo0 + a_off(2, ks), l2 + b_off(h2, 0, ks), wide ? idesc_n2 : idesc_n1);
-          if constexpr (OWN_KEYS || HAS_GO) {
-            umma_ss_lo<wide>(sc + C::COL_FP, a_lo0 + a_off(3, 0), l2 + b_off(h2, 0, 0), idesc_n1);
+          if constexpr (HAS_GT) {
+            constexpr bool wide = !OWN_KEYS || HAS_GO;  // [E | FP] in one instruction
+            umma_ss_lo<false>(sc + C::COL_E, a_lo0 + a_off(2, 0), l2 + b_off(h2, 0, 0), wide ? idesc_n2 : idesc_n1);
 #pragma unroll
             for (int ks = 1; ks < 8; ++ks)
-              umma_ss_lo<true>(sc + C::COL_FP, a_lo0 + a_off(3, ks), l2 + b_off(h2, 0, ks), idesc_n1);
-          }
-        } else {
-          // FP = V gO^T (own keys: own2 loop3^T) or gO V^T (own queries: own3 loop2^T)
-          constexpr int fa = OWN_KEYS ? 2 : 3, fb = OWN_KEYS ? 1 : 0;
-          umma_ss_lo<false>(sc + C::COL_FP, a_lo0 + a_off(fa, 0), l2 + b_off(h2, fb, 0), idesc_n1);
+              umma_ss_lo<true>(sc + C::COL_E, a_lo0 + a_off(2, ks), l2 + b_off(h2, 0, ks), wide ? idesc_n2 : idesc_n1);
+            if constexpr (OWN_KEYS || HAS_GO) {
+              umma_ss_lo<wide>(sc + C::COL_FP, a_lo0 + a_off(3, 0), l2 + b_off(h2, 0, 0), idesc_n1);
 #pragma unroll
-          for (int ks = 1; ks < 8; ++ks)
-            umma_ss_lo<true>(sc + C::COL_FP, a_lo0 + a_off(fa, ks), l2 + b_off(h2, fb, ks), idesc_n1);
-        }
-        if constexpr (OWN_KEYS) tc_commit(loop_empty + (t % STAGES)); else tc_commit(y_empty);
-        tc_commit(s_full + (t & 1));
+              for (int ks = 1; ks < 8; ++ks)
+                umma_ss_lo<true>(sc + C::COL_FP, a_lo0 + a_off(3, ks), l2 + b_off(h2, 0, ks), idesc_n1);
+            }
+          } else {
+            // FP = V gO^T (own keys: own2 loop3^T) or gO V^T (own queries: own3 loop2^T)
+            constexpr int fa = OWN_KEYS ? 2 : 3, fb = OWN_KEYS ? 1 : 0;
+            umma_ss_lo<false>(sc + C::COL_FP, a_lo0 + a_off(fa, 0), l2 + b_off(h2, fb, 0), idesc_n1);
+#pragma unroll
+            for (int ks = 1; ks < 8; ++ks)
+              umma_ss_lo<true>(sc + C::COL_FP, a_lo0 + a_off(fa, ks), l2 + b_off(h2, fb, ks), idesc_n1);
+          }
+          if constexpr (OWN_KEYS) tc_commit(loop_empty + (t % STAGES)); else tc_commit(y_empty);
+          tc_commit(s_full + (t & 1));
         }
         return true;
       };
@@ -443,31 +444,31 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
           const uint32_t sc = tmem + (t & 1) * C::SC_COLS;
           const uint32_t acc = t > 0;
           if (elect_one()) {
-          // Contraction step kk = NP * term + piece: rows 16 * piece .. of X tile (slot + term), operand piece at
-          // column 16 * piece + 8 * term of the accumulator it was written over.
-          // dK or dQ += gS x0 + gtS x1
-          umma_ts_lo_dyn(tmem + C::COL_OUT0, sc + C::COL_S, mx, idesc_out, acc);
+            // Contraction step kk = NP * term + piece: rows 16 * piece .. of X tile (slot + term), operand piece at
+            // column 16 * piece + 8 * term of the accumulator it was written over.
+            // dK or dQ += gS x0 + gtS x1
+            umma_ts_lo_dyn(tmem + C::COL_OUT0, sc + C::COL_S, mx, idesc_out, acc);
 #pragma unroll
-          for (int kk = 1; kk < (HAS_GT ? 2 : 1) * NP; ++kk)
-            umma_ts_lo<true>(tmem + C::COL_OUT0, sc + C::COL_S + 16 * (kk % NP) + 8 * (kk / NP), mx + kk * 128, idesc_out);
-          if constexpr (OWN_KEYS) {
-            if constexpr (HAS_GT) {
-              // dV += A G + P gO   (X slots 2, 3)
-              constexpr uint32_t o2 = (2 * C::LQ_BYTES) >> 4;
-              umma_ts_lo_dyn(tmem + C::COL_OUT1, sc + C::COL_TS, mx + o2, idesc_out, acc);
+            for (int kk = 1; kk < (HAS_GT ? 2 : 1) * NP; ++kk)
+              umma_ts_lo<true>(tmem + C::COL_OUT0, sc + C::COL_S + 16 * (kk % NP) + 8 * (kk / NP), mx + kk * 128, idesc_out);
+            if constexpr (OWN_KEYS) {
+              if constexpr (HAS_GT) {
+                // dV += A G + P gO   (X slots 2, 3)
+                constexpr uint32_t o2 = (2 * C::LQ_BYTES) >> 4;
+                umma_ts_lo_dyn(tmem + C::COL_OUT1, sc + C::COL_TS, mx + o2, idesc_out, acc);
 #pragma unroll
-              for (int kk = 1; kk < (HAS_GO ? 2 : 1) * NP; ++kk)
-                umma_ts_lo<true>(tmem + C::COL_OUT1, sc + C::COL_TS + 16 * (kk % NP) + 8 * (kk / NP), mx + o2 + kk * 128, idesc_out);
-            } else {
-              // dV += P gO   (X slot 3)
-              constexpr uint32_t o3 = (3 * C::LQ_BYTES) >> 4;
-              umma_ts_lo_dyn(tmem + C::COL_OUT1, sc + C::COL_TS + 8, mx + o3, idesc_out, acc);
+                for (int kk = 1; kk < (HAS_GO ? 2 : 1) * NP; ++kk)
+                  umma_ts_lo<true>(tmem + C::COL_OUT1, sc + C::COL_TS + 16 * (kk % NP) + 8 * (kk / NP), mx + o2 + kk * 128, idesc_out);
+              } else {
+                // dV += P gO   (X slot 3)
+                constexpr uint32_t o3 = (3 * C::LQ_BYTES) >> 4;
+                umma_ts_lo_dyn(tmem + C::COL_OUT1, sc + C::COL_TS + 8, mx + o3, idesc_out, acc);
 #pragma unroll
-              for (int kk = 1; kk < NP; ++kk)
-                umma_ts_lo<true>(tmem + C::COL_OUT1, sc + C::COL_TS + 16 * kk + 8, mx + o3 + kk * 128, idesc_out);
+                for (int kk = 1; kk < NP; ++kk)
+                  umma_ts_lo<true>(tmem + C::COL_OUT1, sc + C::COL_TS + 16 * kk + 8, mx + o3 + kk * 128, idesc_out);
+              }
             }
-          }
-          tc_commit(loop_empty + st);
+            tc_commit(loop_empty + st);
           }
         }
         if (elect_one()) tc_commit(done);

@@ -3,7 +3,8 @@
 // An fp32 number x is the sum of three bf16 numbers, hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid (24 significant bits
 // are 8 + 8 + 8, the differences are exact), and bf16 has fp32's range of exponents, so every entry keeps its precision
 // whatever else its row or column holds.  A product is the six MMAs hi*hi, hi*mid, mid*hi, mid*mid, hi*lo, lo*hi; what is left
-// out (mid*lo, lo*mid, lo*lo) is below 2^-26 of it.
+// out (mid*lo, lo*mid, lo*lo) is at most 2^-24 of it, since |mid| <= 2^-8 and |lo| <= 2^-17 of the leading bit (above 2^-26 for
+// 2.8 % of uniform pairs).  Of entries below 2^-109 bf16 no longer holds all of the lo part.
 //
 // The inputs are split once per call into a caller-owned workspace: three row-major (B*H, L, D) planes of bf16 per tensor,
 // all of them one tensor map (D, L, B*H, planes).
@@ -132,7 +133,7 @@ struct F32RowMask {
 //            L96  n16 384 16/18 31/27 55/51    bias 18/23 33/29 57/68   n16 672 bias 29/25 49/33 100/72
 //            L130 n16 387 25/20 45/31 80/59    bias 25/25 45/33 79/76   ragged boolean 25/31 49/43 82/84, n16 774 43/41 72/61 145/121
 //            L192 n16 384 27/20 51/33 94/57    bias 29/22 55/33 94/70   L512 n16 256 34/30 71/46, bias 36/42 74/65
-//   D = 128  L66  n16 320 25/23 49/39 90/82    causal 25/23 41/39 78/82  bias 25/23 49/41 90/92   ragged boolean 25/33 51/57 92/106
+//   D = 128  L66  n16 320 25/23 49/39 90/82    causal 25/23 41/39 78/82  bias 25/23 49/41 90/92, ragged boolean 25/33 51/57 92/106
 //            L96  n16 324 25/23 51/41 96/86    causal 23/22 41/41 80/88  bias 27/27 53/45 96/100, n16 642 43/31 86/53 176/111
 //            L112 n16 322 31/23 61/43 115/90   causal 29/23 47/43 96/90  bias 29/25 61/45 115/100
 //   D = 32   L192 n16 1032 22/29 41/43 84/86   causal 25/27 41/39 82/76  n16 4104 53/61 119/104 207/203  (64-row tiles fit, 128 do not)

@@ -3,7 +3,7 @@
 //
 // CTA = one 128-row query tile of one (batch, head), 384 threads:
 //   warp 0        TMA producer (one lane), owner of the TMEM allocation
-//   warp 1        MMA issuer (one lane)
+//   warp 1        MMA issuer (converged, one elected lane)
 //   warps 4..11   two warpgroups; thread <-> query row <-> TMEM lane; group w takes the keys [32 w, 32 w + 32) of a tile in the
 //                 softmax and half of the output columns in its registers
 // Shared memory: the parts of Q and tQ (K-major, 128-byte swizzle), and a ring of 16 KiB units, each one part of two tiles of
@@ -149,185 +149,185 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
   // (in the branches of the roles: ptxas holds code behind a join of the two to the smaller number)
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && n_tiles > 0) {
-      prefetch_tmap(&map);
-      auto load = [&](unsigned char* dst, uint64_t* bar, int slot, int part, int x, int y) {
-        tma_load_4d(dst, &map, bar, x, y, bh, slot * 3 + part);
-      };
-      mbar_expect_tx(q_full, (C::Q_PARTS + (DUAL ? 3 : 0)) * NSL * C::PART);
-      for (int p = 0; p < 3; ++p)
-        for (int s = 0; s < NSL; ++s)
-          for (int r = 0; r < 2; ++r) {  // rows m0 + 64 r: beyond the tensor they read as zeros
-            const int off = (p * NSL + s) * C::PART + r * C::TILE;
-            if (p < C::Q_PARTS) load(smem + C::OFF_Q + off, q_full, kSlotQ, p, 64 * s, m0 + 64 * r);
-            if constexpr (DUAL) load(smem + C::OFF_TQ + off, q_full, kSlotTQ, p, 64 * s, m0 + 64 * r);
-          }
-      int u = 0;
-      bool ok = true;
-      // one unit: n tiles of 8 KiB, the i-th from (slot_i, part, column x_i)
-      auto unit = [&](int n, int part, int y, int slot0, int x0, int slot1, int x1) {
-        if (!ok) return;
-        const int st = u % STAGES;
-        if (!(ok = mbar_wait_backoff<64>(empty + st, ((u / STAGES) & 1) ^ 1, ab, kAbortKvEmpty))) return;
-        unsigned char* dst = smem + C::OFF_RING + st * C::UNIT;
-        mbar_expect_tx(full + st, n * C::TILE);
-        load(dst, full + st, slot0, part, x0, y);
-        if (n > 1) load(dst + C::TILE, full + st, slot1, part, x1, y);
-        ++u;
-      };
-      auto scores = [&](int t) {
-        for (int p = 2; p >= 0; --p)
-          for (int s = 0; s < NSL; ++s) unit(TKV ? 2 : 1, p, t * BN, kSlotK, 64 * s, kSlotTK, 64 * s);
-      };
-      scores(0);
-      for (int t = 0; ok && t < n_tiles; ++t) {
-        if (t + 1 < n_tiles) scores(t + 1);
-        if constexpr (NSL == 1) {
-          for (int p = 2; p >= 0; --p) unit(TKV ? 2 : 1, p, t * BN, kSlotV, 0, kSlotTV, 0);
-        } else {
-          for (int p = 2; p >= 0; --p) unit(2, p, t * BN, kSlotV, 0, kSlotV, 64);
-          if constexpr (DUAL)
-            for (int p = 2; p >= 0; --p) {
-              unit(2, p, t * BN, kSlotV, 0, kSlotV, 64);
-              if constexpr (TKV) unit(2, p, t * BN, kSlotTV, 0, kSlotTV, 64);
+    if (warp == 0) {
+      // ------------------------------------------------------------------ TMA producer
+      if (lane == 0 && n_tiles > 0) {
+        prefetch_tmap(&map);
+        auto load = [&](unsigned char* dst, uint64_t* bar, int slot, int part, int x, int y) {
+          tma_load_4d(dst, &map, bar, x, y, bh, slot * 3 + part);
+        };
+        mbar_expect_tx(q_full, (C::Q_PARTS + (DUAL ? 3 : 0)) * NSL * C::PART);
+        for (int p = 0; p < 3; ++p)
+          for (int s = 0; s < NSL; ++s)
+            for (int r = 0; r < 2; ++r) {  // rows m0 + 64 r: beyond the tensor they read as zeros
+              const int off = (p * NSL + s) * C::PART + r * C::TILE;
+              if (p < C::Q_PARTS) load(smem + C::OFF_Q + off, q_full, kSlotQ, p, 64 * s, m0 + 64 * r);
+              if constexpr (DUAL) load(smem + C::OFF_TQ + off, q_full, kSlotTQ, p, 64 * s, m0 + 64 * r);
             }
+        int u = 0;
+        bool ok = true;
+        // one unit: n tiles of 8 KiB, the i-th from (slot_i, part, column x_i)
+        auto unit = [&](int n, int part, int y, int slot0, int x0, int slot1, int x1) {
+          if (!ok) return;
+          const int st = u % STAGES;
+          if (!(ok = mbar_wait_backoff<64>(empty + st, ((u / STAGES) & 1) ^ 1, ab, kAbortKvEmpty))) return;
+          unsigned char* dst = smem + C::OFF_RING + st * C::UNIT;
+          mbar_expect_tx(full + st, n * C::TILE);
+          load(dst, full + st, slot0, part, x0, y);
+          if (n > 1) load(dst + C::TILE, full + st, slot1, part, x1, y);
+          ++u;
+        };
+        auto scores = [&](int t) {
+          for (int p = 2; p >= 0; --p)
+            for (int s = 0; s < NSL; ++s) unit(TKV ? 2 : 1, p, t * BN, kSlotK, 64 * s, kSlotTK, 64 * s);
+        };
+        scores(0);
+        for (int t = 0; ok && t < n_tiles; ++t) {
+          if (t + 1 < n_tiles) scores(t + 1);
+          if constexpr (NSL == 1) {
+            for (int p = 2; p >= 0; --p) unit(TKV ? 2 : 1, p, t * BN, kSlotV, 0, kSlotTV, 0);
+          } else {
+            for (int p = 2; p >= 0; --p) unit(2, p, t * BN, kSlotV, 0, kSlotV, 64);
+            if constexpr (DUAL)
+              for (int p = 2; p >= 0; --p) {
+                unit(2, p, t * BN, kSlotV, 0, kSlotV, 64);
+                if constexpr (TKV) unit(2, p, t * BN, kSlotTV, 0, kSlotTV, 64);
+              }
+          }
         }
       }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer: a converged warp, one elected lane
-    if (n_tiles > 0) {
-      constexpr int F = Fmt<__nv_bfloat16>::kIdesc;
-      constexpr uint32_t id64 = make_idesc(F, BM, 64, 0, 0), id128 = make_idesc(F, BM, 128, 0, 0);
-      constexpr uint32_t id64t = make_idesc(F, BM, 64, 0, 1), id128t = make_idesc(F, BM, 128, 0, 1);  // B MN-major
-      constexpr uint32_t kLoMN = (uint32_t)(C::TILE >> 4) << 16;  // 64-column chunks of an MN-major operand are TILE apart
-      constexpr uint32_t PART16 = C::PART >> 4, UNIT16 = C::UNIT >> 4;
-      constexpr uint32_t id_s = TKV ? id128 : id64;
-      const uint32_t q_lo = kDescLo | (smem_u32(smem + C::OFF_Q) >> 4), tq_lo = kDescLo | (smem_u32(smem + C::OFF_TQ) >> 4);
-      const uint32_t ring16 = smem_u32(smem + C::OFF_RING) >> 4;
-      int st = 0;
-      uint32_t ph = 0;
-      bool ok = mbar_wait_warp(q_full, 0, ab, kAbortQFull);
-      if (C::QLO_TMEM && ok) ok = mbar_wait_warp(qlo_full, 0, ab, kAbortQFull);
-      auto acquire = [&]() -> bool {
-        if (!mbar_wait_warp(full + st, ph, ab, kAbortKvFull)) return ok = false;
-        tc_fence_after();
-        return true;
-      };
-      auto release = [&]() {  // (called by the elected lane)
-        tc_commit(empty + st);
-      };
-      auto next = [&]() {
-        if (++st == STAGES) st = 0, ph ^= 1;
-      };
-      // The scores of tile t: units of parts lo, mid, hi; part p of K meets the parts pa <= 2 - p of Q (tQ), small ones first.
-      auto scores = [&](int t) {
-        const uint32_t sc = tmem + (t & 1) * C::SC;
-#pragma unroll
-        for (int p = 2; p >= 0; --p) {
-#pragma unroll
-          for (int s = 0; s < NSL; ++s) {
-            if (!acquire()) return;
-            const uint32_t bk = kDescLo | (ring16 + st * UNIT16);
-            if (elect_one()) {
-#pragma unroll
-              for (int pa = 2 - p; pa >= 0; --pa) {
-                const uint32_t off = (pa * NSL + s) * PART16;
-                const bool first = p == 2 && s == 0;  // (pa = 0 then)
-#pragma unroll
-                for (int ks = 0; ks < KS; ++ks) {
-                  if (C::QLO_TMEM && pa == 2)
-                    umma_ts_lo<true>(sc, tmem + C::COL_QLO + s * 32 + ks * 8, bk + ks * 2, id_s);
-                  else if (first && ks == 0)
-                    umma_ss_lo<false>(sc, q_lo + off, bk, id_s);
-                  else
-                    umma_ss_lo<true>(sc, q_lo + off + ks * 2, bk + ks * 2, id_s);
-                }
-                if constexpr (DUAL) {
-#pragma unroll
+    } else if (warp == 1) {
+      // ------------------------------------------------------------------ MMA issuer: a converged warp, one elected lane
+      if (n_tiles > 0) {
+        constexpr int F = Fmt<__nv_bfloat16>::kIdesc;
+        constexpr uint32_t id64 = make_idesc(F, BM, 64, 0, 0), id128 = make_idesc(F, BM, 128, 0, 0);
+        constexpr uint32_t id64t = make_idesc(F, BM, 64, 0, 1), id128t = make_idesc(F, BM, 128, 0, 1);  // B MN-major
+        constexpr uint32_t kLoMN = (uint32_t)(C::TILE >> 4) << 16;  // 64-column chunks of an MN-major operand are TILE apart
+        constexpr uint32_t PART16 = C::PART >> 4, UNIT16 = C::UNIT >> 4;
+        constexpr uint32_t id_s = TKV ? id128 : id64;
+        const uint32_t q_lo = kDescLo | (smem_u32(smem + C::OFF_Q) >> 4), tq_lo = kDescLo | (smem_u32(smem + C::OFF_TQ) >> 4);
+        const uint32_t ring16 = smem_u32(smem + C::OFF_RING) >> 4;
+        int st = 0;
+        uint32_t ph = 0;
+        bool ok = mbar_wait_warp(q_full, 0, ab, kAbortQFull);
+        if (C::QLO_TMEM && ok) ok = mbar_wait_warp(qlo_full, 0, ab, kAbortQFull);
+        auto acquire = [&]() -> bool {
+          if (!mbar_wait_warp(full + st, ph, ab, kAbortKvFull)) return ok = false;
+          tc_fence_after();
+          return true;
+        };
+        auto release = [&]() {  // (called by the elected lane)
+          tc_commit(empty + st);
+        };
+        auto next = [&]() {
+          if (++st == STAGES) st = 0, ph ^= 1;
+        };
+        // The scores of tile t: units of parts lo, mid, hi; part p of K meets the parts pa <= 2 - p of Q (tQ), small ones first.
+        auto scores = [&](int t) {
+          const uint32_t sc = tmem + (t & 1) * C::SC;
+  #pragma unroll
+          for (int p = 2; p >= 0; --p) {
+  #pragma unroll
+            for (int s = 0; s < NSL; ++s) {
+              if (!acquire()) return;
+              const uint32_t bk = kDescLo | (ring16 + st * UNIT16);
+              if (elect_one()) {
+  #pragma unroll
+                for (int pa = 2 - p; pa >= 0; --pa) {
+                  const uint32_t off = (pa * NSL + s) * PART16;
+                  const bool first = p == 2 && s == 0;  // (pa = 0 then)
+  #pragma unroll
                   for (int ks = 0; ks < KS; ++ks) {
-                    if (!TKV && first && ks == 0)
-                      umma_ss_lo<false>(sc + 64, tq_lo + off, bk, id64);
+                    if (C::QLO_TMEM && pa == 2)
+                      umma_ts_lo<true>(sc, tmem + C::COL_QLO + s * 32 + ks * 8, bk + ks * 2, id_s);
+                    else if (first && ks == 0)
+                      umma_ss_lo<false>(sc, q_lo + off, bk, id_s);
                     else
-                      umma_ss_lo<true>(sc + 64, tq_lo + off + ks * 2, bk + ks * 2, id64);
+                      umma_ss_lo<true>(sc, q_lo + off + ks * 2, bk + ks * 2, id_s);
+                  }
+                  if constexpr (DUAL) {
+  #pragma unroll
+                    for (int ks = 0; ks < KS; ++ks) {
+                      if (!TKV && first && ks == 0)
+                        umma_ss_lo<false>(sc + 64, tq_lo + off, bk, id64);
+                      else
+                        umma_ss_lo<true>(sc + 64, tq_lo + off + ks * 2, bk + ks * 2, id64);
+                    }
                   }
                 }
-              }
-              release();
-              if (p == 0 && s == NSL - 1) tc_commit(s_full + (t & 1));
-            }
-            next();
-          }
-        }
-      };
-      int piece = 0;
-      // acc (+)= part pa of P (W) x the unit: contraction step kk = 16 keys
-      auto outer = [&](uint32_t acc_col, uint32_t sc, bool w, int pa, uint32_t bm, uint32_t id, bool fresh) {
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          const uint32_t acol = pa < 2 ? sc + (w ? 64 : 0) + 8 * pa + 16 * kk
-                                       : tmem + C::COL_LO + (w ? 16 : 0) + 32 * (kk >> 1) + 8 * (kk & 1);
-          if (fresh && kk == 0)
-            umma_ts_lo<false>(tmem + acc_col, acol, bm, id);
-          else
-            umma_ts_lo<true>(tmem + acc_col, acol, bm + kk * 128, id);
-        }
-      };
-      auto begin_piece = [&]() -> bool {
-        if (piece > 0 && !mbar_wait_warp(acc_free, (piece - 1) & 1, ab, kAbortOFull)) return ok = false;
-        tc_fence_after();
-        ++piece;
-        return true;
-      };
-      auto outputs = [&](int t) {
-        const uint32_t sc = tmem + (t & 1) * C::SC;
-        if (!mbar_wait_warp(p_full + (t & 1), (t >> 1) & 1, ab, kAbortPFull) || !begin_piece()) {
-          ok = false;
-          return;
-        }
-#pragma unroll
-        for (int p = 2; p >= 0; --p) {  // D <= 64: [O | tO'] += P [V | tV], tO' += W V ; D = 128: O += P V
-          if (!acquire()) return;
-          const uint32_t bm = kLoMN | (ring16 + st * UNIT16);
-          if (elect_one()) {
-#pragma unroll
-            for (int pa = 2 - p; pa >= 0; --pa) {
-              outer(C::COL_ACC, sc, false, pa, bm, TKV || NSL == 2 ? id128t : id64t, p == 2);
-              if constexpr (DUAL && NSL == 1) outer(C::COL_ACC + 64, sc, true, pa, bm, id64t, !TKV && p == 2);
-            }
-            release();
-            if (p == 0) tc_commit(acc_full);
-          }
-          next();
-        }
-        if constexpr (DUAL && NSL == 2) {
-          if (!begin_piece()) return;
-#pragma unroll
-          for (int p = 2; p >= 0; --p) {  // tO' += W V + P tV
-#pragma unroll
-            for (int x = 0; x < (TKV ? 2 : 1); ++x) {
-              if (!acquire()) return;
-              const uint32_t bm = kLoMN | (ring16 + st * UNIT16);
-              if (elect_one()) {
-#pragma unroll
-                for (int pa = 2 - p; pa >= 0; --pa) outer(C::COL_ACC, sc, x == 0, pa, bm, id128t, p == 2 && x == 0);
                 release();
-                if (p == 0 && x == (TKV ? 1 : 0)) tc_commit(acc_full);
+                if (p == 0 && s == NSL - 1) tc_commit(s_full + (t & 1));
               }
               next();
             }
           }
+        };
+        int piece = 0;
+        // acc (+)= part pa of P (W) x the unit: contraction step kk = 16 keys
+        auto outer = [&](uint32_t acc_col, uint32_t sc, bool w, int pa, uint32_t bm, uint32_t id, bool fresh) {
+  #pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {
+            const uint32_t acol = pa < 2 ? sc + (w ? 64 : 0) + 8 * pa + 16 * kk
+                                         : tmem + C::COL_LO + (w ? 16 : 0) + 32 * (kk >> 1) + 8 * (kk & 1);
+            if (fresh && kk == 0)
+              umma_ts_lo<false>(tmem + acc_col, acol, bm, id);
+            else
+              umma_ts_lo<true>(tmem + acc_col, acol, bm + kk * 128, id);
+          }
+        };
+        auto begin_piece = [&]() -> bool {
+          if (piece > 0 && !mbar_wait_warp(acc_free, (piece - 1) & 1, ab, kAbortOFull)) return ok = false;
+          tc_fence_after();
+          ++piece;
+          return true;
+        };
+        auto outputs = [&](int t) {
+          const uint32_t sc = tmem + (t & 1) * C::SC;
+          if (!mbar_wait_warp(p_full + (t & 1), (t >> 1) & 1, ab, kAbortPFull) || !begin_piece()) {
+            ok = false;
+            return;
+          }
+  #pragma unroll
+          for (int p = 2; p >= 0; --p) {  // D <= 64: [O | tO'] += P [V | tV], tO' += W V ; D = 128: O += P V
+            if (!acquire()) return;
+            const uint32_t bm = kLoMN | (ring16 + st * UNIT16);
+            if (elect_one()) {
+  #pragma unroll
+              for (int pa = 2 - p; pa >= 0; --pa) {
+                outer(C::COL_ACC, sc, false, pa, bm, TKV || NSL == 2 ? id128t : id64t, p == 2);
+                if constexpr (DUAL && NSL == 1) outer(C::COL_ACC + 64, sc, true, pa, bm, id64t, !TKV && p == 2);
+              }
+              release();
+              if (p == 0) tc_commit(acc_full);
+            }
+            next();
+          }
+          if constexpr (DUAL && NSL == 2) {
+            if (!begin_piece()) return;
+  #pragma unroll
+            for (int p = 2; p >= 0; --p) {  // tO' += W V + P tV
+  #pragma unroll
+              for (int x = 0; x < (TKV ? 2 : 1); ++x) {
+                if (!acquire()) return;
+                const uint32_t bm = kLoMN | (ring16 + st * UNIT16);
+                if (elect_one()) {
+  #pragma unroll
+                  for (int pa = 2 - p; pa >= 0; --pa) outer(C::COL_ACC, sc, x == 0, pa, bm, id128t, p == 2 && x == 0);
+                  release();
+                  if (p == 0 && x == (TKV ? 1 : 0)) tc_commit(acc_full);
+                }
+                next();
+              }
+            }
+          }
+        };
+        if (ok) scores(0);
+        for (int t = 0; ok && t < n_tiles; ++t) {
+          if (t + 1 < n_tiles) scores(t + 1);
+          if (ok) outputs(t);
         }
-      };
-      if (ok) scores(0);
-      for (int t = 0; ok && t < n_tiles; ++t) {
-        if (t + 1 < n_tiles) scores(t + 1);
-        if (ok) outputs(t);
       }
     }
-  }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     // ------------------------------------------------------------------ softmax, outputs

@@ -269,171 +269,171 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
   // The four warps of warpgroup 0 need few registers; the softmax threads hold two score tiles each.  (In the branches of the
   // roles: ptxas holds code behind a join of the two to the smaller number.)
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      prefetch_tmap(&maps.q), prefetch_tmap(&maps.k), prefetch_tmap(&maps.v);
-      if constexpr (DUAL) prefetch_tmap(&maps.tq), prefetch_tmap(&maps.tk), prefetch_tmap(&maps.tv);
-      int g = 0, kact = 0;
-      bool ok = true;
-      PairItem it;
-      for (int k = 0; ok && k < k_max; ++k) {
-        if (!get_item(k, it) || it.n_load == 0) continue;
-        // The Q tiles are single-buffered: both issuers must be through with the previous item's.
-        if (kact > 0 && !mbar_wait(q_empty, (kact - 1) & 1, ab, kAbortQFull)) break;
-        mbar_expect_tx(q_full, C::NQ * C::N_QT * C::Q_BYTES);
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+    if (warp == 0) {
+      // ------------------------------------------------------------------ TMA producer
+      if (lane == 0) {
+        prefetch_tmap(&maps.q), prefetch_tmap(&maps.k), prefetch_tmap(&maps.v);
+        if constexpr (DUAL) prefetch_tmap(&maps.tq), prefetch_tmap(&maps.tk), prefetch_tmap(&maps.tv);
+        int g = 0, kact = 0;
+        bool ok = true;
+        PairItem it;
+        for (int k = 0; ok && k < k_max; ++k) {
+          if (!get_item(k, it) || it.n_load == 0) continue;
+          // The Q tiles are single-buffered: both issuers must be through with the previous item's.
+          if (kact > 0 && !mbar_wait(q_empty, (kact - 1) & 1, ab, kAbortQFull)) break;
+          mbar_expect_tx(q_full, C::NQ * C::N_QT * C::Q_BYTES);
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {  // a tile that starts past L reads as zeros
-          unsigned char* dst = sQ + x * C::N_QT * C::Q_BYTES;
-          tma_load_4d(dst, &maps.q, q_full, 0, it.m0 + x * BM, it.h, it.b);
-          if constexpr (DUAL) tma_load_4d(dst + C::Q_BYTES, &maps.tq, q_full, 0, it.m0 + x * BM, it.h, it.b);
-        }
-        TileUse<MK> use(it);
-        for (int j = 0; j < it.n_load; ++j) {
-          if (use(j) == 0) continue;
-          const int st = g % STAGES;
-          if (!mbar_wait(kv_empty + st, ((g / STAGES) & 1) ^ 1, ab, kAbortKvEmpty)) {
-            ok = false;
-            break;
+          for (int x = 0; x < 2; ++x) {  // a tile that starts past L reads as zeros
+            unsigned char* dst = sQ + x * C::N_QT * C::Q_BYTES;
+            tma_load_4d(dst, &maps.q, q_full, 0, it.m0 + x * BM, it.h, it.b);
+            if constexpr (DUAL) tma_load_4d(dst + C::Q_BYTES, &maps.tq, q_full, 0, it.m0 + x * BM, it.h, it.b);
           }
-          unsigned char* base = sKV + st * C::STAGE_BYTES;
-          mbar_expect_tx(kv_full + st, C::STAGE_BYTES);
-          const int n0 = j * BN;
-          tma_load_4d(base + C::SLOT_K * C::KV_BYTES, &maps.k, kv_full + st, 0, n0, it.h, it.b);
-          if constexpr (DUAL) tma_load_4d(base + C::SLOT_TK * C::KV_BYTES, &maps.tk, kv_full + st, 0, n0, it.h, it.b);
-          tma_load_4d(base + C::SLOT_V * C::KV_BYTES, &maps.v, kv_full + st, 0, n0, it.h, it.b);
-          if constexpr (DUAL) tma_load_4d(base + C::SLOT_TV * C::KV_BYTES, &maps.tv, kv_full + st, 0, n0, it.h, it.b);
-          ++g;
+          TileUse<MK> use(it);
+          for (int j = 0; j < it.n_load; ++j) {
+            if (use(j) == 0) continue;
+            const int st = g % STAGES;
+            if (!mbar_wait(kv_empty + st, ((g / STAGES) & 1) ^ 1, ab, kAbortKvEmpty)) {
+              ok = false;
+              break;
+            }
+            unsigned char* base = sKV + st * C::STAGE_BYTES;
+            mbar_expect_tx(kv_full + st, C::STAGE_BYTES);
+            const int n0 = j * BN;
+            tma_load_4d(base + C::SLOT_K * C::KV_BYTES, &maps.k, kv_full + st, 0, n0, it.h, it.b);
+            if constexpr (DUAL) tma_load_4d(base + C::SLOT_TK * C::KV_BYTES, &maps.tk, kv_full + st, 0, n0, it.h, it.b);
+            tma_load_4d(base + C::SLOT_V * C::KV_BYTES, &maps.v, kv_full + st, 0, n0, it.h, it.b);
+            if constexpr (DUAL) tma_load_4d(base + C::SLOT_TV * C::KV_BYTES, &maps.tv, kv_full + st, 0, n0, it.h, it.b);
+            ++g;
+          }
+          ++kact;
         }
-        ++kact;
       }
-    }
-  } else if (warp <= 2) {
-    // ------------------------------------------------------------------ issuer of query tile X
-    // A converged warp, one elected lane (mbar_wait_warp).  Whatever it executes between two MMAs is pure latency for the tensor
-    // pipe, so stage and barrier cursors, parities and the low words of the operand descriptors live in registers and advance by
-    // additions (descriptor = constant high word kDescHi + (byte address >> 4) in the low word).
-    {
-      const int X = warp - 1;
-      constexpr uint32_t idesc_s = make_idesc(Fmt<T>::kIdesc, BM, BN, 0, 0);       // 128 x 64
-      constexpr uint32_t idesc_s2 = make_idesc(Fmt<T>::kIdesc, BM, 2 * BN, 0, 0);  // 128 x 128: [S | tS]
-      constexpr uint32_t idesc_o = make_idesc(Fmt<T>::kIdesc, BM, D, 0, 1);        // 128 x 64, B MN-major
-      constexpr uint32_t idesc_o2 = make_idesc(Fmt<T>::kIdesc, BM, 2 * D, 0, 1);   // 128 x 128: [O | tO']
-      constexpr uint32_t kLoV = (uint32_t)(C::KV_BYTES >> 4) << 16;  // [V | tV]: 64-column chunks KV_BYTES apart
-      constexpr uint32_t STAGE16 = C::STAGE_BYTES >> 4;
-      const uint32_t q_lo = kDescLo | (smem_u32(sQ + X * C::N_QT * C::Q_BYTES) >> 4), tq_lo = q_lo + (C::Q_BYTES >> 4);
-      const uint32_t p_lo = kDescLo | (smem_u32(sP + X * C::N_P * C::P_BYTES) >> 4), w_lo = p_lo + (C::P_BYTES >> 4);
-      const uint32_t k_lo0 = kDescLo | ((smem_u32(sKV) + C::SLOT_K * C::KV_BYTES) >> 4);
-      const uint32_t v_lo0 = kLoV | ((smem_u32(sKV) + C::SLOT_V * C::KV_BYTES) >> 4);
-      const uint32_t bar_kv_full = smem_u32(kv_full), bar_kv_empty = smem_u32(kv_empty);
-      const uint32_t bar_s_full = smem_u32(s_full + X), bar_s_free = smem_u32(s_free + X);
-      const uint32_t bar_p_full = smem_u32(p_full + X), bar_pv_done = smem_u32(pv_done + X);
-      const uint32_t bar_o_free = smem_u32(o_free + X), bar_q_empty = smem_u32(q_empty);
-      const uint32_t tq = tmem + X * C::COLS_PER_Q;
-      uint32_t st = 0, st_par = 0;  // ring stage of the next loaded tile and the parity of its kv_full phase
-      uint32_t tpar = 0;            // parity of the phase that this query tile's next used tile completes
-      bool any_t = false;           // this query tile has used a tile before
-      int kact = 0, kx = 0;
-      bool ok = true;
-      PairItem it;
+    } else if (warp <= 2) {
+      // ------------------------------------------------------------------ issuer of query tile X
+      // A converged warp, one elected lane (mbar_wait_warp).  Whatever it executes between two MMAs is pure latency for the tensor
+      // pipe, so stage and barrier cursors, parities and the low words of the operand descriptors live in registers and advance by
+      // additions (descriptor = constant high word kDescHi + (byte address >> 4) in the low word).
+      {
+        const int X = warp - 1;
+        constexpr uint32_t idesc_s = make_idesc(Fmt<T>::kIdesc, BM, BN, 0, 0);       // 128 x 64
+        constexpr uint32_t idesc_s2 = make_idesc(Fmt<T>::kIdesc, BM, 2 * BN, 0, 0);  // 128 x 128: [S | tS]
+        constexpr uint32_t idesc_o = make_idesc(Fmt<T>::kIdesc, BM, D, 0, 1);        // 128 x 64, B MN-major
+        constexpr uint32_t idesc_o2 = make_idesc(Fmt<T>::kIdesc, BM, 2 * D, 0, 1);   // 128 x 128: [O | tO']
+        constexpr uint32_t kLoV = (uint32_t)(C::KV_BYTES >> 4) << 16;  // [V | tV]: 64-column chunks KV_BYTES apart
+        constexpr uint32_t STAGE16 = C::STAGE_BYTES >> 4;
+        const uint32_t q_lo = kDescLo | (smem_u32(sQ + X * C::N_QT * C::Q_BYTES) >> 4), tq_lo = q_lo + (C::Q_BYTES >> 4);
+        const uint32_t p_lo = kDescLo | (smem_u32(sP + X * C::N_P * C::P_BYTES) >> 4), w_lo = p_lo + (C::P_BYTES >> 4);
+        const uint32_t k_lo0 = kDescLo | ((smem_u32(sKV) + C::SLOT_K * C::KV_BYTES) >> 4);
+        const uint32_t v_lo0 = kLoV | ((smem_u32(sKV) + C::SLOT_V * C::KV_BYTES) >> 4);
+        const uint32_t bar_kv_full = smem_u32(kv_full), bar_kv_empty = smem_u32(kv_empty);
+        const uint32_t bar_s_full = smem_u32(s_full + X), bar_s_free = smem_u32(s_free + X);
+        const uint32_t bar_p_full = smem_u32(p_full + X), bar_pv_done = smem_u32(pv_done + X);
+        const uint32_t bar_o_free = smem_u32(o_free + X), bar_q_empty = smem_u32(q_empty);
+        const uint32_t tq = tmem + X * C::COLS_PER_Q;
+        uint32_t st = 0, st_par = 0;  // ring stage of the next loaded tile and the parity of its kv_full phase
+        uint32_t tpar = 0;            // parity of the phase that this query tile's next used tile completes
+        bool any_t = false;           // this query tile has used a tile before
+        int kact = 0, kx = 0;
+        bool ok = true;
+        PairItem it;
 
-      // [O | tO'] (+)= P [V | tV] ; tO' += W V for the tile in ring stage pst, whose phases have parity ppar
-      auto issue_pv = [&](uint32_t pst, uint32_t ppar, bool first) -> bool {
-        if (!mbar_wait_warp_u32(bar_p_full, ppar, ab, kAbortPFull)) return false;
-        // The item's first tile overwrites O / tO': the previous item's epilogue must have read them.
-        if (first && kx > 0 && !mbar_wait_warp_u32(bar_o_free, (kx - 1) & 1, ab, kAbortOFull)) return false;
-        tc_fence_after();
-        const uint32_t v_lo = v_lo0 + pst * STAGE16;
-        if (elect_one()) {
-        if constexpr (DUAL) {
-          umma_ss_lo_dyn(tq + C::COL_O, p_lo, v_lo, idesc_o2, first ? 0u : 1u);
-#pragma unroll
-          for (int kk = 1; kk < BN / 16; ++kk) umma_ss_lo<true>(tq + C::COL_O, p_lo + kk * 2, v_lo + kk * 128, idesc_o2);
-#pragma unroll
-          for (int kk = 0; kk < BN / 16; ++kk) umma_ss_lo<true>(tq + C::COL_TO, w_lo + kk * 2, v_lo + kk * 128, idesc_o);
-        } else {  // P from TMEM
-          umma_ts_lo_dyn(tq + C::COL_O, tq + C::COL_P, v_lo, idesc_o, first ? 0u : 1u);
-#pragma unroll
-          for (int kk = 1; kk < BN / 16; ++kk) umma_ts_lo<true>(tq + C::COL_O, tq + C::COL_P + kk * 8, v_lo + kk * 128, idesc_o);
-        }
-        tc_commit_u32(bar_kv_empty + 8 * pst);
-        tc_commit_u32(bar_pv_done);
-        }
-        return true;
-      };
-
-      for (int k = 0; ok && k < k_max; ++k) {
-        if (!get_item(k, it) || it.n_load == 0) continue;
-        // waited for by both issuers in every item, used or not: a parity wait must see every phase
-        if (!mbar_wait_warp(q_full, kact & 1, ab, kAbortQFull)) break;
-        const int my_last = it.last(X);
-        bool pend = false, pend_first = false, first = true;
-        uint32_t pend_st = 0, pend_par = 0;
-        TileUse<MK> use(it);
-        for (int j = 0; j < it.n_load; ++j) {
-          const int m = use(j);
-          if (m == 0) continue;
-          if (!mbar_wait_warp_u32(bar_kv_full + 8 * st, st_par, ab, kAbortKvFull)) {
-            ok = false;
-            break;
-          }
-          if (m & (1 << X)) {
-            // S / tS of the previous tile (of this item or the one before) must be in the softmax threads' registers
-            if (any_t && !mbar_wait_warp_u32(bar_s_free, tpar ^ 1, ab, kAbortSFull)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t k_lo = k_lo0 + st * STAGE16;
-            if (elect_one()) {
+        // [O | tO'] (+)= P [V | tV] ; tO' += W V for the tile in ring stage pst, whose phases have parity ppar
+        auto issue_pv = [&](uint32_t pst, uint32_t ppar, bool first) -> bool {
+          if (!mbar_wait_warp_u32(bar_p_full, ppar, ab, kAbortPFull)) return false;
+          // The item's first tile overwrites O / tO': the previous item's epilogue must have read them.
+          if (first && kx > 0 && !mbar_wait_warp_u32(bar_o_free, (kx - 1) & 1, ab, kAbortOFull)) return false;
+          tc_fence_after();
+          const uint32_t v_lo = v_lo0 + pst * STAGE16;
+          if (elect_one()) {
             if constexpr (DUAL) {
-              umma_ss_lo<false>(tq + C::COL_S, q_lo, k_lo, idesc_s2);  // [S | tS] = Q [K ; tK]^T
+              umma_ss_lo_dyn(tq + C::COL_O, p_lo, v_lo, idesc_o2, first ? 0u : 1u);
 #pragma unroll
-              for (int ks = 1; ks < D / 16; ++ks)
-                if (ks < 2 || a.D > 32) umma_ss_lo<true>(tq + C::COL_S, q_lo + ks * 2, k_lo + ks * 2, idesc_s2);
+              for (int kk = 1; kk < BN / 16; ++kk) umma_ss_lo<true>(tq + C::COL_O, p_lo + kk * 2, v_lo + kk * 128, idesc_o2);
 #pragma unroll
-              for (int ks = 0; ks < D / 16; ++ks)
-                if (ks < 2 || a.D > 32) umma_ss_lo<true>(tq + C::COL_TS, tq_lo + ks * 2, k_lo + ks * 2, idesc_s);  // tS += tQ K^T
-            } else {
-              umma_ss_lo<false>(tq + C::COL_S, q_lo, k_lo, idesc_s);
+              for (int kk = 0; kk < BN / 16; ++kk) umma_ss_lo<true>(tq + C::COL_TO, w_lo + kk * 2, v_lo + kk * 128, idesc_o);
+            } else {  // P from TMEM
+              umma_ts_lo_dyn(tq + C::COL_O, tq + C::COL_P, v_lo, idesc_o, first ? 0u : 1u);
 #pragma unroll
-              for (int ks = 1; ks < D / 16; ++ks)
-                if (ks < 2 || a.D > 32) umma_ss_lo<true>(tq + C::COL_S, q_lo + ks * 2, k_lo + ks * 2, idesc_s);
+              for (int kk = 1; kk < BN / 16; ++kk) umma_ts_lo<true>(tq + C::COL_O, tq + C::COL_P + kk * 8, v_lo + kk * 128, idesc_o);
             }
-            tc_commit_u32(bar_s_full);
-            if (j == my_last) tc_commit_u32(bar_q_empty);  // arrives when the item's last scores are complete
-            }
-            if (pend && !issue_pv(pend_st, pend_par, pend_first)) {
+            tc_commit_u32(bar_kv_empty + 8 * pst);
+            tc_commit_u32(bar_pv_done);
+          }
+          return true;
+        };
+
+        for (int k = 0; ok && k < k_max; ++k) {
+          if (!get_item(k, it) || it.n_load == 0) continue;
+          // waited for by both issuers in every item, used or not: a parity wait must see every phase
+          if (!mbar_wait_warp(q_full, kact & 1, ab, kAbortQFull)) break;
+          const int my_last = it.last(X);
+          bool pend = false, pend_first = false, first = true;
+          uint32_t pend_st = 0, pend_par = 0;
+          TileUse<MK> use(it);
+          for (int j = 0; j < it.n_load; ++j) {
+            const int m = use(j);
+            if (m == 0) continue;
+            if (!mbar_wait_warp_u32(bar_kv_full + 8 * st, st_par, ab, kAbortKvFull)) {
               ok = false;
               break;
             }
-            pend = true, pend_st = st, pend_par = tpar, pend_first = first, first = false;
-            tpar ^= 1, any_t = true;
-          } else {
-            // Loaded for the other query tile only.  A pending output product holds an older ring stage: it goes
-            // out first, or the producer could wait for that stage while this thread waits for the producer.
-            if (pend) {
-              if (!issue_pv(pend_st, pend_par, pend_first)) {
+            if (m & (1 << X)) {
+              // S / tS of the previous tile (of this item or the one before) must be in the softmax threads' registers
+              if (any_t && !mbar_wait_warp_u32(bar_s_free, tpar ^ 1, ab, kAbortSFull)) {
                 ok = false;
                 break;
               }
-              pend = false;
+              tc_fence_after();
+              const uint32_t k_lo = k_lo0 + st * STAGE16;
+              if (elect_one()) {
+                if constexpr (DUAL) {
+                  umma_ss_lo<false>(tq + C::COL_S, q_lo, k_lo, idesc_s2);  // [S | tS] = Q [K ; tK]^T
+#pragma unroll
+                  for (int ks = 1; ks < D / 16; ++ks)
+                    if (ks < 2 || a.D > 32) umma_ss_lo<true>(tq + C::COL_S, q_lo + ks * 2, k_lo + ks * 2, idesc_s2);
+#pragma unroll
+                  for (int ks = 0; ks < D / 16; ++ks)
+                    if (ks < 2 || a.D > 32) umma_ss_lo<true>(tq + C::COL_TS, tq_lo + ks * 2, k_lo + ks * 2, idesc_s);  // tS += tQ K^T
+                } else {
+                  umma_ss_lo<false>(tq + C::COL_S, q_lo, k_lo, idesc_s);
+#pragma unroll
+                  for (int ks = 1; ks < D / 16; ++ks)
+                    if (ks < 2 || a.D > 32) umma_ss_lo<true>(tq + C::COL_S, q_lo + ks * 2, k_lo + ks * 2, idesc_s);
+                }
+                tc_commit_u32(bar_s_full);
+                if (j == my_last) tc_commit_u32(bar_q_empty);  // arrives when the item's last scores are complete
+              }
+              if (pend && !issue_pv(pend_st, pend_par, pend_first)) {
+                ok = false;
+                break;
+              }
+              pend = true, pend_st = st, pend_par = tpar, pend_first = first, first = false;
+              tpar ^= 1, any_t = true;
+            } else {
+              // Loaded for the other query tile only.  A pending output product holds an older ring stage: it goes
+              // out first, or the producer could wait for that stage while this thread waits for the producer.
+              if (pend) {
+                if (!issue_pv(pend_st, pend_par, pend_first)) {
+                  ok = false;
+                  break;
+                }
+                pend = false;
+              }
+              if (elect_one()) mbar_arrive(kv_empty + st);
             }
-            if (elect_one()) mbar_arrive(kv_empty + st);
+            if (++st == STAGES) st = 0, st_par ^= 1;
           }
-          if (++st == STAGES) st = 0, st_par ^= 1;
+          if (!ok) break;
+          if (pend && !issue_pv(pend_st, pend_par, pend_first)) break;
+          if (!first)
+            ++kx;  // this query tile used key tiles in the item (its q_empty arrival went out with the last scores)
+          else if (elect_one())
+            mbar_arrive(q_empty);
+          ++kact;
         }
-        if (!ok) break;
-        if (pend && !issue_pv(pend_st, pend_par, pend_first)) break;
-        if (!first)
-          ++kx;  // this query tile used key tiles in the item (its q_empty arrival went out with the last scores)
-        else if (elect_one())
-          mbar_arrive(q_empty);
-        ++kact;
       }
     }
-  }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     // ------------------------------------------------------------------ softmax + epilogue of query tile X

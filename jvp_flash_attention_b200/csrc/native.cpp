@@ -266,7 +266,7 @@ void pack(const MaskDesc& m, const Tensor& q, Tensor& bits_out, Tensor* bits_t_o
 // those of its verification.
 //
 // Packing reads the mask once (HBM bound) and saves a kernel that reads it one 16-byte piece per row and sub-tile.
-// B2 H12 L2048 D64, 100 MB of mask: packing 32 us; forward with tangents 168 -> 151 us, backward through tO 239 -> 186.
+// B2 H12 L2048 D64, 100 MB of mask: packing 32 to 36 us; forward with tangents 168 -> 151 us, backward through tO 239 -> 186.
 // So it pays with a backward, for a mask that several heads share, and where the bytes' layout would send the call to
 // the register-tiled kernels.  Where there is no memory for the bits the kernels read the bytes.
 void pack_mask(Call& call, const Tensor& q, bool backward) {
@@ -391,7 +391,8 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
 
   // One scratch allocation: the three row statistics, and fp32 dQ where the single-pass kernel takes it (head dimension 64,
   // 16-bit; index masks, and as far as rows are whole 16-byte pieces a boolean mask without tile bitmaps or, through O
-  // alone, a bias of the tensors' type).
+  // alone, a bias of the tensors' type).  Such a bias through tO has a workspace instead, below (from 96 key tiles on and up to
+  // 512 MiB; else the two launches).
   bool single = g_single_pass && !(skip & JVPFA_SKIP_DKDV) && sizes[3] == 64 && q.scalar_type() != at::kFloat;
   if (m.c.kind == JVPFA_MASK_BOOL)
     single = single && !m.tile_live.defined() && !m.tile_live_t.defined() && whole_pieces(m, sizes[2]);

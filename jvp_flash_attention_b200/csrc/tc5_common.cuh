@@ -180,11 +180,7 @@ struct AbortState {
   int* global_status;      // device global
 };
 
-// Bounded wait.  Returns false (and latches the abort state) when the budget runs out or when
-// another thread of the CTA has already given up.  A measured mbarrier hand-off between two warps
-// costs ~200 cycles; reading the clock costs several tens of cycles, so the wait first polls
-// without looking at it.  The budget and the abort flag are checked in the out-of-line part.
-// First failure wins; the code also goes to the host-visible mirror whose device address sits beside the status word
+// What a wait that gives up leaves for everybody.  First failure wins; the code also goes to the host-visible mirror whose device address sits beside the status word
 // (two ints further, 8-byte aligned), so that the host learns of it without synchronising.
 __device__ __forceinline__ void publish_abort(int* global_status, int code) {
   if (atomicCAS(global_status, 0, code) == 0) {
@@ -195,8 +191,6 @@ __device__ __forceinline__ void publish_abort(int* global_status, int code) {
     }
   }
 }
-static __device__ __noinline__ bool mbar_wait_slow_u32(uint32_t bar, uint32_t parity, volatile int* cta_flag,
-                                                       int* global_status, int code);
 __device__ __forceinline__ bool mbar_try_wait_u32(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -208,15 +202,11 @@ __device__ __forceinline__ bool mbar_try_wait_u32(uint32_t bar, uint32_t parity)
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait_u32(uint32_t bar, uint32_t parity, const AbortState& ab, int code) {
-#pragma unroll 1
-  for (int i = 0; i < 128; ++i)
-    if (mbar_try_wait_u32(bar, parity)) return true;
-  return mbar_wait_slow_u32(bar, parity, ab.cta_flag, ab.global_status, code);
-}
-// The general form.  Measured on the forward kernels (two CTAs per SM, many warps waiting at once):
+// Bounded wait.  Returns false (and latches the abort state) when the budget runs out or when
+// another thread of the CTA has already given up.  A measured mbarrier hand-off between two warps
+// costs ~200 cycles.  Measured on the forward kernels (two CTAs per SM, many warps waiting at once):
 // a poll loop that reads the clock right after the first failed attempt is ~5 % faster overall
-// than the tight loop above, which takes issue slots from the warps that compute.
+// than one that polls 128 times first, which takes issue slots from the warps that compute.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const AbortState& ab, int code) {
   const uint32_t addr = smem_u32(bar);
   if (mbar_try_wait_u32(addr, parity)) return true;
@@ -255,23 +245,6 @@ __device__ __forceinline__ bool mbar_wait_backoff(uint64_t* bar, uint32_t parity
     }
   }
 }
-static __device__ __noinline__ bool mbar_wait_slow_u32(uint32_t bar, uint32_t parity, volatile int* cta_flag,
-                                                       int* global_status, int code) {
-  const long long t0 = clock64();
-  int polls = 0;
-  while (true) {
-    if (mbar_try_wait_u32(bar, parity)) return true;
-    if ((++polls & 63) == 0) {
-      if (*cta_flag != 0) return false;
-      if (clock64() - t0 > kWaitBudgetCycles) {
-        *cta_flag = code;
-        publish_abort(global_status, code);
-        return false;
-      }
-    }
-  }
-}
-
 // The wait of an issuing warp, by all of its lanes with one outcome for them (a lane that gave up takes the others along: what
 // follows needs all of them).  A warp that stays converged keeps descriptors and loop counters in uniform registers, where
 // tcgen05.mma takes its operands from, and only the instructions themselves are one lane's (`elect_one`).  Issued from a branch of

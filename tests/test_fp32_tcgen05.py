@@ -91,8 +91,8 @@ def _rel(x, r):
     (333, "bias_row", 3),
 ])
 def test_forward_on_three_bf16_parts(D, L, kind, n_tangents):
-    """A product is exact to 2^-26 of its operands and an accumulator takes 24 instructions a key tile, truncated at 2^-24 of
-    it or of its small parts: 1e-5 of the largest entry, the fp32 bound of the parity tests, and no further from 64 bits than
+    """A product is exact to 2^-24 of its operands and an accumulator takes up to 48 instructions a key tile, each truncated at 2^-24
+    of what is there by then: 1e-5 of the largest entry, the fp32 bound of the parity tests, and no further from 64 bits than
     the register-tiled kernels (1.2 times, for the luck of a few rows)."""
     B, H = 2, 3
     g = torch.Generator().manual_seed(L + D)
