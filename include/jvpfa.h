@@ -47,7 +47,8 @@ typedef enum {
 typedef enum {
   JVPFA_BF16 = 0,
   JVPFA_FP16 = 1,
-  JVPFA_FP32 = 2,      /* fp32 tensors; every product as three MMAs on a hi/lo split of 22 bits (error ~1e-6 relative) */
+  JVPFA_FP32 = 2,      /* fp32 tensors; every product as three MMAs on a hi/lo split of 22 bits, or with a workspace as six
+                          on three bf16 parts, 24 bits (error ~1e-6 relative) */
   JVPFA_FP32_TF32 = 3  /* fp32 tensors; every product as one TF32 MMA, the precision of upstream's fp32 path
                           (tl.dot on TF32 tensor cores, jvp_attention.py:233-236); error ~5e-4 relative, 1.7 to
                           2.2 times as fast (B2 H8 L2048 D64).  Not a bias dtype: an fp32 bias is JVPFA_FP32. */
