@@ -79,6 +79,15 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
+// The encoder is a driver call and wants a current context, which a thread that has made no runtime call yet does not have (its
+// memory may come from an allocator's cache): it is given its device's then.
+template <typename Encode>
+static bool encode_in_context(Encode encode) {
+  if (encode() == CUDA_SUCCESS) return true;
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && encode() == CUDA_SUCCESS;
+}
+
 bool encode_map4d(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int D, int L, int H, int B, const int64_t* st,
                   int box_rows) {
   EncodeTiledFn fn = get_encode_fn();
@@ -91,9 +100,10 @@ bool encode_map4d(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int D
   cuuint64_t strides[3] = {sl * 2, sh * 2, sb * 2};
   cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = fn(m, dt, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
+  return encode_in_context([&]() {
+    return fn(m, dt, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
 }
 
 // Row-major fp32 (B, H, L, D) tensor as a 4-D map with 32-column (128-byte) swizzled boxes: target of TMA reductions.
@@ -104,10 +114,11 @@ bool encode_map4d_f32(CUtensorMap* m, const void* ptr, int D, int L, int H, int 
   cuuint64_t strides[3] = {(cuuint64_t)D * 4, (cuuint64_t)L * D * 4, (cuuint64_t)H * L * D * 4};
   cuuint32_t box[4] = {32, (cuuint32_t)box_rows, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(ptr), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
+  return encode_in_context([&]() {
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(ptr), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
 }
 
 bool encode_map_parts(CUtensorMap* m, const void* ptr, int D, int L, int BH, int planes) {

@@ -2,6 +2,9 @@
 fill 16-byte pieces, the forms of the register-tiled kernels, the range of fp32, gradients that nobody asked for, and what a
 call takes of memory and of the interpreter."""
 import ctypes
+import pathlib
+import subprocess
+import sys
 import threading
 import time
 
@@ -420,6 +423,34 @@ def test_other_threads_run_while_the_launch_queue_is_full(kind):
         stop.set()
         other.join()
     assert waited > 0.2 and max(pauses) < waited / 4, (waited, max(pauses))
+
+
+@pytest.mark.parametrize("dt", ["bfloat16", "float32"])
+def test_first_calls_of_several_threads(dt):
+    """In a process of its own: threads that have made no CUDA call before, and whose buffers come from torch's cache, call the library
+    at once.  (The tensor maps are encoded by the driver, which refuses a thread that has no current context.)"""
+    code = f"""
+import threading, torch
+import jvp_flash_attention_b200.jvp_attention as ja
+from jvp_flash_attention_b200 import _lib
+x = torch.randn(2, 16, 256, 64, device="cuda", dtype=torch.{dt})
+cached = [torch.empty_like(x) for _ in range(64)] + [torch.empty(1 << 24, dtype=torch.uint8, device="cuda") for _ in range(16)]
+del cached
+_lib.load(), _lib.native(), torch.cuda.synchronize()
+start, out = threading.Barrier(8), [None] * 8
+def call(n):
+    start.wait()
+    try:
+        out[n] = ja.attention(x, x, x)
+    except Exception as e:
+        out[n] = e
+threads = [threading.Thread(target=call, args=(n,)) for n in range(8)]
+[t.start() for t in threads], [t.join() for t in threads]
+assert all(isinstance(o, torch.Tensor) for o in out), out
+torch.cuda.synchronize()
+assert all(torch.equal(o, out[0]) for o in out) and _lib.device_status() == 0
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300, cwd=pathlib.Path(__file__).parent.parent)
 
 
 @pytest.mark.parametrize("L", [34, 130, 1000, 4200])
