@@ -3,6 +3,8 @@
 //   D <= 64 -> fwd_tc5_pair64.cu  (two query tiles per CTA share every key stage)
 //   D = 128 -> fwd_tc5_pipe128.cu (score products of the next key tile under the softmax of this one)
 // Both follow the register-tiled kernel in fwd_generic.cu in what they compute (jvp_attention.py:125-336, 1011-1033).
+#include <mutex>
+
 #include "tc5_common.cuh"
 
 namespace jvpfa {
@@ -18,9 +20,12 @@ struct StatusSlot {
 };
 StatusSlot* status_slot() {
   static StatusSlot cache[64];
+  static std::mutex setup;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
   StatusSlot& sl = cache[dev];
+  if (__atomic_load_n(&sl.dev, __ATOMIC_ACQUIRE)) return &sl;
+  std::lock_guard<std::mutex> lock(setup);  // (calls are launched without the interpreter lock)
   if (!sl.dev) {
     int* p = nullptr;
     if (cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_tc5_status) != cudaSuccess) return nullptr;
@@ -36,7 +41,7 @@ StatusSlot* status_slot() {
       }
     }
     (void)cudaGetLastError();  // a missing mirror only costs the early warning
-    sl.dev = p;
+    __atomic_store_n(&sl.dev, p, __ATOMIC_RELEASE);
   }
   return &sl;
 }
@@ -66,16 +71,12 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 static EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
+  static const EncodeTiledFn fn = []() -> EncodeTiledFn {  // (once, and whoever comes meanwhile waits for it)
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
+    const cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q);
+    return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<EncodeTiledFn>(p) : nullptr;
+  }();
   return fn;
 }
 
