@@ -492,7 +492,7 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
       if (mbar_wait(meet + quarter, n_tiles & 1, ab, kAbortAux)) {
         l_run = sums[row] + sums[BM + row];
         mu_run = sums[2 * BM + row] + sums[3 * BM + row];
-        const bool none = !(l_run > 0.f);
+        const bool none = !(l_run > 0.f);  // no key, or what is not a number: sums of zeros stay zeros, and NaN stays NaN
         const float inv_l = none ? 0.f : 1.f / l_run;
         const float mu = mu_run * inv_l;
         if (i < L) {
@@ -507,12 +507,12 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
             for (int c = 0; c < C::W_OUT / 4; ++c) {
               float o[4];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) o[e] = none ? 0.f : acc_o[4 * c + e] * inv_l;
+              for (int e = 0; e < 4; ++e) o[e] = acc_o[4 * c + e] * inv_l;
               po[c] = make_float4(o[0], o[1], o[2], o[3]);
               if constexpr (DUAL) {
                 float u[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) u[e] = none ? 0.f : acc_t[4 * c + e] * inv_l - mu * o[e];
+                for (int e = 0; e < 4; ++e) u[e] = acc_t[4 * c + e] * inv_l - mu * o[e];
                 pt[c] = make_float4(u[0], u[1], u[2], u[3]);
               }
             }

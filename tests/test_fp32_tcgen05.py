@@ -401,6 +401,32 @@ def test_a_large_entry_costs_the_others_nothing(D, big):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+@pytest.mark.parametrize("where", ["q", "k", "v", "tq", "tk", "tv", "go"])
+def test_what_is_not_finite_reaches_what_it_reached(monkeypatch, D, bad, where):
+    """One entry that is not a number, or Inf: the results that are finite are those of the register-tiled kernels, with and without
+    rows that have no key.  (Of the gradients under a mask some more: a masked pair has none here, where those kernels have 0 * NaN.)"""
+    from jvp_flash_attention_b200 import jvp_attention as ja
+
+    (B, H, L), g, ts = _range_inputs(D)
+    q, k, v, tq, tk, tv, go = (x.to(DEV) for x in ts)
+    dict(q=q, k=k, v=v, tq=tq, tk=tk, tv=tv, go=go)[where][:, ::2, L // 3, 7] = bad
+    mask = torch.rand(B, 1, L, L, generator=g).to(DEV) > 0.3
+    mask[:, :, 5] = False
+    for m in (None, mask):
+        finite = {}
+        for impl in (_lib.IMPL_GENERIC, _lib.IMPL_AUTO):
+            monkeypatch.setattr(ja, "KERNEL_IMPL", impl)
+            dual = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, attn_mask=m), (q, k, v), (tq, tk, tv))
+            a = [x.clone().requires_grad_() for x in (q, k, v)]
+            o = ja.attention(*a, attn_mask=m)
+            finite[impl] = [torch.isfinite(x.detach()) for x in (*dual, o, *torch.autograd.grad(o, a, go))]
+        for n, (x, y) in enumerate(zip(finite[_lib.IMPL_GENERIC], finite[_lib.IMPL_AUTO])):
+            assert torch.equal(x, y if m is None or n < 3 else x & y), (n, m is not None, x.float().mean().item(), y.float().mean().item())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64, 128])
 def test_rows_and_channels_of_very_different_magnitude(D):
     """Rows of V and its tangent up to a factor of 2^40 apart, masked-out keys that hold 1e15, and a channel of q a million times
     larger where k is that much smaller: 1e-5 of P |V| for O, of the head's largest V for tO, of a gradient's largest entry."""
