@@ -936,6 +936,8 @@ int launch_bwd_f32_tc5(const jvpfa_bwd_args& a, cudaStream_t stream) {
   s.plane = (long long)a.B * a.H * a.L * a.D;
   s.H = a.H, s.L = a.L, s.D = a.D;
   if (a.mask.kind == JVPFA_MASK_KVLEN) s.kv_len = a.mask.kv_len, s.padded = 1u << kDqSlotK | 1u << kDqSlotV;
+  // (dQ alone: the rows that attend such a key have a delta, or a cterm, that is not a number)
+  if (a.mask.kind == JVPFA_MASK_CAUSAL && (a.flags & JVPFA_SKIP_DKDV)) s.clean = 1u << kDqSlotK | 1u << kDqSlotV;
   s.set(kDqSlotQ, a.q, a.in_stride), s.set(kDqSlotK, a.k, a.in_stride), s.set(kDqSlotV, a.v, a.in_stride);
   if (a.gto) {
     s.set(kDqSlotA, a.tq, a.in_stride), s.set(kDqSlotB, a.gto, nullptr);

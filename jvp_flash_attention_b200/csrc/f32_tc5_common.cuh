@@ -16,6 +16,7 @@ namespace jvpfa {
 namespace tc5 {
 
 constexpr int kF32MaxSlots = 6;
+constexpr int kSplitBlock = 256 * 8;  // elements that a block of the splitting pass takes
 
 // Beside the status word: a wait of an fp32 kernel gave up.  Only this ends a later one on entry: an fp32 call that is queued, or
 // replayed, behind a 16-bit launch that gave up is computed, as on the register-tiled kernels.
@@ -31,6 +32,11 @@ struct SplitArgs {
   // into the products whole, and an Inf or a NaN there would reach every row through its probability of 0.
   const int32_t* kv_len;
   unsigned padded;
+  // Causal: what is not finite in the slots of `clean` is written as zero, for the same reason (rows of a query tile that end before
+  // the key).  `found` (or null): which blocks of kSplitBlock elements of those slots, one after another, hold such an entry; the
+  // kernel then looks at the entries themselves for the rows that attend them.
+  unsigned clean;
+  uint32_t* found;
   void set(int slot, const void* p, const int64_t* in_stride) {  // in_stride all zero or null: row-major
     src[slot] = static_cast<const float*>(p);
     const bool strided = in_stride && (in_stride[0] | in_stride[1] | in_stride[2]) != 0;

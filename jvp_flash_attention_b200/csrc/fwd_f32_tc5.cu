@@ -34,6 +34,7 @@ struct FwdF32Cfg {
   static constexpr int BM = 128, BN = 64;
   static constexpr bool DUAL = MODE != kPrimal;  // has tQ
   static constexpr bool TKV = MODE == kDual;     // has tK, tV
+  static constexpr int SLOTS = MODE == kPrimal ? 3 : TKV ? 6 : 4;  // tensors in the workspace
   static constexpr int NSL = D > 64 ? 2 : 1;     // 64-column slices of D
   static constexpr int KS = D < 64 ? D / 16 : 4;  // contraction steps of a slice
   static constexpr int NTHREADS = 384;
@@ -353,6 +354,16 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
       mbar_arrive(qlo_full);
     }
     const F32RowMask<MK> rm(a.mask, a.mask_bits, b, h, a.H, i, L);
+    // Causal: whether V or tV holds what is not finite up to the last key of this tile, block by block of the splitting pass.
+    const long long plane = (long long)BH * L * D, n_blocks = (plane + kSplitBlock - 1) / kSplitBlock;
+    const uint32_t* found = reinterpret_cast<const uint32_t*>(parts + C::SLOTS * 3 * plane);
+    const long long block0 = (long long)bh * L * D / kSplitBlock, block1 = ((long long)bh * L + min(L, m0 + BM)) * D / kSplitBlock;
+    bool any_found = false;
+    if (MK == 0 && causal) {
+      for (long long x = block0 + lane; x <= min(block1, n_blocks - 1); x += 32)
+        any_found = any_found || found[x] != 0u || (TKV && found[n_blocks + x] != 0u);
+      any_found = __any_sync(0xffffffffu, any_found);
+    }
     float acc_o[C::W_OUT], acc_t[DUAL ? C::W_OUT : 1];
 #pragma unroll
     for (int x = 0; x < C::W_OUT; ++x) {
@@ -501,6 +512,28 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
             if constexpr (DUAL) a.mu[(size_t)bh * L + i] = mu;
           }
           if (D > 32 || w == 0) {
+            if constexpr (MK == 0) {
+              if (any_found) {  // the columns in which a key that this row attends is not finite
+                const bool strided = (a.in_stride[0] | a.in_stride[1] | a.in_stride[2]) != 0;
+                const long long row_stride = strided ? a.in_stride[2] : D;
+                const long long head = (strided ? b * a.in_stride[0] + h * a.in_stride[1] : (long long)bh * L * D) + C::W_OUT * w;
+                for (long long x = block0; x <= min(block1, n_blocks - 1); ++x) {
+                  if (found[x] == 0u && !(TKV && found[n_blocks + x] != 0u)) continue;
+                  const long long first = x * kSplitBlock / D - (long long)bh * L, end = min((long long)i + 1, first + kSplitBlock / D);
+                  for (long long j = max(first, 0ll); j < end; ++j) {
+#pragma unroll
+                    for (int c = 0; c < C::W_OUT; ++c) {
+                      if (!isfinite(reinterpret_cast<const float*>(a.v)[head + j * row_stride + c])) {
+                        acc_o[c] = poison_f32();
+                        if constexpr (DUAL) acc_t[c] = poison_f32();
+                      }
+                      if constexpr (TKV)
+                        if (!isfinite(reinterpret_cast<const float*>(a.tv)[head + j * row_stride + c])) acc_t[c] = poison_f32();
+                    }
+                  }
+                }
+              }
+            }
             float4* po = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.o) + ((size_t)bh * L + i) * D + C::W_OUT * w);
             float4* pt = DUAL ? reinterpret_cast<float4*>(reinterpret_cast<float*>(a.to) + ((size_t)bh * L + i) * D + C::W_OUT * w) : nullptr;
 #pragma unroll
@@ -544,35 +577,47 @@ fwd_f32_tc5_kernel(const jvpfa_fwd_args a, const __grid_constant__ CUtensorMap m
 // ---- the parts of the inputs ----------------------------------------------------------------------------------------
 // Eight elements of a row per thread.
 __global__ void __launch_bounds__(256) split3_kernel(const SplitArgs s) {
-  const long long e = ((long long)blockIdx.x * 256 + threadIdx.x) * 8;
-  if (e >= s.plane) return;
+  const long long e = (long long)blockIdx.x * kSplitBlock + threadIdx.x * 8;
   const int slot = blockIdx.y;
-  const long long row = e / s.D;
-  const int col = (int)(e - row * s.D);
-  const long long bh = row / s.L;
-  const int i = (int)(row - bh * s.L);
-  float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
-  if (s.kv_len == nullptr || !((s.padded >> slot) & 1u) || i < s.kv_len[bh / s.H]) {
-    const float4* src = reinterpret_cast<const float4*>(s.src[slot] + (bh / s.H) * s.st[slot][0] + (bh % s.H) * s.st[slot][1] +
-                                                        (long long)i * s.st[slot][2] + col);
-    x0 = __ldg(src), x1 = __ldg(src + 1);
-  }
-  const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-  uint32_t r[3][4];
+  const bool clean = (s.clean >> slot) & 1u;
+  bool found = false;
+  if (e < s.plane) {
+    const long long row = e / s.D;
+    const int col = (int)(e - row * s.D);
+    const long long bh = row / s.L;
+    const int i = (int)(row - bh * s.L);
+    float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
+    if (s.kv_len == nullptr || !((s.padded >> slot) & 1u) || i < s.kv_len[bh / s.H]) {
+      const float4* src = reinterpret_cast<const float4*>(s.src[slot] + (bh / s.H) * s.st[slot][0] + (bh % s.H) * s.st[slot][1] +
+                                                          (long long)i * s.st[slot][2] + col);
+      x0 = __ldg(src), x1 = __ldg(src + 1);
+    }
+    float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+    if (clean) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    float h[2], m[2], l[2];
-    split3(x[2 * c], h[0], m[0], l[0]);
-    split3(x[2 * c + 1], h[1], m[1], l[1]);
-    r[0][c] = pack_bf16(h[0], h[1]), r[1][c] = pack_bf16(m[0], m[1]), r[2][c] = pack_bf16(l[0], l[1]);
-  }
+      for (int c = 0; c < 8; ++c)
+        if (!isfinite(x[c])) found = true, x[c] = 0.f;
+    }
+    uint32_t r[3][4];
 #pragma unroll
-  for (int p = 0; p < 3; ++p)
-    *reinterpret_cast<uint4*>(s.dst + ((long long)slot * 3 + p) * s.plane + e) = make_uint4(r[p][0], r[p][1], r[p][2], r[p][3]);
+    for (int c = 0; c < 4; ++c) {
+      float h[2], m[2], l[2];
+      split3(x[2 * c], h[0], m[0], l[0]);
+      split3(x[2 * c + 1], h[1], m[1], l[1]);
+      r[0][c] = pack_bf16(h[0], h[1]), r[1][c] = pack_bf16(m[0], m[1]), r[2][c] = pack_bf16(l[0], l[1]);
+    }
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+      *reinterpret_cast<uint4*>(s.dst + ((long long)slot * 3 + p) * s.plane + e) = make_uint4(r[p][0], r[p][1], r[p][2], r[p][3]);
+  }
+  if (clean && s.found != nullptr) {
+    const int any = __syncthreads_or(found);
+    if (threadIdx.x == 0) s.found[__popc(s.clean & ((1u << slot) - 1u)) * gridDim.x + blockIdx.x] = any;
+  }
 }
 
 int launch_split3(const SplitArgs& s, int slots, cudaStream_t stream) {
-  const dim3 grid((unsigned)((s.plane / 8 + 255) / 256), slots);
+  const dim3 grid((unsigned)((s.plane + kSplitBlock - 1) / kSplitBlock), slots);
   split3_kernel<<<grid, 256, 0, stream>>>(s);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -619,7 +664,8 @@ static int fwd_f32_slots(const jvpfa_fwd_args& a) { return !a.tq ? 3 : (a.flags 
 long long fwd_f32_tc5_workspace(const jvpfa_fwd_args& a) {
   if (a.dtype != JVPFA_FP32 || a.impl == JVPFA_IMPL_GENERIC) return 0;
   if (a.impl == JVPFA_IMPL_AUTO && !tc5::f32_rows_enough(a.mask, a.B, a.H, a.L, a.D)) return 0;
-  return (long long)fwd_f32_slots(a) * 3 * 2 * a.B * a.H * a.L * a.D;
+  const long long plane = (long long)a.B * a.H * a.L * a.D, blocks = (plane + tc5::kSplitBlock - 1) / tc5::kSplitBlock;
+  return fwd_f32_slots(a) * 3 * 2 * plane + (a.mask.kind == JVPFA_MASK_CAUSAL ? 2 * 4 * blocks : 0);
 }
 
 bool fwd_f32_tc5_eligible(const jvpfa_fwd_args& a) {
@@ -642,6 +688,10 @@ int launch_fwd_f32_tc5(const jvpfa_fwd_args& a, cudaStream_t stream) {
   if (a.mask.kind == JVPFA_MASK_KVLEN) {
     s.kv_len = a.mask.kv_len;
     s.padded = 1u << kSlotK | 1u << kSlotV | 1u << kSlotTK | 1u << kSlotTV;
+  }
+  if (a.mask.kind == JVPFA_MASK_CAUSAL) {
+    s.clean = 1u << kSlotV | (slots == 6 ? 1u << kSlotTV : 0u);
+    s.found = reinterpret_cast<uint32_t*>(s.dst + slots * 3 * s.plane);
   }
   const void* src[kF32MaxSlots] = {a.q, a.k, a.v, a.tq, a.tk, a.tv};
   for (int n = 0; n < slots; ++n) s.set(n, src[n], a.in_stride);

@@ -401,6 +401,46 @@ def test_a_large_entry_costs_the_others_nothing(D, big):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("bad", [math.nan, -math.inf])
+@pytest.mark.parametrize("what,first", [("tail", 352), ("tail", 65), ("v", 130), ("tv", 447), ("k", 300), ("strided", 201)])
+def test_rows_before_a_key_that_is_not_finite(D, bad, what, first):
+    """Causal: rows that end before the key are what they are without it, also in its own tile, and the rows that attend it are not
+    finite where its value belongs: in its column, or in all of them."""
+    from jvp_flash_attention_b200 import jvp_attention as ja
+
+    (B, H, L), g, ts = _range_inputs(D)
+    q, k, v, tq, tk, tv, go = (x.to(DEV) for x in ts)
+    if what == "strided":
+        q, k, v, tq, tk, tv = (x.transpose(1, 2).contiguous().transpose(1, 2) for x in (q, k, v, tq, tk, tv))
+
+    def run(*leaves):
+        q_, k_, v_, tq_, tk_, tv_ = leaves
+        dual = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, causal=True), (q_, k_, v_), (tq_, tk_, tv_))
+        along_q = q_.clone().requires_grad_()
+        o = ja.attention(along_q, k_, v_, causal=True)
+        (dq,) = torch.autograd.grad(o, along_q, go, create_graph=True)
+        return *dual, o.detach(), dq.detach(), torch.autograd.grad(dq, along_q, tq_)[0]
+
+    clean = run(q, k, v, tq, tk, tv)
+    if what in ("tail", "strided"):
+        for x in (k, v, tk, tv):
+            x[:, :, first:] = bad
+    else:
+        dict(v=v, tv=tv, k=k)[what][:, :, first, 5] = bad
+    got = run(q, k, v, tq, tk, tv)
+    for n, (x, y) in enumerate(zip(got, clean)):
+        assert torch.equal(x[:, :, :first], y[:, :, :first]), n
+        if what == "tv" and n != 1:  # only tO has anything to do with it
+            assert torch.equal(x, y), n
+        elif what in ("v", "tv") and n < 3:
+            assert not torch.isfinite(x[:, :, first:, 5]).any(), n
+            assert torch.equal(x[..., :5], y[..., :5]) and torch.equal(x[..., 6:], y[..., 6:]), n
+        else:
+            assert not torch.isfinite(x[:, :, first:]).any(), n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64, 128])
 @pytest.mark.parametrize("bad", [math.nan, math.inf])
 @pytest.mark.parametrize("where", ["q", "k", "v", "tq", "tk", "tv", "go"])
 def test_what_is_not_finite_reaches_what_it_reached(monkeypatch, D, bad, where):
