@@ -656,7 +656,7 @@ def run_ours(args, rank, world, local):
         pre_bytes = 3 * n_el * 2 + 4 * B * H * L * 4
         kernels = [
             {"name": "fwd_tc5_pair64_kernel (fwd_dual)", "ms": br["fwd_dual"], "mma_executed": 6, "mma_algorithmic": 6},
-            {"name": "bwd_tc5_fused64_kernel + dq_convert_kernel (dQ, dK, dV in one pass)", "ms": br["bwd"],
+            {"name": "bwd_tc5_fused64_kernel + fused64_finish_kernel (dQ, dK, dV in one pass)", "ms": br["bwd"],
              "mma_executed": 10, "mma_algorithmic": 10},
             {"name": "bwd_tc5_d64_kernel x2 (two-launch backward; not part of the step)", "ms": br["bwd_two_launch_kernels"],
              "mma_executed": 15, "mma_algorithmic": 10},
@@ -699,7 +699,7 @@ def run_ours(args, rank, world, local):
                                   "memsets": 1},
             "roofline": {"bound": "tensor",
                          "kernel": "jvpfa_fwd (fwd_tc5_pair64_kernel)" if dom == "fwd_dual" else
-                         "jvpfa_bwd (bwd_tc5_fused64_kernel + dq_convert_kernel, timed as one call; 10 algorithmic "
+                         "jvpfa_bwd (bwd_tc5_fused64_kernel + fused64_finish_kernel, timed as one call; 10 algorithmic "
                          "MMAs, 10 executed)",
                          "achieved": ach, "peak": peaks["burst"],
                          "unit": "TFLOP/s", "frac": ach / peaks["burst"],

@@ -228,7 +228,7 @@ int64_t jvpfa_bwd_workspace(const jvpfa_bwd_args* args) {
   jvpfa_bwd_args full;
   const jvpfa_bwd_args* a = current_bwd_args(args, &full);
   if (validate_bwd(a) != JVPFA_OK) return 0;
-  return a->dtype == JVPFA_FP32 ? bwd_f32_tc5_workspace(*a) : bwd_bias_workspace(*a);
+  return a->dtype == JVPFA_FP32 ? bwd_f32_tc5_workspace(*a) : bwd_fused64_workspace(*a);
 }
 
 int jvpfa_fwd(const jvpfa_fwd_args* args, void* stream) {

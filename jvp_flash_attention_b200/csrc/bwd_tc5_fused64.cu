@@ -125,22 +125,102 @@ __device__ __forceinline__ void mma_ss_dyn(uint32_t d_tmem, uint32_t a_lo, uint3
 }
 
 struct FItem {
-  int bh, b, h, own0, loop_begin, n_sub;
+  int bh, b, h, own0, loop_begin, n_sub;  // a key tile and the n_sub sub-tiles of it that are this CTA's
 };
+
+// ---- Key tiles shared out among CTAs -----------------------------------------------------------
+// Dealt whole, 192 key tiles take two rounds of 148 CTAs where 1.3 rounds' worth of work is there, and 32 key tiles leave 116 SMs idle.
+// With a workspace the sub-tiles of all key tiles are one line that is cut into as many equal pieces as there are CTAs; a key
+// tile that is cut leaves its shares of dK and dV (fp32) in the workspace, and the kernel that converts dQ adds them up in their
+// order.  The line is ordered by head, key tile, sub-tile; a key tile's beginning (own tiles, first scores, epilogue) counts as kOpen
+// sub-tiles.  Measured on a B200 (start of the kernel, a sub-tile, a beginning; us): through O 5, 0.9, 2; through tO 7, 1.4, 2; both 6,
+// 1.7, 3.
+//
+// Dealt whole -> shared out, us with the kernel that follows, bf16, H24 L1024 / H4 L1024: through O 41.9 -> 35.9 / 21.6 -> 16.0, through tO
+// 59.6 -> 51.0 / 29.2 -> 20.2, both 70.4 -> 58.8 / 34.5 -> 22.0; B2 H12 L2048 with a boolean mask through tO 169 -> 158; fp16 B8 H12 L1024,
+// lengths in [L/2, L], both 177 -> 155.
+constexpr int kOpen = 2;
+constexpr int kMinPiece = 2;                       // a cut leaves at least so many sub-tiles on either side
+constexpr int kShareFloats = 128 * 64;             // one share of dK or dV, in 16-byte pieces: [16 pieces][128 keys]
+constexpr long long kShareHead = 16 * 1024;        // bytes: where each CTA begins, {key tile, sub-tile}
+constexpr long long split_bytes(int ctas) { return kShareHead + (long long)ctas * 4 * kShareFloats * 4; }
+
+// By one whole warp: where CTA c of G begins, as the number of the key tile (head * key tiles of a head + key tile) and the sub-tile.
+// A head's key tiles 0 .. T-1 have first - slope * r sub-tiles each.
+__device__ __forceinline__ int2 split_begin(const jvpfa_bwd_args& a, int c, int G) {
+  const int lane = threadIdx.x & 31;
+  const int first = (a.L + 63) / 64, slope = a.mask.kind == JVPFA_MASK_CAUSAL ? 2 : 0;
+  const int BH = a.B * a.H, per_head = (a.L + 127) / 128;
+  if (c <= 0) return make_int2(0, 0);
+  if (c >= G) return make_int2(BH * per_head, 0);
+  auto tiles = [&](int b) {
+    int n = a.L;
+    if (a.mask.kind == JVPFA_MASK_KVLEN) n = max(0, min(a.mask.kv_len[b], a.L));
+    return (n + 127) / 128;
+  };
+  auto upto = [&](int r) { return r * (first + kOpen) - slope * r * (r - 1) / 2; };  // (the host sees to 32 bits)
+  int b = 0;
+  int pos;
+  if (a.mask.kind != JVPFA_MASK_KVLEN) {
+    const int head = upto(tiles(0));
+    pos = (int)((unsigned)(BH * head) * (unsigned)c / (unsigned)G);
+    b = pos / head / a.H;
+    pos -= b * a.H * head;
+  } else {
+    auto batch = [&](int x) { return x < a.B ? a.H * upto(tiles(x)) : 0; };
+    int total = 0;
+    for (int x = lane; x < a.B; x += 32) total += batch(x);
+    for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
+    pos = (int)((unsigned)total * (unsigned)c / (unsigned)G);
+    b = a.B;
+    for (int x0 = 0; x0 < a.B; x0 += 32) {  // the entry that holds this place of the line
+      const int mine = batch(x0 + lane);
+      int upto_me = mine;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, upto_me, d);
+        if (lane >= d) upto_me += o;
+      }
+      const unsigned beyond = __ballot_sync(0xffffffffu, upto_me > pos);
+      if (beyond) {
+        const int src = __ffs(beyond) - 1;
+        b = x0 + src;
+        pos -= __shfl_sync(0xffffffffu, upto_me - mine, src);
+        break;
+      }
+      pos -= __shfl_sync(0xffffffffu, upto_me, 31);
+    }
+    if (b == a.B) return make_int2(BH * per_head, 0);  // (no key is attended to)
+  }
+  const int T = tiles(b);
+  const int head = upto(T);
+  const int bh = b * a.H + pos / head;
+  pos %= head;
+  int lo = 0, hi = T - 1;  // the last key tile that begins at or before pos
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (upto(mid) <= pos) lo = mid; else hi = mid - 1;
+  }
+  int r = lo;
+  const int n = first - slope * r;
+  int s = pos - upto(r) - kOpen;
+  if (s < kMinPiece) s = 0;
+  if (s > n - kMinPiece) s = 0, ++r;
+  return make_int2(bh * per_head + r, s);
+}
 
 // MK: 0 = none / causal / key padding (index comparisons); 1 = boolean mask, as bits or as bytes of any strides (each elementwise
 // thread requests the next sub-tile's 32 entries of its key when the scores of this one have left its registers); 2 = additive
 // bias of the element type, requested the same way.
 //
 // dQ of a bias call through tO is summed in a fixed order, as the two launches that served it sum it: a key tile's share goes to
-// a buffer of its own (dq_acc: [key tile][B*H][L][D] floats) and dq_sum_kernel adds them up.  Measured on a B200, the two
+// a buffer of its own (dq_acc: [key tile][B*H][L][D] floats) and fused64_finish_kernel adds them up.  Measured on a B200, the two
 // launches / this with the sum, us, bf16 through both outputs: B2 H12 L512 42 / 38, L1024 134 / 105, L2048 353 / 290, H4 L4096
 // 229 / 187; with 48 key tiles (B2 H12 L256) 22 / 28, with 32 (H1 L4096) 124 / 173.
 template <bool HAS_GT, int MK>
 constexpr bool kDqParts = HAS_GT && MK == 2;
-template <typename T, bool HAS_GO, bool HAS_GT, int MK>
+template <typename T, bool HAS_GO, bool HAS_GT, int MK, bool CUT>
 __global__ void __launch_bounds__(512, 1)
-bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps maps, float* dq_acc, int* status) {
+bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps maps, float* dq_acc, float* shares, int* status) {
   using C = BwdFCfg<HAS_GO, HAS_GT>;
   constexpr int D = 64, OWN = C::OWN, BL = C::BL, STAGES = C::STAGES, GSTAGES = C::GSTAGES;
 
@@ -184,20 +264,40 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
   const int n_own_tiles = (L + OWN - 1) / OWN;
   const int n_items = n_own_tiles * BH;
   const int G = (int)gridDim.x, cta = (int)blockIdx.x;
-  const int k_max = (n_items + G - 1) / G;
   unsigned char* order = smem + C::TILE_BYTES + 256;  // behind the barriers
-  const bool sorted = a.mask.kind == JVPFA_MASK_KVLEN && a.B <= kMaxSortedBatch && n_items > G;
-  if (sorted) {
+  int* s_cut = reinterpret_cast<int*>(smem + C::TILE_BYTES + 384);  // CUT: {key tile, sub-tile} where this CTA and the next begin
+  const bool sorted = !CUT && a.mask.kind == JVPFA_MASK_KVLEN && a.B <= kMaxSortedBatch && n_items > G;
+  if constexpr (CUT) {
+    if (warp < 2) {
+      const int2 at = split_begin(a, cta + warp, G);
+      if (lane == 0) {
+        s_cut[2 * warp] = at.x, s_cut[2 * warp + 1] = at.y;
+        if (warp == 0) reinterpret_cast<int2*>(shares)[cta] = at;
+      }
+    }
+    __syncthreads();
+  } else if (sorted) {
     sort_batch(a.mask, a.B, order);
     __syncthreads();
   }
 
-  // Item k of this CTA: ranked heaviest first (causal: the first key tile sees every query), dealt in serpentine order.
-  auto get_item = [&](int k, FItem& it) -> bool {
-    const int w = k * G + ((k & 1) ? (G - 1 - cta) : cta);
-    if (w >= n_items) return false;
-    const int rank = w / BH;
-    it.bh = w - rank * BH;
+  // This CTA's items, by `walk`: shared out, the key tile's number; dealt whole, the round, in serpentine order and ranked heaviest
+  // first (causal: the first key tile sees every query).
+  auto begin_items = [&]() { return CUT ? s_cut[0] : 0; };
+  auto first_sub = [&](int w) { return w == s_cut[0] ? s_cut[1] : 0; };
+  auto get_item = [&](int walk, FItem& it) -> bool {
+    int rank, s0 = 0;
+    if constexpr (CUT) {
+      s0 = first_sub(walk);
+      if (walk > s_cut[2] || (walk == s_cut[2] && s0 >= s_cut[3])) return false;
+      it.bh = walk / n_own_tiles;
+      rank = walk - it.bh * n_own_tiles;
+    } else {
+      const int w = walk * G + ((walk & 1) ? (G - 1 - cta) : cta);
+      if (w >= n_items) return false;
+      rank = w / BH;
+      it.bh = w - rank * BH;
+    }
     it.b = it.bh / a.H;
     it.h = it.bh - it.b * a.H;
     if (sorted) it.b = order[it.b], it.bh = it.b * a.H + it.h;
@@ -210,7 +310,18 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
     it.loop_begin = causal ? (it.own0 / BL) * BL : 0;
     it.n_sub = (L - it.loop_begin + BL - 1) / BL;
     if (it.own0 >= n_valid) it.n_sub = 0;
+    if constexpr (CUT) {
+      it.loop_begin += s0 * BL;
+      it.n_sub = (walk == s_cut[2] ? s_cut[3] : it.n_sub) - s0;
+    }
     return true;
+  };
+  // Place of an item's share, which = 0 dK, 1 dV; nullptr: the item is a whole key tile.
+  auto share = [&](int walk, int which) -> float* {
+    if (!CUT) return nullptr;
+    const bool cut_before = first_sub(walk) > 0;
+    if (!cut_before && walk != s_cut[2]) return nullptr;
+    return shares + kShareHead / 4 + (size_t)(2 * (2 * cta + (cut_before ? 0 : 1)) + which) * kShareFloats;
   };
   auto valid_keys = [&](int b) {
     int n_valid = L;
@@ -225,9 +336,9 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
   // not to be trusted
   auto poison = [&]() {
     FItem it;
-    for (int k = 0; k < k_max; ++k) {
-      if (!get_item(k, it)) continue;
+    for (int walk = begin_items(); get_item(walk, it); ++walk) {
       const int i = it.own0 + tid;
+      if (tid < OWN && share(walk, 0)) share(walk, 0)[4 * tid] = share(walk, 1)[4 * tid] = poison_f32();
       if (tid < OWN && i < L) {
         poison_row<T>(a.dk, (size_t)it.bh * L + i, D);
         poison_row<T>(a.dv, (size_t)it.bh * L + i, D);
@@ -302,8 +413,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       int g = 0, kact = 0;
       bool ok = true;
       FItem it;
-      for (int k = 0; ok && k < k_max; ++k) {
-        if (!get_item(k, it) || it.n_sub == 0) continue;
+      for (int walk = begin_items(); ok && get_item(walk, it); ++walk) {
+        if (it.n_sub == 0) continue;
         // The own tiles are single-buffered: every MMA that reads the previous item's must be complete.
         const int oset = kact % C::OWN_BUFS, ouse = kact / C::OWN_BUFS;  // set of own tiles and how often it was used
         if (ouse > 0 && !mbar_wait_backoff(own_free + oset, (ouse - 1) & 1, ab, kAbortBwdOwn)) break;
@@ -418,8 +529,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 #pragma unroll
             for (int ks = 1; ks < D / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 2, id);
           };
-          for (int k = 0; ok && k < k_max; ++k) {
-            if (!get_item(k, it) || it.n_sub == 0) continue;
+          for (int walk = begin_items(); ok && get_item(walk, it); ++walk) {
+            if (it.n_sub == 0) continue;
             const int oset = kact % C::OWN_BUFS;
             if (!mbar_wait_warp(own_full + oset, (kact / C::OWN_BUFS) & 1, ab, kAbortBwdOwn)) break;
             own_k = own_k0 + oset * OWNSET16;
@@ -487,8 +598,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 #pragma unroll
             for (int ks = 1; ks < BL / 16; ++ks) umma_ts_lo<true>(tmem + col, tmem + a_col + ks * 8, b_lo + ks * 128, idesc_kv);
           };
-          for (int k = 0; ok && k < k_max; ++k) {
-            if (!get_item(k, it) || it.n_sub == 0) continue;
+          for (int walk = begin_items(); ok && get_item(walk, it); ++walk) {
+            if (it.n_sub == 0) continue;
             for (int s = 0; s < it.n_sub; ++s, ++g) {
               const int st = g % STAGES;
               if (!mbar_wait_warp(p_full + (g & 1), (g >> 1) & 1, ab, kAbortBwdPFull) ||
@@ -537,8 +648,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 #pragma unroll
             for (int ks = 1; ks < OWN / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 128, b_lo + ks * 128, idesc_dq);
           };
-          for (int k = 0; ok && k < k_max; ++k) {
-            if (!get_item(k, it) || it.n_sub == 0) continue;
+          for (int walk = begin_items(); ok && get_item(walk, it); ++walk) {
+            if (it.n_sub == 0) continue;
             own_mn = own_mn0 + (kact % C::OWN_BUFS) * OWNSET16;
             for (int s = 0; s < it.n_sub; ++s, ++g) {
               if (!mbar_wait_warp(p_full + (g & 1), (g >> 1) & 1, ab, kAbortBwdPFull) ||
@@ -601,15 +712,23 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             Elem<T>::pack(__uint_as_float(r1[8 * x + 6]) * mul, __uint_as_float(r1[8 * x + 7]) * mul));
     };
 
-    for (int k = 0; alive && k < k_max; ++k) {
-      if (!get_item(k, it)) continue;
+    auto store_zeros = [&](int bh, int own_idx) {  // nothing attends these keys (they are all padding): the gradients are zero
+      uint32_t z[32];
+#pragma unroll
+      for (int x = 0; x < 32; ++x) z[x] = 0u;
+      store_row(wg == 0 ? a.dk : a.dv, bh, own_idx, z, z, 0.f);
+    };
+    if (CUT && a.mask.kind == JVPFA_MASK_KVLEN) {  // (weightless on the line: dealt to all CTAs alike)
+      for (int w = cta; w < n_items; w += G) {
+        const int bh = w / n_own_tiles, own0 = (w - bh * n_own_tiles) * OWN;
+        if (own0 >= valid_keys(bh / a.H)) store_zeros(bh, own0 + row);
+      }
+    }
+
+    for (int walk = begin_items(); alive && get_item(walk, it); ++walk) {
       const int own_idx = it.own0 + row;
       if (it.n_sub == 0) {
-        // nothing attends these keys (they are all padding): the gradients are zero
-        uint32_t z[32];
-#pragma unroll
-        for (int x = 0; x < 32; ++x) z[x] = 0u;
-        store_row(wg == 0 ? a.dk : a.dv, it.bh, own_idx, z, z, 0.f);
+        if (!CUT) store_zeros(it.bh, own_idx);
         continue;
       }
       const int n_valid = valid_keys(it.b);
@@ -765,7 +884,16 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
         tmem_wait_ld();
         tc_fence_before();
         mbar_arrive(acc_free);
-        store_row(wg == 0 ? a.dk : a.dv, it.bh, own_idx, r0, r1, wg == 0 ? a.sm_scale : 1.f);
+        if (float* const to = share(walk, wg)) {
+          uint4* p = reinterpret_cast<uint4*>(to) + row;
+#pragma unroll
+          for (int x = 0; x < 8; ++x) {
+            p[x * OWN] = make_uint4(r0[4 * x], r0[4 * x + 1], r0[4 * x + 2], r0[4 * x + 3]);
+            p[(8 + x) * OWN] = make_uint4(r1[4 * x], r1[4 * x + 1], r1[4 * x + 2], r1[4 * x + 3]);
+          }
+        } else {
+          store_row(wg == 0 ? a.dk : a.dv, it.bh, own_idx, r0, r1, wg == 0 ? a.sm_scale : 1.f);
+        }
       }
       ++kact;
     }
@@ -782,8 +910,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
     // the loop is taken from rb_ok, which one thread writes before a meeting and all read after it, so nobody can be
     // missing at the next one; and nothing between two meetings waits on another role.
     auto rb_meet = [&]() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
-    for (int k = 0; alive && k < k_max; ++k) {
-      if (!get_item(k, it) || it.n_sub == 0) continue;
+    for (int walk = begin_items(); alive && get_item(walk, it); ++walk) {
+      if (it.n_sub == 0) continue;
       for (int s = 0; s < it.n_sub; ++s, ++g) {
         // one thread polls for the warpgroup (every polling warp is traffic on the shared-memory port)
         if (tid == 384) *rb_ok = mbar_wait(dq_full, g & 1, ab, kAbortBwdDone) ? 1 : 0;
@@ -849,30 +977,67 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
   }
 }
 
-// dq = T(dq_acc * scale), 8 elements per thread
+// dK and dV of the key tiles that were cut: the sum of their shares, in the order of the line.  Block x of 8 * (ctas - 1) looks at
+// where CTA x / 8 + 1 begins: if that is the first cut of a key tile, the tile is this block's, an eighth of it (256 threads of 8
+// columns; blocks 0-3 of the eight dK, the others dV).
 template <typename T>
-__global__ void dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dq, long long n8, float scale) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n8) return;
-  const float4 lo = reinterpret_cast<const float4*>(acc)[2 * i], hi = reinterpret_cast<const float4*>(acc)[2 * i + 1];
-  reinterpret_cast<uint4*>(dq)[i] = make_uint4(Elem<T>::pack(lo.x * scale, lo.y * scale), Elem<T>::pack(lo.z * scale, lo.w * scale),
-                                               Elem<T>::pack(hi.x * scale, hi.y * scale), Elem<T>::pack(hi.z * scale, hi.w * scale));
+__device__ __forceinline__ void sum_shares(const jvpfa_bwd_args& a, const float* shares, int ctas, int block) {
+  const int2* begin = reinterpret_cast<const int2*>(shares);
+  const int j = block / 8 + 1, which = (block >> 2) & 1;
+  const int2 at = begin[j], before = begin[j - 1];
+  if (at.y == 0 || (before.x == at.x && before.y > 0)) return;
+  const int row = threadIdx.x & 127, piece = 4 * (block & 3) + 2 * (threadIdx.x >> 7);
+  const float4* p = reinterpret_cast<const float4*>(shares + kShareHead / 4) + piece * 128 + row;
+  auto slot = [&](int n) { return p + (size_t)(2 * n + which) * (kShareFloats / 4); };
+  const float4* q = slot(2 * (j - 1) + 1);  // the share that begins the tile is its CTA's last
+  float4 lo = q[0], hi = q[128];
+  int2 cur = at;
+  for (int m = j; m < ctas; ++m) {
+    const int2 next = m + 1 < ctas ? begin[m + 1] : make_int2(-1, 0);
+    if (next.x != cur.x || next.y != cur.y) {  // (else CTA m has nothing to do)
+      q = slot(2 * m);
+      const float4 l = q[0], h = q[128];
+      lo.x += l.x, lo.y += l.y, lo.z += l.z, lo.w += l.w;
+      hi.x += h.x, hi.y += h.y, hi.z += h.z, hi.w += h.w;
+    }
+    if (next.x != at.x || next.y == 0) break;
+    cur = next;
+  }
+  const int per_head = (a.L + 127) / 128, bh = at.x / per_head, key = (at.x - bh * per_head) * 128 + row;
+  if (key >= a.L) return;
+  const float mul = which ? 1.f : a.sm_scale;
+  T* out = reinterpret_cast<T*>(which ? a.dv : a.dk) + ((size_t)bh * a.L + key) * 64 + piece * 4;
+  *reinterpret_cast<uint4*>(out) = make_uint4(Elem<T>::pack(lo.x * mul, lo.y * mul), Elem<T>::pack(lo.z * mul, lo.w * mul),
+                                              Elem<T>::pack(hi.x * mul, hi.y * mul), Elem<T>::pack(hi.z * mul, hi.w * mul));
 }
 
-// dq = T(scale * sum of the n_parts key tiles' shares, in their order), 4 elements per thread.  Bound by reading them (B2 H12 L1024:
-// 50 MB, most of it still in L2).
+// What follows the single pass: dK and dV of cut key tiles (the first `cut` blocks), and dQ:
+//   n_parts = 0: dq = T(scale * the accumulation buffer), 8 elements per thread
+//   n_parts > 0: dq = T(scale * sum of the n_parts key tiles' shares of dQ, in their order), 4 elements per thread.  Bound by reading
+//                them (B2 H12 L1024: 50 MB, most of it still in L2).
 template <typename T>
-__global__ void __launch_bounds__(256) dq_sum_kernel(const float* __restrict__ parts, T* __restrict__ dq, long long n4, int n_parts, float scale) {
-  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+__global__ void __launch_bounds__(256)
+fused64_finish_kernel(const jvpfa_bwd_args a, const float* __restrict__ acc, long long n, int n_parts, const float* __restrict__ shares, int ctas, int cut) {
+  if ((int)blockIdx.x < cut) return sum_shares<T>(a, shares, ctas, blockIdx.x);
+  const long long i = (long long)((int)blockIdx.x - cut) * 256 + threadIdx.x;
+  const float scale = a.sm_scale;
+  if (n_parts == 0) {
+    if (i >= n / 8) return;
+    const float4 lo = reinterpret_cast<const float4*>(acc)[2 * i], hi = reinterpret_cast<const float4*>(acc)[2 * i + 1];
+    reinterpret_cast<uint4*>(a.dq)[i] = make_uint4(Elem<T>::pack(lo.x * scale, lo.y * scale), Elem<T>::pack(lo.z * scale, lo.w * scale),
+                                                   Elem<T>::pack(hi.x * scale, hi.y * scale), Elem<T>::pack(hi.z * scale, hi.w * scale));
+    return;
+  }
+  const long long n4 = n / 4;
   if (i >= n4) return;
-  const float4* p = reinterpret_cast<const float4*>(parts) + i;
+  const float4* p = reinterpret_cast<const float4*>(acc) + i;
   float4 s = __ldcs(p);
 #pragma unroll 8
   for (int k = 1; k < n_parts; ++k) {
     const float4 x = __ldcs(p + k * n4);
     s.x += x.x, s.y += x.y, s.z += x.z, s.w += x.w;
   }
-  reinterpret_cast<uint2*>(dq)[i] = make_uint2(Elem<T>::pack(s.x * scale, s.y * scale), Elem<T>::pack(s.z * scale, s.w * scale));
+  reinterpret_cast<uint2*>(a.dq)[i] = make_uint2(Elem<T>::pack(s.x * scale, s.y * scale), Elem<T>::pack(s.z * scale, s.w * scale));
 }
 
 static int fused_sm_count() {
@@ -885,6 +1050,58 @@ static int fused_sm_count() {
     cache[dev] = n;
   }
   return cache[dev];
+}
+
+// Floats for a key tile's share of dQ, of every key tile: as many bytes as the (B, H, L, L) bias itself has, up to half a GiB.
+// From 96 key tiles on: with fewer the two launches, of as many CTAs each, fill more of the 148 SMs.
+static long long bwd_bias_workspace(const jvpfa_bwd_args& a) {
+  if ((a.dtype != JVPFA_BF16 && a.dtype != JVPFA_FP16) || a.impl == JVPFA_IMPL_GENERIC || a.D != 64) return 0;
+  if (a.mask.kind != JVPFA_MASK_BIAS || a.gto == nullptr || (a.flags & JVPFA_SKIP_DKDV)) return 0;
+  if ((a.L & 15) != 0 || !tc5_mask_layout(a.mask, a.dtype, a.L)) return 0;
+  const long long key_tiles = (long long)((a.L + 127) / 128) * a.B * a.H;
+  if (key_tiles < 96) return 0;
+  const long long bytes = key_tiles * a.L * a.D * 4;
+  return bytes <= (1ll << 29) ? bytes : 0;
+}
+
+// CTAs among which the key tiles' sub-tiles are shared out; 0: the key tiles are dealt whole.  Both in sub-tiles of the CTA that has
+// the most: dealt whole, in rounds; shared out, an equal part, one more beginning of a key tile, and the time of 2.5 us that the
+// shares' way through the workspace takes.  A twenty-fifth less is asked for: the last round of key tiles dealt whole has the memory to itself.
+// (Lengths of a key padding are not known here: as if there were none.)  fp16 B3 H12 L1330 causal through O, which this leaves whole: 46
+// us, 51 shared out.
+static int split_ctas(const jvpfa_bwd_args& a, int sms) {
+  const int open = kOpen, shares = a.gto ? 2 : 3;
+  const long long T = (a.L + 127) / 128, S = (a.L + 63) / 64, items = T * a.B * a.H;
+  const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL;
+  const long long subs = (long long)a.B * a.H * (causal ? T * S - T * (T - 1) : T * S), cost = subs + items * open;
+  const long long ctas = subs / 4 < sms ? subs / 4 : sms;
+  if (ctas < 2 || cost * ctas >= 1ll << 32) return 0;  // (the line's places times CTAs fit 32 bits; that many rounds need no cuts)
+  const long long G = items < sms ? items : sms, rounds = (items + G - 1) / G;
+  long long whole = rounds * (S + open);
+  if (causal) {
+    whole = 0;
+    if (rounds > 8) return 0;  // (the lightest are dealt last and even out)
+    for (int at = 0; at <= 8; ++at) {
+      const long long c = (G - 1) * at / 8;
+      long long load = 0;
+      for (long long k = 0; k < rounds; ++k) {
+        const long long w = k * G + ((k & 1) ? G - 1 - c : c);
+        if (w < items) load += S - 2 * (w / ((long long)a.B * a.H)) + open;
+      }
+      whole = load > whole ? load : whole;
+    }
+  }
+  return (cost / ctas + open + shares) * 25 < whole * 24 ? (int)ctas : 0;
+}
+
+template <typename T, bool HAS_GO, bool HAS_GT, int MK, bool CUT>
+static cudaError_t run_fused64(const jvpfa_bwd_args& a, const BwdFMaps& m, float* dq_acc, float* shares, int* status, int grid, cudaStream_t stream) {
+  using C = BwdFCfg<HAS_GO, HAS_GT>;
+  auto kern = bwd_tc5_fused64_kernel<T, HAS_GO, HAS_GT, MK, CUT>;
+  static SmemOptIn opt_in;
+  if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return cudaErrorInvalidValue;
+  kern<<<grid, C::NTHREADS, C::SMEM_BYTES, stream>>>(a, m, dq_acc, shares, status);
+  return cudaGetLastError();
 }
 
 template <typename T, bool HAS_GO, bool HAS_GT, int MK>
@@ -927,26 +1144,30 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
     set_last_cuda_error(e, "cudaMemsetAsync(dq_accum)");
     return JVPFA_ERR_CUDA;
   }
-  auto kern = bwd_tc5_fused64_kernel<T, HAS_GO, HAS_GT, MK>;
-  static SmemOptIn opt_in;
-  if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return JVPFA_ERR_CUDA;
   const long long n_items = (long long)n_key_tiles * a.B * a.H;
-  const int grid = (int)(n_items < sms ? n_items : sms);
-  kern<<<grid, C::NTHREADS, C::SMEM_BYTES, stream>>>(a, m, dq_acc, status);
-  e = cudaGetLastError();
+  int grid = (int)(n_items < sms ? n_items : sms);
+  const long long used = parts ? bwd_bias_workspace(a) : 0;  // the split's workspace lies behind dQ's shares
+  const int ctas = split_ctas(a, sms);
+  float* shares = nullptr;
+  if (ctas > 0 && a.workspace != nullptr && (reinterpret_cast<uintptr_t>(a.workspace) & 15u) == 0 &&
+      a.workspace_bytes >= used + split_bytes(ctas)) {
+    shares = reinterpret_cast<float*>(static_cast<char*>(a.workspace) + used);
+    grid = ctas;
+  }
+  e = shares ? run_fused64<T, HAS_GO, HAS_GT, MK, true>(a, m, dq_acc, shares, status, grid, stream)
+             : run_fused64<T, HAS_GO, HAS_GT, MK, false>(a, m, dq_acc, nullptr, status, grid, stream);
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch bwd_tc5_fused64");
     return JVPFA_ERR_CUDA;
   }
-  const long long n8 = (long long)(n / 8);
-  if (a.flags & JVPFA_SKIP_DQ) return JVPFA_OK;
-  if (parts)
-    dq_sum_kernel<T><<<(unsigned)((2 * n8 + 255) / 256), 256, 0, stream>>>(dq_acc, reinterpret_cast<T*>(a.dq), 2 * n8, n_key_tiles, a.sm_scale);
-  else
-    dq_convert_kernel<T><<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(dq_acc, reinterpret_cast<T*>(a.dq), n8, a.sm_scale);
+  const int cut = shares ? 8 * (ctas - 1) : 0;
+  const long long per_block = parts ? 256 * 4 : 256 * 8;
+  const long long blocks = cut + (a.flags & JVPFA_SKIP_DQ ? 0 : ((long long)n + per_block - 1) / per_block);
+  if (blocks == 0) return JVPFA_OK;
+  fused64_finish_kernel<T><<<(unsigned)blocks, 256, 0, stream>>>(a, dq_acc, (long long)n, parts ? n_key_tiles : 0, shares, ctas, cut);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
-    set_last_cuda_error(e, "launch dq_convert");
+    set_last_cuda_error(e, "launch fused64_finish");
     return JVPFA_ERR_CUDA;
   }
   return JVPFA_OK;
@@ -982,7 +1203,7 @@ bool bwd_tc5_fused64_eligible(const jvpfa_bwd_args& a) {
   if (a.D != 64) return false;
   const int k = a.mask.kind;
   if (k == JVPFA_MASK_BIAS && a.gto != nullptr) {
-    const long long need = bwd_bias_workspace(a);
+    const long long need = tc5::bwd_bias_workspace(a);
     return need > 0 && a.workspace != nullptr && a.workspace_bytes >= need && (reinterpret_cast<uintptr_t>(a.workspace) & 15u) == 0;
   }
   if (a.dq_accum == nullptr || (reinterpret_cast<uintptr_t>(a.dq_accum) & 15u) != 0) return false;
@@ -993,16 +1214,18 @@ bool bwd_tc5_fused64_eligible(const jvpfa_bwd_args& a) {
   return k != JVPFA_MASK_BOOL || (a.mask_tile_live == nullptr && a.mask_tile_live_t == nullptr);
 }
 
-// Floats for a key tile's share of dQ, of every key tile: as many bytes as the (B, H, L, L) bias itself has, up to half a GiB.
-// From 96 key tiles on: with fewer the two launches, of as many CTAs each, fill more of the 148 SMs.
-long long bwd_bias_workspace(const jvpfa_bwd_args& a) {
-  if ((a.dtype != JVPFA_BF16 && a.dtype != JVPFA_FP16) || a.impl == JVPFA_IMPL_GENERIC || a.D != 64) return 0;
-  if (a.mask.kind != JVPFA_MASK_BIAS || a.gto == nullptr || (a.flags & JVPFA_SKIP_DKDV)) return 0;
-  if ((a.L & 15) != 0 || !tc5_mask_layout(a.mask, a.dtype, a.L)) return 0;
-  const long long key_tiles = (long long)((a.L + 127) / 128) * a.B * a.H;
-  if (key_tiles < 96) return 0;
-  const long long bytes = key_tiles * a.L * a.D * 4;
-  return bytes <= (1ll << 29) ? bytes : 0;
+// What the launch can use: shares of dQ (needed for a bias through tO), and of dK and dV where key tiles are cut.
+long long bwd_fused64_workspace(const jvpfa_bwd_args& a) {
+  if ((a.dtype != JVPFA_BF16 && a.dtype != JVPFA_FP16) || a.impl == JVPFA_IMPL_GENERIC || a.D != 64 || (a.flags & JVPFA_SKIP_DKDV)) return 0;
+  long long parts = 0;
+  if (a.mask.kind == JVPFA_MASK_BIAS && a.gto != nullptr) {
+    parts = tc5::bwd_bias_workspace(a);
+    if (parts == 0) return 0;
+  } else if (!bwd_tc5_fused64_eligible(a)) {
+    return 0;
+  }
+  const int ctas = tc5::split_ctas(a, tc5::fused_sm_count());
+  return parts + (ctas ? tc5::split_bytes(ctas) : 0);
 }
 
 int launch_bwd_tc5_fused64(const jvpfa_bwd_args& a, cudaStream_t s) {

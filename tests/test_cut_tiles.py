@@ -1,0 +1,57 @@
+"""Tiles shared out among CTAs: a tile that is cut leaves partial sums in a workspace, which are added up in a fixed order."""
+import pytest
+import torch
+
+from jvp_flash_attention_b200 import _lib
+from jvp_flash_attention_b200 import jvp_attention as ja
+from oracle import jvp_attention_oracle as orc
+
+DEV = "cuda:0"
+
+
+def _mask(kind, B, H, L, dt, g):
+    if kind == "keys":  # entries of one and of few keys, whole and ragged ones
+        lens = torch.tensor([2, 1, L, L // 2 + 3, L - 1] * B)[:B] if B > 1 else torch.tensor([L // 2 + 3])
+        return (torch.arange(L)[None, :] < lens[:, None])[:, None, None, :]
+    if kind == "bool":
+        return (torch.rand(B, H, L, L, generator=g) > 0.5) | torch.eye(L, dtype=torch.bool)
+    if kind == "bias":
+        return torch.randn(B, H, L, L, generator=g).clamp(-5, 5).to(dt)
+    return None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["none", "causal", "keys", "bool", "bias"])
+@pytest.mark.parametrize("B,H,L", [(1, 1, 1024), (1, 3, 1000), (5, 2, 720), (2, 12, 1024), (1, 150, 256)])
+@pytest.mark.parametrize("cot,dt", [("o", torch.float16), ("t", torch.bfloat16), ("both", torch.bfloat16)])
+def test_backward_of_cut_key_tiles(kind, B, H, L, cot, dt):
+    """Against the float64 oracle: 2e-2 of the largest entry at least 1, the 16-bit bound of the parity tests, and in the 2-norm 1e-2 for
+    bf16 and 2e-3 for fp16 (operands of 8 and 11 significant bits, four roundings on the longest way); dK and dV bit for bit the same
+    from run to run, also in a workspace full of NaN."""
+    g = torch.Generator().manual_seed(L + H)
+    ts = [(torch.randn(B, H, L, 64, generator=g) * (0.1 if n in (3, 4, 5) else 1.0)).to(dt) for n in range(8)]
+    mask, causal = _mask(kind, B, H, L, dt, g), kind == "causal"
+    n = min(H, 2)  # (the oracle looks at some of the heads)
+    few = lambda x: None if x is None else x[:, -n:] if x.shape[1] > 1 else x  # noqa: E731
+    go, gt = ts[6] if cot != "t" else None, ts[7] if cot != "o" else None
+    ref = orc.grads_through_both(*(few(x) for x in (*ts[:6], go, gt)), attn_mask=few(mask), causal=causal)
+    a = [x.to(DEV).requires_grad_() for x in ts[:3]]
+    m = None if mask is None else mask.to(DEV)
+    o, to = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, attn_mask=m, causal=causal), tuple(a), tuple(x.to(DEV) for x in ts[3:6]))
+    outs = [(x, w.to(DEV)) for x, w in ((o, go), (to, gt)) if w is not None]
+
+    def run():
+        junk = torch.full((1 << 24,), float("nan"), device=DEV)  # what the next allocations find
+        del junk
+        return torch.autograd.grad([x for x, _ in outs], a, [w for _, w in outs], retain_graph=True)
+
+    first = run()
+    for _ in range(3):
+        for x, y in zip(run()[1:], first[1:]):
+            assert torch.equal(x, y)
+    assert _lib.device_status() == 0
+    rel = 1e-2 if dt == torch.bfloat16 else 2e-3
+    for name, x, r in zip(("dq", "dk", "dv"), first, ref[2:]):
+        x = few(x).double().cpu()
+        assert orc.max_abs_err(x, r) <= 2e-2 * max(1.0, r.abs().max().item()), name
+        assert (x - r).norm() <= rel * r.norm() + 1e-6, name
