@@ -213,7 +213,8 @@ int jvpfa_fwd_uses_tcgen05(const jvpfa_fwd_args* args) {
 int64_t jvpfa_fwd_workspace(const jvpfa_fwd_args* args) {
   jvpfa_fwd_args full;
   const jvpfa_fwd_args* a = current_fwd_args(args, &full);
-  return validate_fwd(a) == JVPFA_OK ? fwd_f32_tc5_workspace(*a) : 0;
+  if (validate_fwd(a) != JVPFA_OK) return 0;
+  return a->dtype == JVPFA_FP32 ? fwd_f32_tc5_workspace(*a) : fwd_pair64_workspace(*a);
 }
 
 int jvpfa_bwd_uses_tcgen05(const jvpfa_bwd_args* args) {

@@ -140,72 +140,16 @@ struct FItem {
 // 59.6 -> 51.0 / 29.2 -> 20.2, both 70.4 -> 58.8 / 34.5 -> 22.0; B2 H12 L2048 with a boolean mask through tO 169 -> 158; fp16 B8 H12 L1024,
 // lengths in [L/2, L], both 177 -> 155.
 constexpr int kOpen = 2;
-constexpr int kMinPiece = 2;                       // a cut leaves at least so many sub-tiles on either side
 constexpr int kShareFloats = 128 * 64;             // one share of dK or dV, in 16-byte pieces: [16 pieces][128 keys]
 constexpr long long kShareHead = 16 * 1024;        // bytes: where each CTA begins, {key tile, sub-tile}
 constexpr long long split_bytes(int ctas) { return kShareHead + (long long)ctas * 4 * kShareFloats * 4; }
 
-// By one whole warp: where CTA c of G begins, as the number of the key tile (head * key tiles of a head + key tile) and the sub-tile.
-// A head's key tiles 0 .. T-1 have first - slope * r sub-tiles each.
 __device__ __forceinline__ int2 split_begin(const jvpfa_bwd_args& a, int c, int G) {
-  const int lane = threadIdx.x & 31;
-  const int first = (a.L + 63) / 64, slope = a.mask.kind == JVPFA_MASK_CAUSAL ? 2 : 0;
-  const int BH = a.B * a.H, per_head = (a.L + 127) / 128;
-  if (c <= 0) return make_int2(0, 0);
-  if (c >= G) return make_int2(BH * per_head, 0);
-  auto tiles = [&](int b) {
-    int n = a.L;
-    if (a.mask.kind == JVPFA_MASK_KVLEN) n = max(0, min(a.mask.kv_len[b], a.L));
-    return (n + 127) / 128;
-  };
-  auto upto = [&](int r) { return r * (first + kOpen) - slope * r * (r - 1) / 2; };  // (the host sees to 32 bits)
-  int b = 0;
-  int pos;
-  if (a.mask.kind != JVPFA_MASK_KVLEN) {
-    const int head = upto(tiles(0));
-    pos = (int)((unsigned)(BH * head) * (unsigned)c / (unsigned)G);
-    b = pos / head / a.H;
-    pos -= b * a.H * head;
-  } else {
-    auto batch = [&](int x) { return x < a.B ? a.H * upto(tiles(x)) : 0; };
-    int total = 0;
-    for (int x = lane; x < a.B; x += 32) total += batch(x);
-    for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
-    pos = (int)((unsigned)total * (unsigned)c / (unsigned)G);
-    b = a.B;
-    for (int x0 = 0; x0 < a.B; x0 += 32) {  // the entry that holds this place of the line
-      const int mine = batch(x0 + lane);
-      int upto_me = mine;
-      for (int d = 1; d < 32; d <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, upto_me, d);
-        if (lane >= d) upto_me += o;
-      }
-      const unsigned beyond = __ballot_sync(0xffffffffu, upto_me > pos);
-      if (beyond) {
-        const int src = __ffs(beyond) - 1;
-        b = x0 + src;
-        pos -= __shfl_sync(0xffffffffu, upto_me - mine, src);
-        break;
-      }
-      pos -= __shfl_sync(0xffffffffu, upto_me, 31);
-    }
-    if (b == a.B) return make_int2(BH * per_head, 0);  // (no key is attended to)
-  }
-  const int T = tiles(b);
-  const int head = upto(T);
-  const int bh = b * a.H + pos / head;
-  pos %= head;
-  int lo = 0, hi = T - 1;  // the last key tile that begins at or before pos
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) / 2;
-    if (upto(mid) <= pos) lo = mid; else hi = mid - 1;
-  }
-  int r = lo;
-  const int n = first - slope * r;
-  int s = pos - upto(r) - kOpen;
-  if (s < kMinPiece) s = 0;
-  if (s > n - kMinPiece) s = 0, ++r;
-  return make_int2(bh * per_head + r, s);
+  const int slope = a.mask.kind == JVPFA_MASK_CAUSAL ? -2 : 0, first = (a.L + 63) / 64;
+  return cut_begin(
+      a.mask.kind == JVPFA_MASK_KVLEN, a.B, a.H, (a.L + 127) / 128, slope, kOpen, 0, c, G,
+      [&](int b) { return ((a.mask.kind == JVPFA_MASK_KVLEN ? max(0, min(a.mask.kv_len[b], a.L)) : a.L) + 127) / 128; },
+      [&](int) { return first; }, [&](int, int r) { return first + slope * r; });
 }
 
 // MK: 0 = none / causal / key padding (index comparisons); 1 = boolean mask, as bits or as bytes of any strides (each elementwise
@@ -319,9 +263,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
   // Place of an item's share, which = 0 dK, 1 dV; nullptr: the item is a whole key tile.
   auto share = [&](int walk, int which) -> float* {
     if (!CUT) return nullptr;
-    const bool cut_before = first_sub(walk) > 0;
-    if (!cut_before && walk != s_cut[2]) return nullptr;
-    return shares + kShareHead / 4 + (size_t)(2 * (2 * cta + (cut_before ? 0 : 1)) + which) * kShareFloats;
+    const int place = cut_place(s_cut, walk, cta);
+    return place < 0 ? nullptr : shares + kShareHead / 4 + (size_t)(2 * place + which) * kShareFloats;
   };
   auto valid_keys = [&](int b) {
     int n_valid = L;
@@ -982,28 +925,18 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 // columns; blocks 0-3 of the eight dK, the others dV).
 template <typename T>
 __device__ __forceinline__ void sum_shares(const jvpfa_bwd_args& a, const float* shares, int ctas, int block) {
-  const int2* begin = reinterpret_cast<const int2*>(shares);
-  const int j = block / 8 + 1, which = (block >> 2) & 1;
-  const int2 at = begin[j], before = begin[j - 1];
-  if (at.y == 0 || (before.x == at.x && before.y > 0)) return;
-  const int row = threadIdx.x & 127, piece = 4 * (block & 3) + 2 * (threadIdx.x >> 7);
+  const int which = (block >> 2) & 1, row = threadIdx.x & 127, piece = 4 * (block & 3) + 2 * (threadIdx.x >> 7);
   const float4* p = reinterpret_cast<const float4*>(shares + kShareHead / 4) + piece * 128 + row;
-  auto slot = [&](int n) { return p + (size_t)(2 * n + which) * (kShareFloats / 4); };
-  const float4* q = slot(2 * (j - 1) + 1);  // the share that begins the tile is its CTA's last
-  float4 lo = q[0], hi = q[128];
-  int2 cur = at;
-  for (int m = j; m < ctas; ++m) {
-    const int2 next = m + 1 < ctas ? begin[m + 1] : make_int2(-1, 0);
-    if (next.x != cur.x || next.y != cur.y) {  // (else CTA m has nothing to do)
-      q = slot(2 * m);
-      const float4 l = q[0], h = q[128];
-      lo.x += l.x, lo.y += l.y, lo.z += l.z, lo.w += l.w;
-      hi.x += h.x, hi.y += h.y, hi.z += h.z, hi.w += h.w;
-    }
-    if (next.x != at.x || next.y == 0) break;
-    cur = next;
-  }
-  const int per_head = (a.L + 127) / 128, bh = at.x / per_head, key = (at.x - bh * per_head) * 128 + row;
+  float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+  int item;
+  if (!cut_shares(reinterpret_cast<const int2*>(shares), ctas, block / 8 + 1, &item, [&](int place) {
+        const float4* q = p + (size_t)(2 * place + which) * (kShareFloats / 4);
+        const float4 l = q[0], h = q[128];
+        lo.x += l.x, lo.y += l.y, lo.z += l.z, lo.w += l.w;
+        hi.x += h.x, hi.y += h.y, hi.z += h.z, hi.w += h.w;
+      }))
+    return;
+  const int per_head = (a.L + 127) / 128, bh = item / per_head, key = (item - bh * per_head) * 128 + row;
   if (key >= a.L) return;
   const float mul = which ? 1.f : a.sm_scale;
   T* out = reinterpret_cast<T*>(which ? a.dv : a.dk) + ((size_t)bh * a.L + key) * 64 + piece * 4;
@@ -1075,7 +1008,7 @@ static int split_ctas(const jvpfa_bwd_args& a, int sms) {
   const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL;
   const long long subs = (long long)a.B * a.H * (causal ? T * S - T * (T - 1) : T * S), cost = subs + items * open;
   const long long ctas = subs / 4 < sms ? subs / 4 : sms;
-  if (ctas < 2 || cost * ctas >= 1ll << 32) return 0;  // (the line's places times CTAs fit 32 bits; that many rounds need no cuts)
+  if (ctas < 2 || !cut_fits(cost, ctas)) return 0;  // (that many rounds need no cuts)
   const long long G = items < sms ? items : sms, rounds = (items + G - 1) / G;
   long long whole = rounds * (S + open);
   if (causal) {

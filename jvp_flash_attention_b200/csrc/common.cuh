@@ -523,6 +523,7 @@ int launch_bwd_tc5_d64(const jvpfa_bwd_args& a, cudaStream_t stream);
 int launch_bwd_tc5_fused64(const jvpfa_bwd_args& a, cudaStream_t stream);
 bool bwd_tc5_fused64_eligible(const jvpfa_bwd_args& a);
 long long bwd_fused64_workspace(const jvpfa_bwd_args& a);
+long long fwd_pair64_workspace(const jvpfa_fwd_args& a);
 int launch_fwd_tc5_pair64(const jvpfa_fwd_args& a, cudaStream_t stream);
 int launch_fwd_tc5_pipe128(const jvpfa_fwd_args& a, cudaStream_t stream);
 bool bwd_tc5_pipe128_eligible(const jvpfa_bwd_args& a);

@@ -95,7 +95,7 @@ struct PairItem {
   int bh, b, h, m0, n_valid;
   int nt0, nt1;      // key tiles in range of each query tile (0: the tile has no row or no key)
   int last0, last1;  // index of the last key tile each query tile uses, -1 when it uses none
-  int n_load;        // key tiles to walk: max(nt0, nt1)
+  int j0, n_load;    // key tiles to walk: [j0, n_load), up to max(nt0, nt1) where the item is not cut
   const unsigned long long *live0, *live1;  // MK == 3: the query tiles' words of the tile bitmap
   __device__ __forceinline__ int nt(int x) const { return x ? nt1 : nt0; }
   __device__ __forceinline__ int last(int x) const { return x ? last1 : last0; }
@@ -122,9 +122,35 @@ struct TileUse {
   }
 };
 
-template <typename T, bool DUAL, int MK>
+// ---- Pairs shared out among CTAs ----------------------------------------------------------------
+// Dealt whole, 192 pairs (B2 H12 L2048) take two rounds of 148 CTAs where 1.3 rounds' worth of work is there, and 16 leave 132 SMs idle.
+// With a workspace the key tiles of all pairs are one line that is cut into equal pieces (cut_begin); a pair that is cut leaves what
+// each CTA has of it, O and tO' before the division and the rows' statistics, all fp32, in the workspace, and pair64_finish_kernel
+// merges them in their order.  A pair's beginning counts as kPairOpen key tiles.
+constexpr int kPairOpen = 2;
+template <bool DUAL>
+struct PairShare {  // floats: [query tile][16-byte piece of O, then of tO'][128 rows], then [128 rows]{maximum, sum, sum of W, -}
+  static constexpr int PIECES = DUAL ? 32 : 16;
+  static constexpr int TILE = (PIECES + 1) * 128 * 4;
+  static constexpr int SIZE = 2 * TILE;
+  static constexpr long long HEAD = 16 * 1024;  // bytes: where each CTA begins, {pair, key tile}
+  static constexpr long long bytes(int ctas) { return HEAD + (long long)ctas * 2 * SIZE * 4; }
+};
+__device__ __forceinline__ int2 pair_begin(const jvpfa_fwd_args& a, int whole, int c, int G) {
+  const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL;
+  const int n_pairs = (a.L + 255) / 256, n_keys = (a.L + 63) / 64;
+  auto first = [&](int b) {
+    if (causal) return 4;
+    return a.mask.kind == JVPFA_MASK_KVLEN ? (max(0, min(a.mask.kv_len[b], a.L)) + 63) / 64 : n_keys;
+  };
+  return cut_begin(
+      a.mask.kind == JVPFA_MASK_KVLEN, a.B, a.H, n_pairs, causal ? 4 : 0, kPairOpen, whole, c, G, [&](int) { return n_pairs; }, first,
+      [&](int b, int r) { return causal ? min(n_keys, 4 * r + 4) : first(b); });
+}
+
+template <typename T, bool DUAL, int MK, bool CUT>
 __global__ void __launch_bounds__(384, 1)
-fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMaps maps, int* status) {
+fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMaps maps, float* shares, int whole, int* status) {
   using C = FwdPairCfg<DUAL>;
   constexpr int D = 64, BM = C::BM, BN = C::BN, STAGES = C::STAGES;
 
@@ -158,21 +184,38 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
   const int n_pairs = (n_q_tiles + 1) / 2;
   const int n_items = n_pairs * BH;
   const int G = (int)gridDim.x, cta = (int)blockIdx.x;
-  const int k_max = (n_items + G - 1) / G;
   unsigned char* order = smem + C::OFF_ORDER;
-  const bool sorted = a.mask.kind == JVPFA_MASK_KVLEN && a.B <= kMaxSortedBatch && n_items > G;
+  int* s_cut = reinterpret_cast<int*>(order);  // CUT: {pair, key tile} where this CTA and the next begin
+  if constexpr (CUT) {
+    grid_launch_dependents();
+    if (warp < 2) {
+      const int2 at = pair_begin(a, whole, cta + warp, G);
+      if (lane == 0) {
+        s_cut[2 * warp] = at.x, s_cut[2 * warp + 1] = at.y;
+        if (warp == 0) reinterpret_cast<int2*>(shares)[cta] = at;
+      }
+    }
+    __syncthreads();
+  }
+  const bool sorted = !CUT && a.mask.kind == JVPFA_MASK_KVLEN && a.B <= kMaxSortedBatch && n_items > G;
   if (sorted) {
     sort_batch(a.mask, a.B, order);
     __syncthreads();
   }
 
-  // Item k of this CTA: items are ranked heaviest first (for causal masks the last pair is the longest) and
-  // dealt in serpentine order.
-  auto get_item = [&](int k, PairItem& it) -> bool {
-    const int w = k * G + ((k & 1) ? (G - 1 - cta) : cta);
+  // Item `walk` of this CTA.  Dealt whole, the round: items are ranked heaviest first (for causal masks the last pair is the longest) and
+  // dealt in serpentine order.  Shared out: `whole` rounds, from -whole to -1, then the pairs from s_cut[0] on.
+  auto begin_items = [&]() { return CUT ? -whole : 0; };
+  auto get_item = [&](int walk, PairItem& it) -> bool {
+    const int w = CUT ? (walk < 0 ? (walk + whole) * G + cta : s_cut[0] + walk) : walk * G + ((walk & 1) ? (G - 1 - cta) : cta);
+    int j0 = 0;
+    if constexpr (CUT) {
+      if (walk == 0) j0 = s_cut[1];
+      if (walk >= 0 && (w > s_cut[2] || (w == s_cut[2] && j0 >= s_cut[3]))) return false;
+    }
     if (w >= n_items) return false;
     int pair;
-    if (causal) {
+    if (!CUT && causal) {
       const int rank = w / BH;
       it.bh = w - rank * BH;
       pair = n_pairs - 1 - rank;
@@ -217,16 +260,34 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
       scan(0, it.nt0, it.last0, it.live0);
       scan(1, it.nt1, it.last1, it.live1);
     }
+    it.j0 = j0;
     it.n_load = max(it.nt0, it.nt1);
+    if constexpr (CUT) {
+      if (w == s_cut[2]) it.n_load = s_cut[3];
+      it.last0 = min(it.nt0, it.n_load) - 1, it.last1 = min(it.nt1, it.n_load) - 1;
+      if (it.last0 < j0) it.last0 = -1;
+      if (it.last1 < j0) it.last1 = -1;
+    }
     return true;
+  };
+  // This thread's place in the workspace for its row of query tile x of the item, which is cut; nullptr: it is not.
+  auto share = [&](int walk, int x, int row) -> float4* {
+    if (!CUT) return nullptr;
+    const int place = walk < 0 ? -1 : cut_place(s_cut, s_cut[0] + walk, cta);
+    return place < 0 ? nullptr
+                     : reinterpret_cast<float4*>(shares + PairShare<DUAL>::HEAD / 4 + (size_t)place * PairShare<DUAL>::SIZE +
+                                                 x * PairShare<DUAL>::TILE) + row;
   };
 
   // lse = NaN for every row of this CTA's items: the results of this launch are not to be trusted
   auto poison = [&]() {
     PairItem it;
-    for (int k = 0; k < k_max; ++k) {
-      if (!get_item(k, it)) continue;
+    for (int walk = begin_items(); get_item(walk, it); ++walk) {
       const int i = it.m0 + tid;
+      if (CUT && tid < 2 * BM) {
+        float4* to = share(walk, tid / BM, tid % BM);
+        if (to) to[PairShare<DUAL>::PIECES * BM] = make_float4(poison_f32(), poison_f32(), poison_f32(), 0.f);
+      }
       if (tid < 2 * BM && i < L) a.lse[(size_t)it.bh * L + i] = poison_f32();
     }
   };
@@ -278,8 +339,8 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         int g = 0, kact = 0;
         bool ok = true;
         PairItem it;
-        for (int k = 0; ok && k < k_max; ++k) {
-          if (!get_item(k, it) || it.n_load == 0) continue;
+        for (int walk = begin_items(); ok && get_item(walk, it); ++walk) {
+          if (it.n_load == 0) continue;
           // The Q tiles are single-buffered: both issuers must be through with the previous item's.
           if (kact > 0 && !mbar_wait(q_empty, (kact - 1) & 1, ab, kAbortQFull)) break;
           mbar_expect_tx(q_full, C::NQ * C::N_QT * C::Q_BYTES);
@@ -290,7 +351,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
             if constexpr (DUAL) tma_load_4d(dst + C::Q_BYTES, &maps.tq, q_full, 0, it.m0 + x * BM, it.h, it.b);
           }
           TileUse<MK> use(it);
-          for (int j = 0; j < it.n_load; ++j) {
+          for (int j = it.j0; j < it.n_load; ++j) {
             if (use(j) == 0) continue;
             const int st = g % STAGES;
             if (!mbar_wait(kv_empty + st, ((g / STAGES) & 1) ^ 1, ab, kAbortKvEmpty)) {
@@ -363,15 +424,15 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
           return true;
         };
 
-        for (int k = 0; ok && k < k_max; ++k) {
-          if (!get_item(k, it) || it.n_load == 0) continue;
+        for (int walk = begin_items(); ok && get_item(walk, it); ++walk) {
+          if (it.n_load == 0) continue;
           // waited for by both issuers in every item, used or not: a parity wait must see every phase
           if (!mbar_wait_warp(q_full, kact & 1, ab, kAbortQFull)) break;
           const int my_last = it.last(X);
           bool pend = false, pend_first = false, first = true;
           uint32_t pend_st = 0, pend_par = 0;
           TileUse<MK> use(it);
-          for (int j = 0; j < it.n_load; ++j) {
+          for (int j = it.j0; j < it.n_load; ++j) {
             const int m = use(j);
             if (m == 0) continue;
             if (!mbar_wait_warp_u32(bar_kv_full + 8 * st, st_par, ab, kAbortKvFull)) {
@@ -450,7 +511,6 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
     const float2 c2 = make_float2(scale_log2, scale_log2);
     const float2 sc2 = make_float2(a.sm_scale, a.sm_scale);
     bool alive = true;
-    int kx = 0;
     uint32_t t = 0;
 
     // The item's O / tO rows leave through the query tile's P / W buffers (idle between items) and one TMA store
@@ -535,14 +595,38 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
       return true;
     };
 
+    // What this CTA has of a row of a pair that is cut.
+    auto store_share = [&](float4* to, float m_used, float l_run, float mu_run) -> bool {
+      if (!mbar_wait(pv_done + X, (t - 1) & 1, ab, kAbortOFull)) return false;
+      tc_fence_after();
+      to[PairShare<DUAL>::PIECES * BM] = make_float4(m_used, l_run, mu_run, 0.f);
+#pragma unroll 1
+      for (int c = 0; c < PairShare<DUAL>::PIECES; c += 8) {
+        uint32_t r[32];
+        tmem_ld32(tO + 4 * c, r);  // (tO' follows O)
+        tmem_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          reinterpret_cast<uint4*>(to)[(c + e) * BM] = make_uint4(r[4 * e], r[4 * e + 1], r[4 * e + 2], r[4 * e + 3]);
+      }
+      tc_fence_before();
+      mbar_arrive(o_free + X);
+      return true;
+    };
+
     PairItem it;
-    for (int k = 0; alive && k < k_max; ++k) {
-      if (!get_item(k, it)) continue;
+    for (int walk = begin_items(); alive && get_item(walk, it); ++walk) {
       const int mX = it.m0 + X * BM;
       const int i = mX + row;
+      const bool used = !CUT || it.last(X) >= 0;
       if (it.last(X) < 0) {  // no live key for this query tile: zeros, lse = +inf
-        alive = epilogue(it, i, -INFINITY, 0.f, 0.f, false);
-        continue;
+        if constexpr (!CUT) {
+          alive = epilogue(it, i, -INFINITY, 0.f, 0.f, false);
+          continue;
+        } else if (float4* const to = share(walk, X, row)) {
+          to[PairShare<DUAL>::PIECES * BM] = make_float4(-INFINITY, 0.f, 0.f, 0.f);
+          continue;
+        }
       }
       const float slack = a.flags & kExactRowMax ? 0.f : 8.f;
       float m_used = -INFINITY, l_run = 0.f, mu_run = 0.f;
@@ -585,10 +669,10 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         }
       };
       constexpr bool AHEAD = MK == 1;
-      if constexpr (AHEAD) fetch_mask(0);
+      if constexpr (AHEAD) fetch_mask(it.j0 * BN);
       TileUse<MK> use(it);
       bool first = true;  // the item's first tile used by this query tile
-      for (int j = 0; j < it.n_load; ++j) {
+      for (int j = it.j0; j < it.n_load; ++j) {
         if (!(use(j) & (1 << X))) continue;
         const int n0 = j * BN;
         if constexpr (MK != 0 && !AHEAD) fetch_mask(n0);
@@ -599,11 +683,11 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         }
         tc_fence_after();
         uint32_t x0[32], x1[32];
-        uint32_t t0[DUAL && MK != 2 ? 32 : 1], t1[DUAL && MK != 2 ? 32 : 1];
+        uint32_t t0[DUAL && MK != 2 && !CUT ? 32 : 1], t1[DUAL && MK != 2 && !CUT ? 32 : 1];
         tmem_ld32(tS, x0);
         tmem_ld32(tS + 32, x1);
         // (the tangent scores together with the scores; beside a bias half a tile at a time, when it has been added)
-        constexpr bool TS_LATER = DUAL && MK == 2;
+        constexpr bool TS_LATER = DUAL && (MK == 2 || CUT);
         if constexpr (DUAL && !TS_LATER) {
           tmem_ld32(tTS, t0);
           tmem_ld32(tTS + 32, t1);
@@ -779,10 +863,12 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         ++t;
       }
       if (!alive) break;
-      if (!epilogue(it, i, m_used, l_run, mu_run, true)) break;
-      ++kx;
+      if (float4* const to = share(walk, X, row)) {
+        if (!store_share(to, m_used, l_run, mu_run)) break;
+      } else {
+        if (!epilogue(it, i, m_used, l_run, mu_run, used)) break;
+      }
     }
-    (void)kx;
     if (row == 0) tma_store_wait_all();  // shared memory must outlive the stores that read it
   }
   tc_fence_before();
@@ -801,6 +887,88 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
   }
 }
 
+// The rows of the pairs that were cut.  Block x of 8 * (ctas - 1) looks at where CTA x / 8 + 1 begins; a pair that is cut there first is
+// this block's, an eighth of it: 128 rows of one query tile, 8 columns a thread of O and, at the same places, of tO.  Bound by reading
+// the shares (B2 H12 L2048: 40 MB, in L2); nearly all pairs have two, so two are requested before the first is looked at.
+template <typename T, bool DUAL>
+__global__ void __launch_bounds__(256) pair64_finish_kernel(const jvpfa_fwd_args a, const float* __restrict__ shares, int ctas) {
+  using S = PairShare<DUAL>;
+  grid_wait();
+  const int2* begin = reinterpret_cast<const int2*>(shares);
+  const int j = blockIdx.x / 8 + 1;
+  const int2 first = begin[j], before = begin[j - 1];
+  int2 next = j + 1 < ctas ? begin[j + 1] : make_int2(-1, 0);
+  if (first.y == 0 || (before.x == first.x && before.y > 0)) return;
+  const int x = (blockIdx.x >> 2) & 1, row = threadIdx.x & 127, piece = 4 * (blockIdx.x & 3) + 2 * (threadIdx.x >> 7);
+  const float4* base = reinterpret_cast<const float4*>(shares + S::HEAD / 4) + x * (S::TILE / 4) + row;
+  struct Share {
+    float4 st, o[2], to[DUAL ? 2 : 1];
+  };
+  auto load = [&](int place, Share& v) {
+    const float4* p = base + (size_t)place * (S::SIZE / 4);
+    v.st = p[S::PIECES * 128];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      v.o[h] = p[(piece + h) * 128];
+      if constexpr (DUAL) v.to[h] = p[(16 + piece + h) * 128];
+    }
+  };
+  float m = -INFINITY, l = 0.f, mu = 0.f, o[8] = {}, to[8] = {};
+  auto add = [&](const Share& v) {
+    if (v.st.x == -INFINITY) return;  // no key of the share (and nothing but its statistics is there)
+    const float top = fmaxf(m, v.st.x), keep = fast_exp2(m - top), w = fast_exp2(v.st.x - top);
+    m = top;
+    l = keep * l + w * v.st.y;
+    mu = keep * mu + w * v.st.z;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      o[4 * h] = keep * o[4 * h] + w * v.o[h].x, o[4 * h + 1] = keep * o[4 * h + 1] + w * v.o[h].y;
+      o[4 * h + 2] = keep * o[4 * h + 2] + w * v.o[h].z, o[4 * h + 3] = keep * o[4 * h + 3] + w * v.o[h].w;
+      if constexpr (DUAL) {
+        to[4 * h] = keep * to[4 * h] + w * v.to[h].x, to[4 * h + 1] = keep * to[4 * h + 1] + w * v.to[h].y;
+        to[4 * h + 2] = keep * to[4 * h + 2] + w * v.to[h].z, to[4 * h + 3] = keep * to[4 * h + 3] + w * v.to[h].w;
+      }
+    }
+  };
+  Share u, v;
+  load(2 * (j - 1) + 1, u);  // the share that begins the pair is its CTA's last
+  v.st.x = -INFINITY;
+  if (next.x != first.x || next.y != first.y) load(2 * j, v);  // (else CTA j has nothing to do)
+  add(u);
+  add(v);
+  int2 cur = next;
+  for (int c = j + 1; cur.x == first.x && cur.y > 0; ++c) {
+    next = c + 1 < ctas ? begin[c + 1] : make_int2(-1, 0);
+    if (next.x != cur.x || next.y != cur.y) {
+      load(2 * c, u);
+      add(u);
+    }
+    cur = next;
+  }
+  const int item = first.x;
+  const int n_pairs = (a.L + 255) / 256, bh = item / n_pairs, i = (item - bh * n_pairs) * 256 + x * 128 + row;
+  if (i >= a.L) return;
+  const bool empty = !(l > 0.f);
+  const float inv_l = empty ? 0.f : 1.f / l, mu_n = mu * inv_l;
+  const size_t at = (size_t)bh * a.L + i;
+  if (piece == 0) {
+    a.lse[at] = empty ? INFINITY : m + log2f(l);
+    if constexpr (DUAL) a.mu[at] = mu_n;
+  }
+  if (4 * piece >= a.D) return;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    o[e] *= inv_l;
+    if constexpr (DUAL) to[e] = to[e] * inv_l - mu_n * o[e];
+  }
+  auto store = [&](void* p, const float (&v)[8]) {
+    *reinterpret_cast<uint4*>(static_cast<T*>(p) + at * a.D + 4 * piece) =
+        make_uint4(Elem<T>::pack(v[0], v[1]), Elem<T>::pack(v[2], v[3]), Elem<T>::pack(v[4], v[5]), Elem<T>::pack(v[6], v[7]));
+  };
+  store(a.o, o);
+  if constexpr (DUAL) store(a.to, to);
+}
+
 static int pair_sm_count() {
   static int cache[64] = {};
   int dev = 0;
@@ -811,6 +979,53 @@ static int pair_sm_count() {
     cache[dev] = n;
   }
   return cache[dev];
+}
+
+// How the pairs are dealt: `ctas` CTAs among which their key tiles are shared out, after `whole` rounds of pairs as a whole; ctas = 0: all
+// as a whole.  Both ways in key tiles of the CTA that has the most.  The shares' way through the workspace takes as long as 8, and 12
+// where most CTAs have two of them.  Measured on a B200, replayed from a graph, us whole / shared out, bf16 with tangents: H4 L1024 29 / 21, H16 L1024 30 / 28,
+// H24 L1024 31 / 35, H4 L2048 51 / 30, H16 L2048 54 / 62, H24 L2048 99 / 82, H12 L4096 186 / 138; causal H16 L1024 28 / 24, H24 L2048 52 / 55, H8
+// L4096 94 / 62; without tangents H4 L1024 20 / 15, H24 L1024 21 / 23.  (All pairs in the line; with whole rounds first H24 L2048 79.)
+// Where tiles are stepped over their numbers are not known here: whole.  (Lengths of a key padding are not known either: as if there were none.)
+struct PairDeal {
+  int ctas, whole;
+};
+static PairDeal deal_pairs(const jvpfa_fwd_args& a, int sms) {
+  constexpr PairDeal all_whole{0, 0};
+  if (a.mask.kind == JVPFA_MASK_BOOL && a.mask_tile_live != nullptr) return all_whole;
+  const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL;
+  const long long P = (a.L + 255) / 256, N = (a.L + 63) / 64, BH = (long long)a.B * a.H, items = P * BH;
+  const long long steps = BH * (causal ? (P - 1) * P * 2 + N : P * N), line = BH * (causal ? P * (P + 1) * 2 : P * N) + items * kPairOpen;
+  const long long ctas = steps / 4 < sms ? steps / 4 : sms;
+  if (ctas < 2 || !cut_fits(line, ctas)) return all_whole;
+  const long long G = items < sms ? items : sms, rounds = (items + G - 1) / G;
+  long long most = rounds * N;
+  if (causal) {
+    most = 0;
+    if (rounds > 8) return all_whole;  // (the lightest are dealt last and even out)
+    for (int at = 0; at <= 8; ++at) {
+      const long long c = (G - 1) * at / 8;
+      long long load = 0;
+      for (long long k = 0; k < rounds; ++k) {
+        const long long w = k * G + ((k & 1) ? G - 1 - c : c);
+        if (w < items) load += N < 4 * (P - w / BH) ? N : 4 * (P - w / BH);
+      }
+      most = load > most ? load : most;
+    }
+  }
+  const long long whole = causal || a.mask.kind == JVPFA_MASK_KVLEN ? 0 : items / ctas;
+  const long long shared = whole > 0 ? whole * N + (items - whole * ctas) * N / ctas + 8 : steps / ctas + (2 * items > ctas ? 12 : 8);
+  return shared * 25 < most * 24 ? PairDeal{(int)ctas, (int)whole} : all_whole;
+}
+
+template <typename T, bool DUAL, int MK, bool CUT>
+static cudaError_t run_pair64(const jvpfa_fwd_args& a, const FwdPairMaps& maps, float* shares, int whole, int* status, int grid, cudaStream_t stream) {
+  using C = FwdPairCfg<DUAL>;
+  auto kern = fwd_tc5_pair64_kernel<T, DUAL, MK, CUT>;
+  static SmemOptIn opt_in;
+  if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return cudaErrorInvalidValue;
+  kern<<<grid, C::NTHREADS, C::SMEM_BYTES, stream>>>(a, maps, shares, whole, status);
+  return cudaGetLastError();
 }
 
 template <typename T, bool DUAL, int MK>
@@ -842,9 +1057,6 @@ static int launch_pair64(const jvpfa_fwd_args& a, cudaStream_t stream) {
     set_last_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled(fwd pair64)");
     return JVPFA_ERR_CUDA;
   }
-  auto kern = fwd_tc5_pair64_kernel<T, DUAL, MK>;
-  static SmemOptIn opt_in;
-  if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return JVPFA_ERR_CUDA;
   const int sms = pair_sm_count();
   if (sms <= 0) {
     set_last_cuda_error(cudaErrorUnknown, "multiprocessor count");
@@ -853,8 +1065,22 @@ static int launch_pair64(const jvpfa_fwd_args& a, cudaStream_t stream) {
   const long long n_q_tiles = (a.L + C::BM - 1) / C::BM;
   const long long n_items = ((n_q_tiles + 1) / 2) * BH;
   const int grid = (int)(n_items < sms ? n_items : sms);
-  kern<<<grid, C::NTHREADS, C::SMEM_BYTES, stream>>>(a, maps, status);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e;
+  if constexpr (MK != 3) {
+    const auto [ctas, whole] = deal_pairs(a, sms);
+    if (ctas > 0 && a.workspace != nullptr && (reinterpret_cast<uintptr_t>(a.workspace) & 15u) == 0 &&
+        a.workspace_bytes >= PairShare<DUAL>::bytes(ctas)) {
+      float* shares = static_cast<float*>(a.workspace);
+      e = run_pair64<T, DUAL, MK, true>(a, maps, shares, whole, status, ctas, stream);
+      if (e == cudaSuccess) {
+        e = launch_behind(pair64_finish_kernel<T, DUAL>, 8 * (ctas - 1), 256, 0, stream, a, static_cast<const float*>(shares), ctas);
+      }
+    } else {
+      e = run_pair64<T, DUAL, MK, false>(a, maps, nullptr, 0, status, grid, stream);
+    }
+  } else {
+    e = run_pair64<T, DUAL, MK, false>(a, maps, nullptr, 0, status, grid, stream);
+  }
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch fwd_tc5_pair64");
     return JVPFA_ERR_CUDA;
@@ -873,6 +1099,13 @@ static int launch_pair64_t(const jvpfa_fwd_args& a, cudaStream_t s) {
 }
 
 }  // namespace tc5
+
+// What the launch can use where pairs are cut.
+long long fwd_pair64_workspace(const jvpfa_fwd_args& a) {
+  if (a.impl == JVPFA_IMPL_GENERIC || a.D > 64 || !fwd_tc5_eligible(a)) return 0;
+  const int ctas = tc5::deal_pairs(a, tc5::pair_sm_count()).ctas;
+  return ctas == 0 ? 0 : a.tq != nullptr ? tc5::PairShare<true>::bytes(ctas) : tc5::PairShare<false>::bytes(ctas);
+}
 
 int launch_fwd_tc5_pair64(const jvpfa_fwd_args& a, cudaStream_t s) {
   return a.dtype == JVPFA_BF16 ? tc5::launch_pair64_t<__nv_bfloat16>(a, s) : tc5::launch_pair64_t<__half>(a, s);

@@ -293,14 +293,14 @@ Tensor workspace_of(int64_t bytes, const Tensor& q) {
 
 py::object or_none(const Tensor& t) { return t.defined() ? py::cast(t) : py::object(py::none()); }
 
-// Gives an fp32 launch its workspace, and a boolean mask whose rows cannot be read 16 bytes at a time as bits (returned: they
+// Gives a launch its workspace, and an fp32 launch a boolean mask whose rows cannot be read 16 bytes at a time as bits (returned: they
 // live as long as the launch is being issued).
 template <typename Args>
 Tensor use_workspace(Args& a, const Tensor& workspace, const Call& call, const Tensor& q) {
   Tensor bits;
   if (!workspace.defined()) return bits;
   a.workspace = workspace.data_ptr(), a.workspace_bytes = workspace.numel();
-  if (a.mask.kind == JVPFA_MASK_BOOL && !whole_pieces(*call.mask, q.size(2))) {
+  if (q.scalar_type() == at::kFloat && a.mask.kind == JVPFA_MASK_BOOL && !whole_pieces(*call.mask, q.size(2))) {
     pack(*call.mask, q, bits, nullptr);
     a.mask_bits = data(bits);
   }
@@ -352,9 +352,10 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
   a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
   for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
-  const Tensor workspace = workspace_of(call.parts ? jvpfa_fwd_workspace(&a) : 0, q);
+  const bool fp32 = q.scalar_type() == at::kFloat;
+  const Tensor workspace = workspace_of(!fp32 || call.parts ? jvpfa_fwd_workspace(&a) : 0, q);
   const Tensor bits = use_workspace(a, workspace, call, q);
-  r.parts = workspace.defined();
+  r.parts = fp32 && workspace.defined();
   check_status(jvpfa_fwd(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "jvpfa_fwd");
   return r;
 }

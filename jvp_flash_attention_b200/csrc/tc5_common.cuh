@@ -301,6 +301,116 @@ __device__ __forceinline__ void sort_batch(const jvpfa_mask& m, int B, unsigned 
   }
 }
 
+// ---- Launches that follow one another ----------------------------------------------------------
+// A kernel launched by launch_behind is set up while the one before it on its stream still runs, and waits for that one's results where it
+// says grid_wait, before it reads or writes anything that the other may write or read; every block says so, or the kernel after it
+// could start too early.  The one before says from where on its successor may be set up.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... Params, typename... Args>
+cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr, cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  return e == cudaSuccess ? cudaGetLastError() : e;
+}
+
+// ---- Items shared out among CTAs --------------------------------------------------------------
+// Persistent kernels whose items (each with a loop of n steps) would leave a round of CTAs half empty share their steps out: the items
+// in a line, by head and by place in the head, cut into as many equal pieces as there are CTAs.  An item's beginning counts as `open`
+// steps.  Item r of a head of batch entry b stands for first(b) + slope * r steps (it may have fewer), tiles(b) of the per_head items
+// of a head stand in the line.  Where all items are alike, `whole` rounds of items are dealt whole and only the rest, from item whole * G on, is the line: fewer cuts.
+constexpr int kMinPiece = 2;  // a cut leaves at least so many steps on either side
+// By one whole warp: where CTA c of G begins, {head * per_head + r, step}.  steps(b, r): how many item r has.  The line's length times
+// G fits 32 bits (cut_fits).
+template <typename Tiles, typename First, typename Steps>
+__device__ __forceinline__ int2 cut_begin(bool by_entry, int B, int H, int per_head, int slope, int open, int whole, int c, int G, Tiles tiles,
+                                          First first, Steps steps) {
+  const int lane = threadIdx.x & 31;
+  if (c <= 0) return make_int2(whole * G, 0);
+  if (c >= G) return make_int2(B * H * per_head, 0);
+  if (!by_entry && slope == 0) {
+    const int n = first(0), item = n + open;
+    const int pos = (int)((unsigned)((B * H * per_head - whole * G) * item) * (unsigned)c / (unsigned)G);
+    int w = pos / item, s = pos - w * item - open;
+    if (s < kMinPiece) s = 0;
+    if (s > n - kMinPiece) s = 0, ++w;
+    return make_int2(whole * G + w, s);
+  }
+  auto upto = [&](int b, int r) { return r * (first(b) + open) + slope * (r * (r - 1) / 2); };
+  int b = 0, pos;
+  if (!by_entry) {  // all heads alike
+    const int head = upto(0, tiles(0));
+    pos = (int)((unsigned)(B * H * head) * (unsigned)c / (unsigned)G);
+    b = pos / head / H;
+    pos -= b * H * head;
+  } else {
+    auto batch = [&](int x) { return x < B ? H * upto(x, tiles(x)) : 0; };
+    int total = 0;
+    for (int x = lane; x < B; x += 32) total += batch(x);
+    for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
+    pos = (int)((unsigned)total * (unsigned)c / (unsigned)G);
+    b = B;
+    for (int x0 = 0; x0 < B; x0 += 32) {  // the entry that holds this place of the line
+      const int mine = batch(x0 + lane);
+      int upto_me = mine;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, upto_me, d);
+        if (lane >= d) upto_me += o;
+      }
+      const unsigned beyond = __ballot_sync(0xffffffffu, upto_me > pos);
+      if (beyond) {
+        const int src = __ffs(beyond) - 1;
+        b = x0 + src;
+        pos -= __shfl_sync(0xffffffffu, upto_me - mine, src);
+        break;
+      }
+      pos -= __shfl_sync(0xffffffffu, upto_me, 31);
+    }
+    if (b == B) return make_int2(B * H * per_head, 0);  // (an empty line)
+  }
+  const int T = tiles(b), head = upto(b, T);
+  const int bh = b * H + pos / head;
+  pos %= head;
+  int lo = 0, hi = T - 1;  // the last item that begins at or before pos
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (upto(b, mid) <= pos) lo = mid; else hi = mid - 1;
+  }
+  int r = lo, s = pos - upto(b, r) - open;
+  if (s < kMinPiece) s = 0;
+  if (s > steps(b, r) - kMinPiece) s = 0, ++r;
+  return make_int2(bh * per_head + r, s);
+}
+inline bool cut_fits(long long line, long long ctas) { return line * ctas < 1ll << 32 && line < 1ll << 31; }
+// CTA c's place in the workspace for its share of item w, which is not its as a whole: 2 c where it takes the item over, else 2 c + 1;
+// -1 where the whole item is its.  at: {item, step} where this CTA and the next begin.
+__device__ __forceinline__ int cut_place(const int* at, int w, int c) {
+  const bool before = w == at[0] && at[1] > 0;
+  return before || w == at[2] ? 2 * c + (before ? 0 : 1) : -1;
+}
+// Calls add(place) for the shares, in their order, of the item that is cut first where CTA j begins; false, and no call, if no item is.
+// begin: where each of the CTAs begins; item: the item.
+template <typename Add>
+__device__ __forceinline__ bool cut_shares(const int2* begin, int ctas, int j, int* item, Add add) {
+  const int2 at = begin[j], before = begin[j - 1];
+  if (at.y == 0 || (before.x == at.x && before.y > 0)) return false;
+  *item = at.x;
+  add(2 * (j - 1) + 1);  // the share that begins the item is its CTA's last
+  int2 cur = at;
+  for (int m = j; m < ctas; ++m) {
+    const int2 next = m + 1 < ctas ? begin[m + 1] : make_int2(-1, 0);
+    if (next.x != cur.x || next.y != cur.y) add(2 * m);  // (else CTA m has nothing to do)
+    if (next.x != at.x || next.y == 0) break;
+    cur = next;
+  }
+  return true;
+}
+
 // ---- TMA -----------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y,
                                             int z, int w) {
