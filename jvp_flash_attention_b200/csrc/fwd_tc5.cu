@@ -122,6 +122,11 @@ bool encode_map4d_f32(CUtensorMap* m, const void* ptr, int D, int L, int H, int 
   });
 }
 
+bool encode_map_bias(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int L, int rows, int H, int B, const int64_t* st,
+                     int box_rows) {
+  return encode_map4d(m, dt, ptr, L, rows, H, B, st, box_rows);
+}
+
 bool encode_map_parts(CUtensorMap* m, const void* ptr, int D, int L, int BH, int planes) {
   return encode_map4d(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, ptr, D, L, BH, planes, nullptr, 64);
 }

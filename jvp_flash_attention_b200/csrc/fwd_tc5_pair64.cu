@@ -23,8 +23,11 @@
 //
 // Masks (template parameter MK): 0 = none / causal / key padding by index comparison; 1 = uint8 mask;
 // 2 = additive bias of the element type; 3 = uint8 mask with the tile bitmap written by jvpfa_mask_tiles
-// (one bit per 128-query x 64-key tile).  A softmax thread owns one query row, so its share of a mask tile
-// is 64 consecutive elements, fetched as 16-byte read-only loads before the thread waits for the scores.
+// (one bit per 128-query x 64-key tile).  A softmax thread owns one query row, so its share of a boolean mask's tile is two words of
+// packed bits or 64 bytes, which it fetches itself.  A bias comes by TMA, a 128 x 64 tile for each query tile; its 32 KiB of
+// shared memory are what K and V with rings of their own save: K's stages are free when the scores exist, so two of each serve as
+// three of both.  (Fetched by the threads, 32 rows of a warp at a time, the bias took the L1 longer than the tile's arithmetic: a key
+// tile of a pair 3.05 us with tangents on a B200 where 1.5 without a mask; now 1.95.  B2 H12 L1024: with tangents 50 -> 36 us, without 33 -> 28.)
 // With a bitmap the two query tiles may need different key tiles: the producer loads the union, and an
 // issuer that does not use a loaded tile only releases it.
 #include "tc5_common.cuh"
@@ -32,13 +35,13 @@
 namespace jvpfa {
 namespace tc5 {
 
-template <bool DUAL>
+template <bool DUAL, bool BIAS>
 struct FwdPairCfg {
   static constexpr int D = 64;
   static constexpr int BM = 128;  // rows of one query tile
   static constexpr int NQ = 2;    // query tiles per CTA
   static constexpr int BN = 64;
-  static constexpr int STAGES = 3;
+  static constexpr int STAGES = BIAS ? 2 : 3;  // of K, V together, or with a bias of either
   static constexpr int NTHREADS = 384;  // warpgroup 0: TMA producer, two issuers, one idle warp; warpgroups 1, 2: softmax
   static constexpr int Q_BYTES = BM * D * 2;   // 16 KiB
   static constexpr int KV_BYTES = BN * D * 2;  // 8 KiB
@@ -46,12 +49,15 @@ struct FwdPairCfg {
   static constexpr int N_QT = DUAL ? 2 : 1;    // Q, tQ
   static constexpr int N_KV = DUAL ? 4 : 2;    // K, tK, V, tV
   static constexpr int N_P = DUAL ? 2 : 1;     // P, W
-  static constexpr int SLOT_K = 0, SLOT_TK = 1, SLOT_V = DUAL ? 2 : 1, SLOT_TV = 3;
-  static constexpr int STAGE_BYTES = N_KV * KV_BYTES;
+  static constexpr int HALF_BYTES = N_KV / 2 * KV_BYTES;               // K (, tK) or V (, tV) of a key tile
+  static constexpr int STAGE_BYTES = BIAS ? HALF_BYTES : 2 * HALF_BYTES;  // from one stage to the next
   static constexpr int OFF_Q = 0;
-  static constexpr int OFF_KV = NQ * N_QT * Q_BYTES;
-  static constexpr int OFF_P = OFF_KV + STAGES * STAGE_BYTES;
-  static constexpr int TILE_BYTES = OFF_P + NQ * N_P * P_BYTES;
+  static constexpr int OFF_K = NQ * N_QT * Q_BYTES;
+  static constexpr int OFF_V = OFF_K + (BIAS ? STAGES : 1) * HALF_BYTES;
+  static constexpr int OFF_P = OFF_K + STAGES * 2 * HALF_BYTES;
+  static constexpr int B_BYTES = BM * BN * 2;  // a bias tile
+  static constexpr int OFF_B = OFF_P + NQ * N_P * P_BYTES;
+  static constexpr int TILE_BYTES = OFF_B + (BIAS ? NQ * B_BYTES : 0);
   static constexpr int OFF_ORDER = TILE_BYTES + 256;  // behind the barriers
   static constexpr int SMEM_BYTES = OFF_ORDER + kMaxSortedBatch + 1024;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
@@ -68,6 +74,7 @@ struct FwdPairCfg {
 
 struct FwdPairMaps {
   CUtensorMap q, tq, k, tk, v, tv;
+  CUtensorMap bias;   // MK = 2; its own extents: a dimension that broadcasts has one entry
   CUtensorMap o, to;  // outputs, stored tile-wise from shared memory
 };
 
@@ -85,6 +92,9 @@ __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bu
 
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void lds_v4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 // Makes this thread's shared-memory writes visible to the async proxy (the tensor core reads operands through it).
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -151,8 +161,9 @@ __device__ __forceinline__ int2 pair_begin(const jvpfa_fwd_args& a, int whole, i
 template <typename T, bool DUAL, int MK, bool CUT>
 __global__ void __launch_bounds__(384, 1)
 fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMaps maps, float* shares, int whole, int* status) {
-  using C = FwdPairCfg<DUAL>;
+  using C = FwdPairCfg<DUAL, MK == 2>;
   constexpr int D = 64, BM = C::BM, BN = C::BN, STAGES = C::STAGES;
+  constexpr bool BIAS = MK == 2;
 
   const bool dead_on_entry = *(volatile int*)status != 0;  // an earlier bounded wait gave up
 
@@ -160,20 +171,26 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
   const uint32_t raw = smem_u32(smem_raw);
   unsigned char* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
   unsigned char* sQ = smem + C::OFF_Q;    // [query tile][Q, tQ]
-  unsigned char* sKV = smem + C::OFF_KV;  // [stage][K, tK, V, tV]
+  unsigned char* sK = smem + C::OFF_K;    // [stage][K, tK]; V, tV behind each stage's, or with a bias behind them all
+  unsigned char* sV = smem + C::OFF_V;
+  unsigned char* sB = smem + C::OFF_B;    // [query tile] bias
   unsigned char* sP = smem + C::OFF_P;    // [query tile][P, W]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::TILE_BYTES);
   uint64_t* q_full = bars + 0;
   uint64_t* q_empty = bars + 1;   // both issuers are through with the item's Q tiles
   uint64_t* kv_full = bars + 2;   // [STAGES]
   uint64_t* kv_empty = kv_full + STAGES;  // [STAGES], one arrival per issuer
-  uint64_t* s_full = kv_empty + STAGES;   // [2] per query tile from here on
+  uint64_t* v_full = kv_empty + STAGES;   // BIAS: V's ring; kv_full and kv_empty are K's
+  uint64_t* v_empty = v_full + (BIAS ? STAGES : 0);
+  uint64_t* s_full = v_empty + (BIAS ? STAGES : 0);  // [2] per query tile from here on
   uint64_t* s_free = s_full + 2;          // the softmax threads hold the scores in registers
   uint64_t* p_full = s_free + 2;          // P / W are in shared memory
   uint64_t* pv_done = p_full + 2;         // the tile's output MMAs are complete
   uint64_t* o_free = pv_done + 2;         // the epilogue has read the item's accumulators
   uint64_t* wg_bar = o_free + 2;          // meeting point of a softmax warpgroup's 128 threads (bounded, unlike bar.sync)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wg_bar + 2);
+  uint64_t* b_full = wg_bar + 2;          // BIAS: a tile of it is there
+  uint64_t* b_empty = b_full + (BIAS ? 2 : 0);  // ... has been added
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(b_empty + (BIAS ? 2 : 0));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -302,6 +319,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(kv_full + s, 1);
       mbar_init(kv_empty + s, 2);
+      if (BIAS) mbar_init(v_full + s, 1), mbar_init(v_empty + s, 2);
     }
     for (int x = 0; x < 2; ++x) {
       mbar_init(s_full + x, 1);
@@ -310,6 +328,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
       mbar_init(pv_done + x, 1);
       mbar_init(o_free + x, 128);
       mbar_init(wg_bar + x, 128);
+      if (BIAS) mbar_init(b_full + x, 1), mbar_init(b_empty + x, 128);
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -336,7 +355,8 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
       if (lane == 0) {
         prefetch_tmap(&maps.q), prefetch_tmap(&maps.k), prefetch_tmap(&maps.v);
         if constexpr (DUAL) prefetch_tmap(&maps.tq), prefetch_tmap(&maps.tk), prefetch_tmap(&maps.tv);
-        int g = 0, kact = 0;
+        if constexpr (BIAS) prefetch_tmap(&maps.bias);
+        int g = 0, kact = 0, nb0 = 0, nb1 = 0;  // nb: bias tiles of either query tile
         bool ok = true;
         PairItem it;
         for (int walk = begin_items(); ok && get_item(walk, it); ++walk) {
@@ -352,19 +372,40 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
           }
           TileUse<MK> use(it);
           for (int j = it.j0; j < it.n_load; ++j) {
-            if (use(j) == 0) continue;
-            const int st = g % STAGES;
-            if (!mbar_wait(kv_empty + st, ((g / STAGES) & 1) ^ 1, ab, kAbortKvEmpty)) {
+            const int m = use(j);
+            if (m == 0) continue;
+            const int st = g % STAGES, n0 = j * BN;
+            const uint32_t free_par = ((g / STAGES) & 1) ^ 1;
+            if (!mbar_wait(kv_empty + st, free_par, ab, kAbortKvEmpty)) {
               ok = false;
               break;
             }
-            unsigned char* base = sKV + st * C::STAGE_BYTES;
-            mbar_expect_tx(kv_full + st, C::STAGE_BYTES);
-            const int n0 = j * BN;
-            tma_load_4d(base + C::SLOT_K * C::KV_BYTES, &maps.k, kv_full + st, 0, n0, it.h, it.b);
-            if constexpr (DUAL) tma_load_4d(base + C::SLOT_TK * C::KV_BYTES, &maps.tk, kv_full + st, 0, n0, it.h, it.b);
-            tma_load_4d(base + C::SLOT_V * C::KV_BYTES, &maps.v, kv_full + st, 0, n0, it.h, it.b);
-            if constexpr (DUAL) tma_load_4d(base + C::SLOT_TV * C::KV_BYTES, &maps.tv, kv_full + st, 0, n0, it.h, it.b);
+            unsigned char *kd = sK + st * C::STAGE_BYTES, *vd = sV + st * C::STAGE_BYTES;
+            mbar_expect_tx(kv_full + st, (BIAS ? 1 : 2) * C::HALF_BYTES);
+            tma_load_4d(kd, &maps.k, kv_full + st, 0, n0, it.h, it.b);
+            if constexpr (DUAL) tma_load_4d(kd + C::KV_BYTES, &maps.tk, kv_full + st, 0, n0, it.h, it.b);
+            uint64_t* const vbar = BIAS ? v_full + st : kv_full + st;
+            if constexpr (BIAS) {
+              // one bias tile for each query tile that uses the key tile, when the one before has been added
+              bool got = true;
+              for (int x = 0; x < 2 && got; ++x) {
+                if (!(m & (1 << x))) continue;
+                int& nb = x ? nb1 : nb0;
+                got = mbar_wait(b_empty + x, (nb & 1) ^ 1, ab, kAbortAux);
+                if (!got) break;
+                ++nb;
+                mbar_expect_tx(b_full + x, C::B_BYTES);
+                tma_load_4d(sB + x * C::B_BYTES, &maps.bias, b_full + x, n0, a.mask.stride[2] ? it.m0 + x * BM : 0,
+                            a.mask.stride[1] ? it.h : 0, a.mask.stride[0] ? it.b : 0);
+              }
+              if (!got || !mbar_wait(v_empty + st, free_par, ab, kAbortKvEmpty)) {
+                ok = false;
+                break;
+              }
+              mbar_expect_tx(vbar, C::HALF_BYTES);
+            }
+            tma_load_4d(vd, &maps.v, vbar, 0, n0, it.h, it.b);
+            if constexpr (DUAL) tma_load_4d(vd + C::KV_BYTES, &maps.tv, vbar, 0, n0, it.h, it.b);
             ++g;
           }
           ++kact;
@@ -385,9 +426,10 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         constexpr uint32_t STAGE16 = C::STAGE_BYTES >> 4;
         const uint32_t q_lo = kDescLo | (smem_u32(sQ + X * C::N_QT * C::Q_BYTES) >> 4), tq_lo = q_lo + (C::Q_BYTES >> 4);
         const uint32_t p_lo = kDescLo | (smem_u32(sP + X * C::N_P * C::P_BYTES) >> 4), w_lo = p_lo + (C::P_BYTES >> 4);
-        const uint32_t k_lo0 = kDescLo | ((smem_u32(sKV) + C::SLOT_K * C::KV_BYTES) >> 4);
-        const uint32_t v_lo0 = kLoV | ((smem_u32(sKV) + C::SLOT_V * C::KV_BYTES) >> 4);
+        const uint32_t k_lo0 = kDescLo | (smem_u32(sK) >> 4);
+        const uint32_t v_lo0 = kLoV | (smem_u32(sV) >> 4);
         const uint32_t bar_kv_full = smem_u32(kv_full), bar_kv_empty = smem_u32(kv_empty);
+        const uint32_t bar_v_full = smem_u32(v_full), bar_v_empty = smem_u32(BIAS ? v_empty : kv_empty);
         const uint32_t bar_s_full = smem_u32(s_full + X), bar_s_free = smem_u32(s_free + X);
         const uint32_t bar_p_full = smem_u32(p_full + X), bar_pv_done = smem_u32(pv_done + X);
         const uint32_t bar_o_free = smem_u32(o_free + X), bar_q_empty = smem_u32(q_empty);
@@ -399,9 +441,10 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         bool ok = true;
         PairItem it;
 
-        // [O | tO'] (+)= P [V | tV] ; tO' += W V for the tile in ring stage pst, whose phases have parity ppar
-        auto issue_pv = [&](uint32_t pst, uint32_t ppar, bool first) -> bool {
+        // [O | tO'] (+)= P [V | tV] ; tO' += W V for the tile in ring stage pst, whose phases have parity ppar (of V's stage: vpar)
+        auto issue_pv = [&](uint32_t pst, uint32_t ppar, uint32_t vpar, bool first) -> bool {
           if (!mbar_wait_warp_u32(bar_p_full, ppar, ab, kAbortPFull)) return false;
+          if (BIAS && !mbar_wait_warp_u32(bar_v_full + 8 * pst, vpar, ab, kAbortKvFull)) return false;
           // The item's first tile overwrites O / tO': the previous item's epilogue must have read them.
           if (first && kx > 0 && !mbar_wait_warp_u32(bar_o_free, (kx - 1) & 1, ab, kAbortOFull)) return false;
           tc_fence_after();
@@ -418,7 +461,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
 #pragma unroll
               for (int kk = 1; kk < BN / 16; ++kk) umma_ts_lo<true>(tq + C::COL_O, tq + C::COL_P + kk * 8, v_lo + kk * 128, idesc_o);
             }
-            tc_commit_u32(bar_kv_empty + 8 * pst);
+            tc_commit_u32(bar_v_empty + 8 * pst);
             tc_commit_u32(bar_pv_done);
           }
           return true;
@@ -430,7 +473,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
           if (!mbar_wait_warp(q_full, kact & 1, ab, kAbortQFull)) break;
           const int my_last = it.last(X);
           bool pend = false, pend_first = false, first = true;
-          uint32_t pend_st = 0, pend_par = 0;
+          uint32_t pend_st = 0, pend_par = 0, pend_vpar = 0;
           TileUse<MK> use(it);
           for (int j = it.j0; j < it.n_load; ++j) {
             const int m = use(j);
@@ -463,30 +506,38 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
                     if (ks < 2 || a.D > 32) umma_ss_lo<true>(tq + C::COL_S, q_lo + ks * 2, k_lo + ks * 2, idesc_s);
                 }
                 tc_commit_u32(bar_s_full);
+                if constexpr (BIAS) tc_commit_u32(bar_kv_empty + 8 * st);
                 if (j == my_last) tc_commit_u32(bar_q_empty);  // arrives when the item's last scores are complete
               }
-              if (pend && !issue_pv(pend_st, pend_par, pend_first)) {
+              if (pend && !issue_pv(pend_st, pend_par, pend_vpar, pend_first)) {
                 ok = false;
                 break;
               }
-              pend = true, pend_st = st, pend_par = tpar, pend_first = first, first = false;
+              pend = true, pend_st = st, pend_par = tpar, pend_vpar = st_par, pend_first = first, first = false;
               tpar ^= 1, any_t = true;
             } else {
               // Loaded for the other query tile only.  A pending output product holds an older ring stage: it goes
               // out first, or the producer could wait for that stage while this thread waits for the producer.
               if (pend) {
-                if (!issue_pv(pend_st, pend_par, pend_first)) {
+                if (!issue_pv(pend_st, pend_par, pend_vpar, pend_first)) {
                   ok = false;
                   break;
                 }
                 pend = false;
               }
-              if (elect_one()) mbar_arrive(kv_empty + st);
+              if (BIAS && !mbar_wait_warp_u32(bar_v_full + 8 * st, st_par, ab, kAbortKvFull)) {  // (its stage's turn, not an earlier one)
+                ok = false;
+                break;
+              }
+              if (elect_one()) {
+                mbar_arrive(kv_empty + st);
+                if (BIAS) mbar_arrive(v_empty + st);
+              }
             }
             if (++st == STAGES) st = 0, st_par ^= 1;
           }
           if (!ok) break;
-          if (pend && !issue_pv(pend_st, pend_par, pend_first)) break;
+          if (pend && !issue_pv(pend_st, pend_par, pend_vpar, pend_first)) break;
           if (!first)
             ++kx;  // this query tile used key tiles in the item (its q_empty arrival went out with the last scores)
           else if (elect_one())
@@ -632,23 +683,18 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
       float m_used = -INFINITY, l_run = 0.f, mu_run = 0.f;
       // MK != 0: this thread's row of the mask / bias (rows past L are clamped; their results are not stored)
       constexpr bool BOOLM = MK == 1 || MK == 3;
-      constexpr int MESZ = BOOLM ? 1 : 2;       // bytes per mask element
-      constexpr int MW = MK == 2 ? 32 : 1;      // 32-bit words per row of a 64-key tile of bias elements
       const unsigned char* mrow = nullptr;
       const uint32_t* brow = nullptr;  // packed boolean mask
       if constexpr (BOOLM) {
         if (a.mask_bits != nullptr)
           brow = mask_bit_row(a.mask_bits, a.mask, mask_head(a.mask, it.b, it.h, a.H), min(i, L - 1), L);
       }
-      if constexpr (MK != 0)
-        mrow = reinterpret_cast<const unsigned char*>(a.mask.ptr) +
-               ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] +
-                (long long)min(i, L - 1) * a.mask.stride[2]) * MESZ;
-      // The mask's piece of a tile.  Where the next tile is known that of a boolean mask is requested as soon as this one's has been
+      if constexpr (BOOLM)
+        mrow = reinterpret_cast<const unsigned char*>(a.mask.ptr) + (long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] +
+               (long long)min(i, L - 1) * a.mask.stride[2];
+      // The mask's piece of a tile.  Where the next tile is known it is requested as soon as this one's has been
       // used: at its own tile's beginning the scores are there already, and the loads would be waited for.  (Without a condition,
-      // zeros beyond the last tile: else this tile's piece would have to be kept.)  A bias is requested at its own tile's
-      // beginning: a tile ahead its 32 registers are in the way (forward with tangents B2 H12 L1024 50 -> 52 us, B8 H6 L1056 3 % more).
-      uint32_t mw[MW];
+      // zeros beyond the last tile: else this tile's piece would have to be kept.)
       uint2 next_keys = make_uint2(~0u, ~0u);
       auto fetch_mask = [&](int n0) {
         if constexpr (BOOLM) {
@@ -659,14 +705,6 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
             next_keys.y = mask_piece_bits(mrow + n0 + 32, n0 + 32, L) | mask_piece_bits(mrow + n0 + 48, n0 + 48, L) << 16;
           }
         }
-        if constexpr (MK == 2) {
-#pragma unroll
-          for (int q4 = 0; q4 < MW / 4; ++q4) {
-            uint4 r = make_uint4(0u, 0u, 0u, 0u);
-            if (n0 + q4 * (16 / MESZ) < L) r = ldg_nc_v4(mrow + (size_t)n0 * MESZ + 16 * q4);
-            mw[4 * q4] = r.x, mw[4 * q4 + 1] = r.y, mw[4 * q4 + 2] = r.z, mw[4 * q4 + 3] = r.w;
-          }
-        }
       };
       constexpr bool AHEAD = MK == 1;
       if constexpr (AHEAD) fetch_mask(it.j0 * BN);
@@ -675,7 +713,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
       for (int j = it.j0; j < it.n_load; ++j) {
         if (!(use(j) & (1 << X))) continue;
         const int n0 = j * BN;
-        if constexpr (MK != 0 && !AHEAD) fetch_mask(n0);
+        if constexpr (MK == 3) fetch_mask(n0);
         uint2 keys = next_keys;  // BOOLM: bit c of (x, y) = the mask lets this row attend key n0 + c
         if (!mbar_wait(s_full + X, t & 1, ab, kAbortSFull)) {
           alive = false;
@@ -683,17 +721,10 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         }
         tc_fence_after();
         uint32_t x0[32], x1[32];
-        uint32_t t0[DUAL && MK != 2 && !CUT ? 32 : 1], t1[DUAL && MK != 2 && !CUT ? 32 : 1];
         tmem_ld32(tS, x0);
         tmem_ld32(tS + 32, x1);
-        // (the tangent scores together with the scores; beside a bias half a tile at a time, when it has been added)
-        constexpr bool TS_LATER = DUAL && (MK == 2 || CUT);
-        if constexpr (DUAL && !TS_LATER) {
-          tmem_ld32(tTS, t0);
-          tmem_ld32(tTS + 32, t1);
-        }
         tmem_wait_ld();
-        if constexpr (!TS_LATER) {
+        if constexpr (!DUAL) {  // (the tangent scores follow half a tile at a time, when their probabilities are formed)
           tc_fence_before();
           mbar_arrive(s_free + X);
         }
@@ -733,25 +764,36 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
           }
           mx = max3(mxa, mxb, fmaxf(mxc, mxd)) * scale_log2;
         } else {
+          if (!mbar_wait(b_full + X, t & 1, ab, kAbortAux)) {
+            alive = false;
+            break;
+          }
+          // this row of the tile (a bias of one row: the first): 16-byte piece c sits at position c ^ (row & 7)
+          const uint32_t brow_sm = smem_u32(sB + X * C::B_BYTES) + (a.mask.stride[2] ? row * 128 : 0), bsw = a.mask.stride[2] ? sw : 0u;
           float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
-          for (int c = 0; c < 16; ++c) {
-            float2 v0 = __fmul2_rn(pf2(x0[2 * c], x0[2 * c + 1]), c2);
-            float2 v1 = __fmul2_rn(pf2(x1[2 * c], x1[2 * c + 1]), c2);
-            {  // scores are in log2 units: bias * log2(e)
+          for (int q = 0; q < 4; ++q) {
+            uint32_t w0[4], w1[4];
+            lds_v4(brow_sm + (((uint32_t)q ^ bsw) << 4), w0);
+            lds_v4(brow_sm + (((uint32_t)(4 + q) ^ bsw) << 4), w1);
+            if (q == 3) mbar_arrive(b_empty + X);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int c = 4 * q + e;
+              // scores are in log2 units: bias * log2(e)
               const float2 l2 = make_float2(kLog2e, kLog2e);
-              v0 = __ffma2_rn(unpack2<T>(mw[c]), l2, v0);
-              v1 = __ffma2_rn(unpack2<T>(mw[16 + c]), l2, v1);
+              float2 v0 = __ffma2_rn(unpack2<T>(w0[e]), l2, __fmul2_rn(pf2(x0[2 * c], x0[2 * c + 1]), c2));
+              float2 v1 = __ffma2_rn(unpack2<T>(w1[e]), l2, __fmul2_rn(pf2(x1[2 * c], x1[2 * c + 1]), c2));
+              if (partial) {
+                if (2 * c >= col_hi) v0.x = -INFINITY;
+                if (2 * c + 1 >= col_hi) v0.y = -INFINITY;
+                if (32 + 2 * c >= col_hi) v1.x = -INFINITY;
+                if (33 + 2 * c >= col_hi) v1.y = -INFINITY;
+              }
+              x0[2 * c] = __float_as_uint(v0.x), x0[2 * c + 1] = __float_as_uint(v0.y);
+              x1[2 * c] = __float_as_uint(v1.x), x1[2 * c + 1] = __float_as_uint(v1.y);
+              mx0 = fmaxf(mx0, v0.x), mx1 = fmaxf(mx1, v0.y), mx2 = fmaxf(mx2, v1.x), mx3 = fmaxf(mx3, v1.y);
             }
-            if (partial) {
-              if (2 * c >= col_hi) v0.x = -INFINITY;
-              if (2 * c + 1 >= col_hi) v0.y = -INFINITY;
-              if (32 + 2 * c >= col_hi) v1.x = -INFINITY;
-              if (33 + 2 * c >= col_hi) v1.y = -INFINITY;
-            }
-            x0[2 * c] = __float_as_uint(v0.x), x0[2 * c + 1] = __float_as_uint(v0.y);
-            x1[2 * c] = __float_as_uint(v1.x), x1[2 * c + 1] = __float_as_uint(v1.y);
-            mx0 = fmaxf(mx0, v0.x), mx1 = fmaxf(mx1, v0.y), mx2 = fmaxf(mx2, v1.x), mx3 = fmaxf(mx3, v1.y);
           }
           mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
         }
@@ -806,16 +848,15 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           uint32_t* xs = hh ? x1 : x0;
-          uint32_t tt[TS_LATER ? 32 : 1];
-          if constexpr (TS_LATER) {
-            tmem_ld32(tTS + 32 * hh, tt);
+          uint32_t ts[DUAL ? 32 : 1];
+          if constexpr (DUAL) {
+            tmem_ld32(tTS + 32 * hh, ts);
             tmem_wait_ld();
             if (hh == 1) {
               tc_fence_before();
               mbar_arrive(s_free + X);  // both score accumulators are in registers now
             }
           }
-          const uint32_t* ts = TS_LATER ? tt : hh ? t1 : t0;
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
             float2 e;
@@ -1020,7 +1061,7 @@ static PairDeal deal_pairs(const jvpfa_fwd_args& a, int sms) {
 
 template <typename T, bool DUAL, int MK, bool CUT>
 static cudaError_t run_pair64(const jvpfa_fwd_args& a, const FwdPairMaps& maps, float* shares, int whole, int* status, int grid, cudaStream_t stream) {
-  using C = FwdPairCfg<DUAL>;
+  using C = FwdPairCfg<DUAL, MK == 2>;
   auto kern = fwd_tc5_pair64_kernel<T, DUAL, MK, CUT>;
   static SmemOptIn opt_in;
   if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return cudaErrorInvalidValue;
@@ -1030,7 +1071,7 @@ static cudaError_t run_pair64(const jvpfa_fwd_args& a, const FwdPairMaps& maps, 
 
 template <typename T, bool DUAL, int MK>
 static int launch_pair64(const jvpfa_fwd_args& a, cudaStream_t stream) {
-  using C = FwdPairCfg<DUAL>;
+  using C = FwdPairCfg<DUAL, MK == 2>;
   int* status = tc5_status_device_ptr();
   if (!status) {
     set_last_cuda_error(cudaErrorUnknown, "status word address");
@@ -1053,6 +1094,12 @@ static int launch_pair64(const jvpfa_fwd_args& a, cudaStream_t stream) {
     ok = ok && encode_map4d(&maps.to, dt, a.to, a.D, a.L, a.H, a.B, nullptr, C::BM);
   else
     maps.to = maps.o;
+  maps.bias = maps.q;
+  if (MK == 2) {  // rows in whole 16-byte pieces (tc5_mask_layout); a dimension without a stride has one entry, whose stride is not used
+    const int64_t* ms = a.mask.stride;
+    const int64_t bias_st[3] = {ms[0] ? ms[0] : 8, ms[1] ? ms[1] : 8, ms[2] ? ms[2] : 8};
+    ok = ok && encode_map_bias(&maps.bias, dt, a.mask.ptr, a.L, ms[2] ? a.L : 1, ms[1] ? a.H : 1, ms[0] ? a.B : 1, bias_st, C::BM);
+  }
   if (!ok) {
     set_last_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled(fwd pair64)");
     return JVPFA_ERR_CUDA;

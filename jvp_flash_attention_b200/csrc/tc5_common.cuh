@@ -145,6 +145,9 @@ __device__ __forceinline__ uint32_t first_columns(int n) { return n >= 32 ? ~0u 
 // out-of-range rows and columns read as zero.  Defined in fwd_tc5.cu.
 bool encode_map4d(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int D, int L, int H, int B, const int64_t* stride_bhl,
                   int box_rows);
+// (L keys, rows, heads, entries) view of a 16-bit bias, box = 64 keys x box_rows rows.
+bool encode_map_bias(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int L, int rows, int H, int B, const int64_t* stride_bhl,
+                     int box_rows);
 // Row-major fp32 (B, H, L, D) tensor, 32-column boxes with 128-byte swizzle (target of TMA reductions).
 bool encode_map4d_f32(CUtensorMap* m, const void* ptr, int D, int L, int H, int B, int box_rows);
 
