@@ -33,6 +33,7 @@ struct Vec16 {
 
 template <typename T, int D>
 __global__ void __launch_bounds__(256) pre_kernel(const jvpfa_pre_args a, long long rows) {
+  behind_previous();  // (for the kernel behind this one)
   constexpr int VEC = 16 / (int)sizeof(T);
   constexpr int TPR = D / VEC;  // threads per row (4..32)
   constexpr int RPB = 256 / TPR;

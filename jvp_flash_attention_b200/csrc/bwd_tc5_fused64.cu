@@ -168,6 +168,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
   using C = BwdFCfg<HAS_GO, HAS_GT>;
   constexpr int D = 64, OWN = C::OWN, BL = C::BL, STAGES = C::STAGES, GSTAGES = C::GSTAGES;
 
+  behind_previous();
   const bool dead_on_entry = *(volatile int*)status != 0;  // an earlier bounded wait gave up
 
   extern __shared__ __align__(1024) unsigned char smem[];  // (the tiles' swizzle repeats every 1024 bytes)
@@ -950,7 +951,8 @@ __device__ __forceinline__ void sum_shares(const jvpfa_bwd_args& a, const float*
 //                them (B2 H12 L1024: 50 MB, most of it still in L2).
 template <typename T>
 __global__ void __launch_bounds__(256)
-fused64_finish_kernel(const jvpfa_bwd_args a, const float* __restrict__ acc, long long n, int n_parts, const float* __restrict__ shares, int ctas, int cut) {
+fused64_finish_kernel(const jvpfa_bwd_args a, const float* acc, long long n, int n_parts, const float* shares, int ctas, int cut) {
+  behind_previous();
   if ((int)blockIdx.x < cut) return sum_shares<T>(a, shares, ctas, blockIdx.x);
   const long long i = (long long)((int)blockIdx.x - cut) * 256 + threadIdx.x;
   const float scale = a.sm_scale;
@@ -1033,8 +1035,7 @@ static cudaError_t run_fused64(const jvpfa_bwd_args& a, const BwdFMaps& m, float
   auto kern = bwd_tc5_fused64_kernel<T, HAS_GO, HAS_GT, MK, CUT>;
   static SmemOptIn opt_in;
   if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return cudaErrorInvalidValue;
-  kern<<<grid, C::NTHREADS, C::SMEM_BYTES, stream>>>(a, m, dq_acc, shares, status);
-  return cudaGetLastError();
+  return launch_behind(kern, grid, C::NTHREADS, C::SMEM_BYTES, stream, a, m, dq_acc, shares, status);
 }
 
 template <typename T, bool HAS_GO, bool HAS_GT, int MK>
@@ -1097,8 +1098,8 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
   const long long per_block = parts ? 256 * 4 : 256 * 8;
   const long long blocks = cut + (a.flags & JVPFA_SKIP_DQ ? 0 : ((long long)n + per_block - 1) / per_block);
   if (blocks == 0) return JVPFA_OK;
-  fused64_finish_kernel<T><<<(unsigned)blocks, 256, 0, stream>>>(a, dq_acc, (long long)n, parts ? n_key_tiles : 0, shares, ctas, cut);
-  e = cudaGetLastError();
+  e = launch_behind(fused64_finish_kernel<T>, (unsigned)blocks, 256, 0, stream, a, static_cast<const float*>(dq_acc), (long long)n,
+                    parts ? n_key_tiles : 0, static_cast<const float*>(shares), ctas, cut);
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch fused64_finish");
     return JVPFA_ERR_CUDA;

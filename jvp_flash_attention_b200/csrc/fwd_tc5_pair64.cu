@@ -165,6 +165,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
   constexpr int D = 64, BM = C::BM, BN = C::BN, STAGES = C::STAGES;
   constexpr bool BIAS = MK == 2;
 
+  behind_previous();
   const bool dead_on_entry = *(volatile int*)status != 0;  // an earlier bounded wait gave up
 
   extern __shared__ unsigned char smem_raw[];
@@ -204,7 +205,6 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
   unsigned char* order = smem + C::OFF_ORDER;
   int* s_cut = reinterpret_cast<int*>(order);  // CUT: {pair, key tile} where this CTA and the next begin
   if constexpr (CUT) {
-    grid_launch_dependents();
     if (warp < 2) {
       const int2 at = pair_begin(a, whole, cta + warp, G);
       if (lane == 0) {
@@ -932,9 +932,9 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
 // this block's, an eighth of it: 128 rows of one query tile, 8 columns a thread of O and, at the same places, of tO.  Bound by reading
 // the shares (B2 H12 L2048: 40 MB, in L2); nearly all pairs have two, so two are requested before the first is looked at.
 template <typename T, bool DUAL>
-__global__ void __launch_bounds__(256) pair64_finish_kernel(const jvpfa_fwd_args a, const float* __restrict__ shares, int ctas) {
+__global__ void __launch_bounds__(256) pair64_finish_kernel(const jvpfa_fwd_args a, const float* shares, int ctas) {
   using S = PairShare<DUAL>;
-  grid_wait();
+  behind_previous();
   const int2* begin = reinterpret_cast<const int2*>(shares);
   const int j = blockIdx.x / 8 + 1;
   const int2 first = begin[j], before = begin[j - 1];
@@ -1065,8 +1065,7 @@ static cudaError_t run_pair64(const jvpfa_fwd_args& a, const FwdPairMaps& maps, 
   auto kern = fwd_tc5_pair64_kernel<T, DUAL, MK, CUT>;
   static SmemOptIn opt_in;
   if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return cudaErrorInvalidValue;
-  kern<<<grid, C::NTHREADS, C::SMEM_BYTES, stream>>>(a, maps, shares, whole, status);
-  return cudaGetLastError();
+  return launch_behind(kern, grid, C::NTHREADS, C::SMEM_BYTES, stream, a, maps, shares, whole, status);
 }
 
 template <typename T, bool DUAL, int MK>

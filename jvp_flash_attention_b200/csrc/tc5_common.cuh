@@ -304,24 +304,6 @@ __device__ __forceinline__ void sort_batch(const jvpfa_mask& m, int B, unsigned 
   }
 }
 
-// ---- Launches that follow one another ----------------------------------------------------------
-// A kernel launched by launch_behind is set up while the one before it on its stream still runs, and waits for that one's results where it
-// says grid_wait, before it reads or writes anything that the other may write or read; every block says so, or the kernel after it
-// could start too early.  The one before says from where on its successor may be set up.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-template <typename... Params, typename... Args>
-cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr, cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
-  return e == cudaSuccess ? cudaGetLastError() : e;
-}
-
 // ---- Items shared out among CTAs --------------------------------------------------------------
 // Persistent kernels whose items (each with a loop of n steps) would leave a round of CTAs half empty share their steps out: the items
 // in a line, by head and by place in the head, cut into as many equal pieces as there are CTAs.  An item's beginning counts as `open`
