@@ -680,28 +680,35 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       if (MK == 1 && a.mask_bits_t != nullptr)
         bcol = mask_bit_col(a.mask_bits_t, a.mask, mask_head(a.mask, it.b, it.h, a.H), min(own_idx, L - 1), L);
       // What the mask holds for this key and the 32 queries from l0 on (MK = 1: a bit each, packed one word, else byte by byte;
-      // MK = 2: the bias elements, 16 bit each, of the tensors' type).  Requested a sub-tile ahead, when the scores of this one have
+      // MK = 2: the bias elements, 16 bit each, of the tensors' type; two neighbouring lanes take two keys' elements of 16 queries each and
+      // change half of them when they are used: half the loads and half the registers of an element at a time (us on a B200 for
+      // H37 L2048: through O 238 -> 200, through tO 304 -> 252, both 352 -> 282).  Requested a sub-tile ahead, when the scores of this one have
       // left their registers: behind that the scores of the next are long there, and the loads would be waited for.  Indices are
       // clamped into the tensor; what lies outside is switched off by col_hi and by lse = +inf of the padding queries.
-      uint32_t next_live = 0xffffffffu, braw[MK == 2 ? 32 : 1];
+      uint32_t next_live = 0xffffffffu, braw[MK == 2 ? 16 : 1];
       auto fetch_mask = [&](int l0) {
         if (MK == 1 && bcol != nullptr) {
           next_live = l0 < L ? ldg_nc_u32(bcol + (a.mask.stride[2] ? l0 >> 5 : 0)) : 0u;
-        } else if constexpr (MK != 0) {
-          constexpr int MESZ = MK == 1 ? 1 : 2;
-          const long long step = a.mask.stride[2] * MESZ;  // to the next query; the last one's element stands for those beyond
+        } else if constexpr (MK == 2) {
+          const long long step = a.mask.stride[2] * 2;  // to the next query; the last one's elements stand for those beyond
+          const int q0 = l0 + 16 * (lane & 1);          // (L is a multiple of 16 and so is q0: the 16 queries are all there or none is)
           const unsigned char* el = reinterpret_cast<const unsigned char*>(a.mask.ptr) +
-                                    ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] +
-                                     (long long)min(own_idx, L - 1) * a.mask.stride[3]) * MESZ + min(l0, L - 1) * step;
+                                    ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] + min(own_idx - (lane & 1), L - 2)) * 2 +
+                                    min(q0, L - 16) * step;
+#pragma unroll
+          for (int x = 0; x < 16; ++x) {
+            braw[x] = ldg_nc_u32(el);
+            el += step;
+          }
+        } else if constexpr (MK == 1) {
+          const long long step = a.mask.stride[2];
+          const unsigned char* el = reinterpret_cast<const unsigned char*>(a.mask.ptr) + (long long)it.b * a.mask.stride[0] +
+                                    (long long)it.h * a.mask.stride[1] + (long long)min(own_idx, L - 1) * a.mask.stride[3] + min(l0, L - 1) * step;
           const int left = L - 1 - l0;
+          next_live = 0u;
 #pragma unroll
           for (int col = 0; col < 32; ++col) {
-            if constexpr (MK == 1) {
-              if (col == 0) next_live = 0u;
-              next_live |= (ldg_nc_u8(el) != 0u ? 1u : 0u) << col;
-            } else {
-              braw[col] = ldg_nc_u16(el);
-            }
+            next_live |= (ldg_nc_u8(el) != 0u ? 1u : 0u) << col;
             if (col < left) el += step;
           }
         }
@@ -718,9 +725,15 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
         }
         tc_fence_after();
         uint32_t bias[MK == 2 ? 16 : 1];
-        if constexpr (MK == 2) {  // in pairs before the scores come: 16 registers beside their 128
+        if constexpr (MK == 2) {  // this lane's key, queries 2 x and 2 x + 1 in bias[x]; lane pairs: even keys' elements are the low halves
+          const bool odd = lane & 1;
 #pragma unroll
-          for (int x = 0; x < 16; ++x) bias[x] = braw[2 * x] | (braw[2 * x + 1] << 16);
+          for (int x = 0; x < 8; ++x) {
+            const uint32_t lo = __byte_perm(braw[2 * x], braw[2 * x + 1], 0x5410), hi = __byte_perm(braw[2 * x], braw[2 * x + 1], 0x7632);
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
+            bias[x] = odd ? other : lo;
+            bias[8 + x] = odd ? hi : other;
+          }
         }
         uint32_t sv[32], fp[32], ts[HAS_GT ? 32 : 1], ev[HAS_GT ? 32 : 1];
         tmem_ld32(tbase + C::COL_S, sv);
