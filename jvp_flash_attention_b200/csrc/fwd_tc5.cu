@@ -122,9 +122,10 @@ bool encode_map4d_f32(CUtensorMap* m, const void* ptr, int D, int L, int H, int 
   });
 }
 
-bool encode_map_bias(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int L, int rows, int H, int B, const int64_t* st,
-                     int box_rows) {
-  return encode_map4d(m, dt, ptr, L, rows, H, B, st, box_rows);
+bool encode_map_bias(CUtensorMap* m, CUtensorMapDataType dt, const jvpfa_mask& mask, int L, int H, int B, int box_rows) {
+  const int64_t* ms = mask.stride;
+  const int64_t st[3] = {ms[0] ? ms[0] : 8, ms[1] ? ms[1] : 8, ms[2] ? ms[2] : 8};  // (8: of one entry, not used)
+  return encode_map4d(m, dt, mask.ptr, L, ms[2] ? L : 1, ms[1] ? H : 1, ms[0] ? B : 1, st, box_rows);
 }
 
 bool encode_map_parts(CUtensorMap* m, const void* ptr, int D, int L, int BH, int planes) {

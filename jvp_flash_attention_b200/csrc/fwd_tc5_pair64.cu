@@ -93,9 +93,6 @@ __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bu
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
-__device__ __forceinline__ void lds_v4(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
 // Makes this thread's shared-memory writes visible to the async proxy (the tensor core reads operands through it).
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
@@ -1094,11 +1091,7 @@ static int launch_pair64(const jvpfa_fwd_args& a, cudaStream_t stream) {
   else
     maps.to = maps.o;
   maps.bias = maps.q;
-  if (MK == 2) {  // rows in whole 16-byte pieces (tc5_mask_layout); a dimension without a stride has one entry, whose stride is not used
-    const int64_t* ms = a.mask.stride;
-    const int64_t bias_st[3] = {ms[0] ? ms[0] : 8, ms[1] ? ms[1] : 8, ms[2] ? ms[2] : 8};
-    ok = ok && encode_map_bias(&maps.bias, dt, a.mask.ptr, a.L, ms[2] ? a.L : 1, ms[1] ? a.H : 1, ms[0] ? a.B : 1, bias_st, C::BM);
-  }
+  if (MK == 2) ok = ok && encode_map_bias(&maps.bias, dt, a.mask, a.L, a.H, a.B, C::BM);
   if (!ok) {
     set_last_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled(fwd pair64)");
     return JVPFA_ERR_CUDA;

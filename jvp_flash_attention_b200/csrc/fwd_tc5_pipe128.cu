@@ -26,7 +26,7 @@
 namespace jvpfa {
 namespace tc5 {
 
-template <bool DUAL>
+template <bool DUAL, bool BIAS = false>
 struct FwdPipeCfg {
   static constexpr int D = 128;
   static constexpr int BM = 128;
@@ -44,8 +44,9 @@ struct FwdPipeCfg {
   // the live key tiles of the CTA's query tile, in order (boolean masks with a tile bitmap: the others are not visited)
   static constexpr int MAX_KEY_TILES = 1024;
   static constexpr int OFF_IDS = OFF_V + STAGES * V_STAGE;
-  static constexpr int TILE_BYTES = OFF_IDS + MAX_KEY_TILES * 2;
-  static constexpr int SMEM_BYTES = TILE_BYTES + 256 /*barriers*/ + 1024 /*alignment slack*/;
+  // a bias tile (128 rows x 64 keys) in the list's place; without tangents no room is left for alignment, or two CTAs would not fit an SM
+  static constexpr int TILE_BYTES = OFF_IDS + (BIAS ? BM * BN * 2 : MAX_KEY_TILES * 2);
+  static constexpr int SMEM_BYTES = TILE_BYTES + 256 /*barriers*/ + (BIAS ? 0 : 1024) /*alignment slack*/;
   static constexpr int SC_COLS = DUAL ? 2 * BN : BN;  // one score buffer
   static constexpr int COL_O = 2 * SC_COLS;
   static constexpr int COL_TO = COL_O + D;
@@ -54,22 +55,27 @@ struct FwdPipeCfg {
 
 struct FwdPipeMaps {
   CUtensorMap q, tq, k, tk, v, tv;
+  CUtensorMap bias;  // MK = 2; its own extents: a dimension that broadcasts has one entry
 };
 
-// MK: 0 = none / causal / key padding; 1 = uint8 mask; 2 = bias of the element type T (the softmax thread of a
-// query row reads its 64 mask elements of the tile with 16-byte loads before it waits for the scores, or 8 bytes of a boolean
-// mask given as bits; the layout is the host's responsibility: tc5_mask_layout); 3 = uint8 mask with the bitmap of 128 x 64
+// MK: 0 = none / causal / key padding; 1 = uint8 mask (the softmax thread of a
+// query row reads its 64 mask elements of the tile with 16-byte loads before it waits for the scores, or 8 bytes of a
+// mask given as bits; the layout is the host's responsibility: tc5_mask_layout); 2 = bias of the element type T, a 128 x 64 tile of it
+// by TMA (rows read by the threads took the L1 longer than a tile's products: H4 L4736 on a B200, us, with tangents 139 -> 107, without
+// 122 -> 80); 3 = uint8 mask with the bitmap of 128 x 64
 // tiles that hold a true entry (jvpfa_mask_tiles): the CTA lists its query tile's live key tiles once and every role
 // walks that list, so tiles without a true entry are neither loaded nor multiplied.
 template <typename T, bool DUAL, int MK>
 __global__ void __launch_bounds__(192, 1)
 fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMaps maps, int* status) {
-  using C = FwdPipeCfg<DUAL>;
+  using C = FwdPipeCfg<DUAL, MK == 2>;
   constexpr int D = C::D, BM = C::BM, BN = C::BN, STAGES = C::STAGES;
   const bool dead_on_entry = *(volatile int*)status != 0;  // an earlier bounded wait gave up
 
-  extern __shared__ unsigned char smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  uint32_t raw = smem_u32(smem_raw);
+  // (The base is kept from the compiler: with a constant one the issuing thread makes every descriptor word anew, 103 -> 115 us.)
+  asm volatile("" : "+r"(raw));
   unsigned char* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
   unsigned char* sQ = smem + C::OFF_Q;
   unsigned char* sTQ = sQ + C::Q_BYTES;  // DUAL only
@@ -88,6 +94,9 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* n_live = reinterpret_cast<int*>(tmem_slot + 2);  // MK == 3: length of the list
+  uint64_t* b_full = bars + 18;   // MK == 2: the tile's bias is there ...
+  uint64_t* b_empty = bars + 19;  // ... and has been added
+  const unsigned char* sB = smem + C::OFF_IDS;
   const unsigned short* ids = reinterpret_cast<const unsigned short*>(smem + C::OFF_IDS);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -115,6 +124,11 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
   auto poison = [&]() {
     if (tid < BM && m0 + tid < L) a.lse[(size_t)bh * L + m0 + tid] = poison_f32();
   };
+  if (MK == 2 && (raw & 1023u) != 0) {  // (does not happen: the array is declared so)
+    if (tid == 0) publish_abort(status, kAbortAux);
+    poison();
+    return;
+  }
   if (dead_on_entry) {
     poison();
     return;
@@ -122,6 +136,7 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
 
   if (tid == 0) {
     mbar_init(q_full, 1);
+    if (MK == 2) mbar_init(b_full, 1), mbar_init(b_empty, 128);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(k_full + s, 1);
       mbar_init(k_empty + s, 1);
@@ -201,11 +216,20 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
         }
         return true;
       };
-      // Stages come free in the order S(t) done, PV(t-1) done, S(t+1) done, ...: the loads are requested in it.
-      bool ok = load_k(0);
+      auto load_b = [&](int t) -> bool {
+        if (MK != 2) return true;
+        if (!mbar_wait(b_empty, (t & 1) ^ 1, ab, kAbortAux)) return false;
+        mbar_expect_tx(b_full, BM * BN * 2);
+        tma_load_4d(smem + C::OFF_IDS, &maps.bias, b_full, t * BN, a.mask.stride[2] ? m0 : 0, a.mask.stride[1] ? tma_h : 0,
+                    a.mask.stride[0] ? tma_b : 0);
+        return true;
+      };
+      // Stages come free in the order S(t) done, (bias t added,) PV(t-1) done, S(t+1) done, ...: the loads are requested in it.
+      bool ok = load_k(0) && load_b(0);
       if (ok && n_tiles > 1) ok = load_k(1);
       for (int t = 0; ok && t < n_tiles; ++t) {
         ok = load_v(t);
+        if (ok && t + 1 < n_tiles) ok = load_b(t + 1);
         if (ok && t + 2 < n_tiles) ok = load_k(t + 2);
       }
     }
@@ -282,24 +306,23 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
     bool alive = true;
 
     constexpr bool BOOLM = MK == 1 || MK == 3;
-    constexpr int MESZ = BOOLM ? 1 : 2;   // bytes per mask element
-    constexpr int MW = MK == 2 ? 32 : 1;  // 32-bit words per row of a 64-key tile of bias elements
+    // this row of the bias tile (a bias of one row: the first): 16-byte piece c sits at position c ^ (row & 7)
+    const int b_row = MK == 2 && a.mask.stride[2] ? row : 0;
+    const uint32_t b_addr = smem_u32(sB) + b_row * 128, b_sw = (uint32_t)(b_row & 7);
     const unsigned char* mrow = nullptr;
     const uint32_t* brow = nullptr;  // packed boolean mask
     if constexpr (BOOLM) {
       if (a.mask_bits != nullptr)
         brow = mask_bit_row(a.mask_bits, a.mask, mask_head(a.mask, tma_b, tma_h, a.H), min(i, L - 1), L);
     }
-    if constexpr (MK != 0)
-      mrow = reinterpret_cast<const unsigned char*>(a.mask.ptr) +
-             ((long long)tma_b * a.mask.stride[0] + (long long)tma_h * a.mask.stride[1] +
-              (long long)min(i, L - 1) * a.mask.stride[2]) * MESZ;
+    if constexpr (BOOLM)
+      mrow = reinterpret_cast<const unsigned char*>(a.mask.ptr) + (long long)tma_b * a.mask.stride[0] + (long long)tma_h * a.mask.stride[1] +
+             (long long)min(i, L - 1) * a.mask.stride[2];
 
     for (int t = 0; t < n_tiles; ++t) {
       const int n0 = key_tile(t) * BN;
       const int st = t & 1;
       const uint32_t tS = tmem + lane_off + st * C::SC_COLS, tTS = tS + BN;
-      uint32_t mw[MW];
       uint2 keys = make_uint2(~0u, ~0u);  // BOOLM: bit c of (x, y) = the mask lets this row attend key n0 + c
       if constexpr (BOOLM) {
         if (brow != nullptr) {
@@ -307,14 +330,6 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
         } else {
           keys.x = mask_piece_bits(mrow + n0, n0, L) | mask_piece_bits(mrow + n0 + 16, n0 + 16, L) << 16;
           keys.y = mask_piece_bits(mrow + n0 + 32, n0 + 32, L) | mask_piece_bits(mrow + n0 + 48, n0 + 48, L) << 16;
-        }
-      }
-      if constexpr (MK == 2) {  // issued before the wait: the loads fly while the scores are formed
-#pragma unroll
-        for (int q4 = 0; q4 < MW / 4; ++q4) {
-          uint4 r = make_uint4(0u, 0u, 0u, 0u);
-          if (n0 + q4 * (16 / MESZ) < L) r = ldg_nc_v4(mrow + (size_t)n0 * MESZ + 16 * q4);
-          mw[4 * q4] = r.x, mw[4 * q4 + 1] = r.y, mw[4 * q4 + 2] = r.z, mw[4 * q4 + 3] = r.w;
         }
       }
       if (!mbar_wait(s_full + st, (t >> 1) & 1, ab, kAbortSFull)) {
@@ -366,8 +381,18 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
         mx = max3(mxa, mxb, fmaxf(mxc, mxd)) * scale_log2;
       } else {
         float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+        if (MK == 2 && !mbar_wait(b_full, t & 1, ab, kAbortAux)) {
+          alive = false;
+          break;
+        }
+        uint32_t w0[4], w1[4];  // MK == 2: four words of the row's bias, and those 32 keys on
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
+          if (MK == 2 && (c & 3) == 0) {
+            lds_v4(b_addr + (((uint32_t)(c >> 2) ^ b_sw) << 4), w0);
+            lds_v4(b_addr + (((uint32_t)(4 + (c >> 2)) ^ b_sw) << 4), w1);
+            if (c == 12) mbar_arrive(b_empty);
+          }
           float2 v0 = __fmul2_rn(pf2(x0[2 * c], x0[2 * c + 1]), c2);
           float2 v1 = __fmul2_rn(pf2(x1[2 * c], x1[2 * c + 1]), c2);
           if constexpr (BOOLM) {
@@ -378,8 +403,8 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
           }
           if constexpr (MK == 2) {  // scores are in log2 units: bias * log2(e)
             const float2 l2 = make_float2(kLog2e, kLog2e);
-            v0 = __ffma2_rn(unpack2<T>(mw[c]), l2, v0);
-            v1 = __ffma2_rn(unpack2<T>(mw[16 + c]), l2, v1);
+            v0 = __ffma2_rn(unpack2<T>(w0[c & 3]), l2, v0);
+            v1 = __ffma2_rn(unpack2<T>(w1[c & 3]), l2, v1);
           }
           if (!BOOLM && partial) {
             if (2 * c >= col_hi) v0.x = -INFINITY;
@@ -545,7 +570,7 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
 
 template <typename T, bool DUAL, int MK>
 static int launch_pipe128(const jvpfa_fwd_args& a, cudaStream_t stream) {
-  using C = FwdPipeCfg<DUAL>;
+  using C = FwdPipeCfg<DUAL, MK == 2>;
   int* status = tc5_status_device_ptr();
   if (!status) {
     set_last_cuda_error(cudaErrorUnknown, "status word address");
@@ -561,6 +586,8 @@ static int launch_pipe128(const jvpfa_fwd_args& a, cudaStream_t stream) {
     ok = ok && enc(&maps.tq, a.tq, C::BM) && enc(&maps.tk, a.tk, C::BN) && enc(&maps.tv, a.tv, C::BN);
   else
     maps.tq = maps.tk = maps.tv = maps.q;
+  maps.bias = maps.q;
+  if (MK == 2) ok = ok && encode_map_bias(&maps.bias, dt, a.mask, a.L, a.H, a.B, C::BM);
   if (!ok) {
     set_last_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled");
     return JVPFA_ERR_CUDA;

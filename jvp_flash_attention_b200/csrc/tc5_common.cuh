@@ -145,13 +145,17 @@ __device__ __forceinline__ uint32_t first_columns(int n) { return n >= 32 ? ~0u 
 // out-of-range rows and columns read as zero.  Defined in fwd_tc5.cu.
 bool encode_map4d(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int D, int L, int H, int B, const int64_t* stride_bhl,
                   int box_rows);
-// (L keys, rows, heads, entries) view of a 16-bit bias, box = 64 keys x box_rows rows.
-bool encode_map_bias(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int L, int rows, int H, int B, const int64_t* stride_bhl,
-                     int box_rows);
+// (keys, rows, heads, entries) view of a 16-bit bias whose rows are whole 16-byte pieces (tc5_mask_layout), box = 64 keys x box_rows rows;
+// a dimension that broadcasts (stride 0) has one entry.
+bool encode_map_bias(CUtensorMap* m, CUtensorMapDataType dt, const jvpfa_mask& mask, int L, int H, int B, int box_rows);
 // Row-major fp32 (B, H, L, D) tensor, 32-column boxes with 128-byte swizzle (target of TMA reductions).
 bool encode_map4d_f32(CUtensorMap* m, const void* ptr, int D, int L, int H, int B, int box_rows);
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void lds_v4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
 
 // ---- mbarrier ------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
