@@ -18,10 +18,10 @@
 // buffer to the output type at the end.  The order of those additions varies from run to run, so dQ is reproducible to
 // rounding, not bitwise.  (With a bias and through tO a key tile's share is stored instead, see kDqParts.)
 //
-// Measured on a B200, cycles of a sub-tile with every SM at work (37 heads, L2048): through O 1830, through tO 2730, both 3410
-// (4030 with one ring of two stages for all four streamed tiles); the tensor pipe's own time is 1024, 1860 and 2050.  What
-// bounds it: the elementwise threads are busy four fifths of the time (two warps for a scheduler, so their latencies show).  ncu,
-// B4 H16 L2048 causal through tO: tensor pipe 56 % of active cycles, operand reads 62 % and ld/st.shared 45 % of their peaks.
+// Measured on a B200, cycles of a sub-tile inside an item (clock marks in one CTA, every SM at work): through O 1660, through tO 2310,
+// both 2600; the tensor pipe's own time is 1024, 1860 and 2050, so that with tangents it is busy four fifths of the time, and
+// through O the elementwise threads are (two warps for a scheduler, so their latencies show).  A key tile's beginning costs 7.6 k
+// cycles more.  Before the looks at the barriers were taken together and dV's products went first: 2060, 2760, 3130.
 //
 // Warps: 0 TMA producer (+ per-query statistics), 1 score issuer, 2 dK/dV issuer, 3 dQ issuer,
 // 4..11 two elementwise warpgroups (thread <-> key row; group w takes query columns [32w, 32w+32) of every
@@ -557,11 +557,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
               const uint32_t lp = ring_mn + st * STAGE16;
               const uint32_t lg = C::TWO_RINGS ? gring_mn + (g % GSTAGES) * GSTAGE16 : lp;
               const uint32_t acc = s > 0;
-              if (elect_one()) {
-                outer(C::COL_DK, C::OUT_GS, lp + C::SLOT_Q * LOOP16, acc);                        // dK += gS^T Q
-                if constexpr (HAS_GT) outer(C::COL_DK, C::OUT_GT, lp + C::SLOT_TQ * LOOP16, 1);  // dK += gtS^T tQ
-                if constexpr (C::TWO_RINGS) tc_commit(loop_empty + st);
-              }
+              // dV first: the stage of G and gO (two stages where they have a ring of their own) and the packed A and P come free
+              // earlier, which the next scores and the elementwise threads wait for
               if (elect_one()) {
                 if constexpr (HAS_GT) {
                   outer_t(C::COL_DV, C::COL_AV, lg + C::SLOT_G * LOOP16, acc);  // dV += A^T G
@@ -569,9 +566,14 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
                 } else {
                   outer_t(C::COL_DV, C::COL_P, lg + C::SLOT_GO * LOOP16, acc);  // dV += P^T gO
                 }
-                tc_commit(C::TWO_RINGS ? g_empty + g % GSTAGES : loop_empty + st);
-                tc_commit(out_free + ob);
+                if constexpr (C::TWO_RINGS) tc_commit(g_empty + g % GSTAGES);
                 tc_commit(av_free);
+              }
+              if (elect_one()) {
+                outer(C::COL_DK, C::OUT_GS, lp + C::SLOT_Q * LOOP16, acc);                        // dK += gS^T Q
+                if constexpr (HAS_GT) outer(C::COL_DK, C::OUT_GT, lp + C::SLOT_TQ * LOOP16, 1);  // dK += gtS^T tQ
+                tc_commit(loop_empty + st);
+                tc_commit(out_free + ob);
                 if (s == it.n_sub - 1) tc_commit(done);
               }
             }
@@ -718,8 +720,13 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
         const int st = g % GSTAGES;  // of the statistics
         const int l0 = it.loop_begin + s * BL + 32 * wg;  // first query of this group's columns
         uint32_t live = next_live;  // MK = 1: bit col = the mask lets query l0 + col attend this key
-        if (!mbar_wait(stat_full + st, (g / GSTAGES) & 1, ab, kAbortBwdLoopFull) ||
-            !mbar_wait(s_full, g & 1, ab, kAbortBwdSFull)) {
+        // A look at a barrier takes 100 to 170 cycles also when its phase is long complete, so the looks are taken together, or ahead
+        // of their need and under other work: three of four in a row were 540 of a sub-tile's 2760 cycles (through tO).
+        const int ob = g % C::N_OBUF, use = g / C::N_OBUF;
+        const uint32_t stat_ok = mbar_test(stat_full + st, (g / GSTAGES) & 1), s_ok = mbar_test(s_full, g & 1);
+        const uint32_t out_ok = use == 0 ? 1u : mbar_test(out_free + ob, (use - 1) & 1);
+        if ((!stat_ok && !mbar_wait(stat_full + st, (g / GSTAGES) & 1, ab, kAbortBwdLoopFull)) ||
+            (!s_ok && !mbar_wait(s_full, g & 1, ab, kAbortBwdSFull))) {
           alive = false;
           break;
         }
@@ -745,6 +752,11 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
         tmem_wait_ld();
         tc_fence_before();
         mbar_arrive(s_free);
+        // The products of the sub-tile that used this result buffer last must have read it.
+        if (!out_ok && !mbar_wait(out_free + ob, (use - 1) & 1, ab, kAbortBwdPFull)) {
+          alive = false;
+          break;
+        }
         // (key j = own_idx, query i = l0 + col) is dead if j >= n_valid, or causal and j > i: columns in [col_lo, col_hi) live
         int col_lo = 0, col_hi = 32;
         if (own_idx >= n_valid) col_hi = 0;
@@ -789,33 +801,31 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           }
           if constexpr (HAS_GO) pk_p[x] = Elem<T>::pack(p.x, p.y);
         };
+        // Queries 8 c .. 8 c + 7 of this group (chunk 4 wg + c of the row) are written as soon as they are there.
+        uint32_t av_ok = 0u;
+        auto chunk = [&](int c, auto masked_c) {
+#pragma unroll
+          for (int x = 4 * c; x < 4 * c + 4; ++x) pair(x, masked_c);
+          const uint32_t off = out_row + ob * C::OBUF_BYTES + (((uint32_t)(4 * wg + c) ^ sw) << 4);
+          sts_v4(off + C::OUT_GS * C::OUT_BYTES, pk_gs[4 * c], pk_gs[4 * c + 1], pk_gs[4 * c + 2], pk_gs[4 * c + 3]);
+          if constexpr (HAS_GT) sts_v4(off + C::OUT_GT * C::OUT_BYTES, pk_gt[4 * c], pk_gt[4 * c + 1], pk_gt[4 * c + 2], pk_gt[4 * c + 3]);
+          if (c == 2) av_ok = g == 0 ? 1u : mbar_test_quiet(av_free, (g - 1) & 1);
+        };
         if constexpr (MK == 1) {  // the index range (key padding of the own tile) joins the mask bits
           const int lo = max(col_lo, 0), hi = min(col_hi, 32);
           live &= hi > lo ? ((hi - lo >= 32 ? 0xffffffffu : ((1u << (hi - lo)) - 1u)) << lo) : 0u;
         }
         if (__any_sync(0xffffffffu, MK == 1 ? live != 0xffffffffu : (col_lo > 0 || col_hi < 32))) {
 #pragma unroll
-          for (int x = 0; x < 16; ++x) pair(x, IntC<1>{});
+          for (int c = 0; c < 4; ++c) chunk(c, IntC<1>{});
         } else {
 #pragma unroll
-          for (int x = 0; x < 16; ++x) pair(x, IntC<0>{});
+          for (int c = 0; c < 4; ++c) chunk(c, IntC<0>{});
         }
         if constexpr (MK != 0) fetch_mask(l0 + BL);  // (behind the last one too: else this one's would have to be kept)
-        // The products of the sub-tile that used this result buffer last must have read it.
-        const int ob = g % C::N_OBUF, use = g / C::N_OBUF;
-        if (use > 0 && !mbar_wait(out_free + ob, (use - 1) & 1, ab, kAbortBwdPFull)) {
-          alive = false;
-          break;
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {  // chunk 4 wg + c = this group's queries 8c .. 8c+7
-          const uint32_t off = out_row + ob * C::OBUF_BYTES + (((uint32_t)(4 * wg + c) ^ sw) << 4);
-          sts_v4(off + C::OUT_GS * C::OUT_BYTES, pk_gs[4 * c], pk_gs[4 * c + 1], pk_gs[4 * c + 2], pk_gs[4 * c + 3]);
-          if constexpr (HAS_GT) sts_v4(off + C::OUT_GT * C::OUT_BYTES, pk_gt[4 * c], pk_gt[4 * c + 1], pk_gt[4 * c + 2], pk_gt[4 * c + 3]);
-        }
         // A and P go to their TMEM columns (this group's 32 queries = 16 packed columns) once the previous
         // sub-tile's dV products have read them
-        if (g > 0 && !mbar_wait(av_free, (g - 1) & 1, ab, kAbortBwdPFull)) {
+        if (!av_ok && !mbar_wait(av_free, (g - 1) & 1, ab, kAbortBwdPFull)) {
           alive = false;
           break;
         }
@@ -823,9 +833,9 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + 16 * wg;
           if constexpr (HAS_GT) tmem_st16(trow + C::COL_AV, pk_av);
           if constexpr (HAS_GO) tmem_st16(trow + C::COL_P, pk_p);
+          fence_async_smem();
           tmem_wait_st();
         }
-        fence_async_smem();
         tc_fence_before();
         mbar_arrive(p_full + (g & 1));
       }

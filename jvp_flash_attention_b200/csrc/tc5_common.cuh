@@ -209,6 +209,29 @@ __device__ __forceinline__ bool mbar_try_wait_u32(uint32_t bar, uint32_t parity)
       : "memory");
   return ok != 0;
 }
+// One look, without waiting.  (`quiet`: loads and stores may be moved across it; for barriers that guard nothing but what volatile
+// instructions behind it touch.)
+__device__ __forceinline__ uint32_t mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok;
+}
+__device__ __forceinline__ uint32_t mbar_test_quiet(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity));
+  return ok;
+}
 // Bounded wait.  Returns false (and latches the abort state) when the budget runs out or when
 // another thread of the CTA has already given up.  A measured mbarrier hand-off between two warps
 // costs ~200 cycles.  Measured on the forward kernels (two CTAs per SM, many warps waiting at once):
