@@ -839,12 +839,15 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         }
         // Exponentials, row sums, W = P * tS * scale and the packing to 16 bit in one loop per half tile, so that
         // the special-function unit's latency is covered by the arithmetic of the neighbouring columns.
+        // The P / W tiles are single-buffered: the previous tile's output MMAs must have read them.  (A look at the barrier takes 100
+        // cycles and more also when they are long complete: it is taken under the first half's arithmetic.)
+        const uint32_t pv_ok = t == 0 || prev_pv_seen ? 1u : mbar_test_quiet(pv_done + X, (t - 1) & 1);
         const float2 nm2 = make_float2(-m_eff, -m_eff);
         float2 ls2 = make_float2(0.f, 0.f), ms2 = make_float2(0.f, 0.f);
-        uint32_t pp[32], wp[DUAL ? 32 : 1];
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           uint32_t* xs = hh ? x1 : x0;
+          uint32_t pp[16], wp[DUAL ? 16 : 1];
           uint32_t ts[DUAL ? 32 : 1];
           if constexpr (DUAL) {
             tmem_ld32(tTS + 32 * hh, ts);
@@ -863,38 +866,37 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
               e = __fadd2_rn(pf2(xs[2 * c], xs[2 * c + 1]), nm2);
             const float2 pv = make_float2(fast_exp2(e.x), fast_exp2(e.y));
             ls2 = __fadd2_rn(ls2, pv);
-            pp[16 * hh + c] = Elem<T>::pack(pv.x, pv.y);
+            pp[c] = Elem<T>::pack(pv.x, pv.y);
             if constexpr (DUAL) {
               const float2 w = __fmul2_rn(pv, __fmul2_rn(pf2(ts[2 * c], ts[2 * c + 1]), sc2));
               ms2 = __fadd2_rn(ms2, w);
-              wp[16 * hh + c] = Elem<T>::pack(w.x, w.y);
+              wp[c] = Elem<T>::pack(w.x, w.y);
             }
           }
+          if (hh == 0 && ((!pv_ok && !mbar_wait(pv_done + X, (t - 1) & 1, ab, kAbortOFull)) ||
+                          (first && !release_staging()))) {  // (the previous item's output store has read the buffers)
+            alive = false;
+            break;
+          }
+          if constexpr (DUAL) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {  // chunk 4 hh + c = key columns 8 (4 hh + c) ..
+              const uint32_t off = ((uint32_t)(4 * hh + c) ^ sw) << 4;
+              st_shared_v4(pP + off, pp[4 * c], pp[4 * c + 1], pp[4 * c + 2], pp[4 * c + 3]);
+              st_shared_v4(pW + off, wp[4 * c], wp[4 * c + 1], wp[4 * c + 2], wp[4 * c + 3]);
+            }
+          } else {
+            tmem_st16(tq + C::COL_P + 16 * hh, pp);
+          }
         }
+        if (!alive) break;
 
         l_run = l_run * alpha + (ls2.x + ls2.y);
         if constexpr (DUAL) mu_run = mu_run * alpha + (ms2.x + ms2.y);
-        // The P / W tiles are single-buffered: the previous tile's output MMAs must have read them.
-        if (t > 0 && !prev_pv_seen && !mbar_wait(pv_done + X, (t - 1) & 1, ab, kAbortOFull)) {
-          alive = false;
-          break;
-        }
-        if (first && !release_staging()) {  // the previous item's output store has read the buffers
-          alive = false;
-          break;
-        }
-        if constexpr (DUAL) {
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {  // chunk c = key columns 8c .. 8c+7
-            const uint32_t off = ((uint32_t)c ^ sw) << 4;
-            st_shared_v4(pP + off, pp[4 * c], pp[4 * c + 1], pp[4 * c + 2], pp[4 * c + 3]);
-            st_shared_v4(pW + off, wp[4 * c], wp[4 * c + 1], wp[4 * c + 2], wp[4 * c + 3]);
-          }
+        if constexpr (DUAL)
           fence_proxy_async_smem();
-        } else {
-          tmem_st32(tq + C::COL_P, pp);
+        else
           tmem_wait_st();
-        }
         tc_fence_before();
         mbar_arrive(p_full + X);
         first = false;
