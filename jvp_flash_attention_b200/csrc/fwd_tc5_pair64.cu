@@ -842,21 +842,21 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
         // The P / W tiles are single-buffered: the previous tile's output MMAs must have read them.  (A look at the barrier takes 100
         // cycles and more also when they are long complete: it is taken under the first half's arithmetic.)
         const uint32_t pv_ok = t == 0 || prev_pv_seen ? 1u : mbar_test_quiet(pv_done + X, (t - 1) & 1);
+        uint32_t ts0[DUAL ? 32 : 1], ts1[DUAL ? 32 : 1];
+        if constexpr (DUAL) {
+          tmem_ld32(tTS, ts0);
+          tmem_ld32(tTS + 32, ts1);
+          tmem_wait_ld();
+          tc_fence_before();
+          mbar_arrive(s_free + X);  // both score accumulators are in registers now
+        }
         const float2 nm2 = make_float2(-m_eff, -m_eff);
         float2 ls2 = make_float2(0.f, 0.f), ms2 = make_float2(0.f, 0.f);
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           uint32_t* xs = hh ? x1 : x0;
           uint32_t pp[16], wp[DUAL ? 16 : 1];
-          uint32_t ts[DUAL ? 32 : 1];
-          if constexpr (DUAL) {
-            tmem_ld32(tTS + 32 * hh, ts);
-            tmem_wait_ld();
-            if (hh == 1) {
-              tc_fence_before();
-              mbar_arrive(s_free + X);  // both score accumulators are in registers now
-            }
-          }
+          const uint32_t* ts = hh ? ts1 : ts0;
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
             float2 e;
