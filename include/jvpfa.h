@@ -124,18 +124,20 @@ typedef struct {
   const void* mask_bits;
   /* 0 or JVPFA_ZERO_TKV.  (struct_size up to mask_tile_live: 0.) */
   int32_t flags;
-  /* Optional caller-owned scratch of the call, JVPFA_FP32 only: jvpfa_fwd_workspace() bytes, 16-byte aligned, contents
-   * irrelevant.  With it the call runs on the tcgen05 tensor cores, which multiply three bf16 parts of every entry; the
-   * parts are made there first.  NULL or too small: the register-tiled kernels.  (struct_size up to flags: NULL.) */
+  /* Optional caller-owned scratch of the call: jvpfa_fwd_workspace() bytes, 16-byte aligned, contents irrelevant.
+   * JVPFA_FP32: with it the call runs on the tcgen05 tensor cores, which multiply three bf16 parts of every entry; the
+   * parts are made there first.  NULL or too small: the register-tiled kernels.  16-bit types, D <= 64: with it the query tiles are
+   * shared out among the SMs where whole ones would leave many idle, and what two SMs have of a tile is merged there; NULL or
+   * too small: whole query tiles.  (struct_size up to flags: NULL.) */
   void* workspace;
   int64_t workspace_bytes;
 } jvpfa_fwd_args;
 
 int jvpfa_fwd(const jvpfa_fwd_args* args, void* stream);
 
-/* Bytes of jvpfa_fwd_args.workspace with which this call (workspace itself not looked at) runs on the tcgen05 kernels;
- * 0 if it gains nothing from one, or for arguments that jvpfa_fwd refuses.  impl JVPFA_IMPL_TCGEN05: whether it gains or not.
- * Pure host logic. */
+/* Bytes of jvpfa_fwd_args.workspace that this call (workspace itself not looked at) can use: fp32, to run on the tcgen05 kernels (impl
+ * JVPFA_IMPL_TCGEN05: whether it gains or not); 16 bit, to share tiles out.  0 if it gains nothing from one, or for arguments that
+ * jvpfa_fwd refuses.  Host logic; the number of SMs is the current device's. */
 int64_t jvpfa_fwd_workspace(const jvpfa_fwd_args* args);
 
 /*
@@ -217,7 +219,8 @@ typedef struct {
   int64_t workspace_bytes;
 } jvpfa_bwd_args;
 
-/* As jvpfa_fwd_workspace.  Non-zero for JVPFA_FP32 through O, and for dQ alone (JVPFA_SKIP_DKDV) through tO with
+/* As jvpfa_fwd_workspace.  Non-zero for 16-bit types at D = 64 where the one pass (dq_accum) shares key tiles out among the SMs; for
+ * JVPFA_FP32 through O, and for dQ alone (JVPFA_SKIP_DKDV) through tO with
  * JVPFA_ZERO_TKV; and for 16-bit types at D = 64 through tO with a BIAS of their type (key stride 1, 16-byte aligned rows,
  * L % 16 == 0), where the backward then is one pass, bitwise reproducible, that leaves a share of dQ for each 128 keys there.
  * The fp32 ones recompute the scores as jvpfa_fwd with its workspace forms them, the other kernels as jvpfa_fwd without:
