@@ -90,3 +90,43 @@ def test_forward_of_cut_pairs(kind, B, H, L, D, dual, dt):
         x = few(x).double().cpu()
         assert orc.max_abs_err(x, r) <= 2e-2 * max(1.0, r.abs().max().item()), name
         assert (x - r).norm() <= rel * r.norm(), name
+
+
+def _bias_forms(B, H, L, dt):
+    g = torch.Generator().manual_seed(L)
+    r = lambda *s: torch.randn(*s, generator=g).clamp(-5, 5).to(dt).to(DEV)  # noqa: E731
+    forms = {"full": r(B, H, L, L), "heads": r(1, H, L, L), "entries": r(B, 1, L, L), "one": r(1, 1, L, L), "row": r(B, 1, 1, L),
+             "row of each head": r(B, H, 1, L), "heads first": r(H, B, L, L).transpose(0, 1), "expanded": r(1, 1, L, L).expand(B, H, L, L),
+             "wider rows": r(B, H, L, L + 24)[..., :L], "rows apart": r(B, H, L, 2, L)[:, :, :, 1], "at an odd place": r(B, H, L, L + 3)[..., 3:]}
+    if L % 16 == 0:  # every row eight elements on from the one before: rows that overlap in memory
+        forms["overlapping rows"] = r(1, 1, 8 * L + L).as_strided((1, 1, L, L), (9 * L, 9 * L, 8, 1))
+    return forms
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,H,L,D", [(2, 3, 336, 64), (2, 2, 200, 64), (1, 3, 130, 128), (2, 2, 256, 128), (2, 2, 144, 32)])
+def test_every_layout_of_a_bias(B, H, L, D, dt):
+    """The forward with and without tangents and the backward: a bias of any layout gives what its row-major copy gives, the forward
+    bit for bit, and that is the float64 oracle's within the bounds above."""
+    g = torch.Generator().manual_seed(L + D)
+    ts = [(torch.randn(B, H, L, D, generator=g) * (0.1 if n in (3, 4, 5) else 1.0)).to(dt).to(DEV) for n in range(8)]
+
+    def run(m):
+        a = [x.detach().requires_grad_() for x in ts[:3]]
+        o, to = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, attn_mask=m), tuple(a), tuple(ts[3:6]))
+        dk, dv = torch.autograd.grad((o, to), a[1:], (ts[6], ts[7]))
+        return ja.attention(*ts[:3], attn_mask=m), o.detach(), to.detach(), dk, dv
+
+    for name, m in _bias_forms(B, H, L, dt).items():
+        got, want = run(m), run(m.expand(B, H, L, L).contiguous())
+        # (rows that begin off 16-byte boundaries, and a ragged one for all queries, are the register-tiled kernels')
+        if name != "at an odd place" and (L % 16 == 0 or name not in ("row", "row of each head")):
+            for x, y in zip(got[:3], want[:3]):
+                assert torch.equal(x, y), name
+        ref = orc.sdpa_jvp(*(x.cpu() for x in ts[:6]), m.expand(B, H, L, L).cpu(), False, None)
+        for x, r in zip(got[1:3], ref):
+            assert orc.max_abs_err(x, r) <= 2e-2 * max(1.0, r.abs().max().item()), name
+        for x, y in zip(got[3:], want[3:]):  # (a broadcast bias may be served by another backward kernel)
+            assert (x.double() - y.double()).norm() <= (1e-2 if dt == torch.bfloat16 else 2e-3) * y.double().norm(), name
+    assert _lib.device_status() == 0
