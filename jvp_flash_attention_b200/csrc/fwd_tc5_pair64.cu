@@ -1022,10 +1022,11 @@ static int pair_sm_count() {
 }
 
 // How the pairs are dealt: `ctas` CTAs among which their key tiles are shared out, after `whole` rounds of pairs as a whole; ctas = 0: all
-// as a whole.  Both ways in key tiles of the CTA that has the most.  The shares' way through the workspace takes as long as 8, and 12
-// where most CTAs have two of them.  Measured on a B200, replayed from a graph, us whole / shared out, bf16 with tangents: H4 L1024 29 / 21, H16 L1024 30 / 28,
-// H24 L1024 31 / 35, H4 L2048 51 / 30, H16 L2048 54 / 62, H24 L2048 99 / 82, H12 L4096 186 / 138; causal H16 L1024 28 / 24, H24 L2048 52 / 55, H8
-// L4096 94 / 62; without tangents H4 L1024 20 / 15, H24 L1024 21 / 23.  (All pairs in the line; with whole rounds first H24 L2048 79.)
+// as a whole.  Both ways in key tiles of the CTA that has the most.  The shares' way through the workspace takes as long as 8, 9 behind whole
+// rounds, and 12 where most CTAs have two of them; a twentieth less is asked for.  Measured on a B200, replayed from a graph, us whole /
+// shared out, bf16 with tangents: H4 L1024 27 / 20, H16 L1024 27 / 26, H24 L1024 31 / 35 (left whole), H48 L1024 52 / 47, H4 L2048 46 / 28, H24
+// L2048 91 / 74, H30 L2048 91 / 90 and with a bias 123 / 125, H12 L4096 169 / 129; causal H16 L1024 25 / 23, H24 L2048 52 / 55
+// (left whole), H8 L4096 86 / 59; without tangents H4 L1024 19 / 14, H24 L1024 21 / 23 (left whole).
 // Where tiles are stepped over their numbers are not known here: whole.  (Lengths of a key padding are not known either: as if there were none.)
 struct PairDeal {
   int ctas, whole;
@@ -1054,8 +1055,8 @@ static PairDeal deal_pairs(const jvpfa_fwd_args& a, int sms) {
     }
   }
   const long long whole = causal || a.mask.kind == JVPFA_MASK_KVLEN ? 0 : items / ctas;
-  const long long shared = whole > 0 ? whole * N + (items - whole * ctas) * N / ctas + 8 : steps / ctas + (2 * items > ctas ? 12 : 8);
-  return shared * 25 < most * 24 ? PairDeal{(int)ctas, (int)whole} : all_whole;
+  const long long shared = whole > 0 ? whole * N + (items - whole * ctas) * N / ctas + 9 : steps / ctas + (2 * items > ctas ? 12 : 8);
+  return shared * 20 < most * 19 ? PairDeal{(int)ctas, (int)whole} : all_whole;
 }
 
 template <typename T, bool DUAL, int MK, bool CUT>
