@@ -136,7 +136,7 @@ struct TileUse {
 // merges them in their order.  A pair's beginning counts as kPairOpen key tiles.
 constexpr int kPairOpen = 2;
 template <bool DUAL>
-struct PairShare {  // floats: [query tile][16-byte piece of O, then of tO'][128 rows], then [128 rows]{maximum, sum, sum of W, -}
+struct PairShare {  // floats: [query tile][16-byte piece of O, then of tO'][128 rows], then [128 rows]{maximum, sum, sum of W, 1: no key, no accumulators}
   static constexpr int PIECES = DUAL ? 32 : 16;
   static constexpr int TILE = (PIECES + 1) * 128 * 4;
   static constexpr int SIZE = 2 * TILE;
@@ -672,7 +672,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
           alive = epilogue(it, i, -INFINITY, 0.f, 0.f, false);
           continue;
         } else if (float4* const to = share(walk, X, row)) {
-          to[PairShare<DUAL>::PIECES * BM] = make_float4(-INFINITY, 0.f, 0.f, 0.f);
+          to[PairShare<DUAL>::PIECES * BM] = make_float4(-INFINITY, 0.f, 0.f, 1.f);
           continue;
         }
       }
@@ -955,8 +955,10 @@ __global__ void __launch_bounds__(256) pair64_finish_kernel(const jvpfa_fwd_args
   };
   float m = -INFINITY, l = 0.f, mu = 0.f, o[8] = {}, to[8] = {};
   auto add = [&](const Share& v) {
-    if (v.st.x == -INFINITY) return;  // no key of the share (and nothing but its statistics is there)
-    const float top = fmaxf(m, v.st.x), keep = fast_exp2(m - top), w = fast_exp2(v.st.x - top);
+    if (v.st.w != 0.f) return;  // no key of the share, and nothing but its statistics is there
+    // As in the loop over key tiles, the reference is 0 where the maximum is -inf: maxima pass over what is not a number, so a share of
+    // such a maximum may have sums that are none.
+    const float top = fmaxf(m, v.st.x), ref = top == -INFINITY ? 0.f : top, keep = fast_exp2(m - ref), w = fast_exp2(v.st.x - ref);
     m = top;
     l = keep * l + w * v.st.y;
     mu = keep * mu + w * v.st.z;
@@ -972,7 +974,7 @@ __global__ void __launch_bounds__(256) pair64_finish_kernel(const jvpfa_fwd_args
   };
   Share u, v;
   load(2 * (j - 1) + 1, u);  // the share that begins the pair is its CTA's last
-  v.st.x = -INFINITY;
+  v.st.w = 1.f;
   if (next.x != first.x || next.y != first.y) load(2 * j, v);  // (else CTA j has nothing to do)
   add(u);
   add(v);

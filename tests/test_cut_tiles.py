@@ -1,10 +1,14 @@
 """Tiles shared out among CTAs: a tile that is cut leaves partial sums in a workspace, which are added up in a fixed order."""
+import ctypes
+import math
+
 import pytest
 import torch
 
 from jvp_flash_attention_b200 import _lib
 from jvp_flash_attention_b200 import jvp_attention as ja
 from oracle import jvp_attention_oracle as orc
+from tests.test_fp32_tcgen05 import _fwd_args
 
 DEV = "cuda:0"
 
@@ -90,6 +94,74 @@ def test_forward_of_cut_pairs(kind, B, H, L, D, dual, dt):
         x = few(x).double().cpu()
         assert orc.max_abs_err(x, r) <= 2e-2 * max(1.0, r.abs().max().item()), name
         assert (x - r).norm() <= rel * r.norm(), name
+
+
+def _spec(kind, mask):
+    """A mask (on the device) as the C ABI takes it."""
+    if kind == "keys":
+        return _lib.MaskSpec(_lib.MASK_KVLEN, mask[:, 0, 0].sum(-1).to(torch.int32))
+    if mask is None:
+        return _lib.MaskSpec(_lib.MASK_CAUSAL if kind == "causal" else _lib.MASK_NONE)
+    dt = _lib.BF16 if mask.dtype == torch.bool else _lib.DTYPE_ENUM[mask.dtype]
+    return _lib.MaskSpec(_lib.MASK_BOOL if kind == "bool" else _lib.MASK_BIAS, mask, mask.stride(), dt)
+
+
+class _Forward:
+    """jvpfa_fwd on q, k, v and, as far as given, their tangents.  cut: with the workspace that it asks for, full of NaN."""
+
+    def __init__(self, ts, spec, cut):
+        B, H, L, D = ts[0].shape
+        dual = len(ts) == 6
+        nan = lambda *s, dt=torch.float32: torch.full(s, math.nan, device=DEV, dtype=dt)  # noqa: E731
+        self.out = [nan(B, H, L, D, dt=ts[0].dtype), nan(B, H, L, D, dt=ts[0].dtype) if dual else None, nan(B, H, L), nan(B, H, L) if dual else None]
+        self.args = a = _fwd_args(ts[:3], ts[3:], spec.to_c(), self.out, _lib.IMPL_TCGEN05)
+        a.dtype = _lib.DTYPE_ENUM[ts[0].dtype]
+        self.kept = ts, spec
+        if cut:
+            n = _lib.load().jvpfa_fwd_workspace(ctypes.byref(a))
+            assert n > 0, "this call is not cut"
+            self.workspace = nan(n // 4)
+            a.workspace, a.workspace_bytes = self.workspace.data_ptr(), n
+            self.ctas = (n - 16384) // (2 * 2 * (33 if dual else 17) * 128 * 16)
+
+    def launch(self):
+        _lib.check(_lib.load().jvpfa_fwd(ctypes.byref(self.args), torch.cuda.current_stream().cuda_stream), "jvpfa_fwd")
+        return [x for x in self.out if x is not None]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [64, 32])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind,B,H,L", [("none", 1, 3, 1040), ("causal", 1, 3, 1040), ("bool", 1, 3, 1040), ("bias", 1, 3, 1040),
+                                        ("none", 2, 12, 2048), ("bool", 2, 12, 2048), ("bias", 2, 12, 2048)])
+def test_what_is_not_finite_reaches_in_cut_pairs_what_it_reaches_in_whole_ones(kind, B, H, L, dt, D):
+    """Entries that are not a number, or Inf; rows without a key, with two in two pieces, and whose bias is the type's lowest value: the
+    results that are finite are those of whole pairs, and where lse is +Inf (no key, or no number) it is there."""
+    g = torch.Generator(device=DEV).manual_seed(L + D)
+    ts = [(torch.randn(B, H, L, D, device=DEV, generator=g) * (0.1 if n > 2 else 1.0)).to(dt) for n in range(6)]
+    mask, bad_key = None, L // 3
+    if kind == "bool":
+        mask = torch.rand(B, H, L, L, device=DEV, generator=g) > 0.5
+        mask[:, :, 5] = mask[:, :, 7] = False
+        mask[:, :, 7, [bad_key, L - 1]] = True
+    elif kind == "bias":
+        mask = torch.randn(B, H, L, L, device=DEV, generator=g).to(dt)
+        mask[:, :, 5] = torch.finfo(dt).min
+        mask[:, :, 6] = -math.inf
+        mask[:, :, 7, : L // 2] = -math.inf
+    spec = _spec(kind, mask)
+    for n in (3, 6):
+        for bad in (math.nan, math.inf):
+            for where in range(n):
+                x = [t.clone() if m == where else t for m, t in enumerate(ts[:n])]
+                x[where][:, ::2, bad_key, 7] = bad
+                if where == 0:
+                    x[0][:, 1] = bad  # a head throughout
+                got, want = _Forward(x, spec, True).launch(), _Forward(x, spec, False).launch()
+                for m, (u, w) in enumerate(zip(got, want)):
+                    assert torch.equal(torch.isfinite(u), torch.isfinite(w)), (n, bad, where, m)
+                    assert u.dim() == 4 or torch.equal(torch.isposinf(u), torch.isposinf(w)), (n, bad, where, m)
+    assert _lib.device_status() == 0
 
 
 def _bias_forms(B, H, L, dt):
