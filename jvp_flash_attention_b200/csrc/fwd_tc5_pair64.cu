@@ -954,11 +954,13 @@ __global__ void __launch_bounds__(256) pair64_finish_kernel(const jvpfa_fwd_args
     }
   };
   float m = -INFINITY, l = 0.f, mu = 0.f, o[8] = {}, to[8] = {};
+  bool gave_up = false;
   auto add = [&](const Share& v) {
     if (v.st.w != 0.f) return;  // no key of the share, and nothing but its statistics is there
     // As in the loop over key tiles, the reference is 0 where the maximum is -inf: maxima pass over what is not a number, so a share of
     // such a maximum may have sums that are none.
     const float top = fmaxf(m, v.st.x), ref = top == -INFINITY ? 0.f : top, keep = fast_exp2(m - ref), w = fast_exp2(v.st.x - ref);
+    gave_up = gave_up || isnan(v.st.x);  // (a CTA that gave up wrote it: no maximum is NaN)
     m = top;
     l = keep * l + w * v.st.y;
     mu = keep * mu + w * v.st.z;
@@ -994,7 +996,7 @@ __global__ void __launch_bounds__(256) pair64_finish_kernel(const jvpfa_fwd_args
   const float inv_l = empty ? 0.f : 1.f / l, mu_n = mu * inv_l;
   const size_t at = (size_t)bh * a.L + i;
   if (piece == 0) {
-    a.lse[at] = empty ? INFINITY : m + log2f(l);
+    a.lse[at] = gave_up ? poison_f32() : empty ? INFINITY : m + log2f(l);
     if constexpr (DUAL) a.mu[at] = mu_n;
   }
   if (4 * piece >= a.D) return;

@@ -164,6 +164,48 @@ def test_what_is_not_finite_reaches_in_cut_pairs_what_it_reaches_in_whole_ones(k
     assert _lib.device_status() == 0
 
 
+def _replayed_behind_a_launch_that_gave_up(step):
+    """What `step` returns, replayed from a graph over results of 1 with the status word set (from the host, as a thread that gives up a
+    wait would) and without."""
+    side = torch.cuda.Stream()  # (the legacy stream's graph nodes cannot be captured)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step()
+    seen = []
+    for code in (5, 0):
+        if code:
+            _lib.device_status_inject(code)
+        try:
+            for x in got:
+                x.fill_(1.0)
+            graph.replay()
+            torch.cuda.synchronize()
+            seen.append([x.clone() for x in got])
+        finally:
+            assert _lib.device_status(clear=True) == code
+    return seen
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [3, 6])
+@pytest.mark.parametrize("kind,B,H,L", [("none", 1, 3, 1040), ("causal", 1, 3, 1040), ("none", 2, 12, 2048), ("keys", 5, 2, 1104), ("bias", 1, 3, 1040)])
+def test_rows_of_cut_pairs_are_marked_where_the_forward_gave_up(kind, B, H, L, n):
+    """lse of every row holds NaN then (jvpfa_device_status), also of a pair whose shares are merged by a later kernel."""
+    g = torch.Generator().manual_seed(L)
+    ts = [torch.randn(B, H, L, 64, generator=g).to(torch.bfloat16).to(DEV) for _ in range(n)]
+    mask = _mask(kind, B, H, L, torch.bfloat16, g)
+    f = _Forward(ts, _spec(kind, None if mask is None else mask.to(DEV)), True)
+    gave_up, after = _replayed_behind_a_launch_that_gave_up(f.launch)
+    assert torch.isnan(gave_up[n // 3]).all()
+    f.launch()
+    for x, y in zip(after, [x for x in f.out if x is not None]):
+        assert torch.equal(x, y)
+
+
 def _bias_forms(B, H, L, dt):
     g = torch.Generator().manual_seed(L)
     r = lambda *s: torch.randn(*s, generator=g).clamp(-5, 5).to(dt).to(DEV)  # noqa: E731
