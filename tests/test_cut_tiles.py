@@ -206,6 +206,30 @@ def test_rows_of_cut_pairs_are_marked_where_the_forward_gave_up(kind, B, H, L, n
         assert torch.equal(x, y)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("through", ["o", "t", "both"])
+@pytest.mark.parametrize("kind", ["none", "causal", "keys", "bool", "bias"])
+def test_rows_of_cut_key_tiles_are_marked_where_the_backward_gave_up(kind, through):
+    """Every row of dQ, dK and dV holds NaN then, also those of keys that are all padding, which weigh nothing on the line."""
+    B, H, L = (8, 12, 400) if kind == "bias" else (5, 2, 720)
+    g = torch.Generator().manual_seed(L)
+    q, k, v, tq, tk, tv, go, gt = (torch.randn(B, H, L, 64, generator=g).to(torch.bfloat16).to(DEV) for _ in range(8))
+    mask = _mask(kind, B, H, L, torch.bfloat16, g)
+    m = None if mask is None else mask.to(DEV)
+    a = [x.requires_grad_() for x in (q, k, v)]
+
+    def step():
+        o, to = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, attn_mask=m, causal=kind == "causal"), tuple(a), (tq, tk, tv))
+        outs = [(o, go)] * (through != "t") + [(to, gt)] * (through != "o")
+        return list(torch.autograd.grad([x for x, _ in outs], a, [w for _, w in outs]))
+
+    gave_up, after = _replayed_behind_a_launch_that_gave_up(step)
+    for name, x in zip(("dq", "dk", "dv"), gave_up):
+        assert torch.isnan(x).any(-1).all(), name
+    for x, y in zip(after[1:], step()[1:]):  # (dQ has no fixed order of summation)
+        assert torch.equal(x, y)
+
+
 def _bias_forms(B, H, L, dt):
     g = torch.Generator().manual_seed(L)
     r = lambda *s: torch.randn(*s, generator=g).clamp(-5, 5).to(dt).to(DEV)  # noqa: E731
