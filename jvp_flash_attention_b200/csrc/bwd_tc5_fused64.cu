@@ -829,6 +829,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           alive = false;
           break;
         }
+        tc_fence_after();  // (behind the look or the wait: the stores follow what av_free says has been read)
         {
           const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + 16 * wg;
           if constexpr (HAS_GT) tmem_st16(trow + C::COL_AV, pk_av);

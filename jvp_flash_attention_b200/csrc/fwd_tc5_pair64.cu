@@ -886,6 +886,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
               st_shared_v4(pW + off, wp[4 * c], wp[4 * c + 1], wp[4 * c + 2], wp[4 * c + 3]);
             }
           } else {
+            if (hh == 0) tc_fence_after();  // (behind the look or the wait: the stores follow what pv_done says has been read)
             tmem_st16(tq + C::COL_P + 16 * hh, pp);
           }
         }
