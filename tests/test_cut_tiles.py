@@ -24,14 +24,54 @@ def _mask(kind, B, H, L, dt, g):
     return None
 
 
+def _host_mask(kind, H, L, dt):
+    """For the host logic alone, with rows as the native layer gives them to the kernels (addresses that nothing follows)."""
+    if kind in ("none", "causal", "keys"):
+        return _lib.Mask(kind={"none": _lib.MASK_NONE, "causal": _lib.MASK_CAUSAL, "keys": _lib.MASK_KVLEN}[kind], kv_len=1 << 20)
+    m = _lib.Mask(kind=_lib.MASK_BOOL if kind == "bool" else _lib.MASK_BIAS, bias_dtype=_lib.DTYPE_ENUM[dt], ptr=1 << 20)
+    row = (L + 15) // 16 * 16
+    m.stride[:] = [H * L * row, L * row, row, 1]
+    return m
+
+
+def _backward_is_cut(kind, B, H, L, dt, cot):
+    """Whether the workspace that the call asks for holds more than a bias's shares of dQ."""
+    x = 1 << 20
+    a = _lib.BwdArgs(struct_size=ctypes.sizeof(_lib.BwdArgs), dtype=_lib.DTYPE_ENUM[dt], B=B, H=H, L=L, D=64, sm_scale=0.125, q=x, k=x, v=x, lse=x,
+                     delta=x, dq=x, dk=x, dv=x, mask=_host_mask(kind, H, L, dt))
+    if cot != "o":
+        a.tq = a.tk = a.tv = a.gto = a.mu = a.eps = a.cterm = x
+    if cot != "t":
+        a.go = x
+    parts = 0
+    if kind == "bias" and cot != "o":
+        parts = (L + 127) // 128 * B * H * L * 64 * 4
+    else:
+        a.dq_accum = x
+    return _lib.load().jvpfa_bwd_workspace(ctypes.byref(a)) > parts
+
+
+def _forward_is_cut(kind, B, H, L, D, dt, dual):
+    class At(int):
+        shape = (B, H, L, D)
+    x = At(1 << 20)
+    a = _fwd_args([x] * 3, [x] * 3 * dual, _host_mask(kind, H, L, dt), [x, x if dual else None, x, x if dual else None], _lib.IMPL_AUTO)
+    a.dtype, a.mask_bits = _lib.DTYPE_ENUM[dt], x if kind == "bool" else None
+    return _lib.load().jvpfa_fwd_workspace(ctypes.byref(a)) > 0
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["none", "causal", "keys", "bool", "bias"])
-@pytest.mark.parametrize("B,H,L", [(1, 1, 1024), (1, 3, 1000), (5, 2, 720), (2, 12, 1024), (1, 150, 256)])
+@pytest.mark.parametrize("B,H,L", [(1, 1, 1024), (1, 3, 1000), (5, 2, 720), (2, 12, 1024), (1, 150, 256), (36, 1, 720)])
 @pytest.mark.parametrize("cot,dt", [("o", torch.float16), ("t", torch.bfloat16), ("both", torch.bfloat16)])
 def test_backward_of_cut_key_tiles(kind, B, H, L, cot, dt):
     """Against the float64 oracle: 2e-2 of the largest entry at least 1, the 16-bit bound of the parity tests, and in the 2-norm 1e-2 for
     bf16 and 2e-3 for fp16 (operands of 8 and 11 significant bits, four roundings on the longest way); dK and dV bit for bit the same
-    from run to run, also in a workspace full of NaN."""
+    from run to run, also in a workspace full of NaN.  (Left whole, by the rule: causal ones of many heads; the two launches' are a mask whose rows
+    are not whole 16-byte pieces, and a bias through tO below 96 key tiles.)"""
+    left = (kind == "causal" and B * H >= 24) or (kind in ("bool", "bias") and L % 16 != 0)
+    left = left or (kind == "bias" and cot != "o" and (L + 127) // 128 * B * H < 96)
+    assert _backward_is_cut(kind, B, H, L, dt, cot) != left
     g = torch.Generator().manual_seed(L + H)
     ts = [(torch.randn(B, H, L, 64, generator=g) * (0.1 if n in (3, 4, 5) else 1.0)).to(dt) for n in range(8)]
     mask, causal = _mask(kind, B, H, L, dt, g), kind == "causal"
@@ -63,11 +103,12 @@ def test_backward_of_cut_key_tiles(kind, B, H, L, cot, dt):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["none", "causal", "keys", "bool", "bias"])
-@pytest.mark.parametrize("B,H,L,D", [(1, 1, 2048, 64), (1, 3, 1000, 64), (5, 2, 1104, 64), (2, 12, 1024, 64), (1, 3, 1330, 32)])
+@pytest.mark.parametrize("B,H,L,D", [(1, 1, 2048, 64), (1, 3, 1000, 64), (5, 2, 1104, 64), (2, 12, 1024, 64), (1, 3, 1330, 32), (2, 12, 2048, 64)])
 @pytest.mark.parametrize("dual,dt", [(False, torch.bfloat16), (True, torch.float16), (True, torch.bfloat16)])
 def test_forward_of_cut_pairs(kind, B, H, L, D, dual, dt):
-    """Against the float64 oracle, bounds as above (one rounding fewer on the way), lse and mu as in the parity tests; bit for bit the same
-    from run to run, also in a workspace full of NaN.  A row's running maximum is one for each of its pieces."""
+    """Against the float64 oracle, bounds as above (one rounding fewer on the way); bit for bit the same from run to run, also in a workspace
+    full of NaN.  A row's running maximum is one for each of its pieces.  (Left whole, by the rule: 24 heads of L 1024, and causal ones.)"""
+    assert _forward_is_cut(kind, B, H, L, D, dt, dual) != (B * H == 24 and (L == 1024 or kind == "causal"))
     g = torch.Generator().manual_seed(L + H + D)
     ts = [(torch.randn(B, H, L, D, generator=g) * (0.1 if n in (3, 4, 5) else 1.0)).to(dt) for n in range(6)]
     ts[0][..., ::7, :] *= 4  # rows whose maximum moves from piece to piece
@@ -116,7 +157,7 @@ class _Forward:
         self.out = [nan(B, H, L, D, dt=ts[0].dtype), nan(B, H, L, D, dt=ts[0].dtype) if dual else None, nan(B, H, L), nan(B, H, L) if dual else None]
         self.args = a = _fwd_args(ts[:3], ts[3:], spec.to_c(), self.out, _lib.IMPL_TCGEN05)
         a.dtype = _lib.DTYPE_ENUM[ts[0].dtype]
-        self.kept = ts, spec
+        self.kept = ts, spec  # (what the arguments point to)
         if cut:
             n = _lib.load().jvpfa_fwd_workspace(ctypes.byref(a))
             assert n > 0, "this call is not cut"
@@ -127,6 +168,94 @@ class _Forward:
     def launch(self):
         _lib.check(_lib.load().jvpfa_fwd(ctypes.byref(self.args), torch.cuda.current_stream().cuda_stream), "jvpfa_fwd")
         return [x for x in self.out if x is not None]
+
+    def begins(self):
+        """[pair, key tile] where each of the CTAs began."""
+        return self.workspace[:4096].view(torch.int32)[:2 * self.ctas].view(-1, 2).tolist()
+
+
+def _begins(weights, steps, first, G):
+    """Where G CTAs begin, [item, step], on the line of the items from `first` on: weights[w] is how long item w is on it (0: it is not), two
+    more than the steps that it stands for; it has steps[w].  A cut leaves two steps on either side, or is moved to the item's beginning or its end
+    (of an item with fewer than two steps, always to its end)."""
+    line = [(w, x) for w, x in enumerate(weights) if w >= first and x > 0]
+    total = sum(x for _, x in line)
+    begins = []
+    for c in range(G):
+        pos, at = total * c // G, [len(weights), 0] if c else [first, 0]
+        for w, x in line if c else ():
+            if pos < x:
+                s = pos - 2 if pos >= 4 else 0
+                at = [w, s] if s <= steps[w] - 2 else [w + 1, 0]
+                break
+            pos -= x
+        begins.append(at)
+    return begins
+
+
+def _line_of_pairs(kind, B, H, L, lens):
+    """(weights, steps) of the forward's query pairs."""
+    P, N = (L + 255) // 256, (L + 63) // 64
+    steps = [min(N, 4 * r + 4) if kind == "causal" else (lens[b] + 63) // 64 if kind == "keys" else N for b in range(B) for _ in range(H) for r in range(P)]
+    stands_for = [4 * r + 4 for _ in range(B * H) for r in range(P)] if kind == "causal" else steps
+    return [x + 2 for x in stands_for], steps
+
+
+@pytest.mark.parametrize("kind", ["none", "causal", "keys"])
+def test_pieces_of_a_line_of_pairs(kind):
+    """On the model that the kernel is held against below: pieces follow one another, are alike, and no cut leaves fewer than two steps."""
+    g = torch.Generator().manual_seed(3)
+    r = lambda lo, hi: int(torch.randint(lo, hi + 1, (1,), generator=g))  # noqa: E731
+    for _ in range(60):
+        B, H, L = r(1, 40), r(1, 12), r(32, 3000)
+        lens = [r(0, L) for _ in range(B)]
+        weights, steps = _line_of_pairs(kind, B, H, L, lens)
+        G = min(148, sum(steps) // 4)
+        if G < 2:
+            continue
+        whole = 0 if kind != "none" else len(steps) // G
+        begins = _begins(weights, steps, whole * G, G) + [[len(steps), 0]]
+        piece = sum(weights[whole * G:]) / G
+        for (w0, s0), (w1, s1) in zip(begins, begins[1:]):
+            assert (w0, s0) <= (w1, s1) and (s1 == 0 or 2 <= s1 <= steps[w1] - 2)
+            took = sum(weights[w0:w1]) + (s1 + 2 if s1 else 0) - (s0 + 2 if s0 else 0)
+            assert took <= piece + 8, (took, piece)  # (a first cut moves back by up to 3, a last one on by up to 4, and rounding)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt,n", [(torch.bfloat16, 6), (torch.float16, 3)])
+@pytest.mark.parametrize("kind,B,H,L,D,whole", [
+    ("none", 1, 1, 2048, 64, 0), ("causal", 1, 3, 1040, 64, 0), ("keys", 5, 2, 1104, 64, 0), ("keys", 36, 1, 1104, 64, 0),
+    ("none", 36, 1, 1104, 64, 1), ("none", 2, 12, 2048, 64, 1), ("bool", 2, 12, 2048, 64, 1), ("bias", 2, 12, 2048, 64, 1),
+    ("none", 4, 16, 2048, 64, 3), ("bool", 1, 3, 1040, 32, 0), ("bias", 1, 3, 1040, 32, 0),
+])
+def test_where_pairs_are_cut_and_their_statistics(kind, B, H, L, D, whole, dt, n):
+    """O, tO, lse and mu of the first and the last head against the float64 oracle, in the parity tests' bounds and as above, with empty
+    sequences and rows that have no key; and every CTA's beginning against the model."""
+    g = torch.Generator().manual_seed(L + H + B)
+    ts = [(torch.randn(B, H, L, D, generator=g) * (0.1 if m > 2 else 1.0)).to(dt) for m in range(n)]
+    ts[0][..., ::7, :] *= 4
+    mask = _mask(kind, B, H, L, dt, g)
+    if kind == "keys":
+        mask[1] = False  # an empty sequence
+    if kind == "bool":
+        mask[:, :, 5] = False
+    f = _Forward([x.to(DEV) for x in ts], _spec(kind, None if mask is None else mask.to(DEV)), True)
+    got = dict(zip(("o", "to", "lse", "mu") if n == 6 else ("o", "lse"), f.launch()))
+    weights, steps = _line_of_pairs(kind, B, H, L, mask[:, 0, 0].sum(-1).tolist() if kind == "keys" else None)
+    assert f.begins() == _begins(weights, steps, whole * f.ctas, f.ctas)
+    assert _lib.device_status() == 0
+    rel = 1e-2 if dt == torch.bfloat16 else 2e-3
+    for b, h in ((0, 0), (B - 1, H - 1)) + (((1, 0),) if kind == "keys" else ()):
+        one = lambda x: None if x is None else x[b:b + 1, h:h + 1] if x.shape[1] > 1 else x[b:b + 1]  # noqa: E731
+        want = orc.tiled_forward(*(one(x) for x in ts), attn_mask=one(mask), causal=kind == "causal", block=256)
+        for name, x in got.items():
+            x, r = one(x).double().cpu(), torch.from_numpy(want[name])
+            none = torch.isinf(r)  # (lse of a row without a key)
+            assert torch.equal(torch.isposinf(x), none), name
+            x, r = x.masked_fill(none, 0.0), r.masked_fill(none, 0.0)
+            assert orc.max_abs_err(x, r) <= {"mu": 5e-2}.get(name, 2e-2 * max(1.0, r.abs().max().item()) if name != "lse" else 2e-2), name
+            assert name in ("lse", "mu") or (x - r).norm() <= rel * r.norm(), name
 
 
 @pytest.mark.gpu
