@@ -47,7 +47,11 @@ def test_bias_through_the_tangent(dt, cot, B, H, L, heads):
 
 def test_which_bias_backwards_take_a_workspace():
     """Host logic: from 96 key tiles on, as many bytes as a (B, H, L, L) bias of 16 bits when L is a multiple of 128; none for
-    what the two launches keep."""
+    what the two launches keep.  (Where there is a GPU, and key tiles are shared out among its SMs, room for their shares of dK and dV is
+    added: 16 KiB, and 128 KiB for each of the CTAs, one an SM.)"""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 0
+    shares = (0, *(16384 + 131072 * n for n in range(2, sms + 1)))
+
     def need(L=256, D=64, B=4, H=12, go=True, gto=True, dtype=_lib.BF16, bias=_lib.BF16, flags=0, impl=_lib.IMPL_AUTO):
         x = 1 << 20
         a = _lib.BwdArgs(struct_size=ctypes.sizeof(_lib.BwdArgs), dtype=dtype, B=B, H=H, L=L, D=D, impl=impl, sm_scale=0.125, q=x, k=x, v=x,
@@ -60,9 +64,10 @@ def test_which_bias_backwards_take_a_workspace():
         a.mask.stride[:] = [H * L * L, L * L, L, 1]
         return _lib.load().jvpfa_bwd_workspace(ctypes.byref(a))
 
-    assert need() == need(go=False) == 2 * 4 * 12 * 256 * 256
-    assert need(L=272) == 3 * 4 * 12 * 272 * 64 * 4
+    for through_both in (True, False):
+        assert need(go=through_both) - 2 * 4 * 12 * 256 * 256 in shares
+    assert need(L=272) - 3 * 4 * 12 * 272 * 64 * 4 in shares
     assert need(B=5, H=19, L=128) == 0 and need(B=6, H=16, L=16) > 0
     assert need(gto=False) == 0 and need(D=128) == 0 and need(L=264) == 0 and need(flags=2) == 0  # (2: no dK, dV asked for)
     assert need(bias=_lib.FP32) == 0 and need(bias=_lib.FP16) == 0 and need(impl=_lib.IMPL_GENERIC) == 0
-    assert need(L=8192, B=1, H=4) == 1 << 29 and need(L=8192, B=1, H=5) == 0
+    assert need(L=8192, B=1, H=4) - (1 << 29) in shares and need(L=8192, B=1, H=5) == 0
