@@ -13,6 +13,7 @@ import torch
 
 from jvp_flash_attention_b200 import _lib
 from jvp_flash_attention_b200 import jvp_attention as ja
+from tests.test_cut_tiles import _backward_is_cut, _forward_is_cut
 
 pytestmark = pytest.mark.gpu
 
@@ -150,3 +151,38 @@ def test_repeated_launches_with_a_bias_through_the_tangent(cot):
     asked = [(to, d["gto"])] + [(o, d["go"])] * (cot == "both")
     outs = [torch.empty_like(d["q"]) for _ in range(3)]
     _soak(_into(outs, lambda: torch.autograd.grad([x for x, _ in asked], a, [w for _, w in asked], retain_graph=True)), outs)
+
+
+def _cut_mask(kind, B, H, L):
+    g = torch.Generator(device=DEV).manual_seed(L)
+    if kind == "keys":
+        lens = torch.tensor([L, L // 2 + 3, 200, L - 1, 64], device=DEV)[:B]
+        return (torch.arange(L, device=DEV)[None] < lens[:, None])[:, None, None]
+    if kind == "bool":
+        return (torch.rand(B, H, L, L, device=DEV, generator=g) > 0.5) | torch.eye(L, dtype=torch.bool, device=DEV)
+    return torch.randn(B, H, L, L, device=DEV, generator=g).to(torch.bfloat16) if kind == "bias" else None
+
+
+@pytest.mark.parametrize("kind,B,H,L", [("none", 1, 3, 1040), ("causal", 1, 3, 1040), ("keys", 5, 2, 1104), ("bool", 1, 3, 1040),
+                                        ("bias", 2, 6, 1040), ("none", 2, 12, 2048)])
+def test_repeated_launches_with_tiles_shared_out(kind, B, H, L):
+    """The forward, without tangents and with, and the single pass through each output and both, where the rules cut tiles: the public API,
+    whose calls have a workspace.  (dQ has no fixed order, but for a bias through tO, from 96 key tiles on.)"""
+    d = _tensors(B, H, L, 64, torch.bfloat16, seed=3)
+    kw = dict(causal=kind == "causal", attn_mask=_cut_mask(kind, B, H, L))
+    assert _forward_is_cut(kind, B, H, L, 64, torch.bfloat16, True) and _forward_is_cut(kind, B, H, L, 64, torch.bfloat16, False)
+    outs = [torch.empty_like(d["q"]) for _ in range(3)]
+    _soak(_into(outs[:1], lambda: [ja.attention(d["q"], d["k"], d["v"], **kw)]), outs[:1])
+    a = [d[n].clone().requires_grad_() for n in "qkv"]
+
+    def dual():
+        return torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, **kw), tuple(a), (d["tq"], d["tk"], d["tv"]))
+
+    _soak(_into(outs[:2], lambda: [x.detach() for x in dual()]), outs[:2])
+    o, to = dual()
+    for cot in ("o", "t", "both"):
+        assert _backward_is_cut(kind, B, H, L, torch.bfloat16, cot)
+        asked = [(to, d["gto"])] * (cot != "o") + [(o, d["go"])] * (cot != "t")
+        fixed = kind == "bias" and cot != "o"
+        _soak(_into(outs, lambda: torch.autograd.grad([x for x, _ in asked], a, [w for _, w in asked], retain_graph=True)),
+              outs if fixed else outs[1:], close=[] if fixed else outs[:1])
