@@ -128,12 +128,15 @@ def run_fused64(n_subs, stages, seed, single_p_full=False, slow_dq=0.0, own_bufs
                 yield from wait_p_full(g)
                 if s == 0 and kact > 0:
                     yield from w.wait(acc_free, (kact - 1) & 1, ("acc_read", kact - 1))
+                # dV's products go first: the stage of G and gO, where they have a ring of their own, and the packed A and P are read
                 if g_stages:
                     gs = g % g_stages
                     w.later(lambda g=g, gs=gs: (w.tally(("gf", g), 2, ("g_free", g)), g_empty[gs].arrive()))
-                w.later(lambda g=g, st=st, ob=ob: (w.tally(("rf", g), 2, ("ring_free", g)), loop_empty[st].arrive(),
-                                                   w.tally(("of", g), 2, ("out_read", g)), out_free[ob].arrive(),
-                                                   w.events.add(("av_read", g)), av_free.arrive()))
+                w.later(lambda g=g: (w.events.add(("av_read", g)), av_free.arrive()))
+                yield
+                # ... then dK's
+                w.later(lambda g=g, st=st: (w.tally(("rf", g), 2, ("ring_free", g)), loop_empty[st].arrive()))
+                w.later(lambda g=g, ob=ob: (w.tally(("of", g), 2, ("out_read", g)), out_free[ob].arrive()))
                 g += 1
                 yield
             w.later(lambda kact=kact: (w.events.add(("done", kact)), done.arrive()))
@@ -159,14 +162,20 @@ def run_fused64(n_subs, stages, seed, single_p_full=False, slow_dq=0.0, own_bufs
         for kact, (k, n) in enumerate(items):
             for _ in range(n):
                 st, ob, use = g % n_stat, g & 1, g >> 1
+                # looks ahead of the need, without waiting: what a look sees as complete is not waited for
+                out_ok = use == 0 or out_free[ob].passed((use - 1) & 1)
+                assert use == 0 or not out_ok or ("out_read", g - 2) in w.events, "looked before the products had read"
                 yield from w.wait(stat_full[st], (g // n_stat) & 1, ("stat", g))
                 yield from w.wait(s_full, g & 1, ("scores", g))
                 w.tally(("sr", g), GROUPS, ("scores_read", g))
                 s_free.arrive()
                 yield
-                if use > 0:
+                if not out_ok:
                     yield from w.wait(out_free[ob], (use - 1) & 1, ("out_read", g - 2))
-                if g > 0:
+                av_ok = g == 0 or av_free.passed((g - 1) & 1)
+                assert g == 0 or not av_ok or ("av_read", g - 1) in w.events, "looked before dV's products had read"
+                yield
+                if not av_ok:
                     yield from w.wait(av_free, (g - 1) & 1, ("av_read", g - 1))
                 w.tally(("p", g), GROUPS, ("operands", g))
                 p_full[0 if single_p_full else ob].arrive()
