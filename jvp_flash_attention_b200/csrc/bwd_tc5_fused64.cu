@@ -19,7 +19,7 @@
 // rounding, not bitwise.  (With a bias and through tO a key tile's share is stored instead, see kDqParts.)
 //
 // Measured on a B200, cycles of a sub-tile inside an item (clock marks in one CTA, every SM at work): through O 1660, through tO 2310,
-// both 2600; the tensor pipe's own time is 1024, 1860 and 2050, so that with tangents it is busy four fifths of the time, and
+// both 2600; the tensor pipe's own time is 1024, 1860 and 2050, so that with tangents it is busy four fifths of a sub-tile, and
 // through O the elementwise threads are (two warps for a scheduler, so their latencies show).  A key tile's beginning costs 7.6 k
 // cycles more.  Before the looks at the barriers were taken together and dV's products went first: 2060, 2760, 3130.
 //

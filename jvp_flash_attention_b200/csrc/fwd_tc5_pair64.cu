@@ -131,9 +131,9 @@ struct TileUse {
 
 // ---- Pairs shared out among CTAs ----------------------------------------------------------------
 // Dealt whole, 192 pairs (B2 H12 L2048) take two rounds of 148 CTAs where 1.3 rounds' worth of work is there, and 16 leave 132 SMs idle.
-// With a workspace the key tiles of all pairs are one line that is cut into equal pieces (cut_begin); a pair that is cut leaves what
-// each CTA has of it, O and tO' before the division and the rows' statistics, all fp32, in the workspace, and pair64_finish_kernel
-// merges them in their order.  A pair's beginning counts as kPairOpen key tiles.
+// With a workspace whole rounds of pairs are dealt whole (where all pairs are alike; else none), and the key tiles of the rest are one line
+// that is cut into equal pieces (cut_begin); a pair that is cut leaves what each CTA has of it, O and tO' before the division and the
+// rows' statistics, all fp32, in the workspace, and pair64_finish_kernel merges them in their order.  A pair's beginning counts as kPairOpen key tiles.
 constexpr int kPairOpen = 2;
 template <bool DUAL>
 struct PairShare {  // floats: [query tile][16-byte piece of O, then of tO'][128 rows], then [128 rows]{maximum, sum, sum of W, 1: no key, no accumulators}
@@ -930,7 +930,8 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
 
 // The rows of the pairs that were cut.  Block x of 8 * (ctas - 1) looks at where CTA x / 8 + 1 begins; a pair that is cut there first is
 // this block's, an eighth of it: 128 rows of one query tile, 8 columns a thread of O and, at the same places, of tO.  Bound by reading
-// the shares (B2 H12 L2048: 40 MB, in L2); nearly all pairs have two, so two are requested before the first is looked at.
+// the shares: B2 H12 L2048 with tangents, 44 pairs among 148 CTAs, has 168 of 135 KB, 22.7 MB (11.8 us).  A pair has two shares at least,
+// and two are requested before the first is looked at; those beyond (one or two there) are read one after another.
 template <typename T, bool DUAL>
 __global__ void __launch_bounds__(256) pair64_finish_kernel(const jvpfa_fwd_args a, const float* shares, int ctas) {
   using S = PairShare<DUAL>;

@@ -18,6 +18,10 @@ Behaviour that goes beyond upstream, on purpose:
   (upstream scales the bias as well and ignores it in backward, jvp_attention.py:247-251,
   1519-1522), and a float mask without ``MASK_CONST`` entries is accepted (upstream raises
   ``UserWarning``, jvp_attention.py:2459-2462).
+
+Calls of one shape give the same bits from run to run, but for dQ of 16-bit calls at head dimension 64 (see
+``_lib.bwd``, ``dq_accum``).  16-bit calls at head dimension 64 and below cut their tiles among the SMs by the number
+of heads, so a head's last bits may differ between calls that compute it beside different numbers of others.
 """
 from __future__ import annotations
 
