@@ -27,7 +27,7 @@
 extern "C" {
 #endif
 
-#define JVPFA_VERSION 102 /* major*100 + minor; 101: fields after the last of 100 in four structs; 102: workspace in two */
+#define JVPFA_VERSION 103 /* major*100 + minor; 101: fields after the last of 100 in four structs; 102: workspace in two; 103: kv_len_host in two */
 
 typedef enum {
   JVPFA_OK = 0,
@@ -131,6 +131,10 @@ typedef struct {
    * too small: whole query tiles.  (struct_size up to flags: NULL.) */
   void* workspace;
   int64_t workspace_bytes;
+  /* Optional, JVPFA_MASK_KVLEN only: the B lengths of mask.kv_len in host memory, read while the call is made.  Whether sharing
+   * tiles out gains anything goes by them.  They decide nothing else: the kernels read mask.kv_len.  NULL: whole tiles.
+   * (struct_size up to workspace_bytes: NULL.) */
+  const int32_t* kv_len_host;
 } jvpfa_fwd_args;
 
 int jvpfa_fwd(const jvpfa_fwd_args* args, void* stream);
@@ -217,6 +221,7 @@ typedef struct {
    * mask_bits_t: NULL.) */
   void* workspace;
   int64_t workspace_bytes;
+  const int32_t* kv_len_host; /* as in jvpfa_fwd_args */
 } jvpfa_bwd_args;
 
 /* As jvpfa_fwd_workspace.  Non-zero for 16-bit types at D = 64 where the one pass (dq_accum) shares key tiles out among the SMs; for

@@ -94,6 +94,7 @@ class FwdArgs(C.Structure):
         ("flags", C.c_int32),
         ("workspace", C.c_void_p),
         ("workspace_bytes", C.c_int64),
+        ("kv_len_host", C.c_void_p),
     ]
 
 
@@ -152,6 +153,7 @@ class BwdArgs(C.Structure):
         ("mask_bits_t", C.c_void_p),
         ("workspace", C.c_void_p),
         ("workspace_bytes", C.c_int64),
+        ("kv_len_host", C.c_void_p),
     ]
 
 
@@ -313,7 +315,7 @@ class MaskSpec:
     bias, or int32 kv_len) and ``strides`` are the broadcast element strides of a (B,H,L,L) view.
     """
 
-    __slots__ = ("kind", "tensor", "strides", "bias_dtype", "tile_live", "tile_live_t", "fp32_mode", "fp32_parts", "_native")
+    __slots__ = ("kind", "tensor", "strides", "bias_dtype", "tile_live", "tile_live_t", "fp32_mode", "fp32_parts", "kv_len_host", "_native")
 
     def __init__(self, kind=MASK_NONE, tensor=None, strides=(0, 0, 0, 0), bias_dtype=FP32):
         self.kind = kind
@@ -322,6 +324,7 @@ class MaskSpec:
         self.bias_dtype = bias_dtype
         self.tile_live = None  # MASK_BOOL: bitmap from mask_tiles(), lets the forward step over dead tiles
         self.tile_live_t = None  # ... and its transpose (per 128-key tile), for the backward launch that owns keys
+        self.kv_len_host = None  # MASK_KVLEN: the lengths once more, as a list: whether cutting tiles pays goes by them
         self._native = None  # the native layer's form of this description, made on first use
         self.fp32_parts = False  # the forward of this call had a workspace for the fp32 tcgen05 kernels: so does a backward through O
         self.fp32_mode = None  # fp32 precision the forward of this call ran under ("3xtf32" / "tf32"); None = current
@@ -330,7 +333,7 @@ class MaskSpec:
         """This (by now complete) description as the native layer takes it."""
         if self._native is None:
             self._native = native().MaskDesc(self.kind, self.bias_dtype, self.tensor, self.strides, self.tile_live,
-                                             self.tile_live_t, copy.copy(self))
+                                             self.tile_live_t, self.kv_len_host or [], copy.copy(self))
         return self._native
 
     def to_c(self) -> Mask:

@@ -158,10 +158,10 @@ static const Args* current_args(const Args* a, Args* full, Sizes... earlier) {
   return full;
 }
 static const jvpfa_fwd_args* current_fwd_args(const jvpfa_fwd_args* a, jvpfa_fwd_args* full) {
-  return current_args(a, full, offsetof(jvpfa_fwd_args, mask_bits), offsetof(jvpfa_fwd_args, workspace));
+  return current_args(a, full, offsetof(jvpfa_fwd_args, mask_bits), offsetof(jvpfa_fwd_args, workspace), offsetof(jvpfa_fwd_args, kv_len_host));
 }
 static const jvpfa_bwd_args* current_bwd_args(const jvpfa_bwd_args* a, jvpfa_bwd_args* full) {
-  return current_args(a, full, offsetof(jvpfa_bwd_args, flags), offsetof(jvpfa_bwd_args, workspace));
+  return current_args(a, full, offsetof(jvpfa_bwd_args, flags), offsetof(jvpfa_bwd_args, workspace), offsetof(jvpfa_bwd_args, kv_len_host));
 }
 
 static int validate_pre(const jvpfa_pre_args* a) {

@@ -158,8 +158,8 @@ __device__ __forceinline__ int2 split_begin(const jvpfa_bwd_args& a, int c, int 
 //
 // dQ of a bias call through tO is summed in a fixed order, as the two launches that served it sum it: a key tile's share goes to
 // a buffer of its own (dq_acc: [key tile][B*H][L][D] floats) and fused64_finish_kernel adds them up.  Measured on a B200, the two
-// launches / this with the sum, us, bf16 through both outputs: B2 H12 L512 42 / 38, L1024 134 / 105, L2048 353 / 290, H4 L4096
-// 229 / 187; with 48 key tiles (B2 H12 L256) 22 / 28, with 32 (H1 L4096) 124 / 173.
+// launches / this with the sum, us, bf16 through both outputs: B2 H12 L512 34 / 25, L1024 121 / 75, L2048 342 / 255, H4 L4096
+// 226 / 172; with 48 key tiles (B2 H12 L256) 22 / 28, with 32 (H1 L4096) 124 / 173, both before key tiles were shared out.
 template <bool HAS_GT, int MK>
 constexpr bool kDqParts = HAS_GT && MK == 2;
 template <typename T, bool HAS_GO, bool HAS_GT, int MK, bool CUT>
@@ -1026,29 +1026,34 @@ static long long bwd_bias_workspace(const jvpfa_bwd_args& a) {
 // CTAs among which the key tiles' sub-tiles are shared out; 0: the key tiles are dealt whole.  Both in sub-tiles of the CTA that has
 // the most: dealt whole, in rounds; shared out, an equal part, one more beginning of a key tile, and the time of 2.5 us that the
 // shares' way through the workspace takes.  A twenty-fifth less is asked for: the last round of key tiles dealt whole has the memory to itself.
-// (Lengths of a key padding are not known here: as if there were none.)  fp16 B3 H12 L1330 causal through O, which this leaves whole: 46
-// us, 51 shared out.
+// fp16 B3 H12 L1330 causal through O, which this leaves whole: 46 us, 51 shared out.
+// Key padding: whole where the lengths are not known here.  With them the shares' way counts as 4 sub-tiles (5 through O) and 3 more where each CTA
+// has two of them, and a twentieth less is asked for (pieces end anywhere in ragged entries, so more tiles are cut).  340 draws of B to 70, H
+// to 16, L 256 to 4096 and lengths of L / 20 to L, through O / tO / both: 2 / 4 / 5 are more than 2 % slower than whole tiles, 7 % at most; by L
+// alone, and with the price above, every sixth was, 26 % at most (B2 H20 L1000, lengths 280 and 400, forward and backward 66 us whole, 74 shared out).
 static int split_ctas(const jvpfa_bwd_args& a, int sms) {
   const int open = kOpen, shares = a.gto ? 2 : 3;
-  const long long T = (a.L + 127) / 128, S = (a.L + 63) / 64, items = T * a.B * a.H;
-  const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL;
-  const long long subs = (long long)a.B * a.H * (causal ? T * S - T * (T - 1) : T * S), cost = subs + items * open;
+  const long long T = (a.L + 127) / 128, S = (a.L + 63) / 64, BH = (long long)a.B * a.H, items = T * BH;
+  const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL, keys = a.mask.kind == JVPFA_MASK_KVLEN;
+  if (keys && a.kv_len_host == nullptr) return 0;
+  const long long G = items < sms ? items : sms;
+  const HostLengths lengths(a.kv_len_host, a.B, a.L, keys && a.B <= kMaxSortedBatch && items > G);
+  long long live = items;  // key tiles that are not all padding
+  if (keys) {
+    live = 0;
+    for (int b = 0; b < a.B; ++b) live += lengths.tiles(b, 128) * a.H;
+  }
+  const long long subs = causal ? BH * (T * S - T * (T - 1)) : live * S, cost = subs + live * open;
   const long long ctas = subs / 4 < sms ? subs / 4 : sms;
-  if (ctas < 2 || !cut_fits(cost, ctas)) return 0;  // (that many rounds need no cuts)
-  const long long G = items < sms ? items : sms, rounds = (items + G - 1) / G;
-  long long whole = rounds * (S + open);
-  if (causal) {
-    whole = 0;
-    if (rounds > 8) return 0;  // (the lightest are dealt last and even out)
-    for (int at = 0; at <= 8; ++at) {
-      const long long c = (G - 1) * at / 8;
-      long long load = 0;
-      for (long long k = 0; k < rounds; ++k) {
-        const long long w = k * G + ((k & 1) ? G - 1 - c : c);
-        if (w < items) load += S - 2 * (w / ((long long)a.B * a.H)) + open;
-      }
-      whole = load > whole ? load : whole;
-    }
+  if (ctas < 2 || !cut_fits(items * (S + open), ctas)) return 0;  // (that many rounds need no cuts)
+  const long long rounds = (items + G - 1) / G;
+  if (rounds > (causal ? 8 : keys ? 16 : rounds)) return 0;  // (the lightest are dealt last and even out)
+  const long long whole = causal ? most_loaded(items, G, 8, [&](long long w) { return S - 2 * (w / BH) + open; })
+                          : keys ? most_loaded(items, G, 16, [&](long long w) { return lengths.tiles(w % BH / a.H, 128) > w / BH ? S + open : 0; })
+                                 : rounds * (S + open);
+  if (keys) {
+    const long long two = live < ctas ? live : ctas;  // CTAs that have two shares
+    return (cost + (open + shares + 2) * ctas + 3 * two) * 20 < whole * ctas * 19 ? (int)ctas : 0;
   }
   return (cost / ctas + open + shares) * 25 < whole * 24 ? (int)ctas : 0;
 }

@@ -1033,35 +1033,36 @@ static int pair_sm_count() {
 // shared out, bf16 with tangents: H4 L1024 27 / 20, H16 L1024 27 / 26, H24 L1024 31 / 35 (left whole), H48 L1024 52 / 47, H4 L2048 46 / 28, H24
 // L2048 91 / 74, H30 L2048 91 / 90 and with a bias 123 / 125, H12 L4096 169 / 129; causal H16 L1024 25 / 23, H24 L2048 52 / 55
 // (left whole), H8 L4096 86 / 59; without tangents H4 L1024 19 / 14, H24 L1024 21 / 23 (left whole).
-// Where tiles are stepped over their numbers are not known here: whole.  (Lengths of a key padding are not known either: as if there were none.)
+// Where tiles are stepped over their numbers are not known here: whole.
+// Key padding: whole where the lengths are not known here either.  With them the way of the shares counts as one more (pieces end anywhere in
+// ragged entries, so more pairs are cut).  Without tangents, lengths of about L / 10 and L / 2, whole / shared out as if there were no padding: B2 H12
+// L2048 13.2 / 19.3 and 29.3 / 31.2, B8 H2 L1024 7.6 / 13.0 and 12.7 / 16.3 (left whole), H4 L4096 12.0 / 15.8 (left whole) and 35.9 / 26.1.
 struct PairDeal {
   int ctas, whole;
 };
 static PairDeal deal_pairs(const jvpfa_fwd_args& a, int sms) {
   constexpr PairDeal all_whole{0, 0};
   if (a.mask.kind == JVPFA_MASK_BOOL && a.mask_tile_live != nullptr) return all_whole;
-  const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL;
+  const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL, keys = a.mask.kind == JVPFA_MASK_KVLEN;
+  if (keys && a.kv_len_host == nullptr) return all_whole;
   const long long P = (a.L + 255) / 256, N = (a.L + 63) / 64, BH = (long long)a.B * a.H, items = P * BH;
-  const long long steps = BH * (causal ? (P - 1) * P * 2 + N : P * N), line = BH * (causal ? P * (P + 1) * 2 : P * N) + items * kPairOpen;
+  const long long line = BH * (causal ? P * (P + 1) * 2 : P * N) + items * kPairOpen;  // (of keys: at most)
+  const long long G = items < sms ? items : sms;
+  const HostLengths lengths(a.kv_len_host, a.B, a.L, keys && a.B <= kMaxSortedBatch && items > G);
+  long long steps = BH * (causal ? (P - 1) * P * 2 + N : P * N);
+  if (keys) {
+    steps = 0;
+    for (int b = 0; b < a.B; ++b) steps += lengths.tiles(b, 64) * a.H * P;
+  }
   const long long ctas = steps / 4 < sms ? steps / 4 : sms;
   if (ctas < 2 || !cut_fits(line, ctas)) return all_whole;
-  const long long G = items < sms ? items : sms, rounds = (items + G - 1) / G;
-  long long most = rounds * N;
-  if (causal) {
-    most = 0;
-    if (rounds > 8) return all_whole;  // (the lightest are dealt last and even out)
-    for (int at = 0; at <= 8; ++at) {
-      const long long c = (G - 1) * at / 8;
-      long long load = 0;
-      for (long long k = 0; k < rounds; ++k) {
-        const long long w = k * G + ((k & 1) ? G - 1 - c : c);
-        if (w < items) load += N < 4 * (P - w / BH) ? N : 4 * (P - w / BH);
-      }
-      most = load > most ? load : most;
-    }
-  }
-  const long long whole = causal || a.mask.kind == JVPFA_MASK_KVLEN ? 0 : items / ctas;
-  const long long shared = whole > 0 ? whole * N + (items - whole * ctas) * N / ctas + 9 : steps / ctas + (2 * items > ctas ? 12 : 8);
+  const long long rounds = (items + G - 1) / G;
+  if (rounds > (causal ? 8 : keys ? 16 : rounds)) return all_whole;  // (the lightest are dealt last and even out)
+  const long long most = causal ? most_loaded(items, G, 8, [&](long long w) { return N < 4 * (P - w / BH) ? N : 4 * (P - w / BH); })
+                         : keys ? most_loaded(items, G, 16, [&](long long w) { return lengths.tiles(w / (a.H * P), 64); })
+                                : rounds * N;
+  const long long whole = causal || keys ? 0 : items / ctas;
+  const long long shared = whole > 0 ? whole * N + (items - whole * ctas) * N / ctas + 9 : steps / ctas + (2 * items > ctas ? 12 : 8) + keys;
   return shared * 20 < most * 19 ? PairDeal{(int)ctas, (int)whole} : all_whole;
 }
 

@@ -104,8 +104,8 @@ __global__ void __launch_bounds__(kCheckThreads) mask_check_kernel(const jvpfa_m
 // transposed as 8 x 8 bits, and the CTA's eight warps (256 rows) pass the transposed words through shared memory so that
 // they leave as 32-byte pieces.  B2 H12 L2048 (100 MB) 32 us, 36 where other kernels' lines leave L2 meanwhile; one head of L4096
 // (17 MB) 8 us; 16 bytes of up to eight rows at a time and a transposition bit by bit took 60 and 25 us.
-// With the packed mask, B2 H12 L2048 D64 and nine tenths random False: forward with tangents 168 -> 151 us, backward
-// through tO 239 -> 186 us.
+// With the packed mask, B2 H12 L2048 D64 and nine tenths random False: forward with tangents 140 -> 86 us, backward
+// through tO 221 -> 142 us.
 constexpr int kPackRows = 256, kPackKeys = 256;
 
 __device__ __forceinline__ uint32_t nonzero_bits(uint32_t w) {  // bytes -> four bits

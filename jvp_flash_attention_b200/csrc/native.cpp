@@ -32,6 +32,7 @@
 #include <memory>
 #include <optional>
 #include <string>
+#include <vector>
 
 #include "jvpfa.h"
 
@@ -56,11 +57,13 @@ py::object& python_module() {
 struct MaskDesc {
   jvpfa_mask c{};
   Tensor tensor, tile_live, tile_live_t;
+  std::vector<int32_t> kv_len;  // JVPFA_MASK_KVLEN: the lengths on the host
   std::shared_ptr<py::object> spec;
 
   MaskDesc(int kind, int bias_dtype, std::optional<Tensor> t, std::array<int64_t, 4> strides, std::optional<Tensor> live,
-           std::optional<Tensor> live_t, py::object spec_)
-      : spec(new py::object(std::move(spec_)), [](py::object* o) {
+           std::optional<Tensor> live_t, std::vector<int32_t> kv_len_, py::object spec_)
+      : kv_len(std::move(kv_len_)),
+        spec(new py::object(std::move(spec_)), [](py::object* o) {
           py::gil_scoped_acquire gil;
           delete o;
         }) {
@@ -189,6 +192,9 @@ struct Inputs {
 };
 
 // ---- masks -----------------------------------------------------------------------------------------------------------
+// The lengths of a key padding where they are known on the host.
+const int32_t* host_lengths(const MaskDesc& m, int B) { return m.kv_len.size() == (size_t)B ? m.kv_len.data() : nullptr; }
+
 // Whether the launches of a call may take the forms that only the 16-bit tensor-core kernels read.
 bool takes_16_bit_forms(const Tensor& q) { return q.is_cuda() && q.scalar_type() != at::kFloat && g_impl != JVPFA_IMPL_GENERIC; }
 
@@ -266,7 +272,7 @@ void pack(const MaskDesc& m, const Tensor& q, Tensor& bits_out, Tensor* bits_t_o
 // those of its verification.
 //
 // Packing reads the mask once (HBM bound) and saves a kernel that reads it one 16-byte piece per row and sub-tile.
-// B2 H12 L2048 D64, 100 MB of mask: packing 32 to 36 us; forward with tangents 168 -> 151 us, backward through tO 239 -> 186.
+// B2 H12 L2048 D64, 100 MB of mask: packing 28 to 32 us; forward with tangents 140 -> 86 us, backward through tO 221 -> 142.
 // So it pays with a backward, for a mask that several heads share, and where the bytes' layout would send the call to
 // the register-tiled kernels.  Where there is no memory for the bits the kernels read the bytes.
 void pack_mask(Call& call, const Tensor& q, bool backward) {
@@ -352,6 +358,7 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
   a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
   for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
+  a.kv_len_host = host_lengths(*call.mask, a.B);
   const bool fp32 = q.scalar_type() == at::kFloat;
   const Tensor workspace = workspace_of(!fp32 || call.parts ? jvpfa_fwd_workspace(&a) : 0, q);
   const Tensor bits = use_workspace(a, workspace, call, q);
@@ -442,6 +449,7 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
   a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
   for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
+  a.kv_len_host = host_lengths(m, a.B);
   const Tensor workspace = workspace_of((q.scalar_type() == at::kFloat ? call.parts : g_single_pass.load()) ? jvpfa_bwd_workspace(&a) : 0, q);
   const Tensor bits = use_workspace(a, workspace, call, q);
   check_status(jvpfa_bwd(&a, stream), "jvpfa_bwd");
@@ -736,7 +744,8 @@ PYBIND11_MODULE(_native, m) {
       .def("__enter__", [](NoFunctorchScope& s) { s.guard.emplace(); })
       .def("__exit__", [](NoFunctorchScope& s, py::args) { s.guard.reset(); });
   py::class_<MaskDesc, MaskPtr>(m, "MaskDesc")
-      .def(py::init<int, int, std::optional<Tensor>, std::array<int64_t, 4>, std::optional<Tensor>, std::optional<Tensor>, py::object>());
+      .def(py::init<int, int, std::optional<Tensor>, std::array<int64_t, 4>, std::optional<Tensor>, std::optional<Tensor>,
+                    std::vector<int32_t>, py::object>());
   m.def("attend", &attend);
   m.def("set_impl", [](int v) { g_impl = v; });
   m.def("set_single_pass", [](bool v) { g_single_pass = v; });

@@ -399,6 +399,40 @@ __device__ __forceinline__ int2 cut_begin(bool by_entry, int B, int H, int per_h
   return make_int2(bh * per_head + r, s);
 }
 inline bool cut_fits(long long line, long long ctas) { return line * ctas < 1ll << 32 && line < 1ll << 31; }
+// Items dealt whole in serpentine order to G CTAs: the load of the CTA that has most, of `looks` + 1 of them.  load(w): of item w.
+template <typename Load>
+long long most_loaded(long long items, long long G, int looks, Load load) {
+  long long most = 0;
+  for (int at = 0; at <= looks; ++at) {
+    const long long c = (G - 1) * at / looks;
+    long long sum = 0;
+    for (long long k = 0; k * G < items; ++k) {
+      const long long w = k * G + ((k & 1) ? G - 1 - c : c);
+      if (w < items) sum += load(w);
+    }
+    most = sum > most ? sum : most;
+  }
+  return most;
+}
+// The lengths of a key padding on the host, for the rules: tiles of `tile` keys of the batch entry that whole items meet r-th (where the
+// kernel sorts them by length, `sorted`, the r-th longest).
+struct HostLengths {
+  const int32_t* len;
+  int L;
+  bool sorted;
+  unsigned char order[kMaxSortedBatch];
+  HostLengths(const int32_t* l, int B, int L_, bool s) : len(l), L(L_), sorted(s) {
+    for (int b = 0; s && b < B; ++b) {
+      int r = b;
+      for (; r > 0 && len[order[r - 1]] < len[b]; --r) order[r] = order[r - 1];
+      order[r] = (unsigned char)b;
+    }
+  }
+  long long tiles(long long r, int tile) const {
+    const int n = len[sorted ? order[r] : r];
+    return ((n < 0 ? 0 : n > L ? L : n) + tile - 1) / tile;
+  }
+};
 // CTA c's place in the workspace for its share of item w, which is not its as a whole: 2 c where it takes the item over, else 2 c + 1;
 // -1 where the whole item is its.  at: {item, step} where this CTA and the next begin.
 __device__ __forceinline__ int cut_place(const int* at, int w, int c) {

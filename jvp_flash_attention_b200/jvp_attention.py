@@ -202,12 +202,14 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, verify: boo
             rows = m.reshape(mz, N)
             lens = rows.sum(dim=-1, dtype=torch.int32)
             prefix = torch.arange(N, device=m.device).unsqueeze(0) < lens.unsqueeze(1)
-            is_prefix, min_len = torch.stack(((prefix == rows).all().to(torch.int32), lens.min())).tolist()
+            is_prefix, *host_lens = torch.cat(((prefix == rows).all().to(torch.int32).view(1), lens)).tolist()
             if is_prefix:
                 if verify:
-                    assert min_len > 0, "The attention mask cannot be all False for any head."
+                    assert min(host_lens) > 0, "The attention mask cannot be all False for any head."
                 kv_len = lens.expand(Z).contiguous() if mz == 1 else lens.contiguous()
-                return _lib.MaskSpec(_lib.MASK_KVLEN, kv_len), 1, attn_mask
+                spec = _lib.MaskSpec(_lib.MASK_KVLEN, kv_len)
+                spec.kv_len_host = host_lens * Z if mz == 1 else host_lens
+                return spec, 1, attn_mask
         m8 = m.view(torch.uint8) if m.is_contiguous() or m.stride(-1) == 1 else m.contiguous().view(torch.uint8)
         spec = _lib.MaskSpec(_lib.MASK_BOOL, m8, bstrides(m8))
         every_head_live = True

@@ -13,10 +13,14 @@ from tests.test_fp32_tcgen05 import _fwd_args
 DEV = "cuda:0"
 
 
+def _lengths(B, L):
+    """Whole and ragged entries, of one and of few keys."""
+    return ([L, L // 2 + 3, 2, 1, L - 1] * B)[:B] if B > 1 else [L - 3]
+
+
 def _mask(kind, B, H, L, dt, g):
-    if kind == "keys":  # entries of one and of few keys, whole and ragged ones
-        lens = torch.tensor([2, 1, L, L // 2 + 3, L - 1] * B)[:B] if B > 1 else torch.tensor([L // 2 + 3])
-        return (torch.arange(L)[None, :] < lens[:, None])[:, None, None, :]
+    if kind == "keys":
+        return (torch.arange(L)[None, :] < torch.tensor(_lengths(B, L))[:, None])[:, None, None, :]
     if kind == "bool":
         return (torch.rand(B, H, L, L, generator=g) > 0.5) | torch.eye(L, dtype=torch.bool)
     if kind == "bias":
@@ -34,8 +38,13 @@ def _host_mask(kind, H, L, dt):
     return m
 
 
-def _backward_is_cut(kind, B, H, L, dt, cot):
+def _on_the_host(lengths):
+    return (ctypes.c_int32 * len(lengths))(*lengths)
+
+
+def _backward_is_cut(kind, B, H, L, dt, cot, lengths=None):
     """Whether the workspace that the call asks for holds more than a bias's shares of dQ."""
+    lengths = _on_the_host(lengths or _lengths(B, L))
     x = 1 << 20
     a = _lib.BwdArgs(struct_size=ctypes.sizeof(_lib.BwdArgs), dtype=_lib.DTYPE_ENUM[dt], B=B, H=H, L=L, D=64, sm_scale=0.125, q=x, k=x, v=x, lse=x,
                      delta=x, dq=x, dk=x, dv=x, mask=_host_mask(kind, H, L, dt))
@@ -43,6 +52,8 @@ def _backward_is_cut(kind, B, H, L, dt, cot):
         a.tq = a.tk = a.tv = a.gto = a.mu = a.eps = a.cterm = x
     if cot != "t":
         a.go = x
+    if kind == "keys":
+        a.kv_len_host = ctypes.addressof(lengths)
     parts = 0
     if kind == "bias" and cot != "o":
         parts = (L + 127) // 128 * B * H * L * 64 * 4
@@ -51,12 +62,15 @@ def _backward_is_cut(kind, B, H, L, dt, cot):
     return _lib.load().jvpfa_bwd_workspace(ctypes.byref(a)) > parts
 
 
-def _forward_is_cut(kind, B, H, L, D, dt, dual):
+def _forward_is_cut(kind, B, H, L, D, dt, dual, lengths=None):
+    lengths = _on_the_host(lengths or _lengths(B, L))
     class At(int):
         shape = (B, H, L, D)
     x = At(1 << 20)
     a = _fwd_args([x] * 3, [x] * 3 * dual, _host_mask(kind, H, L, dt), [x, x if dual else None, x, x if dual else None], _lib.IMPL_AUTO)
     a.dtype, a.mask_bits = _lib.DTYPE_ENUM[dt], x if kind == "bool" else None
+    if kind == "keys":
+        a.kv_len_host = ctypes.addressof(lengths)
     return _lib.load().jvpfa_fwd_workspace(ctypes.byref(a)) > 0
 
 
@@ -67,9 +81,9 @@ def _forward_is_cut(kind, B, H, L, D, dt, dual):
 def test_backward_of_cut_key_tiles(kind, B, H, L, cot, dt):
     """Against the float64 oracle: 2e-2 of the largest entry at least 1, the 16-bit bound of the parity tests, and in the 2-norm 1e-2 for
     bf16 and 2e-3 for fp16 (operands of 8 and 11 significant bits, four roundings on the longest way); dK and dV bit for bit the same
-    from run to run, also in a workspace full of NaN.  (Left whole, by the rule: causal ones of many heads; the two launches' are a mask whose rows
-    are not whole 16-byte pieces, and a bias through tO below 96 key tiles.)"""
-    left = (kind == "causal" and B * H >= 24) or (kind in ("bool", "bias") and L % 16 != 0)
+    from run to run, also in a workspace full of NaN.  (Left whole, by the rule: causal ones and a padded one of many heads; the two launches'
+    are a mask whose rows are not whole 16-byte pieces, and a bias through tO below 96 key tiles.)"""
+    left = (kind == "causal" and B * H >= 24) or (kind == "keys" and H == 150) or (kind in ("bool", "bias") and L % 16 != 0)
     left = left or (kind == "bias" and cot != "o" and (L + 127) // 128 * B * H < 96)
     assert _backward_is_cut(kind, B, H, L, dt, cot) != left
     g = torch.Generator().manual_seed(L + H)
@@ -107,8 +121,8 @@ def test_backward_of_cut_key_tiles(kind, B, H, L, cot, dt):
 @pytest.mark.parametrize("dual,dt", [(False, torch.bfloat16), (True, torch.float16), (True, torch.bfloat16)])
 def test_forward_of_cut_pairs(kind, B, H, L, D, dual, dt):
     """Against the float64 oracle, bounds as above (one rounding fewer on the way); bit for bit the same from run to run, also in a workspace
-    full of NaN.  A row's running maximum is one for each of its pieces.  (Left whole, by the rule: 24 heads of L 1024, and causal ones.)"""
-    assert _forward_is_cut(kind, B, H, L, D, dt, dual) != (B * H == 24 and (L == 1024 or kind == "causal"))
+    full of NaN.  A row's running maximum is one for each of its pieces.  (Left whole, by the rule: 24 heads of L 1024, and causal and padded ones.)"""
+    assert _forward_is_cut(kind, B, H, L, D, dt, dual) != (B * H == 24 and (L == 1024 or kind in ("causal", "keys")))
     g = torch.Generator().manual_seed(L + H + D)
     ts = [(torch.randn(B, H, L, D, generator=g) * (0.1 if n in (3, 4, 5) else 1.0)).to(dt) for n in range(6)]
     ts[0][..., ::7, :] *= 4  # rows whose maximum moves from piece to piece
@@ -148,7 +162,8 @@ def _spec(kind, mask):
 
 
 class _Forward:
-    """jvpfa_fwd on q, k, v and, as far as given, their tangents.  cut: with the workspace that it asks for, full of NaN."""
+    """jvpfa_fwd on q, k, v and, as far as given, their tangents.  cut: with the workspace that it asks for, full of NaN (key padding: that
+    it asks for where the host says that no key is padding, which decides nothing else)."""
 
     def __init__(self, ts, spec, cut):
         B, H, L, D = ts[0].shape
@@ -157,7 +172,9 @@ class _Forward:
         self.out = [nan(B, H, L, D, dt=ts[0].dtype), nan(B, H, L, D, dt=ts[0].dtype) if dual else None, nan(B, H, L), nan(B, H, L) if dual else None]
         self.args = a = _fwd_args(ts[:3], ts[3:], spec.to_c(), self.out, _lib.IMPL_TCGEN05)
         a.dtype = _lib.DTYPE_ENUM[ts[0].dtype]
-        self.kept = ts, spec  # (what the arguments point to)
+        self.kept = ts, spec, _on_the_host([L] * B)  # (what the arguments point to)
+        if spec.kind == _lib.MASK_KVLEN:
+            a.kv_len_host = ctypes.addressof(self.kept[2])
         if cut:
             n = _lib.load().jvpfa_fwd_workspace(ctypes.byref(a))
             assert n > 0, "this call is not cut"
@@ -225,8 +242,8 @@ def test_pieces_of_a_line_of_pairs(kind):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dt,n", [(torch.bfloat16, 6), (torch.float16, 3)])
 @pytest.mark.parametrize("kind,B,H,L,D,whole", [
-    ("none", 1, 1, 2048, 64, 0), ("causal", 1, 3, 1040, 64, 0), ("keys", 5, 2, 1104, 64, 0), ("keys", 36, 1, 1104, 64, 0),
-    ("none", 36, 1, 1104, 64, 1), ("none", 2, 12, 2048, 64, 1), ("bool", 2, 12, 2048, 64, 1), ("bias", 2, 12, 2048, 64, 1),
+    ("none", 1, 1, 2048, 64, 0), ("causal", 1, 3, 1040, 64, 0), ("keys", 5, 2, 1104, 64, 0), ("keys", 38, 1, 1024, 64, 0),
+    ("none", 38, 1, 1024, 64, 1), ("none", 2, 12, 2048, 64, 1), ("bool", 2, 12, 2048, 64, 1), ("bias", 2, 12, 2048, 64, 1),
     ("none", 4, 16, 2048, 64, 3), ("bool", 1, 3, 1040, 32, 0), ("bias", 1, 3, 1040, 32, 0),
 ])
 def test_where_pairs_are_cut_and_their_statistics(kind, B, H, L, D, whole, dt, n):
@@ -317,6 +334,26 @@ def _replayed_behind_a_launch_that_gave_up(step):
         finally:
             assert _lib.device_status(clear=True) == code
     return seen
+
+
+@pytest.mark.gpu
+def test_key_padding_is_cut_by_its_lengths():
+    """Short entries leave whole tiles the better deal, as if the tensors were that short; so they are where the host does not know the lengths."""
+    dt = torch.bfloat16
+    for (B, H, L), lengths, forward, backward in (((8, 2, 1024), [1024] * 8, True, False), ((8, 2, 1024), [512] * 8, False, True),
+                                                  ((8, 2, 1024), [32] * 8, False, None), ((1, 4, 4096), [4096], True, False), ((1, 4, 4096), [1024], True, True),
+                                                  ((1, 4, 4096), [128], False, True), ((2, 20, 1000), [280, 400], False, False),
+                                                  ((2, 20, 512), [268, 384], False, False), ((8, 12, 256), [100] * 8, False, False)):
+        for dual in (False, True):
+            assert _forward_is_cut("keys", B, H, L, 64, dt, dual, lengths) == forward, (B, H, L, lengths)
+        for cot in ("o", "t", "both") if backward is not None else ():
+            assert _backward_is_cut("keys", B, H, L, dt, cot, lengths) == backward, (B, H, L, lengths, cot)
+    x = torch.zeros(1, 4, 4096, 64, dtype=dt, device=DEV)
+    f = _Forward([x, x, x], _lib.MaskSpec(_lib.MASK_KVLEN, torch.full((1,), 4096, dtype=torch.int32, device=DEV)), True)
+    f.args.kv_len_host = None
+    assert _lib.load().jvpfa_fwd_workspace(ctypes.byref(f.args)) == 0
+    spec = ja.classify_mask(torch.ones(1, 1, 1, 4096, dtype=torch.bool, device=DEV), False, 3, 4, 4096, dt, True)[0]
+    assert spec.kv_len_host == [4096] * 3
 
 
 @pytest.mark.gpu

@@ -13,7 +13,7 @@ import torch
 
 from jvp_flash_attention_b200 import _lib
 from jvp_flash_attention_b200 import jvp_attention as ja
-from tests.test_cut_tiles import _backward_is_cut, _forward_is_cut
+from tests.test_cut_tiles import _backward_is_cut, _forward_is_cut, _lengths
 
 pytestmark = pytest.mark.gpu
 
@@ -156,8 +156,7 @@ def test_repeated_launches_with_a_bias_through_the_tangent(cot):
 def _cut_mask(kind, B, H, L):
     g = torch.Generator(device=DEV).manual_seed(L)
     if kind == "keys":
-        lens = torch.tensor([L, L // 2 + 3, 200, L - 1, 64], device=DEV)[:B]
-        return (torch.arange(L, device=DEV)[None] < lens[:, None])[:, None, None]
+        return (torch.arange(L, device=DEV)[None] < torch.tensor(_lengths(B, L), device=DEV)[:, None])[:, None, None]
     if kind == "bool":
         return (torch.rand(B, H, L, L, device=DEV, generator=g) > 0.5) | torch.eye(L, dtype=torch.bool, device=DEV)
     return torch.randn(B, H, L, L, device=DEV, generator=g).to(torch.bfloat16) if kind == "bias" else None
