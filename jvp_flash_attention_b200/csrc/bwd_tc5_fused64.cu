@@ -1024,15 +1024,17 @@ static long long bwd_bias_workspace(const jvpfa_bwd_args& a) {
 }
 
 // CTAs among which the key tiles' sub-tiles are shared out; 0: the key tiles are dealt whole.  Both in sub-tiles of the CTA that has
-// the most: dealt whole, in rounds; shared out, an equal part, one more beginning of a key tile, and the time of 2.5 us that the
-// shares' way through the workspace takes.  A twenty-fifth less is asked for: the last round of key tiles dealt whole has the memory to itself.
-// fp16 B3 H12 L1330 causal through O, which this leaves whole: 46 us, 51 shared out.
-// Key padding: whole where the lengths are not known here.  With them the shares' way counts as 4 sub-tiles (5 through O) and 3 more where each CTA
-// has two of them, and a twentieth less is asked for (pieces end anywhere in ragged entries, so more tiles are cut).  340 draws of B to 70, H
-// to 16, L 256 to 4096 and lengths of L / 20 to L, through O / tO / both: 2 / 4 / 5 are more than 2 % slower than whole tiles, 7 % at most; by L
-// alone, and with the price above, every sixth was, 26 % at most (B2 H20 L1000, lengths 280 and 400, forward and backward 66 us whole, 74 shared out).
+// the most: dealt whole, in rounds; shared out, an equal part, one more beginning of a key tile, and the time of the shares' way through
+// the workspace: 2 sub-tiles (3 through O) and 2 (1) more where each CTA has two shares.  A twenty-fifth less is asked for: the last round
+// of key tiles dealt whole has the memory to itself.  800 draws of B to 32, H to 40, L 256 to 4096 and every mask, where the shares' way at
+// 2 (3) had these cut: 6 / 17 / 12 % of them were more than 2 % slower than whole tiles through O / tO / both (B3 H6 L640 through tO 27.3 whole, 32.6
+// shared out), with this price 4 / 5 / 3 %, 12 % at most.  fp16 B3 H12 L1330 causal through O, left whole: 46 us, 51 shared out.
+// Key padding: whole where the lengths are not known here.  With them 4 sub-tiles (5) and 3 more, and a twentieth less is asked for (pieces end
+// anywhere in ragged entries, so more tiles are cut).  340 draws of B to 70, H to 16, L 256 to 4096 and lengths of L / 20 to L, through O /
+// tO / both: 2 / 4 / 5 are more than 2 % slower than whole tiles, 7 % at most; by L alone, and with 2 (3) sub-tiles, every sixth was, 26 % at
+// most (B2 H20 L1000, lengths 280 and 400, forward and backward 66 us whole, 74 shared out).
 static int split_ctas(const jvpfa_bwd_args& a, int sms) {
-  const int open = kOpen, shares = a.gto ? 2 : 3;
+  const int open = kOpen;
   const long long T = (a.L + 127) / 128, S = (a.L + 63) / 64, BH = (long long)a.B * a.H, items = T * BH;
   const bool causal = a.mask.kind == JVPFA_MASK_CAUSAL, keys = a.mask.kind == JVPFA_MASK_KVLEN;
   if (keys && a.kv_len_host == nullptr) return 0;
@@ -1051,11 +1053,9 @@ static int split_ctas(const jvpfa_bwd_args& a, int sms) {
   const long long whole = causal ? most_loaded(items, G, 8, [&](long long w) { return S - 2 * (w / BH) + open; })
                           : keys ? most_loaded(items, G, 16, [&](long long w) { return lengths.tiles(w % BH / a.H, 128) > w / BH ? S + open : 0; })
                                  : rounds * (S + open);
-  if (keys) {
-    const long long two = live < ctas ? live : ctas;  // CTAs that have two shares
-    return (cost + (open + shares + 2) * ctas + 3 * two) * 20 < whole * ctas * 19 ? (int)ctas : 0;
-  }
-  return (cost / ctas + open + shares) * 25 < whole * 24 ? (int)ctas : 0;
+  const int way = (a.gto ? 2 : 3) + (keys ? 2 : 0), more = keys ? 3 : a.gto ? 2 : 1, of = keys ? 20 : 25;
+  const long long two = live < ctas ? live : ctas;  // CTAs that have two shares
+  return (cost + (open + way) * ctas + more * two) * of < whole * ctas * (of - 1) ? (int)ctas : 0;
 }
 
 template <typename T, bool HAS_GO, bool HAS_GT, int MK, bool CUT>

@@ -81,9 +81,9 @@ def _forward_is_cut(kind, B, H, L, D, dt, dual, lengths=None):
 def test_backward_of_cut_key_tiles(kind, B, H, L, cot, dt):
     """Against the float64 oracle: 2e-2 of the largest entry at least 1, the 16-bit bound of the parity tests, and in the 2-norm 1e-2 for
     bf16 and 2e-3 for fp16 (operands of 8 and 11 significant bits, four roundings on the longest way); dK and dV bit for bit the same
-    from run to run, also in a workspace full of NaN.  (Left whole, by the rule: causal ones and a padded one of many heads; the two launches'
-    are a mask whose rows are not whole 16-byte pieces, and a bias through tO below 96 key tiles.)"""
-    left = (kind == "causal" and B * H >= 24) or (kind == "keys" and H == 150) or (kind in ("bool", "bias") and L % 16 != 0)
+    from run to run, also in a workspace full of NaN.  (Left whole, by the rule: causal ones of many heads, and short ones of 150; the two
+    launches' are a mask whose rows are not whole 16-byte pieces, and a bias through tO below 96 key tiles.)"""
+    left = (kind == "causal" and B * H >= 24) or H == 150 or (kind in ("bool", "bias") and L % 16 != 0)
     left = left or (kind == "bias" and cot != "o" and (L + 127) // 128 * B * H < 96)
     assert _backward_is_cut(kind, B, H, L, dt, cot) != left
     g = torch.Generator().manual_seed(L + H)

@@ -163,7 +163,7 @@ def _cut_mask(kind, B, H, L):
 
 
 @pytest.mark.parametrize("kind,B,H,L", [("none", 1, 3, 1040), ("causal", 1, 3, 1040), ("keys", 5, 2, 1104), ("bool", 1, 3, 1040),
-                                        ("bias", 2, 6, 1040), ("none", 2, 12, 2048)])
+                                        ("bias", 1, 6, 2064), ("none", 2, 12, 2048)])
 def test_repeated_launches_with_tiles_shared_out(kind, B, H, L):
     """The forward, without tangents and with, and the single pass through each output and both, where the rules cut tiles: the public API,
     whose calls have a workspace.  (dQ has no fixed order, but for a bias through tO, from 96 key tiles on.)"""
