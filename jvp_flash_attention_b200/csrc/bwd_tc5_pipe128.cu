@@ -6,7 +6,7 @@
 // instances of one template:
 //   "own" side  : 128 rows, one per TMEM lane; four operand tiles resident in smem
 //                 own keys: K, tK, V, tV        own queries: Q, tQ, G, gO        (G = cotangent of tO)
-//   "loop" side : tiles of BL rows (32 with own keys, 48 with own queries) streamed by TMA, the tensors of a stage
+//   "loop" side : tiles of BL rows (32 with own keys, 48 with own queries, 64 and 96 without tangents) streamed by TMA, the tensors of a stage
 //                 adjacent.  Own keys: Q, tQ, G, gO in one three-stage ring.  Own queries: K, tK in a three-stage
 //                 ring (the output products read them again), V, tV in a one-stage ring that comes free as soon
 //                 as the tile's scores exist.
@@ -43,7 +43,10 @@ struct BwdPipeCfg {
   // Rows of a loop tile.  An MMA instruction of N = 32 costs 40 cycles and one of N = 64 48 (mbar_wait_warp's comment), so wider tiles
   // cost less per column.  Own keys: dK | dV take 256 TMEM columns, which leaves two score buffers of 4 x 32; own
   // queries: dQ takes 128, which leaves two buffers of 4 x 48.
-  static constexpr int BL = OWN_KEYS ? 32 : 48;
+  //   Without tangents there are S and FP alone, half of the operand tiles too: two buffers of 2 x 64 beside dK | dV, of 2 x 96 beside dQ.
+  // Most of a tile's time is its hand-overs (16 columns a thread in either case).  Both launches on a B200, bf16, tiles of 32 and 48 -> 64 and
+  // 96: B1 H16 L8192 2290 -> 1528 us, B3 H7 L4032 with 3/4 of the keys 658 -> 407, B6 H16 L648 with bias 200 -> 161, B2 H8 L1024 51.5 -> 50.
+  static constexpr int BL = HAS_GT ? (OWN_KEYS ? 32 : 48) : OWN_KEYS ? 64 : 96;
   static constexpr int NP = BL / 16;                // 16-column pieces = elementwise warpgroups
   static constexpr int NTHREADS = 64 + 128 * NP + 32;  // producer, issuer, NP elementwise warpgroups, second issuer
   static constexpr int WARP_ISSUER2 = 2 + 4 * NP;
@@ -52,29 +55,34 @@ struct BwdPipeCfg {
   static constexpr int LQ_BYTES = BL * 128;         // one loop tensor, one 64-column half
   // Ring X holds the loop tensors that the output products read again (they stay until the tile's outputs are done);
   // ring Y those that only the score products read (free as soon as the scores exist).  Own keys: all four in X.
-  static constexpr int NX = OWN_KEYS ? 4 : 2;
-  static constexpr int NY = 4 - NX;
+  // Without tangents there is room for one ring of both tensors.
+  static constexpr int SLOTS = HAS_GT ? 4 : 2;      // operand tiles of either side
+  static constexpr int NX = OWN_KEYS || !HAS_GT ? SLOTS : 2;
+  static constexpr int NY = SLOTS - NX;
+  // Which of a side's tiles a slot is: K, tK, V, tV; Q, tQ, G, gO; without tangents the first and the one that FP is formed of
+  static constexpr int slot(int s) { return HAS_GT || s == 0 ? s : 1; }
   static constexpr int XSTAGES = 3;
   static constexpr int X_HALF = NX * LQ_BYTES;      // [x0 | x1 (| x2 | x3)] of one half
   static constexpr int X_STAGE = 2 * X_HALF;
   static constexpr int Y_HALF = NY * LQ_BYTES;
   static constexpr int Y_STAGE = 2 * Y_HALF;        // one stage
-  static constexpr int OFF_X = 4 * OWN_BYTES;
+  static constexpr int OFF_X = SLOTS * OWN_BYTES;
   static constexpr int OFF_Y = OFF_X + XSTAGES * X_STAGE;
-  static constexpr int TILE_BYTES = OFF_Y + Y_STAGE;  // 224 KiB
+  static constexpr int TILE_BYTES = OFF_Y + Y_STAGE;  // 224 KiB; without tangents 160 and 208
   static constexpr int STAT_BYTES = OWN_KEYS ? XSTAGES * BL * 16 : 0;
   static constexpr int SMEM_BYTES = TILE_BYTES + STAT_BYTES + 256 + 1024;
   // tensors actually loaded
   static constexpr int N_KEY = HAS_GT ? 4 : 2;                               // K, V (+ tK, tV)
   static constexpr int N_QRY = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0);      // Q (+ gO) (+ tQ, G)
   static constexpr int N_OWN = OWN_KEYS ? N_KEY : N_QRY;
-  static constexpr int N_X = OWN_KEYS ? N_QRY : (HAS_GT ? 2 : 1);            // own queries: K (+ tK)
-  static constexpr int N_Y = OWN_KEYS ? 0 : (HAS_GT ? 2 : 1);                // own queries: V (+ tV)
+  static constexpr int N_X = OWN_KEYS ? N_QRY : 2;                           // own queries: K, tK or K, V
+  static constexpr int N_Y = NY;                                             // own queries: V, tV
   // TMEM columns
-  static constexpr int SC_COLS = 4 * BL;  // one buffer: S | TS | E | FP
-  static constexpr int COL_S = 0, COL_TS = BL, COL_E = 2 * BL, COL_FP = 3 * BL;
+  static constexpr int SC_COLS = SLOTS * BL;  // one buffer: S | TS | E | FP, or S | FP
+  static constexpr int COL_S = 0, COL_TS = BL, COL_E = 2 * BL, COL_FP = (SLOTS - 1) * BL;
   // Packed operands: piece h (columns 16h .. 16h+15 of the tile) of gS at COL_S + 16h, of gtS 8 columns on;
-  // of A at COL_TS + 16h, of P 8 columns on.
+  // of A at COL_TS + 16h, of P 8 columns on.  Without tangents P takes gtS's place (FP's columns are the second issuer's).
+  static constexpr int COL_P = HAS_GT ? COL_TS + 8 : COL_S + 8;
   static constexpr int COL_OUT0 = 2 * SC_COLS;
   static constexpr int COL_OUT1 = COL_OUT0 + D;
   static constexpr int COLS_ALLOC = 512;
@@ -82,11 +90,12 @@ struct BwdPipeCfg {
 };
 static_assert(BwdPipeCfg<true, true, true>::SMEM_BYTES <= 227 * 1024, "shared memory budget");
 static_assert(BwdPipeCfg<false, true, true>::SMEM_BYTES <= 227 * 1024, "shared memory budget");
+static_assert(BwdPipeCfg<false, true, false>::SMEM_BYTES <= 227 * 1024, "shared memory budget");
 
 // MK == 3: walks the loop tiles of a CTA that hold a true mask entry, in order.  The bitmaps of jvpfa_mask_tiles have one
 // bit per 128-query x 64-key tile.  Own keys: w points at the transposed bitmap's entry of the own 128-key tile (bit =
-// 128-query tile, four 32-row loop tiles each).  Own queries: w points at the bitmap's entry of the own 128-query tile
-// (bit = 64-key tile); a 48-key loop tile is live if one of the one or two 64-key tiles it overlaps is.
+// 128-query tile, four 32-row or two 64-row loop tiles each).  Own queries: w points at the bitmap's entry of the own 128-query tile
+// (bit = 64-key tile); a 48- or 96-key loop tile is live if one of the one or two 64-key tiles it overlaps is.
 template <bool OWN_KEYS, int BL>
 struct LoopWalk {
   const unsigned long long* w = nullptr;
@@ -161,7 +170,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
   }
   // Tile ranges.  Own keys: heaviest (lowest) key tiles come first by construction; own queries: reversed so that
   // the heaviest (highest) query tiles start first.
-  int own0, loop_begin, n_tiles;
+  int own0, loop_begin, n_tiles, n_end = L;
   if constexpr (OWN_KEYS) {
     own0 = blockIdx.x * OWN;
     loop_begin = causal ? own0 : 0;
@@ -170,7 +179,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
   } else {
     own0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * OWN;
     loop_begin = 0;
-    int n_end = n_valid;
+    n_end = n_valid;
     if (causal) n_end = min(n_end, own0 + OWN);
     n_tiles = (n_end + BL - 1) / BL;
   }
@@ -216,7 +225,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
     mbar_init(own_full, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(loop_full + s, OWN_KEYS ? 2 : 1);  // TMA bytes (+ the row statistics, own keys)
-      mbar_init(loop_empty + s, OWN_KEYS ? 2 : 1);  // own keys: both issuing threads read the stage
+      mbar_init(loop_empty + s, C::NY == 0 ? 2 : 1);  // one ring: both issuing threads read the stage
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(s_full + s, 2);  // one commit per issuing thread
@@ -261,15 +270,16 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
       if (s == 3) return HAS_GO ? &maps.go : nullptr;
       if (!HAS_GT) return nullptr;
       return s == 1 ? &maps.tq : &maps.g;
-    } else {  // K, tK
+    } else {  // K, tK; without tangents K, V
       if (s == 0) return &maps.k;
+      if (s == 2) return HAS_GT ? nullptr : &maps.v;
       return (s == 1 && HAS_GT) ? &maps.tk : nullptr;
     }
   };
   auto y_map = [&](int s) -> const CUtensorMap* {  // own queries: V, tV
-    if (OWN_KEYS) return nullptr;
+    if (C::NY == 0) return nullptr;
     if (s == 0) return &maps.v;
-    return (s == 1 && HAS_GT) ? &maps.tv : nullptr;
+    return s == 1 ? &maps.tv : nullptr;
   };
 
   if (warp == 0) {
@@ -282,7 +292,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
           const CUtensorMap* m = own_map(s);
           if (m == nullptr) continue;
           for (int hf = 0; hf < 2; ++hf)
-            tma_load_4d(sOwn + s * C::OWN_BYTES + hf * C::OWN_HALF, m, own_full, hf * 64, own0, tma_h, tma_b);
+            tma_load_4d(sOwn + C::slot(s) * C::OWN_BYTES + hf * C::OWN_HALF, m, own_full, hf * 64, own0, tma_h, tma_b);
         }
       }
       auto walk = walk0;
@@ -295,11 +305,11 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
           unsigned char* base = sX + st * C::X_STAGE;
           mbar_expect_tx(loop_full + st, C::N_X * 2 * C::LQ_BYTES);
 #pragma unroll
-          for (int s = 0; s < C::NX; ++s) {
+          for (int s = 0; s < 4; ++s) {
             const CUtensorMap* m = x_map(s);
             if (m == nullptr) continue;
             for (int hf = 0; hf < 2; ++hf)
-              tma_load_4d(base + hf * C::X_HALF + s * C::LQ_BYTES, m, loop_full + st, hf * 64, l0, tma_h, tma_b);
+              tma_load_4d(base + hf * C::X_HALF + C::slot(s) * C::LQ_BYTES, m, loop_full + st, hf * 64, l0, tma_h, tma_b);
           }
         }
         if constexpr (C::NY > 0) {
@@ -319,8 +329,9 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
         if constexpr (OWN_KEYS) {
           // per-query statistics of this tile, combined once for all 128 key rows; fetched after the tile
           // loads have been issued, so that the two latencies overlap
-          {
-            const int i = l0 + lane;
+#pragma unroll
+          for (int k = lane; k < BL; k += 32) {
+            const int i = l0 + k;
             float4 s4 = make_float4(INFINITY, 0.f, 0.f, 0.f);
             if (i < L) {
               s4.x = a.lse[stat_off + i];
@@ -331,7 +342,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
                 s4.w += a.cterm[stat_off + i] + s4.z * s4.y;
               }
             }
-            sStat[st * BL + lane] = s4;
+            sStat[st * BL + k] = s4;
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(loop_full + st);  // second arrival: the statistics are in place
@@ -389,16 +400,16 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
       // X stage (own keys) or slots 0, 1 of ring Y (own queries)
       auto issue_e = [&](int t) -> bool {
         uint32_t l2;
-        if constexpr (OWN_KEYS) {
+        if constexpr (C::NY == 0) {
           const int st = t % STAGES;
           if (!mbar_wait_warp(loop_full + st, (t / STAGES) & 1, ab, kAbortBwdLoopFull)) return false;
-          l2 = (kDescLo | (smem_u32(sX + st * C::X_STAGE) >> 4)) + ((2 * C::LQ_BYTES) >> 4);
+          l2 = (kDescLo | (smem_u32(sX + st * C::X_STAGE) >> 4)) + ((C::slot(2) * C::LQ_BYTES) >> 4);
         } else {
           if (!mbar_wait_warp(y_full, t & 1, ab, kAbortBwdLoopFull)) return false;
           l2 = kDescLo | (smem_u32(sY) >> 4);
         }
         tc_fence_after();
-        constexpr uint32_t h2 = OWN_KEYS ? C::X_HALF : C::Y_HALF;
+        constexpr uint32_t h2 = C::NY == 0 ? C::X_HALF : C::Y_HALF;
         const uint32_t sc = tmem + (t & 1) * C::SC_COLS;
         if (elect_one()) {
           if constexpr (HAS_GT) {
@@ -414,14 +425,13 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
                 umma_ss_lo<true>(sc + C::COL_FP, a_lo0 + a_off(3, ks), l2 + b_off(h2, 0, ks), idesc_n1);
             }
           } else {
-            // FP = V gO^T (own keys: own2 loop3^T) or gO V^T (own queries: own3 loop2^T)
-            constexpr int fa = OWN_KEYS ? 2 : 3, fb = OWN_KEYS ? 1 : 0;
-            umma_ss_lo<false>(sc + C::COL_FP, a_lo0 + a_off(fa, 0), l2 + b_off(h2, fb, 0), idesc_n1);
+            // FP = V gO^T or gO V^T: the second tile of either side
+            umma_ss_lo<false>(sc + C::COL_FP, a_lo0 + a_off(1, 0), l2 + b_off(h2, 0, 0), idesc_n1);
 #pragma unroll
             for (int ks = 1; ks < 8; ++ks)
-              umma_ss_lo<true>(sc + C::COL_FP, a_lo0 + a_off(fa, ks), l2 + b_off(h2, fb, ks), idesc_n1);
+              umma_ss_lo<true>(sc + C::COL_FP, a_lo0 + a_off(1, ks), l2 + b_off(h2, 0, ks), idesc_n1);
           }
-          if constexpr (OWN_KEYS) tc_commit(loop_empty + (t % STAGES)); else tc_commit(y_empty);
+          if constexpr (C::NY == 0) tc_commit(loop_empty + (t % STAGES)); else tc_commit(y_empty);
           tc_commit(s_full + (t & 1));
         }
         return true;
@@ -435,8 +445,19 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
         }
       } else {
         if (ok) ok = issue_s(0);
+        auto walk = walk0;
         for (int t = 0; ok && t < n_tiles; ++t) {
           if (t + 1 < n_tiles && !issue_s(t + 1)) break;
+          // Own queries, wide tiles: the 16-key pieces that hold a key in range and in a live 64-key tile.  What K and V hold in others
+          // reaches no row.
+          uint32_t pieces = ~0u;
+          if constexpr (!OWN_KEYS && !HAS_GT) {
+            const int l0 = MK == 3 ? walk.next() * BL : t * BL;
+            pieces = 0u;
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+              if (l0 + 16 * p < n_end && (MK != 3 || walk.bit((l0 + 16 * p) >> 6))) pieces |= 1u << p;
+          }
           if (!mbar_wait_warp(p_full + (t & 1), (t >> 1) & 1, ab, kAbortBwdPFull)) break;
           tc_fence_after();
           const int st = t % STAGES;
@@ -447,10 +468,18 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
             // Contraction step kk = NP * term + piece: rows 16 * piece .. of X tile (slot + term), operand piece at
             // column 16 * piece + 8 * term of the accumulator it was written over.
             // dK or dQ += gS x0 + gtS x1
-            umma_ts_lo_dyn(tmem + C::COL_OUT0, sc + C::COL_S, mx, idesc_out, acc);
+            if constexpr (!OWN_KEYS && !HAS_GT) {
+              const uint32_t first = pieces & (0u - pieces);
 #pragma unroll
-            for (int kk = 1; kk < (HAS_GT ? 2 : 1) * NP; ++kk)
-              umma_ts_lo<true>(tmem + C::COL_OUT0, sc + C::COL_S + 16 * (kk % NP) + 8 * (kk / NP), mx + kk * 128, idesc_out);
+              for (int kk = 0; kk < NP; ++kk)
+                if ((pieces >> kk) & 1u)
+                  umma_ts_lo_dyn(tmem + C::COL_OUT0, sc + C::COL_S + 16 * kk, mx + kk * 128, idesc_out, first == 1u << kk ? acc : 1u);
+            } else {
+              umma_ts_lo_dyn(tmem + C::COL_OUT0, sc + C::COL_S, mx, idesc_out, acc);
+#pragma unroll
+              for (int kk = 1; kk < (HAS_GT ? 2 : 1) * NP; ++kk)
+                umma_ts_lo<true>(tmem + C::COL_OUT0, sc + C::COL_S + 16 * (kk % NP) + 8 * (kk / NP), mx + kk * 128, idesc_out);
+            }
             if constexpr (OWN_KEYS) {
               if constexpr (HAS_GT) {
                 // dV += A G + P gO   (X slots 2, 3)
@@ -460,12 +489,12 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
                 for (int kk = 1; kk < (HAS_GO ? 2 : 1) * NP; ++kk)
                   umma_ts_lo<true>(tmem + C::COL_OUT1, sc + C::COL_TS + 16 * (kk % NP) + 8 * (kk / NP), mx + o2 + kk * 128, idesc_out);
               } else {
-                // dV += P gO   (X slot 3)
-                constexpr uint32_t o3 = (3 * C::LQ_BYTES) >> 4;
-                umma_ts_lo_dyn(tmem + C::COL_OUT1, sc + C::COL_TS + 8, mx + o3, idesc_out, acc);
+                // dV += P gO
+                constexpr uint32_t o3 = (C::slot(3) * C::LQ_BYTES) >> 4;
+                umma_ts_lo_dyn(tmem + C::COL_OUT1, sc + C::COL_P, mx + o3, idesc_out, acc);
 #pragma unroll
                 for (int kk = 1; kk < NP; ++kk)
-                  umma_ts_lo<true>(tmem + C::COL_OUT1, sc + C::COL_TS + 16 * kk + 8, mx + o3 + kk * 128, idesc_out);
+                  umma_ts_lo<true>(tmem + C::COL_OUT1, sc + C::COL_P + 16 * kk, mx + o3 + kk * 128, idesc_out);
               }
             }
             tc_commit(loop_empty + st);
@@ -630,7 +659,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
       tmem_st8(sc + C::COL_S, pk_gs);
       if constexpr (HAS_GT) tmem_st8(sc + C::COL_S + 8, pk_gt);
       if constexpr (HAS_GT && OWN_KEYS) tmem_st8(sc + C::COL_TS, pk_av);
-      if constexpr (OWN_KEYS && (HAS_GO || !HAS_GT)) tmem_st8(sc + C::COL_TS + 8, pk_p);
+      if constexpr (OWN_KEYS && (HAS_GO || !HAS_GT)) tmem_st8(sc + C::COL_P, pk_p);
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(p_full + (t & 1));
