@@ -469,6 +469,11 @@ __device__ __forceinline__ bool cut_shares(const int2* begin, int ctas, int j, i
 }
 
 // ---- TMA -----------------------------------------------------------------------------------
+// Into L2 alone.
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int x, int y, int z, int w) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(x), "r"(y), "r"(z), "r"(w)
+               : "memory");
+}
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y,
                                             int z, int w) {
   asm volatile(
