@@ -174,38 +174,54 @@ __global__ void __launch_bounds__(256, 4) mask_pack_kernel(const jvpfa_mask m, i
       }
     }
   } else {
-    // Rows that begin anywhere: three aligned words hold eight bytes of a row, where all that a lane reads lies inside the mask.  Else
-    // byte by byte, in order of columns, so that all rows are in flight at once.  (From DRAM, us, row after row and byte after byte / so:
-    // 77 heads of L66 22 / 12, 43 of L130 27 / 12, 24 of L1330 57 / 35, of L2046 91 / 60.)
+    // Rows that begin anywhere: three aligned words hold eight bytes of a row.  Where one of them would reach out of the mask, in its first
+    // or last rows, the row's bytes are read one by one.  (All rows of such a lane were, one column after the other, and a launch takes as long
+    // as its slowest warp.  From DRAM, us, before / so: 16 heads of L58 25 / 7, 77 of L66 11 / 7, 15 of L154 33 / 8, 43 of L130 11 / 8, 63 of
+    // L338 21 / 9, 24 of L1330 31 / 21, of L2046 51 / 36, one of L4098 13 / 10.)
+    // Where keys lie apart, or strides run backwards, byte by byte, in order of columns, so that all rows are in flight at once.
     const int n = min(8, L - col);  // <= 0: beyond the end
     const int rows = min(32, n_rows - row0);
     const unsigned char* first = reinterpret_cast<const unsigned char*>(m.ptr);
     const unsigned char* end = first + (long long)(gridDim.z / n_h - 1) * m.stride[0] + (long long)(n_h - 1) * m.stride[1] +
                                (long long)(n_rows - 1) * rs + (long long)(L - 1) * ks + 1;
-    const bool words = ks == 1 && rs >= 0 && m.stride[0] >= 0 && m.stride[1] >= 0 && n > 0 && rows > 0 &&
-                       p0 - (reinterpret_cast<uintptr_t>(p0) & 3u) >= first && p0 + (long long)(rows - 1) * rs + 12 <= end;
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = 0u;
-    if (words) {
-      const uint32_t cols = (1u << n) - 1u;
+    if (ks == 1 && rs >= 0 && m.stride[0] >= 0 && m.stride[1] >= 0) {
+      int r0 = 0, r1 = n > 0 ? max(rows, 0) : 0;  // rows [r0, r1): all of their words lie inside the mask
+      const int r_end = r1;
+      while (r1 > 0 && p0 + (long long)(r1 - 1) * rs + 12 > end) --r1;
+      while (r0 < r1 && p0 + (long long)r0 * rs < first + 3) ++r0;
+      const uint32_t cols = n > 0 ? (1u << n) - 1u : 0u;
+      if (r0 < r1) {
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        uint32_t v[8][3], shift[8];
+        for (int j = 0; j < 8; j += 2) {
+          uint32_t v[8][3], shift[8];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          const unsigned char* p = p0 + (long long)(4 * j + r) * rs;
-          shift[r] = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3u);
+          for (int r = 0; r < 8; ++r) {
+            const unsigned char* p = p0 + (long long)(4 * j + r) * rs;
+            shift[r] = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3u);
 #pragma unroll
-          for (int w = 0; w < 3; ++w) {
-            v[r][w] = 0u;
-            if (4 * j + r < rows) v[r][w] = __ldg(reinterpret_cast<const uint32_t*>(p - shift[r]) + w);
+            for (int w = 0; w < 3; ++w) {
+              v[r][w] = 0u;
+              if (4 * j + r >= r0 && 4 * j + r < r1) v[r][w] = __ldg(reinterpret_cast<const uint32_t*>(p - shift[r]) + w);
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            const uint32_t lo = __funnelshift_r(v[r][0], v[r][1], 8 * shift[r]), hi = __funnelshift_r(v[r][1], v[r][2], 8 * shift[r]);
+            x[j + (r >> 2)] |= ((nonzero_bits(lo) | nonzero_bits(hi) << 4) & cols) << (8 * (r & 3));
           }
         }
+      }
+      for (int r = r0 > 0 ? 0 : r1; r < r_end; r = r + 1 == r0 ? r1 : r + 1) {
+        uint32_t byte[8], set = 0u;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          const uint32_t lo = __funnelshift_r(v[r][0], v[r][1], 8 * shift[r]), hi = __funnelshift_r(v[r][1], v[r][2], 8 * shift[r]);
-          x[j + (r >> 2)] |= ((nonzero_bits(lo) | nonzero_bits(hi) << 4) & cols) << (8 * (r & 3));
-        }
+        for (int c = 0; c < 8; ++c) byte[c] = c < n ? __ldg(p0 + (long long)r * rs + c) : 0u;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) set |= (byte[c] != 0u ? 1u : 0u) << c;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (r >> 2 == j) x[j] |= set << (8 * (r & 3));
       }
     } else {
       for (int c = 0; c < n; ++c) {
