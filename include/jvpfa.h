@@ -340,6 +340,22 @@ typedef struct {
 
 int jvpfa_mask_tiles(const jvpfa_mask_tiles_args* args, void* stream);
 
+/*
+ * jvpfa_pad_bias -- a bias of 16-bit elements with its rows padded, to whole 16-byte pieces as the tensor-core kernels take one.
+ * No upstream counterpart.
+ *
+ * The bias (kind BIAS, bias_dtype bf16 or fp16) may have any layout; n_b, n_h are its own extents (1 where it broadcasts), its rows L.
+ *   out   n_b*n_h * L * width elements, width a multiple of 8 and at least L: the entries, and zeros behind a row's end.  16-byte aligned.
+ */
+typedef struct {
+  int32_t struct_size; /* sizeof(jvpfa_pad_bias_args) */
+  int32_t n_b, n_h, L, width;
+  jvpfa_mask mask;
+  void* out;
+} jvpfa_pad_bias_args;
+
+int jvpfa_pad_bias(const jvpfa_pad_bias_args* args, void* stream);
+
 /* Human-readable text for a jvpfa_status (static storage, never NULL). */
 const char* jvpfa_strerror(int status);
 

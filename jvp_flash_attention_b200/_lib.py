@@ -52,6 +52,7 @@ EXPORTS = (
     "jvpfa_bwd_noalloc",
     "jvpfa_mask_check",
     "jvpfa_mask_tiles",
+    "jvpfa_pad_bias",
 )
 
 NOALLOC_MAX_ROWS = 524288  # JVPFA_NOALLOC_MAX_ROWS
@@ -214,6 +215,18 @@ class MaskTilesArgs(C.Structure):
     ]
 
 
+class PadBiasArgs(C.Structure):
+    _fields_ = [
+        ("struct_size", C.c_int32),
+        ("n_b", C.c_int32),
+        ("n_h", C.c_int32),
+        ("L", C.c_int32),
+        ("width", C.c_int32),
+        ("mask", Mask),
+        ("out", C.c_void_p),
+    ]
+
+
 _lib = None
 
 
@@ -258,6 +271,8 @@ def load() -> C.CDLL:
     lib.jvpfa_mask_check.restype = C.c_int
     lib.jvpfa_mask_tiles.argtypes = [C.POINTER(MaskTilesArgs), C.c_void_p]
     lib.jvpfa_mask_tiles.restype = C.c_int
+    lib.jvpfa_pad_bias.argtypes = [C.POINTER(PadBiasArgs), C.c_void_p]
+    lib.jvpfa_pad_bias.restype = C.c_int
     _lib = lib
     return lib
 

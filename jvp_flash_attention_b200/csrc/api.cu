@@ -314,6 +314,19 @@ int jvpfa_mask_tiles(const jvpfa_mask_tiles_args* args, void* stream) {
   return launch_mask_tiles(*a, static_cast<cudaStream_t>(stream));
 }
 
+int jvpfa_pad_bias(const jvpfa_pad_bias_args* a, void* stream) {
+  if (!a) return JVPFA_ERR_NULL;
+  if (a->struct_size != (int32_t)sizeof(jvpfa_pad_bias_args)) return JVPFA_ERR_STRUCT;
+  if (a->n_b < 1 || a->n_h < 1 || a->L < 1 || a->width < a->L || (a->width & 7) != 0) return JVPFA_ERR_SHAPE;
+  if (!a->out) return JVPFA_ERR_NULL;
+  if (!aligned16(a->out)) return JVPFA_ERR_ALIGN;
+  if (a->mask.kind != JVPFA_MASK_BIAS || !a->mask.ptr) return JVPFA_ERR_MASK;
+  if (a->mask.bias_dtype != JVPFA_BF16 && a->mask.bias_dtype != JVPFA_FP16) return JVPFA_ERR_DTYPE;
+  const int rc = check_arch();
+  if (rc) return rc;
+  return launch_pad_bias(*a, static_cast<cudaStream_t>(stream));
+}
+
 int jvpfa_device_status(int* status, int clear) {
   if (!status) return JVPFA_ERR_NULL;
   return tc5_read_status(status, clear);

@@ -533,6 +533,7 @@ int launch_pre(const jvpfa_pre_args& a, cudaStream_t stream);
 int launch_bwd_generic(const jvpfa_bwd_args& a, cudaStream_t stream);
 int launch_mask_check(const jvpfa_mask_check_args& a, cudaStream_t stream);
 int launch_mask_tiles(const jvpfa_mask_tiles_args& a, cudaStream_t stream);
+int launch_pad_bias(const jvpfa_pad_bias_args& a, cudaStream_t stream);
 int launch_fwd_tc5(const jvpfa_fwd_args& a, cudaStream_t stream);
 bool fwd_tc5_eligible(const jvpfa_fwd_args& a);
 bool tc5_head_dim(int D, int L);

@@ -303,7 +303,56 @@ __global__ void __launch_bounds__(256, 4) mask_pack_kernel(const jvpfa_mask m, i
   }
 }
 
+// One warp for a row, eight elements (16 bytes stored) a lane at a time.  HBM bound: reads and writes two bytes an element.  Rows begin at any
+// multiple of an element; pairs of them are one load where all rows begin at a multiple of two (an even length).  The generic strided copy
+// that it stands for looks each element's place up by itself: B2 H3 L3698 (82 million
+// elements) on a B200 182 -> 56 us, B2 H11 L1450 102 -> 29.
+constexpr int kPadUnroll = 4;
+__global__ void __launch_bounds__(256) pad_bias_kernel(const jvpfa_mask m, int n_h, int L, int width, long long n_rows, uint16_t* out, bool pairs) {
+  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= n_rows) return;
+  const long long head = row / L;
+  const int i = (int)(row - head * L), b = (int)(head / n_h), h = (int)(head - (long long)b * n_h);
+  const long long ks = m.stride[3];
+  const uint16_t* src = reinterpret_cast<const uint16_t*>(m.ptr) + b * m.stride[0] + h * m.stride[1] + i * m.stride[2];
+  uint16_t* dst = out + row * width;
+  for (int p0 = (threadIdx.x & 31) * 8; p0 < width; p0 += 256 * kPadUnroll) {
+    uint32_t w[kPadUnroll][4];
+#pragma unroll
+    for (int u = 0; u < kPadUnroll; ++u) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int j = p0 + 256 * u + 2 * e;
+        w[u][e] = 0u;
+        if (pairs && j + 1 < L) {
+          w[u][e] = __ldg(reinterpret_cast<const uint32_t*>(src + j));
+        } else {
+          if (j < L) w[u][e] = __ldg(src + j * ks);
+          if (j + 1 < L) w[u][e] |= (uint32_t)__ldg(src + (j + 1) * ks) << 16;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kPadUnroll; ++u)
+      if (p0 + 256 * u < width) *reinterpret_cast<uint4*>(dst + p0 + 256 * u) = make_uint4(w[u][0], w[u][1], w[u][2], w[u][3]);
+  }
+}
+
 }  // namespace
+
+int launch_pad_bias(const jvpfa_pad_bias_args& a, cudaStream_t stream) {
+  const long long n_rows = (long long)a.n_b * a.n_h * a.L, blocks = (n_rows + 7) / 8;
+  if (blocks > 0x7fffffffLL) return JVPFA_ERR_TOO_LARGE;
+  bool pairs = a.mask.stride[3] == 1 && (reinterpret_cast<uintptr_t>(a.mask.ptr) & 3u) == 0;
+  for (int d = 0; d < 3; ++d) pairs = pairs && (a.mask.stride[d] & 1) == 0;
+  pad_bias_kernel<<<(unsigned)blocks, 256, 0, stream>>>(a.mask, a.n_h, a.L, a.width, n_rows, static_cast<uint16_t*>(a.out), pairs);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_last_cuda_error(e, "launch pad_bias");
+    return JVPFA_ERR_CUDA;
+  }
+  return JVPFA_OK;
+}
 
 int launch_mask_tiles(const jvpfa_mask_tiles_args& a, cudaStream_t stream) {
   const int n_kt = (a.L + 63) / 64;

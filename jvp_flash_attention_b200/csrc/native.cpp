@@ -207,19 +207,19 @@ Tensor padded_bias(const MaskDesc& m, const Tensor& q) {
   if (m.c.kind != JVPFA_MASK_BIAS || !takes_16_bit_forms(q) || m.tensor.scalar_type() != q.scalar_type() || m.c.stride[2] == 0) return {};
   const int64_t L = q.size(2), step = 16 / m.tensor.element_size();
   if (L <= 64 || L % step == 0) return {};
-  NoFunctorch nf;
-  at::AutoDispatchBelowADInplaceOrView below;
-  Tensor own = m.tensor;
-  for (int d = 0; d < 2; ++d)
-    if (m.c.stride[d] == 0) own = own.narrow(d, 0, 1);
+  const int64_t n_b = m.c.stride[0] ? m.tensor.size(0) : 1, n_h = m.c.stride[1] ? m.tensor.size(1) : 1;
   Tensor padded;
   try {
-    padded = empty({own.size(0), own.size(1), L, (L + step - 1) / step * step}, own.scalar_type(), own.device());
+    padded = empty({n_b, n_h, L, (L + step - 1) / step * step}, m.tensor.scalar_type(), m.tensor.device());
   } catch (const c10::OutOfMemoryError&) {
     return {};
   }
-  padded = padded.narrow(3, 0, L);
-  padded.copy_(own);
+  jvpfa_pad_bias_args a{};
+  a.struct_size = sizeof(a);
+  a.n_b = (int)n_b, a.n_h = (int)n_h, a.L = (int)L, a.width = (int)padded.size(3);
+  a.mask = m.c;
+  a.out = padded.data_ptr();
+  check_status(jvpfa_pad_bias(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "jvpfa_pad_bias");
   return padded;
 }
 
