@@ -9,10 +9,10 @@ from jvp_flash_attention_b200 import _lib
 DEV = "cuda:0"
 
 
-def _args(m, out, **fields):
+def _args(m, padded, **fields):
     spec = _lib.MaskSpec(_lib.MASK_BIAS, m, tuple(0 if n == 1 else s for n, s in zip(m.shape, m.stride())), _lib.DTYPE_ENUM[m.dtype])
-    a = _lib.PadBiasArgs(struct_size=ctypes.sizeof(_lib.PadBiasArgs), n_b=m.shape[0], n_h=m.shape[1], L=m.shape[2], width=out.shape[3], mask=spec.to_c(),
-                         out=out.data_ptr())
+    a = _lib.PadBiasArgs(struct_size=ctypes.sizeof(_lib.PadBiasArgs), n_b=m.shape[0], n_h=m.shape[1], L=m.shape[2], width=padded.shape[3], mask=spec.to_c(),
+                         out=padded.data_ptr())
     a.mask.stride[3] = m.stride(3)
     for name, value in fields.items():
         setattr(a, name, value)
