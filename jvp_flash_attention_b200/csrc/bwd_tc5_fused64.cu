@@ -693,14 +693,23 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           next_live = l0 < L ? ldg_nc_u32(bcol + (a.mask.stride[2] ? l0 >> 5 : 0)) : 0u;
         } else if constexpr (MK == 2) {
           const long long step = a.mask.stride[2] * 2;  // to the next query; the last one's elements stand for those beyond
-          const int q0 = l0 + 16 * (lane & 1);          // (L is a multiple of 16 and so is q0: the 16 queries are all there or none is)
+          const int q0 = l0 + 16 * (lane & 1);
+          // (the last pair of an odd length ends in its row's padding)
           const unsigned char* el = reinterpret_cast<const unsigned char*>(a.mask.ptr) +
-                                    ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] + min(own_idx - (lane & 1), L - 2)) * 2 +
-                                    min(q0, L - 16) * step;
+                                    ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] + min(own_idx - (lane & 1), (L - 1) & ~1)) * 2 +
+                                    min(q0, L - 1) * step;
+          if (q0 + 16 <= L) {
 #pragma unroll
-          for (int x = 0; x < 16; ++x) {
-            braw[x] = ldg_nc_u32(el);
-            el += step;
+            for (int x = 0; x < 16; ++x) {
+              braw[x] = ldg_nc_u32(el);
+              el += step;
+            }
+          } else {
+#pragma unroll
+            for (int x = 0; x < 16; ++x) {
+              braw[x] = ldg_nc_u32(el);
+              if (q0 + x + 1 < L) el += step;
+            }
           }
         } else if constexpr (MK == 1) {
           const long long step = a.mask.stride[2];
@@ -1016,7 +1025,8 @@ static int fused_sm_count() {
 static long long bwd_bias_workspace(const jvpfa_bwd_args& a) {
   if ((a.dtype != JVPFA_BF16 && a.dtype != JVPFA_FP16) || a.impl == JVPFA_IMPL_GENERIC || a.D != 64) return 0;
   if (a.mask.kind != JVPFA_MASK_BIAS || a.gto == nullptr || (a.flags & JVPFA_SKIP_DKDV)) return 0;
-  if ((a.L & 15) != 0 || !tc5_mask_layout(a.mask, a.dtype, a.L)) return 0;
+  // rows of whole 32-byte pieces, padded to them where the length does not fill them
+  if (((a.L & 15) != 0 && a.mask.stride[2] < ((a.L + 15) & ~15)) || !tc5_mask_layout(a.mask, a.dtype, a.L)) return 0;
   const long long key_tiles = (long long)((a.L + 127) / 128) * a.B * a.H;
   if (key_tiles < 96) return 0;
   const long long bytes = key_tiles * a.L * a.D * 4;

@@ -198,15 +198,15 @@ const int32_t* host_lengths(const MaskDesc& m, int B) { return m.kv_len.size() =
 // Whether the launches of a call may take the forms that only the 16-bit tensor-core kernels read.
 bool takes_16_bit_forms(const Tensor& q) { return q.is_cuda() && q.scalar_type() != at::kFloat && g_impl != JVPFA_IMPL_GENERIC; }
 
-// A ragged bias of the tensors' type with its rows padded to whole 16-byte pieces, the form in which the tensor-core kernels
-// take a bias (what lies beyond the row's end is not looked at); undefined for every other mask.  Up to one tile of keys a
+// A ragged bias of the tensors' type with its rows padded to whole 32-byte pieces: the tensor-core kernels take rows of whole 16-byte
+// pieces, the single-pass backward through tO of 32 (`single_pass`; what lies beyond the row's end is not looked at); undefined for every other mask.  Up to one tile of keys a
 // bias is read element by element, whatever its layout.  Dimensions that broadcast are not written out, and the copy lives
 // for one launch: layers that share a bias do not hold a copy each until their backward.  Where there is no memory for it the
 // bias is read in place, by the register-tiled kernels.
-Tensor padded_bias(const MaskDesc& m, const Tensor& q) {
+Tensor padded_bias(const MaskDesc& m, const Tensor& q, bool single_pass = false) {
   if (m.c.kind != JVPFA_MASK_BIAS || !takes_16_bit_forms(q) || m.tensor.scalar_type() != q.scalar_type() || m.c.stride[2] == 0) return {};
-  const int64_t L = q.size(2), step = 16 / m.tensor.element_size();
-  if (L <= 64 || L % step == 0) return {};
+  const int64_t L = q.size(2), step = 16;  // elements
+  if (L <= 64 || L % (single_pass ? step : 8) == 0) return {};
   const int64_t n_b = m.c.stride[0] ? m.tensor.size(0) : 1, n_h = m.c.stride[1] ? m.tensor.size(1) : 1;
   Tensor padded;
   try {
@@ -424,7 +424,8 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   if (!(skip & JVPFA_SKIP_DQ)) g[0] = empty(sizes, q.scalar_type(), q.device());
   if (!(skip & JVPFA_SKIP_DKDV))
     for (int i = 1; i < 3; ++i) g[i] = empty(sizes, q.scalar_type(), q.device());
-  const Tensor padded = padded_bias(m, q);
+  const bool one_pass = g_single_pass && gto.defined() && sizes[3] == 64 && !(skip & JVPFA_SKIP_DKDV) && (sizes[2] + 127) / 128 * sizes[0] * sizes[1] >= 96;
+  const Tensor padded = padded_bias(m, q, one_pass);
   jvpfa_bwd_args a{};
   a.struct_size = sizeof(a);
   a.dtype = p.dtype;
