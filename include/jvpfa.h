@@ -226,8 +226,9 @@ typedef struct {
 
 /* As jvpfa_fwd_workspace.  Non-zero for 16-bit types at D = 64 where the one pass (dq_accum) shares key tiles out among the SMs; for
  * JVPFA_FP32 through O, and for dQ alone (JVPFA_SKIP_DKDV) through tO with
- * JVPFA_ZERO_TKV; and for 16-bit types at D = 64 through tO with a BIAS of their type (key stride 1, 16-byte aligned rows,
- * L % 16 == 0), where the backward then is one pass, bitwise reproducible, that leaves a share of dQ for each 128 keys there.
+ * JVPFA_ZERO_TKV; and for 16-bit types at D = 64 through tO with a BIAS of their type (key stride 1, 16-byte aligned rows that have room for L
+ * rounded up to 16 elements), and at D = 32 (no KVLEN; BOOL with bits and without tile bitmaps; BIAS as before), where the backward then is one pass,
+ * bitwise reproducible, that leaves a share of dQ for each 128 keys there.
  * The fp32 ones recompute the scores as jvpfa_fwd with its workspace forms them, the other kernels as jvpfa_fwd without:
  * lse and mu fit the scores to the last bit when both calls of a pair are given a workspace, or neither. */
 int64_t jvpfa_bwd_workspace(const jvpfa_bwd_args* args);

@@ -3,7 +3,8 @@
 //   head dimension 64 : bwd_tc5_fused64.cu (one pass; needs a buffer for dQ; index masks, boolean masks
 //                       without tile bitmaps, bias) or bwd_tc5_d64.cu (two launches; every mask kind, steps
 //                       over dead tiles)
-//   head dimension 32 : bwd_tc5_d64.cu, on half-filled tiles
+//   head dimension 32 : on half-filled tiles, bwd_tc5_fused64.cu with a workspace for dQ's shares (not key padding, nor with
+//                       tile bitmaps), else bwd_tc5_d64.cu
 //   head dimension 128: bwd_tc5_pipe128.cu (two launches; every mask kind)
 #include "tc5_common.cuh"
 

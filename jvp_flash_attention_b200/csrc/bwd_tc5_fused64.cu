@@ -160,8 +160,14 @@ __device__ __forceinline__ int2 split_begin(const jvpfa_bwd_args& a, int c, int 
 // a buffer of its own (dq_acc: [key tile][B*H][L][D] floats) and fused64_finish_kernel adds them up.  Measured on a B200, the two
 // launches / this with the sum, us, bf16 through both outputs: B2 H12 L512 34 / 25, L1024 121 / 75, L2048 342 / 255, H4 L4096
 // 226 / 172; with 48 key tiles (B2 H12 L256) 22 / 28, with 32 (H1 L4096) 124 / 173, both before key tiles were shared out.
-template <bool HAS_GT, int MK>
-constexpr bool kDqParts = HAS_GT && MK == 2;
+//
+// At head dimension 32 it always is, whatever the mask and the cotangents (key padding and tile bitmaps keep the two launches): tensor maps end at
+// column 32, contractions over D stop half-way, and a key tile's share of dQ has half the bytes.  Two launches / this with the sum, us, bf16 through
+// O / tO / both: B4 H8 L1000 56 / 40, 70 / 54, 78 / 58; B1 H5 L4096 177 / 83, 225 / 112, 254 / 124; B5 H9 L1732 with a bias 649 / 318, 723 / 384,
+// 736 / 424; B4 H16 L2048 causal 173 / 137, 221 / 195, 249 / 222; B8 H12 L130 21 / 16, 24 / 20, 25 / 21; B1 H1 L1024 20 / 14, 24 / 17, 26 / 18.
+__host__ __device__ __forceinline__ bool dq_parts(const jvpfa_bwd_args& a) {
+  return a.D == 32 || (a.mask.kind == JVPFA_MASK_BIAS && a.gto != nullptr);
+}
 template <typename T, bool HAS_GO, bool HAS_GT, int MK, bool CUT>
 __global__ void __launch_bounds__(512, 1)
 bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps maps, float* dq_acc, float* shares, int* status) {
@@ -276,6 +282,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
     return n_valid;
   };
 
+  const bool parts = dq_parts(a);
   // NaN into the rows of dK, dV and of the dQ accumulator that this CTA's items own: this launch's results are
   // not to be trusted
   auto poison = [&]() {
@@ -284,9 +291,9 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       const int i = it.own0 + tid;
       if (tid < OWN && share(walk, 0)) share(walk, 0)[4 * tid] = share(walk, 1)[4 * tid] = poison_f32();
       if (tid < OWN && i < L) {
-        poison_row<T>(a.dk, (size_t)it.bh * L + i, D);
-        poison_row<T>(a.dv, (size_t)it.bh * L + i, D);
-        dq_acc[((kDqParts<HAS_GT, MK> ? (size_t)(it.own0 / OWN) * BH * L : 0) + (size_t)it.bh * L + i) * D] = poison_f32();
+        poison_row<T>(a.dk, (size_t)it.bh * L + i, a.D);
+        poison_row<T>(a.dv, (size_t)it.bh * L + i, a.D);
+        dq_acc[((parts ? (size_t)(it.own0 / OWN) * BH * L : 0) + (size_t)it.bh * L + i) * a.D] = poison_f32();
       }
     }
   };
@@ -471,7 +478,8 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             else
               umma_ss_lo<true>(tmem + col, a_lo, b_lo, id);
 #pragma unroll
-            for (int ks = 1; ks < D / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 2, id);
+            for (int ks = 1; ks < D / 16; ++ks)
+              if (ks < 2 || a.D > 32) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 2, id);
           };
           for (int walk = begin_items(); ok && get_item(walk, it); ++walk) {
             if (it.n_sub == 0) continue;
@@ -641,7 +649,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 
     auto store_row = [&](void* gptr, int bh, int own_idx, const uint32_t (&r0)[32], const uint32_t (&r1)[32], float mul) {
       if (own_idx >= L) return;
-      T* gp = reinterpret_cast<T*>(gptr) + ((size_t)bh * L + own_idx) * D;
+      T* gp = reinterpret_cast<T*>(gptr) + ((size_t)bh * L + own_idx) * a.D;
 #pragma unroll
       for (int x = 0; x < 4; ++x)
         reinterpret_cast<uint4*>(gp)[x] = make_uint4(
@@ -649,6 +657,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             Elem<T>::pack(__uint_as_float(r0[8 * x + 2]) * mul, __uint_as_float(r0[8 * x + 3]) * mul),
             Elem<T>::pack(__uint_as_float(r0[8 * x + 4]) * mul, __uint_as_float(r0[8 * x + 5]) * mul),
             Elem<T>::pack(__uint_as_float(r0[8 * x + 6]) * mul, __uint_as_float(r0[8 * x + 7]) * mul));
+      if (a.D == 32) return;
 #pragma unroll
       for (int x = 0; x < 4; ++x)
         reinterpret_cast<uint4*>(gp)[4 + x] = make_uint4(
@@ -917,16 +926,16 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             sts_v4(rowa + (((uint32_t)c ^ sw) << 4), r0[4 * c], r0[4 * c + 1], r0[4 * c + 2], r0[4 * c + 3]);
-            sts_v4(rowa + 8192 + (((uint32_t)c ^ sw) << 4), r1[4 * c], r1[4 * c + 1], r1[4 * c + 2], r1[4 * c + 3]);
+            if (a.D > 32) sts_v4(rowa + 8192 + (((uint32_t)c ^ sw) << 4), r1[4 * c], r1[4 * c + 1], r1[4 * c + 2], r1[4 * c + 3]);
           }
         }
         fence_async_smem();
         rb_meet();
         if (tid == 384) {
           const int i0 = it.loop_begin + s * BL;
-          if constexpr (kDqParts<HAS_GT, MK>) {
+          if (parts) {
             tma_store_part_4d(&maps.dq, dqs, 0, i0, it.bh, it.own0 / OWN);
-            tma_store_part_4d(&maps.dq, dqs + 8192, 32, i0, it.bh, it.own0 / OWN);
+            if (a.D > 32) tma_store_part_4d(&maps.dq, dqs + 8192, 32, i0, it.bh, it.own0 / OWN);
           } else {
             tma_reduce_add_4d(&maps.dq, dqs, 0, i0, it.h, it.b);
             tma_reduce_add_4d(&maps.dq, dqs + 8192, 32, i0, it.h, it.b);
@@ -972,8 +981,9 @@ __device__ __forceinline__ void sum_shares(const jvpfa_bwd_args& a, const float*
     return;
   const int per_head = (a.L + 127) / 128, bh = item / per_head, key = (item - bh * per_head) * 128 + row;
   if (key >= a.L) return;
+  if (4 * piece >= a.D) return;
   const float mul = which ? 1.f : a.sm_scale;
-  T* out = reinterpret_cast<T*>(which ? a.dv : a.dk) + ((size_t)bh * a.L + key) * 64 + piece * 4;
+  T* out = reinterpret_cast<T*>(which ? a.dv : a.dk) + ((size_t)bh * a.L + key) * a.D + piece * 4;
   *reinterpret_cast<uint4*>(out) = make_uint4(Elem<T>::pack(lo.x * mul, lo.y * mul), Elem<T>::pack(lo.z * mul, lo.w * mul),
                                               Elem<T>::pack(hi.x * mul, hi.y * mul), Elem<T>::pack(hi.z * mul, hi.w * mul));
 }
@@ -999,6 +1009,8 @@ fused64_finish_kernel(const jvpfa_bwd_args a, const float* acc, long long n, int
   const long long n4 = n / 4;
   if (i >= n4) return;
   const float4* p = reinterpret_cast<const float4*>(acc) + i;
+  // (causal: a query has a share of the key tiles up to its own)
+  if (a.mask.kind == JVPFA_MASK_CAUSAL) n_parts = min(n_parts, (int)(4 * i / a.D % a.L) / 128 + 1);
   float4 s = __ldcs(p);
 #pragma unroll 8
   for (int k = 1; k < n_parts; ++k) {
@@ -1020,17 +1032,26 @@ static int fused_sm_count() {
   return cache[dev];
 }
 
-// Floats for a key tile's share of dQ, of every key tile: as many bytes as the (B, H, L, L) bias itself has, up to half a GiB.
-// From 96 key tiles on: with fewer the two launches, of as many CTAs each, fill more of the 148 SMs.
-static long long bwd_bias_workspace(const jvpfa_bwd_args& a) {
-  if ((a.dtype != JVPFA_BF16 && a.dtype != JVPFA_FP16) || a.impl == JVPFA_IMPL_GENERIC || a.D != 64) return 0;
-  if (a.mask.kind != JVPFA_MASK_BIAS || a.gto == nullptr || (a.flags & JVPFA_SKIP_DKDV)) return 0;
-  // rows of whole 32-byte pieces, padded to them where the length does not fill them
-  if (((a.L & 15) != 0 && a.mask.stride[2] < ((a.L + 15) & ~15)) || !tc5_mask_layout(a.mask, a.dtype, a.L)) return 0;
+// Floats for a key tile's share of dQ, of every key tile: as many bytes as the (B, H, L, L) bias itself has, up to half a GiB; at
+// head dimension 32 half as many, up to a quarter.  From 96 key tiles on: with fewer the two launches, of as many CTAs each, fill more of the 148 SMs.
+// At head dimension 32, where key tiles are shared out, that only holds for short ones: both launches fit the SMs at once up to 74 tiles (through both,
+// B2 H8 L512, 64 tiles: 18.8 / 21.2 us; B2 H10 L512, 80 tiles: 27.4 / 21.9; from L1024 on B1 H8 28 / 26 and fewer heads more), causal ones, of half the
+// work, up to twice as many (B2 H12 L512 19.1 / 22.4, B1 H14 L778 23.9 / 24.9; B2 H17 L512, 136 tiles, 23.5 / 23.1; B2 H20 L512 26.2 / 23.7).
+static long long bwd_parts_workspace(const jvpfa_bwd_args& a) {
+  if ((a.dtype != JVPFA_BF16 && a.dtype != JVPFA_FP16) || a.impl == JVPFA_IMPL_GENERIC || (a.flags & JVPFA_SKIP_DKDV)) return 0;
+  if (a.D > 64 || !tc5_head_dim(a.D, a.L) || !dq_parts(a)) return 0;
+  if (a.mask.kind == JVPFA_MASK_BIAS) {
+    // rows of whole 32-byte pieces, padded to them where the length does not fill them
+    if (((a.L & 15) != 0 && a.mask.stride[2] < ((a.L + 15) & ~15)) || !tc5_mask_layout(a.mask, a.dtype, a.L)) return 0;
+  } else if (a.mask.kind == JVPFA_MASK_BOOL) {
+    if (a.mask_tile_live != nullptr || a.mask_tile_live_t != nullptr || a.mask_bits_t == nullptr) return 0;
+  } else if (a.mask.kind == JVPFA_MASK_KVLEN) {
+    return 0;  // (the sum would have to know which key tiles are all padding)
+  }
   const long long key_tiles = (long long)((a.L + 127) / 128) * a.B * a.H;
-  if (key_tiles < 96) return 0;
+  if (a.D == 32 ? a.L < 1024 && key_tiles < (a.mask.kind == JVPFA_MASK_CAUSAL ? 144 : 75) : key_tiles < 96) return 0;
   const long long bytes = key_tiles * a.L * a.D * 4;
-  return bytes <= (1ll << 29) ? bytes : 0;
+  return bytes <= (a.D == 32 ? 1ll << 28 : 1ll << 29) ? bytes : 0;
 }
 
 // CTAs among which the key tiles' sub-tiles are shared out; 0: the key tiles are dealt whole.  Both in sub-tiles of the CTA that has
@@ -1088,19 +1109,19 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
   BwdFMaps m;
   const CUtensorMapDataType dt = Fmt<T>::kTma;
   const int64_t* st = a.in_stride;
-  bool ok = encode_map4d(&m.k, dt, a.k, C::D, a.L, a.H, a.B, st, C::OWN) && encode_map4d(&m.v, dt, a.v, C::D, a.L, a.H, a.B, st, C::OWN) &&
-            encode_map4d(&m.q, dt, a.q, C::D, a.L, a.H, a.B, st, C::BL);
+  bool ok = encode_map4d(&m.k, dt, a.k, a.D, a.L, a.H, a.B, st, C::OWN) && encode_map4d(&m.v, dt, a.v, a.D, a.L, a.H, a.B, st, C::OWN) &&
+            encode_map4d(&m.q, dt, a.q, a.D, a.L, a.H, a.B, st, C::BL);
   m.tk = m.tv = m.k;
   m.go = m.tq = m.g = m.q;
-  if (HAS_GO) ok = ok && encode_map4d(&m.go, dt, a.go, C::D, a.L, a.H, a.B, nullptr, C::BL);
+  if (HAS_GO) ok = ok && encode_map4d(&m.go, dt, a.go, a.D, a.L, a.H, a.B, nullptr, C::BL);
   if (HAS_GT)
-    ok = ok && encode_map4d(&m.tk, dt, a.tk, C::D, a.L, a.H, a.B, st, C::OWN) && encode_map4d(&m.tv, dt, a.tv, C::D, a.L, a.H, a.B, st, C::OWN) &&
-         encode_map4d(&m.tq, dt, a.tq, C::D, a.L, a.H, a.B, st, C::BL) && encode_map4d(&m.g, dt, a.gto, C::D, a.L, a.H, a.B, nullptr, C::BL);
-  constexpr bool parts = kDqParts<HAS_GT, MK>;
+    ok = ok && encode_map4d(&m.tk, dt, a.tk, a.D, a.L, a.H, a.B, st, C::OWN) && encode_map4d(&m.tv, dt, a.tv, a.D, a.L, a.H, a.B, st, C::OWN) &&
+         encode_map4d(&m.tq, dt, a.tq, a.D, a.L, a.H, a.B, st, C::BL) && encode_map4d(&m.g, dt, a.gto, a.D, a.L, a.H, a.B, nullptr, C::BL);
+  const bool parts = dq_parts(a);
   float* dq_acc = parts ? static_cast<float*>(a.workspace) : a.dq_accum;
   const int n_key_tiles = (a.L + C::OWN - 1) / C::OWN;
-  ok = ok && (parts ? encode_map4d_f32(&m.dq, dq_acc, C::D, a.L, a.B * a.H, n_key_tiles, C::BL)
-                    : encode_map4d_f32(&m.dq, dq_acc, C::D, a.L, a.H, a.B, C::BL));
+  ok = ok && (parts ? encode_map4d_f32(&m.dq, dq_acc, a.D, a.L, a.B * a.H, n_key_tiles, C::BL)
+                    : encode_map4d_f32(&m.dq, dq_acc, a.D, a.L, a.H, a.B, C::BL));
   if (!ok) {
     set_last_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled(bwd fused64)");
     return JVPFA_ERR_CUDA;
@@ -1110,7 +1131,7 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
     set_last_cuda_error(cudaErrorUnknown, "multiprocessor count");
     return JVPFA_ERR_CUDA;
   }
-  const size_t n = (size_t)a.B * a.H * a.L * C::D;
+  const size_t n = (size_t)a.B * a.H * a.L * a.D;
   cudaError_t e = cudaSuccess;
   if (!parts && !(a.flags & JVPFA_DQ_ACCUM_IS_ZERO)) e = cudaMemsetAsync(a.dq_accum, 0, n * sizeof(float), stream);
   if (e != cudaSuccess) {
@@ -1119,7 +1140,7 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
   }
   const long long n_items = (long long)n_key_tiles * a.B * a.H;
   int grid = (int)(n_items < sms ? n_items : sms);
-  const long long used = parts ? bwd_bias_workspace(a) : 0;  // the split's workspace lies behind dQ's shares
+  const long long used = parts ? bwd_parts_workspace(a) : 0;  // the split's workspace lies behind dQ's shares
   const int ctas = split_ctas(a, sms);
   float* shares = nullptr;
   if (ctas > 0 && a.workspace != nullptr && (reinterpret_cast<uintptr_t>(a.workspace) & 15u) == 0 &&
@@ -1173,12 +1194,12 @@ static int launch_fused64_t(const jvpfa_bwd_args& a, cudaStream_t s) {
 // nor masks and bias whose rows are not whole 16-byte pieces, which the kernels of a fixed order have always served (B4 H8 L1000
 // D32, both outputs: 85 us here, 99 us there; a whole step: 209 us with either).
 bool bwd_tc5_fused64_eligible(const jvpfa_bwd_args& a) {
-  if (a.D != 64) return false;
   const int k = a.mask.kind;
-  if (k == JVPFA_MASK_BIAS && a.gto != nullptr) {
-    const long long need = tc5::bwd_bias_workspace(a);
+  if (tc5::dq_parts(a)) {
+    const long long need = tc5::bwd_parts_workspace(a);
     return need > 0 && a.workspace != nullptr && a.workspace_bytes >= need && (reinterpret_cast<uintptr_t>(a.workspace) & 15u) == 0;
   }
+  if (a.D != 64) return false;
   if (a.dq_accum == nullptr || (reinterpret_cast<uintptr_t>(a.dq_accum) & 15u) != 0) return false;
   if (k == JVPFA_MASK_NONE || k == JVPFA_MASK_CAUSAL || k == JVPFA_MASK_KVLEN) return true;
   if ((a.L & 15) != 0 || !tc5_mask_layout(a.mask, a.dtype, a.L)) return false;
@@ -1189,10 +1210,10 @@ bool bwd_tc5_fused64_eligible(const jvpfa_bwd_args& a) {
 
 // What the launch can use: shares of dQ (needed for a bias through tO), and of dK and dV where key tiles are cut.
 long long bwd_fused64_workspace(const jvpfa_bwd_args& a) {
-  if ((a.dtype != JVPFA_BF16 && a.dtype != JVPFA_FP16) || a.impl == JVPFA_IMPL_GENERIC || a.D != 64 || (a.flags & JVPFA_SKIP_DKDV)) return 0;
+  if ((a.dtype != JVPFA_BF16 && a.dtype != JVPFA_FP16) || a.impl == JVPFA_IMPL_GENERIC || a.D > 64 || (a.flags & JVPFA_SKIP_DKDV)) return 0;
   long long parts = 0;
-  if (a.mask.kind == JVPFA_MASK_BIAS && a.gto != nullptr) {
-    parts = tc5::bwd_bias_workspace(a);
+  if (tc5::dq_parts(a)) {
+    parts = tc5::bwd_parts_workspace(a);
     if (parts == 0) return 0;
   } else if (!bwd_tc5_fused64_eligible(a)) {
     return 0;

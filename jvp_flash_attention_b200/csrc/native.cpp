@@ -399,8 +399,8 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
 
   // One scratch allocation: the three row statistics, and fp32 dQ where the single-pass kernel takes it (head dimension 64,
   // 16-bit; index masks, and as far as rows are whole 16-byte pieces a boolean mask without tile bitmaps or, through O
-  // alone, a bias of the tensors' type).  Such a bias through tO has a workspace instead, below (from 96 key tiles on and up to
-  // 512 MiB; else the two launches).
+  // alone, a bias of the tensors' type).  Such a bias through tO, and head dimension 32, have a workspace instead, below
+  // (bwd_parts_workspace; else the two launches).
   bool single = g_single_pass && !(skip & JVPFA_SKIP_DKDV) && sizes[3] == 64 && q.scalar_type() != at::kFloat;
   if (m.c.kind == JVPFA_MASK_BOOL)
     single = single && !m.tile_live.defined() && !m.tile_live_t.defined() && whole_pieces(m, sizes[2]);
@@ -424,7 +424,10 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   if (!(skip & JVPFA_SKIP_DQ)) g[0] = empty(sizes, q.scalar_type(), q.device());
   if (!(skip & JVPFA_SKIP_DKDV))
     for (int i = 1; i < 3; ++i) g[i] = empty(sizes, q.scalar_type(), q.device());
-  const bool one_pass = g_single_pass && gto.defined() && sizes[3] == 64 && !(skip & JVPFA_SKIP_DKDV) && (sizes[2] + 127) / 128 * sizes[0] * sizes[1] >= 96;
+  // (whether the single pass takes the bias then: bwd_parts_workspace)
+  const int64_t key_tiles = (sizes[2] + 127) / 128 * sizes[0] * sizes[1];
+  const bool one_pass = g_single_pass && !(skip & JVPFA_SKIP_DKDV) &&
+                        (sizes[3] == 32 ? sizes[2] >= 1024 || key_tiles >= 75 : gto.defined() && sizes[3] == 64 && key_tiles >= 96);
   const Tensor padded = padded_bias(m, q, one_pass);
   jvpfa_bwd_args a{};
   a.struct_size = sizeof(a);
