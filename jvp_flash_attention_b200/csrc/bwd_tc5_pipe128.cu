@@ -70,7 +70,8 @@ struct BwdPipeCfg {
   static constexpr int OFF_Y = OFF_X + XSTAGES * X_STAGE;
   static constexpr int TILE_BYTES = OFF_Y + Y_STAGE;  // 224 KiB; without tangents 160 and 208
   static constexpr int STAT_BYTES = OWN_KEYS ? XSTAGES * BL * 16 : 0;
-  static constexpr int SMEM_BYTES = TILE_BYTES + STAT_BYTES + 256 + 1024;
+  static constexpr int LIVE_WORDS = 64;  // MK = 3: a bit for each loop tile
+  static constexpr int SMEM_BYTES = TILE_BYTES + STAT_BYTES + 256 + 4 * LIVE_WORDS + 1024;
   // tensors actually loaded
   static constexpr int N_KEY = HAS_GT ? 4 : 2;                               // K, V (+ tK, tV)
   static constexpr int N_QRY = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0);      // Q (+ gO) (+ tQ, G)
@@ -99,6 +100,7 @@ static_assert(BwdPipeCfg<false, true, false>::SMEM_BYTES <= 227 * 1024, "shared 
 template <bool OWN_KEYS, int BL>
 struct LoopWalk {
   const unsigned long long* w = nullptr;
+  const uint32_t* listed = nullptr;  // a bit for each loop tile, in shared memory
   int n_cand = 0, n_bits = 1, c = 0;
   bool rows = true;  // false: the mask has one row for all queries
   __device__ __forceinline__ bool bit(int b) const { return (__ldg(w + (b >> 6)) >> (b & 63)) & 1ull; }
@@ -111,12 +113,26 @@ struct LoopWalk {
     }
   }
   __device__ __forceinline__ int next() {  // index of the next live loop tile (the caller asks no more often than there are)
+    if (listed != nullptr) {
+      uint32_t word;
+      while ((word = listed[c >> 5] >> (c & 31)) == 0u) c = (c | 31) + 1;
+      c += __ffs((int)word);
+      return c - 1;
+    }
     while (c < n_cand && !live(c)) ++c;
     return c++;
   }
-  __device__ __forceinline__ int count() const {
+  // By a whole warp: how many there are, and, as far as there is room for a bit each, which.  (One thread alone counted them, tile after
+  // tile, and every role stepped over the dead ones by itself, both before the first load: B1 H8 L4096, a
+  // window of 1024 keys, both launches through O / tO / both 128 / 172 / 192 -> 99 / 150 / 171 us; B1 H4 L8192 - / 292 / 325 -> 158 / 251 / 284.)
+  __device__ __forceinline__ int list(uint32_t* words, int n_words) {
     int n = 0;
-    for (int cc = 0; cc < n_cand; ++cc) n += live(cc) ? 1 : 0;
+    for (int c0 = 0; c0 < n_cand; c0 += 32) {
+      const int cc = c0 + (int)(threadIdx.x & 31);
+      const uint32_t alive = __ballot_sync(0xffffffffu, cc < n_cand && live(cc));
+      if (n_cand <= 32 * n_words) words[c0 >> 5] = alive;
+      n += __popc(alive);
+    }
     return n;
   }
 };
@@ -157,6 +173,7 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* n_live = reinterpret_cast<int*>(tmem_slot + 2);  // MK == 3: live loop tiles of this CTA
+  uint32_t* live_words = reinterpret_cast<uint32_t*>(smem + C::TILE_BYTES + C::STAT_BYTES + 256);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int L = a.L;
@@ -236,7 +253,10 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
     mbar_init(y_empty, 1);
     *abort_flag = 0;
     fence_mbar_init();
-    if constexpr (MK == 3) *n_live = walk0.count();
+  }
+  if (MK == 3 && warp == 1) {
+    const int n = walk0.list(live_words, C::LIVE_WORDS);
+    if (lane == 0) *n_live = n;
   }
   if (warp == 0) {
     tmem_alloc(tmem_slot, C::COLS_ALLOC);
@@ -247,7 +267,10 @@ bwd_tc5_pipe128_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdPipeMa
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const AbortState ab{abort_flag, status};
-  if constexpr (MK == 3) n_tiles = *n_live;
+  if constexpr (MK == 3) {
+    if (n_tiles <= 32 * C::LIVE_WORDS) walk0.listed = live_words;
+    n_tiles = *n_live;
+  }
 
   // Tensor map of own slot s / loop slot s (nullptr: the slot is not used by this instance).
   auto own_map = [&](int s) -> const CUtensorMap* {
