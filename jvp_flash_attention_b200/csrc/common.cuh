@@ -526,6 +526,25 @@ template <typename T, int D>
 constexpr bool kBwdRowsDual = Elem<T>::k16 ? D <= 64 : !Elem<T>::kSplit && D == 32;
 
 // Host-side launch helpers implemented by each kernel translation unit.
+// 16-row groups of a CTA of the fp32 register-tiled kernels, 1, 2 or 4 (and 8, 4 or 2 parts of the loop side): 64 rows share every tile that is
+// brought in, and 16 take cost1 percent of their time for a row, 32 cost2; but one CTA fills an SM, so what counts are rounds of 148.  Causal: as
+// much work as half the rows, and the longest CTA comes on top.  Measured against the model on a B200, us by 16 / 32 / 64 rows, D = 128, forward with
+// tangents and backward through tO: B1 H37 L512 (2 rounds of 64 rows) 493 / 398 / 342 and 1231 / 1100 / 911, B3 H7 L256 99 / 106 / 90 and 238 /
+// 281 / 231, B2 H12 L512 356 / 299 / 340 and 895 / 815 / 895, B2 H5 L1920 causal 965 / 933 / 1047 and 2407 / 2522 / 2709; D = 32 B2 H4 L256 13 / 18 /
+// 26 and 32 / 50 / 80.  (By the number of rows alone, 64 from 592 groups of 16 on and 32 from 296: 281, 895 and 2709.)
+// Without tangents two CTAs of short row tiles fit an SM, and the number of rows does decide (B1 H2 L1410, 16 / 32 rows: 84 / 109).
+inline int row_groups(int B, int H, int L, bool tangents, bool causal, int cost1, int cost2) {
+  const long long rows16 = tiles16(B, H, L);
+  if (!tangents) return rows16 < 2 * 148 ? 1 : rows16 < 4 * 148 ? 2 : 4;
+  const long long BH = (long long)B * H;
+  auto time = [&](int rg, int cost) {
+    const long long ctas = BH * ((L + 16 * rg - 1) / (16 * rg));
+    return (causal ? ctas * rg + 2 * 148 * rg : (ctas + 147) / 148 * rg * 2 * 148) * cost;
+  };
+  const long long one = time(1, cost1), two = time(2, cost2), four = time(4, 100);
+  return four <= one && four <= two ? 4 : two <= one ? 2 : 1;
+}
+
 int launch_fwd_generic(const jvpfa_fwd_args& a, cudaStream_t stream);
 int launch_fwd_rows(const jvpfa_fwd_args& a, cudaStream_t stream);
 int launch_bwd_rows(const jvpfa_bwd_args& a, cudaStream_t stream);

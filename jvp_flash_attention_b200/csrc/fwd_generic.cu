@@ -436,15 +436,15 @@ static int launch_split(const jvpfa_fwd_args& a, cudaStream_t s) {
   return launch_one<T, D, true, true, RG, KG>(a, s);
 }
 
-// Rows x key parts of a CTA.  64 rows share every key tile that is brought in, so they are the choice once they give
-// each of the 148 SMs a CTA; below that shorter row tiles (whose warps share out the keys) put more SMs to work.
+// Rows x key parts of a CTA: row_groups.
 template <typename T, int D>
 static int launch_d(const jvpfa_fwd_args& a, cudaStream_t s) {
   const long long rows16 = tiles16(a.B, a.H, a.L);
   if (rows16 >= kFwdRowsFrom<T, D> && !(a.flags & JVPFA_ZERO_TKV) && (!a.tq || kFwdRowsDual<T, D>)) return launch_fwd_rows(a, s);
   if constexpr (!Elem<T>::k16) {
-    if (rows16 < 2 * 148) return launch_split<T, D, 1, 8>(a, s);
-    if (rows16 < 4 * 148) return launch_split<T, D, 2, 4>(a, s);
+    const int rg = row_groups(a.B, a.H, a.L, a.tq != nullptr, a.mask.kind == JVPFA_MASK_CAUSAL, 145, 122);
+    if (rg == 1) return launch_split<T, D, 1, 8>(a, s);
+    if (rg == 2) return launch_split<T, D, 2, 4>(a, s);
   }
   return launch_split<T, D, 4, 2>(a, s);
 }
