@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(32 * RG * KG, kTwoOnAnSm<T, D, HAS_GT, RG> ? 2
 
     // this warp's queries of the tile (none of them may see its keys: nothing to do)
     const int mw = m0 + kg * LW;
-    if (mw < L && !(mv.kind == JVPFA_MASK_CAUSAL && mw + LW <= n0 + r0)) {
+    if (mw < L && !(mv.kind == JVPFA_MASK_CAUSAL && mw + LW <= n0 + r0) && !dead_queries(a, b, h, n0, mw, min(mw + LW, L))) {
       const T* sQ = sLoop + (size_t)stage * LOOP_TILES * BM * LD + kg * LW * LD;
       const T* sGO = sQ + BM * LD;                           // HAS_GO
       const T* sTQ = sQ + (1 + (HAS_GO ? 1 : 0)) * BM * LD;  // HAS_GT
@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(32 * RG * KG, kTwoOnAnSm<T, D, HAS_GT, RG> ? 2
     __syncthreads();
 
     const int nw = n0 + kg * LW;  // this warp's keys of the tile
-    if (nw < n_end && !(mv.kind == JVPFA_MASK_CAUSAL && nw > m0 + r0 + 15)) {
+    if (nw < n_end && !(mv.kind == JVPFA_MASK_CAUSAL && nw > m0 + r0 + 15) && !dead_keys(a, b, h, m0, nw, min(nw + LW, n_end))) {
       const T* sK = sLoop + (size_t)stage * LOOP_TILES * BN * LD + kg * LW * LD;
       const T* sV = sK + BN * LD;
       const T* sTK = sK + 2 * BN * LD;

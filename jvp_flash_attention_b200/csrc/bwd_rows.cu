@@ -190,6 +190,10 @@ __global__ void __launch_bounds__(128) bwd_dkdv_rows_kernel(const jvpfa_bwd_args
       stage = 0;
     }
     __syncthreads();
+    if (dead_queries(a, b, h, n0, m0, min(m0 + BM, L))) {  // (all warps alike)
+      __syncthreads();
+      continue;
+    }
 
     const T* base = sLoop + (size_t)stage * LOOP_TILES * BM * LD;
     const T* sQ = base;
@@ -385,6 +389,10 @@ __global__ void __launch_bounds__(128) bwd_dq_rows_kernel(const jvpfa_bwd_args a
       stage = 0;
     }
     __syncthreads();
+    if (dead_keys(a, b, h, m0, n0, min(n0 + BN, n_end))) {  // (all warps alike)
+      __syncthreads();
+      continue;
+    }
 
     const T* sK = sLoop + (size_t)stage * LOOP_TILES * BN * LD;
     const T* sV = sK + BN * LD;

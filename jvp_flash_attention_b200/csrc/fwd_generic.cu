@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
 
     const int n0 = it * BN + kg * BW;  // this warp's keys of the tile
     // (a part beyond the end, or above the diagonal of the warp's rows, is nobody's work; the barrier below is everybody's)
-    if (n0 < n_end && !(mv.kind == JVPFA_MASK_CAUSAL && n0 > m0 + r0 + 15)) {
+    if (n0 < n_end && !(mv.kind == JVPFA_MASK_CAUSAL && n0 > m0 + r0 + 15) && !dead_keys(a, b, h, m0, n0, min(n0 + BW, n_end))) {
     const T* sK = sKV + (size_t)stage * NKV * BN * LD + kg * BW * LD;
     const T* sV = sK + BN * LD;
     const T* sTK = sK + 2 * BN * LD;

@@ -102,6 +102,10 @@ __global__ void __launch_bounds__(128) fwd_rows_kernel(const jvpfa_fwd_args a) {
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
+    if (dead_keys(a, b, h, m0, n0, min(n0 + BN, n_end))) {  // (all warps alike)
+      __syncthreads();
+      continue;
+    }
 
     const T* sK = sKV + (size_t)(it & 1) * NKV * BN * LD;
     const T* sV = sK + BN * LD;
