@@ -168,7 +168,9 @@ __device__ __forceinline__ int2 split_begin(const jvpfa_bwd_args& a, int c, int 
 __host__ __device__ __forceinline__ bool dq_parts(const jvpfa_bwd_args& a) {
   return a.D == 32 || (a.mask.kind == JVPFA_MASK_BIAS && a.gto != nullptr);
 }
-template <typename T, bool HAS_GO, bool HAS_GT, int MK, bool CUT>
+// HD: the head dimension, 64 or 32.  RAG, of a bias: its length is not a multiple of 16.  (Known at run time alone they cost the D = 64 kernels up to
+// 4 and 5 %.)
+template <typename T, bool HAS_GO, bool HAS_GT, int MK, bool CUT, int HD, bool RAG>
 __global__ void __launch_bounds__(512, 1)
 bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps maps, float* dq_acc, float* shares, int* status) {
   using C = BwdFCfg<HAS_GO, HAS_GT>;
@@ -282,7 +284,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
     return n_valid;
   };
 
-  const bool parts = dq_parts(a);
+  constexpr bool parts = HD == 32 || (HAS_GT && MK == 2);  // dq_parts
   // NaN into the rows of dK, dV and of the dQ accumulator that this CTA's items own: this launch's results are
   // not to be trusted
   auto poison = [&]() {
@@ -291,9 +293,9 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
       const int i = it.own0 + tid;
       if (tid < OWN && share(walk, 0)) share(walk, 0)[4 * tid] = share(walk, 1)[4 * tid] = poison_f32();
       if (tid < OWN && i < L) {
-        poison_row<T>(a.dk, (size_t)it.bh * L + i, a.D);
-        poison_row<T>(a.dv, (size_t)it.bh * L + i, a.D);
-        dq_acc[((parts ? (size_t)(it.own0 / OWN) * BH * L : 0) + (size_t)it.bh * L + i) * a.D] = poison_f32();
+        poison_row<T>(a.dk, (size_t)it.bh * L + i, HD);
+        poison_row<T>(a.dv, (size_t)it.bh * L + i, HD);
+        dq_acc[((parts ? (size_t)(it.own0 / OWN) * BH * L : 0) + (size_t)it.bh * L + i) * HD] = poison_f32();
       }
     }
   };
@@ -478,8 +480,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             else
               umma_ss_lo<true>(tmem + col, a_lo, b_lo, id);
 #pragma unroll
-            for (int ks = 1; ks < D / 16; ++ks)
-              if (ks < 2 || a.D > 32) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 2, id);
+            for (int ks = 1; ks < HD / 16; ++ks) umma_ss_lo<true>(tmem + col, a_lo + ks * 2, b_lo + ks * 2, id);
           };
           for (int walk = begin_items(); ok && get_item(walk, it); ++walk) {
             if (it.n_sub == 0) continue;
@@ -649,7 +650,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 
     auto store_row = [&](void* gptr, int bh, int own_idx, const uint32_t (&r0)[32], const uint32_t (&r1)[32], float mul) {
       if (own_idx >= L) return;
-      T* gp = reinterpret_cast<T*>(gptr) + ((size_t)bh * L + own_idx) * a.D;
+      T* gp = reinterpret_cast<T*>(gptr) + ((size_t)bh * L + own_idx) * HD;
 #pragma unroll
       for (int x = 0; x < 4; ++x)
         reinterpret_cast<uint4*>(gp)[x] = make_uint4(
@@ -657,7 +658,7 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
             Elem<T>::pack(__uint_as_float(r0[8 * x + 2]) * mul, __uint_as_float(r0[8 * x + 3]) * mul),
             Elem<T>::pack(__uint_as_float(r0[8 * x + 4]) * mul, __uint_as_float(r0[8 * x + 5]) * mul),
             Elem<T>::pack(__uint_as_float(r0[8 * x + 6]) * mul, __uint_as_float(r0[8 * x + 7]) * mul));
-      if (a.D == 32) return;
+      if constexpr (HD == 32) return;
 #pragma unroll
       for (int x = 0; x < 4; ++x)
         reinterpret_cast<uint4*>(gp)[4 + x] = make_uint4(
@@ -702,23 +703,17 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
           next_live = l0 < L ? ldg_nc_u32(bcol + (a.mask.stride[2] ? l0 >> 5 : 0)) : 0u;
         } else if constexpr (MK == 2) {
           const long long step = a.mask.stride[2] * 2;  // to the next query; the last one's elements stand for those beyond
+          // (not ragged: L is a multiple of 16 and so is q0, and the 16 queries are all there or none is; else the last pair of an odd length ends in
+          // its row's padding)
           const int q0 = l0 + 16 * (lane & 1);
-          // (the last pair of an odd length ends in its row's padding)
           const unsigned char* el = reinterpret_cast<const unsigned char*>(a.mask.ptr) +
-                                    ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] + min(own_idx - (lane & 1), (L - 1) & ~1)) * 2 +
-                                    min(q0, L - 1) * step;
-          if (q0 + 16 <= L) {
+                                    ((long long)it.b * a.mask.stride[0] + (long long)it.h * a.mask.stride[1] +
+                                     min(own_idx - (lane & 1), RAG ? (L - 1) & ~1 : L - 2)) * 2 +
+                                    min(q0, RAG ? L - 1 : L - 16) * step;
 #pragma unroll
-            for (int x = 0; x < 16; ++x) {
-              braw[x] = ldg_nc_u32(el);
-              el += step;
-            }
-          } else {
-#pragma unroll
-            for (int x = 0; x < 16; ++x) {
-              braw[x] = ldg_nc_u32(el);
-              if (q0 + x + 1 < L) el += step;
-            }
+          for (int x = 0; x < 16; ++x) {
+            braw[x] = ldg_nc_u32(el);
+            if (!RAG || q0 + x + 1 < L) el += step;
           }
         } else if constexpr (MK == 1) {
           const long long step = a.mask.stride[2];
@@ -926,16 +921,16 @@ bwd_tc5_fused64_kernel(const jvpfa_bwd_args a, const __grid_constant__ BwdFMaps 
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             sts_v4(rowa + (((uint32_t)c ^ sw) << 4), r0[4 * c], r0[4 * c + 1], r0[4 * c + 2], r0[4 * c + 3]);
-            if (a.D > 32) sts_v4(rowa + 8192 + (((uint32_t)c ^ sw) << 4), r1[4 * c], r1[4 * c + 1], r1[4 * c + 2], r1[4 * c + 3]);
+            if (HD > 32) sts_v4(rowa + 8192 + (((uint32_t)c ^ sw) << 4), r1[4 * c], r1[4 * c + 1], r1[4 * c + 2], r1[4 * c + 3]);
           }
         }
         fence_async_smem();
         rb_meet();
         if (tid == 384) {
           const int i0 = it.loop_begin + s * BL;
-          if (parts) {
+          if constexpr (parts) {
             tma_store_part_4d(&maps.dq, dqs, 0, i0, it.bh, it.own0 / OWN);
-            if (a.D > 32) tma_store_part_4d(&maps.dq, dqs + 8192, 32, i0, it.bh, it.own0 / OWN);
+            if (HD > 32) tma_store_part_4d(&maps.dq, dqs + 8192, 32, i0, it.bh, it.own0 / OWN);
           } else {
             tma_reduce_add_4d(&maps.dq, dqs, 0, i0, it.h, it.b);
             tma_reduce_add_4d(&maps.dq, dqs + 8192, 32, i0, it.h, it.b);
@@ -992,7 +987,8 @@ __device__ __forceinline__ void sum_shares(const jvpfa_bwd_args& a, const float*
 //   n_parts = 0: dq = T(scale * the accumulation buffer), 8 elements per thread
 //   n_parts > 0: dq = T(scale * sum of the n_parts key tiles' shares of dQ, in their order), 4 elements per thread.  Bound by reading
 //                them (B2 H12 L1024: 50 MB, most of it still in L2).
-template <typename T>
+// CAUSAL: a query has a share of the key tiles up to its own.
+template <typename T, bool CAUSAL>
 __global__ void __launch_bounds__(256)
 fused64_finish_kernel(const jvpfa_bwd_args a, const float* acc, long long n, int n_parts, const float* shares, int ctas, int cut) {
   behind_previous();
@@ -1009,8 +1005,7 @@ fused64_finish_kernel(const jvpfa_bwd_args a, const float* acc, long long n, int
   const long long n4 = n / 4;
   if (i >= n4) return;
   const float4* p = reinterpret_cast<const float4*>(acc) + i;
-  // (causal: a query has a share of the key tiles up to its own)
-  if (a.mask.kind == JVPFA_MASK_CAUSAL) n_parts = min(n_parts, (int)(4 * i / a.D % a.L) / 128 + 1);
+  if constexpr (CAUSAL) n_parts = min(n_parts, (int)(4 * i / a.D % a.L) / 128 + 1);
   float4 s = __ldcs(p);
 #pragma unroll 8
   for (int k = 1; k < n_parts; ++k) {
@@ -1089,13 +1084,23 @@ static int split_ctas(const jvpfa_bwd_args& a, int sms) {
   return (cost + (open + way) * ctas + more * two) * of < whole * ctas * (of - 1) ? (int)ctas : 0;
 }
 
-template <typename T, bool HAS_GO, bool HAS_GT, int MK, bool CUT>
-static cudaError_t run_fused64(const jvpfa_bwd_args& a, const BwdFMaps& m, float* dq_acc, float* shares, int* status, int grid, cudaStream_t stream) {
+template <typename T, bool HAS_GO, bool HAS_GT, int MK, bool CUT, int HD, bool RAG>
+static cudaError_t run_fused64_d(const jvpfa_bwd_args& a, const BwdFMaps& m, float* dq_acc, float* shares, int* status, int grid, cudaStream_t stream) {
   using C = BwdFCfg<HAS_GO, HAS_GT>;
-  auto kern = bwd_tc5_fused64_kernel<T, HAS_GO, HAS_GT, MK, CUT>;
+  auto kern = bwd_tc5_fused64_kernel<T, HAS_GO, HAS_GT, MK, CUT, HD, RAG>;
   static SmemOptIn opt_in;
   if (!opt_in.ensure(reinterpret_cast<const void*>(kern), C::SMEM_BYTES)) return cudaErrorInvalidValue;
   return launch_behind(kern, grid, C::NTHREADS, C::SMEM_BYTES, stream, a, m, dq_acc, shares, status);
+}
+
+template <typename T, bool HAS_GO, bool HAS_GT, int MK, bool CUT>
+static cudaError_t run_fused64(const jvpfa_bwd_args& a, const BwdFMaps& m, float* dq_acc, float* shares, int* status, int grid, cudaStream_t stream) {
+  if constexpr (MK == 2)
+    if ((a.L & 15) != 0)
+      return a.D == 32 ? run_fused64_d<T, HAS_GO, HAS_GT, MK, CUT, 32, true>(a, m, dq_acc, shares, status, grid, stream)
+                       : run_fused64_d<T, HAS_GO, HAS_GT, MK, CUT, 64, true>(a, m, dq_acc, shares, status, grid, stream);
+  return a.D == 32 ? run_fused64_d<T, HAS_GO, HAS_GT, MK, CUT, 32, false>(a, m, dq_acc, shares, status, grid, stream)
+                   : run_fused64_d<T, HAS_GO, HAS_GT, MK, CUT, 64, false>(a, m, dq_acc, shares, status, grid, stream);
 }
 
 template <typename T, bool HAS_GO, bool HAS_GT, int MK>
@@ -1158,7 +1163,8 @@ static int launch_fused64(const jvpfa_bwd_args& a, cudaStream_t stream) {
   const long long per_block = parts ? 256 * 4 : 256 * 8;
   const long long blocks = cut + (a.flags & JVPFA_SKIP_DQ ? 0 : ((long long)n + per_block - 1) / per_block);
   if (blocks == 0) return JVPFA_OK;
-  e = launch_behind(fused64_finish_kernel<T>, (unsigned)blocks, 256, 0, stream, a, static_cast<const float*>(dq_acc), (long long)n,
+  auto finish = parts && a.mask.kind == JVPFA_MASK_CAUSAL ? fused64_finish_kernel<T, true> : fused64_finish_kernel<T, false>;
+  e = launch_behind(finish, (unsigned)blocks, 256, 0, stream, a, static_cast<const float*>(dq_acc), (long long)n,
                     parts ? n_key_tiles : 0, static_cast<const float*>(shares), ctas, cut);
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "launch fused64_finish");
