@@ -16,7 +16,7 @@
 // A dQ sub-tile is read back by a fourth warpgroup (an M = 64 accumulator sits in lanes 0..15 of each
 // 32-lane quarter) and added to an fp32 accumulation buffer in global memory with TMA reductions; a small kernel converts that
 // buffer to the output type at the end.  The order of those additions varies from run to run, so dQ is reproducible to
-// rounding, not bitwise.  (With a bias and through tO a key tile's share is stored instead, see kDqParts.)
+// rounding, not bitwise.  (With a bias and through tO a key tile's share is stored instead, see dq_parts; at D = 32 always.)
 //
 // Measured on a B200, cycles of a sub-tile inside an item (clock marks in one CTA, every SM at work): through O 1660, through tO 2310,
 // both 2600; the tensor pipe's own time is 1024, 1860 and 2050, so that with tangents it is busy four fifths of a sub-tile, and
