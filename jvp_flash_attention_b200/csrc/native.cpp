@@ -521,19 +521,23 @@ struct AttnBwdNode : public Node {
       NoFunctorch nf;
       at::AutoDispatchBelowADInplaceOrView below;
       // In the layout of q, k and v where the kernels read that in place: else all six, and again the backward's, are copied to row-major
-      // (bf16 B3 H10 L3392 D128, views of (B, L, H, D): 254 of the 1530 us of a Hessian-vector product).
+      // (bf16 B3 H10 L3392 D128, views of (B, L, H, D): 254 of the 1530 us of a Hessian-vector product).  A tensor of the layout of q with
+      // gaps between its rows (slices of one packed projection) is not made anew: only tangents that come in it are read in place, and
+      // else row-major ones cost the fewest copies, those of q, k and v.
+      const int n = zero_tkv ? 1 : 3;
+      auto aligned = [](const Tensor& x) { return (reinterpret_cast<uintptr_t>(x.const_data_ptr()) & 15u) == 0; };
       int64_t st[3];
-      const bool shared = common_layout({&qp, &kp, &vp}, st);
-      for (int i = 0; i < (zero_tkv ? 1 : 3); ++i) {
-        if (!u[i].defined()) {
-          t[i] = shared ? at::zeros_like(qp) : at::zeros_like(qp, at::MemoryFormat::Contiguous);
-          continue;
-        }
-        t[i] = unwrap(u[i]);
-        if (!shared)
-          t[i] = t[i].contiguous();
-        else if (t[i].strides() != qp.strides() || (reinterpret_cast<uintptr_t>(t[i].const_data_ptr()) & 15u) != 0)
-          t[i] = at::empty_like(qp).copy_(t[i]);
+      bool views = common_layout({&qp, &kp, &vp}, st) && st[2] != 0;
+      const bool gaps = views && !qp.is_non_overlapping_and_dense();
+      for (int i = 0; i < n; ++i) {
+        if (u[i].defined()) t[i] = unwrap(u[i]);
+        if (gaps) views = views && t[i].defined() && t[i].strides() == qp.strides() && aligned(t[i]);
+      }
+      for (int i = 0; i < n; ++i) {
+        if (!t[i].defined())
+          t[i] = views ? at::zeros_like(qp) : at::zeros_like(qp, at::MemoryFormat::Contiguous);
+        else if ((views ? t[i].strides() != qp.strides() : !t[i].is_contiguous()) || !aligned(t[i]))
+          t[i] = (views ? at::empty_like(qp) : at::empty_like(qp, at::MemoryFormat::Contiguous)).copy_(t[i]);
       }
     }
     const int skip = unused_gradients(task_should_compute_output(0), task_should_compute_output(1) || task_should_compute_output(2));

@@ -3,6 +3,8 @@ import pytest
 import torch
 
 from jvp_flash_attention_b200 import jvp_attention as ja
+from tests import _oracle_launchers as stand_in
+from tests.test_autograd_wiring import cpu_kernels  # noqa: F401
 
 DEV = "cuda:0"
 
@@ -38,3 +40,43 @@ def test_layouts_give_what_row_major_tensors_give(D, dt, inputs, direction):
 
     got, want = hvp(q, k, v, u), hvp(*(t.contiguous() for t in (q, k, v, u)))
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("inputs", ["views", "packed", "row-major"])
+@pytest.mark.parametrize("direction", ["views", "packed", "row-major", "q alone"])
+def test_what_the_kernels_are_handed(cpu_kernels, monkeypatch, inputs, direction):  # noqa: F811
+    """Tangents in the layout of q, k and v as far as that takes no copy of q, k or v; else row-major, and never copied where they come so."""
+    B, H, L, D = 2, 3, 32, 32
+    g = torch.Generator().manual_seed(1)
+    r = lambda *s: torch.randn(*s, generator=g, dtype=torch.float64)  # noqa: E731
+
+    def three(layout):
+        if layout == "packed":
+            return list(r(B, L, 3, H, D).permute(2, 0, 3, 1, 4))
+        if layout == "views":
+            return [r(B, L, H, D).transpose(1, 2) for _ in range(3)]
+        return [r(B, H, L, D) for _ in range(3)]
+
+    seen = []
+
+    def launch_fwd(*a):
+        seen.append(a)
+        return tuple(None if y is None else y.contiguous() for y in stand_in.launch_fwd(*a))
+
+    monkeypatch.setattr(ja, "_launch_fwd", launch_fwd)
+    x = [t.requires_grad_() for t in three(inputs)]
+    u = three("row-major" if direction == "q alone" else direction)
+    o = ja.attention(*x)
+    grads = torch.autograd.grad(o, x, r(B, H, L, D), create_graph=True)
+    if direction == "q alone":
+        torch.autograd.grad(grads[0], x, u[0])
+        u = u[:1]
+    else:
+        torch.autograd.grad(grads, x, u)
+    given, in_place = seen[-1][3:6], inputs == "views" or inputs == direction
+    for t in given:
+        assert t.stride() == x[0].stride() if in_place else t.is_contiguous()
+    for t, y in zip(given, u):
+        assert torch.equal(t, y)
+        if y.stride() == t.stride():
+            assert t.data_ptr() == y.data_ptr()
