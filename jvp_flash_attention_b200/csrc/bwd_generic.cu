@@ -254,8 +254,9 @@ __device__ __forceinline__ void gemm_out(float (*out)[4], const float (*at0)[4],
 template <typename T, int D, bool HAS_GT, int RG>
 constexpr bool kTwoOnAnSm = !Elem<T>::k16 && D == 32 && HAS_GT && RG == 4;
 
-// TKV: K and V have tangents (JVPFA_ZERO_TKV leaves out what they would be multiplied by; it comes without gO).
-template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
+// TKV: K and V have tangents (JVPFA_ZERO_TKV leaves out what they would be multiplied by; it comes without gO).  TILES: parts of loop tiles
+// without a true mask entry are left out (dead_queries, dead_keys).
+template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG, bool TILES>
 __global__ void __launch_bounds__(32 * RG * KG, kTwoOnAnSm<T, D, HAS_GT, RG> ? 2 : 0) bwd_dkdv_kernel(const jvpfa_bwd_args a) {
   using C = BwdCfg<T, D, RG, KG>;
   constexpr int BN = C::OWN, BM = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES, LW = C::LW;
@@ -362,7 +363,7 @@ __global__ void __launch_bounds__(32 * RG * KG, kTwoOnAnSm<T, D, HAS_GT, RG> ? 2
 
     // this warp's queries of the tile (none of them may see its keys: nothing to do)
     const int mw = m0 + kg * LW;
-    if (mw < L && !(mv.kind == JVPFA_MASK_CAUSAL && mw + LW <= n0 + r0) && !dead_queries(a, b, h, n0, mw, min(mw + LW, L))) {
+    if (mw < L && !(mv.kind == JVPFA_MASK_CAUSAL && mw + LW <= n0 + r0) && !(TILES && dead_queries(a, b, h, n0, mw, min(mw + LW, L)))) {
       const T* sQ = sLoop + (size_t)stage * LOOP_TILES * BM * LD + kg * LW * LD;
       const T* sGO = sQ + BM * LD;                           // HAS_GO
       const T* sTQ = sQ + (1 + (HAS_GO ? 1 : 0)) * BM * LD;  // HAS_GT
@@ -435,7 +436,7 @@ __global__ void __launch_bounds__(32 * RG * KG, kTwoOnAnSm<T, D, HAS_GT, RG> ? 2
 }
 
 // ---- dQ: CTA owns 64 queries, loops over key tiles (rows = queries, columns = keys). ----
-template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
+template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG, bool TILES>
 __global__ void __launch_bounds__(32 * RG * KG, kTwoOnAnSm<T, D, HAS_GT, RG> ? 2 : 0) bwd_dq_kernel(const jvpfa_bwd_args a) {
   using C = BwdCfg<T, D, RG, KG>;
   constexpr int BM = C::OWN, BN = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES, LW = C::LW;
@@ -537,7 +538,7 @@ __global__ void __launch_bounds__(32 * RG * KG, kTwoOnAnSm<T, D, HAS_GT, RG> ? 2
     __syncthreads();
 
     const int nw = n0 + kg * LW;  // this warp's keys of the tile
-    if (nw < n_end && !(mv.kind == JVPFA_MASK_CAUSAL && nw > m0 + r0 + 15) && !dead_keys(a, b, h, m0, nw, min(nw + LW, n_end))) {
+    if (nw < n_end && !(mv.kind == JVPFA_MASK_CAUSAL && nw > m0 + r0 + 15) && !(TILES && dead_keys(a, b, h, m0, nw, min(nw + LW, n_end)))) {
       const T* sK = sLoop + (size_t)stage * LOOP_TILES * BN * LD + kg * LW * LD;
       const T* sV = sK + BN * LD;
       const T* sTK = sK + 2 * BN * LD;
@@ -594,15 +595,17 @@ __global__ void __launch_bounds__(32 * RG * KG, kTwoOnAnSm<T, D, HAS_GT, RG> ? 2
   smem_tile_to_global<T, BM, D, NT>(reinterpret_cast<T*>(a.dq) + head_off, sQ, LD, m0, L, tid);
 }
 
-template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG>
+template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TKV, int RG, int KG, bool TILES = false>
 static int launch_bwd_one(const jvpfa_bwd_args& a, cudaStream_t stream) {
+  if constexpr (!Elem<T>::k16 && !TILES)
+    if (with_tiles(a)) return launch_bwd_one<T, D, HAS_GO, HAS_GT, TKV, RG, KG, true>(a, stream);
   using C = BwdCfg<T, D, RG, KG>;
   constexpr int keys = TKV ? 4 : 2, queries = 1 + (HAS_GO ? 1 : 0) + (HAS_GT ? 2 : 0);  // tiles of each side
   constexpr size_t smem_kv = C::smem(keys, queries, true);
   constexpr size_t smem_q = C::smem(queries, keys, false);
   static_assert(smem_kv <= 227 * 1024 && smem_q <= 227 * 1024, "shared memory of one CTA");
-  auto k1 = bwd_dkdv_kernel<T, D, HAS_GO, HAS_GT, TKV, RG, KG>;
-  auto k2 = bwd_dq_kernel<T, D, HAS_GO, HAS_GT, TKV, RG, KG>;
+  auto k1 = bwd_dkdv_kernel<T, D, HAS_GO, HAS_GT, TKV, RG, KG, TILES>;
+  auto k2 = bwd_dq_kernel<T, D, HAS_GO, HAS_GT, TKV, RG, KG, TILES>;
   static SmemOptIn opt_in1, opt_in2;
   if (!opt_in1.ensure(reinterpret_cast<const void*>(k1), smem_kv) || !opt_in2.ensure(reinterpret_cast<const void*>(k2), smem_q))
     return JVPFA_ERR_CUDA;

@@ -88,7 +88,7 @@ __device__ __forceinline__ void gemm_acc_nn(float (*out)[4], const float (*atile
 
 // ---- dK, dV: CTA owns 64 keys, loops over query tiles.  Tiles are held transposed
 // (rows = keys, columns = queries) so that P^T etc. feed the second MMAs from registers. ----
-template <typename T, int D, bool HAS_GO, bool HAS_GT>
+template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TILES>
 __global__ void __launch_bounds__(128) bwd_dkdv_rows_kernel(const jvpfa_bwd_args a) {
   using C = BwdRowsCfg<T, D>;
   constexpr int BN = C::OWN, BM = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES;
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(128) bwd_dkdv_rows_kernel(const jvpfa_bwd_args
       stage = 0;
     }
     __syncthreads();
-    if (dead_queries(a, b, h, n0, m0, min(m0 + BM, L))) {  // (all warps alike)
+    if (TILES && dead_queries(a, b, h, n0, m0, min(m0 + BM, L))) {  // (all warps alike)
       __syncthreads();
       continue;
     }
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(128) bwd_dkdv_rows_kernel(const jvpfa_bwd_args
 }
 
 // ---- dQ: CTA owns 64 queries, loops over key tiles (rows = queries, columns = keys). ----
-template <typename T, int D, bool HAS_GO, bool HAS_GT>
+template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TILES>
 __global__ void __launch_bounds__(128) bwd_dq_rows_kernel(const jvpfa_bwd_args a) {
   using C = BwdRowsCfg<T, D>;
   constexpr int BM = C::OWN, BN = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES;
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(128) bwd_dq_rows_kernel(const jvpfa_bwd_args a
       stage = 0;
     }
     __syncthreads();
-    if (dead_keys(a, b, h, m0, n0, min(n0 + BN, n_end))) {  // (all warps alike)
+    if (TILES && dead_keys(a, b, h, m0, n0, min(n0 + BN, n_end))) {  // (all warps alike)
       __syncthreads();
       continue;
     }
@@ -466,15 +466,17 @@ __global__ void __launch_bounds__(128) bwd_dq_rows_kernel(const jvpfa_bwd_args a
   smem_tile_to_global<T, BM, D, NT>(reinterpret_cast<T*>(a.dq) + head_off, sQ, LD, m0, L, tid);
 }
 
-template <typename T, int D, bool HAS_GO, bool HAS_GT>
+template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TILES = false>
 static int launch_bwd_one(const jvpfa_bwd_args& a, cudaStream_t stream) {
+  if constexpr (!Elem<T>::k16 && !TILES)
+    if (with_tiles(a)) return launch_bwd_one<T, D, HAS_GO, HAS_GT, true>(a, stream);
   using C = BwdRowsCfg<T, D>;
   constexpr int go = HAS_GO ? 1 : 0, gt = HAS_GT ? 1 : 0;
   constexpr size_t smem_kv = C::smem(gt ? 4 : 2, 1 + go + 2 * gt, true);
   constexpr size_t smem_q = C::smem(1 + go + 2 * gt, gt ? 4 : 2, false);
   static_assert(smem_kv <= 227 * 1024 && smem_q <= 227 * 1024, "shared memory of one CTA");
-  auto k1 = bwd_dkdv_rows_kernel<T, D, HAS_GO, HAS_GT>;
-  auto k2 = bwd_dq_rows_kernel<T, D, HAS_GO, HAS_GT>;
+  auto k1 = bwd_dkdv_rows_kernel<T, D, HAS_GO, HAS_GT, TILES>;
+  auto k2 = bwd_dq_rows_kernel<T, D, HAS_GO, HAS_GT, TILES>;
   static SmemOptIn opt_in1, opt_in2;
   if (!opt_in1.ensure(reinterpret_cast<const void*>(k1), smem_kv) || !opt_in2.ensure(reinterpret_cast<const void*>(k2), smem_q))
     return JVPFA_ERR_CUDA;

@@ -525,12 +525,16 @@ constexpr bool kFwdRowsDual = Elem<T>::k16 ? D > 32 : Elem<T>::kSplit ? D == 64 
 template <typename T, int D>
 constexpr bool kBwdRowsDual = Elem<T>::k16 ? D <= 64 : !Elem<T>::kSplit && D == 32;
 
-// Host-side launch helpers implemented by each kernel translation unit.
 // Whether a part of a loop tile of the register-tiled kernels holds no true entry for the own tile, by the bitmaps of jvpfa_mask_tiles.  The tile is
-// staged all the same and its products left out, which costs calls without bitmaps little: a list of live tiles to step along took a quarter less
-// (66 and 188 us of the first shape below) but made unmasked calls up to 3 % slower, for its registers.  fp32, windows of a quarter of the length, us before / so, forward with tangents and backward through
+// staged all the same and its products left out.  fp32 (and TF32) alone, in instances of their own (TILES): in those of other calls the test took
+// registers, which cost most of them 1 to 3 % and TF32 at D = 64 through tO, which no longer fitted two CTAs on an SM, up to 1.4 times (B1 H8 L1000 275 /
+// 366 us).  fp32, windows of a quarter of the length, us before / so, forward with tangents and backward through
 // tO: B1 H2 L1410 D64 172 / 90 and 436 / 236, B2 H10 L1408 D32 390 / 211 and 1023 / 601, B1 H1 L704 D128
 // 88 / 61 and 206 / 139.
+inline bool with_tiles(const jvpfa_fwd_args& a) { return a.mask.kind == JVPFA_MASK_BOOL && a.mask_tile_live != nullptr; }
+inline bool with_tiles(const jvpfa_bwd_args& a) {  // (both or neither)
+  return a.mask.kind == JVPFA_MASK_BOOL && a.mask_tile_live != nullptr && a.mask_tile_live_t != nullptr;
+}
 __device__ __forceinline__ long long bitmap_head(const jvpfa_mask& m, int b, int h, int H) {  // (a dimension that broadcasts has one entry)
   return (m.stride[0] ? (long long)b * (m.stride[1] ? H : 1) : 0) + (m.stride[1] ? h : 0);
 }
@@ -543,13 +547,11 @@ __device__ __forceinline__ bool no_bit(const void* bitmap, long long word, int f
 // Own queries from m0 on (of one 128-query tile) and keys [n0, n1).
 template <typename Args>
 __device__ __forceinline__ bool dead_keys(const Args& a, int b, int h, int m0, int n0, int n1) {
-  if (a.mask.kind != JVPFA_MASK_BOOL || a.mask_tile_live == nullptr) return false;
   const long long head = bitmap_head(a.mask, b, h, a.H);
   return no_bit(a.mask_tile_live, (a.mask.stride[2] ? head * ((a.L + 127) / 128) + m0 / 128 : head) * (((a.L + 63) / 64 + 63) / 64), n0 >> 6, (n1 - 1) >> 6);
 }
 // Own keys from n0 on (of one 128-key tile) and queries [m0, m1).
 __device__ __forceinline__ bool dead_queries(const jvpfa_bwd_args& a, int b, int h, int n0, int m0, int m1) {
-  if (a.mask.kind != JVPFA_MASK_BOOL || a.mask_tile_live_t == nullptr) return false;
   const bool rows = a.mask.stride[2] != 0;
   const int n_t128 = (a.L + 127) / 128;
   return no_bit(a.mask_tile_live_t, (bitmap_head(a.mask, b, h, a.H) * n_t128 + n0 / 128) * (rows ? (n_t128 + 63) / 64 : 1), rows ? m0 >> 7 : 0,
@@ -575,6 +577,7 @@ inline int row_groups(int B, int H, int L, bool tangents, bool causal, int cost1
   return four <= one && four <= two ? 4 : two <= one ? 2 : 1;
 }
 
+// Host-side launch helpers implemented by each kernel translation unit.
 int launch_fwd_generic(const jvpfa_fwd_args& a, cudaStream_t stream);
 int launch_fwd_rows(const jvpfa_fwd_args& a, cudaStream_t stream);
 int launch_bwd_rows(const jvpfa_bwd_args& a, cudaStream_t stream);

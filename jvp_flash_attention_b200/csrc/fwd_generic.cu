@@ -46,7 +46,8 @@ struct FwdCfg {
 };
 
 // TKV: K and V have tangents (JVPFA_ZERO_TKV leaves them, and two of the six products, out).
-template <typename T, int D, bool DUAL, bool TKV, int RG, int KG>
+// TILES: parts of key tiles without a true mask entry are left out (dead_keys).
+template <typename T, int D, bool DUAL, bool TKV, int RG, int KG, bool TILES>
 __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_fwd_args a) {
   using C = FwdCfg<T, D, RG, KG>;
   constexpr int BM = C::BM, BN = C::BN, BW = C::BW, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES;
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
 
     const int n0 = it * BN + kg * BW;  // this warp's keys of the tile
     // (a part beyond the end, or above the diagonal of the warp's rows, is nobody's work; the barrier below is everybody's)
-    if (n0 < n_end && !(mv.kind == JVPFA_MASK_CAUSAL && n0 > m0 + r0 + 15) && !dead_keys(a, b, h, m0, n0, min(n0 + BW, n_end))) {
+    if (n0 < n_end && !(mv.kind == JVPFA_MASK_CAUSAL && n0 > m0 + r0 + 15) && !(TILES && dead_keys(a, b, h, m0, n0, min(n0 + BW, n_end)))) {
     const T* sK = sKV + (size_t)stage * NKV * BN * LD + kg * BW * LD;
     const T* sV = sK + BN * LD;
     const T* sTK = sK + 2 * BN * LD;
@@ -410,12 +411,14 @@ __global__ void __launch_bounds__(32 * RG * KG) fwd_generic_kernel(const jvpfa_f
   }
 }
 
-template <typename T, int D, bool DUAL, bool TKV, int RG, int KG>
+template <typename T, int D, bool DUAL, bool TKV, int RG, int KG, bool TILES = false>
 static int launch_one(const jvpfa_fwd_args& a, cudaStream_t stream) {
+  if constexpr (!Elem<T>::k16 && !TILES)
+    if (with_tiles(a)) return launch_one<T, D, DUAL, TKV, RG, KG, true>(a, stream);
   using C = FwdCfg<T, D, RG, KG>;
   constexpr size_t smem = C::smem(DUAL, TKV);
   static_assert(smem <= 227 * 1024, "shared memory of one CTA");
-  auto kern = fwd_generic_kernel<T, D, DUAL, TKV, RG, KG>;
+  auto kern = fwd_generic_kernel<T, D, DUAL, TKV, RG, KG, TILES>;
   static SmemOptIn opt_in;
   if (!opt_in.ensure(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_CUDA;
   dim3 grid((a.L + C::BM - 1) / C::BM, a.B * a.H);

@@ -20,7 +20,8 @@ struct FwdRowsCfg {
   }
 };
 
-template <typename T, int D, bool DUAL>
+// TILES: key tiles without a true mask entry are left out (dead_keys).
+template <typename T, int D, bool DUAL, bool TILES>
 __global__ void __launch_bounds__(128) fwd_rows_kernel(const jvpfa_fwd_args a) {
   using C = FwdRowsCfg<T, D>;
   constexpr int BM = C::BM, BN = C::BN, LD = C::LD, NT = C::NTHREADS;
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(128) fwd_rows_kernel(const jvpfa_fwd_args a) {
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
-    if (dead_keys(a, b, h, m0, n0, min(n0 + BN, n_end))) {  // (all warps alike)
+    if (TILES && dead_keys(a, b, h, m0, n0, min(n0 + BN, n_end))) {  // (all warps alike)
       __syncthreads();
       continue;
     }
@@ -334,11 +335,13 @@ __global__ void __launch_bounds__(128) fwd_rows_kernel(const jvpfa_fwd_args a) {
   }
 }
 
-template <typename T, int D, bool DUAL>
+template <typename T, int D, bool DUAL, bool TILES = false>
 static int launch_one(const jvpfa_fwd_args& a, cudaStream_t stream) {
+  if constexpr (!Elem<T>::k16 && !TILES)
+    if (with_tiles(a)) return launch_one<T, D, DUAL, true>(a, stream);
   using C = FwdRowsCfg<T, D>;
   constexpr size_t smem = C::smem(DUAL);
-  auto kern = fwd_rows_kernel<T, D, DUAL>;
+  auto kern = fwd_rows_kernel<T, D, DUAL, TILES>;
   static SmemOptIn opt_in;
   if (!opt_in.ensure(reinterpret_cast<const void*>(kern), smem)) return JVPFA_ERR_CUDA;
   dim3 grid((a.L + C::BM - 1) / C::BM, a.B * a.H);

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from jvp_flash_attention_b200 import _lib
+from jvp_flash_attention_b200 import jvp_attention as ja
 from oracle import jvp_attention_oracle as orc
 
 DEV = "cuda:0"
@@ -59,3 +60,34 @@ def test_same_as_visiting_every_tile(kind, B, H, L, D, dt, impl):
     for name, x, r in zip(("O", "tO", "dq", "dk", "dv"), (*runs[1][:2], *runs[1][4:]), ref):
         x = few(x).double().cpu()
         assert (x - r).norm() <= rel * r.norm(), (name, ((x - r).norm() / r.norm()).item())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,L,D", [(1, 2, 450, 64), (2, 24, 448, 32)])
+@pytest.mark.parametrize("missing", ["mask_tile_live", "mask_tile_live_t"])
+def test_one_bitmap_alone_decides_nothing(monkeypatch, B, H, L, D, missing):
+    """The backward takes both bitmaps or neither; here the other one calls every tile dead."""
+    g = torch.Generator().manual_seed(L + D)
+    q, k, v, _, _, _, go, _ = (torch.randn(B, H, L, D, generator=g).to(DEV) for _ in range(8))
+    m = _mask("window", B, H, L, g).to(DEV)
+    spec = _lib.MaskSpec(_lib.MASK_BOOL, m.view(torch.uint8), m.stride())
+    live, _, live_t = (torch.zeros_like(x) for x in _lib.mask_tiles(spec, L))
+    o, lse, stats = torch.empty_like(q), torch.empty(B, H, L, device=DEV), torch.empty(3, B, H, L, device=DEV)
+    _lib.fwd(q, k, v, None, None, None, o, None, lse, None, spec, D**-0.5, _lib.IMPL_GENERIC)
+    _lib.bwd_preprocess(o, None, go, None, None, *stats)
+    launch = _lib._launch
+
+    def one_bitmap(x, fn, a):
+        setattr(a, missing, None)
+        return launch(x, fn, a)
+
+    runs = []
+    for tiles in ((None, None), (live, live_t)):
+        spec.tile_live, spec.tile_live_t = tiles
+        if tiles[0] is not None:
+            monkeypatch.setattr(_lib, "_launch", one_bitmap)
+        grads = [torch.empty_like(q) for _ in range(3)]
+        _lib.bwd(q, k, v, None, None, None, go, None, lse, None, *stats, *grads, spec, D**-0.5, _lib.IMPL_GENERIC)
+        runs.append(grads)
+    for x, y in zip(*runs):
+        assert torch.equal(x, y)
