@@ -116,8 +116,9 @@ typedef struct {
    * elements.  Upstream always copies: jvp_attention.py:2733-2734, 2787-2788.  Outputs are always (B,H,L,D)
    * row-major. */
   int64_t in_stride[3];
-  /* Optional, JVPFA_MASK_BOOL only: the bitmap written by jvpfa_mask_tiles for this mask.  The tcgen05
-   * kernel then steps over 128 x 64 tiles without a true entry; other kernels ignore it.  NULL = none. */
+  /* Optional, JVPFA_MASK_BOOL only: the bitmap written by jvpfa_mask_tiles for this mask, as it is when the call runs.  The 16-bit tcgen05
+   * kernels then step over 128 x 64 tiles without a true entry, and the fp32 register-tiled ones leave their products out; other kernels
+   * ignore it.  NULL = none. */
   const void* mask_tile_live;
   /* Optional, JVPFA_MASK_BOOL only: `bits` of jvpfa_mask_tiles.  The tcgen05 kernels read it instead of the bytes, whose
    * layout then does not matter to them.  A caller built without this field (struct_size up to mask_tile_live): NULL. */
@@ -198,9 +199,9 @@ typedef struct {
   void *dq, *dk, *dv;
   jvpfa_mask mask;
   int64_t in_stride[3]; /* of q, k, v, tq, tk, tv, as in jvpfa_fwd_args; go, gto, dq, dk, dv are row-major */
-  /* Optional, JVPFA_MASK_BOOL only, both or neither: tile_live and tile_live_t of jvpfa_mask_tiles.  The two-launch
-   * tcgen05 kernels (D = 64: L <= 8192) then visit only the loop tiles that overlap a live tile; other kernels ignore
-   * them. */
+  /* Optional, JVPFA_MASK_BOOL only, both or neither (one alone is ignored): tile_live and tile_live_t of jvpfa_mask_tiles, for the mask as it is
+   * when the call runs.  The two-launch 16-bit tcgen05 kernels (D = 64: L <= 8192) then visit only the loop tiles that overlap a live tile, and the
+   * fp32 register-tiled ones leave the products of others out; other kernels ignore them. */
   const void* mask_tile_live;
   const void* mask_tile_live_t;
   /* Optional caller-owned scratch: B*H*L*D floats, 16-byte aligned, contents irrelevant on entry.  With it (D = 64,

@@ -93,8 +93,9 @@ struct Call {
   // A boolean mask as bits, by rows and transposed: the form the 16-bit tensor-core kernels read best, made by this call for
   // its forward and backward (pack_mask).
   Tensor bits, bits_t;
+  Tensor tiles;  // fp32: both tile bitmaps, made by this call for its register-tiled launches (make_tiles)
 
-  void drop_tensors() { bits = bits_t = Tensor(); }
+  void drop_tensors() { bits = bits_t = tiles = Tensor(); }
 };
 
 bool is_wrapped(const Tensor& x) {
@@ -285,6 +286,33 @@ void pack_mask(Call& call, const Tensor& q, bool backward) {
   pack(m, q, call.bits, backward ? &call.bits_t : nullptr);
 }
 
+// The tile bitmaps of a call's fp32 launches on the register-tiled kernels, [tile_live | tile_live_t], for a boolean mask whose verification left
+// tiles to step over.  These launches visited every tile before they knew of bitmaps, and their results were the mask's present entries' whatever
+// had been written since; so theirs are made anew, like the bits (B1 H8 L2048, a window as one (L, L) mask: 5 us).  The 16-bit
+// kernels are given those of the verification.  Left undefined where there is no memory: every tile is visited then.
+void make_tiles(Call& call, const Tensor& q) {
+  const MaskDesc& m = *call.mask;
+  if (call.tiles.defined() || q.scalar_type() != at::kFloat || !m.tile_live.defined() || !m.tile_live_t.defined()) return;
+  const int64_t L = q.size(2), n = m.tile_live.numel();
+  jvpfa_mask_tiles_args a{};
+  a.struct_size = sizeof(a);
+  a.n_b = m.c.stride[0] ? (int)m.tensor.size(0) : 1, a.n_h = m.c.stride[1] ? (int)m.tensor.size(1) : 1;
+  a.n_rows = m.c.stride[2] ? (int)L : 1, a.L = (int)L;
+  a.mask = m.c;
+  Tensor tiles;
+  try {
+    NoFunctorch nf;
+    at::AutoDispatchBelowADInplaceOrView below;
+    tiles = at::zeros({n + m.tile_live_t.numel()}, q.options().dtype(at::kLong).requires_grad(false));
+  } catch (const c10::OutOfMemoryError&) {
+    return;
+  }
+  a.tile_live = tiles.data_ptr();
+  a.tile_live_t = static_cast<int64_t*>(tiles.data_ptr()) + n;
+  check_status(jvpfa_mask_tiles(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "jvpfa_mask_tiles");
+  call.tiles = tiles;
+}
+
 // ---- launches ------------------------------------------------------------------------------------------------------
 // The workspace of a launch, which its kernels on the call's stream are the last to use; undefined for 0 bytes, and where
 // there is no memory for it (the kernels that need none serve the call then).
@@ -315,7 +343,7 @@ Tensor use_workspace(Args& a, const Tensor& workspace, const Call& call, const T
 
 // tq without tk and tv: JVPFA_ZERO_TKV.
 FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& tq, const Tensor& tk, const Tensor& tv,
-                     const Call& call) {
+                     Call& call) {
   const bool dual = tq.defined();
   FwdResult r;
   if (!q.is_cuda()) {
@@ -352,24 +380,28 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   a.to = dual ? r.to.data_ptr() : nullptr;
   a.mu = dual ? static_cast<float*>(r.mu.data_ptr()) : nullptr;
   a.mask = c_mask(*call.mask, padded);
-  a.mask_tile_live = data(call.mask->tile_live);
+  const bool fp32 = q.scalar_type() == at::kFloat;
+  a.mask_tile_live = fp32 ? nullptr : data(call.mask->tile_live);
   a.mask_bits = data(call.bits);
   a.flags = dual && !tk.defined() ? JVPFA_ZERO_TKV : 0;
   a.q = data(in.q), a.k = data(in.k), a.v = data(in.v);
   a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
   for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
   a.kv_len_host = host_lengths(*call.mask, a.B);
-  const bool fp32 = q.scalar_type() == at::kFloat;
   const Tensor workspace = workspace_of(!fp32 || call.parts ? jvpfa_fwd_workspace(&a) : 0, q);
   const Tensor bits = use_workspace(a, workspace, call, q);
   r.parts = fp32 && workspace.defined();
+  if (fp32 && !r.parts) {
+    make_tiles(call, q);
+    a.mask_tile_live = data(call.tiles);
+  }
   check_status(jvpfa_fwd(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "jvpfa_fwd");
   return r;
 }
 
 // Gradients of <go, O> + <gto, tO> with respect to q, k, v; those named in `skip` (JVPFA_SKIP_*) stay undefined.
 Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, Tensor tk, Tensor tv, const Tensor& o, Tensor to,
-                 const Tensor& lse, Tensor mu, Tensor go, Tensor gto, const Call& call, int skip = 0) {
+                 const Tensor& lse, Tensor mu, Tensor go, Tensor gto, Call& call, int skip = 0) {
   if (!q.is_cuda()) {
     py::gil_scoped_acquire gil;
     NoFunctorch nf;
@@ -443,7 +475,8 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   if (g[0].defined()) a.dq = g[0].data_ptr();
   if (g[1].defined()) a.dk = g[1].data_ptr(), a.dv = g[2].data_ptr();
   a.mask = c_mask(*call.mask, padded);
-  if (m.tile_live.defined() && m.tile_live_t.defined() && a.L <= 8192) {
+  const bool fp32 = q.scalar_type() == at::kFloat;
+  if (!fp32 && m.tile_live.defined() && m.tile_live_t.defined() && a.L <= 8192) {
     a.mask_tile_live = data(m.tile_live);
     a.mask_tile_live_t = data(m.tile_live_t);
   }
@@ -454,8 +487,12 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
   for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
   a.kv_len_host = host_lengths(m, a.B);
-  const Tensor workspace = workspace_of((q.scalar_type() == at::kFloat ? call.parts : g_single_pass.load()) ? jvpfa_bwd_workspace(&a) : 0, q);
+  const Tensor workspace = workspace_of((fp32 ? call.parts : g_single_pass.load()) ? jvpfa_bwd_workspace(&a) : 0, q);
   const Tensor bits = use_workspace(a, workspace, call, q);
+  if (fp32 && !workspace.defined() && a.L <= 8192) {
+    make_tiles(call, q);
+    if (call.tiles.defined()) a.mask_tile_live = call.tiles.data_ptr(), a.mask_tile_live_t = static_cast<int64_t*>(call.tiles.data_ptr()) + m.tile_live.numel();
+  }
   check_status(jvpfa_bwd(&a, stream), "jvpfa_bwd");
   return g;
 }
@@ -565,7 +602,7 @@ struct AttnBwdNode : public Node {
 };
 
 Grads backward_through_o(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& go,
-                         const Call& call, int skip) {
+                         Call& call, int skip) {
   if (is_wrapped(go)) {  // the cotangent belongs to a functorch transform: a Function, which the transform differentiates or refuses
     py::gil_scoped_acquire gil;
     py::tuple g = python_module().attr("_backward_under_functorch")(q, k, v, o, lse, go, *call.mask->spec, call.scale, call.tf32, call.parts);

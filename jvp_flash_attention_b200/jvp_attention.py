@@ -248,8 +248,19 @@ def _in_place_layout(ts):
         return [None if t is None else t.contiguous() for t in ts], None
 
 
+def _without_old_tiles(spec: _lib.MaskSpec, q: Tensor) -> _lib.MaskSpec:
+    """fp32 launches visit every tile here: the bitmaps are those of the mask's verification, and what these kernels read
+    are its present entries (the native layer makes bitmaps of these for them)."""
+    if spec.tile_live is None or q.dtype != torch.float32:
+        return spec
+    spec = copy.copy(spec)
+    spec.tile_live = spec.tile_live_t = None
+    return spec
+
+
 def _launch_fwd(q, k, v, tq, tk, tv, spec: _lib.MaskSpec, sm_scale: float):
     """Allocates outputs and runs the fused forward.  Returns (o, to | None, lse, mu | None)."""
+    spec = _without_old_tiles(spec, q)
     ins, st = _in_place_layout([_unwrap(x) for x in (q, k, v, tq, tk, tv)])
     Z, H, N, _ = ins[0].shape
     o = torch.empty(ins[0].shape, device=ins[0].device, dtype=ins[0].dtype)
@@ -263,6 +274,7 @@ def _launch_fwd(q, k, v, tq, tk, tv, spec: _lib.MaskSpec, sm_scale: float):
 
 def _launch_bwd(q, k, v, tq, tk, tv, o, to, lse, mu, go, gto, spec: _lib.MaskSpec, sm_scale: float):
     """Runs preprocess + backward for cotangents ``go`` (of O) and/or ``gto`` (of tO)."""
+    spec = _without_old_tiles(spec, q)
     q, k, v, tq, tk, tv, o, to, lse, mu, go, gto = (
         _unwrap(x) for x in (q, k, v, tq, tk, tv, o, to, lse, mu, go, gto)
     )

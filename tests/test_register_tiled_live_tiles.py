@@ -91,3 +91,42 @@ def test_one_bitmap_alone_decides_nothing(monkeypatch, B, H, L, D, missing):
         runs.append(grads)
     for x, y in zip(*runs):
         assert torch.equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ["data", "graph", "functorch"])
+@pytest.mark.parametrize("B,H,L,D", [(1, 2, 450, 64), (2, 6, 448, 128), (1, 3, 300, 32)])
+def test_a_window_written_behind_the_version_counter(how, B, H, L, D):
+    """fp32: what the kernels read are the mask's present entries, also where the verified ones left tiles dead."""
+    g = torch.Generator().manual_seed(D)
+    q, k, v, tq, tk, tv, go, gt = (torch.randn(B, H, L, D, generator=g).to(DEV) for _ in range(8))
+    first = _mask("window", 1, 1, L, g).to(DEV)
+    second = first.flip(-1) | torch.eye(L, dtype=torch.bool, device=DEV)
+    a = [x.requires_grad_() for x in (q, k, v)]
+
+    def run(m):
+        if how == "functorch":
+            o, back = torch.func.vjp(lambda *x: ja.attention(*x, attn_mask=m), *(x.detach() for x in a))
+            return (o, *back(go))
+        o, to = torch.func.jvp(lambda *x: ja.JVPAttn.fwd_dual(*x, attn_mask=m), tuple(a), (tq, tk, tv))
+        return (o, to, *torch.autograd.grad((o, to), a, (go, gt)))
+
+    want = [x.detach().clone() for x in run(second.clone())]
+    mask = first.clone()
+    if how != "graph":
+        run(mask)
+        mask.data.copy_(second)
+        got = run(mask)
+    else:
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            run(mask)
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = run(mask)
+        mask.copy_(second)
+        graph.replay()
+    for x, y in zip(got, want):
+        assert torch.equal(x, y)
