@@ -199,25 +199,26 @@ const int32_t* host_lengths(const MaskDesc& m, int B) { return m.kv_len.size() =
 // Whether the launches of a call may take the forms that only the 16-bit tensor-core kernels read.
 bool takes_16_bit_forms(const Tensor& q) { return q.is_cuda() && q.scalar_type() != at::kFloat && g_impl != JVPFA_IMPL_GENERIC; }
 
-// A ragged bias of the tensors' type with its rows padded to whole 32-byte pieces: the tensor-core kernels take rows of whole 16-byte
-// pieces, the single-pass backward through tO of 32 (`single_pass`; what lies beyond the row's end is not looked at); undefined for every other mask.  Up to one tile of keys a
+// A bias of the tensors' type with its rows padded to whole pieces of 16 elements, where its length does not fill the pieces of `step` that the
+// launch takes: 8, 16 bytes, or 16 for the single-pass backward (padding_for_one_pass; what lies beyond the row's end is not looked at);
+// undefined for every other mask.  Up to one tile of keys a
 // bias is read element by element, whatever its layout.  Dimensions that broadcast are not written out, and the copy lives
 // for one launch: layers that share a bias do not hold a copy each until their backward.  Where there is no memory for it the
 // bias is read in place, by the register-tiled kernels.
-Tensor padded_bias(const MaskDesc& m, const Tensor& q, bool single_pass = false) {
+Tensor padded_bias(const MaskDesc& m, const Tensor& q, int64_t step = 8) {
   if (m.c.kind != JVPFA_MASK_BIAS || !takes_16_bit_forms(q) || m.tensor.scalar_type() != q.scalar_type() || m.c.stride[2] == 0) return {};
-  const int64_t L = q.size(2), step = 16;  // elements
-  if (L <= 64 || L % (single_pass ? step : 8) == 0) return {};
+  const int64_t L = q.size(2), width = (L + 15) / 16 * 16;
+  if (L <= 64 || L % step == 0) return {};
   const int64_t n_b = m.c.stride[0] ? m.tensor.size(0) : 1, n_h = m.c.stride[1] ? m.tensor.size(1) : 1;
   Tensor padded;
   try {
-    padded = empty({n_b, n_h, L, (L + step - 1) / step * step}, m.tensor.scalar_type(), m.tensor.device());
+    padded = empty({n_b, n_h, L, width}, m.tensor.scalar_type(), m.tensor.device());
   } catch (const c10::OutOfMemoryError&) {
     return {};
   }
   jvpfa_pad_bias_args a{};
   a.struct_size = sizeof(a);
-  a.n_b = (int)n_b, a.n_h = (int)n_h, a.L = (int)L, a.width = (int)padded.size(3);
+  a.n_b = (int)n_b, a.n_h = (int)n_h, a.L = (int)L, a.width = (int)width;
   a.mask = m.c;
   a.out = padded.data_ptr();
   check_status(jvpfa_pad_bias(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "jvpfa_pad_bias");
@@ -231,6 +232,22 @@ jvpfa_mask c_mask(const MaskDesc& m, const Tensor& padded) {
     for (int d = 0; d < 4; ++d) c.stride[d] = padded.size(d) == 1 ? 0 : padded.stride(d);
   }
   return c;
+}
+
+// Whether a backward becomes one pass when its bias gets rows of whole 32-byte pieces, which those of L % 16 == 8 are not.  The library's own rule is
+// asked: where it stays with two launches they would read a copy that nobody needs (bf16 through tO, backward with / without it, us: B2 H12 L4104 D64,
+// 0.8 GB of bias, 1523 / 1247, B1 H64 L2056 D64 1060 / 886, D = 32 B1 H61 L2056 988 / 835).
+bool padding_for_one_pass(const jvpfa_bwd_args& a) {
+  if (a.mask.kind != JVPFA_MASK_BIAS || a.dtype == JVPFA_FP32 || a.L <= 64 || a.L % 16 != 8 || !g_single_pass) return false;
+  if (jvpfa_bwd_workspace(&a) > 0) return false;
+  jvpfa_bwd_args padded = a;
+  const int64_t width = a.L + 8, n_h = a.mask.stride[1] ? a.H : 1;
+  padded.mask.ptr = a.q;  // any 16-byte aligned address; nothing is read
+  padded.mask.stride[0] = a.mask.stride[0] ? n_h * a.L * width : 0;
+  padded.mask.stride[1] = a.mask.stride[1] ? a.L * width : 0;
+  padded.mask.stride[2] = width;
+  padded.mask.stride[3] = 1;
+  return jvpfa_bwd_workspace(&padded) > 0;
 }
 
 // Whether the mask's own entries can be read as 16-byte pieces of its rows.
@@ -456,11 +473,6 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   if (!(skip & JVPFA_SKIP_DQ)) g[0] = empty(sizes, q.scalar_type(), q.device());
   if (!(skip & JVPFA_SKIP_DKDV))
     for (int i = 1; i < 3; ++i) g[i] = empty(sizes, q.scalar_type(), q.device());
-  // (whether the single pass takes the bias then: bwd_parts_workspace)
-  const int64_t key_tiles = (sizes[2] + 127) / 128 * sizes[0] * sizes[1];
-  const bool one_pass = g_single_pass && !(skip & JVPFA_SKIP_DKDV) &&
-                        (sizes[3] == 32 ? sizes[2] >= 1024 || key_tiles >= 75 : gto.defined() && sizes[3] == 64 && key_tiles >= 96);
-  const Tensor padded = padded_bias(m, q, one_pass);
   jvpfa_bwd_args a{};
   a.struct_size = sizeof(a);
   a.dtype = p.dtype;
@@ -474,7 +486,7 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.flags = skip | (single ? JVPFA_DQ_ACCUM_IS_ZERO : 0) | (tq.defined() && !tk.defined() ? JVPFA_ZERO_TKV : 0);
   if (g[0].defined()) a.dq = g[0].data_ptr();
   if (g[1].defined()) a.dk = g[1].data_ptr(), a.dv = g[2].data_ptr();
-  a.mask = c_mask(*call.mask, padded);
+  a.mask = m.c;
   const bool fp32 = q.scalar_type() == at::kFloat;
   if (!fp32 && m.tile_live.defined() && m.tile_live_t.defined() && a.L <= 8192) {
     a.mask_tile_live = data(m.tile_live);
@@ -487,6 +499,8 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.tq = data(in.tq), a.tk = data(in.tk), a.tv = data(in.tv);
   for (int d = 0; d < 3; ++d) a.in_stride[d] = in.st[d];
   a.kv_len_host = host_lengths(m, a.B);
+  const Tensor padded = padded_bias(m, q, padding_for_one_pass(a) ? 16 : 8);
+  a.mask = c_mask(m, padded);
   const Tensor workspace = workspace_of((fp32 ? call.parts : g_single_pass.load()) ? jvpfa_bwd_workspace(&a) : 0, q);
   const Tensor bits = use_workspace(a, workspace, call, q);
   if (fp32 && !workspace.defined() && a.L <= 8192) {
