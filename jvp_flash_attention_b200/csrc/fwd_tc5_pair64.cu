@@ -777,7 +777,7 @@ fwd_tc5_pair64_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPairMap
             uint32_t w0[4], w1[4];
             lds_v4(brow_sm + (((uint32_t)q ^ bsw) << 4), w0);
             lds_v4(brow_sm + (((uint32_t)(4 + q) ^ bsw) << 4), w1);
-            if (q == 3) mbar_arrive_behind(b_empty + X, w1[3]);
+            if (q == 3) mbar_arrive_behind(b_empty + X, w1[3], opaque_zero(a));
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const int c = 4 * q + e;

@@ -417,7 +417,7 @@ fwd_tc5_pipe128_kernel(const jvpfa_fwd_args a, const __grid_constant__ FwdPipeMa
           x0[2 * c] = __float_as_uint(v0.x), x0[2 * c + 1] = __float_as_uint(v0.y);
           x1[2 * c] = __float_as_uint(v1.x), x1[2 * c + 1] = __float_as_uint(v1.y);
           mx0 = fmaxf(mx0, v0.x), mx1 = fmaxf(mx1, v0.y), mx2 = fmaxf(mx2, v1.x), mx3 = fmaxf(mx3, v1.y);
-          if (MK == 2 && c == 15) mbar_arrive_behind(b_empty, w1[3]);
+          if (MK == 2 && c == 15) mbar_arrive_behind(b_empty, w1[3], opaque_zero(a));
         }
         mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
       }

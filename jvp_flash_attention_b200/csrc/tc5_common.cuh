@@ -172,14 +172,16 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 // ... when `v`, the word that a warp's last load from shared memory returns, is there (they return in their order).  An arrival does not wait for loads from shared memory in flight, and may
 // overtake them: one that stood right behind a tile's last load (16 softmax warps, the smem port busy with the first tiles of a CTA) let
-// the next tile be copied over what those loads had yet to read, once in about fifty launches.  (Nothing is greater than infinity; a
-// predicate is what keeps the instruction behind v.)
-__device__ __forceinline__ void mbar_arrive_behind(uint64_t* bar, uint32_t v) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.gt.f32 p, %1, 0f7F800000;\n\t"
-      "@!p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar)), "f"(__uint_as_float(v))
-      : "memory");
+// the next tile be copied over what those loads had yet to read, once in about fifty launches.  The barrier's address is formed with v, of which
+// `none` keeps no bit: a value that is zero in every launch and that no compiler knows (opaque_zero), so that nothing can take the arrival for one
+// that does not depend on v.
+__device__ __forceinline__ void mbar_arrive_behind(uint64_t* bar, uint32_t v, uint32_t none) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar) + (v & none)) : "memory");
+}
+// The sign of a launch's struct_size, which the host has compared with the size itself.
+template <typename Args>
+__device__ __forceinline__ uint32_t opaque_zero(const Args& a) {
+  return (uint32_t)(a.struct_size >> 31);
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
