@@ -1095,10 +1095,13 @@ static cudaError_t run_fused64_d(const jvpfa_bwd_args& a, const BwdFMaps& m, flo
 
 template <typename T, bool HAS_GO, bool HAS_GT, int MK, bool CUT>
 static cudaError_t run_fused64(const jvpfa_bwd_args& a, const BwdFMaps& m, float* dq_acc, float* shares, int* status, int grid, cudaStream_t stream) {
-  if constexpr (MK == 2)
-    if ((a.L & 15) != 0)
-      return a.D == 32 ? run_fused64_d<T, HAS_GO, HAS_GT, MK, CUT, 32, true>(a, m, dq_acc, shares, status, grid, stream)
-                       : run_fused64_d<T, HAS_GO, HAS_GT, MK, CUT, 64, true>(a, m, dq_acc, shares, status, grid, stream);
+  if constexpr (MK == 2) {
+    if ((a.L & 15) != 0) {
+      // (D = 64 through O alone: bwd_tc5_fused64_eligible takes no ragged bias)
+      if (!HAS_GT || a.D == 32) return run_fused64_d<T, HAS_GO, HAS_GT, MK, CUT, 32, true>(a, m, dq_acc, shares, status, grid, stream);
+      if constexpr (HAS_GT) return run_fused64_d<T, HAS_GO, HAS_GT, MK, CUT, 64, true>(a, m, dq_acc, shares, status, grid, stream);
+    }
+  }
   return a.D == 32 ? run_fused64_d<T, HAS_GO, HAS_GT, MK, CUT, 32, false>(a, m, dq_acc, shares, status, grid, stream)
                    : run_fused64_d<T, HAS_GO, HAS_GT, MK, CUT, 64, false>(a, m, dq_acc, shares, status, grid, stream);
 }
@@ -1193,12 +1196,11 @@ static int launch_fused64_t(const jvpfa_bwd_args& a, cudaStream_t s) {
 
 }  // namespace tc5
 
-// The single-pass kernel serves D = 64 with index masks (none, causal, key padding), boolean masks that come without tile
-// bitmaps, and a bias of the tensors' type, when the caller provides the fp32 buffer for dQ: dq_accum, or for a bias through tO
-// the workspace, in which dQ is summed in a fixed order.
-// What dq_accum takes is summed in no fixed order, so only what callers know to be summed so goes there: not head dimension 32,
-// nor masks and bias whose rows are not whole 16-byte pieces, which the kernels of a fixed order have always served (B4 H8 L1000
-// D32, both outputs: 85 us here, 99 us there; a whole step: 209 us with either).
+// The single-pass kernel serves, where the caller provides a place for dQ:
+//   D = 64, in dq_accum: index masks (none, causal, key padding), boolean masks that come without tile bitmaps, and through O alone a
+//           bias of the tensors' type.  What goes there is summed in no fixed order, so masks and bias whose rows are not whole 16-byte
+//           pieces, which kernels of a fixed order have always served, stay with those
+//   D = 64 with a bias through tO, and D = 32, in the workspace, where dQ is summed in a fixed order: bwd_parts_workspace
 bool bwd_tc5_fused64_eligible(const jvpfa_bwd_args& a) {
   const int k = a.mask.kind;
   if (tc5::dq_parts(a)) {
