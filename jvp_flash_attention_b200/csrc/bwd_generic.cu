@@ -636,7 +636,7 @@ static int launch_bwd_d(const jvpfa_bwd_args& a, cudaStream_t s) {
   const long long rows16 = tiles16(a.B, a.H, a.L);
   if (rows16 >= kBwdRowsFrom<T, D> && (!a.gto || kBwdRowsDual<T, D>)) return launch_bwd_rows(a, s);  // (JVPFA_ZERO_TKV: fp32 with gto)
   if constexpr (!Elem<T>::k16) {
-    const int rg = row_groups(a.B, a.H, a.L, a.gto != nullptr, a.mask.kind == JVPFA_MASK_CAUSAL, 132, 115);
+    const int rg = row_groups(a.B, a.H, a.L, a.gto != nullptr, a.mask.kind == JVPFA_MASK_CAUSAL, kBwdRowGroups<T, D>);
     if (rg == 1) return launch_bwd_split<T, D, 1, 8>(a, s);
     if (rg == 2) return launch_bwd_split<T, D, 2, 4>(a, s);
   }

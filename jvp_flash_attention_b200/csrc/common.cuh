@@ -558,23 +558,49 @@ __device__ __forceinline__ bool dead_queries(const jvpfa_bwd_args& a, int b, int
                 rows ? (m1 - 1) >> 7 : 0);
 }
 
-// 16-row groups of a CTA of the fp32 register-tiled kernels, 1, 2 or 4 (and 8, 4 or 2 parts of the loop side): 64 rows share every tile that is
-// brought in, and 16 take cost1 percent of their time for a row, 32 cost2; but one CTA fills an SM, so what counts are rounds of 148.  Causal: as
-// much work as half the rows, and the longest CTA comes on top.  Measured against the model on a B200, us by 16 / 32 / 64 rows, D = 128, forward with
-// tangents and backward through tO: B1 H37 L512 (2 rounds of 64 rows) 493 / 398 / 342 and 1231 / 1100 / 911, B3 H7 L256 99 / 106 / 90 and 238 /
-// 281 / 231, B2 H12 L512 356 / 299 / 340 and 895 / 815 / 895, B2 H5 L1920 causal 965 / 933 / 1047 and 2407 / 2522 / 2709; D = 32 B2 H4 L256 13 / 18 /
-// 26 and 32 / 50 / 80.  (By the number of rows alone, 64 from 592 groups of 16 on and 32 from 296: 281, 895 and 2709.)
+// 16-row groups of a CTA of the fp32 register-tiled kernels with tangents, 1, 2 or 4 (and 8, 4 or 2 parts of the loop side).  64 rows share every tile
+// that is brought in, and 16 take cost1 percent of their time for a row, 32 cost2, but a launch takes rounds of as many CTAs as 148 SMs hold: fit of
+// each kind on one, of which each but the first adds `beside` percent of its time.  Causal: half the work, evened out, and `tail` percent of a CTA's.
+// `fit` is what registers and shared memory allow (-Xptxas -v: D >= 64 takes 129 to 255 registers at 256 threads, but for TF32's backward in 32
+// rows; D = 32 at most 128, and 80 in TF32's backward in 32 rows), the rest a fit to 2896 draws on a B200 (B*H of 1 to 300, L of 66 to 2400, 60 to 1500
+// groups, forward and backward through tO), in each of which all three kinds were timed.  Slower than the best of the three by so much in the mean, of
+// draws where they differ, by the number of rows alone (64 from 592 groups on, 32 from 296) / as if one CTA of any filled an SM, with cost1 of 145
+// and 132 / by this rule: fp32 forward D = 32 6.4 / 3.4 / 1.5 %, 64 4.7 / 0.7 / 0.7, 128 4.7 / 1.0 / 0.6, backward 7.1 / 2.3 / 1.0, 8.0 / 3.0 / 0.8,
+// 7.7 / 1.5 / 0.8; TF32 forward 4.0 / 6.0 / 1.5, 8.1 / 5.4 / 1.1, 7.9 / 0.8 / 0.3, backward 3.3 / 4.6 / 0.7, 10.4 / 12.6 / 0.5, 6.7 / 6.0 / 0.4.  us by 16 /
+// 32 / 64 rows: TF32 backward D = 64 B1 H241 L92 causal 146 / 72 / 99, forward D = 32 B3 H41 L66 19 / 15 / 11; fp32 forward D = 32 B1 H131 L76 25 / 19 / 19,
+// backward D = 64 B1 H282 L72 218 / 157 / 187.
 // Without tangents two CTAs of short row tiles fit an SM, and the number of rows does decide (B1 H2 L1410, 16 / 32 rows: 84 / 109).
-inline int row_groups(int B, int H, int L, bool tangents, bool causal, int cost1, int cost2) {
+struct RowGroups {
+  int fit[3];
+  int cost1, cost2, beside, tail;
+};
+template <typename T, int D>
+constexpr RowGroups kFwdRowGroups = Elem<T>::kSplit ? (D == 32   ? RowGroups{{2, 2, 2}, 174, 111, 25, 217}
+                                                       : D == 64 ? RowGroups{{1, 1, 1}, 179, 110, 0, 180}
+                                                                 : RowGroups{{1, 1, 1}, 175, 102, 0, 225})
+                                                    : (D == 32   ? RowGroups{{2, 2, 2}, 194, 137, 14, 60}
+                                                       : D == 64 ? RowGroups{{1, 1, 1}, 219, 151, 0, 75}
+                                                                 : RowGroups{{1, 1, 1}, 146, 103, 0, 63});
+template <typename T, int D>
+constexpr RowGroups kBwdRowGroups = Elem<T>::kSplit ? (D == 32   ? RowGroups{{2, 2, 2}, 134, 111, 56, 97}
+                                                       : D == 64 ? RowGroups{{1, 1, 1}, 158, 108, 0, 143}
+                                                                 : RowGroups{{1, 1, 1}, 135, 114, 0, 88})
+                                                    : (D == 32   ? RowGroups{{2, 3, 2}, 153, 147, 18, 32}
+                                                       : D == 64 ? RowGroups{{1, 2, 1}, 216, 132, 48, 244}
+                                                                 : RowGroups{{1, 1, 1}, 222, 150, 0, 89});
+inline int row_groups(int B, int H, int L, bool tangents, bool causal, const RowGroups& kinds) {
   const long long rows16 = tiles16(B, H, L);
   if (!tangents) return rows16 < 2 * 148 ? 1 : rows16 < 4 * 148 ? 2 : 4;
   const long long BH = (long long)B * H;
-  auto time = [&](int rg, int cost) {
-    const long long ctas = BH * ((L + 16 * rg - 1) / (16 * rg));
-    return (causal ? ctas * rg + 2 * 148 * rg : (ctas + 147) / 148 * rg * 2 * 148) * cost;
+  auto time = [&](int rg, int fit, int cost) {
+    const long long ctas = BH * ((L + 16 * rg - 1) / (16 * rg)), deep = (ctas + 147) / 148, last = deep % fit;
+    const int full = 100 + (fit - 1) * kinds.beside;
+    const double t = causal ? (double)(ctas * full) / (2 * 148 * fit) + kinds.tail
+                            : (double)(deep / fit * full + (last ? 100 + (last - 1) * kinds.beside : 0));
+    return t * rg * cost;
   };
-  const long long one = time(1, cost1), two = time(2, cost2), four = time(4, 100);
-  return four <= one && four <= two ? 4 : two <= one ? 2 : 1;
+  const double one = time(1, kinds.fit[0], kinds.cost1), two = time(2, kinds.fit[1], kinds.cost2), four = time(4, kinds.fit[2], 100);
+  return one <= two && one <= four ? 1 : two <= four ? 2 : 4;
 }
 
 // Host-side launch helpers implemented by each kernel translation unit.

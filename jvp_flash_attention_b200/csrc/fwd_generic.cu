@@ -445,7 +445,7 @@ static int launch_d(const jvpfa_fwd_args& a, cudaStream_t s) {
   const long long rows16 = tiles16(a.B, a.H, a.L);
   if (rows16 >= kFwdRowsFrom<T, D> && !(a.flags & JVPFA_ZERO_TKV) && (!a.tq || kFwdRowsDual<T, D>)) return launch_fwd_rows(a, s);
   if constexpr (!Elem<T>::k16) {
-    const int rg = row_groups(a.B, a.H, a.L, a.tq != nullptr, a.mask.kind == JVPFA_MASK_CAUSAL, 145, 122);
+    const int rg = row_groups(a.B, a.H, a.L, a.tq != nullptr, a.mask.kind == JVPFA_MASK_CAUSAL, kFwdRowGroups<T, D>);
     if (rg == 1) return launch_split<T, D, 1, 8>(a, s);
     if (rg == 2) return launch_split<T, D, 2, 4>(a, s);
   }
