@@ -42,6 +42,19 @@ def test_rows_are_padded(L, layout, dt):
         assert torch.equal(out[..., :L], want) and not out[..., L:].any()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,width", [(1, 8), (33, 128), (113, 120), (120, 128), (121, 128), (128, 136), (129, 136), (249, 256), (250, 256), (255, 264), (505, 512), (506, 520), (1023, 1024), (1025, 1032)])
+@pytest.mark.parametrize("heads", [(1, 1), (3, 5)])
+def test_edges_of_what_a_warp_takes(L, width, heads):
+    """Rows of up to 128, 256, 512 and more elements, and heads that end within a block's rows: entries bit for bit, zeros behind them, nothing elsewhere."""
+    g = torch.Generator(device=DEV).manual_seed(L)
+    m = torch.randn(*heads, L, L, generator=g, device=DEV).to(torch.bfloat16)
+    out = torch.full((heads[0] * heads[1] * L * width + 64,), 3.0, dtype=m.dtype, device=DEV)
+    view = out[:-64].view(*heads, L, width)
+    _lib.check(_lib.load().jvpfa_pad_bias(ctypes.byref(_args(m, view)), torch.cuda.current_stream().cuda_stream), "jvpfa_pad_bias")
+    assert torch.equal(view[..., :L], m) and not view[..., L:].any() and (out[-64:] == 3).all()
+
+
 def test_what_is_refused():
     """Host logic, before anything is launched."""
     m, out = torch.zeros(1, 1, 66, 66, dtype=torch.float16), torch.zeros(1, 1, 66, 72, dtype=torch.float16)
