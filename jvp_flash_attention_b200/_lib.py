@@ -330,7 +330,7 @@ class MaskSpec:
     bias, or int32 kv_len) and ``strides`` are the broadcast element strides of a (B,H,L,L) view.
     """
 
-    __slots__ = ("kind", "tensor", "strides", "bias_dtype", "tile_live", "tile_live_t", "fp32_mode", "fp32_parts", "kv_len_host", "_native")
+    __slots__ = ("kind", "tensor", "strides", "bias_dtype", "tile_live", "tile_live_t", "tile_dead", "fp32_mode", "fp32_parts", "kv_len_host", "_native")
 
     def __init__(self, kind=MASK_NONE, tensor=None, strides=(0, 0, 0, 0), bias_dtype=FP32):
         self.kind = kind
@@ -339,6 +339,7 @@ class MaskSpec:
         self.bias_dtype = bias_dtype
         self.tile_live = None  # MASK_BOOL: bitmap from mask_tiles(), lets the forward step over dead tiles
         self.tile_live_t = None  # ... and its transpose (per 128-key tile), for the backward launch that owns keys
+        self.tile_dead = 1.0  # ... and the share of tiles that are dead, as far as it was counted
         self.kv_len_host = None  # MASK_KVLEN: the lengths once more, as a list: whether cutting tiles pays goes by them
         self._native = None  # the native layer's form of this description, made on first use
         self.fp32_parts = False  # the forward of this call had a workspace for the fp32 tcgen05 kernels: so does a backward through O
@@ -348,7 +349,7 @@ class MaskSpec:
         """This (by now complete) description as the native layer takes it."""
         if self._native is None:
             self._native = native().MaskDesc(self.kind, self.bias_dtype, self.tensor, self.strides, self.tile_live,
-                                             self.tile_live_t, self.kv_len_host or [], copy.copy(self))
+                                             self.tile_live_t, self.kv_len_host or [], self.tile_dead, copy.copy(self))
         return self._native
 
     def to_c(self) -> Mask:

@@ -58,11 +58,13 @@ struct MaskDesc {
   jvpfa_mask c{};
   Tensor tensor, tile_live, tile_live_t;
   std::vector<int32_t> kv_len;  // JVPFA_MASK_KVLEN: the lengths on the host
+  double dead;                  // with tile bitmaps: the share of tiles that verification found without a true entry
   std::shared_ptr<py::object> spec;
 
   MaskDesc(int kind, int bias_dtype, std::optional<Tensor> t, std::array<int64_t, 4> strides, std::optional<Tensor> live,
-           std::optional<Tensor> live_t, std::vector<int32_t> kv_len_, py::object spec_)
+           std::optional<Tensor> live_t, std::vector<int32_t> kv_len_, double dead_, py::object spec_)
       : kv_len(std::move(kv_len_)),
+        dead(dead_),
         spec(new py::object(std::move(spec_)), [](py::object* o) {
           py::gil_scoped_acquire gil;
           delete o;
@@ -307,10 +309,16 @@ void pack_mask(Call& call, const Tensor& q, bool backward) {
 // tiles to step over.  These launches visited every tile before they knew of bitmaps, and their results were the mask's present entries' whatever
 // had been written since; so theirs are made anew, like the bits (B1 H8 L2048, a window as one (L, L) mask: 5 us).  The 16-bit
 // kernels are given those of the verification.  Left undefined where there is no memory: every tile is visited then.
-void make_tiles(Call& call, const Tensor& q) {
+// And where dead tiles are no more than the bitmaps cost: 11 us of the launch by a rough model of it, in which a key takes 0.03 us, and more where
+// there are rows for every SM.  Of 550 forwards on a B200 (windows of a quarter and half the length, key padding, L 160 to 3000), with bitmaps made
+// for all 148 took more than 3 % longer than without any, up to 1.79 times (TF32 B1 H7 L170 D32 7.5 / 13.5 us); by this rule 5, 1.14 at most, and
+// of the 309 that gain as much 284 have them.  Of 573 backward launches that find none 349 gain, 7 more would, and 25 take longer, 1.09 at most.
+void make_tiles(Call& call, const Tensor& q, bool tangents, bool backward) {
   const MaskDesc& m = *call.mask;
   if (call.tiles.defined() || q.scalar_type() != at::kFloat || !m.tile_live.defined() || !m.tile_live_t.defined()) return;
   const int64_t L = q.size(2), n = m.tile_live.numel();
+  const double deep = (double)(q.size(0) * q.size(1) * ((L + 15) / 16)) / 148, width = (double)q.size(3) / 32 * (tangents ? 1.8 : 1) * (call.tf32 ? 1 : 1.8);
+  if (m.dead * L * (0.03 + 0.004 * width * deep) * (backward ? 1.5 : 1) < 11) return;
   jvpfa_mask_tiles_args a{};
   a.struct_size = sizeof(a);
   a.n_b = m.c.stride[0] ? (int)m.tensor.size(0) : 1, a.n_h = m.c.stride[1] ? (int)m.tensor.size(1) : 1;
@@ -409,7 +417,7 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   const Tensor bits = use_workspace(a, workspace, call, q);
   r.parts = fp32 && workspace.defined();
   if (fp32 && !r.parts) {
-    make_tiles(call, q);
+    make_tiles(call, q, dual, false);
     a.mask_tile_live = data(call.tiles);
   }
   check_status(jvpfa_fwd(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "jvpfa_fwd");
@@ -504,7 +512,7 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   const Tensor workspace = workspace_of((fp32 ? call.parts : g_single_pass.load()) ? jvpfa_bwd_workspace(&a) : 0, q);
   const Tensor bits = use_workspace(a, workspace, call, q);
   if (fp32 && !workspace.defined() && a.L <= 8192) {
-    make_tiles(call, q);
+    make_tiles(call, q, gto.defined(), true);
     if (call.tiles.defined()) a.mask_tile_live = call.tiles.data_ptr(), a.mask_tile_live_t = static_cast<int64_t*>(call.tiles.data_ptr()) + m.tile_live.numel();
   }
   check_status(jvpfa_bwd(&a, stream), "jvpfa_bwd");
@@ -818,7 +826,7 @@ PYBIND11_MODULE(_native, m) {
       .def("__exit__", [](NoFunctorchScope& s, py::args) { s.guard.reset(); });
   py::class_<MaskDesc, MaskPtr>(m, "MaskDesc")
       .def(py::init<int, int, std::optional<Tensor>, std::array<int64_t, 4>, std::optional<Tensor>, std::optional<Tensor>,
-                    std::vector<int32_t>, py::object>());
+                    std::vector<int32_t>, double, py::object>());
   m.def("attend", &attend);
   m.def("set_impl", [](int v) { g_impl = v; });
   m.def("set_single_pass", [](bool v) { g_single_pass = v; });

@@ -221,6 +221,7 @@ def _classify_mask_tensor(attn_mask: Tensor, Z: int, H: int, N: int, verify: boo
             *heads, n_live = head_live.tolist()  # the one read-back
             every_head_live = all(heads)
             n_entries = spec.tile_live.numel() // (((N + 63) // 64 + 63) // 64)
+            spec.tile_dead = 1.0 - n_live / (n_entries * ((N + 63) // 64))
             if n_live > 0.85 * n_entries * ((N + 63) // 64):
                 spec.tile_live = spec.tile_live_t = None  # (nearly) every tile is live: the plain loops are quicker
         assert every_head_live, "The attention mask cannot be all False for any head."

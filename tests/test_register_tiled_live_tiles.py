@@ -130,3 +130,26 @@ def test_a_window_written_behind_the_version_counter(how, B, H, L, D):
         graph.replay()
     for x, y in zip(got, want):
         assert torch.equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,L,D,tangents,made", [(1, 7, 170, 32, False, False), (4, 1, 370, 64, False, False), (6, 6, 450, 64, True, True), (1, 1, 2600, 32, False, True)])
+def test_bitmaps_are_made_where_they_pay(B, H, L, D, tangents, made):
+    """fp32: one allocation more than a call without a mask has, or none."""
+    g = torch.Generator().manual_seed(L)
+    ts = [torch.randn(B, H, L, D, generator=g).to(DEV) for _ in range(6)]
+    window = _mask("window", 1, 1, L, g).to(DEV).expand(B, H, L, L)
+
+    def allocations(m):
+        call = lambda *x: ja.JVPAttn.fwd_dual(*x, attn_mask=m) if tangents else ja.attention(*x, attn_mask=m)  # noqa: E731
+        for _ in range(2):  # the first verifies the mask
+            before = torch.cuda.memory_stats()["allocation.all.allocated"]
+            with torch.no_grad():
+                torch.func.jvp(call, tuple(ts[:3]), tuple(ts[3:])) if tangents else call(*ts[:3])
+        return torch.cuda.memory_stats()["allocation.all.allocated"] - before
+
+    prev = ja.set_fp32_precision("tf32")
+    try:
+        assert allocations(window) - allocations(None) == made
+    finally:
+        ja.set_fp32_precision(prev)
