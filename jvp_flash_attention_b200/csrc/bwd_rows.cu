@@ -289,9 +289,14 @@ __global__ void __launch_bounds__(128) bwd_dkdv_rows_kernel(const jvpfa_bwd_args
   smem_tile_to_global<T, BN, D, NT>(reinterpret_cast<T*>(a.dv) + head_off, sV, LD, n0, L, tid);
 }
 
+// CTAs of a dQ kernel that an SM shall hold, where ptxas by itself stays just above the registers for them (0: as it comes).  TF32 D = 32 through both
+// outputs takes 178, of which two fit, and 164 without a spill; both launches, us: B1 H37 L610 314 -> 260, with a bias B2 H13 L1016 1137 -> 889.
+template <typename T, int D, bool HAS_GT>
+constexpr int kDqRowsAnSm = !Elem<T>::k16 && !Elem<T>::kSplit && D == 32 && HAS_GT ? 3 : 0;
+
 // ---- dQ: CTA owns 64 queries, loops over key tiles (rows = queries, columns = keys). ----
 template <typename T, int D, bool HAS_GO, bool HAS_GT, bool TILES>
-__global__ void __launch_bounds__(128) bwd_dq_rows_kernel(const jvpfa_bwd_args a) {
+__global__ void __launch_bounds__(128, kDqRowsAnSm<T, D, HAS_GT>) bwd_dq_rows_kernel(const jvpfa_bwd_args a) {
   using C = BwdRowsCfg<T, D>;
   constexpr int BM = C::OWN, BN = C::LOOP, LD = C::LD, NT = C::NTHREADS, STAGES = C::STAGES;
   constexpr int NK = BN / 8;

@@ -20,9 +20,14 @@ struct FwdRowsCfg {
   }
 };
 
+// CTAs that an SM shall hold, where ptxas by itself stays just above the registers for them (0: as it comes).  TF32 D = 32 takes 91
+// registers, of which five fit, and 80 without a spill: with a bias B2 H69 L336 100 -> 69 us, B1 H160 L268 77 -> 59.
+template <typename T, int D, bool DUAL>
+constexpr int kFwdRowsAnSm = !Elem<T>::k16 && !Elem<T>::kSplit && D == 32 && !DUAL ? 6 : 0;
+
 // TILES: key tiles without a true mask entry are left out (dead_keys).
 template <typename T, int D, bool DUAL, bool TILES>
-__global__ void __launch_bounds__(128) fwd_rows_kernel(const jvpfa_fwd_args a) {
+__global__ void __launch_bounds__(128, kFwdRowsAnSm<T, D, DUAL>) fwd_rows_kernel(const jvpfa_fwd_args a) {
   using C = FwdRowsCfg<T, D>;
   constexpr int BM = C::BM, BN = C::BN, LD = C::LD, NT = C::NTHREADS;
   constexpr int KS = Elem<T>::kKStep;
