@@ -136,7 +136,7 @@ bool encode_map_parts(CUtensorMap* m, const void* ptr, int D, int L, int BH, int
 
 // Head dimension 32 runs on the D = 64 kernels: the tensor maps end at column 32, so TMA fills the other half of every tile with zeros and clips what is stored, and the contractions over D stop
 // half-way.  An MMA costs the same for 32 output columns as for 64, so little is wasted (B4 H8 L1000, bf16: forward with tangents
-// 150 -> 46 us, backward through both outputs 325 -> 99 us, now 60, against the register-tiled kernels).  Up to one 64-row tile the
+// 150 -> 46 us, backward through both outputs 325 -> 99 us in two launches, 58 in one, against the register-tiled kernels).  Up to one 64-row tile the
 // register-tiled kernels stay: a 256-row pair of query tiles would be mostly padding.
 bool tc5_head_dim(int D, int L) { return D == 64 || D == 128 || (D == 32 && L > 64); }
 
