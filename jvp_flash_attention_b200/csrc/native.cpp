@@ -95,7 +95,7 @@ struct Call {
   // A boolean mask as bits, by rows and transposed: the form the 16-bit tensor-core kernels read best, made by this call for
   // its forward and backward (pack_mask).
   Tensor bits, bits_t;
-  Tensor tiles;  // fp32: both tile bitmaps, made by this call for its register-tiled launches (make_tiles)
+  Tensor tiles;  // fp32: both tile bitmaps, made by this call's forward for its register-tiled launches (make_tiles)
 
   void drop_tensors() { bits = bits_t = tiles = Tensor(); }
 };
@@ -313,12 +313,12 @@ void pack_mask(Call& call, const Tensor& q, bool backward) {
 // there are rows for every SM.  Of 550 forwards on a B200 (windows of a quarter and half the length, key padding, L 160 to 3000), with bitmaps made
 // for all 148 took more than 3 % longer than without any, up to 1.79 times (TF32 B1 H7 L170 D32 7.5 / 13.5 us); by this rule 5, 1.14 at most, and
 // of the 309 that gain as much 284 have them.  Of 573 backward launches that find none 349 gain, 7 more would, and 25 take longer, 1.09 at most.
-void make_tiles(Call& call, const Tensor& q, bool tangents, bool backward) {
+Tensor make_tiles(const Call& call, const Tensor& q, bool tangents, bool backward) {
   const MaskDesc& m = *call.mask;
-  if (call.tiles.defined() || q.scalar_type() != at::kFloat || !m.tile_live.defined() || !m.tile_live_t.defined()) return;
+  if (q.scalar_type() != at::kFloat || !m.tile_live.defined() || !m.tile_live_t.defined()) return {};
   const int64_t L = q.size(2), n = m.tile_live.numel();
   const double deep = (double)(q.size(0) * q.size(1) * ((L + 15) / 16)) / 148, width = (double)q.size(3) / 32 * (tangents ? 1.8 : 1) * (call.tf32 ? 1 : 1.8);
-  if (m.dead * L * (0.03 + 0.004 * width * deep) * (backward ? 1.5 : 1) < 11) return;
+  if (m.dead * L * (0.03 + 0.004 * width * deep) * (backward ? 1.5 : 1) < 11) return {};
   jvpfa_mask_tiles_args a{};
   a.struct_size = sizeof(a);
   a.n_b = m.c.stride[0] ? (int)m.tensor.size(0) : 1, a.n_h = m.c.stride[1] ? (int)m.tensor.size(1) : 1;
@@ -330,12 +330,12 @@ void make_tiles(Call& call, const Tensor& q, bool tangents, bool backward) {
     at::AutoDispatchBelowADInplaceOrView below;
     tiles = at::zeros({n + m.tile_live_t.numel()}, q.options().dtype(at::kLong).requires_grad(false));
   } catch (const c10::OutOfMemoryError&) {
-    return;
+    return {};
   }
   a.tile_live = tiles.data_ptr();
   a.tile_live_t = static_cast<int64_t*>(tiles.data_ptr()) + n;
   check_status(jvpfa_mask_tiles(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "jvpfa_mask_tiles");
-  call.tiles = tiles;
+  return tiles;
 }
 
 // ---- launches ------------------------------------------------------------------------------------------------------
@@ -417,7 +417,7 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   const Tensor bits = use_workspace(a, workspace, call, q);
   r.parts = fp32 && workspace.defined();
   if (fp32 && !r.parts) {
-    make_tiles(call, q, dual, false);
+    call.tiles = make_tiles(call, q, dual, false);
     a.mask_tile_live = data(call.tiles);
   }
   check_status(jvpfa_fwd(&a, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "jvpfa_fwd");
@@ -426,7 +426,7 @@ FwdResult launch_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
 
 // Gradients of <go, O> + <gto, tO> with respect to q, k, v; those named in `skip` (JVPFA_SKIP_*) stay undefined.
 Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, Tensor tk, Tensor tv, const Tensor& o, Tensor to,
-                 const Tensor& lse, Tensor mu, Tensor go, Tensor gto, Call& call, int skip = 0) {
+                 const Tensor& lse, Tensor mu, Tensor go, Tensor gto, const Call& call, int skip = 0) {
   if (!q.is_cuda()) {
     py::gil_scoped_acquire gil;
     NoFunctorch nf;
@@ -511,9 +511,11 @@ Grads launch_bwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor tq, T
   a.mask = c_mask(m, padded);
   const Tensor workspace = workspace_of((fp32 ? call.parts : g_single_pass.load()) ? jvpfa_bwd_workspace(&a) : 0, q);
   const Tensor bits = use_workspace(a, workspace, call, q);
+  // (Bitmaps that a backward makes are its own: of one that is being captured they hold nothing before a replay, and another may come first.)
+  Tensor tiles;
   if (fp32 && !workspace.defined() && a.L <= 8192) {
-    make_tiles(call, q, gto.defined(), true);
-    if (call.tiles.defined()) a.mask_tile_live = call.tiles.data_ptr(), a.mask_tile_live_t = static_cast<int64_t*>(call.tiles.data_ptr()) + m.tile_live.numel();
+    tiles = call.tiles.defined() ? call.tiles : make_tiles(call, q, gto.defined(), true);
+    if (tiles.defined()) a.mask_tile_live = tiles.data_ptr(), a.mask_tile_live_t = static_cast<int64_t*>(tiles.data_ptr()) + m.tile_live.numel();
   }
   check_status(jvpfa_bwd(&a, stream), "jvpfa_bwd");
   return g;
@@ -624,7 +626,7 @@ struct AttnBwdNode : public Node {
 };
 
 Grads backward_through_o(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& go,
-                         Call& call, int skip) {
+                         const Call& call, int skip) {
   if (is_wrapped(go)) {  // the cotangent belongs to a functorch transform: a Function, which the transform differentiates or refuses
     py::gil_scoped_acquire gil;
     py::tuple g = python_module().attr("_backward_under_functorch")(q, k, v, o, lse, go, *call.mask->spec, call.scale, call.tf32, call.parts);

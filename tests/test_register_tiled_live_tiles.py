@@ -153,3 +153,26 @@ def test_bitmaps_are_made_where_they_pay(B, H, L, D, tangents, made):
         assert allocations(window) - allocations(None) == made
     finally:
         ja.set_fp32_precision(prev)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L", [400, 450, 500, 600])
+def test_a_captured_backward_leaves_no_bitmaps_to_others(L):
+    """fp32, forwards that are too short to make bitmaps: a backward of the same graph runs between another's capture and its replay."""
+    g = torch.Generator().manual_seed(L)
+    q, k, v, go = (torch.randn(1, 2, L, 64, generator=g).to(DEV) for _ in range(4))
+    m = _mask("window", 1, 1, L, g).to(DEV)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        a = [x.requires_grad_() for x in (q, k, v)]
+        want = torch.autograd.grad(ja.attention(*a, attn_mask=m), a, go)
+        o = ja.attention(*a, attn_mask=m)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            captured = torch.autograd.grad(o, a, go, retain_graph=True)
+        got = torch.autograd.grad(o, a, go, retain_graph=True)
+        graph.replay()
+    torch.cuda.synchronize()
+    for x, y, z in zip(got, captured, want):
+        assert torch.equal(x, z) and torch.equal(y, z)
